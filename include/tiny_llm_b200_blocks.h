@@ -274,29 +274,30 @@ int tlb_shift_mix(const void *h, long long h_token, const void *mu, int parts, i
 int tlb_moe_route(const void *h, const void *w, const void *b, int tokens, int dim, int experts, int top, int scoring, const void *choice_bias,
                   float weight_scale, int group_count, int group_keep, const void *aux_w, float *aux, int32_t *idx, float *gate, int dtype, void *stream);
 
-/* Rows per expert tile of the grouped products: 32, or 64 for the tensor-core kernels (bf16, reduction length % 8 == 0)
- * when experts get many rows (half the weight traffic per row). */
+/* Rows per tile of the list of pairs grouped by expert. */
 #define TLB_MOE_TILE_ROWS 32
 /* upper bound of sorted rows (pairs grouped by expert, every group padded to whole tiles) */
-long long tlb_moe_max_rows(int tokens, int top, int experts, int tile_rows);
-/* Group the (token, choice) pairs by expert: sorted_pair [max_rows] (pair id or -1), tile_expert [max_rows / tile_rows],
- * counters [2] = {tiles in use, rows in use}.  One launch, no host involvement. */
-int tlb_moe_sort(const int32_t *idx, int tokens, int top, int experts, int tile_rows, int32_t *sorted_pair, int32_t *tile_expert,
-                 int32_t *counters, void *stream);
+long long tlb_moe_max_rows(int tokens, int top, int experts);
+/* int32 values of the lists that tlb_moe_sort makes for the grouped products (16-byte aligned) */
+long long tlb_moe_lists_ints(int tokens, int top, int experts);
+/* Group the (token, choice) pairs by expert.  One launch, no host involvement; ids outside [0, experts) are skipped. */
+int tlb_moe_sort(const int32_t *idx, int tokens, int top, int experts, int32_t *lists, void *stream);
 /* inter[row, :] = act(Wg[e] h[token(row)]) * (Wu[e] h[token(row)]); Wg, Wu [experts, ff, dim]; inter [max_rows, ff]; act, limit and
- * slope as for tlb_gated_act. */
-int tlb_moe_gate_up(const void *h, const void *wg, const void *wu, const int32_t *sorted_pair, const int32_t *tile_expert,
-                    const int32_t *counters, int tokens, int top, int experts, int tile_rows, int dim, int ff, int act, float limit,
-                    float slope, void *inter, int dtype, void *stream);
+ * slope as for tlb_gated_act.  The products run on tcgen05 for bf16 with dim % 8 == 0 and 16-byte aligned operands. */
+int tlb_moe_gate_up(const void *h, const void *wg, const void *wu, int32_t *lists, int tokens, int top, int experts, int dim, int ff, int act,
+                    float limit, float slope, void *inter, int dtype, void *stream);
 /* Experts without a gate: inter[row, :] = act(Wu[e] a[src(row)]) with a = h (token rows, rows_are_pairs = 0) or one row per
  * (token, choice) pair (rows_are_pairs = 1).  act 0 = silu, 1 = gelu (tanh form), 2 = squared relu. */
-int tlb_moe_up(const void *a, const void *wu, const int32_t *sorted_pair, const int32_t *tile_expert, const int32_t *counters, int tokens,
-               int top, int experts, int tile_rows, int dim, int ff, int act, int rows_are_pairs, void *inter, int dtype, void *stream);
+int tlb_moe_up(const void *a, const void *wu, int32_t *lists, int tokens, int top, int experts, int dim, int ff, int act, int rows_are_pairs,
+               void *inter, int dtype, void *stream);
+/* How many waits of tensor-core kernels have run into their limit (0 in a sound process; such a launch's results are wrong).
+ * Synchronises the device. */
+long long tlb_tc_gave_up(void);
 /* out[t * top + k, :] = gate[t, k] * h[t, :] rounded to `dtype`: inputs of experts whose weight multiplies the input. */
 int tlb_moe_scale_rows(const void *h, const float *gate, void *out, int tokens, int top, int dim, int dtype, void *stream);
 /* pair_out[pair, :] = Wd[e] inter[row, :] (fp32); Wd [experts, dim, ff]. */
-int tlb_moe_down(const void *inter, const void *wd, const int32_t *sorted_pair, const int32_t *tile_expert, const int32_t *counters,
-                 int tokens, int top, int experts, int tile_rows, int dim, int ff, float *pair_out, int dtype, void *stream);
+int tlb_moe_down(const void *inter, const void *wd, int32_t *lists, int tokens, int top, int experts, int dim, int ff, float *pair_out, int dtype,
+                 void *stream);
 /* y[t,:] = sum_k gate[t,k] * pair_out[t*top+k,:] (+ shared_gate[t] * shared[t,:] if shared != NULL, stored in `dtype`; shared_gate
  * NULL: 1), fp32, in choice order;
  * gate == NULL: every weight is 1.  idx != NULL: a choice with idx[t,k] >= experts is an identity expert (the router has

@@ -4,8 +4,9 @@
 // The pairs of one expert occupy whole 32-row tiles of a sorted row list, so every CTA of the grouped products reads
 // ONE expert's weights; rows are gathered from / scattered to token order through the list.  Each output row is a sum
 // over the reduction index in a fixed order and the combination adds a token's choices in choice order, so a token's
-// result does not depend on which other tokens are in the batch.
-#include "blocks_common.cuh"
+// result does not depend on which other tokens are in the batch.  bfloat16 products run on the tensor cores
+// (blocks_moe_tc.cu); the kernel here serves fp32 and rows that are no multiple of 16 bytes.
+#include "blocks_moe.cuh"
 
 namespace tlb {
 
@@ -13,13 +14,6 @@ constexpr int kTileRows = TLB_MOE_TILE_ROWS;
 
 __device__ __forceinline__ float moe_act(float z, int act) {
     return act == 2 ? (z > 0.f ? z * z : 0.f) : act_apply(z, act);  // 2: squared ReLU
-}
-
-// Which rows of `a` a tile's rows read: the sorted rows themselves (the second product), the token of the pair, or the pair.
-constexpr int kGatherSorted = 0, kGatherToken = 1, kGatherPair = 2;
-__device__ __forceinline__ int moe_src_row(int pair, int sorted_row, int top, int gather) {
-    if (pair < 0) return -1;
-    return gather == kGatherSorted ? sorted_row : gather == kGatherToken ? pair / top : pair;
 }
 
 // W consecutive entries of a row as floats.
@@ -173,37 +167,6 @@ moe_route_kernel(const T *__restrict__ h, const T *__restrict__ w, const T *__re
         gate[(size_t)t * top + k] = scoring == 2 ? gate[(size_t)t * top + k] / (denom + 1e-20f) * weight_scale : gate[(size_t)t * top + k] / denom;
 }
 
-// Single CTA: histogram, padded exclusive scan, scatter.
-__global__ void moe_sort_kernel(const int32_t *__restrict__ idx, int pairs, int experts, int max_rows, int tile_rows, int32_t *__restrict__ sorted_pair,
-                                int32_t *__restrict__ tile_expert, int32_t *__restrict__ counters) {
-    extern __shared__ int sm[];
-    int *count = sm, *start = sm + experts, *cursor = sm + 2 * experts;
-    for (int e = threadIdx.x; e < experts; e += blockDim.x) count[e] = 0, cursor[e] = 0;
-    for (int r = threadIdx.x; r < max_rows; r += blockDim.x) sorted_pair[r] = -1;
-    __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-        int e = idx[p];
-        if (e >= 0 && e < experts) atomicAdd(&count[e], 1);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int row = 0;
-        for (int e = 0; e < experts; ++e) {
-            start[e] = row;
-            int tiles = (count[e] + tile_rows - 1) / tile_rows;
-            for (int i = 0; i < tiles; ++i) tile_expert[row / tile_rows + i] = e;
-            row += tiles * tile_rows;
-        }
-        counters[0] = row / tile_rows;
-        counters[1] = row;
-    }
-    __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
-        int e = idx[p];
-        if (e >= 0 && e < experts) sorted_pair[start[e] + atomicAdd(&cursor[e], 1)] = p;
-    }
-}
-
 // C tile [32 rows x 64 columns] of  A[rows, K] . W[e][cols, K]^T, fp32 accumulation in k order.
 // 256 threads: thread (ty, tx) owns rows 2 ty .. 2 ty + 1 and columns tx + 16 c, c = 0..3.
 constexpr int kBN = 64, kBK = 16;
@@ -275,121 +238,6 @@ moe_grouped_kernel(const T *__restrict__ a, const T *__restrict__ w1, const T *_
     }
 }
 
-
-// ---- the grouped products on the tensor cores (bf16, K % 8 == 0) ------------------------------------------------
-// One CTA = one 32- or 64-row expert tile x 128 output columns; 8 warps = 2 row halves x 4 column quarters (4 x 2 for 64 rows), each
-// mma.sync m16n8k16 over 32-wide reduction blocks that cp.async brings into a two-stage ring (A rows gathered
-// through the sorted pair list).  fp32 accumulators; the reduction order of a row is k ascending in both kernels.
-constexpr int kTN = 128, kTK = 32, kTS = kTK + 8;  // row stride 40 elements = 80 B: (80 / 16) odd, conflict-free ldmatrix
-
-__device__ __forceinline__ void moe_ldm_x4(uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3, const void *p) {
-    uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(a));
-}
-__device__ __forceinline__ void moe_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void moe_cp16(void *dst, const void *src, bool ok) {
-    uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-    int bytes = ok ? 16 : 0;  // src-size 0: the 16 bytes are zero-filled
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
-
-template <bool GATED, int BM>
-__global__ void __launch_bounds__(256)
-moe_grouped_mma_kernel(const bf16 *__restrict__ a, const bf16 *__restrict__ w1, const bf16 *__restrict__ w2, const int32_t *__restrict__ sorted_pair,
-                       const int32_t *__restrict__ tile_expert, const int32_t *__restrict__ counters, int top, int K, int N, int act, float limit,
-                       float slope, int gather, bf16 *__restrict__ inter, float *__restrict__ pair_out) {
-    if ((int)blockIdx.x >= counters[0]) return;
-    constexpr int MT = BM / 16;          // 16-row halves/quarters of the tile
-    constexpr int NW = 8 / MT;           // warps along the columns
-    constexpr int NPW = kTN / NW / 8;    // 8-column blocks per warp
-    extern __shared__ __align__(16) unsigned char moe_smem[];
-    bf16 (*sa)[BM * kTS] = reinterpret_cast<bf16 (*)[BM * kTS]>(moe_smem);                              // [2]
-    bf16 (*sb1)[kTN * kTS] = reinterpret_cast<bf16 (*)[kTN * kTS]>(moe_smem + 2 * BM * kTS * 2);        // [2]
-    bf16 (*sb2)[kTN * kTS] = reinterpret_cast<bf16 (*)[kTN * kTS]>(moe_smem + 2 * (BM + kTN) * kTS * 2);  // [2], gated only
-    __shared__ int src_row[BM];
-    const int e = tile_expert[blockIdx.x];
-    const int row0 = blockIdx.x * BM, col0 = blockIdx.y * kTN;
-    if (threadIdx.x < BM) {
-        src_row[threadIdx.x] = moe_src_row(sorted_pair[row0 + threadIdx.x], row0 + (int)threadIdx.x, top, gather);
-    }
-    __syncthreads();
-    const bf16 *wa = w1 + (size_t)e * N * K;
-    const bf16 *wb = GATED ? w2 + (size_t)e * N * K : nullptr;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int mt = warp % MT, nq = warp / MT;
-
-    auto stage = [&](int kb, int buf) {
-        int k0 = kb * kTK;
-        if (threadIdx.x < BM * 4) {  // A: BM rows x 4 pieces of 8
-            int r = threadIdx.x >> 2, piece = threadIdx.x & 3;
-            int sr = src_row[r], k = k0 + piece * 8;
-            bool ok = sr >= 0 && k < K;
-            moe_cp16(&sa[buf][r * kTS + piece * 8], a + (ok ? (size_t)sr * K + k : 0), ok);
-        }
-        for (int c = threadIdx.x; c < kTN * 4; c += 256) {  // B: 128 rows x 4 pieces
-            int n = c >> 2, piece = c & 3;
-            int k = k0 + piece * 8;
-            bool ok = col0 + n < N && k < K;
-            size_t off = ok ? (size_t)(col0 + n) * K + k : 0;
-            moe_cp16(&sb1[buf][n * kTS + piece * 8], wa + off, ok);
-            if (GATED) moe_cp16(&sb2[buf][n * kTS + piece * 8], wb + off, ok);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-
-    float c1[NPW][4] = {}, c2[GATED ? NPW : 1][4] = {};
-    const int kblocks = (K + kTK - 1) / kTK;
-    stage(0, 0);
-    for (int kb = 0; kb < kblocks; ++kb) {
-        int buf = kb & 1;
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();  // this block has landed; everybody is done with the other buffer
-        if (kb + 1 < kblocks) stage(kb + 1, buf ^ 1);
-#pragma unroll
-        for (int ks = 0; ks < kTK / 16; ++ks) {
-            uint32_t a0, a1, a2, a3;
-            moe_ldm_x4(a0, a1, a2, a3, &sa[buf][(mt * 16 + (lane & 15)) * kTS + ks * 16 + (lane >> 4) * 8]);
-#pragma unroll
-            for (int np = 0; np < NPW / 2; ++np) {  // two n8 tiles per ldmatrix.x4: rows n..n+7 and n+8..n+15, k halves 0 / 8
-                int n = nq * (8 * NPW) + np * 16 + (lane & 7) + ((lane >> 4) & 1) * 8;
-                int kk = ks * 16 + ((lane >> 3) & 1) * 8;
-                uint32_t b0, b1, b2, b3;
-                moe_ldm_x4(b0, b1, b2, b3, &sb1[buf][n * kTS + kk]);
-                moe_mma(c1[2 * np], a0, a1, a2, a3, b0, b1);
-                moe_mma(c1[2 * np + 1], a0, a1, a2, a3, b2, b3);
-                if (GATED) {
-                    moe_ldm_x4(b0, b1, b2, b3, &sb2[buf][n * kTS + kk]);
-                    moe_mma(c2[2 * np], a0, a1, a2, a3, b0, b1);
-                    moe_mma(c2[2 * np + 1], a0, a1, a2, a3, b2, b3);
-                }
-            }
-        }
-    }
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        int row = row0 + mt * 16 + g + half * 8;
-        int pair = sorted_pair[row];
-        if (pair < 0) continue;
-#pragma unroll
-        for (int i = 0; i < NPW; ++i) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                int col = col0 + nq * (8 * NPW) + i * 8 + 2 * t + j;
-                if (col >= N) continue;
-                float v = c1[i][half * 2 + j];
-                if (GATED) inter[(size_t)row * N + col] = __float2bfloat16_rn(gated_pair(v, c2[i][half * 2 + j], act, limit, slope));
-                else if (inter) inter[(size_t)row * N + col] = __float2bfloat16_rn(moe_act(v, act));
-                else pair_out[(size_t)pair * N + col] = v;
-            }
-        }
-    }
-}
-
 // out[pair, :] = gate[pair] * h[pair / top, :] rounded to T: the rows of experts whose weight multiplies their input.
 template <typename T>
 __global__ void moe_scale_rows_kernel(const T *__restrict__ h, const float *__restrict__ gate, T *__restrict__ out, int top, int dim) {
@@ -419,22 +267,21 @@ __global__ void moe_combine_kernel(const float *__restrict__ pair_out, const flo
 
 using namespace tlb;
 
-template <bool GATED, int BM>
-static int launch_grouped_mma(dim3 grid, cudaStream_t st, const bf16 *a, const bf16 *w1, const bf16 *w2, const int32_t *sorted_pair,
-                              const int32_t *tile_expert, const int32_t *counters, int top, int K, int N, int act, float limit, float slope, int gather, bf16 *inter,
-                              float *pair_out) {
-    size_t smem = (size_t)2 * (BM + kTN * (GATED ? 2 : 1)) * kTS * sizeof(bf16);
-    auto kernel = moe_grouped_mma_kernel<GATED, BM>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return tl::fail(TL_ECUDA, "moe_grouped: %s", cudaGetErrorString(e));
+static int moe_product(const char *what, const MoeProduct &p, int dtype, cudaStream_t st) {
+    if (moe_tc_ok(dtype, p.K, p.x, p.w0, p.w1)) {
+        if (int e = moe_tc_product(p, st)) return e;
+    } else {
+        const dim3 grid((unsigned)(tlb_moe_max_rows(p.tokens, p.top, p.experts) / kTileRows), ceil_div(p.N, kBN));
+        const MoeLists &l = p.lists;
+        if (p.w1)
+            TLB_DISPATCH(dtype, what, moe_grouped_kernel<T, true><<<grid, 256, 0, st>>>((const T *)p.x, (const T *)p.w0, (const T *)p.w1, l.sorted_pair, l.tile_expert,
+                                                                                        l.counters, p.top, p.K, p.N, p.act, p.limit, p.slope, p.gather, (T *)p.inter, p.pair_out));
+        else
+            TLB_DISPATCH(dtype, what, moe_grouped_kernel<T, false><<<grid, 256, 0, st>>>((const T *)p.x, (const T *)p.w0, nullptr, l.sorted_pair, l.tile_expert,
+                                                                                         l.counters, p.top, p.K, p.N, p.act, p.limit, p.slope, p.gather, (T *)p.inter, p.pair_out));
     }
-    kernel<<<grid, 256, smem, st>>>(a, w1, w2, sorted_pair, tile_expert, counters, top, K, N, act, limit, slope, gather, inter, pair_out);
+    TL_LAUNCH_CHECK(what);
     return TL_OK;
-}
-
-static bool moe_mma_ok(int dtype, int k, const void *a, const void *w1, const void *w2) {
-    return dtype == TL_BF16 && k % 8 == 0 && tl::aligned16(a) && tl::aligned16(w1) && (!w2 || tl::aligned16(w2));
 }
 
 extern "C" {
@@ -466,78 +313,23 @@ int tlb_moe_route(const void *h, const void *w, const void *b, int tokens, int d
     return TL_OK;
 }
 
-long long tlb_moe_max_rows(int tokens, int top, int experts, int tile_rows) {
-    long long pairs = (long long)tokens * top;
-    long long groups = pairs < experts ? pairs : experts;  // at most min(pairs, experts) groups carry padding
-    long long rows = pairs + groups * (tile_rows - 1);
-    return (rows + tile_rows - 1) / tile_rows * tile_rows;
-}
-
-int tlb_moe_sort(const int32_t *idx, int tokens, int top, int experts, int tile_rows, int32_t *sorted_pair, int32_t *tile_expert,
-                 int32_t *counters, void *stream) {
+int tlb_moe_gate_up(const void *h, const void *wg, const void *wu, int32_t *lists, int tokens, int top, int experts, int dim, int ff, int act, float limit,
+                    float slope, void *inter, int dtype, void *stream) {
     if (tokens <= 0) return TL_OK;
-    if (!idx || !sorted_pair || !tile_expert || !counters || top <= 0 || experts <= 0 || (tile_rows != 32 && tile_rows != 64))
-        return tl::fail(TL_EINVAL, "moe_sort: bad argument");
-    size_t smem = (size_t)3 * experts * sizeof(int);
-    if (smem > 48 * 1024) return tl::fail(TL_EINVAL, "moe_sort: %d experts do not fit", experts);
-    moe_sort_kernel<<<1, 1024, smem, as_stream(stream)>>>(idx, tokens * top, experts, (int)tlb_moe_max_rows(tokens, top, experts, tile_rows), tile_rows,
-                                                          sorted_pair, tile_expert, counters);
-    TL_LAUNCH_CHECK("moe_sort");
-    return TL_OK;
-}
-
-// The tensor-core kernels take 32- or 64-row expert tiles (64 halves the weight traffic per row when experts get many
-// rows); the fp32 kernels 32 only.
-int tlb_moe_gate_up(const void *h, const void *wg, const void *wu, const int32_t *sorted_pair, const int32_t *tile_expert, const int32_t *counters,
-                    int tokens, int top, int experts, int tile_rows, int dim, int ff, int act, float limit, float slope, void *inter, int dtype, void *stream) {
-    if (tokens <= 0) return TL_OK;
-    if (!h || !wg || !wu || !sorted_pair || !tile_expert || !counters || !inter || dim <= 0 || ff <= 0 || top <= 0 || (act != 0 && act != 1 && act != 3) ||
-        (act == 3 && !(limit > 0.f)))
+    if (!h || !wg || !wu || !lists || !inter || experts <= 0 || dim <= 0 || ff <= 0 || top <= 0 || (act != 0 && act != 1 && act != 3) || (act == 3 && !(limit > 0.f)))
         return tl::fail(TL_EINVAL, "moe_gate_up: bad argument");
-    if (moe_mma_ok(dtype, dim, h, wg, wu)) {
-        dim3 tc((unsigned)(tlb_moe_max_rows(tokens, top, experts, tile_rows) / tile_rows), ceil_div(ff, kTN));
-        int rc = tile_rows == 64 ? launch_grouped_mma<true, 64>(tc, as_stream(stream), (const bf16 *)h, (const bf16 *)wg, (const bf16 *)wu, sorted_pair,
-                                                                tile_expert, counters, top, dim, ff, act, limit, slope, kGatherToken, (bf16 *)inter, nullptr)
-                                 : launch_grouped_mma<true, 32>(tc, as_stream(stream), (const bf16 *)h, (const bf16 *)wg, (const bf16 *)wu, sorted_pair,
-                                                                tile_expert, counters, top, dim, ff, act, limit, slope, kGatherToken, (bf16 *)inter, nullptr);
-        if (rc != TL_OK) return rc;
-        TL_LAUNCH_CHECK("moe_gate_up");
-        return TL_OK;
-    }
-    if (tile_rows != kTileRows) return tl::fail(TL_EINVAL, "moe_gate_up: %d-row tiles need the tensor-core kernel", tile_rows);
-    dim3 grid((unsigned)(tlb_moe_max_rows(tokens, top, experts, kTileRows) / kTileRows), ceil_div(ff, kBN));
-    TLB_DISPATCH(dtype, "moe_gate_up",
-                 moe_grouped_kernel<T, true><<<grid, 256, 0, as_stream(stream)>>>((const T *)h, (const T *)wg, (const T *)wu, sorted_pair, tile_expert,
-                                                                                 counters, top, dim, ff, act, limit, slope, kGatherToken, (T *)inter, nullptr));
-    TL_LAUNCH_CHECK("moe_gate_up");
-    return TL_OK;
+    return moe_product("moe_gate_up", {h, wg, wu, moe_lists(lists, tokens, top, experts), tokens, top, experts, dim, ff, act, kGatherToken, limit, slope, inter, nullptr}, dtype,
+                       as_stream(stream));
 }
 
 // The first product of experts without a gate: inter[row, :] = act(W[e] a[src(row)]), a = token rows (rows_are_pairs = 0) or one row per
 // (token, choice) pair (rows_are_pairs = 1: the scaled copies tlb_moe_scale_rows makes).
-int tlb_moe_up(const void *a, const void *wu, const int32_t *sorted_pair, const int32_t *tile_expert, const int32_t *counters, int tokens, int top,
-               int experts, int tile_rows, int dim, int ff, int act, int rows_are_pairs, void *inter, int dtype, void *stream) {
+int tlb_moe_up(const void *a, const void *wu, int32_t *lists, int tokens, int top, int experts, int dim, int ff, int act, int rows_are_pairs, void *inter, int dtype,
+               void *stream) {
     if (tokens <= 0) return TL_OK;
-    if (!a || !wu || !sorted_pair || !tile_expert || !counters || !inter || dim <= 0 || ff <= 0 || top <= 0 || act < 0 || act > 2)
-        return tl::fail(TL_EINVAL, "moe_up: bad argument");
-    int gather = rows_are_pairs ? kGatherPair : kGatherToken;
-    if (moe_mma_ok(dtype, dim, a, wu, nullptr)) {
-        dim3 tc((unsigned)(tlb_moe_max_rows(tokens, top, experts, tile_rows) / tile_rows), ceil_div(ff, kTN));
-        int rc = tile_rows == 64 ? launch_grouped_mma<false, 64>(tc, as_stream(stream), (const bf16 *)a, (const bf16 *)wu, nullptr, sorted_pair, tile_expert,
-                                                                 counters, top, dim, ff, act, 0.f, 1.f, gather, (bf16 *)inter, nullptr)
-                                 : launch_grouped_mma<false, 32>(tc, as_stream(stream), (const bf16 *)a, (const bf16 *)wu, nullptr, sorted_pair, tile_expert,
-                                                                 counters, top, dim, ff, act, 0.f, 1.f, gather, (bf16 *)inter, nullptr);
-        if (rc != TL_OK) return rc;
-        TL_LAUNCH_CHECK("moe_up");
-        return TL_OK;
-    }
-    if (tile_rows != kTileRows) return tl::fail(TL_EINVAL, "moe_up: %d-row tiles need the tensor-core kernel", tile_rows);
-    dim3 grid((unsigned)(tlb_moe_max_rows(tokens, top, experts, kTileRows) / kTileRows), ceil_div(ff, kBN));
-    TLB_DISPATCH(dtype, "moe_up",
-                 moe_grouped_kernel<T, false><<<grid, 256, 0, as_stream(stream)>>>((const T *)a, (const T *)wu, nullptr, sorted_pair, tile_expert, counters,
-                                                                                  top, dim, ff, act, 0.f, 1.f, gather, (T *)inter, nullptr));
-    TL_LAUNCH_CHECK("moe_up");
-    return TL_OK;
+    if (!a || !wu || !lists || !inter || experts <= 0 || dim <= 0 || ff <= 0 || top <= 0 || act < 0 || act > 2) return tl::fail(TL_EINVAL, "moe_up: bad argument");
+    return moe_product("moe_up", {a, wu, nullptr, moe_lists(lists, tokens, top, experts), tokens, top, experts, dim, ff, act, rows_are_pairs ? kGatherPair : kGatherToken, 0.f,
+                                  1.f, inter, nullptr}, dtype, as_stream(stream));
 }
 
 int tlb_moe_scale_rows(const void *h, const float *gate, void *out, int tokens, int top, int dim, int dtype, void *stream) {
@@ -549,28 +341,11 @@ int tlb_moe_scale_rows(const void *h, const float *gate, void *out, int tokens, 
     return TL_OK;
 }
 
-int tlb_moe_down(const void *inter, const void *wd, const int32_t *sorted_pair, const int32_t *tile_expert, const int32_t *counters, int tokens,
-                 int top, int experts, int tile_rows, int dim, int ff, float *pair_out, int dtype, void *stream) {
+int tlb_moe_down(const void *inter, const void *wd, int32_t *lists, int tokens, int top, int experts, int dim, int ff, float *pair_out, int dtype, void *stream) {
     if (tokens <= 0) return TL_OK;
-    if (!inter || !wd || !sorted_pair || !tile_expert || !counters || !pair_out || dim <= 0 || ff <= 0 || top <= 0)
-        return tl::fail(TL_EINVAL, "moe_down: bad argument");
-    if (moe_mma_ok(dtype, ff, inter, wd, nullptr)) {
-        dim3 tc((unsigned)(tlb_moe_max_rows(tokens, top, experts, tile_rows) / tile_rows), ceil_div(dim, kTN));
-        int rc = tile_rows == 64 ? launch_grouped_mma<false, 64>(tc, as_stream(stream), (const bf16 *)inter, (const bf16 *)wd, nullptr, sorted_pair,
-                                                                 tile_expert, counters, top, ff, dim, 0, 0.f, 1.f, kGatherSorted, nullptr, pair_out)
-                                 : launch_grouped_mma<false, 32>(tc, as_stream(stream), (const bf16 *)inter, (const bf16 *)wd, nullptr, sorted_pair,
-                                                                 tile_expert, counters, top, ff, dim, 0, 0.f, 1.f, kGatherSorted, nullptr, pair_out);
-        if (rc != TL_OK) return rc;
-        TL_LAUNCH_CHECK("moe_down");
-        return TL_OK;
-    }
-    if (tile_rows != kTileRows) return tl::fail(TL_EINVAL, "moe_down: %d-row tiles need the tensor-core kernel", tile_rows);
-    dim3 grid((unsigned)(tlb_moe_max_rows(tokens, top, experts, kTileRows) / kTileRows), ceil_div(dim, kBN));
-    TLB_DISPATCH(dtype, "moe_down",
-                 moe_grouped_kernel<T, false><<<grid, 256, 0, as_stream(stream)>>>((const T *)inter, (const T *)wd, nullptr, sorted_pair, tile_expert,
-                                                                                  counters, top, ff, dim, 0, 0.f, 1.f, kGatherSorted, nullptr, pair_out));
-    TL_LAUNCH_CHECK("moe_down");
-    return TL_OK;
+    if (!inter || !wd || !lists || !pair_out || experts <= 0 || dim <= 0 || ff <= 0 || top <= 0) return tl::fail(TL_EINVAL, "moe_down: bad argument");
+    return moe_product("moe_down", {inter, wd, nullptr, moe_lists(lists, tokens, top, experts), tokens, top, experts, ff, dim, 0, kGatherSorted, 0.f, 1.f, nullptr, pair_out},
+                       dtype, as_stream(stream));
 }
 
 int tlb_moe_combine(const float *pair_out, const float *gate, const void *shared, const float *shared_gate, const int32_t *idx, int experts, const void *h, float *y, int tokens,

@@ -41,7 +41,7 @@ _SIGNATURES = {
     "tlb_streams_step": (_I, [_VP, _VP, _VP, _VP, _VP, _VP, _F, _VP, _I, _I, _I, _I, _VP]),
     "tlb_shift_mix": (_I, [_VP, _LL, _VP, _I, _I, _VP, _I, _I, _VP, _LL, _I, _VP, _LL, _I, _VP]),
     "tlb_moe_route": (_I, [_VP, _VP, _VP, _I, _I, _I, _I, _I, _VP, _F, _I, _I, _VP, _VP, _VP, _VP, _I, _VP]),
-    "tlb_moe_up": (_I, [_VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _I, _VP, _I, _VP]),
+    "tlb_moe_up": (_I, [_VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _VP, _I, _VP]),
     "tlb_moe_scale_rows": (_I, [_VP, _VP, _VP, _I, _I, _I, _I, _VP]),
     "tlb_add_norm": (_I, [_VP, _VP, _I, _VP, _VP, _F, _VP, _VP, _VP, _I, _I, _I, _VP]),
     "tlb_norm_mix2": (_I, [_VP, _VP, _VP, _VP, _F, _F, _VP, _I, _I, _I, _VP]),
@@ -75,18 +75,19 @@ _SIGNATURES = {
     "tlb_tanh_step": (_I, [_VP, _VP, _VP, _F, _VP, _VP, _F, _VP, _VP, _VP, _I, _I, _I, _VP]),
     "tlb_tanh_rows": (_I, [_VP, _VP, _F, _VP, _VP, _VP, _I, _I, _I, _VP]),
     "tlb_moe_combine_tanh": (_I, [_VP, _VP, _VP, _VP, _VP, _VP, _I, _VP, _I, _F, _VP, _VP, _F, _VP, _VP, _VP, _I, _I, _I, _VP]),
-    "tlb_moe_max_rows": (_LL, [_I, _I, _I, _I]),
-    "tlb_moe_sort": (_I, [_VP, _I, _I, _I, _I, _VP, _VP, _VP, _VP]),
-    "tlb_moe_gate_up": (_I, [_VP, _VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _F, _F, _VP, _I, _VP]),
-    "tlb_moe_down": (_I, [_VP, _VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _VP, _I, _VP]),
+    "tlb_moe_max_rows": (_LL, [_I, _I, _I]),
+    "tlb_moe_lists_ints": (_LL, [_I, _I, _I]),
+    "tlb_moe_sort": (_I, [_VP, _I, _I, _I, _VP, _VP]),
+    "tlb_moe_gate_up": (_I, [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _F, _F, _VP, _I, _VP]),
+    "tlb_moe_down": (_I, [_VP, _VP, _VP, _I, _I, _I, _I, _I, _VP, _I, _VP]),
+    "tlb_tc_gave_up": (_LL, []),
     "tlb_moe_combine": (_I, [_VP, _VP, _VP, _VP, _VP, _I, _VP, _VP, _I, _I, _I, _I, _VP]),
     "tlb_argmax_rows": (_I, [_VP, _VP, _I, _I, _VP]),
 }
 EXPORTED_SYMBOLS = tuple(_SIGNATURES)
 
-ABI_VERSION = 7
+ABI_VERSION = 8
 ATTENTION_TILE_TOKENS = 4
-MOE_TILE_ROWS = 32
 ACT_SILU, ACT_GELU_TANH, ACT_RELU_SQUARED, ACT_CLAMPED_SWISH, ACT_TANH = 0, 1, 2, 3, 4
 WEIGHTS_SOFTMAX, WEIGHTS_SIGMOID = 0, 1
 DECAY_SIGMOID, DECAY_DOUBLE_EXP, DECAY_STEP, DECAY_GIVEN = 0, 2, 3, 4
@@ -439,16 +440,11 @@ def moe_experts(h, idx, gate, w_gate, w_up, w_down, act: int, shared=None, scale
     T, D = h.shape
     E, ff, _ = w_up.shape
     top = idx.shape[1]
-    # 64-row expert tiles once the average expert gets that many rows (tensor-core kernels only: bf16, widths % 8 == 0)
-    rows = 64 if (h.dtype == torch.bfloat16 and D % 8 == 0 and ff % 8 == 0 and T * top >= 64 * E) else MOE_TILE_ROWS
-    max_rows = int(lib.tlb_moe_max_rows(T, top, E, rows))
     dev, code, st = h.device, _code(h.dtype), _stream(h)
-    sorted_pair = torch.empty(max_rows, dtype=torch.int32, device=dev)
-    tile_expert = torch.empty(max_rows // rows, dtype=torch.int32, device=dev)
-    counters = torch.empty(2, dtype=torch.int32, device=dev)
-    inter = torch.empty((max_rows, ff), dtype=h.dtype, device=dev)
+    lists = torch.empty(int(lib.tlb_moe_lists_ints(T, top, E)), dtype=torch.int32, device=dev)
+    inter = torch.empty((int(lib.tlb_moe_max_rows(T, top, E)), ff), dtype=h.dtype, device=dev)
     pair_out = torch.empty((T * top, D), dtype=torch.float32, device=dev)
-    _check(lib.tlb_moe_sort(_ptr(idx), T, top, E, rows, _ptr(sorted_pair), _ptr(tile_expert), _ptr(counters), st))
+    _check(lib.tlb_moe_sort(_ptr(idx), T, top, E, _ptr(lists), st))
     rows_in, per_pair = h, 0
     if scale_input:
         rows_in, per_pair = torch.empty((T * top, D), dtype=h.dtype, device=dev), 1
@@ -456,12 +452,10 @@ def moe_experts(h, idx, gate, w_gate, w_up, w_down, act: int, shared=None, scale
     if w_gate is not None:
         if per_pair:
             raise RuntimeError("moe_experts: gated experts take the router's weight on their output")
-        _check(lib.tlb_moe_gate_up(_ptr(h), _ptr(w_gate), _ptr(w_up), _ptr(sorted_pair), _ptr(tile_expert), _ptr(counters), T, top, E, rows, D, ff, act,
-                                   float(limit), float(slope), _ptr(inter), code, st))
+        _check(lib.tlb_moe_gate_up(_ptr(h), _ptr(w_gate), _ptr(w_up), _ptr(lists), T, top, E, D, ff, act, float(limit), float(slope), _ptr(inter), code, st))
     else:
-        _check(lib.tlb_moe_up(_ptr(rows_in), _ptr(w_up), _ptr(sorted_pair), _ptr(tile_expert), _ptr(counters), T, top, E, rows, D, ff, act, per_pair,
-                              _ptr(inter), code, st))
-    _check(lib.tlb_moe_down(_ptr(inter), _ptr(w_down), _ptr(sorted_pair), _ptr(tile_expert), _ptr(counters), T, top, E, rows, D, ff, _ptr(pair_out), code, st))
+        _check(lib.tlb_moe_up(_ptr(rows_in), _ptr(w_up), _ptr(lists), T, top, E, D, ff, act, per_pair, _ptr(inter), code, st))
+    _check(lib.tlb_moe_down(_ptr(inter), _ptr(w_down), _ptr(lists), T, top, E, D, ff, _ptr(pair_out), code, st))
     if before_sum is not None:
         before_sum()
     if into is not None:
