@@ -265,6 +265,29 @@ int tlb_streams_step(float *xs, const float *x0, const float *y, const void *y_b
 int tlb_shift_mix(const void *h, long long h_token, const void *mu, int parts, int dim, const int32_t *seq_info, int num_seqs, int max_tokens_per_seq,
                   float *state, long long slot_stride, int num_slots, void *out, long long out_part, int dtype, void *stream);
 
+/* Attention of steps with prompt portions on tcgen05 (bf16): arguments as for tlb_paged_attention_flash, but no work list: a CTA
+ * finds its run of tlb_flash_tc_run_tokens tokens in seq_info [num_seqs, 4] (first token, tokens, position of the first, -).
+ * runs: how many there are, sum over the sequences of ceil(tokens / run tokens) (an upper bound will do).  dk, dv multiples of 8 up
+ * to 256, page_size % 64 == 0, at most 128 query heads per key/value head; q 16-byte aligned, its strides multiples of 8. */
+int tlb_flash_tc_run_tokens(int heads, int kv_heads);
+int tlb_flash_tc_supported(int dk, int dv, int heads, int kv_heads, int page_size);
+int tlb_paged_attention_tc(const void *q, long long q_token, long long q_head, int tokens, const void *slab, int num_pages, int page_size, int dk,
+                           int dv, int heads, int kv_heads, const int32_t *block_table, int max_pages, const int32_t *seq_info, int num_seqs,
+                           int runs, int mask, int mask_size, int keep_first, float scale, float softcap, int sink, const void *gate,
+                           long long g_token, int gate_wide, void *out, long long o_token, long long o_head, const float *head_bias, int weights,
+                           void *stream);
+/* The cached rows of every sequence's context (start + tokens of seq_info) one after the other, each sequence from a whole 64-row
+ * page on: rows [total_pages * 64, width], zeros past a sequence's newest token, and table [num_seqs, table_pages] of their pages. */
+int tlb_latent_rows(const void *slab, int num_pages, int page_size, int width, const int32_t *seq_info, int num_seqs, const int32_t *block_table,
+                    int max_pages, void *rows, int32_t *table, int table_pages, int total_pages, void *stream);
+/* Latent attention with keys and values up-projected per head: q [tokens, heads, dim + rot] against k [rows, heads * dim] (head h's
+ * part at h * dim), the part all heads share k_rot [rows, rot], and v (head h at v + h * v_head, rows v_row apart), rows found through
+ * `table` (64-row pages).  dim % 64 == 0, rot <= 64, rot % 8 == 0, dim + rot and dv up to 256.  128 tokens a run. */
+int tlb_latent_attention_heads(const void *q, long long q_token, long long q_head, int tokens, const void *k, long long k_row, const void *v,
+                               long long v_head, long long v_row, const void *k_rot, long long k_rot_row, int dim, int rot, int dv, int heads,
+                               long long rows, const int32_t *table, int table_pages, const int32_t *seq_info, int num_seqs, int runs,
+                               int window, float scale, void *out, long long o_token, long long o_head, const float *sink, void *stream);
+
 /* Router: logits = W h + b in fp32 (h, W, b stored in `dtype`; b may be NULL), the `top` largest per token (lower index
  * wins a tie).  scoring 0: weights = softmax over the chosen logits; 1: weights = sigmoid of each chosen logit, not
  * renormalised; 2: scores = softmax over ALL logits, the choice is made by score + choice_bias (`dtype` [experts] or NULL),

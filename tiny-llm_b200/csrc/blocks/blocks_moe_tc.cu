@@ -393,6 +393,6 @@ int tlb_moe_sort(const int32_t *idx, int tokens, int top, int experts, int32_t *
     return TL_OK;
 }
 
-long long tlb_tc_gave_up(void) { return tc_read_gave_up(); }
+long long tlb_tc_gave_up(void) { return tc_read_gave_up() + flash_tc_gave_up(); }
 
 }  // extern "C"

@@ -28,6 +28,8 @@ static inline long long tc_read_gave_up() {
     return cudaMemcpyFromSymbol(&n, g_tc_gave_up, sizeof(n)) == cudaSuccess ? (long long)n : -1;
 }
 
+long long flash_tc_gave_up();  // of the attention kernels
+
 __device__ __forceinline__ void tc_wait(uint32_t bar, uint32_t parity, volatile int *dead) {
     for (uint32_t spins = 0;; ++spins) {
         uint32_t done;

@@ -48,6 +48,7 @@ BLOCKS_SOURCES = [
     "blocks/blocks_moe.cu",
     "blocks/blocks_moe_tc.cu",
     "blocks/blocks_tc.cu",
+    "blocks/blocks_flash_tc.cu",
     "blocks/blocks_paged_attention.cu",
     "blocks/blocks_paged_attention_mma.cu",
     "blocks/blocks_paged_attention_flash.cu",

@@ -57,6 +57,12 @@ _SIGNATURES = {
     "tlb_paged_attention_flash_supported": (_I, [_I, _I, _I, _I]),
     "tlb_paged_attention_flash": (_I, [_VP, _LL, _LL, _VP, _I, _I, _I, _I, _I, _I, _VP, _I, _VP, _I, _VP, _I, _I, _I, _F, _F, _I, _VP, _LL, _I, _VP, _LL, _LL, _I, _I,
                                        _VP, _I, _VP]),
+    "tlb_flash_tc_run_tokens": (_I, [_I, _I]),
+    "tlb_flash_tc_supported": (_I, [_I, _I, _I, _I, _I]),
+    "tlb_paged_attention_tc": (_I, [_VP, _LL, _LL, _I, _VP, _I, _I, _I, _I, _I, _I, _VP, _I, _VP, _I, _I, _I, _I, _I, _F, _F, _I, _VP, _LL, _I, _VP, _LL, _LL, _VP, _I,
+                                    _VP]),
+    "tlb_latent_rows": (_I, [_VP, _I, _I, _I, _VP, _I, _VP, _I, _VP, _VP, _I, _I, _VP]),
+    "tlb_latent_attention_heads": (_I, [_VP, _LL, _LL, _I, _VP, _LL, _VP, _LL, _LL, _VP, _LL, _I, _I, _I, _I, _LL, _VP, _I, _VP, _I, _I, _I, _F, _VP, _LL, _LL, _VP, _VP]),
     "tlb_kv_prepare": (_I, [_VP, _LL, _LL, _I, _VP, _VP, _LL, _LL, _VP, _LL, _LL, _I, _I, _I, _VP, _F, _VP, _VP, _VP, _I, _I, _I, _VP, _I, _I, _VP]),
     "tlb_qk_whole_prepare": (_I, [_VP, _LL, _I, _VP, _VP, _LL, _VP, _LL, _I, _I, _I, _VP, _F, _I, _I, _D, _VP, _VP, _VP, _I, _I, _I, _VP, _VP, _VP, _I, _I, _VP]),
     "tlb_decay_scan_workspace": (ctypes.c_size_t, [_I, _I, _I, _I, _I]),
@@ -715,6 +721,82 @@ def paged_attention(q, slab, block_table, tiles, tok_pos, *, kv_heads: int, dv: 
                                          block_table.shape[1], _ptr(tiles), tiles.shape[0], _ptr(tok_pos), int(mask), int(mask_size), int(keep_first), float(scale),
                                          float(softcap or 0.0), int(bool(sink)), _ptr(gate), gate.stride(0) if gate is not None else 0, wide, _ptr(out),
                                          out.stride(0), out.stride(1), _ptr(head_bias), int(weights), _code(q.dtype), _stream(q)))
+    return out
+
+
+def flash_tc_run(dtype, heads: int, kv_heads: int, dk: int, dv: int, page_size: int) -> int:
+    """The most consecutive tokens a CTA of the tcgen05 attention kernel takes with these sizes; 0 where it does not serve them
+    (TL_FLASH_TC=0, TL_PAGED_FLASH=0 and TL_PAGED_MMA=0 switch it off)."""
+    lib = library()
+    if dtype != torch.bfloat16 or any(os.environ.get(v, "1") == "0" for v in ("TL_FLASH_TC", "TL_PAGED_FLASH", "TL_PAGED_MMA")):
+        return 0
+    return int(lib.tlb_flash_tc_run_tokens(heads, kv_heads)) if lib.tlb_flash_tc_supported(dk, dv, heads, kv_heads, page_size) else 0
+
+
+def tma_rows(t: torch.Tensor) -> bool:
+    """Whether a bf16 view ``[rows, heads, width]`` can be read by TMA: 16-byte aligned base and strides, unit inner stride."""
+    return t.data_ptr() % 16 == 0 and t.stride(2) == 1 and t.stride(0) % 8 == 0 and t.stride(1) % 8 == 0
+
+
+def paged_attention_tc(q, slab, block_table, seq_info, runs: int, *, kv_heads: int, dv: int, mask: int, mask_size: int, scale: float, softcap: float = 0.0,
+                       sink: bool = False, gate=None, out=None, head_bias=None, weights: int = 0, keep_first: int = 0):
+    """``paged_attention`` on tcgen05 for steps with prompt portions: arguments as there, but the work is read from ``seq_info [S, 4]``
+    (first token, tokens, position of the first, -); ``runs``: the sum over the sequences of ceil(tokens / ``flash_tc_run``), or more."""
+    _gpu("paged_attention_tc", q, slab, block_table, seq_info, gate, out, head_bias)
+    _contig("paged_attention_tc", slab, block_table, seq_info, head_bias)
+    T, H, dk = q.shape
+    P, page_size, width = slab.shape
+    if width != kv_heads * (dk + dv) or q.dtype != torch.bfloat16 or slab.dtype != q.dtype or not tma_rows(q):
+        raise RuntimeError("paged_attention_tc: bfloat16 query and cache that match, the query's strides multiples of 8")
+    if block_table.shape[0] != seq_info.shape[0] or block_table.dtype != torch.int32 or seq_info.dtype != torch.int32 or seq_info.shape[1] != 4:
+        raise RuntimeError("paged_attention_tc: int32 block table and seq_info [S, 4] of the same sequences")
+    if head_bias is not None and (head_bias.dtype != torch.float32 or head_bias.shape != (H,)):
+        raise RuntimeError("paged_attention_tc: head_bias must be float32 [H]")
+    wide = int(gate is not None and gate.shape == (T, H * dv) and dv > 1)
+    if gate is not None and ((gate.shape != (T, H) and not wide) or gate.stride(1) != 1 or gate.dtype != q.dtype):
+        raise RuntimeError("paged_attention_tc: gate must be [T, H] or [T, H * dv] of the query's dtype")
+    if out is None:
+        out = torch.empty((T, H, dv), dtype=q.dtype, device=q.device)
+    elif out.shape != (T, H, dv) or out.dtype != q.dtype or out.stride(2) != 1:
+        raise RuntimeError("paged_attention_tc: out must be [T, H, dv] of the query's dtype with unit inner stride")
+    _check(library().tlb_paged_attention_tc(_ptr(q), q.stride(0), q.stride(1), T, _ptr(slab), P, page_size, dk, dv, H, kv_heads, _ptr(block_table), block_table.shape[1],
+                                            _ptr(seq_info), seq_info.shape[0], int(runs), int(mask), int(mask_size), int(keep_first), float(scale), float(softcap or 0.0),
+                                            int(bool(sink)), _ptr(gate), gate.stride(0) if gate is not None else 0, wide, _ptr(out), out.stride(0), out.stride(1),
+                                            _ptr(head_bias), int(weights), _stream(q)))
+    return out
+
+
+def latent_rows(slab, block_table, seq_info, contexts: list):
+    """-> (rows ``[N, width]``: the cached rows of every sequence's ``contexts[s]`` positions, each sequence from a whole 64-row page
+    on, and the int32 table ``[S, pages]`` of where they are).  ``seq_info`` must say the same contexts (start + tokens)."""
+    _gpu("latent_rows", slab, block_table, seq_info)
+    _contig("latent_rows", slab, block_table, seq_info)
+    P, page_size, width = slab.shape
+    pages = [-(-n // 64) for n in contexts]
+    if len(pages) != seq_info.shape[0] or block_table.shape[0] != len(pages) or slab.dtype != torch.bfloat16:
+        raise RuntimeError("latent_rows: a bfloat16 cache, one context per sequence")
+    rows = torch.empty((64 * sum(pages), width), dtype=slab.dtype, device=slab.device)
+    table = torch.empty((len(pages), max(pages)), dtype=torch.int32, device=slab.device)
+    _check(library().tlb_latent_rows(_ptr(slab), P, page_size, width, _ptr(seq_info), len(pages), _ptr(block_table), block_table.shape[1], _ptr(rows), _ptr(table),
+                                     table.shape[1], sum(pages), _stream(slab)))
+    return rows, table
+
+
+def latent_attention_heads(q, k, v, k_rot, table, seq_info, runs: int, *, dim: int, window: int, scale: float, sink=None):
+    """Latent attention on keys and values up-projected per head: ``q [T, H, dim + rot]``, ``k [N, H * dim]``, ``v [H, N, dv]``, the
+    rotated part all heads share ``k_rot [N, rot]``; rows through ``table`` of ``latent_rows``.  -> ``[T, H, dv]``."""
+    _gpu("latent_attention_heads", q, k, v, k_rot, table, seq_info, sink)
+    _contig("latent_attention_heads", k, v, table, seq_info, sink)
+    T, H, width = q.shape
+    rot, N, dv = width - dim, k.shape[0], v.shape[2]
+    if k.shape != (N, H * dim) or v.shape != (H, N, dv) or k_rot.shape != (N, rot) or k_rot.stride(1) != 1 or not tma_rows(q) or q.dtype != torch.bfloat16:
+        raise RuntimeError("latent_attention_heads: queries, keys and values do not match")
+    if not (q.dtype == k.dtype == v.dtype == k_rot.dtype) or (sink is not None and (sink.dtype != torch.float32 or sink.shape != (H,))):
+        raise RuntimeError("latent_attention_heads: bfloat16 operands, sinks float32 [H]")
+    out = torch.empty((T, H, dv), dtype=q.dtype, device=q.device)
+    _check(library().tlb_latent_attention_heads(_ptr(q), q.stride(0), q.stride(1), T, _ptr(k), k.stride(0), _ptr(v), v.stride(0), v.stride(1), _ptr(k_rot), k_rot.stride(0),
+                                                int(dim), rot, dv, H, N, _ptr(table), table.shape[1], _ptr(seq_info), seq_info.shape[0], int(runs), int(window or 0),
+                                                float(scale), _ptr(out), out.stride(0), out.stride(1), _ptr(sink), _stream(q)))
     return out
 
 

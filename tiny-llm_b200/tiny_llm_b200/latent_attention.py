@@ -20,9 +20,14 @@ the softmax's denominator holds one more term ``exp(sink[h])``, which stands for
 
 from __future__ import annotations
 
+import os
+
 import torch
 
 from .basics import linear, linear_wide
+
+
+PER_HEAD_ENTRIES = 1 << 30  # keys and values up-projected per head: at most 2 GiB of them
 
 
 class LatentAttention:
@@ -55,6 +60,8 @@ class LatentAttention:
         # a caching layer projects q and the latent in ONE product (rows of w_q, then rows of w_dkv)
         self.caches = w_dkv is not None
         self.w_qd = torch.cat([first, w_dkv], dim=0).contiguous() if self.caches else None
+        self.tc = (self.w_o.dtype == torch.bfloat16 and dim % 64 == 0 and rot_dim % 8 == 0 and rot_dim <= 64 and dim + rot_dim <= 256 and vdim % 8 == 0 and vdim <= 256
+                   and os.environ.get("TL_FLASH_TC", "1") != "0")
 
     @property
     def cache_width(self) -> int:
@@ -65,6 +72,40 @@ class LatentAttention:
         from extensions_b200.tiny_llm_ext_b200 import blocks
 
         return blocks.attention_kernel(slab.dtype, self.heads, self.rank, self.rot_dim, slab.shape[1])
+
+    def _per_head(self, plan, q3: torch.Tensor) -> bool:
+        """Whether this step's attention runs on keys and values up-projected per head instead of on the latents themselves.
+
+        Per query, key and head the absorbed form multiplies ``2 rank + rot`` entries, this one ``dim + rot + vdim`` (1088 and 320 at
+        the larger benchmark size), and it runs on tcgen05; its price is the up projection of every cached row and three more
+        launches.  Measured (us): absorbed about 30 + its operations at 110 TFLOP/s; this one about 25 + the up projection at 600
+        TFLOP/s + 1.75 for every 64-key tile of the longest sequence and wave of CTAs.  2048 tokens, 16 heads: 723 and 158; 128 tokens
+        after 4000: 250 and 172; 64 after 4000: 147 and 168.  Below 38 us the calls are bound by the host and launches count."""
+        counts = getattr(plan, "counts", None)
+        if not self.tc or counts is None or plan.max_tokens == 1:
+            return False
+        w = self.window or (1 << 60)
+        pairs = sum(n * min(s, w) + n * min(n, w) // 2 for n, s in zip(counts, plan.starts))
+        rows = sum(counts) + sum(plan.starts)
+        tiles = min(plan.max_context, w + 128) / 64 * max(1.0, sum(-(-n // 128) for n in counts) * self.heads / 296)
+        absorbed = 30 + pairs * self.heads * (2 * self.rank + self.rot_dim) * 2 / 110e6
+        per_head = 25 + 1.75 * tiles + rows * self.rank * self.heads * (self.dim + self.vdim) * 2 / 600e6
+        if absorbed <= max(per_head, 38) or rows * self.heads * (self.dim + self.vdim) > PER_HEAD_ENTRIES:
+            return False
+        from extensions_b200.tiny_llm_ext_b200 import blocks
+
+        return blocks.tma_rows(q3)
+
+    def _attend_heads(self, q3: torch.Tensor, plan, slab: torch.Tensor) -> torch.Tensor:
+        """``[T, heads, vdim]``: the sequences' cached rows side by side, keys and values of every head from them, per-head attention."""
+        from extensions_b200.tiny_llm_ext_b200 import blocks
+
+        rows, table = blocks.latent_rows(slab, plan.block_table, plan.seq_info, [n + s for n, s in zip(plan.counts, plan.starts)])
+        c = rows[:, : self.rank]
+        k = linear(c, self.w_uk.view(self.heads * self.dim, self.rank))
+        v = torch.bmm(c.expand(self.heads, -1, -1), self.w_uv_t)  # [heads, rows, vdim]
+        return blocks.latent_attention_heads(q3, k, v, rows[:, self.rank :], table, plan.seq_info, sum(-(-n // 128) for n in plan.counts), dim=self.dim,
+                                             window=self.window, scale=self.scale, sink=self.sink)
 
     def __call__(self, h: torch.Tensor, plan, slab: torch.Tensor) -> torch.Tensor:
         from extensions_b200.tiny_llm_ext_b200 import blocks
@@ -96,6 +137,9 @@ class LatentAttention:
             blocks.rope_rows(q, plan.tok_pos, heads=H, head_stride=dn + dr, first=dn, dims=self.rot_dims, base=self.rot_base, interleaved=self.interleaved)
             q3 = q.view(T, H, dn + dr)
         kernel, tile_tokens = self.attention_kernel(slab)
+        if kernel == "mma" and self._per_head(plan, q3):
+            o = self._attend_heads(q3, plan, slab)
+            return linear_wide(o.view(T, H * self.vdim), self.w_o)
         q_lat = torch.bmm(q3[:, :, :dn].transpose(0, 1), self.w_uk)          # [H, T, rank]
         o_lat = torch.empty_like(q_lat)
         blocks.latent_attention(q_lat.transpose(0, 1), q3[:, :, dn:], slab, plan.block_table, plan.tiles_for(tile_tokens), plan.tok_pos,

@@ -130,6 +130,7 @@ class PagedGroupedAttention:
         # register-softmax kernel's forms, which take over wherever they serve the sizes
         self.kernel, self.tile_tokens = blocks.paged_attention_kernel(self.w_o.dtype, self.heads, self.kv_heads, self.dim, self.vdim, int(page_size))
         self.forms = blocks.paged_attention_flash_forms(self.w_o.dtype, self.heads, self.kv_heads, self.dim, self.vdim, int(page_size))
+        self.tc_run = blocks.flash_tc_run(self.w_o.dtype, self.heads, self.kv_heads, self.dim, self.vdim, int(page_size))
 
     @property
     def tile_sizes(self) -> list:
@@ -143,6 +144,24 @@ class PagedGroupedAttention:
             return self.kernel, self.tile_tokens
         name = "flash_split" if plan.max_tokens <= self.forms.get("flash_split", 0) else "flash"
         return name, self.forms[name]
+
+    def _tc_runs(self, plan, q3: torch.Tensor, slab: torch.Tensor) -> int:
+        """How many runs of tokens the tcgen05 kernel cuts the step into; 0: the step is for the other kernels.
+
+        A tile of 64 keys takes its CTA about 1.4 us from scores to values, and the kernel does not split a run's keys, so a short
+        portion far into a long context is the register kernel's, which does (64 tokens after 4000, causal, 4 key/value heads of
+        192: 102 us here, 47 us there).  The line where both take as long lies at about 2.2 CTAs for every tile of the longest
+        run (32 CTAs x 17 tiles: 26 and 32 us; 36 x 32: 55 and 31 us; 64 x 24: 43 and 72 us); up to 5 tiles this one wins with any
+        number of CTAs (16 tokens: 7 and 19 us)."""
+        counts = getattr(plan, "counts", None)
+        if not self.tc_run or counts is None or plan.max_tokens <= self.forms.get("flash_split", 0) or slab.shape[1] % 64:
+            return 0
+        from extensions_b200.tiny_llm_ext_b200 import blocks
+
+        reach = plan.max_context if self.mask == MASKS["causal"] else min(plan.max_context, self.mask_size + self.keep_first + self.tc_run)
+        tiles = -(-reach // 64)
+        runs = sum(-(-n // self.tc_run) for n in counts)
+        return runs if (tiles <= 5 or 5 * runs * self.kv_heads >= 11 * tiles) and blocks.tma_rows(q3) else 0
 
     @property
     def cache_width(self) -> int:
@@ -179,6 +198,11 @@ class PagedGroupedAttention:
                                   tok_pos=plan.tok_pos, tok_seq=plan.tok_seq, block_table=plan.block_table, slab=slab)
             elif q_norm is not None:
                 blocks.kv_prepare(q3, None, None, q_norm=q_norm, eps=self.eps)
+        runs = self._tc_runs(plan, q3, slab)
+        if runs:
+            return blocks.paged_attention_tc(q3, slab, plan.block_table, plan.seq_info, runs, kv_heads=G, dv=self.vdim, mask=self.mask, mask_size=self.mask_size,
+                                             keep_first=self.keep_first, scale=self.scale, softcap=self.softcap, sink=self.sink, gate=gate, head_bias=self.head_bias,
+                                             weights=self.weights, out=out)
         kernel, tile = self._kernel(plan)
         return blocks.paged_attention(q3, slab, plan.block_table, plan.tiles_for(tile), plan.tok_pos, kv_heads=G, dv=self.vdim, mask=self.mask,
                                       mask_size=self.mask_size, keep_first=self.keep_first, scale=self.scale, softcap=self.softcap, sink=self.sink, gate=gate,

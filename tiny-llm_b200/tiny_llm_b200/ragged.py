@@ -135,7 +135,7 @@ class RaggedPlan:
         self.max_context = max(o.offset for o in owners)  # the longest sequence after this step's append
         self.want_counts = [len(x) for x in wants]
         self.all_wanted = W == T and all(x == list(range(len(x))) for x in wants)  # the wanted rows are the step's rows, in order
-        self.starts = starts
+        self.starts, self.counts = starts, counts
         self.max_tokens = max(counts)  # the longest entry of the step
         self.owners = owners
         for o, ran in zip(owners, tokens):  # from here on the step runs: what it consumes cannot be taken back from a recurrent state
