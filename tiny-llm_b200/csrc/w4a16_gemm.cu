@@ -89,7 +89,7 @@ struct Deq<__half> {
 // M = 4096 with MT = 1: 470-550 TF/s, 28-33 % of the bf16 peak).
 template <int MT>
 struct GemmSmem {
-    static constexpr int STAGES = MT <= 2 ? GSTAGES_MAX : 2;
+    static constexpr int STAGES = MT <= 2 ? GSTAGES_MAX : MT == 3 ? 3 : 2;
     static constexpr int A_STAGE = MT * G_TILE_BYTES;
     static constexpr int A_OFF = 0;
     static constexpr int B_OFF = STAGES * A_STAGE;
@@ -97,30 +97,46 @@ struct GemmSmem {
     static constexpr int BYTES = BAR_OFF + 256;
 };
 
+// Which tiles a launch's CTAs take: `full` CTAs of MT token tiles each (a feature tile's last group may be shorter), then the
+// groups from number `full` on in pieces of `piece` token tiles.  See gemm_plan.
+struct GemmPlan {
+    int n_tiles, m_tiles, full, piece;
+};
+
 template <typename T, int MT>
 __global__ void __launch_bounds__(G_THREADS, 1) w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const T *__restrict__ scales,
                                                                   const T *__restrict__ biases, const uint32_t *__restrict__ b,
-                                                                  T *__restrict__ out, int M, int N, int K, int vec_store) {
+                                                                  T *__restrict__ out, int M, int N, int K, int vec_store, const GemmPlan plan) {
     extern __shared__ __align__(1024) unsigned char gsm[];
 #if TL_TRACE
-    // per-block cycle stamps of CTA (0,0) (tools/gemm_blocks.py): role 0 = MMA warp (k: activation tile ready, weight tile
+    // per-block cycle stamps of CTA 0 (tools/gemm_blocks.py): role 0 = MMA warp (k: activation tile ready, weight tile
     // ready, MMAs issued), role 1 = first dequantiser thread (k: loop top, math done, stage free, handed over)
     __shared__ unsigned long long trc[2][40][4];
 #define G_TRC(role, i, k)                                                                                                    \
     do {                                                                                                                     \
-        if (blockIdx.x == 0 && blockIdx.y == 0 && (threadIdx.x & 31) == 0 && (i) < 40) trc[role][i][k] = clock64();         \
+        if (blockIdx.x == 0 && (threadIdx.x & 31) == 0 && (i) < 40) trc[role][i][k] = clock64();         \
     } while (0)
 #else
 #define G_TRC(role, i, k) do { } while (0)
 #endif
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_tile = blockIdx.x, m_tile = blockIdx.y;
+    int group = blockIdx.x, m0 = 0, mt = MT;  // feature tiles run fastest, so that CTAs side by side share token tiles
+    if (group >= plan.full) {
+        const int parts = (MT + plan.piece - 1) / plan.piece, rest = group - plan.full;
+        group = plan.full + rest / parts;
+        m0 = rest % parts * plan.piece;
+        mt = min(plan.piece, MT - m0);
+    }
+    const int n_tile = group % plan.n_tiles;
+    const int m_tile = group / plan.n_tiles * MT + m0;  // the CTA's first token tile, of `mt`
+    mt = min(mt, plan.m_tiles - m_tile);
+    if (mt <= 0) return;  // a piece past a short group's end
     const int num_kb = N / GK;
     const int G = N / 128;
 
     using Smem = GemmSmem<MT>;
     constexpr int GSTAGES = Smem::STAGES;
-    constexpr int TMEM_COLS = G_TMEM_COLS * MT;
+    constexpr int TMEM_COLS = MT == 3 ? 512 : G_TMEM_COLS * MT;  // a power of two
     const uint32_t a_base = g_smem_u32(gsm + Smem::A_OFF);
     const uint32_t b_base = g_smem_u32(gsm + Smem::B_OFF);
     const uint32_t bar_base = g_smem_u32(gsm + Smem::BAR_OFF);
@@ -156,10 +172,10 @@ __global__ void __launch_bounds__(G_THREADS, 1) w4a16_gemm_kernel(const __grid_c
         for (int kb = 0; kb < num_kb; ++kb) {
             g_mbar_wait(empty + 8 * s, ph);
             if (g_elect_one()) {
-                g_mbar_expect_tx(full + 8 * s, Smem::A_STAGE);
+                g_mbar_expect_tx(full + 8 * s, mt * G_TILE_BYTES);
 #pragma unroll
                 for (int i = 0; i < MT; ++i)  // token rows beyond M are zero-filled by the TMA unit
-                    g_tma_load_2d(a_base + s * Smem::A_STAGE + i * G_TILE_BYTES, &tmap_a, kb * GK, (m_tile * MT + i) * GM, full + 8 * s);
+                    if (i < mt) g_tma_load_2d(a_base + s * Smem::A_STAGE + i * G_TILE_BYTES, &tmap_a, kb * GK, (m_tile + i) * GM, full + 8 * s);
             }
             __syncwarp();
             if (++s == GSTAGES) s = 0, ph ^= 1u;
@@ -182,6 +198,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) w4a16_gemm_kernel(const __grid_c
                 const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(s * (G_TILE_BYTES >> 4));
 #pragma unroll
                 for (int i = 0; i < MT; ++i) {
+                    if (i >= mt) break;
                     const uint64_t adesc = adesc0 + static_cast<uint64_t>((s * Smem::A_STAGE + i * G_TILE_BYTES) >> 4);
 #pragma unroll
                     for (int k = 0; k < GK / 16; ++k)  // +32 bytes along K per step: +2 in the (addr >> 4) field
@@ -263,7 +280,8 @@ __global__ void __launch_bounds__(G_THREADS, 1) w4a16_gemm_kernel(const __grid_c
 #pragma unroll
         for (int cbi = 0; cbi < 2 * MT; ++cbi) {
             const int i = cbi >> 1, cb = cbi & 1;
-            const int m = (m_tile * MT + i) * GM + q * 32 + lane;
+            if (i >= mt) break;
+            const int m = (m_tile + i) * GM + q * 32 + lane;
             const int col0 = col_half * 64 + cb * 32;
             uint32_t v[32];
             g_tmem_ld32(tmem_d + (static_cast<uint32_t>(q * 32) << 16) + i * G_TMEM_COLS + col0, v);
@@ -293,7 +311,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) w4a16_gemm_kernel(const __grid_c
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "n"(TMEM_COLS) : "memory");
     }
 #if TL_TRACE
-    if (blockIdx.x == 0 && blockIdx.y == 0 && g_trace_buf != nullptr) {  // tag = 20000 + role * 1000 + block * 4 + k
+    if (blockIdx.x == 0 && g_trace_buf != nullptr) {  // tag = 20000 + role * 1000 + block * 4 + k
         for (int e = threadIdx.x; e < 2 * 40 * 4; e += G_THREADS) {
             const int role = e / 160, rest = e - role * 160;
             if (rest / 4 < num_kb && !(role == 0 && (rest & 3) == 3)) {
@@ -340,19 +358,44 @@ bool w4a16_gemm_supported(int M, int N, int K, int dtype) {
 int w4a16_gemm_split(int, int, int, int) { return 1; }
 size_t w4a16_gemm_workspace(int, int, int, int, int) { return 0; }
 
+// Cycles of a 64-wide reduction block with mt token tiles per CTA, measured where every SM has one CTA (148 x 128 features; 9728
+// long: 55, 92 and 112 us for one to three tiles; 2560 long: 38 and 45 us for three and four).
+static int gemm_block_cost(int mt) {
+    static const int cost[5] = {0, 650, 1090, 1330, 1640};
+    return cost[mt];
+}
+
+// How to cut a product of n_tiles x m_tiles tiles (128 features x 128 tokens) into CTAs, one per SM at a time: groups of mt token
+// tiles share a dequantised weight tile, and the groups that would fill only part of a last wave are cut into pieces small enough
+// to fill it.  Returns the cost of a reduction block summed over the waves.  2048 tokens, against fixed groups of four (short
+// reductions) or two: 2560 -> 9728 122 -> 104 us (304 groups: two waves and 8 left over), 9728 -> 2560 150 -> 99 us (160 groups of two
+// were two waves; 120 of three are one), 4096 -> 2560 73 -> 50 us; 512 tokens 2560 -> 4096 41 -> 24 us (64 SMs had had work).
+static long long gemm_plan(int mt, int n_tiles, int m_tiles, GemmPlan &plan) {
+    const int sms = sm_count(), groups = n_tiles * ceil_div(m_tiles, mt), left = groups % sms;
+    plan = {n_tiles, m_tiles, groups - left, mt};
+    if (left == 0) return static_cast<long long>(groups / sms) * gemm_block_cost(mt);
+    for (int piece = 1; piece < mt; ++piece)
+        if (left * ceil_div(mt, piece) <= sms) {
+            plan.piece = piece;
+            break;
+        }
+    return static_cast<long long>(groups / sms) * gemm_block_cost(mt) + gemm_block_cost(plan.piece);
+}
+
 template <typename T, int MT>
 static int gemm_launch(const CUtensorMap &map, const void *scales, const void *biases, const void *b, void *out, int M, int N, int K,
-                       int vec_store, cudaStream_t st) {
+                       int vec_store, const GemmPlan &plan, cudaStream_t st) {
     static bool configured = false;
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(w4a16_gemm_kernel<T, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<MT>::BYTES);
         if (e != cudaSuccess) return fail(TL_ECUDA, "quantized_matmul: cannot raise shared memory limit: %s", cudaGetErrorString(e));
         configured = true;
     }
-    dim3 grid(ceil_div(K, GN), ceil_div(M, GM * MT));
-    w4a16_gemm_kernel<T, MT><<<grid, G_THREADS, GemmSmem<MT>::BYTES, st>>>(map, static_cast<const T *>(scales), static_cast<const T *>(biases),
+    const int groups = plan.n_tiles * ceil_div(plan.m_tiles, MT);
+    const int ctas = plan.full + (groups - plan.full) * ceil_div(MT, plan.piece);
+    w4a16_gemm_kernel<T, MT><<<ctas, G_THREADS, GemmSmem<MT>::BYTES, st>>>(map, static_cast<const T *>(scales), static_cast<const T *>(biases),
                                                                            static_cast<const uint32_t *>(b), static_cast<T *>(out), M, N, K,
-                                                                           vec_store);
+                                                                           vec_store, plan);
     TL_LAUNCH_CHECK("w4a16_gemm");
     return TL_OK;
 }
@@ -373,13 +416,24 @@ static int gemm_t(const void *scales, const void *biases, const void *a, const v
                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(TL_ECUDA, "quantized_matmul: cuTensorMapEncodeTiled failed (%d)", static_cast<int>(r));
     const int vec_store = (K % 8 == 0 && aligned16(out)) ? 1 : 0;
-    // Four token tiles per CTA leave room for a 2-stage ring only: measured at M = 4096, that wins for the
-    // short reductions (N = 2560: q|k|v 641 -> 769 TF/s, gate|up 782 -> 882) and loses for the long ones
-    // (N = 9728: 706 -> 655), so it is used up to N = 3072.  TL_GEMM_MT caps the tile count (A/B runs).
-    static const int mt_max = [] { const char *e = getenv("TL_GEMM_MT"); return e ? atoi(e) : 4; }();
-    if (M > 2 * GM && mt_max >= 4 && N <= 3072) return gemm_launch<T, 4>(map, scales, biases, b, out, M, N, K, vec_store, st);
-    return M > GM && mt_max >= 2 ? gemm_launch<T, 2>(map, scales, biases, b, out, M, N, K, vec_store, st)
-                                 : gemm_launch<T, 1>(map, scales, biases, b, out, M, N, K, vec_store, st);
+    static const int mt_max = [] { const char *e = getenv("TL_GEMM_MT"); return e ? atoi(e) : 4; }();  // caps the token tiles per CTA (A/B runs)
+    const int n_tiles = ceil_div(K, GN), m_tiles = ceil_div(M, GM);
+    GemmPlan plan, best_plan{};
+    int best = 0;
+    long long best_cost = 0;
+    for (int mt = 1; mt <= 4 && mt <= max(mt_max, 1); ++mt) {
+        // Four token tiles leave room for a 2-stage ring only: good for the short reductions, not for the long ones (M = 4096:
+        // N = 2560 gains 13-20 % over two tiles, N = 9728 loses 7 %).
+        if ((mt == 4 && N > 3072) || mt > m_tiles) continue;
+        const long long cost = gemm_plan(mt, n_tiles, m_tiles, plan);
+        if (best == 0 || cost <= best_cost) best = mt, best_cost = cost, best_plan = plan;
+    }
+    switch (best) {
+        case 1: return gemm_launch<T, 1>(map, scales, biases, b, out, M, N, K, vec_store, best_plan, st);
+        case 2: return gemm_launch<T, 2>(map, scales, biases, b, out, M, N, K, vec_store, best_plan, st);
+        case 3: return gemm_launch<T, 3>(map, scales, biases, b, out, M, N, K, vec_store, best_plan, st);
+        default: return gemm_launch<T, 4>(map, scales, biases, b, out, M, N, K, vec_store, best_plan, st);
+    }
 }
 
 int launch_w4a16_gemm(const void *scales, const void *biases, const void *a, const void *b, void *out, int M, int N, int K,
