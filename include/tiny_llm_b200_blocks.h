@@ -182,15 +182,16 @@ int tlb_qk_whole_prepare(void *q, long long q_token, int heads, const void *q_no
  * z_bias `dtype` or NULL, out [T, heads, dv] fp32 contiguous.  dk <= 256.
  * max_tokens_per_seq = the largest token count in seq_info (known to the host).  Up to TLB_DECAY_SCAN_SEGMENT tokens a
  * sequence is walked in one go.  Longer portions are cut at the multiples of the segment length in absolute positions and
- * run in three launches (every segment's local end state and decay product from a zero state; the segments' start
- * states by walking those in order; outputs per segment), which needs tlb_decay_scan_workspace(...) bytes. */
+ * run in three launches (every segment's outputs, local end state and decay product from a zero state; the segments' start
+ * states by walking those in order; what a start state adds to its segment's outputs), which needs
+ * tlb_decay_scan_workspace(...) bytes.  tokens = T. */
 #define TLB_DECAY_SCAN_SEGMENT 64
-size_t tlb_decay_scan_workspace(int num_seqs, int max_tokens_per_seq, int heads, int dk, int dv);
+size_t tlb_decay_scan_workspace(int tokens, int num_seqs, int max_tokens_per_seq, int heads, int dk, int dv);
 int tlb_decay_scan(const void *q, long long q_token, long long q_head, const void *k, long long k_token, long long k_head, const void *v,
                    long long v_token, long long v_head, const float *z, long long z_token, const void *z_bias, float tau, const float *head_decay,
                    const float *rope_cos, const float *rope_sin, int rope_dims, int rope_interleaved, float q_scale, int heads,
-                   int dk, int dv, const int32_t *seq_info, int num_seqs, int max_tokens_per_seq, float *state, long long slot_stride,
-                   int num_slots, float *out, void *workspace, size_t workspace_bytes, int decay_kind, const void *a_log, const void *bonus,
+                   int dk, int dv, const int32_t *seq_info, int num_seqs, int tokens, int max_tokens_per_seq, float *state,
+                   long long slot_stride, int num_slots, float *out, void *workspace, size_t workspace_bytes, int decay_kind, const void *a_log, const void *bonus,
                    int qk_heads, const void *skip, int v_cols, int dtype, void *stream);
 /* decay_kind 0: as above.  2: alpha = exp(-exp(z + z_bias)) per key channel.  3: one decay per head and token,
  * alpha = exp(-exp(a_log[h]) dt), dt = softplus(z[t, h] + z_bias[h]) (z [T, heads]), and the token's key is multiplied by dt

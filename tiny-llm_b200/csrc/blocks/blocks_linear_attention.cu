@@ -6,21 +6,24 @@
 // or, given head_decay, one fixed alpha per head (retention).  With rotation tables the first rope_dims entries of every
 // head of q and k are rotated by the token's tabulated angle while they are staged, in fp32: what enters the recurrence is
 // never rounded back to the projections' type.
-// The columns of S never mix, so a CTA owns 32 of them for one (sequence, head) and walks tokens in order; 4 lanes share
-// a column, each holding every 4th row of it in registers.  The tokens' q, k and decays are staged 16 (8 for dk > 128) at a time in shared
+// The columns of S never mix, so a CTA owns 32 (64, 128) of them for one (sequence, head) and walks tokens in order; 4 lanes share
+// one (two, four) columns, each holding every 4th row of them in registers.  The tokens' q, k and decays are staged 16 (8 for dk > 128) at a time in shared
 // memory as fp32 (the decay is computed there, in fp32, from the fp32 logits).  A sequence that starts at position 0
 // starts from zero, whatever its slot held; otherwise the slot is read, and in both cases written back after the last
 // token.  Single tokens and portions of up to 64 tokens are one walk.  A longer portion is cut into segments at the
-// multiples of 64 in ABSOLUTE positions, which run side by side: every segment's local end state from zero and the
-// product of its decays, then the start state of every segment by walking those in order (S' = decay * S + local), then
-// the outputs of every segment from its start state.  Every sum has an order fixed by token, channel and segment
+// multiples of 64 in ABSOLUTE positions, which run side by side in three launches: every segment's outputs and end state from a
+// zero state (the first one from the sequence's own), with its queries times the decays since its start put aside; the start state
+// of every segment by walking those in order (S' = decay * S + local); and what a start state adds to its segment's outputs, the
+// product of those queries with it.  (The recurrence run once more from the start states instead of that product was half of
+// the time.)  Every sum has an order fixed by token, channel and segment
 // indices alone; the cuts depend on positions only, so how a prompt was cut into steps changes the result by the
 // rounding of the combination at most.
+// 2048 tokens in two sequences, 16 heads of 64 x 128: 208 + 9 + 208 us -> XX.
 #include "blocks_common.cuh"
 
 namespace tlb {
 
-constexpr int kLaCols = 32;    // state columns per CTA
+constexpr int kLaThreads = 128;
 constexpr int kLaLanes = 4;    // lanes per column
 constexpr int kLaSegment = TLB_DECAY_SCAN_SEGMENT;  // positions per segment of a long portion
 
@@ -35,13 +38,13 @@ __device__ __forceinline__ bool la_segment(int p0, int n, int c, int &lo, int &h
     return true;
 }
 
-// One kernel, three uses (pass):
+// One kernel, two uses (pass):
 //   0  the whole portion of a sequence in one CTA per (head, column block): state from the slot (or zero at position 0),
 //      outputs, state back to the slot.  Single tokens and short portions.
-//   1  segment c alone from a ZERO state, no outputs: its local end state and the product of its decays go to the
-//      workspace (the last segment of a sequence is skipped: nobody needs its local state).
-//   3  segment c from the start state that decay_combine_kernel left in the workspace: outputs; the last segment writes
-//      the slot.
+//   1  segment c alone, from a ZERO state (c = 0: as in pass 0): its outputs, and to the workspace its end state, the product of
+//      its decays and (c > 0) its scaled queries times the decays from its first token on, decayed [T, heads, dk]; of a
+//      sequence's last segment also the steps themselves, last_steps [sequences, 64, heads, dk] = (decay, key).  A sequence that
+//      is one segment is done with that.
 //
 // decay_kind chooses where the decay comes from: 0 = sigmoid(z + bias)^(1/tau) per key channel, or head_decay; 2 = exp(-exp(z + bias))
 // per key channel; 3 = one number per head and token, exp(-exp(a_log[h]) dt) with dt = softplus(z[t, h] + bias[h]), and the
@@ -52,47 +55,51 @@ __device__ __forceinline__ bool la_segment(int p0, int n, int c, int &lo, int &h
 // update and sees the token's own k v^T weighted by bonus [heads, dk] instead: o_t = (S + diag(bonus) k_t v_t^T)^T q_t.
 // SCALAR: the decay is one number per head and token (head_decay, decay_kind 3 and 4): it is read once per token, and a row of the
 // state reads 8 bytes of its token's staged numbers instead of 16.
-template <typename T, int KR /* rows per lane: dk <= 4 * KR */, int kLaTokens /* tokens staged at a time */, bool BONUS, bool SCALAR>
-__global__ void __launch_bounds__(kLaCols * kLaLanes, SCALAR && KR == 32 ? 8 : 1)
+// NC: state columns per thread.  A row's staged numbers are read from shared memory once for all of them: with one column the scan
+// was bound by those reads (16 bytes for three multiply-adds, and every 32 columns staged the decays anew).
+template <typename T, int KR /* rows per lane: dk <= 4 * KR */, int kLaTokens /* tokens staged at a time */, bool BONUS, bool SCALAR, int NC>
+__global__ void __launch_bounds__(kLaThreads, NC > 1 ? 4 : SCALAR && KR == 32 ? 8 : 1)
 decay_scan_kernel(const T *__restrict__ q, long long q_token, long long q_head, const T *__restrict__ k, long long k_token, long long k_head,
                   const T *__restrict__ v, long long v_token, long long v_head, const float *__restrict__ z, long long z_token,
                   const T *__restrict__ z_bias, float inv_tau, const float *__restrict__ head_decay, const float *__restrict__ rope_cos,
                   const float *__restrict__ rope_sin, int rope_dims, int rope_interleaved, float q_scale, int heads, int dk, int dv,
                   const int32_t *__restrict__ seq_info,
                   float *__restrict__ state, long long slot_stride, int num_slots, float *__restrict__ out, int pass, int max_segments,
-                  float *__restrict__ seg_state, float *__restrict__ seg_decay, int decay_kind, const T *__restrict__ a_log,
+                  float *__restrict__ seg_state, float *__restrict__ seg_decay, float *__restrict__ decayed, float2 *__restrict__ last_steps, int decay_kind, const T *__restrict__ a_log,
                   const T *__restrict__ bonus, int qk_heads, const T *__restrict__ skip, int v_cols) {
     __shared__ float4 sx[SCALAR ? 1 : kLaTokens * 4 * KR];   // per token and key channel: (decay, k, scaled q, k times the bonus), one 16-byte read per row
     __shared__ float2 skq[SCALAR ? kLaTokens * 4 * KR : 1];  // SCALAR: (k, scaled q)
-    __shared__ float sv[kLaTokens * kLaCols];
+    constexpr int COLS = kLaThreads / kLaLanes * NC;  // per CTA
+    constexpr int BATCH = 4;
+    __shared__ __align__(16) float sv[kLaTokens * COLS];
     __shared__ float sprod[4 * KR];
     __shared__ float2 s_step[kLaTokens];  // SCALAR: the token's (decay, key factor), worked out or read once per token
     __shared__ float2 s_chan[4 * KR];     // per key channel of this head: (the decay logit's bias, the bonus), read once
-    const int colblocks = (dv + kLaCols - 1) / kLaCols;
-    const int s = blockIdx.x, head = blockIdx.y / colblocks, col0 = (blockIdx.y % colblocks) * kLaCols, c = blockIdx.z;
+    const int colblocks = (dv + COLS - 1) / COLS;
+    const int s = blockIdx.x, head = blockIdx.y / colblocks, col0 = (blockIdx.y % colblocks) * COLS, c = blockIdx.z;
     const int seq_first = seq_info[s * 4 + 0], seq_count = seq_info[s * 4 + 1], start = seq_info[s * 4 + 2], slot = seq_info[s * 4 + 3];
     int lo = start, hi = start + seq_count, nseg = 1;
     if (pass != 0 && !la_segment(start, seq_count, c, lo, hi, nseg)) return;
-    if (pass == 1 && c == nseg - 1) return;
     const int first = seq_first + (lo - start), count = hi - lo;
     const int cidx = threadIdx.x / kLaLanes, r = threadIdx.x % kLaLanes;
-    const int col = col0 + cidx;
-    const bool col_ok = col < dv;
+    const int col = col0 + cidx * NC;  // .. col + NC - 1
+    const int cols = min(NC, dv - col);  // <= 0: none
     const bool slot_ok = slot >= 0 && slot < num_slots;
     float *mine = state + (size_t)(slot_ok ? slot : 0) * slot_stride + (size_t)head * dk * dv;
     float *seg = seg_state ? seg_state + (((size_t)s * max_segments + c) * heads + head) * dk * dv : nullptr;
-    const bool from_slot = pass == 0 || (pass == 3 && c == 0);   // else: zero (pass 1) or the combined start state (pass 3)
-    const bool to_slot = pass == 0 || (pass == 3 && c == nseg - 1);
+    const bool from_slot = pass == 0 || c == 0;  // else from zero
+    const bool to_slot = pass == 0 || nseg == 1;
+    const bool keeps_decays = !to_slot && col0 == 0;  // one column block per head
 
-    float S[KR];
+    float S[KR][NC];
 #pragma unroll
     for (int i = 0; i < KR; ++i) {
-        int row = r + kLaLanes * i;
-        bool ok = col_ok && row < dk;
-        if (from_slot) S[i] = (lo > 0 && slot_ok && ok) ? mine[(size_t)row * dv + col] : 0.f;
-        else S[i] = (pass == 3 && ok) ? seg[(size_t)row * dv + col] : 0.f;
+        const int row = r + kLaLanes * i;
+        const float *src = from_slot && lo > 0 && slot_ok ? mine : nullptr;
+#pragma unroll
+        for (int u = 0; u < NC; ++u) S[i][u] = src && row < dk && u < cols ? src[(size_t)row * dv + col + u] : 0.f;
     }
-    if (pass == 1)
+    if (keeps_decays)
         for (int d = threadIdx.x; d < dk; d += blockDim.x) sprod[d] = 1.f;
     for (int d = threadIdx.x; d < dk; d += blockDim.x)
         s_chan[d] = make_float2((z_bias && decay_kind < 3) ? to_f(z_bias[(size_t)head * dk + d]) : 0.f, BONUS ? to_f(bonus[(size_t)head * dk + d]) : 0.f);
@@ -115,42 +122,81 @@ decay_scan_kernel(const T *__restrict__ q, long long q_token, long long q_head, 
                                                       : make_float2(head_decay[head], 1.f);
             __syncthreads();
         }
-        for (int e = threadIdx.x; e < n * dk; e += blockDim.x) {
-            int j = e / dk, d = e - j * dk;
-            size_t tok = (size_t)(first + t0 + j);
-            float alpha, kmul = 1.f;
-            if (SCALAR) alpha = 0.f, kmul = s_step[j].y;
-            else if (decay_kind == 2) alpha = expf(-expf(z[tok * z_token + (size_t)head * dk + d] + s_chan[d].x));
-            else alpha = expf(log_sigmoid(z[tok * z_token + (size_t)head * dk + d] + s_chan[d].x) * inv_tau);
-            const T *kp = k + tok * k_token + (size_t)qk_head * k_head, *qp = q + tok * q_token + (size_t)qk_head * q_head;
-            float kd = to_f(kp[d]), qd = to_f(qp[d]);
-            if (d < rope_dims) {  // rotate the pair this entry belongs to, in fp32, by the token's tabulated angle
-                const int half = rope_dims >> 1;
-                const bool low = rope_interleaved ? !(d & 1) : d < half;
-                const int i = rope_interleaved ? d >> 1 : (low ? d : d - half);
-                const int other = rope_interleaved ? (d ^ 1) : (low ? d + half : d - half);
-                const float c = rope_cos[tok * half + i], sn = low ? -rope_sin[tok * half + i] : rope_sin[tok * half + i];
-                kd = kd * c + to_f(kp[other]) * sn;
-                qd = qd * c + to_f(qp[other]) * sn;
+        // BATCH entries' numbers are on their way at once: one at a time, a chunk's staging was a chain of memory round trips longer
+        // than its multiply-adds
+        for (int e0 = threadIdx.x; e0 < n * dk; e0 += BATCH * kLaThreads) {
+            float zs[BATCH];
+            T ks[BATCH], qs[BATCH];
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u) {
+                const int e = e0 + u * kLaThreads;
+                if (e >= n * dk) break;
+                const int j = e / dk, d = e - j * dk;
+                const size_t tok = (size_t)(first + t0 + j);
+                if (!SCALAR) zs[u] = z[tok * z_token + (size_t)head * dk + d];
+                ks[u] = k[tok * k_token + (size_t)qk_head * k_head + d], qs[u] = q[tok * q_token + (size_t)qk_head * q_head + d];
             }
-            kd *= kmul;
-            if (SCALAR) skq[j * 4 * KR + d] = make_float2(kd, qd * q_scale);
-            else sx[j * 4 * KR + d] = make_float4(alpha, kd, qd * q_scale, BONUS ? kd * s_chan[d].y : 0.f);
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u) {
+                const int e = e0 + u * kLaThreads;
+                if (e >= n * dk) break;
+                const int j = e / dk, d = e - j * dk;
+                const size_t tok = (size_t)(first + t0 + j);
+                float alpha, kmul = 1.f;
+                if (SCALAR) alpha = 0.f, kmul = s_step[j].y;
+                else if (decay_kind == 2) alpha = expf(-expf(zs[u] + s_chan[d].x));
+                else alpha = expf(log_sigmoid(zs[u] + s_chan[d].x) * inv_tau);
+                float kd = to_f(ks[u]), qd = to_f(qs[u]);
+                if (d < rope_dims) {  // rotate the pair this entry belongs to, in fp32, by the token's tabulated angle
+                    const int half = rope_dims >> 1;
+                    const bool low = rope_interleaved ? !(d & 1) : d < half;
+                    const int i = rope_interleaved ? d >> 1 : (low ? d : d - half);
+                    const int other = rope_interleaved ? (d ^ 1) : (low ? d + half : d - half);
+                    const float c = rope_cos[tok * half + i], sn = low ? -rope_sin[tok * half + i] : rope_sin[tok * half + i];
+                    kd = kd * c + to_f(k[tok * k_token + (size_t)qk_head * k_head + other]) * sn;
+                    qd = qd * c + to_f(q[tok * q_token + (size_t)qk_head * q_head + other]) * sn;
+                }
+                kd *= kmul;
+                if (SCALAR) skq[j * 4 * KR + d] = make_float2(kd, qd * q_scale);
+                else sx[j * 4 * KR + d] = make_float4(alpha, kd, qd * q_scale, BONUS ? kd * s_chan[d].y : 0.f);
+            }
         }
-        for (int e = threadIdx.x; e < n * kLaCols; e += blockDim.x) {
-            int j = e / kLaCols, d = e - j * kLaCols;
-            sv[e] = col0 + d < v_cols ? to_f(v[(size_t)(first + t0 + j) * v_token + (size_t)head * v_head + col0 + d]) : col0 + d < dv ? 1.f : 0.f;
+        for (int e0 = threadIdx.x; e0 < n * COLS; e0 += 2 * BATCH * kLaThreads) {
+            T vs[2 * BATCH];
+#pragma unroll
+            for (int u = 0; u < 2 * BATCH; ++u) {
+                const int e = e0 + u * kLaThreads, j = e / COLS, d = e - j * COLS;
+                if (e < n * COLS && col0 + d < v_cols) vs[u] = v[(size_t)(first + t0 + j) * v_token + (size_t)head * v_head + col0 + d];
+            }
+#pragma unroll
+            for (int u = 0; u < 2 * BATCH; ++u) {
+                const int e = e0 + u * kLaThreads, d = e % COLS;
+                if (e < n * COLS) sv[e] = col0 + d < v_cols ? to_f(vs[u]) : col0 + d < dv ? 1.f : 0.f;
+            }
         }
         __syncthreads();
-        if (pass == 1) {  // the segment's decay product per key channel, in token order
+        if (keeps_decays) {  // the segment's decay product per key channel, in token order, and the queries times it
             for (int d = threadIdx.x; d < dk; d += blockDim.x) {
                 float p = sprod[d];
-                for (int j = 0; j < n; ++j) p *= SCALAR ? s_step[j].x : sx[j * 4 * KR + d].x;
+                for (int j = 0; j < n; ++j) {
+                    const float before = p;
+                    p *= SCALAR ? s_step[j].x : sx[j * 4 * KR + d].x;
+                    if (c == nseg - 1)
+                        last_steps[(((size_t)s * kLaSegment + t0 + j) * heads + head) * dk + d] =
+                            SCALAR ? make_float2(s_step[j].x, skq[j * 4 * KR + d].x) : make_float2(sx[j * 4 * KR + d].x, sx[j * 4 * KR + d].y);
+                    if (c > 0)
+                        decayed[((size_t)(first + t0 + j) * heads + head) * dk + d] = (SCALAR ? skq[j * 4 * KR + d].y : sx[j * 4 * KR + d].z) * (BONUS ? before : p);
+                }
                 sprod[d] = p;
             }
         }
         for (int j = 0; j < n; ++j) {
-            const float vj = sv[j * kLaCols + cidx];
+            float vj[NC];
+            if constexpr (NC >= 4) {
+#pragma unroll
+                for (int u = 0; u < NC; u += 4) *reinterpret_cast<float4 *>(vj + u) = *reinterpret_cast<const float4 *>(sv + j * COLS + cidx * NC + u);
+            } else if constexpr (NC == 2) *reinterpret_cast<float2 *>(vj) = *reinterpret_cast<const float2 *>(sv + j * COLS + cidx * NC);
+            else vj[0] = sv[j * COLS + cidx];
             const float4 *xa = sx + (SCALAR ? 0 : j * 4 * KR);
             const float2 *ya = skq + (SCALAR ? j * 4 * KR : 0);
             const float keep = SCALAR ? s_step[j].x : 0.f;
@@ -159,65 +205,77 @@ decay_scan_kernel(const T *__restrict__ q, long long q_token, long long q_head, 
                 const float2 y = ya[row];
                 return make_float4(keep, y.x, y.y, 0.f);
             };
-            float o0 = 0.f, o1 = 0.f;
+            float o[2][NC] = {};  // over this lane's even and odd rows
 #pragma unroll
-            for (int i = 0; i < KR; i += 2) {
-                int row = r + kLaLanes * i;
+            for (int i = 0; i < KR; ++i) {
+                const int row = r + kLaLanes * i;
                 if (row < dk) {
-                    float4 x = staged(row);
-                    if (BONUS) o0 = fmaf(x.z, fmaf(x.w, vj, S[i]), o0);
-                    S[i] = fmaf(x.x, S[i], x.y * vj);
-                    if (!BONUS) o0 = fmaf(x.z, S[i], o0);
-                }
-                if (row + kLaLanes < dk) {
-                    float4 x = staged(row + kLaLanes);
-                    if (BONUS) o1 = fmaf(x.z, fmaf(x.w, vj, S[i + 1]), o1);
-                    S[i + 1] = fmaf(x.x, S[i + 1], x.y * vj);
-                    if (!BONUS) o1 = fmaf(x.z, S[i + 1], o1);
+                    const float4 x = staged(row);
+#pragma unroll
+                    for (int u = 0; u < NC; ++u) {
+                        if (BONUS) o[i & 1][u] = fmaf(x.z, fmaf(x.w, vj[u], S[i][u]), o[i & 1][u]);
+                        S[i][u] = fmaf(x.x, S[i][u], x.y * vj[u]);
+                        if (!BONUS) o[i & 1][u] = fmaf(x.z, S[i][u], o[i & 1][u]);
+                    }
                 }
             }
-            if (pass != 1) {
-                float o = o0 + o1;
-                o += __shfl_xor_sync(0xffffffffu, o, 1);
-                o += __shfl_xor_sync(0xffffffffu, o, 2);
-                if (r == 0 && col_ok) out[((size_t)(first + t0 + j) * heads + head) * dv + col] = fmaf(skipv, vj, o);
+            float y[NC];
+#pragma unroll
+            for (int u = 0; u < NC; ++u) {
+                y[u] = o[0][u] + o[1][u];
+                y[u] += __shfl_xor_sync(0xffffffffu, y[u], 1);
+                y[u] += __shfl_xor_sync(0xffffffffu, y[u], 2);
+                y[u] = fmaf(skipv, vj[u], y[u]);
             }
+            float *to = out + ((size_t)(first + t0 + j) * heads + head) * dv + col;
+            // the lanes of a column group share its stores
+#pragma unroll
+            for (int u = 0; u < NC; ++u)
+                if (u < cols && r == u % kLaLanes) to[u] = y[u];
         }
     }
-    float *dst = to_slot ? (slot_ok ? mine : nullptr) : (pass == 1 ? seg : nullptr);
-    if (dst != nullptr && col_ok) {
+    float *dst = to_slot ? (slot_ok ? mine : nullptr) : seg;
+    if (dst != nullptr) {
 #pragma unroll
         for (int i = 0; i < KR; ++i) {
-            int row = r + kLaLanes * i;
-            if (row < dk) dst[(size_t)row * dv + col] = S[i];
+            const int row = r + kLaLanes * i;
+#pragma unroll
+            for (int u = 0; u < NC; ++u)
+                if (row < dk && u < cols) dst[(size_t)row * dv + col + u] = S[i][u];
         }
     }
-    if (pass == 1 && col0 == 0) {
+    if (keeps_decays) {
         __syncthreads();
         float *pd = seg_decay + (((size_t)s * max_segments + c) * heads + head) * dk;
         for (int d = threadIdx.x; d < dk; d += blockDim.x) pd[d] = sprod[d];
     }
 }
 
-// Between the two passes: walk a sequence's segments in order, S_start[c + 1] = decay[c] * S_start[c] + local[c], and leave
-// every segment's START state where its local end state was.  One thread per state element, (sequence, head) per blockIdx.
+// Walk a sequence's segments in order, S_start[c + 1] = decay[c] * S_start[c] + local[c], and leave every segment's START state
+// where its local end state was (segment 0 began from the sequence's own state: nothing is added to it); then the last segment's
+// tokens from its start state, step by step as the scan itself takes them, to the state the slot gets.  One thread per state
+// element, (sequence, head) per blockIdx.
+template <typename T>
 __global__ void __launch_bounds__(256)
-decay_combine_kernel(const int32_t *__restrict__ seq_info, const float *__restrict__ state, long long slot_stride, int num_slots, int heads, int dk,
-                     int dv, int max_segments, float *__restrict__ seg_state, const float *__restrict__ seg_decay) {
+decay_combine_kernel(const int32_t *__restrict__ seq_info, float *__restrict__ state, long long slot_stride, int num_slots, int heads, int dk,
+                     int dv, int max_segments, float *__restrict__ seg_state, const float *__restrict__ seg_decay, const float2 *__restrict__ last_steps,
+                     const T *__restrict__ v, long long v_token, long long v_head, int v_cols) {
     const int s = blockIdx.x, head = blockIdx.y;
-    const int count = seq_info[s * 4 + 1], start = seq_info[s * 4 + 2], slot = seq_info[s * 4 + 3];
+    const int seq_first = seq_info[s * 4 + 0], count = seq_info[s * 4 + 1], start = seq_info[s * 4 + 2], slot = seq_info[s * 4 + 3];
     int lo, hi, nseg;
     la_segment(start, count, 0, lo, hi, nseg);
     if (nseg <= 1) return;
-    const bool slot_ok = slot >= 0 && slot < num_slots;
-    const float *mine = state + (size_t)(slot_ok ? slot : 0) * slot_stride + (size_t)head * dk * dv;
+    la_segment(start, count, nseg - 1, lo, hi, nseg);
+    const int n = hi - lo;
+    const T *values = v + (size_t)(seq_first + lo - start) * v_token + (size_t)head * v_head;
+    const float2 *steps = last_steps + ((size_t)s * kLaSegment * heads + head) * dk;
     for (int e = blockIdx.z * blockDim.x + threadIdx.x; e < dk * dv; e += gridDim.z * blockDim.x) {
-        const int row = e / dv;
-        float S = (start > 0 && slot_ok) ? mine[e] : 0.f;
-        // eight segments' local states and decays are fetched before the first of them is used: the walk is a chain of
-        // multiply-adds, not of memory round trips
+        const int row = e / dv, col = e - row * dv;
+        float S = 0.f;
+        // eight segments' local states and decays (tokens' steps) are fetched before the first of them is used: the walk is a
+        // chain of multiply-adds, not of memory round trips
         constexpr int kAhead = 8;
-        for (int c0 = 0; c0 + 1 < nseg; c0 += kAhead) {
+        for (int c0 = 0; c0 < nseg; c0 += kAhead) {
             float local[kAhead], decay[kAhead];
 #pragma unroll
             for (int u = 0; u < kAhead; ++u) {
@@ -230,13 +288,77 @@ decay_combine_kernel(const int32_t *__restrict__ seq_info, const float *__restri
 #pragma unroll
             for (int u = 0; u < kAhead; ++u) {
                 const int c = c0 + u;
-                if (c + 1 < nseg) {
+                if (c < nseg) {
                     seg_state[(((size_t)s * max_segments + c) * heads + head) * dk * dv + e] = S;
-                    S = fmaf(decay[u], S, local[u]);
+                    if (c + 1 < nseg) S = fmaf(decay[u], S, local[u]);
                 }
             }
         }
-        seg_state[(((size_t)s * max_segments + (nseg - 1)) * heads + head) * dk * dv + e] = S;
+        if (slot < 0 || slot >= num_slots) continue;
+        for (int t0 = 0; t0 < n; t0 += kAhead) {
+            float2 x[kAhead];
+            float vj[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (t0 + u < n) {
+                    x[u] = steps[(size_t)(t0 + u) * heads * dk + row];
+                    vj[u] = col < v_cols ? to_f(values[(size_t)(t0 + u) * v_token + col]) : 1.f;
+                }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (t0 + u < n) S = fmaf(x[u].x, S, x[u].y * vj[u]);
+        }
+        state[(size_t)slot * slot_stride + (size_t)head * dk * dv + e] = S;
+    }
+}
+
+// out[t, h, :] += decayed[t, h, :] S_start for the tokens of segments 1, 2, ..: a product of up to 64 tokens x dk by dk x 64 columns
+// per CTA, in fp32, k ascending.  Thread: 8 tokens x 4 columns.
+constexpr int kLaOutCols = 64, kLaOutK = 32;
+__global__ void __launch_bounds__(128)
+decay_output_kernel(const int32_t *__restrict__ seq_info, int heads, int dk, int dv, int max_segments, const float *__restrict__ seg_state,
+                    const float *__restrict__ decayed, float *__restrict__ out) {
+    const int colblocks = (dv + kLaOutCols - 1) / kLaOutCols;
+    const int s = blockIdx.x, head = blockIdx.y / colblocks, col0 = (blockIdx.y % colblocks) * kLaOutCols, c = blockIdx.z + 1;
+    const int seq_first = seq_info[s * 4 + 0], count = seq_info[s * 4 + 1], start = seq_info[s * 4 + 2];
+    int lo, hi, nseg;
+    if (!la_segment(start, count, c, lo, hi, nseg)) return;
+    const int first = seq_first + (lo - start), n = hi - lo;
+    const float *S = seg_state + (((size_t)s * max_segments + c) * heads + head) * dk * dv;
+    __shared__ __align__(16) float sq[kLaOutK][kLaSegment + 4], ss[kLaOutK][kLaOutCols];
+    const int tr = threadIdx.x / 16 * 8, tc = threadIdx.x % 16 * 4;
+    float acc[8][4] = {};
+    for (int k0 = 0; k0 < dk; k0 += kLaOutK) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kLaSegment * kLaOutK / 128; ++i) {
+            const int e = threadIdx.x + i * 128, t = e / kLaOutK, k = e % kLaOutK;
+            sq[k][t] = t < n && k0 + k < dk ? decayed[((size_t)(first + t) * heads + head) * dk + k0 + k] : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < kLaOutCols * kLaOutK / 128; ++i) {
+            const int e = threadIdx.x + i * 128, k = e / kLaOutCols, d = e % kLaOutCols;
+            ss[k][d] = k0 + k < dk && col0 + d < dv ? S[(size_t)(k0 + k) * dv + col0 + d] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int k = 0; k < kLaOutK; ++k) {
+            const float4 a = *reinterpret_cast<const float4 *>(&sq[k][tr]), b = *reinterpret_cast<const float4 *>(&sq[k][tr + 4]),
+                         x = *reinterpret_cast<const float4 *>(&ss[k][tc]);
+            const float q[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, y[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(q[i], y[j], acc[i][j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        if (tr + i >= n) break;
+        float *o = out + ((size_t)(first + tr + i) * heads + head) * dv + col0 + tc;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (col0 + tc + j < dv) o[j] += acc[i][j];
     }
 }
 
@@ -282,16 +404,16 @@ using namespace tlb;
 
 extern "C" {
 
-size_t tlb_decay_scan_workspace(int num_seqs, int max_tokens_per_seq, int heads, int dk, int dv) {
+size_t tlb_decay_scan_workspace(int tokens, int num_seqs, int max_tokens_per_seq, int heads, int dk, int dv) {
     if (max_tokens_per_seq <= kLaSegment) return 0;
     size_t segs = (size_t)num_seqs * (2 + (max_tokens_per_seq - 1) / kLaSegment);
-    return segs * heads * ((size_t)dk * dv + dk) * sizeof(float);
+    return (segs * heads * ((size_t)dk * dv + dk) + ((size_t)tokens + 2 * kLaSegment * (size_t)num_seqs) * heads * dk + 1) * sizeof(float);
 }
 
 int tlb_decay_scan(const void *q, long long q_token, long long q_head, const void *k, long long k_token, long long k_head, const void *v,
                    long long v_token, long long v_head, const float *z, long long z_token, const void *z_bias, float tau, const float *head_decay,
                    const float *rope_cos, const float *rope_sin, int rope_dims, int rope_interleaved, float q_scale, int heads,
-                   int dk, int dv, const int32_t *seq_info, int num_seqs, int max_tokens_per_seq, float *state, long long slot_stride, int num_slots,
+                   int dk, int dv, const int32_t *seq_info, int num_seqs, int tokens, int max_tokens_per_seq, float *state, long long slot_stride, int num_slots,
                    float *out, void *workspace, size_t workspace_bytes, int decay_kind, const void *a_log, const void *bonus, int qk_heads,
                    const void *skip, int v_cols, int dtype, void *stream) {
     if (num_seqs <= 0) return TL_OK;
@@ -310,23 +432,39 @@ int tlb_decay_scan(const void *q, long long q_token, long long q_head, const voi
     // portions longer than a segment are cut at absolute multiples of the segment length and run in three passes
     const bool segmented = max_tokens_per_seq > kLaSegment;
     const int max_segments = segmented ? 2 + (max_tokens_per_seq - 1) / kLaSegment : 1;
-    float *seg_state = nullptr, *seg_decay = nullptr;
+    float *seg_state = nullptr, *seg_decay = nullptr, *decayed = nullptr;
+    float2 *last_steps = nullptr;
     if (segmented) {
-        if (!workspace || workspace_bytes < tlb_decay_scan_workspace(num_seqs, max_tokens_per_seq, heads, dk, dv))
+        if (!workspace || workspace_bytes < tlb_decay_scan_workspace(tokens, num_seqs, max_tokens_per_seq, heads, dk, dv))
             return tl::fail(TL_EWORKSPACE, "decay_scan: workspace missing or too small");
         seg_state = (float *)workspace;
         seg_decay = seg_state + (size_t)num_seqs * max_segments * heads * dk * dv;
+        decayed = seg_decay + (size_t)num_seqs * max_segments * heads * dk;
+        float *end = decayed + (size_t)tokens * heads * dk;
+        last_steps = (float2 *)(end + ((uintptr_t)end / 4 & 1));  // 8-byte aligned
     }
     const bool scalar = head_decay || decay_kind >= 3;
     if (scalar && bonus) return tl::fail(TL_EINVAL, "decay_scan: a bonus goes with a decay per key channel");
-    const int colblocks = ceil_div(dv, kLaCols);
     cudaStream_t st = as_stream(stream);
-    int kr = ceil_div(dk, kLaLanes);
-#define TLB_DS_B(KRV, PASS, GZ, BON, SCA)                                                                                                                \
-    decay_scan_kernel<T, KRV, (KRV > 32 ? 8 : 16), BON, SCA><<<dim3(num_seqs, heads * colblocks, GZ), kLaCols * kLaLanes, 0, st>>>(                                           \
+    const int kr = ceil_div(dk, kLaLanes);
+    // Four, two or one columns a thread (64 registers of state): more read a row's staged numbers fewer times, fewer give more CTAs
+    // to hide the staging behind (16 heads, 33 segments: 191 us for both launches of the scan with four, 217 with two; 8 heads: 154
+    // and 117).  A step of few tokens takes one, so that more CTAs share the state's traffic.
+    const auto ctas = [&](int nc) { return (long long)heads * ceil_div(dv, kLaThreads / kLaLanes * nc) * num_seqs * max_segments; };
+    int nc = 1;
+    for (int more = kr <= 16 ? 4 : kr <= 32 ? 2 : 1; more > 1 && max_tokens_per_seq > 4 && nc == 1; more /= 2)
+        if (ctas(more) >= 3 * 148) nc = more;
+#define TLB_DS_N(KRV, PASS, GZ, BON, SCA, NCV)                                                                                                           \
+    decay_scan_kernel<T, KRV, (KRV > 32 ? 8 : 16), BON, SCA, NCV><<<dim3(num_seqs, heads * ceil_div(dv, kLaThreads / kLaLanes * NCV), GZ), kLaThreads, 0, st>>>(  \
         (const T *)q, q_token, q_head, (const T *)k, k_token, k_head, (const T *)v, v_token, v_head, z, z_token, (const T *)z_bias, z ? 1.0f / tau : 0.f, head_decay, \
         rope_cos, rope_sin, rope_dims, rope_interleaved, q_scale, heads, dk, dv, seq_info, state, slot_stride, num_slots, out, PASS, max_segments, seg_state, seg_decay, \
-        decay_kind, (const T *)a_log, (const T *)bonus, qk_heads, (const T *)skip, v_cols)
+        decayed, last_steps, decay_kind, (const T *)a_log, (const T *)bonus, qk_heads, (const T *)skip, v_cols)
+#define TLB_DS_B(KRV, PASS, GZ, BON, SCA)                                                                     \
+    do {                                                                                                      \
+        if (KRV <= 16 && nc == 4) TLB_DS_N(KRV, PASS, GZ, BON, SCA, (KRV <= 16 ? 4 : 1));                      \
+        else if (KRV <= 32 && nc == 2) TLB_DS_N(KRV, PASS, GZ, BON, SCA, (KRV <= 32 ? 2 : 1));                 \
+        else TLB_DS_N(KRV, PASS, GZ, BON, SCA, 1);                                                            \
+    } while (0)
 #define TLB_DS_K(KRV, PASS, GZ) do { if (bonus) TLB_DS_B(KRV, PASS, GZ, true, false); else if (scalar) TLB_DS_B(KRV, PASS, GZ, false, true); else TLB_DS_B(KRV, PASS, GZ, false, false); } while (0)
 #define TLB_DS(PASS, GZ) TLB_DISPATCH(dtype, "decay_scan", if (kr <= 8) TLB_DS_K(8, PASS, GZ); else if (kr <= 16) TLB_DS_K(16, PASS, GZ); else if (kr <= 32) TLB_DS_K(32, PASS, GZ); else TLB_DS_K(64, PASS, GZ))
     if (!segmented) {
@@ -335,15 +473,17 @@ int tlb_decay_scan(const void *q, long long q_token, long long q_head, const voi
         return TL_OK;
     }
     TLB_DS(1, max_segments);
-    TL_LAUNCH_CHECK("decay_scan (local states)");
-    decay_combine_kernel<<<dim3(num_seqs, heads, ceil_div(dk * dv, 256)), 256, 0, st>>>(seq_info, state, slot_stride, num_slots, heads, dk, dv,
-                                                                                           max_segments, seg_state, seg_decay);
+    TL_LAUNCH_CHECK("decay_scan (segments)");
+    TLB_DISPATCH(dtype, "decay_scan", decay_combine_kernel<T><<<dim3(num_seqs, heads, ceil_div(dk * dv, 256)), 256, 0, st>>>(
+                                          seq_info, state, slot_stride, num_slots, heads, dk, dv, max_segments, seg_state, seg_decay, last_steps, (const T *)v, v_token,
+                                          v_head, v_cols));
     TL_LAUNCH_CHECK("decay_scan (combine)");
-    TLB_DS(3, max_segments);
+    decay_output_kernel<<<dim3(num_seqs, heads * ceil_div(dv, kLaOutCols), max_segments - 1), 128, 0, st>>>(seq_info, heads, dk, dv, max_segments, seg_state, decayed, out);
     TL_LAUNCH_CHECK("decay_scan (outputs)");
 #undef TLB_DS
 #undef TLB_DS_K
 #undef TLB_DS_B
+#undef TLB_DS_N
     return TL_OK;
 }
 

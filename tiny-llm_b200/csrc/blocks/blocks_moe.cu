@@ -39,12 +39,17 @@ __device__ __forceinline__ void moe_load(const bf16 *p, float (&x)[W]) {
     }
 }
 
+template <typename T, int W>
+struct __align__(W * sizeof(T)) MoePiece {
+    T v[W];
+};
+
 // A CTA routes TOK tokens, so that a row of weights is fetched once for all of them: their rows of h are staged in shared memory,
-// the warps share the experts, four rows of weights in flight each (a logit is one warp's dot product in a lane order fixed by the
+// the warps share the experts, two or four rows of weights in flight each (a logit is one warp's dot product in a lane order fixed by the
 // width, whatever TOK and the launch are), then warp i picks token i's top-k.  W: entries per access (16 bytes where rows allow).
 // aux_w: one more row of weights that is no router output; aux[t] = sigmoid(aux_w . h_t) (the gate of a shared expert).
 template <typename T, int TOK, int W>
-__global__ void __launch_bounds__(TOK == 1 ? 1024 : 256)
+__global__ void __launch_bounds__(TOK == 1 ? 512 : 256, TOK == 1 ? 1 : 4)
 moe_route_kernel(const T *__restrict__ h, const T *__restrict__ w, const T *__restrict__ b, int tokens, int dim, int experts, int top, int scoring,
                  const T *__restrict__ choice_bias, float weight_scale, int group_count, int group_keep, const T *__restrict__ aux_w,
                  float *__restrict__ aux, int32_t *__restrict__ idx, float *__restrict__ gate) {
@@ -59,7 +64,7 @@ moe_route_kernel(const T *__restrict__ h, const T *__restrict__ w, const T *__re
         else *reinterpret_cast<uint4 *>(x + d) = *reinterpret_cast<const uint4 *>(h + (size_t)t0 * dim + d);
     }
     __syncthreads();
-    constexpr int ROWS = 4;
+    constexpr int ROWS = TOK == 1 ? 4 : 2;
     const int outputs = experts + (aux_w ? 1 : 0);
     for (int e0 = warp; e0 < outputs; e0 += warps * ROWS) {
         float acc[ROWS][TOK];
@@ -71,21 +76,38 @@ moe_route_kernel(const T *__restrict__ h, const T *__restrict__ w, const T *__re
 #pragma unroll
             for (int i = 0; i < TOK; ++i) acc[r][i] = 0.f;
         }
-        for (int d = lane * W; d < dim; d += 32 * W) {
-            float wv[ROWS][W];
+        // a few tokens: two steps of weights are on their way while one is used (16 tokens: 14 -> 11 us).  Many tokens: two rows a warp
+        // and four CTAs an SM hide the round trips better than more registers for weights do (2048 tokens, 64 x 2048 weights: four
+        // rows at one, two and four steps ahead 55, 42 and 74 us, two rows 37).
+        constexpr int AHEAD = TOK == 1 ? 2 : 1;
+        MoePiece<T, W> next[AHEAD][ROWS];
+        auto fetch = [&](int d, MoePiece<T, W> (&to)[ROWS]) {
 #pragma unroll
             for (int r = 0; r < ROWS; ++r)
-                if (e0 + r * warps < outputs) moe_load<W>(row[r] + d, wv[r]);
+                if (d < dim && e0 + r * warps < outputs) to[r] = *reinterpret_cast<const MoePiece<T, W> *>(row[r] + d);
+        };
 #pragma unroll
-            for (int i = 0; i < TOK; ++i) {
-                float xv[W];
-                moe_load<W>(x + (size_t)i * dim + d, xv);
+        for (int u = 0; u < AHEAD; ++u) fetch((u * 32 + lane) * W, next[u]);
+        for (int d0 = lane * W; d0 < dim; d0 += AHEAD * 32 * W) {
 #pragma unroll
-                for (int r = 0; r < ROWS; ++r)
-                    if (e0 + r * warps < outputs) {
+            for (int u = 0; u < AHEAD; ++u) {
+                const int d = d0 + u * 32 * W;
+                if (d >= dim) break;
+                float wv[ROWS][W];
 #pragma unroll
-                        for (int j = 0; j < W; ++j) acc[r][i] = fmaf(xv[j], wv[r][j], acc[r][i]);
-                    }
+                for (int r = 0; r < ROWS; ++r) moe_load<W>(next[u][r].v, wv[r]);
+                fetch(d + AHEAD * 32 * W, next[u]);
+#pragma unroll
+                for (int i = 0; i < TOK; ++i) {
+                    float xv[W];
+                    moe_load<W>(x + (size_t)i * dim + d, xv);
+#pragma unroll
+                    for (int r = 0; r < ROWS; ++r)
+                        if (e0 + r * warps < outputs) {
+#pragma unroll
+                            for (int j = 0; j < W; ++j) acc[r][i] = fmaf(xv[j], wv[r][j], acc[r][i]);
+                        }
+                }
             }
         }
 #pragma unroll
@@ -247,20 +269,45 @@ __global__ void moe_scale_rows_kernel(const T *__restrict__ h, const float *__re
     for (int d = threadIdx.x; d < dim; d += blockDim.x) out[(size_t)pair * dim + d] = from_f<T>(g * to_f(src[d]));
 }
 
-// idx != NULL: a choice whose expert id is >= experts is an identity expert, its output the token's input row h[t, :].
-template <typename T>
-__global__ void moe_combine_kernel(const float *__restrict__ pair_out, const float *__restrict__ gate, const T *__restrict__ shared,
-                                   const float *__restrict__ shared_gate, const int32_t *__restrict__ idx, int experts, const T *__restrict__ h, float *__restrict__ y, int top, int dim) {
-    int t = blockIdx.x;
-    for (int d = threadIdx.x; d < dim; d += blockDim.x) {
-        float s = 0.f;
-        for (int k = 0; k < top; ++k) {
-            const bool same = idx != nullptr && idx[(size_t)t * top + k] >= experts;
-            s = fmaf(gate ? gate[(size_t)t * top + k] : 1.f, same ? to_f(h[(size_t)t * dim + d]) : pair_out[((size_t)t * top + k) * dim + d], s);
-        }
-        if (shared) s = fmaf(shared_gate ? shared_gate[t] : 1.f, to_f(shared[(size_t)t * dim + d]), s);
-        y[(size_t)t * dim + d] = s;
+// idx != NULL: a choice whose expert id is >= experts is an identity expert, its output the token's input row h[t, :].  A thread
+// sums W columns; W = 4: a CTA takes 1024 columns of a token and all its choices' rows are on their way at once (2048 tokens of 6
+// choices and 2048 columns: 37 -> 22 us, 16 tokens: 13 -> 3 us; before, a column and a choice at a time).
+template <typename T, int W>
+__global__ void __launch_bounds__(256)
+moe_combine_kernel(const float *__restrict__ pair_out, const float *__restrict__ gate, const T *__restrict__ shared,
+                   const float *__restrict__ shared_gate, const int32_t *__restrict__ idx, int experts, const T *__restrict__ h, float *__restrict__ y, int top, int dim) {
+    const int t = blockIdx.x, d = (blockIdx.y * 256 + threadIdx.x) * W;
+    if (d >= dim) return;
+    constexpr int AT_ONCE = 8;
+    float s[W] = {};
+    for (int k0 = 0; k0 < top; k0 += AT_ONCE) {
+        float x[AT_ONCE][W];
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; ++u)
+            if (k0 + u < top) {
+                const size_t pair = (size_t)t * top + k0 + u;
+                if (idx != nullptr && idx[pair] >= experts) {
+#pragma unroll
+                    for (int j = 0; j < W; ++j) x[u][j] = to_f(h[(size_t)t * dim + d + j]);
+                } else {
+                    moe_load<W>(pair_out + pair * dim + d, x[u]);
+                }
+            }
+#pragma unroll
+        for (int u = 0; u < AT_ONCE; ++u)
+            if (k0 + u < top) {
+                const float g = gate ? gate[(size_t)t * top + k0 + u] : 1.f;
+#pragma unroll
+                for (int j = 0; j < W; ++j) s[j] = fmaf(g, x[u][j], s[j]);
+            }
     }
+    if (shared) {
+        const float g = shared_gate ? shared_gate[t] : 1.f;
+#pragma unroll
+        for (int j = 0; j < W; ++j) s[j] = fmaf(g, to_f(shared[(size_t)t * dim + d + j]), s[j]);
+    }
+    if constexpr (W == 4) *reinterpret_cast<float4 *>(y + (size_t)t * dim + d) = make_float4(s[0], s[1], s[2], s[3]);
+    else y[(size_t)t * dim + d] = s[0];
 }
 
 }  // namespace tlb
@@ -300,7 +347,7 @@ int tlb_moe_route(const void *h, const void *w, const void *b, int tokens, int d
     const bool wide = dim * es % 16 == 0 && tl::aligned16(h) && tl::aligned16(w) && (!aux_w || tl::aligned16(aux_w));
     // four tokens a CTA once that fills the GPU; few tokens: more warps each, so that no warp walks many rows of weights
     const bool many = tokens >= 4 * 148 * 2 && bytes(4) <= 48 * 1024;
-    const int threads = many || tokens > 148 ? 256 : 1024;
+    const int threads = many || tokens > 148 ? 256 : 512;
 #define TLB_ROUTE(TOK, WV)                                                                                                                         \
     moe_route_kernel<T, TOK, WV><<<ceil_div(tokens, TOK), threads, bytes(TOK), as_stream(stream)>>>(                                                \
         (const T *)h, (const T *)w, (const T *)b, tokens, dim, experts, top, scoring, (const T *)choice_bias, weight_scale, group_count, group_keep, \
@@ -352,8 +399,11 @@ int tlb_moe_combine(const float *pair_out, const float *gate, const void *shared
                     int top, int dim, int dtype, void *stream) {
     if (tokens <= 0) return TL_OK;
     if (!pair_out || !y || top <= 0 || dim <= 0 || (idx && !h)) return tl::fail(TL_EINVAL, "moe_combine: bad argument");
-    TLB_DISPATCH(dtype, "moe_combine",
-                 moe_combine_kernel<T><<<tokens, 256, 0, as_stream(stream)>>>(pair_out, gate, (const T *)shared, shared_gate, idx, experts, (const T *)h, y, top, dim));
+    const bool wide = dim % 4 == 0 && tl::aligned16(pair_out) && tl::aligned16(y);
+    const dim3 grid(tokens, ceil_div(dim, wide ? 1024 : 256));
+#define TLB_COMBINE(WV) moe_combine_kernel<T, WV><<<grid, 256, 0, as_stream(stream)>>>(pair_out, gate, (const T *)shared, shared_gate, idx, experts, (const T *)h, y, top, dim)
+    TLB_DISPATCH(dtype, "moe_combine", if (wide) TLB_COMBINE(4); else TLB_COMBINE(1));
+#undef TLB_COMBINE
     TL_LAUNCH_CHECK("moe_combine");
     return TL_OK;
 }

@@ -65,8 +65,8 @@ _SIGNATURES = {
     "tlb_latent_attention_heads": (_I, [_VP, _LL, _LL, _I, _VP, _LL, _VP, _LL, _LL, _VP, _LL, _I, _I, _I, _I, _LL, _VP, _I, _VP, _I, _I, _I, _F, _VP, _LL, _LL, _VP, _VP]),
     "tlb_kv_prepare": (_I, [_VP, _LL, _LL, _I, _VP, _VP, _LL, _LL, _VP, _LL, _LL, _I, _I, _I, _VP, _F, _VP, _VP, _VP, _I, _I, _I, _VP, _I, _I, _VP]),
     "tlb_qk_whole_prepare": (_I, [_VP, _LL, _I, _VP, _VP, _LL, _VP, _LL, _I, _I, _I, _VP, _F, _I, _I, _D, _VP, _VP, _VP, _I, _I, _I, _VP, _VP, _VP, _I, _I, _VP]),
-    "tlb_decay_scan_workspace": (ctypes.c_size_t, [_I, _I, _I, _I, _I]),
-    "tlb_decay_scan": (_I, [_VP, _LL, _LL, _VP, _LL, _LL, _VP, _LL, _LL, _VP, _LL, _VP, _F, _VP, _VP, _VP, _I, _I, _F, _I, _I, _I, _VP, _I, _I, _VP, _LL, _I,
+    "tlb_decay_scan_workspace": (ctypes.c_size_t, [_I, _I, _I, _I, _I, _I]),
+    "tlb_decay_scan": (_I, [_VP, _LL, _LL, _VP, _LL, _LL, _VP, _LL, _LL, _VP, _LL, _VP, _F, _VP, _VP, _VP, _I, _I, _F, _I, _I, _I, _VP, _I, _I, _I, _VP, _LL, _I,
                             _VP, _VP, ctypes.c_size_t, _I, _VP, _VP, _I, _VP, _I, _I, _VP]),
     "tlb_delta_scan_workspace": (ctypes.c_size_t, [_I, _I, _I, _I, _I]),
     "tlb_delta_scan": (_I, [_VP, _LL, _LL, _VP, _LL, _LL, _VP, _LL, _LL, _VP, _LL, _VP, _I, _LL, _I, _VP, _VP, _F, _F, _I, _I, _I, _I, _VP, _I, _I, _VP, _LL,
@@ -851,11 +851,11 @@ def decay_scan(q, k, v, z, z_bias, *, tau: float = 1.0, q_scale: float, seq_info
         out = torch.empty((T, H, dv), dtype=torch.float32, device=q.device)
     longest = T if max_tokens is None else max(1, min(int(max_tokens), T))
     lib = library()
-    nbytes = int(lib.tlb_decay_scan_workspace(seq_info.shape[0], longest, H, dk, dv))
+    nbytes = int(lib.tlb_decay_scan_workspace(T, seq_info.shape[0], longest, H, dk, dv))
     ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device) if nbytes else None
     _check(lib.tlb_decay_scan(_ptr(q), q.stride(0), q.stride(1), _ptr(k), k.stride(0), k.stride(1), _ptr(v), v.stride(0), v.stride(1), _ptr(z),
                               z.stride(0) if z is not None else 0, _ptr(z_bias), float(tau), _ptr(head_decay), _ptr(cs), _ptr(sn), int(rope_dims),
-                              int(bool(rope_interleaved)), float(q_scale), H, dk, dv, _ptr(seq_info), seq_info.shape[0], longest, _ptr(state),
+                              int(bool(rope_interleaved)), float(q_scale), H, dk, dv, _ptr(seq_info), seq_info.shape[0], T, longest, _ptr(state),
                               state.stride(0), state.shape[0], _ptr(out), _ptr(ws), nbytes, int(decay_kind), _ptr(a_log), _ptr(bonus), G, _ptr(skip), v_cols,
                               _code(q.dtype), _stream(q)))
     return out
