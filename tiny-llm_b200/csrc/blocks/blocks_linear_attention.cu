@@ -18,7 +18,10 @@
 // the time.)  Every sum has an order fixed by token, channel and segment
 // indices alone; the cuts depend on positions only, so how a prompt was cut into steps changes the result by the
 // rounding of the combination at most.
-// 2048 tokens in two sequences, 16 heads of 64 x 128: 208 + 9 + 208 us -> XX.
+// 2048 tokens in two sequences, 16 heads of 64 x 128: 208 + 9 + 208 us (the recurrence twice, a column a thread) -> 99 + 19 + 24.
+// The scan is bound by instructions and the staging's round trips: 25 M of its 50 M are multiply-adds.
+#include <type_traits>
+
 #include "blocks_common.cuh"
 
 namespace tlb {
@@ -58,7 +61,7 @@ __device__ __forceinline__ bool la_segment(int p0, int n, int c, int &lo, int &h
 // NC: state columns per thread.  A row's staged numbers are read from shared memory once for all of them: with one column the scan
 // was bound by those reads (16 bytes for three multiply-adds, and every 32 columns staged the decays anew).
 template <typename T, int KR /* rows per lane: dk <= 4 * KR */, int kLaTokens /* tokens staged at a time */, bool BONUS, bool SCALAR, int NC>
-__global__ void __launch_bounds__(kLaThreads, NC > 1 ? 4 : SCALAR && KR == 32 ? 8 : 1)
+__global__ void __launch_bounds__(kLaThreads, NC > 1 ? (KR == 32 ? 3 : 4) : SCALAR && KR == 32 ? 8 : 1)
 decay_scan_kernel(const T *__restrict__ q, long long q_token, long long q_head, const T *__restrict__ k, long long k_token, long long k_head,
                   const T *__restrict__ v, long long v_token, long long v_head, const float *__restrict__ z, long long z_token,
                   const T *__restrict__ z_bias, float inv_tau, const float *__restrict__ head_decay, const float *__restrict__ rope_cos,
@@ -206,32 +209,48 @@ decay_scan_kernel(const T *__restrict__ q, long long q_token, long long q_head, 
                 return make_float4(keep, y.x, y.y, 0.f);
             };
             float o[2][NC] = {};  // over this lane's even and odd rows
+            auto rows = [&](auto whole) {  // whole: dk = 4 KR, no row to leave out
 #pragma unroll
-            for (int i = 0; i < KR; ++i) {
-                const int row = r + kLaLanes * i;
-                if (row < dk) {
-                    const float4 x = staged(row);
+                for (int i = 0; i < KR; ++i) {
+                    const int row = r + kLaLanes * i;
+                    if (decltype(whole)::value || row < dk) {
+                        const float4 x = staged(row);
 #pragma unroll
-                    for (int u = 0; u < NC; ++u) {
-                        if (BONUS) o[i & 1][u] = fmaf(x.z, fmaf(x.w, vj[u], S[i][u]), o[i & 1][u]);
-                        S[i][u] = fmaf(x.x, S[i][u], x.y * vj[u]);
-                        if (!BONUS) o[i & 1][u] = fmaf(x.z, S[i][u], o[i & 1][u]);
+                        for (int u = 0; u < NC; ++u) {
+                            if (BONUS) o[i & 1][u] = fmaf(x.z, fmaf(x.w, vj[u], S[i][u]), o[i & 1][u]);
+                            S[i][u] = fmaf(x.x, S[i][u], x.y * vj[u]);
+                            if (!BONUS) o[i & 1][u] = fmaf(x.z, S[i][u], o[i & 1][u]);
+                        }
                     }
                 }
-            }
-            float y[NC];
-#pragma unroll
-            for (int u = 0; u < NC; ++u) {
-                y[u] = o[0][u] + o[1][u];
-                y[u] += __shfl_xor_sync(0xffffffffu, y[u], 1);
-                y[u] += __shfl_xor_sync(0xffffffffu, y[u], 2);
-                y[u] = fmaf(skipv, vj[u], y[u]);
-            }
+            };
+            if ((NC > 1 || KR <= 16) && dk == 4 * KR) rows(std::true_type{});
+            else rows(std::false_type{});
+            // the four lanes' sums: ((0 + 1) + (2 + 3)), each lane ending with its share of the columns
             float *to = out + ((size_t)(first + t0 + j) * heads + head) * dv + col;
-            // the lanes of a column group share its stores
+            if constexpr (NC == 4) {
+                const bool odd = r & 1, high = r & 2;
+                float y[4], w[2];
 #pragma unroll
-            for (int u = 0; u < NC; ++u)
-                if (u < cols && r == u % kLaLanes) to[u] = y[u];
+                for (int u = 0; u < 4; ++u) y[u] = o[0][u] + o[1][u];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {  // columns u and u + 2 of this lane's parity: 0, 2 or 1, 3
+                    const float keep_y = odd ? y[2 * u + 1] : y[2 * u], give = odd ? y[2 * u] : y[2 * u + 1];
+                    w[u] = keep_y + __shfl_xor_sync(0xffffffffu, give, 1);
+                }
+                const float mine_y = high ? w[1] : w[0], give = high ? w[0] : w[1];
+                const float sum = mine_y + __shfl_xor_sync(0xffffffffu, give, 2);
+                const float vr = r == 0 ? vj[0] : r == 1 ? vj[1] : r == 2 ? vj[2] : vj[3];
+                if (r < cols) to[r] = fmaf(skipv, vr, sum);
+            } else {
+#pragma unroll
+                for (int u = 0; u < NC; ++u) {
+                    float y = o[0][u] + o[1][u];
+                    y += __shfl_xor_sync(0xffffffffu, y, 1);
+                    y += __shfl_xor_sync(0xffffffffu, y, 2);
+                    if (u < cols && r == u) to[u] = fmaf(skipv, vj[u], y);
+                }
+            }
         }
     }
     float *dst = to_slot ? (slot_ok ? mine : nullptr) : seg;
@@ -253,9 +272,9 @@ decay_scan_kernel(const T *__restrict__ q, long long q_token, long long q_head, 
 
 // Walk a sequence's segments in order, S_start[c + 1] = decay[c] * S_start[c] + local[c], and leave every segment's START state
 // where its local end state was (segment 0 began from the sequence's own state: nothing is added to it); then the last segment's
-// tokens from its start state, step by step as the scan itself takes them, to the state the slot gets.  One thread per state
-// element, (sequence, head) per blockIdx.
-template <typename T>
+// tokens from its start state, step by step as the scan itself takes them, to the state the slot gets.  One thread per W
+// neighbouring state elements of a row (W = 4: a row's numbers and the addresses are had once for four), (sequence, head) per blockIdx.
+template <typename T, int W>
 __global__ void __launch_bounds__(256)
 decay_combine_kernel(const int32_t *__restrict__ seq_info, float *__restrict__ state, long long slot_stride, int num_slots, int heads, int dk,
                      int dv, int max_segments, float *__restrict__ seg_state, const float *__restrict__ seg_decay, const float2 *__restrict__ last_steps,
@@ -269,52 +288,66 @@ decay_combine_kernel(const int32_t *__restrict__ seq_info, float *__restrict__ s
     const int n = hi - lo;
     const T *values = v + (size_t)(seq_first + lo - start) * v_token + (size_t)head * v_head;
     const float2 *steps = last_steps + ((size_t)s * kLaSegment * heads + head) * dk;
-    for (int e = blockIdx.z * blockDim.x + threadIdx.x; e < dk * dv; e += gridDim.z * blockDim.x) {
+    for (int e = (blockIdx.z * blockDim.x + threadIdx.x) * W; e < dk * dv; e += gridDim.z * blockDim.x * W) {
         const int row = e / dv, col = e - row * dv;
-        float S = 0.f;
+        float S[W] = {};
         // eight segments' local states and decays (tokens' steps) are fetched before the first of them is used: the walk is a
         // chain of multiply-adds, not of memory round trips
         constexpr int kAhead = 8;
-        for (int c0 = 0; c0 < nseg; c0 += kAhead) {
-            float local[kAhead], decay[kAhead];
+        float *seg = seg_state + ((size_t)s * max_segments * heads + head) * dk * dv + e;
+        const float *dec = seg_decay + ((size_t)s * max_segments * heads + head) * dk + row;
+        const size_t seg_step = (size_t)heads * dk * dv, dec_step = (size_t)heads * dk;
+        for (int c0 = 0; c0 < nseg; c0 += kAhead, seg += kAhead * seg_step, dec += kAhead * dec_step) {
+            float local[kAhead][W], decay[kAhead];
 #pragma unroll
-            for (int u = 0; u < kAhead; ++u) {
-                const int c = c0 + u;
-                if (c + 1 < nseg) {
-                    local[u] = seg_state[(((size_t)s * max_segments + c) * heads + head) * dk * dv + e];
-                    decay[u] = seg_decay[(((size_t)s * max_segments + c) * heads + head) * dk + row];
+            for (int u = 0; u < kAhead; ++u)
+                if (c0 + u + 1 < nseg) {
+                    if constexpr (W == 4) *reinterpret_cast<float4 *>(local[u]) = *reinterpret_cast<const float4 *>(seg + u * seg_step);
+                    else local[u][0] = seg[u * seg_step];
+                    decay[u] = dec[u * dec_step];
                 }
-            }
 #pragma unroll
-            for (int u = 0; u < kAhead; ++u) {
-                const int c = c0 + u;
-                if (c < nseg) {
-                    seg_state[(((size_t)s * max_segments + c) * heads + head) * dk * dv + e] = S;
-                    if (c + 1 < nseg) S = fmaf(decay[u], S, local[u]);
+            for (int u = 0; u < kAhead; ++u)
+                if (c0 + u < nseg) {
+                    if constexpr (W == 4) *reinterpret_cast<float4 *>(seg + u * seg_step) = make_float4(S[0], S[1], S[2], S[3]);
+                    else seg[u * seg_step] = S[0];
+                    if (c0 + u + 1 < nseg) {
+#pragma unroll
+                        for (int w = 0; w < W; ++w) S[w] = fmaf(decay[u], S[w], local[u][w]);
+                    }
                 }
-            }
         }
         if (slot < 0 || slot >= num_slots) continue;
-        for (int t0 = 0; t0 < n; t0 += kAhead) {
+        const float2 *step = steps + row;
+        const T *value = values + col;
+        for (int t0 = 0; t0 < n; t0 += kAhead, step += kAhead * dec_step, value += kAhead * v_token) {
             float2 x[kAhead];
-            float vj[kAhead];
+            T vj[kAhead][W];
 #pragma unroll
             for (int u = 0; u < kAhead; ++u)
                 if (t0 + u < n) {
-                    x[u] = steps[(size_t)(t0 + u) * heads * dk + row];
-                    vj[u] = col < v_cols ? to_f(values[(size_t)(t0 + u) * v_token + col]) : 1.f;
+                    x[u] = step[u * dec_step];
+#pragma unroll
+                    for (int w = 0; w < W; ++w)
+                        if (col + w < v_cols) vj[u][w] = value[u * v_token + w];
                 }
 #pragma unroll
             for (int u = 0; u < kAhead; ++u)
-                if (t0 + u < n) S = fmaf(x[u].x, S, x[u].y * vj[u]);
+                if (t0 + u < n) {
+#pragma unroll
+                    for (int w = 0; w < W; ++w) S[w] = fmaf(x[u].x, S[w], x[u].y * (col + w < v_cols ? to_f(vj[u][w]) : 1.f));
+                }
         }
-        state[(size_t)slot * slot_stride + (size_t)head * dk * dv + e] = S;
+        float *to = state + (size_t)slot * slot_stride + (size_t)head * dk * dv + e;
+#pragma unroll
+        for (int w = 0; w < W; ++w) to[w] = S[w];
     }
 }
 
-// out[t, h, :] += decayed[t, h, :] S_start for the tokens of segments 1, 2, ..: a product of up to 64 tokens x dk by dk x 64 columns
-// per CTA, in fp32, k ascending.  Thread: 8 tokens x 4 columns.
-constexpr int kLaOutCols = 64, kLaOutK = 32;
+// out[t, h, :] += decayed[t, h, :] S_start for the tokens of segments 1, 2, ..: a product of up to 64 tokens x dk by dk x 128 columns
+// per CTA, in fp32, k ascending.  Thread: 8 tokens x 8 columns (two runs of four).  VEC: rows are whole 16-byte pieces.
+constexpr int kLaOutCols = 128, kLaOutK = 32;
+template <bool VEC>
 __global__ void __launch_bounds__(128)
 decay_output_kernel(const int32_t *__restrict__ seq_info, int heads, int dk, int dv, int max_segments, const float *__restrict__ seg_state,
                     const float *__restrict__ decayed, float *__restrict__ out) {
@@ -324,41 +357,70 @@ decay_output_kernel(const int32_t *__restrict__ seq_info, int heads, int dk, int
     int lo, hi, nseg;
     if (!la_segment(start, count, c, lo, hi, nseg)) return;
     const int first = seq_first + (lo - start), n = hi - lo;
-    const float *S = seg_state + (((size_t)s * max_segments + c) * heads + head) * dk * dv;
+    const float *S = seg_state + (((size_t)s * max_segments + c) * heads + head) * dk * dv + col0;
+    const float *Q = decayed + ((size_t)first * heads + head) * dk;
     __shared__ __align__(16) float sq[kLaOutK][kLaSegment + 4], ss[kLaOutK][kLaOutCols];
     const int tr = threadIdx.x / 16 * 8, tc = threadIdx.x % 16 * 4;
-    float acc[8][4] = {};
+    float acc[8][8] = {};
     for (int k0 = 0; k0 < dk; k0 += kLaOutK) {
-        __syncthreads();
+        float4 q4[4], s4[8];
+        auto piece = [&](const float *p, int left) {  // up to four entries of a row, zeros past its end
+            if (VEC) return left > 0 ? *reinterpret_cast<const float4 *>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+            return make_float4(left > 0 ? p[0] : 0.f, left > 1 ? p[1] : 0.f, left > 2 ? p[2] : 0.f, left > 3 ? p[3] : 0.f);
+        };
 #pragma unroll
-        for (int i = 0; i < kLaSegment * kLaOutK / 128; ++i) {
-            const int e = threadIdx.x + i * 128, t = e / kLaOutK, k = e % kLaOutK;
-            sq[k][t] = t < n && k0 + k < dk ? decayed[((size_t)(first + t) * heads + head) * dk + k0 + k] : 0.f;
+        for (int i = 0; i < 4; ++i) {  // 64 tokens x 8 pieces of k
+            const int e = threadIdx.x + i * 128, t = e / 8, k = k0 + e % 8 * 4;
+            q4[i] = piece(Q + (size_t)t * heads * dk + k, t < n ? dk - k : 0);
         }
 #pragma unroll
-        for (int i = 0; i < kLaOutCols * kLaOutK / 128; ++i) {
-            const int e = threadIdx.x + i * 128, k = e / kLaOutCols, d = e % kLaOutCols;
-            ss[k][d] = k0 + k < dk && col0 + d < dv ? S[(size_t)(k0 + k) * dv + col0 + d] : 0.f;
+        for (int i = 0; i < 8; ++i) {  // 32 k x 32 pieces of columns
+            const int e = threadIdx.x + i * 128, k = k0 + e / 32, d = e % 32 * 4;
+            s4[i] = piece(S + (size_t)k * dv + d, k < dk ? dv - col0 - d : 0);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int e = threadIdx.x + i * 128, t = e / 8, k = e % 8 * 4;
+            sq[k][t] = q4[i].x, sq[k + 1][t] = q4[i].y, sq[k + 2][t] = q4[i].z, sq[k + 3][t] = q4[i].w;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int e = threadIdx.x + i * 128;
+            *reinterpret_cast<float4 *>(&ss[e / 32][e % 32 * 4]) = s4[i];
         }
         __syncthreads();
 #pragma unroll 8
         for (int k = 0; k < kLaOutK; ++k) {
-            const float4 a = *reinterpret_cast<const float4 *>(&sq[k][tr]), b = *reinterpret_cast<const float4 *>(&sq[k][tr + 4]),
-                         x = *reinterpret_cast<const float4 *>(&ss[k][tc]);
-            const float q[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, y[4] = {x.x, x.y, x.z, x.w};
+            float q[8], x[8];
+            *reinterpret_cast<float4 *>(q) = *reinterpret_cast<const float4 *>(&sq[k][tr]);
+            *reinterpret_cast<float4 *>(q + 4) = *reinterpret_cast<const float4 *>(&sq[k][tr + 4]);
+            *reinterpret_cast<float4 *>(x) = *reinterpret_cast<const float4 *>(&ss[k][tc]);
+            *reinterpret_cast<float4 *>(x + 4) = *reinterpret_cast<const float4 *>(&ss[k][tc + 64]);
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(q[i], y[j], acc[i][j]);
+                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(q[i], x[j], acc[i][j]);
         }
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         if (tr + i >= n) break;
-        float *o = out + ((size_t)(first + tr + i) * heads + head) * dv + col0 + tc;
+        float *o = out + ((size_t)(first + tr + i) * heads + head) * dv + col0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (col0 + tc + j < dv) o[j] += acc[i][j];
+        for (int h = 0; h < 2; ++h) {
+            const int d = tc + 64 * h;
+            if (VEC) {
+                if (col0 + d >= dv) continue;
+                float4 y = *reinterpret_cast<const float4 *>(o + d);
+                y.x += acc[i][4 * h], y.y += acc[i][4 * h + 1], y.z += acc[i][4 * h + 2], y.w += acc[i][4 * h + 3];
+                *reinterpret_cast<float4 *>(o + d) = y;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (col0 + d + j < dv) o[d + j] += acc[i][4 * h + j];
+            }
+        }
     }
 }
 
@@ -474,11 +536,16 @@ int tlb_decay_scan(const void *q, long long q_token, long long q_head, const voi
     }
     TLB_DS(1, max_segments);
     TL_LAUNCH_CHECK("decay_scan (segments)");
-    TLB_DISPATCH(dtype, "decay_scan", decay_combine_kernel<T><<<dim3(num_seqs, heads, ceil_div(dk * dv, 256)), 256, 0, st>>>(
-                                          seq_info, state, slot_stride, num_slots, heads, dk, dv, max_segments, seg_state, seg_decay, last_steps, (const T *)v, v_token,
-                                          v_head, v_cols));
+    const bool vec = dk % 4 == 0 && dv % 4 == 0 && tl::aligned16(workspace) && tl::aligned16(out);
+#define TLB_COMBINE(W)                                                                                                                          \
+    decay_combine_kernel<T, W><<<dim3(num_seqs, heads, ceil_div(dk * dv, 256 * W)), 256, 0, st>>>(seq_info, state, slot_stride, num_slots, heads, dk, dv, max_segments, \
+                                                                                                 seg_state, seg_decay, last_steps, (const T *)v, v_token, v_head, v_cols)
+    TLB_DISPATCH(dtype, "decay_scan", if (vec) TLB_COMBINE(4); else TLB_COMBINE(1));
+#undef TLB_COMBINE
     TL_LAUNCH_CHECK("decay_scan (combine)");
-    decay_output_kernel<<<dim3(num_seqs, heads * ceil_div(dv, kLaOutCols), max_segments - 1), 128, 0, st>>>(seq_info, heads, dk, dv, max_segments, seg_state, decayed, out);
+    const dim3 og(num_seqs, heads * ceil_div(dv, kLaOutCols), max_segments - 1);
+    if (vec) decay_output_kernel<true><<<og, 128, 0, st>>>(seq_info, heads, dk, dv, max_segments, seg_state, decayed, out);
+    else decay_output_kernel<false><<<og, 128, 0, st>>>(seq_info, heads, dk, dv, max_segments, seg_state, decayed, out);
     TL_LAUNCH_CHECK("decay_scan (outputs)");
 #undef TLB_DS
 #undef TLB_DS_K
