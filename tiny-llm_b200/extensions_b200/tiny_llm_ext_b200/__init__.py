@@ -143,10 +143,12 @@ def _contig(op: str, **named: torch.Tensor) -> None:
             raise RuntimeError(f"{op}: {name} must be contiguous")
 
 
+# The current stream's handle without a torch.cuda.Stream object around it (1.5 us a call; a layer makes a dozen).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda device: torch.cuda.current_stream(device).cuda_stream)
+
+
 def _stream_ptr(stream, ref: torch.Tensor) -> int:
-    if stream is None:
-        return torch.cuda.current_stream(ref.device).cuda_stream
-    return stream.cuda_stream
+    return _raw_stream(ref.get_device()) if stream is None else stream.cuda_stream
 
 
 def _check(code: int) -> None:
@@ -193,6 +195,36 @@ def quantized_matmul(
     stream=None,
 ):
     """``a [M,N] @ dequant(b [K,N/8]).T -> [M,K]`` (bindings.cpp:16-33)."""
+    dtype = a.dtype
+    try:  # one pass over the attributes; what does not fit goes through the checks one by one, for their messages
+        (M, N), (K, words) = a.shape, b.shape
+        fits = (
+            dtype in _HALF and scales.dtype is dtype and biases.dtype is dtype and b.dtype in _PACKED and bits == 4 and group_size == 128 and transpose_b
+            and N % 128 == 0 and words * 8 == N and scales.shape == (K, N // 128) and biases.shape == (K, N // 128)
+            and a.is_cuda and b.is_cuda and scales.is_cuda and biases.is_cuda
+            and a.is_contiguous() and b.is_contiguous() and scales.is_contiguous() and biases.is_contiguous()
+        )
+    except ValueError:  # not two dimensions
+        fits = False
+    if not fits:
+        _check_quantized_matmul(scales, biases, group_size, bits, a, b, transpose_b)
+        M, N = a.shape
+        K = b.shape[0]
+    out = a.new_empty((M, K))
+    code = _DTYPE_CODE[dtype]
+    ws_bytes = _lib.tl_quantized_matmul_workspace(M, N, K, code, int(use_simdgroup), int(use_split_k))
+    ws = _zero_workspace(ws_bytes, a.device) if ws_bytes else None
+    _check(
+        _lib.tl_quantized_matmul(
+            scales.data_ptr(), biases.data_ptr(), a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, code,
+            int(use_simdgroup), int(use_split_k), None if ws is None else ws.data_ptr(), ws_bytes,
+            _stream_ptr(stream, a),
+        )
+    )
+    return out
+
+
+def _check_quantized_matmul(scales, biases, group_size, bits, a, b, transpose_b) -> None:
     if scales.dtype not in _HALF:
         raise RuntimeError("quantized_matmul: scales must be float16 or bfloat16")
     if scales.dtype != biases.dtype:
@@ -223,20 +255,6 @@ def quantized_matmul(
         raise RuntimeError("quantized_matmul: a must have the same number of columns as b")
     _gpu("quantized_matmul", scales, biases, a, b)
     _contig("quantized_matmul", a=a, b=b, scales=scales, biases=biases)
-    M, N = a.shape
-    K = b.shape[0]
-    out = torch.empty((M, K), dtype=a.dtype, device=a.device)
-    code = _DTYPE_CODE[a.dtype]
-    ws_bytes = _lib.tl_quantized_matmul_workspace(M, N, K, code, int(use_simdgroup), int(use_split_k))
-    ws = _zero_workspace(ws_bytes, a.device)
-    _check(
-        _lib.tl_quantized_matmul(
-            scales.data_ptr(), biases.data_ptr(), a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, code,
-            int(use_simdgroup), int(use_split_k), None if ws is None else ws.data_ptr(), ws_bytes,
-            _stream_ptr(stream, a),
-        )
-    )
-    return out
 
 
 def quantized_embedding(indices, scales, biases, weight, group_size, bits, stream=None):
@@ -302,8 +320,9 @@ def swiglu(gate, up, stream=None):
         raise RuntimeError("swiglu: expected float32, float16, or bfloat16")
     if gate.dtype != up.dtype or gate.shape != up.shape:
         raise RuntimeError("swiglu: gate and up must have the same shape and dtype")
-    _gpu("swiglu", gate, up)
-    _contig("swiglu", gate=gate, up=up)
+    if not (gate.is_cuda and up.is_cuda and gate.is_contiguous() and up.is_contiguous()):
+        _gpu("swiglu", gate, up)
+        _contig("swiglu", gate=gate, up=up)
     out = torch.empty_like(gate)
     _check(_lib.tl_swiglu(gate.data_ptr(), up.data_ptr(), out.data_ptr(), gate.numel(), _DTYPE_CODE[gate.dtype], _stream_ptr(stream, gate)))
     return out

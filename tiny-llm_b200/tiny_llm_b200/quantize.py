@@ -135,23 +135,14 @@ def quantized_matmul_vanilla(
 def quantized_linear(x: torch.Tensor, w: QuantizedWeights, bias: torch.Tensor | None = None) -> torch.Tensor:
     """quantize.py:49-90 - <= 8 rows go to the matvec kernel when the weights
     allow it, everything else to ``quantized_matmul`` with the weight's flags."""
-    n_rows = 1
-    for extent in x.shape[:-1]:
-        n_rows *= extent
-    if n_rows <= 8 and w.use_simdgroup_matvec:
-        y = quantized_matvec_custom(w.scales, w.biases, w.group_size, w.bits, x, w.weight, True)
-    else:
-        y = quantized_matmul(
-            w.scales,
-            w.biases,
-            w.group_size,
-            w.bits,
-            x,
-            w.weight,
-            True,
-            use_simdgroup=w.use_simdgroup_matmul,
-            use_split_k=w.use_split_k_matmul,
-        )
+    lead = x.shape[:-1]
+    rows = x.reshape(-1, x.shape[-1])
+    if not rows.is_contiguous():
+        rows = rows.contiguous()
+    few = rows.shape[0] <= 8 and w.use_simdgroup_matvec
+    # at most 8 rows rely on the extension's default use_simdgroup=True to reach the weight-streaming kernel (quantized_matvec_custom)
+    y = tiny_llm_ext_b200.quantized_matmul(w.scales.contiguous(), w.biases.contiguous(), w.group_size, w.bits, rows, w.weight.contiguous(), True,
+                                           *(() if few else (w.use_simdgroup_matmul, w.use_split_k_matmul))).reshape(*lead, -1)
     return y if bias is None else y + bias
 
 
