@@ -231,28 +231,44 @@ __global__ void norm_mix2_kernel(const float *__restrict__ a, const T *__restric
         y[base + d] = coef * (a[base + d] * ia * to_f(wa[d]) + b[base + d] * ib * to_f(wb[d]));
 }
 
+// In place: pairs (u, v) of a row's heads turned by the position's angles.  A pair's angle is evaluated once per row, in double, and
+// shared by the heads (kRopePairs at a time); the threads then take (head, pair) side by side.
+constexpr int kRopePairs = 64;
+template <typename T>
+__device__ __forceinline__ void rope_heads(T *row, long long head_stride, int heads, int dims, int interleaved, double log2_base, double inv_factor, int pos,
+                                           float2 *angles /* shared [kRopePairs] */) {
+    const int half = dims / 2;
+    for (int i0 = 0; i0 < half; i0 += kRopePairs) {
+        const int n = min(kRopePairs, half - i0);
+        __syncthreads();
+        for (int j = threadIdx.x; j < n; j += blockDim.x) {
+            float c, s;
+            if (inv_factor == 1.0) rope_angle(pos, i0 + j, dims, log2_base, c, s);
+            else {  // linear scaling: every frequency divided by the factor
+                double sn, cs;
+                sincos((double)pos * exp2(-2.0 * (double)(i0 + j) / (double)dims * log2_base) * inv_factor, &sn, &cs);
+                c = (float)cs, s = (float)sn;
+            }
+            angles[j] = make_float2(c, s);
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < heads * n; e += blockDim.x) {
+            const int hd = e / n, j = e - hd * n, i = i0 + j;
+            const float c = angles[j].x, s = angles[j].y;
+            T *p = row + (size_t)hd * head_stride;
+            T *pa = p + (interleaved ? 2 * i : i), *pb = p + (interleaved ? 2 * i + 1 : i + half);
+            const float u = to_f(*pa), v = to_f(*pb);
+            *pa = from_f<T>(u * c - v * s);
+            *pb = from_f<T>(v * c + u * s);
+        }
+    }
+}
+
 template <typename T>
 __global__ void rope_rows_kernel(T *x, long long row_stride, long long head_stride, int first, int heads, int dims, int interleaved,
                                  double log2_base, double inv_factor, const int32_t *__restrict__ tok_pos) {
-    int row = blockIdx.x;
-    int pos = tok_pos[row];
-    int half = dims / 2;
-    for (int i = threadIdx.x; i < half; i += blockDim.x) {
-        float c, s;
-        if (inv_factor == 1.0) rope_angle(pos, i, dims, log2_base, c, s);
-        else {  // linear scaling: every frequency divided by the factor
-            double sn, cs;
-            sincos((double)pos * exp2(-2.0 * (double)i / (double)dims * log2_base) * inv_factor, &sn, &cs);
-            c = (float)cs, s = (float)sn;
-        }
-        int a = interleaved ? 2 * i : i, b = interleaved ? 2 * i + 1 : i + half;
-        for (int hd = 0; hd < heads; ++hd) {
-            T *p = x + (size_t)row * row_stride + (size_t)hd * head_stride + first;
-            float u = to_f(p[a]), v = to_f(p[b]);
-            p[a] = from_f<T>(u * c - v * s);
-            p[b] = from_f<T>(v * c + u * s);
-        }
-    }
+    __shared__ float2 angles[kRopePairs];
+    rope_heads(x + (size_t)blockIdx.x * row_stride + first, head_stride, heads, dims, interleaved, log2_base, inv_factor, tok_pos[blockIdx.x], angles);
 }
 
 template <typename T>
@@ -265,19 +281,10 @@ __global__ void latent_append_kernel(const T *__restrict__ down, const T *__rest
     int pos = tok_pos[t];
     int width = rank + rot;
     const T *src = down + (size_t)t * down_stride;
-    if (q != nullptr) {  // the same launch rotates the token's query heads in place (same angles as the shared key part)
-        int half = rot_dims / 2;
-        for (int i = threadIdx.x; i < half * q_heads; i += blockDim.x) {
-            int hd = i / half, k = i - hd * half;
-            float c, s;
-            rope_angle(pos, k, rot_dims, log2_base, c, s);
-            int a = interleaved ? 2 * k : k, b = interleaved ? 2 * k + 1 : k + half;
-            T *p = q + (size_t)t * q_stride + (size_t)hd * q_head_stride + q_first;
-            float u = to_f(p[a]), v = to_f(p[b]);
-            p[a] = from_f<T>(u * c - v * s);
-            p[b] = from_f<T>(v * c + u * s);
-        }
-    }
+    __shared__ float2 angles[kRopePairs];
+    // the same launch rotates the token's query heads in place (same angles as the shared key part; every head evaluating them for
+    // itself took most of the launch: 2048 tokens of 16 heads, 32 pairs, 19.7 -> 13.1 us)
+    if (q != nullptr) rope_heads(q + (size_t)t * q_stride + q_first, (long long)q_head_stride, q_heads, rot_dims, interleaved, log2_base, 1.0, pos, angles);
     int page = block_table[(size_t)tok_seq[t] * max_pages + pos / page_size];
     bool ok = page >= 0 && page < num_pages;  // a bad table entry drops the write instead of corrupting another page
     T *dst = slab + ((size_t)(ok ? page : 0) * page_size + pos % page_size) * width;
@@ -293,7 +300,8 @@ __global__ void latent_append_kernel(const T *__restrict__ down, const T *__rest
     int half = rot_dims / 2;
     for (int i = threadIdx.x; i < half; i += blockDim.x) {
         float c, s;
-        rope_angle(pos, i, rot_dims, log2_base, c, s);
+        if (q != nullptr && half <= kRopePairs) c = angles[i].x, s = angles[i].y;  // still there from the queries
+        else rope_angle(pos, i, rot_dims, log2_base, c, s);
         int a = interleaved ? 2 * i : i, b = interleaved ? 2 * i + 1 : i + half;
         float u = to_f(src[rank + a]), v = to_f(src[rank + b]);
         dst[rank + a] = from_f<T>(u * c - v * s);
@@ -479,7 +487,7 @@ int tlb_rope_rows(void *x, long long row_stride, long long head_stride, int firs
     if (!x || !tok_pos || heads <= 0 || (dims & 1) || base <= 0 || !(factor > 0)) return tl::fail(TL_EINVAL, "rope_rows: bad argument");
     double lb = log2(base);
     TLB_DISPATCH(dtype, "rope_rows",
-                 rope_rows_kernel<T><<<rows, 64, 0, as_stream(stream)>>>((T *)x, row_stride, head_stride, first, heads, dims, interleaved, lb, 1.0 / factor, tok_pos));
+                 rope_rows_kernel<T><<<rows, 128, 0, as_stream(stream)>>>((T *)x, row_stride, head_stride, first, heads, dims, interleaved, lb, 1.0 / factor, tok_pos));
     TL_LAUNCH_CHECK("rope_rows");
     return TL_OK;
 }
