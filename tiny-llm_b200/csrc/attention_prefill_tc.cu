@@ -32,6 +32,7 @@
 #include <stdlib.h>
 #include <math_constants.h>
 
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 
@@ -86,7 +87,7 @@ __device__ __forceinline__ float tc_ex2(float x) {
 struct TcArgs {
     const int32_t *block_table, *context_lens;
     bf16 *out;
-    int L, Hq, Hkv, G, RH;       // RH = query positions per CTA = 128 / G
+    int L, Hq, Hkv, G, RH;       // RH = query positions per CTA: 128 / G, or L where that is fewer
     int page_size, max_pages, num_pages;
     int tiles_per_page;          // page_size / 64
     float scale_log2;
@@ -125,6 +126,10 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     const int tps = a.splits > 1 ? max((all_tiles + a.splits - 1) / a.splits, 1) : a.tiles_per_split;
     const int t0 = min(split * tps, all_tiles);
     const int n_tiles = min(tps, all_tiles - t0);  // this CTA: global tiles t0 .. t0 + n_tiles - 1
+    // MMA rows in use: row = head of the group x RH + position.  A few new tokens have few rows, side by side in the first warps (one for
+    // 4 heads x 1 token): the other softmax warps have nothing to do and leave the issue slots to those of the SM's other CTA.  With the
+    // rows 128 / G apart all four warps went through every tile for one live lane each: 32 requests of 7200 tokens, 8 x 4 heads, 155 -> 140 us.
+    const int rows = a.RH * a.G;
 
     const uint32_t q_base = g_smem_u32(tsm + TC_Q_OFF), p_base = g_smem_u32(tsm + TC_P_OFF);
     const uint32_t k_base = g_smem_u32(tsm + TC_K_OFF), v_base = g_smem_u32(tsm + TC_V_OFF);
@@ -142,7 +147,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         g_mbar_init(q_full, 1);
         g_mbar_init(s_full, 1);
         g_mbar_init(s_full + 8, 1);
-        g_mbar_init(p_full, TC_SOFTMAX_THREADS / 32);  // one arrival per softmax warp
+        g_mbar_init(p_full, (rows + 31) / 32);  // one arrival per softmax warp that has rows
         g_mbar_init(pv_done, 1);
         for (int i = 0; i < TC_STAGES; ++i) {
             g_mbar_init(k_full + 8 * i, 1);
@@ -169,7 +174,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         if (n_tiles > 0) {  // whole warp, one elected lane issues (see the MMA warp)
             const int head0 = b * a.Hq + kvh * a.G;
             if (g_elect_one()) {
-                g_mbar_expect_tx(q_full, TC_Q_BYTES);
+                g_mbar_expect_tx(q_full, rows * TC_D * 2);
                 g_tma_load_3d(q_base, &tmap_q, 0, q0, head0, q_full);
                 g_tma_load_3d(q_base + TC_Q_BYTES / 2, &tmap_q, 64, q0, head0, q_full);
             }
@@ -257,12 +262,13 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
                 if (++vs == TC_STAGES) vs = 0, vph ^= 1u;
             }
         }
-    } else {
+    } else if (warp * 32 < rows) {
         // ------------------------------------------------------------ softmax warps (thread = row = TMEM lane)
         const int r = threadIdx.x;                 // 0..127
         const int g = r / a.RH, lq = r - g * a.RH;  // query head of the KV group, position inside the block
         const int l = q0 + lq;
-        const bool row_valid = l < a.L && ctx > 0;
+        const bool stored = r < rows && l < a.L;
+        const bool row_valid = stored && ctx > 0;
         // last key this row may see (bottom-right causal alignment, paged_attention.metal:411)
         const int limit = !row_valid ? -1 : (a.is_causal ? min(ctx - 1, l + (ctx - a.L)) : ctx - 1);
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
@@ -372,13 +378,13 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
 #pragma unroll
                     for (int c = 0; c < 32; ++c) ov[c] = 0u;
                 }
-                if (l < a.L) {
+                if (stored) {
 #pragma unroll
                     for (int c = 0; c < 32; c += 4)
                         *reinterpret_cast<uint4 *>(po + cb * 32 + c) = make_uint4(ov[c], ov[c + 1], ov[c + 2], ov[c + 3]);
                 }
             }
-            if (l < a.L) {
+            if (stored) {
                 a.ws_m[slot] = (m_used == -CUDART_INF_F || !row_valid) ? -1e30f : m_used;
                 a.ws_l[slot] = row_valid ? l_sum : 0.f;
             }
@@ -394,7 +400,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
 #pragma unroll
                 for (int c = 0; c < 32; ++c) ov[c] = 0u;
             }
-            if (l < a.L) {
+            if (stored) {
 #pragma unroll
                 for (int c = 0; c < 32; c += 8) {
                     uint4 o;
@@ -481,7 +487,7 @@ int launch_paged_prefill_tc(const void *q, const void *kp, const void *vp, const
     const int B = rows / num_heads;
     TcArgs a{};
     a.block_table = bt, a.context_lens = cl, a.out = static_cast<bf16 *>(out);
-    a.L = L, a.Hq = num_heads, a.Hkv = num_kv_heads, a.G = G, a.RH = TC_BM / G;
+    a.L = L, a.Hq = num_heads, a.Hkv = num_kv_heads, a.G = G, a.RH = std::min(TC_BM / G, L);
     a.page_size = page_size, a.max_pages = max_pages, a.num_pages = num_pages;
     a.tiles_per_page = page_size / TC_BN;
     a.scale_log2 = scale * TC_LOG2E;
