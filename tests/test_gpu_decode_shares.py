@@ -1,0 +1,71 @@
+"""Attention of a few new tokens, its key tiles dealt out over all requests and heads, against float64: requests of very different
+lengths, idle slots, shares that end inside a head and at its end, more pieces than eight, one to eight tokens, one to 128 query rows,
+a bad table entry, and a captured launch whose lengths change."""
+
+import pytest
+import torch
+
+from extensions_b200 import tiny_llm_ext_b200 as ext
+
+pytestmark = pytest.mark.gpu
+PAGE = 128
+
+
+def inputs(lens, heads, kv, L, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    pages = [-(-max(n, 1) // PAGE) for n in lens]
+    table = torch.full((len(lens), max(max(pages), 8) + 1), -1, dtype=torch.int32)
+    order, at = torch.randperm(sum(pages), generator=torch.Generator().manual_seed(seed)).int(), 0
+    for b, n in enumerate(pages):
+        table[b, :n], at = order[at : at + n], at + n
+    q = torch.randn(len(lens) * heads, L, 128, generator=g, device="cuda").bfloat16()
+    k, v = (torch.randn(sum(pages), kv, PAGE, 128, generator=g, device="cuda").bfloat16() for _ in range(2))
+    return q, k, v, table.cuda(), torch.tensor(lens, dtype=torch.int32, device="cuda")
+
+
+def check(got, q, k, v, table, lens, heads, kv, L, causal):
+    group = heads // kv
+    for b, n in enumerate(lens.tolist()):
+        out = got[b * heads : (b + 1) * heads].double()
+        if n <= 0:
+            assert torch.count_nonzero(out) == 0
+            continue
+        ids = table[b, : -(-n // PAGE)].long()
+        ok = ((ids >= 0) & (ids < k.shape[0])).repeat_interleave(PAGE)[:n]
+        keys, values = (t[ids.clamp(0, k.shape[0] - 1)].transpose(1, 2).reshape(-1, kv, 128)[:n].double().repeat_interleave(group, 1) for t in (k, v))
+        s = torch.einsum("hld,nhd->hln", q[b * heads : (b + 1) * heads].double(), keys) * 128**-0.5
+        limit = torch.arange(L, device="cuda")[:, None] + (n - L) if causal else torch.full((L, 1), n - 1, device="cuda")
+        see = (torch.arange(n, device="cuda")[None] <= limit) & ok[None]
+        p = torch.nan_to_num(torch.softmax(s.masked_fill(~see, -torch.inf), -1))
+        want, size = torch.einsum("hln,nhd->hld", p, values), torch.einsum("hln,nhd->hld", p, values.abs())
+        # the weights and the result are rounded to 8 bits (half a unit each), the rest is 32-bit sums and a 2^-22 exponential
+        assert bool(((out - want).abs() <= 2.0**-8 * (size + want.abs()) + 1e-6).all()), (b, float((out - want).abs().max()))
+
+
+CASES = [
+    # lengths, heads, kv heads, new tokens
+    ([5000] + [70] * 31, 32, 8, 1), ([200 + 331 * i % 2900 for i in range(20)], 8, 2, 1), ([64, 0, 128, 192, 0, 0, 257, 1500], 16, 4, 1), ([4096] * 8, 32, 8, 1),
+    ([9000], 2, 1, 1), ([12000], 32, 8, 1), ([0, 0, 1100], 8, 8, 1), ([1030, 3, 700], 16, 2, 4), ([8, 1031, 512, 2000], 32, 8, 8), ([1500, 40], 16, 1, 8),
+    ([1200] * 40, 64, 8, 2), ([100] * 300, 4, 2, 1), ([2, 1500], 4, 4, 5), ([0] * 5 + [1025], 32, 8, 3),
+]
+
+
+@pytest.mark.parametrize("lens,heads,kv,L", CASES)
+@pytest.mark.parametrize("causal", [True, False])
+def test_against_float64(lens, heads, kv, L, causal):
+    q, k, v, table, n = inputs(lens, heads, kv, L)
+    check(ext.paged_attention(q, k, v, table, n, scale=128**-0.5, is_causal=causal, num_heads=heads, num_kv_heads=kv), q, k, v, table, n, heads, kv, L, causal)
+
+
+def test_bad_entries_and_lengths_that_change_under_a_captured_launch():
+    q, k, v, table, n = inputs([3000, 1500, 2200, 90], 16, 4, 1)
+    table[0, 3], table[2, 0], table[1, 5] = 10_000, -7, k.shape[0]
+    call = lambda: ext.paged_attention(q, k, v, table, n, scale=128**-0.5, is_causal=True, num_heads=16, num_kv_heads=4)
+    check(call(), q, k, v, table, n, 16, 4, 1, True)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        held = call()
+    for lens in ([3000, 1500, 2200, 90], [1, 1500, 0, 64], [0, 0, 0, 0], [65, 64, 63, 1]):
+        n.copy_(torch.tensor(lens))
+        graph.replay()
+        check(held, q, k, v, table, n, 16, 4, 1, True)

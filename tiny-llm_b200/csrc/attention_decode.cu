@@ -470,13 +470,6 @@ __global__ void __launch_bounds__(GQA_THREADS) paged_gqa_merge_kernel(const floa
     out[qi * GQA_D + d] = __float2bfloat16_rn(gl == 0.f ? 0.f : o / gl);
 }
 
-int launch_paged_gqa_merge(const float *ws_o, const float *ws_m, const float *ws_l, void *out, int rows_total, int splits, cudaStream_t st) {
-    launch_chained(paged_gqa_merge_kernel, dim3(static_cast<unsigned>(rows_total)), dim3(GQA_THREADS), 0, st, ws_o, ws_m, ws_l,
-                   static_cast<__nv_bfloat16 *>(out), splits);
-    TL_LAUNCH_CHECK("paged_gqa_merge");
-    return TL_OK;
-}
-
 size_t paged_decode_workspace(int rows, int L, int D, int num_kv_heads, int num_heads, int dtype) {
     if (dtype != TL_BF16 || D != GQA_D) return 0;
     return static_cast<size_t>(rows) * L * GQA_MAX_SPLITS * (GQA_D + 2) * sizeof(float);
@@ -565,8 +558,8 @@ int launch_paged_decode(const void *q, const void *kp, const void *vp, const int
     if (fast && tc_mode != 0 && aligned16(out) && rows % num_heads == 0 && group > 0 && L <= 128 / group &&
         paged_prefill_tc_supported(L, num_pages, page_size, num_kv_heads, num_heads) &&
         (tc_mode == 1 || static_cast<long long>(max_pages) * page_size >= tc_min_keys))
-        return launch_paged_prefill_tc(q, kp, vp, bt, cl, out, rows, L, num_pages, page_size, max_pages, scale, is_causal, num_kv_heads,
-                                       num_heads, true, ws, ws_bytes, st);
+        return launch_paged_decode_tc(q, kp, vp, bt, cl, out, rows, L, num_pages, page_size, max_pages, scale, is_causal, num_kv_heads,
+                                      num_heads, ws, ws_bytes, st);
     if (fast)
         return launch_paged_gqa(q, kp, vp, bt, cl, out, rows, L, num_pages, page_size, max_pages, scale, is_causal,
                                 num_kv_heads, num_heads, true, ws, ws_bytes, st);
@@ -585,7 +578,7 @@ int launch_paged_prefill(const void *q, const void *kp, const void *vp, const in
     static const bool fa_off = [] { const char *e = getenv("TL_PREFILL_FA"); return e != nullptr && e[0] == '0'; }();
     if (fast && !fa_off && aligned16(out) && rows % num_heads == 0 && paged_prefill_tc_supported(L, num_pages, page_size, num_kv_heads, num_heads))
         return launch_paged_prefill_tc(q, kp, vp, bt, cl, out, rows, L, num_pages, page_size, max_pages, scale, is_causal, num_kv_heads,
-                                       num_heads, false, nullptr, 0, st);
+                                       num_heads, st);
     if (fast && !fa_off && rows <= 65535)  // tensor-core flash kernel (attention_prefill.cu); TL_PREFILL_FA=0: CUDA-core control
         return launch_paged_prefill_fa(q, kp, vp, bt, cl, out, rows, L, num_pages, page_size, max_pages, scale, is_causal, num_kv_heads,
                                        num_heads, st);

@@ -1,5 +1,5 @@
 // Paged causal FlashAttention prefill on the 5th-generation tensor cores (tcgen05 + TMEM + TMA),
-// bf16, head_dim 128, L > 8.
+// bf16, head_dim 128, L > 8; and the same arithmetic for a few new tokens (L <= 8) further down.
 //
 // Replaces paged_attention_mma_bf16_d128 (/root/reference/src/extensions_ref/src/
 // paged_attention.metal:250-506): same arithmetic - fp32 scores in base 2 (:414 scale_log2),
@@ -92,11 +92,7 @@ struct TcArgs {
     int tiles_per_page;          // page_size / 64
     float scale_log2;
     int is_causal;
-    // split-KV (decode, L <= 8): CTA (query block, split) covers key tiles [split * tiles_per_split, ...) and
-    // leaves an unnormalised partial (O fp32, running max in log2 units, sum) for paged_gqa_merge_kernel
-    int splits, tiles_per_split;
-    int out_token_major;  // unsplit launches only: out[(b, l, head), :] instead of [(b, head, l), :] (the layout the o-projection takes)
-    float *ws_o, *ws_m, *ws_l;
+    int out_token_major;  // out[(b, l, head), :] instead of [(b, head, l), :] (the layout the o-projection takes)
 };
 
 // PT: the probabilities of a tile stay in TENSOR memory - P_j (bf16 pairs, 32 columns) overwrites the first half of the
@@ -111,24 +107,15 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     extern __shared__ __align__(1024) unsigned char tsm[];
     griddep_launch();  // programmatic dependent launch (common.cuh): the successor may set itself up under this grid
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int split = static_cast<int>(blockIdx.x) % a.splits;
-    const int qb = static_cast<int>(gridDim.x) / a.splits - 1 - static_cast<int>(blockIdx.x) / a.splits;  // long (late) query blocks first
+    const int qb = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);  // long (late) query blocks first
     const int kvh = blockIdx.y, b = blockIdx.z;
     const int q0 = qb * a.RH;
     const int ctx = min(a.context_lens[b], a.max_pages * a.page_size);
     // keys any row of this CTA may see: [0, key_end)
     const int last_row = min(q0 + a.RH, a.L) - 1;
     const int key_end = ctx <= 0 ? 0 : (a.is_causal ? min(ctx, max(ctx - a.L + last_row + 1, 0)) : ctx);
-    const int all_tiles = (key_end + TC_BN - 1) / TC_BN;
-    // Split-KV: the launch fixes the NUMBER of splits from the block table's width (the grid of a captured graph cannot
-    // follow the context), the tiles are dealt out here from the request's real length, so a request far below the
-    // bound still keeps all its splits busy.
-    const int tps = a.splits > 1 ? max((all_tiles + a.splits - 1) / a.splits, 1) : a.tiles_per_split;
-    const int t0 = min(split * tps, all_tiles);
-    const int n_tiles = min(tps, all_tiles - t0);  // this CTA: global tiles t0 .. t0 + n_tiles - 1
-    // MMA rows in use: row = head of the group x RH + position.  A few new tokens have few rows, side by side in the first warps (one for
-    // 4 heads x 1 token): the other softmax warps have nothing to do and leave the issue slots to those of the SM's other CTA.  With the
-    // rows 128 / G apart all four warps went through every tile for one live lane each: 32 requests of 7200 tokens, 8 x 4 heads, 155 -> 140 us.
+    const int n_tiles = (key_end + TC_BN - 1) / TC_BN;
+    // MMA rows in use: row = head of the group x RH + position (side by side: warps without rows leave at once)
     const int rows = a.RH * a.G;
 
     const uint32_t q_base = g_smem_u32(tsm + TC_Q_OFF), p_base = g_smem_u32(tsm + TC_P_OFF);
@@ -183,10 +170,10 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             int s = 0;
             uint32_t ph = 1;  // producer side: first pass through the ring does not wait
             for (int j = 0; j < n_tiles; ++j) {
-                const int lp = (t0 + j) / a.tiles_per_page;
+                const int lp = j / a.tiles_per_page;
                 int pid = table[lp];
                 if (pid < 0 || pid >= a.num_pages) pid = a.num_pages;  // outside the tensor: the TMA unit writes zeros
-                const int slot0 = (t0 + j - lp * a.tiles_per_page) * TC_BN;
+                const int slot0 = (j - lp * a.tiles_per_page) * TC_BN;
                 g_mbar_wait(k_empty + 8 * s, ph);
                 if (g_elect_one()) {
                     g_mbar_expect_tx(k_full + 8 * s, TC_KV_TILE);
@@ -275,7 +262,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         float m_used = -CUDART_INF_F, l_sum = 0.f;
         const int32_t *table = a.block_table + static_cast<size_t>(b) * a.max_pages;
         for (int j = 0; j < n_tiles; ++j) {
-            const int lp = (t0 + j) / a.tiles_per_page;
+            const int lp = j / a.tiles_per_page;
             const int pid = table[lp];
             const bool page_ok = pid >= 0 && pid < a.num_pages;
             g_mbar_wait(s_full + 8 * (j & 1), (j >> 1) & 1);
@@ -284,7 +271,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             g_tmem_ld32_nowait(tmem + lane_base + (j & 1) * TC_BN, sv[0]);
             g_tmem_ld32_nowait(tmem + lane_base + (j & 1) * TC_BN + 32, sv[1]);
             g_tmem_ld_wait();
-            const int key0 = (t0 + j) * TC_BN;
+            const int key0 = j * TC_BN;
             const int visible = page_ok ? min(limit - key0 + 1, TC_BN) : 0;  // keys [0, visible) of the tile
             // raw maximum (the scale is positive, so it commutes with max); masking only on boundary tiles
             float raw_max = -CUDART_INF_F;
@@ -366,29 +353,6 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             g_tc_fence_after();
         }
         const size_t out_row = static_cast<size_t>(b * a.Hq + kvh * a.G + g) * a.L + l;
-        if (a.splits > 1) {  // unnormalised partial for the merge kernel (attention_decode.cu: paged_gqa_merge_kernel)
-            const size_t slot = out_row * a.splits + split;
-            float *po = a.ws_o + slot * TC_D;
-#pragma unroll
-            for (int cb = 0; cb < TC_D / 32; ++cb) {
-                uint32_t ov[32];
-                if (n_tiles > 0) {  // warp-uniform: tcgen05.ld is warp-collective, rows beyond L take part too
-                    g_tmem_ld32(tmem + lane_base + TC_TMEM_O + cb * 32, ov);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 32; ++c) ov[c] = 0u;
-                }
-                if (stored) {
-#pragma unroll
-                    for (int c = 0; c < 32; c += 4)
-                        *reinterpret_cast<uint4 *>(po + cb * 32 + c) = make_uint4(ov[c], ov[c + 1], ov[c + 2], ov[c + 3]);
-                }
-            }
-            if (stored) {
-                a.ws_m[slot] = (m_used == -CUDART_INF_F || !row_valid) ? -1e30f : m_used;
-                a.ws_l[slot] = row_valid ? l_sum : 0.f;
-            }
-        } else {
         const float inv = (l_sum == 0.f || !row_valid) ? 0.f : 1.0f / l_sum;
         bf16 *dst = a.out + (a.out_token_major ? (static_cast<size_t>(b) * a.L + l) * a.Hq + (kvh * a.G + g) : out_row) * TC_D;
 #pragma unroll
@@ -412,7 +376,6 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
                 }
             }
         }
-        }
     }
     g_tc_fence_before();
     __syncthreads();
@@ -420,6 +383,418 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         g_tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TC_TMEM_COLS) : "memory");
     }
+}
+
+// ---------------------------------------------------------------- a few new tokens --
+// Decode (G heads x L tokens of a key/value head in at most 128 rows): the launch is as many CTAs as the GPU holds at a time, and
+// the key tiles of ALL requests and key/value heads, one after another, are dealt to them in equal shares.  A share may end in the
+// middle of a (request, head) and go on with the next; a (request, head) in one share is finished there, one in several leaves a
+// partial result per share for decode_merge_tc_kernel.  What is dealt out are the requests' real lengths, read on the device, so a
+// captured launch follows them.  (Before, every (request, head) had its own CTAs, as many for all as suited a full block table: requests
+// of very different lengths waited for the longest, which alone on its SM takes 1.3 us a tile, and more than one wave of CTAs
+// waited for a last, emptier one.  One new token, 32 heads over 8: 32 requests of 200 to 7200 tokens 124 -> 72 us, 64 of 100 to 4100
+// 123 -> 96, 8 of 300 to 7300 39 -> 28, one of 8000 beside 31 of 200 134 -> 18.)
+// The query rows sit side by side (row = head of the group x L + token), so that only the softmax warps that have rows
+// run; up to 32 rows there is one, and room for two query stages and a third key and value stage.
+struct DecodeTcArgs {
+    const int32_t *block_table, *context_lens;
+    bf16 *out;
+    int L, Hq, Hkv, G, requests;
+    int page_size, max_pages, num_pages, tiles_per_page;
+    float scale_log2;
+    int is_causal;
+    int ctas, max_pieces;  // of the attention launch; pieces of a (request, head) that the workspace has room for (>= 2)
+    float *ws_o, *ws_m, *ws_l;
+};
+constexpr int DC_MIN_TILES = 4;  // of a share: below it a CTA's fixed cost (set-up, queries, first tile: 3 to 4 us) outweighs what it saves
+
+__device__ __forceinline__ int dc_context(const DecodeTcArgs &a, int r) { return min(max(a.context_lens[r], 0), a.max_pages * a.page_size); }
+__device__ __forceinline__ int dc_tiles(const DecodeTcArgs &a, int r) { return (dc_context(a, r) + TC_BN - 1) / TC_BN; }
+
+// The tiles of all heads of all requests, those before `request` and the tiles of a share; called by whole warps.  Where every
+// (request, head) can have a CTA and the longest is within a quarter of an equal share, per is 0 and each keeps to its own: the launch is
+// bound by HBM then, and cutting only adds partial results (32 requests of 2000 tokens, 8 heads: 49 us cut, 45 whole; of 7200: 151 and 143).
+struct DecodeDeal {
+    int total, before, per;
+};
+__device__ __forceinline__ DecodeDeal dc_deal(const DecodeTcArgs &a, int request) {
+    int total = 0, before = 0, longest = 0;
+    for (int r = threadIdx.x & 31; r < a.requests; r += 32) {
+        const int n = dc_tiles(a, r);
+        total += n, longest = max(longest, n);
+        if (r < request) before += n;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        total += __shfl_xor_sync(0xffffffffu, total, o);
+        before += __shfl_xor_sync(0xffffffffu, before, o);
+        longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+    }
+    total *= a.Hkv, before *= a.Hkv;
+    // n tiles touch at most ceil(n / per) + 1 shares
+    if (a.requests * a.Hkv <= a.ctas && static_cast<long long>(longest) * 4 * a.ctas <= 5LL * total) return {total, before, 0};
+    const int per = max(max((total + a.ctas - 1) / a.ctas, (longest + a.max_pieces - 2) / (a.max_pieces - 1)), DC_MIN_TILES);
+    return {total, before, per};
+}
+
+// A share's walk over the (request, key/value head) pairs it touches.  Every role of the CTA walks it by itself.
+struct DecodeWalk {
+    int pos, end;       // of the share, in tiles over all requests and heads
+    int b, tiles, base; // the request, its tiles a head, where its tiles begin
+    int kvh, t0, n;     // this stretch: the head, its first tile and how many
+    __device__ __forceinline__ void stretch() {
+        const int off = pos - base;
+        kvh = off / tiles, t0 = off - kvh * tiles, n = min(tiles - t0, end - pos);
+    }
+    __device__ __forceinline__ void start(const DecodeTcArgs &a, int begin, int stop) {  // whole warps; begin < stop <= total
+        pos = begin, end = stop;
+        const int lane = threadIdx.x & 31;
+        int run = 0;
+        for (int r0 = 0; r0 < a.requests; r0 += 32) {
+            const int mine = r0 + lane < a.requests ? dc_tiles(a, r0 + lane) : 0;
+            int upto = mine * a.Hkv;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += below;
+            }
+            const unsigned past = __ballot_sync(0xffffffffu, pos < run + upto);
+            if (past) {
+                const int src = __ffs(past) - 1;
+                b = r0 + src, tiles = __shfl_sync(0xffffffffu, mine, src), base = run + __shfl_sync(0xffffffffu, upto, src) - tiles * a.Hkv;
+                break;
+            }
+            run += __shfl_sync(0xffffffffu, upto, 31);
+        }
+        stretch();
+    }
+    __device__ __forceinline__ void own(int request, int head, int all) {
+        pos = 0, end = all, b = request, tiles = all, base = 0, kvh = head, t0 = 0, n = all;
+    }
+    __device__ __forceinline__ bool next(const DecodeTcArgs &a) {
+        pos += n;
+        if (pos >= end) return false;
+        if (pos == base + tiles * a.Hkv) {
+            base = pos;
+            do tiles = dc_tiles(a, ++b);
+            while (tiles == 0);
+        }
+        stretch();
+        return true;
+    }
+};
+
+// Bounded wait: past the limit the CTA is marked (which ends all its further waits) and its rows come out as NaN.
+__device__ __forceinline__ void dc_wait(uint32_t bar, uint32_t parity, volatile int *dead) {
+    for (uint32_t spins = 0;; ++spins) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done || *dead) return;
+        if (spins > (1u << 22)) {
+            *dead = 1;
+            return;
+        }
+    }
+}
+
+template <int SW>  // softmax warps: rows / 32
+struct DecodeTcShape {
+    static constexpr int q_half = SW * 32 * 128, q_stages = SW == 1 ? 2 : 1, stages = SW == 1 ? 3 : 2;
+    static constexpr int k_off = q_stages * 2 * q_half, v_off = k_off + stages * TC_KV_TILE, bar_off = v_off + stages * TC_KV_TILE;
+    static constexpr int smem = bar_off + 256, threads = 32 * (SW + 2);
+    // the score product reads 128 rows from every query half, whatever they hold
+    static_assert((q_stages * 2 - 1) * q_half + 128 * 128 <= bar_off, "rows past the queries lie in shared memory");
+};
+
+template <int SW>
+__global__ void __launch_bounds__(DecodeTcShape<SW>::threads, 2)
+paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                       const DecodeTcArgs a) {
+    using Z = DecodeTcShape<SW>;
+    extern __shared__ __align__(1024) unsigned char tsm[];
+    griddep_launch();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // context lengths and block tables are step inputs uploaded before the chain
+    const DecodeDeal deal = dc_deal(a, 0);
+    DecodeWalk w;
+    const bool own = deal.per == 0;
+    const int request = own ? blockIdx.x / a.Hkv : 0, alone = own && request < a.requests ? dc_tiles(a, request) : 0;
+    if (own ? alone == 0 : static_cast<long long>(blockIdx.x) * deal.per >= deal.total) {
+        griddep_wait();  // also without work: what follows relies on this launch ending after the one before it
+        return;
+    }
+    if (own) w.own(request, blockIdx.x - request * a.Hkv, alone);
+    else w.start(a, blockIdx.x * deal.per, min((blockIdx.x + 1) * deal.per, deal.total));
+    const int share = w.end - w.pos;
+    const int rows = a.G * a.L;
+
+    const uint32_t q_base = g_smem_u32(tsm), k_base = g_smem_u32(tsm + Z::k_off), v_base = g_smem_u32(tsm + Z::v_off);
+    const uint32_t bar = g_smem_u32(tsm + Z::bar_off);
+    const uint32_t s_full = bar /* two: one per score buffer */, p_full = bar + 16, pv_done = bar + 24, q_full = bar + 32, q_empty = bar + 48;
+    const uint32_t k_full = bar + 64, k_empty = k_full + 24, v_full = k_full + 48, v_empty = k_full + 72;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tsm + Z::bar_off + 64 + 96);
+    volatile int *dead = reinterpret_cast<volatile int *>(tsm + Z::bar_off + 64 + 100);
+
+    if (warp == SW && lane == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_q) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_k) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_v) : "memory");
+    }
+    if (warp == SW + 1 && lane == 0) {
+        *dead = 0;
+        g_mbar_init(s_full, 1);
+        g_mbar_init(s_full + 8, 1);
+        g_mbar_init(p_full, (rows + 31) / 32);  // one arrival per softmax warp that has rows
+        g_mbar_init(pv_done, 1);
+        for (int i = 0; i < Z::q_stages; ++i) g_mbar_init(q_full + 8 * i, 1), g_mbar_init(q_empty + 8 * i, 1);
+        for (int i = 0; i < Z::stages; ++i) {
+            g_mbar_init(k_full + 8 * i, 1), g_mbar_init(k_empty + 8 * i, 1);
+            g_mbar_init(v_full + 8 * i, 1), g_mbar_init(v_empty + 8 * i, 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(g_smem_u32(tmem_slot)), "n"(TC_TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    g_tc_fence_before();
+    __syncthreads();
+    g_tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    // q and the newest K/V rows are the predecessor's output, and this grid overwrites buffers (output, partials) that the
+    // predecessor may still read
+    griddep_wait();
+
+    if (warp == SW) {
+        // ------------------------------------------------------------ TMA producer (whole warp, one elected lane issues)
+        int s = 0, qs = 0;
+        uint32_t ph = 1, qph = 1;  // producer side: the first pass through a ring does not wait
+        do {
+            dc_wait(q_empty + 8 * qs, qph, dead);
+            if (g_elect_one()) {
+                const int head0 = w.b * a.Hq + w.kvh * a.G;
+                const uint32_t q_at = q_base + qs * 2 * Z::q_half;
+                g_mbar_expect_tx(q_full + 8 * qs, rows * TC_D * 2);
+                g_tma_load_3d(q_at, &tmap_q, 0, 0, head0, q_full + 8 * qs);
+                g_tma_load_3d(q_at + Z::q_half, &tmap_q, 64, 0, head0, q_full + 8 * qs);
+            }
+            __syncwarp();
+            if (++qs == Z::q_stages) qs = 0, qph ^= 1u;
+            const int32_t *table = a.block_table + static_cast<size_t>(w.b) * a.max_pages;
+            for (int t = w.t0; t < w.t0 + w.n; ++t) {
+                const int lp = t / a.tiles_per_page, slot0 = (t - lp * a.tiles_per_page) * TC_BN;
+                int pid = table[lp];
+                if (pid < 0 || pid >= a.num_pages) pid = a.num_pages;  // outside the tensor: the TMA unit writes zeros
+                dc_wait(k_empty + 8 * s, ph, dead);
+                if (g_elect_one()) {
+                    g_mbar_expect_tx(k_full + 8 * s, TC_KV_TILE);
+                    g_tma_load_4d(k_base + s * TC_KV_TILE, &tmap_k, 0, slot0, w.kvh, pid, k_full + 8 * s);
+                    g_tma_load_4d(k_base + s * TC_KV_TILE + TC_KV_TILE / 2, &tmap_k, 64, slot0, w.kvh, pid, k_full + 8 * s);
+                }
+                __syncwarp();
+                dc_wait(v_empty + 8 * s, ph, dead);
+                if (g_elect_one()) {
+                    g_mbar_expect_tx(v_full + 8 * s, TC_KV_TILE);
+                    g_tma_load_4d(v_base + s * TC_KV_TILE, &tmap_v, 0, slot0, w.kvh, pid, v_full + 8 * s);
+                    g_tma_load_4d(v_base + s * TC_KV_TILE + TC_KV_TILE / 2, &tmap_v, 64, slot0, w.kvh, pid, v_full + 8 * s);
+                }
+                __syncwarp();
+                if (++s == Z::stages) s = 0, ph ^= 1u;
+            }
+        } while (w.next(a));
+    } else if (warp == SW + 1) {
+        // ------------------------------------------------------------ MMA issuer: scores one tile ahead, across stretches too
+        constexpr uint32_t idesc_s = tc_instr_desc(TC_BN, false), idesc_o = tc_instr_desc(TC_D, true);
+        const uint64_t qdesc0 = g_smem_desc_sw128(q_base, 0, 1024), kdesc0 = g_smem_desc_sw128(k_base, 0, 1024);
+        const uint64_t vdesc0 = g_smem_desc_sw128(v_base, TC_KV_TILE / 2, 1024);
+        DecodeWalk ahead = w;
+        int ks = 0, vs = 0, qs = 0, left = ahead.n, value = 0;  // left: tiles of the stretch whose scores are still to come; value: this stretch's tile
+        uint32_t kph = 0, vph = 0, qph = 0;
+        bool fresh = true, more = true;
+        auto issue_scores = [&](int j) {
+            if (fresh) dc_wait(q_full + 8 * qs, qph, dead);
+            fresh = false;
+            dc_wait(k_full + 8 * ks, kph, dead);
+            g_tc_fence_after();
+            const bool last = --left == 0;
+            if (g_elect_one()) {
+                const uint64_t kd = kdesc0 + static_cast<uint64_t>(ks * (TC_KV_TILE >> 4)), qd = qdesc0 + static_cast<uint64_t>(qs * (2 * Z::q_half >> 4));
+#pragma unroll
+                for (int k = 0; k < TC_D / 16; ++k) {
+                    const uint32_t half = (k >> 2), kk = (k & 3);
+                    g_tc_mma(tmem + (j & 1) * TC_BN, qd + half * (Z::q_half >> 4) + 2 * kk, kd + half * (TC_KV_TILE / 2 >> 4) + 2 * kk, idesc_s, k > 0 ? 1u : 0u);
+                }
+                g_tc_commit(k_empty + 8 * ks);
+                if (last) g_tc_commit(q_empty + 8 * qs);
+                g_tc_commit(s_full + 8 * (j & 1));
+            }
+            __syncwarp();
+            if (++ks == Z::stages) ks = 0, kph ^= 1u;
+            if (last) {
+                if (++qs == Z::q_stages) qs = 0, qph ^= 1u;
+                more = ahead.next(a), left = ahead.n, fresh = true;
+            }
+        };
+        issue_scores(0);
+        for (int j = 0; j < share; ++j) {
+            // score buffer (j+1)&1 was last read for tile j-1, whose P has been waited for below
+            if (more) issue_scores(j + 1);
+            // a new stretch's first product overwrites O: the softmax warps arrive for it after they have read the old one
+            dc_wait(p_full, j & 1, dead);
+            dc_wait(v_full + 8 * vs, vph, dead);
+            g_tc_fence_after();
+            if (g_elect_one()) {
+                const uint64_t vd = vdesc0 + static_cast<uint64_t>(vs * (TC_KV_TILE >> 4));
+#pragma unroll
+                for (int k = 0; k < TC_BN / 16; ++k)  // 16 keys = 8 columns of bf16 pairs per K step
+                    g_tc_mma_ts(tmem + TC_TMEM_O, tmem + (j & 1) * TC_BN + 8 * k, vd + k * (2048 >> 4), idesc_o, (value > 0 || k > 0) ? 1u : 0u);
+                g_tc_commit(v_empty + 8 * vs);
+                g_tc_commit(pv_done);
+            }
+            __syncwarp();
+            if (++vs == Z::stages) vs = 0, vph ^= 1u;
+            if (++value == w.n) value = 0, w.next(a);
+        }
+    } else if (warp * 32 < rows) {
+        // ------------------------------------------------------------ softmax warps (thread = row = TMEM lane)
+        const int r = threadIdx.x, g = r / a.L, l = r - g * a.L;
+        const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
+        int j = 0;  // tile of the share
+        do {
+            const int ctx = dc_context(a, w.b);
+            const int limit = r >= rows ? -1 : (a.is_causal ? min(ctx - 1, l + (ctx - a.L)) : ctx - 1);  // the last key this row may see
+            const int32_t *table = a.block_table + static_cast<size_t>(w.b) * a.max_pages;
+            float m_used = -CUDART_INF_F, l_sum = 0.f;
+            for (int i = 0; i < w.n; ++i, ++j) {
+                const int pid = table[(w.t0 + i) / a.tiles_per_page];
+                const int visible = pid >= 0 && pid < a.num_pages ? min(limit - (w.t0 + i) * TC_BN + 1, TC_BN) : 0;  // keys [0, visible) of the tile
+                dc_wait(s_full + 8 * (j & 1), (j >> 1) & 1, dead);
+                g_tc_fence_after();
+                uint32_t sv[2][32];
+                g_tmem_ld32_nowait(tmem + lane_base + (j & 1) * TC_BN, sv[0]);
+                g_tmem_ld32_nowait(tmem + lane_base + (j & 1) * TC_BN + 32, sv[1]);
+                g_tmem_ld_wait();
+                float raw_max = -CUDART_INF_F;  // the scale is positive, so it commutes with max
+                if (visible < TC_BN)
+#pragma unroll
+                    for (int c = 0; c < TC_BN; ++c)
+                        if (c >= visible) sv[c >> 5][c & 31] = 0xff800000u;  // -inf: exp2 gives exactly 0
+#pragma unroll
+                for (int c = 0; c < TC_BN; ++c) raw_max = fmaxf(raw_max, __uint_as_float(sv[c >> 5][c & 31]));
+                const float tile_max = raw_max * a.scale_log2;
+                // lazy rescale: keep the stale maximum unless this tile exceeds it by more than 2^8
+                const bool grow = tile_max > m_used + TC_RESCALE_THRESHOLD || (m_used == -CUDART_INF_F && tile_max != -CUDART_INF_F);
+                if (__any_sync(0xffffffffu, grow) && i > 0) {
+                    dc_wait(pv_done, (j - 1) & 1, dead);  // O must be stable while it is rescaled
+                    g_tc_fence_after();
+                    const float m_new = grow ? tile_max : m_used;
+                    const float alpha = (grow && m_used != -CUDART_INF_F) ? exp2f(m_used - m_new) : (grow ? 0.f : 1.f);
+                    l_sum *= alpha;
+#pragma unroll
+                    for (int cb = 0; cb < TC_D / 32; ++cb) {
+                        uint32_t ov[32];
+                        g_tmem_ld32(tmem + lane_base + TC_TMEM_O + cb * 32, ov);
+#pragma unroll
+                        for (int c = 0; c < 32; ++c) ov[c] = __float_as_uint(__uint_as_float(ov[c]) * alpha);
+                        g_tmem_st32(tmem + lane_base + TC_TMEM_O + cb * 32, ov);
+                    }
+                    g_tmem_st_wait();
+                    m_used = m_new;
+                } else if (grow) {
+                    m_used = tile_max;  // first tile: nothing accumulated yet
+                }
+                const float m_eff = m_used == -CUDART_INF_F ? 0.f : m_used;
+                float tile_sum = 0.f;
+                uint32_t pk[32];  // 64 bf16 probabilities, over the first 32 columns of the score buffer just read
+#pragma unroll
+                for (int c = 0; c < TC_BN; c += 2) {
+                    const float p0 = tc_ex2(fmaf(__uint_as_float(sv[c >> 5][c & 31]), a.scale_log2, -m_eff));
+                    const float p1 = tc_ex2(fmaf(__uint_as_float(sv[c >> 5][(c & 31) + 1]), a.scale_log2, -m_eff));
+                    tile_sum += p0 + p1;
+                    pk[c / 2] = pack2<bf16>(p0, p1);
+                }
+                l_sum += tile_sum;
+                g_tmem_st32(tmem + lane_base + (j & 1) * TC_BN, pk);
+                g_tmem_st_wait();
+                if (j > 0) dc_wait(pv_done, (j - 1) & 1, dead);  // one phase of p_full at a time (see the prompt kernel)
+                g_tc_fence_before();
+                __syncwarp();
+                if (lane == 0) g_mbar_arrive(p_full);
+            }
+            dc_wait(pv_done, (j - 1) & 1, dead);
+            g_tc_fence_after();
+            const size_t out_row = static_cast<size_t>(w.b * a.Hq + w.kvh * a.G + g) * a.L + l;
+            const bool whole = w.n == w.tiles;
+            const float inv = whole ? (l_sum == 0.f ? 0.f : 1.0f / l_sum) : 1.f, bad = *dead ? CUDART_NAN_F : 1.f;
+            const size_t slot = out_row * a.max_pieces + (whole ? 0 : blockIdx.x - (w.base + w.kvh * w.tiles) / deal.per);
+#pragma unroll
+            for (int cb = 0; cb < TC_D / 32; ++cb) {
+                uint32_t ov[32];
+                g_tmem_ld32(tmem + lane_base + TC_TMEM_O + cb * 32, ov);
+                if (r >= rows) continue;
+                if (whole) {
+                    bf16 *dst = a.out + out_row * TC_D + cb * 32;
+#pragma unroll
+                    for (int c = 0; c < 32; c += 8) {
+                        uint32_t o[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            o[e] = pack2<bf16>(__uint_as_float(ov[c + 2 * e]) * inv * bad, __uint_as_float(ov[c + 2 * e + 1]) * inv * bad);
+                        *reinterpret_cast<uint4 *>(dst + c) = make_uint4(o[0], o[1], o[2], o[3]);
+                    }
+                } else {
+                    float *po = a.ws_o + slot * TC_D + cb * 32;
+#pragma unroll
+                    for (int c = 0; c < 32; c += 4) *reinterpret_cast<uint4 *>(po + c) = make_uint4(ov[c], ov[c + 1], ov[c + 2], ov[c + 3]);
+                }
+            }
+            if (!whole && r < rows) a.ws_m[slot] = m_used == -CUDART_INF_F ? -1e30f : m_used, a.ws_l[slot] = l_sum * bad;
+        } while (w.next(a));
+    }
+    g_tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        if (*dead)
+            for (int i = 0; i < 2000; ++i) __nanosleep(1000);  // copies in flight land first
+        g_tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TC_TMEM_COLS) : "memory");
+    }
+}
+
+// One CTA per row: the pieces' sums brought to their common maximum and divided, in the pieces' order.  Rows that one CTA finished are
+// left alone, rows of a request without keys are zero.
+__global__ void __launch_bounds__(TC_D) decode_merge_tc_kernel(const DecodeTcArgs a) {
+    griddep_launch();
+    const int row = blockIdx.x, d = threadIdx.x, lane = d & 31;
+    const int b = row / (a.Hq * a.L), kvh = (row - b * a.Hq * a.L) / (a.G * a.L);
+    const DecodeDeal deal = dc_deal(a, b);
+    const int tiles = dc_tiles(a, b), u0 = deal.before + kvh * tiles;
+    const int pieces = tiles == 0 ? 0 : deal.per == 0 ? 1 : (u0 + tiles - 1) / deal.per - u0 / deal.per + 1;
+    griddep_wait();
+    if (pieces == 1) return;
+    const float *pm = a.ws_m + static_cast<size_t>(row) * a.max_pieces, *pl = a.ws_l + static_cast<size_t>(row) * a.max_pieces;
+    const float *po = a.ws_o + static_cast<size_t>(row) * a.max_pieces * TC_D + d;
+    float v[8];  // the first columns go out beside the weights (the workspace is rewritten by every layer: read through L2)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = j < pieces ? __ldcg(po + static_cast<size_t>(j) * TC_D) : 0.f;
+    const float m = lane < pieces ? __ldcg(pm + lane) : -1e30f, s = lane < pieces ? __ldcg(pl + lane) : 0.f;  // at most 32 pieces
+    const float gm = warp_max(m), f = exp2f(m - gm), gl = warp_sum(s * f);
+    float o = 0.f;
+    for (int s0 = 0; s0 < pieces; s0 += 8) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float fj = __shfl_sync(0xffffffffu, f, (s0 + j) & 31);
+            if (s0 + j < pieces) o += v[j] * fj;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (s0 + 8 + j < pieces) v[j] = __ldcg(po + static_cast<size_t>(s0 + 8 + j) * TC_D);
+    }
+    a.out[static_cast<size_t>(row) * TC_D + d] = __float2bfloat16_rn(gl == 0.f ? 0.f : o / gl);
 }
 
 // ---------------------------------------------------------------- host side --
@@ -477,12 +852,21 @@ bool paged_prefill_tc_supported(int L, int num_pages, int page_size, int num_kv_
     return L > 0 && num_pages > 0 && page_size >= TC_BN && page_size % TC_BN == 0;
 }
 
-// allow_split (decode, L <= 8): the key range of every (request, KV head) is cut into up to GQA_MAX_SPLITS (32, the
-// size paged_decode_workspace() budgets for) pieces of >= 4 tiles so that a small batch still fills the GPU; the
-// partials are combined by paged_gqa_merge_kernel.
+// Tensor maps of the queries (boxes of RH positions x G heads) and of the pages (boxes of one tile).
+static int attention_maps(CUtensorMap *mq, CUtensorMap *mk, CUtensorMap *mv, const void *q, const void *kp, const void *vp, int rows, int L, int RH, int G, int num_pages,
+                          int page_size, int num_kv_heads) {
+    const cuuint64_t qdims[3] = {TC_D, static_cast<cuuint64_t>(L), static_cast<cuuint64_t>(rows)};
+    const cuuint32_t qbox[3] = {64, static_cast<cuuint32_t>(RH), static_cast<cuuint32_t>(G)};
+    if (int e = cached_map(mq, q, 3, qdims, qbox)) return e;
+    const cuuint64_t dims[4] = {TC_D, static_cast<cuuint64_t>(page_size), static_cast<cuuint64_t>(num_kv_heads), static_cast<cuuint64_t>(num_pages)};
+    const cuuint32_t box[4] = {64, TC_BN, 1, 1};
+    if (int e = cached_map(mk, kp, 4, dims, box)) return e;
+    return cached_map(mv, vp, 4, dims, box);
+}
+
 int launch_paged_prefill_tc(const void *q, const void *kp, const void *vp, const int32_t *bt, const int32_t *cl, void *out, int rows,
                             int L, int num_pages, int page_size, int max_pages, float scale, int is_causal, int num_kv_heads,
-                            int num_heads, bool allow_split, void *ws, size_t ws_bytes, cudaStream_t st, bool out_token_major) {
+                            int num_heads, cudaStream_t st, bool out_token_major) {
     const int G = num_heads / num_kv_heads;
     const int B = rows / num_heads;
     TcArgs a{};
@@ -493,17 +877,7 @@ int launch_paged_prefill_tc(const void *q, const void *kp, const void *vp, const
     a.scale_log2 = scale * TC_LOG2E;
     a.is_causal = is_causal;
     CUtensorMap mq, mk, mv;
-    {
-        const cuuint64_t dims[3] = {TC_D, static_cast<cuuint64_t>(L), static_cast<cuuint64_t>(rows)};
-        const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(a.RH), static_cast<cuuint32_t>(G)};
-        if (int e = cached_map(&mq, q, 3, dims, box)) return e;
-    }
-    {
-        const cuuint64_t dims[4] = {TC_D, static_cast<cuuint64_t>(page_size), static_cast<cuuint64_t>(num_kv_heads), static_cast<cuuint64_t>(num_pages)};
-        const cuuint32_t box[4] = {64, TC_BN, 1, 1};
-        if (int e = cached_map(&mk, kp, 4, dims, box)) return e;
-        if (int e = cached_map(&mv, vp, 4, dims, box)) return e;
-    }
+    if (int e = attention_maps(&mq, &mk, &mv, q, kp, vp, rows, L, a.RH, G, num_pages, page_size, num_kv_heads)) return e;
     static bool configured = false;
     if (!configured) {
         if (cudaFuncSetAttribute(paged_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES) != cudaSuccess ||
@@ -514,43 +888,48 @@ int launch_paged_prefill_tc(const void *q, const void *kp, const void *vp, const
         configured = true;
     }
     const int q_blocks = (L + a.RH - 1) / a.RH;
-    const long long max_tiles = (static_cast<long long>(max_pages) * page_size + TC_BN - 1) / TC_BN;
     a.out_token_major = out_token_major ? 1 : 0;
-    a.splits = 1;
-    a.tiles_per_split = static_cast<int>(max_tiles < 1 ? 1 : max_tiles);
-    if (allow_split && ws != nullptr && !out_token_major) {
-        // Split count: the one that minimises waves x (tiles per CTA + fixed cost) + merge launch, in units of one 64-key
-        // tile (~1.45 us of HBM time at a 1/296 share), with 296 CTA slots, ~3 tiles of fixed cost per CTA (set-up, Q load,
-        // epilogue) and 2 + splits / 4 for the merge launch (it reads one partial per split and row).  (The first policy aimed at 4 x #SMs CTAs: at 64 requests x 1024 tokens
-        // that is 1024 CTAs in 3.5 -> 4 waves plus a merge, 60 us, where 512 unsplit CTAs need 2 waves.)
-        const long long base = static_cast<long long>(q_blocks) * num_kv_heads * B;
-        const long long slots = 2LL * sm_count();
-        const size_t rows_total = static_cast<size_t>(rows) * L;
-        long long best = 1, best_cost = -1;
-        for (long long sp = 1; sp <= 32 && sp <= (max_tiles > 1 ? max_tiles : 1); ++sp) {
-            const long long tps = (max_tiles + sp - 1) / sp;
-            const long long real = (max_tiles + tps - 1) / tps;
-            if (real != sp) continue;
-            if (sp > 1 && ws_bytes < rows_total * sp * (TC_D + 2) * sizeof(float)) break;
-            const long long waves = (base * sp + slots - 1) / slots;
-            const long long cost = 4 * waves * (tps + 3) + (sp > 1 ? 8 + sp : 0);  // x 4: quarter-tile units
-            if (best_cost < 0 || cost < best_cost) best_cost = cost, best = sp;
-        }
-        if (best > 1) {
-            a.splits = static_cast<int>(best), a.tiles_per_split = static_cast<int>((max_tiles + best - 1) / best);
-            a.ws_o = static_cast<float *>(ws);
-            a.ws_m = a.ws_o + rows_total * best * TC_D;
-            a.ws_l = a.ws_m + rows_total * best;
-        }
-    }
-    dim3 grid(q_blocks * a.splits, num_kv_heads, B);
+    dim3 grid(q_blocks, num_kv_heads, B);
     if (grid.y > 65535 || grid.z > 65535) return fail(TL_EINVAL, "paged_attention: too many heads / requests for one launch");
     static const bool p_tmem = [] { const char *e = getenv("TL_FA_P_TMEM"); return e == nullptr || e[0] != '0'; }();  // 0: P through shared memory (control)
     cudaError_t le = p_tmem ? launch_chained(paged_prefill_tc_kernel<true>, grid, dim3(TC_THREADS), TC_SMEM_BYTES, st, mq, mk, mv, a)
                             : launch_chained(paged_prefill_tc_kernel<false>, grid, dim3(TC_THREADS), TC_SMEM_BYTES, st, mq, mk, mv, a);
     if (le != cudaSuccess) return fail(TL_ECUDA, "paged_attention: launch failed: %s", cudaGetErrorString(le));
     TL_LAUNCH_CHECK("paged_prefill_tc");
-    if (a.splits > 1) return launch_paged_gqa_merge(a.ws_o, a.ws_m, a.ws_l, out, rows * L, a.splits, st);
+    return TL_OK;
+}
+
+int launch_paged_decode_tc(const void *q, const void *kp, const void *vp, const int32_t *bt, const int32_t *cl, void *out, int rows, int L,
+                           int num_pages, int page_size, int max_pages, float scale, int is_causal, int num_kv_heads, int num_heads, void *ws,
+                           size_t ws_bytes, cudaStream_t st) {
+    const size_t rows_total = static_cast<size_t>(rows) * L;
+    const long long pieces = ws == nullptr ? 0 : std::min<long long>(32, ws_bytes / (rows_total * (TC_D + 2) * sizeof(float)));
+    const long long most = (static_cast<long long>(max_pages) * page_size + TC_BN - 1) / TC_BN * num_kv_heads * (rows / num_heads);
+    if (pieces < 2 || most > (1LL << 30))  // no room for partial results, or more tiles than an int counts: a CTA per (request, head)
+        return launch_paged_prefill_tc(q, kp, vp, bt, cl, out, rows, L, num_pages, page_size, max_pages, scale, is_causal, num_kv_heads, num_heads, st);
+    DecodeTcArgs a{};
+    a.block_table = bt, a.context_lens = cl, a.out = static_cast<bf16 *>(out);
+    a.L = L, a.Hq = num_heads, a.Hkv = num_kv_heads, a.G = num_heads / num_kv_heads, a.requests = rows / num_heads;
+    a.page_size = page_size, a.max_pages = max_pages, a.num_pages = num_pages, a.tiles_per_page = page_size / TC_BN;
+    a.scale_log2 = scale * TC_LOG2E, a.is_causal = is_causal;
+    a.ctas = static_cast<int>(std::max(1LL, std::min(2LL * sm_count(), (most + DC_MIN_TILES - 1) / DC_MIN_TILES)));
+    a.max_pieces = static_cast<int>(pieces);
+    a.ws_o = static_cast<float *>(ws), a.ws_m = a.ws_o + rows_total * pieces * TC_D, a.ws_l = a.ws_m + rows_total * pieces;
+    CUtensorMap mq, mk, mv;
+    if (int e = attention_maps(&mq, &mk, &mv, q, kp, vp, rows, L, L, a.G, num_pages, page_size, num_kv_heads)) return e;
+    const bool narrow = a.G * L <= 32;
+    static const bool configured = cudaFuncSetAttribute(paged_decode_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeTcShape<1>::smem) == cudaSuccess &&
+                                   cudaFuncSetAttribute(paged_decode_tc_kernel<1>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) == cudaSuccess &&
+                                   cudaFuncSetAttribute(paged_decode_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeTcShape<4>::smem) == cudaSuccess &&
+                                   cudaFuncSetAttribute(paged_decode_tc_kernel<4>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) == cudaSuccess;
+    if (!configured) return fail(TL_ECUDA, "paged_attention: cannot raise shared memory limit");
+    cudaError_t le = narrow ? launch_chained(paged_decode_tc_kernel<1>, dim3(a.ctas), dim3(DecodeTcShape<1>::threads), DecodeTcShape<1>::smem, st, mq, mk, mv, a)
+                            : launch_chained(paged_decode_tc_kernel<4>, dim3(a.ctas), dim3(DecodeTcShape<4>::threads), DecodeTcShape<4>::smem, st, mq, mk, mv, a);
+    if (le != cudaSuccess) return fail(TL_ECUDA, "paged_attention: launch failed: %s", cudaGetErrorString(le));
+    TL_LAUNCH_CHECK("paged_decode_tc");
+    le = launch_chained(decode_merge_tc_kernel, dim3(static_cast<unsigned>(rows_total)), dim3(TC_D), 0, st, a);
+    if (le != cudaSuccess) return fail(TL_ECUDA, "paged_attention: launch failed: %s", cudaGetErrorString(le));
+    TL_LAUNCH_CHECK("decode_merge_tc");
     return TL_OK;
 }
 

@@ -257,7 +257,7 @@ int tl_paged_attention_token_major(const void *q, const void *key_pages, const v
         !aligned16(value_pages))
         return fail(TL_EINVAL, "paged_attention_token_major: needs the tcgen05 kernel (bf16, D = 128, pages a multiple of 64 slots)");
     return launch_paged_prefill_tc(q, key_pages, value_pages, block_table, context_lens, out, rows, L, num_pages, page_size, max_pages, scale,
-                                   is_causal, num_kv_heads, num_heads, false, nullptr, 0, as_stream(stream), true);
+                                   is_causal, num_kv_heads, num_heads, as_stream(stream), true);
 }
 
 // ------------------------------------------------------------------ misc --
