@@ -80,6 +80,13 @@ int tl_quantized_matmul(const void *scales, const void *biases, const void *a, c
                         int N, int K, int dtype, int use_simdgroup, int use_split_k, void *workspace,
                         size_t workspace_bytes, void *stream);
 
+/* The gated MLP's first half: gate_out = a . dequant(gate)^T and out = silu(gate_out) * (a . dequant(up)^T), both [M, K].  Same kernels
+ * and rounding points as two tl_quantized_matmul calls and tl_swiglu.  Flags of either product: 1 = use_simdgroup, 2 = use_split_k;
+ * the workspace is the larger of their tl_quantized_matmul_workspace. */
+int tl_quantized_gate_up(const void *gate_scales, const void *gate_biases, const void *gate_b, const void *up_scales, const void *up_biases,
+                         const void *up_b, const void *a, void *gate_out, void *out, int M, int N, int K, int dtype, int gate_flags,
+                         int up_flags, void *workspace, size_t workspace_bytes, void *stream);
+
 /* Replaces quantized_embedding (tiny_llm_ext.h:40-41, quantized_matmul.cpp:82-101,
  * :242-273).  indices int32/uint32 [tokens] (bit pattern), weight [vocab, dim/8] u32,
  * scales/biases [vocab, dim/128], out [tokens, dim]. */
@@ -160,7 +167,7 @@ size_t tl_argmax_workspace(int rows, int vocab);
  * epilogues; weights rounded to the activation dtype like every tensor-core path) and needs
  * tl_quantized_matmul_fused_workspace() bytes of workspace. */
 enum { TL_PRO_NONE = 0, TL_PRO_RMSNORM = 1, TL_PRO_SWIGLU = 2 };
-enum { TL_EPI_NONE = 0, TL_EPI_RESIDUAL = 1, TL_EPI_SWIGLU_PAIRS = 2 };
+enum { TL_EPI_NONE = 0, TL_EPI_RESIDUAL = 1, TL_EPI_SWIGLU_PAIRS = 2, TL_EPI_GATED = 3 /* of tl_quantized_gate_up alone */ };
 size_t tl_quantized_matmul_fused_workspace(int M, int N, int K, int lda, int prologue, int dtype);
 int tl_quantized_matmul_fused(const void *scales, const void *biases, const void *b, void *out, const void *p0,
                               const void *p1, const void *residual, int M, int N, int K, int lda, int prologue,

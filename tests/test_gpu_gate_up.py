@@ -1,0 +1,49 @@
+"""The gated MLP's first half in one call - the up projection applies the activation in its epilogue - against two products and swiglu:
+the same bits from every kernel that a number of rows takes, whole and ragged feature tiles, unaligned rows, both types."""
+
+import pytest
+import torch
+
+from extensions_b200 import tiny_llm_ext_b200 as ext
+from tiny_llm_b200.quantize import QuantizedWeights, quantized_gate_up, quantized_linear
+
+pytestmark = pytest.mark.gpu
+
+
+def weight(K, N, dtype, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    scales = (torch.randn(K, N // 128, generator=g, device="cuda") * 0.2 / N**0.5).to(dtype)
+    words = torch.randint(-(2**31), 2**31 - 1, (K, N // 8), generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+    return scales, (scales.float() * -7.5).to(dtype), words
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("K,N", [(1000, 256), (1001, 384), (9728, 2560), (130, 1024)])
+@pytest.mark.parametrize("M", [0, 1, 5, 8, 9, 24, 64, 100, 128, 129, 300, 515, 2048])
+def test_equals_two_products_and_swiglu(M, K, N, dtype):
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    a = torch.randn(M, N, generator=g, device="cuda").to(dtype) * 4
+    gate, up = weight(K, N, dtype, 1), weight(K, N, dtype, 2)
+    for flags in ((True, False), (True, True)) + (((False, False),) if M * K < 10**6 else ()):
+        product = lambda w: ext.quantized_matmul(w[0], w[1], 128, 4, a, w[2], True, *flags)
+        want = ext.swiglu(product(gate), product(up))
+        assert torch.equal(ext.quantized_gate_up(a, gate, up, flags, flags), want)
+    if M == 2048:  # the kernel of thread-block pairs, for every size
+        ext.set_gemm_pairs(2)
+        try:
+            want = ext.swiglu(product(gate), product(up))
+            assert torch.equal(ext.quantized_gate_up(a, gate, up, flags, flags), want)
+        finally:
+            ext.set_gemm_pairs(1)
+
+
+def test_layer_form_mixed_flags_and_refusals():
+    gate, up, odd = (weight(k, 256, torch.bfloat16, s) for k, s in ((264, 1), (264, 2), (272, 3)))
+    wrap = lambda w, **flags: QuantizedWeights(scales=w[0], biases=w[1], group_size=128, bits=4, weight=w[2], **flags)
+    x = torch.randn(3, 40, 256, device="cuda").bfloat16().transpose(0, 1)
+    a, b = wrap(gate), wrap(up, use_simdgroup_matmul=True)
+    assert torch.equal(quantized_gate_up(x, a, b), ext.swiglu(quantized_linear(x, a), quantized_linear(x, b)))
+    with pytest.raises(RuntimeError, match="swiglu: gate and up must have the same shape"):
+        quantized_gate_up(x, a, wrap(odd))
+    with pytest.raises(RuntimeError, match="a must be the same dtype as scales"):
+        quantized_gate_up(x.half(), a, b)

@@ -57,6 +57,7 @@ int launch_w4a16_stream(const void *scales, const void *biases, const void *a, c
 // (so results match rms_norm -> matvec, swiglu -> matvec, matvec -> add):
 //   prologue RMSNORM : a = T(x * rsqrt(mean(x^2)+eps) * w)   (week2_kernels.metal:41-47)
 //   prologue SWIGLU  : a = T(g / (1 + exp(-g)) * u)          (week2_kernels.metal:115-116)
+//   epilogue GATED:    out = T(silu(res) * float(T(acc))), res = the gate projection's output
 //   epilogue RESIDUAL: out = T(float(res) + float(T(acc)))   (qwen3_week3.py:204-206)
 //   epilogue SWIGLU_PAIRS: rows 16c+r / 16c+8+r hold gate / up feature 8c+r;
 //                     out[m, 8c+r] = T(silu(T(acc_gate)) * T(acc_up))  (week2_kernels.metal:115-116)
@@ -81,7 +82,7 @@ constexpr int S5_WARPS = 16;
 #define S5_DEPTH_SMALL 4
 #endif
 enum { PRO_NONE = W4_PRO_NONE, PRO_RMSNORM = W4_PRO_RMSNORM, PRO_SWIGLU = W4_PRO_SWIGLU };
-enum { EPI_NONE = 0, EPI_RESIDUAL = 1, EPI_SWIGLU_PAIRS = 2 };
+enum { EPI_NONE = 0, EPI_RESIDUAL = 1, EPI_SWIGLU_PAIRS = 2, EPI_GATED = 3 };
 
 struct StreamArgs {
     const void *scales, *biases;
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(S5_WARPS * 32, 1) w4a16_stream5_kernel(const S
                       ? static_cast<const T *>(args.p1) + static_cast<size_t>(pass) * args.rows_per_pass * args.lda
                       : static_cast<const T *>(args.p1);
     T *out = static_cast<T *>(args.out) + static_cast<size_t>(pass) * args.rows_per_pass * (args.epilogue == EPI_SWIGLU_PAIRS ? K / 2 : K);
-    const T *res = args.epilogue == EPI_RESIDUAL ? static_cast<const T *>(args.residual) + static_cast<size_t>(pass) * args.rows_per_pass * K
+    const T *res = args.epilogue == EPI_RESIDUAL || args.epilogue == EPI_GATED ? static_cast<const T *>(args.residual) + static_cast<size_t>(pass) * args.rows_per_pass * K
                                                  : nullptr;
     // the residual of this thread's first output: requested now, needed after the stream
     const int outs = chunks * 16 * Mp;
@@ -262,7 +263,7 @@ __global__ void __launch_bounds__(S5_WARPS * 32, 1) w4a16_stream5_kernel(const S
             T vb = from_f<T>(chunk_sum(ch, row, m));
             if (res != nullptr) {
                 const float rv = o == static_cast<int>(threadIdx.x) ? res_first : to_f(res[static_cast<size_t>(m) * K + k]);
-                vb = from_f<T>(rv + to_f(vb));
+                vb = from_f<T>(args.epilogue == EPI_GATED ? (rv / (1.0f + expf(-rv))) * to_f(vb) : rv + to_f(vb));
             }
             out[static_cast<size_t>(m) * K + k] = vb;
         }

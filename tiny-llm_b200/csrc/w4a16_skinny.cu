@@ -48,7 +48,7 @@ constexpr int SK_DEQ_THREADS = 256;
 constexpr int SK_TRC_BLOCKS = 40;
 constexpr int SK_GROUP_WARPS = 4;   // dequantiser warps per group block (two groups alternate blocks)
 constexpr int SK_THREADS = 128 + SK_DEQ_THREADS;
-enum { SK_EPI_NONE = 0, SK_EPI_RESIDUAL = 1, SK_EPI_SWIGLU_PAIRS = 2 };
+enum { SK_EPI_NONE = 0, SK_EPI_RESIDUAL = 1, SK_EPI_SWIGLU_PAIRS = 2, SK_EPI_GATED = 3 };
 
 // Shared memory: activation ring (BSTAGES group blocks of two [NT x 64] tiles) + packed-weight ring (PSTAGES boxes) +
 // barriers.  Tensor memory: D[feature, token] in the first D_COLS columns, then ASTAGES dequantised tiles of 64
@@ -416,7 +416,8 @@ void trace_bind_skinny(unsigned long long *buf, unsigned int *n, unsigned int ca
 // Adds the fp32 partial planes of a split reduction in split order (deterministic: same bits on every run and for
 // every CTA schedule) and applies the epilogue; one thread per output.  All `splits` loads of a thread are independent
 // and in flight together (the first version let the last CTA of a tile do this with dependent round trips: 40 us).
-template <typename T>
+// GATED: out = silu(res) * result, res the gate projection's output.
+template <typename T, bool GATED>
 __global__ void __launch_bounds__(256) w4a16_skinny_reduce_kernel(const float *part, const T *res, T *out, int M, int K, int splits, int epilogue) {
     const size_t plane = static_cast<size_t>(M) * K;
     griddep_launch();
@@ -449,6 +450,10 @@ __global__ void __launch_bounds__(256) w4a16_skinny_reduce_kernel(const float *p
     if (idx >= plane) return;
     T vb = from_f<T>(plane_sum(idx));
     if (epilogue == SK_EPI_RESIDUAL) vb = from_f<T>(to_f(ld_cg(res + idx)) + to_f(vb));
+    if (GATED) {
+        const float gate = to_f(ld_cg(res + idx));
+        vb = from_f<T>((gate / (1.0f + expf(-gate))) * to_f(vb));
+    }
     out[idx] = vb;
 }
 
@@ -647,6 +652,8 @@ static int skinny_t(const void *scales, const void *biases, const void *a, const
         *planes_out = args.splits;
         if (args.splits > 1) return rc;
     }
+    if (rc == TL_OK && args.splits == 1 && epilogue == SK_EPI_GATED)  // the kernel's own epilogue has no activation
+        return launch_swiglu(residual, out, out, static_cast<long long>(M) * K, std::is_same<T, __nv_bfloat16>::value ? TL_BF16 : TL_F16, st);
     if (rc != TL_OK || args.splits == 1) return rc;
     if (normed != nullptr && epilogue == SK_EPI_RESIDUAL && K <= 256 * SK_NORM_PER) {
         cudaError_t e = launch_chained(w4a16_skinny_reduce_norm_kernel<T>, dim3(M), dim3(256), 0, st, static_cast<const float *>(args.partials),
@@ -658,7 +665,7 @@ static int skinny_t(const void *scales, const void *biases, const void *a, const
         return TL_OK;
     }
     const size_t outputs = static_cast<size_t>(M) * (epilogue == SK_EPI_SWIGLU_PAIRS ? K / 2 : K);
-    cudaError_t e = launch_chained(w4a16_skinny_reduce_kernel<T>, dim3(static_cast<unsigned>((outputs + 255) / 256)), dim3(256), 0, st,
+    cudaError_t e = launch_chained(epilogue == SK_EPI_GATED ? w4a16_skinny_reduce_kernel<T, true> : w4a16_skinny_reduce_kernel<T, false>, dim3(static_cast<unsigned>((outputs + 255) / 256)), dim3(256), 0, st,
                                    static_cast<const float *>(args.partials), static_cast<const T *>(residual), static_cast<T *>(out), M, K,
                                    args.splits, epilogue);
     if (e != cudaSuccess) return fail(TL_ECUDA, "w4a16_skinny_reduce: launch failed: %s", cudaGetErrorString(e));

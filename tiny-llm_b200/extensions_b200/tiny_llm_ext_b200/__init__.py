@@ -70,6 +70,7 @@ _SIGNATURES = {
     "tl_device_info": (_I, [ctypes.POINTER(_I)] * 3),
     "tl_quantized_matmul_workspace": (_SZ, [_I] * 6),
     "tl_quantized_matmul": (_I, [_VP] * 5 + [_I] * 6 + [_VP, _SZ, _VP]),
+    "tl_quantized_gate_up": (_I, [_VP] * 9 + [_I] * 6 + [_VP, _SZ, _VP]),
     "tl_quantized_embedding": (_I, [_VP] * 5 + [_I] * 4 + [_VP]),
     "tl_rms_norm": (_I, [_VP] * 3 + [_I, _I, _F, _I, _VP]),
     "tl_rope": (_I, [_VP] * 3 + [_I] * 5 + [_F, _I, _I, _VP]),
@@ -195,21 +196,9 @@ def quantized_matmul(
     stream=None,
 ):
     """``a [M,N] @ dequant(b [K,N/8]).T -> [M,K]`` (bindings.cpp:16-33)."""
-    dtype = a.dtype
-    try:  # one pass over the attributes; what does not fit goes through the checks one by one, for their messages
-        (M, N), (K, words) = a.shape, b.shape
-        fits = (
-            dtype in _HALF and scales.dtype is dtype and biases.dtype is dtype and b.dtype in _PACKED and bits == 4 and group_size == 128 and transpose_b
-            and N % 128 == 0 and words * 8 == N and scales.shape == (K, N // 128) and biases.shape == (K, N // 128)
-            and a.is_cuda and b.is_cuda and scales.is_cuda and biases.is_cuda
-            and a.is_contiguous() and b.is_contiguous() and scales.is_contiguous() and biases.is_contiguous()
-        )
-    except ValueError:  # not two dimensions
-        fits = False
-    if not fits:
+    if not (transpose_b and _quantized_matmul_fits(scales, biases, group_size, bits, a, b)):
         _check_quantized_matmul(scales, biases, group_size, bits, a, b, transpose_b)
-        M, N = a.shape
-        K = b.shape[0]
+    dtype, (M, N), K = a.dtype, a.shape, b.shape[0]
     out = a.new_empty((M, K))
     code = _DTYPE_CODE[dtype]
     ws_bytes = _lib.tl_quantized_matmul_workspace(M, N, K, code, int(use_simdgroup), int(use_split_k))
@@ -222,6 +211,21 @@ def quantized_matmul(
         )
     )
     return out
+
+
+def _quantized_matmul_fits(scales, biases, group_size, bits, a, b) -> bool:
+    """One pass over the attributes; what does not fit goes through the checks one by one, for their messages."""
+    dtype = a.dtype
+    try:
+        (M, N), (K, words) = a.shape, b.shape
+    except ValueError:  # not two dimensions
+        return False
+    return (
+        dtype in _HALF and scales.dtype is dtype and biases.dtype is dtype and b.dtype in _PACKED and bits == 4 and group_size == 128
+        and N % 128 == 0 and words * 8 == N and scales.shape == (K, N // 128) and biases.shape == (K, N // 128)
+        and a.is_cuda and b.is_cuda and scales.is_cuda and biases.is_cuda
+        and a.is_contiguous() and b.is_contiguous() and scales.is_contiguous() and biases.is_contiguous()
+    )
 
 
 def _check_quantized_matmul(scales, biases, group_size, bits, a, b, transpose_b) -> None:
@@ -255,6 +259,29 @@ def _check_quantized_matmul(scales, biases, group_size, bits, a, b, transpose_b)
         raise RuntimeError("quantized_matmul: a must have the same number of columns as b")
     _gpu("quantized_matmul", scales, biases, a, b)
     _contig("quantized_matmul", a=a, b=b, scales=scales, biases=biases)
+
+
+def quantized_gate_up(a, gate, up, gate_flags=(True, False), up_flags=(True, False), stream=None):
+    """``silu(a @ gate.T) * (a @ up.T)`` of two quantised weights ``(scales, biases, packed)`` of one shape: the gate's product, then the
+    up projection with the activation in its epilogue.  The flags are (use_simdgroup, use_split_k) of either product.  The same bits as two
+    ``quantized_matmul`` calls and ``swiglu``."""
+    for scales, biases, packed in (gate, up):
+        if not _quantized_matmul_fits(scales, biases, 128, 4, a, packed):
+            _check_quantized_matmul(scales, biases, 128, 4, a, packed, True)
+    (M, N), K, code = a.shape, gate[2].shape[0], _DTYPE_CODE[a.dtype]
+    if up[2].shape[0] != K:
+        raise RuntimeError("swiglu: gate and up must have the same shape and dtype")
+    gate_out, out = a.new_empty((M, K)), a.new_empty((M, K))
+    ws_bytes = max(_lib.tl_quantized_matmul_workspace(M, N, K, code, int(s), int(k)) for s, k in {gate_flags, up_flags})
+    ws = _zero_workspace(ws_bytes, a.device) if ws_bytes else None
+    _check(
+        _lib.tl_quantized_gate_up(
+            gate[0].data_ptr(), gate[1].data_ptr(), gate[2].data_ptr(), up[0].data_ptr(), up[1].data_ptr(), up[2].data_ptr(), a.data_ptr(),
+            gate_out.data_ptr(), out.data_ptr(), M, N, K, code, int(gate_flags[0]) + 2 * int(gate_flags[1]), int(up_flags[0]) + 2 * int(up_flags[1]),
+            None if ws is None else ws.data_ptr(), ws_bytes, _stream_ptr(stream, a),
+        )
+    )
+    return out
 
 
 def quantized_embedding(indices, scales, biases, weight, group_size, bits, stream=None):

@@ -201,6 +201,9 @@ class DecodeEngine:
         def proj(h, w):
             return ext.quantized_matmul(w.scales, w.biases, w.group_size, w.bits, h, w.weight, True)
 
+        def gate_up(h, mlp):
+            return ext.quantized_gate_up(h, *((w.scales, w.biases, w.weight) for w in (mlp.w_gate, mlp.w_up)))
+
         for i, block in enumerate(m.layers_inner):
             at = block.self_attn
             pool = m.page_pools[i]
@@ -218,7 +221,7 @@ class DecodeEngine:
             x = ext.add(x, proj(y.view(B, Hq * D), at.wo))
             h = ext.rms_norm(x, block.post_attention_layernorm._weight_as(x.dtype, x.device), block.post_attention_layernorm.eps)
             mlp = block.mlp
-            x = ext.add(x, proj(ext.swiglu(proj(h, mlp.w_gate), proj(h, mlp.w_up)), mlp.w_down))
+            x = ext.add(x, proj(gate_up(h, mlp), mlp.w_down))
         x = ext.rms_norm(x, m.norm._weight_as(x.dtype, x.device), m.norm.eps)
         head = m.w_lm_head if m.w_lm_head is not None else m.embedding.weight
         logits = proj(x, head)
@@ -633,6 +636,9 @@ class PrefillEngine:
         def proj(h, w):
             return ext.quantized_matmul(w.scales, w.biases, w.group_size, w.bits, h, w.weight, True)
 
+        def gate_up(h, mlp):
+            return ext.quantized_gate_up(h, *((w.scales, w.biases, w.weight) for w in (mlp.w_gate, mlp.w_up)))
+
         layers = list(m.layers_inner)
         h = normed(x, layers[0].input_layernorm) if skinny else None
         for i, block in enumerate(layers):
@@ -659,7 +665,7 @@ class PrefillEngine:
             else:
                 x = ext.add(x, proj(y, at.wo))
                 h = normed(x, block.post_attention_layernorm)
-                x = ext.add(x, proj(ext.swiglu(proj(h, block.mlp.w_gate), proj(h, block.mlp.w_up)), block.mlp.w_down))
+                x = ext.add(x, proj(gate_up(h, block.mlp), block.mlp.w_down))
         # logits_to_keep = 1: the hidden state is sliced before the final norm (qwen3_week3.py:330-338); RMSNorm is row-wise,
         # so the last row of the already normalised chunk is the same thing
         last = h[L - 1:L] if skinny else normed(x[L - 1:L], m.norm)

@@ -139,11 +139,26 @@ def quantized_linear(x: torch.Tensor, w: QuantizedWeights, bias: torch.Tensor | 
     rows = x.reshape(-1, x.shape[-1])
     if not rows.is_contiguous():
         rows = rows.contiguous()
-    few = rows.shape[0] <= 8 and w.use_simdgroup_matvec
-    # at most 8 rows rely on the extension's default use_simdgroup=True to reach the weight-streaming kernel (quantized_matvec_custom)
     y = tiny_llm_ext_b200.quantized_matmul(w.scales.contiguous(), w.biases.contiguous(), w.group_size, w.bits, rows, w.weight.contiguous(), True,
-                                           *(() if few else (w.use_simdgroup_matmul, w.use_split_k_matmul))).reshape(*lead, -1)
+                                           *_kernel_flags(w, rows.shape[0])).reshape(*lead, -1)
     return y if bias is None else y + bias
+
+
+def _kernel_flags(w: QuantizedWeights, rows: int) -> tuple[bool, bool]:
+    """(use_simdgroup, use_split_k): at most 8 rows take the weight-streaming kernel where the weight allows it."""
+    return (True, False) if rows <= 8 and w.use_simdgroup_matvec else (w.use_simdgroup_matmul, w.use_split_k_matmul)
+
+
+def quantized_gate_up(x: torch.Tensor, gate: QuantizedWeights, up: QuantizedWeights) -> torch.Tensor:
+    """``swiglu(quantized_linear(x, gate), quantized_linear(x, up))``, in one call where the weights have one shape."""
+    if not x.is_cuda or gate.weight.shape != up.weight.shape or (gate.bits, gate.group_size, up.bits, up.group_size) != (4, 128, 4, 128):
+        return tiny_llm_ext_b200.swiglu(quantized_linear(x, gate), quantized_linear(x, up))
+    lead = x.shape[:-1]
+    rows = x.reshape(-1, x.shape[-1])
+    if not rows.is_contiguous():
+        rows = rows.contiguous()
+    parts = [(w.scales.contiguous(), w.biases.contiguous(), w.weight.contiguous()) for w in (gate, up)]
+    return tiny_llm_ext_b200.quantized_gate_up(rows, *parts, _kernel_flags(gate, rows.shape[0]), _kernel_flags(up, rows.shape[0])).reshape(*lead, -1)
 
 
 def dequantize_weights(
