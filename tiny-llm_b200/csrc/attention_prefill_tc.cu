@@ -121,9 +121,9 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     const uint32_t q_base = g_smem_u32(tsm + TC_Q_OFF), p_base = g_smem_u32(tsm + TC_P_OFF);
     const uint32_t k_base = g_smem_u32(tsm + TC_K_OFF), v_base = g_smem_u32(tsm + TC_V_OFF);
     const uint32_t bar = g_smem_u32(tsm + TC_BAR_OFF);
-    const uint32_t q_full = bar, s_full = bar + 8 /* two: one per S buffer */, p_full = bar + 24, pv_done = bar + 32;
-    const uint32_t k_full = bar + 40, k_empty = k_full + 8 * TC_STAGES, v_full = k_full + 16 * TC_STAGES, v_empty = k_full + 24 * TC_STAGES;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tsm + TC_BAR_OFF + 40 + 32 * TC_STAGES);
+    const uint32_t q_full = bar, s_full = bar + 8 /* two: one per S buffer */, p_full = bar + 24, pv_done = bar + 40 /* two of each, by the tile's parity */;
+    const uint32_t k_full = bar + 56, k_empty = k_full + 8 * TC_STAGES, v_full = k_full + 16 * TC_STAGES, v_empty = k_full + 24 * TC_STAGES;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tsm + TC_BAR_OFF + 56 + 32 * TC_STAGES);
 
     if (warp == 4 && lane == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_q) : "memory");
@@ -134,8 +134,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         g_mbar_init(q_full, 1);
         g_mbar_init(s_full, 1);
         g_mbar_init(s_full + 8, 1);
-        g_mbar_init(p_full, (rows + 31) / 32);  // one arrival per softmax warp that has rows
-        g_mbar_init(pv_done, 1);
+        for (int i = 0; i < 2; ++i) g_mbar_init(p_full + 8 * i, (rows + 31) / 32), g_mbar_init(pv_done + 8 * i, 1);  // one arrival per softmax warp that has rows
         for (int i = 0; i < TC_STAGES; ++i) {
             g_mbar_init(k_full + 8 * i, 1);
             g_mbar_init(k_empty + 8 * i, 1);
@@ -230,7 +229,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
                 // score buffer (j+1)&1 was last read for tile j-1, whose P has been waited for below
                 if (j + 1 < n_tiles) issue_scores(j + 1);
                 // ---- O += P V: P K-major [128 x 64 keys], V MN-major [64 keys x 128 d] as loaded from the page
-                g_mbar_wait(p_full, j & 1);
+                g_mbar_wait(p_full + 8 * (j & 1), (j >> 1) & 1);
                 g_mbar_wait(v_full + 8 * vs, vph);
                 g_tc_fence_after();
                 if (g_elect_one()) {
@@ -243,7 +242,7 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
                             g_tc_mma(tmem + TC_TMEM_O, pdesc0 + 2 * k, vd + k * (2048 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
                     }
                     g_tc_commit(v_empty + 8 * vs);
-                    g_tc_commit(pv_done);  // O holds tiles 0..j and the P buffer is free again
+                    g_tc_commit(pv_done + 8 * (j & 1));  // O holds tiles 0..j and the P buffer is free again
                 }
                 __syncwarp();
                 if (++vs == TC_STAGES) vs = 0, vph ^= 1u;
@@ -291,11 +290,11 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             }
             const float tile_max = raw_max * a.scale_log2;  // -inf stays -inf
             if constexpr (!PT)
-                if (j > 0) g_mbar_wait(pv_done, (j - 1) & 1);  // P V of tile j-1 complete: O is stable, the P buffer is free
+                if (j > 0) g_mbar_wait(pv_done + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1);  // P V of tile j-1 complete: O is stable, the P buffer is free
             // lazy rescale: keep the stale maximum unless this tile exceeds it by more than 2^8
             const bool grow = tile_max > m_used + TC_RESCALE_THRESHOLD || (m_used == -CUDART_INF_F && tile_max != -CUDART_INF_F);
             if (__any_sync(0xffffffffu, grow) && j > 0) {
-                if constexpr (PT) g_mbar_wait(pv_done, (j - 1) & 1);  // O must be stable while it is rescaled
+                if constexpr (PT) g_mbar_wait(pv_done + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1);  // O must be stable while it is rescaled
                 g_tc_fence_after();
                 const float m_new = grow ? tile_max : m_used;
                 const float alpha = (grow && m_used != -CUDART_INF_F) ? exp2f(m_used - m_new) : (grow ? 0.f : 1.f);
@@ -330,11 +329,8 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
                 // lane = row, column c = keys (2c, 2c + 1) of the tile: over the first 32 columns of the score buffer just read
                 g_tmem_st32(tmem + lane_base + (j & 1) * TC_BN, pk);
                 g_tmem_st_wait();
-                // Do not ARRIVE for tile j before P V of tile j-1 has completed (its exponentials above did overlap it): p_full
-                // counts four arrivals per phase, and a warp that ran a whole tile ahead would arrive twice in one phase and
-                // complete it without the slowest warp - P V_j then read rows that were not written yet (1907 of 16.7 M
-                // outputs off by up to 3 % in the constant-V test of the first version).
-                if (j > 0) g_mbar_wait(pv_done, (j - 1) & 1);
+                // p_full is two barriers, by the tile's parity: a warp arrives for tile j without waiting for P V of tile j-1 (220 of 1750 cycles a
+                // tile), and cannot arrive for j+2 on the same barrier before all have for j, since S_{j+2} is issued behind P V_j.
             } else {
                 // P row r: 128 bytes = 8 chunks of 16 B, chunk c at (c ^ (r & 7)) - the 128-byte swizzle of a K-major tile
                 unsigned char *prow = tsm + TC_P_OFF + r * 128;
@@ -345,11 +341,11 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             }
             g_tc_fence_before();    // orders this thread's tcgen05.ld / st before the MMAs released by the arrive
             __syncwarp();           // one arrival per warp: 128 arrivals on one mbarrier are 128 serialised shared-memory atomics
-            if (lane == 0) g_mbar_arrive(p_full);
+            if (lane == 0) g_mbar_arrive(p_full + 8 * (j & 1));
         }
         // ---- epilogue: O / sum -> bf16 -> out[(b*Hq + head) * L + l, :]
         if (n_tiles > 0) {
-            g_mbar_wait(pv_done, (n_tiles - 1) & 1);
+            g_mbar_wait(pv_done + 8 * ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1);
             g_tc_fence_after();
         }
         const size_t out_row = static_cast<size_t>(b * a.Hq + kvh * a.G + g) * a.L + l;
@@ -534,10 +530,10 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 
     const uint32_t q_base = g_smem_u32(tsm), k_base = g_smem_u32(tsm + Z::k_off), v_base = g_smem_u32(tsm + Z::v_off);
     const uint32_t bar = g_smem_u32(tsm + Z::bar_off);
-    const uint32_t s_full = bar /* two: one per score buffer */, p_full = bar + 16, pv_done = bar + 24, q_full = bar + 32, q_empty = bar + 48;
-    const uint32_t k_full = bar + 64, k_empty = k_full + 24, v_full = k_full + 48, v_empty = k_full + 72;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tsm + Z::bar_off + 64 + 96);
-    volatile int *dead = reinterpret_cast<volatile int *>(tsm + Z::bar_off + 64 + 100);
+    const uint32_t s_full = bar /* two: one per score buffer */, p_full = bar + 16, pv_done = bar + 32 /* two of each, by the tile's parity */, q_full = bar + 48, q_empty = bar + 64;
+    const uint32_t k_full = bar + 80, k_empty = k_full + 24, v_full = k_full + 48, v_empty = k_full + 72;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tsm + Z::bar_off + 80 + 96);
+    volatile int *dead = reinterpret_cast<volatile int *>(tsm + Z::bar_off + 80 + 100);
 
     if (warp == SW && lane == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_q) : "memory");
@@ -548,8 +544,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         *dead = 0;
         g_mbar_init(s_full, 1);
         g_mbar_init(s_full + 8, 1);
-        g_mbar_init(p_full, (rows + 31) / 32);  // one arrival per softmax warp that has rows
-        g_mbar_init(pv_done, 1);
+        for (int i = 0; i < 2; ++i) g_mbar_init(p_full + 8 * i, (rows + 31) / 32), g_mbar_init(pv_done + 8 * i, 1);  // one arrival per softmax warp that has rows
         for (int i = 0; i < Z::q_stages; ++i) g_mbar_init(q_full + 8 * i, 1), g_mbar_init(q_empty + 8 * i, 1);
         for (int i = 0; i < Z::stages; ++i) {
             g_mbar_init(k_full + 8 * i, 1), g_mbar_init(k_empty + 8 * i, 1);
@@ -644,7 +639,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             // score buffer (j+1)&1 was last read for tile j-1, whose P has been waited for below
             if (more) issue_scores(j + 1);
             // a new stretch's first product overwrites O: the softmax warps arrive for it after they have read the old one
-            dc_wait(p_full, j & 1, dead);
+            dc_wait(p_full + 8 * (j & 1), (j >> 1) & 1, dead);
             dc_wait(v_full + 8 * vs, vph, dead);
             g_tc_fence_after();
             if (g_elect_one()) {
@@ -653,7 +648,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 for (int k = 0; k < TC_BN / 16; ++k)  // 16 keys = 8 columns of bf16 pairs per K step
                     g_tc_mma_ts(tmem + TC_TMEM_O, tmem + (j & 1) * TC_BN + 8 * k, vd + k * (2048 >> 4), idesc_o, (value > 0 || k > 0) ? 1u : 0u);
                 g_tc_commit(v_empty + 8 * vs);
-                g_tc_commit(pv_done);
+                g_tc_commit(pv_done + 8 * (j & 1));
             }
             __syncwarp();
             if (++vs == Z::stages) vs = 0, vph ^= 1u;
@@ -689,7 +684,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 // lazy rescale: keep the stale maximum unless this tile exceeds it by more than 2^8
                 const bool grow = tile_max > m_used + TC_RESCALE_THRESHOLD || (m_used == -CUDART_INF_F && tile_max != -CUDART_INF_F);
                 if (__any_sync(0xffffffffu, grow) && i > 0) {
-                    dc_wait(pv_done, (j - 1) & 1, dead);  // O must be stable while it is rescaled
+                    dc_wait(pv_done + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, dead);  // O must be stable while it is rescaled
                     g_tc_fence_after();
                     const float m_new = grow ? tile_max : m_used;
                     const float alpha = (grow && m_used != -CUDART_INF_F) ? exp2f(m_used - m_new) : (grow ? 0.f : 1.f);
@@ -720,12 +715,11 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 l_sum += tile_sum;
                 g_tmem_st32(tmem + lane_base + (j & 1) * TC_BN, pk);
                 g_tmem_st_wait();
-                if (j > 0) dc_wait(pv_done, (j - 1) & 1, dead);  // one phase of p_full at a time (see the prompt kernel)
                 g_tc_fence_before();
                 __syncwarp();
-                if (lane == 0) g_mbar_arrive(p_full);
+                if (lane == 0) g_mbar_arrive(p_full + 8 * (j & 1));
             }
-            dc_wait(pv_done, (j - 1) & 1, dead);
+            dc_wait(pv_done + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, dead);
             g_tc_fence_after();
             const size_t out_row = static_cast<size_t>(w.b * a.Hq + w.kvh * a.G + g) * a.L + l;
             const bool whole = w.n == w.tiles;

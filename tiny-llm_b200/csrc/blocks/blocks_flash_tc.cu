@@ -123,11 +123,13 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     auto tile_key = [&](int t) { return t < kept_tiles ? t * kXKeys : lo + (t - kept_tiles) * kXKeys; };
 
     const uint32_t base = g_smem_u32(flash_tc_smem), k_at = base + Z::k_off, v_at = base + Z::v_off, bar = base + Z::bar_off;
-    const uint32_t q_full = bar, s_full = bar + 8, p_full = bar + 24, pv_done = bar + 32, k_full = bar + 40, k_empty = bar + 56, v_full = bar + 72, v_empty = bar + 88;
-    volatile int *dead = reinterpret_cast<volatile int *>(flash_tc_smem + Z::bar_off + 104);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(flash_tc_smem + Z::bar_off + 108);
+    const uint32_t q_full = bar, s_full = bar + 8, p_full = bar + 24, pv_done = bar + 40, k_full = bar + 56, k_empty = bar + 72, v_full = bar + 88, v_empty = bar + 104;
+    volatile int *dead = reinterpret_cast<volatile int *>(flash_tc_smem + Z::bar_off + 120);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(flash_tc_smem + Z::bar_off + 124);
     if (warp == 5 && lane == 0) {
-        g_mbar_init(q_full, 1), g_mbar_init(p_full, 4), g_mbar_init(pv_done, 1);
+        g_mbar_init(q_full, 1);
+        // two of each, by the tile's parity: a warp hands its weights over without waiting for the last tile's product
+        for (int i = 0; i < 2; ++i) g_mbar_init(p_full + 8 * i, 4), g_mbar_init(pv_done + 8 * i, 1);
         for (int i = 0; i < 2; ++i) g_mbar_init(s_full + 8 * i, 1), g_mbar_init(k_full + 8 * i, 1), g_mbar_init(k_empty + 8 * i, 1);
         for (int i = 0; i < VST; ++i) g_mbar_init(v_full + 8 * i, 1), g_mbar_init(v_empty + 8 * i, 1);
         *dead = 0;
@@ -205,7 +207,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         scores(0);
         for (int t = 0; t < n_tiles; ++t) {
             if (t + 1 < n_tiles) scores(t + 1);  // its buffer held P_(t-1), read by a product already queued ahead of this one
-            tc_wait(p_full, t & 1, dead);
+            tc_wait(p_full + 8 * (t & 1), (t >> 1) & 1, dead);
             tc_wait(v_full + 8 * vs, vph, dead);
             g_tc_fence_after();
             if (g_elect_one()) {
@@ -213,7 +215,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 #pragma unroll
                 for (int k = 0; k < kXKeys / 16; ++k) g_tc_mma_ts(tmem + O, tmem + (t & 1) * kXKeys + 8 * k, vd + k * (2048 >> 4), idesc_o, t > 0 || k > 0);
                 g_tc_commit(v_empty + 8 * vs);
-                g_tc_commit(pv_done);
+                g_tc_commit(pv_done + 8 * (t & 1));
             }
             __syncwarp();
             if (++vs == VST) vs = 0, vph ^= 1u;
@@ -273,7 +275,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 top *= mult;
                 const bool grow = top > m + 8.0f || (m == -INFINITY && top != -INFINITY);
                 if (__any_sync(0xffffffffu, grow) && t > 0) {
-                    tc_wait(pv_done, (t - 1) & 1, dead);  // O has to be still while it is rescaled
+                    tc_wait(pv_done + 8 * ((t - 1) & 1), ((t - 1) >> 1) & 1, dead);  // O has to be still while it is rescaled
                     g_tc_fence_after();
                     const float to = grow ? top : m;
                     const float alpha = !grow ? 1.f : m == -INFINITY ? 0.f : x_ex2(m - to);
@@ -314,13 +316,11 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 tl::g_fence_proxy_async();
             }
             if (++vs == VST) vs = 0, vph ^= 1u;
-            // not before the last tile's product is done: a warp a whole tile ahead would arrive twice in one phase of p_full
-            if (t > 0) tc_wait(pv_done, (t - 1) & 1, dead);
             g_tc_fence_before();
             __syncwarp();
-            if (lane == 0) g_mbar_arrive(p_full);
+            if (lane == 0) g_mbar_arrive(p_full + 8 * (t & 1));
         }
-        tc_wait(pv_done, (n_tiles - 1) & 1, dead);
+        tc_wait(pv_done + 8 * ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, dead);
         g_tc_fence_after();
         float inv = sum > 0.f ? 1.0f / sum : 0.f;
         if (live && a.gate && !a.gate_wide) inv *= sigmoid(__bfloat162float(a.gate[(size_t)(first + tq) * a.g_token + head0 + hh]));
