@@ -901,6 +901,7 @@ int launch_paged_decode_tc(const void *q, const void *kp, const void *vp, const 
     const long long most = (static_cast<long long>(max_pages) * page_size + TC_BN - 1) / TC_BN * num_kv_heads * (rows / num_heads);
     if (pieces < 2 || most > (1LL << 30))  // no room for partial results, or more tiles than an int counts: a CTA per (request, head)
         return launch_paged_prefill_tc(q, kp, vp, bt, cl, out, rows, L, num_pages, page_size, max_pages, scale, is_causal, num_kv_heads, num_heads, st);
+    if (num_kv_heads > 65535 || rows / num_heads > 65535) return fail(TL_EINVAL, "paged_attention: too many heads / requests for one launch");
     DecodeTcArgs a{};
     a.block_table = bt, a.context_lens = cl, a.out = static_cast<bf16 *>(out);
     a.L = L, a.Hq = num_heads, a.Hkv = num_kv_heads, a.G = num_heads / num_kv_heads, a.requests = rows / num_heads;
