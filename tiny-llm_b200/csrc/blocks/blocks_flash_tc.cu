@@ -128,7 +128,11 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(flash_tc_smem + Z::bar_off + 124);
     if (warp == 5 && lane == 0) {
         g_mbar_init(q_full, 1);
-        // two of each, by the tile's parity: a warp hands its weights over without waiting for the last tile's product
+        // two of each, by the tile's parity: a warp hands its weights over without waiting for the last tile's product.  A wait by
+        // parity passes at once while its barrier is still in the phase BEFORE the one waited for, so a wait that is not made for
+        // every phase needs another reason why that phase is over.  S_t complete means that the products before it, P_(t-2) V_(t-2)
+        // among them, are (the tensor core takes them in order, and a commit covers all before it): enough for pv_done of tile
+        // t - 1, whose phase before is tile t - 3, not for v_full of a single stage (below).
         for (int i = 0; i < 2; ++i) g_mbar_init(p_full + 8 * i, 4), g_mbar_init(pv_done + 8 * i, 1);
         for (int i = 0; i < 2; ++i) g_mbar_init(s_full + 8 * i, 1), g_mbar_init(k_full + 8 * i, 1), g_mbar_init(k_empty + 8 * i, 1);
         for (int i = 0; i < VST; ++i) g_mbar_init(v_full + 8 * i, 1), g_mbar_init(v_empty + 8 * i, 1);
@@ -307,6 +311,11 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             g_tmem_st32(tmem + lanes + (t & 1) * kXKeys, pk);  // column c = keys 2 c and 2 c + 1
             g_tmem_st_wait();
             if (key0 + kXKeys - 1 > hi) {  // values past the newest key: cleared before the product may read them
+                // These warps wait on v_full here only, and a parity says nothing unless the phase before it is known to be over: with
+                // one stage that is V_(t-1), which may still be on its way when S_t is complete (nothing orders its load before K_t's).
+                // Its product is the proof that it landed and was read.  With two stages it is V_(t-2), whose product S_t follows.
+                if constexpr (VST == 1)
+                    if (t > 0) tc_wait(pv_done + 8 * ((t - 1) & 1), ((t - 1) >> 1) & 1, dead);
                 tc_wait(v_full + 8 * vs, vph, dead);
                 if (r < kXKeys && key0 + r > hi) {
 #pragma unroll
