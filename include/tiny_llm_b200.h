@@ -53,6 +53,9 @@ const char *tl_last_error(void);
 int tl_device_info(int *sm_count, int *cc_major, int *cc_minor);
 /* Number of kernels this library has launched since load (bench bookkeeping). */
 long long tl_launch_count(void);
+/* How many waits of tensor-core kernels have run into their limit (0 in a sound process; the rows concerned come out as NaN).
+ * Synchronises the device; -1 if it cannot be read. */
+long long tl_tc_gave_up(void);
 
 /* ---- W4A16 (4-bit, group 128) projections -------------------------------
  * Replaces quantized_matmul (tiny_llm_ext.h:12-21, quantized_matmul.cpp:14-80,

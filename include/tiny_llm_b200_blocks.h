@@ -314,8 +314,8 @@ int tlb_moe_gate_up(const void *h, const void *wg, const void *wu, int32_t *list
  * (token, choice) pair (rows_are_pairs = 1).  act 0 = silu, 1 = gelu (tanh form), 2 = squared relu. */
 int tlb_moe_up(const void *a, const void *wu, int32_t *lists, int tokens, int top, int experts, int dim, int ff, int act, int rows_are_pairs,
                void *inter, int dtype, void *stream);
-/* How many waits of tensor-core kernels have run into their limit (0 in a sound process; such a launch's results are wrong).
- * Synchronises the device. */
+/* How many waits of tensor-core kernels have run into their limit (0 in a sound process; the rows concerned come out as NaN).
+ * Synchronises the device; -1 if it cannot be read. */
 long long tlb_tc_gave_up(void);
 /* out[t * top + k, :] = gate[t, k] * h[t, :] rounded to `dtype`: inputs of experts whose weight multiplies the input. */
 int tlb_moe_scale_rows(const void *h, const float *gate, void *out, int tokens, int top, int dim, int dtype, void *stream);

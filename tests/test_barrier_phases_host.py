@@ -155,8 +155,8 @@ def test_prompt_attention(tiles, value_stages):
     source = KERNEL.read_text()
     clearing = source[source.index("values past the newest key: cleared") :]
     clearing = clearing[: clearing.index("g_fence_proxy_async")]
-    guard = value_stages == 1 and re.search(r"if constexpr \(VST == 1\)\s*if \(t > 0\) tc_wait\(pv_done \+ 8 \* \(\(t - 1\) & 1\), \(\(t - 1\) >> 1\) & 1, dead\);"
-                                            r"\s*tc_wait\(v_full", clearing) is not None
+    guard = value_stages == 1 and re.search(r"if constexpr \(VST == 1\)\s*if \(t > 0\b[^;]*tc_wait\(pv_done \+ 8 \* \(\(t - 1\) & 1\), \(\(t - 1\) >> 1\) & 1, dead\)[^;]*;"
+                                            r"[^;]*tc_wait\(v_full", clearing) is not None
     assert not early_waits(prompt_attention(tiles, value_stages, guard))
 
 

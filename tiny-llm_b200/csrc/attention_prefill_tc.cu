@@ -38,7 +38,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
-#include "tc05.cuh"
+#include "tc_wait.cuh"
 
 namespace tl {
 
@@ -480,23 +480,6 @@ struct DecodeWalk {
     }
 };
 
-// Bounded wait: past the limit the CTA is marked (which ends all its further waits) and its rows come out as NaN.
-__device__ __forceinline__ void dc_wait(uint32_t bar, uint32_t parity, volatile int *dead) {
-    for (uint32_t spins = 0;; ++spins) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done || *dead) return;
-        if (spins > (1u << 22)) {
-            *dead = 1;
-            return;
-        }
-    }
-}
-
 template <int SW>  // softmax warps: rows / 32
 struct DecodeTcShape {
     static constexpr int q_half = SW * 32 * 128, q_stages = SW == 1 ? 2 : 1, stages = SW == 1 ? 3 : 2;
@@ -569,7 +552,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         int s = 0, qs = 0;
         uint32_t ph = 1, qph = 1;  // producer side: the first pass through a ring does not wait
         do {
-            dc_wait(q_empty + 8 * qs, qph, dead);
+            if (!tc_wait(q_empty + 8 * qs, qph, dead)) goto out;
             if (g_elect_one()) {
                 const int head0 = w.b * a.Hq + w.kvh * a.G;
                 const uint32_t q_at = q_base + qs * 2 * Z::q_half;
@@ -584,14 +567,14 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 const int lp = t / a.tiles_per_page, slot0 = (t - lp * a.tiles_per_page) * TC_BN;
                 int pid = table[lp];
                 if (pid < 0 || pid >= a.num_pages) pid = a.num_pages;  // outside the tensor: the TMA unit writes zeros
-                dc_wait(k_empty + 8 * s, ph, dead);
+                if (!tc_wait(k_empty + 8 * s, ph, dead)) goto out;
                 if (g_elect_one()) {
                     g_mbar_expect_tx(k_full + 8 * s, TC_KV_TILE);
                     g_tma_load_4d(k_base + s * TC_KV_TILE, &tmap_k, 0, slot0, w.kvh, pid, k_full + 8 * s);
                     g_tma_load_4d(k_base + s * TC_KV_TILE + TC_KV_TILE / 2, &tmap_k, 64, slot0, w.kvh, pid, k_full + 8 * s);
                 }
                 __syncwarp();
-                dc_wait(v_empty + 8 * s, ph, dead);
+                if (!tc_wait(v_empty + 8 * s, ph, dead)) goto out;
                 if (g_elect_one()) {
                     g_mbar_expect_tx(v_full + 8 * s, TC_KV_TILE);
                     g_tma_load_4d(v_base + s * TC_KV_TILE, &tmap_v, 0, slot0, w.kvh, pid, v_full + 8 * s);
@@ -611,9 +594,9 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         uint32_t kph = 0, vph = 0, qph = 0;
         bool fresh = true, more = true;
         auto issue_scores = [&](int j) {
-            if (fresh) dc_wait(q_full + 8 * qs, qph, dead);
+            if (fresh && !tc_wait(q_full + 8 * qs, qph, dead)) return false;
             fresh = false;
-            dc_wait(k_full + 8 * ks, kph, dead);
+            if (!tc_wait(k_full + 8 * ks, kph, dead)) return false;
             g_tc_fence_after();
             const bool last = --left == 0;
             if (g_elect_one()) {
@@ -633,14 +616,14 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 if (++qs == Z::q_stages) qs = 0, qph ^= 1u;
                 more = ahead.next(a), left = ahead.n, fresh = true;
             }
+            return true;
         };
-        issue_scores(0);
+        if (!issue_scores(0)) goto out;
         for (int j = 0; j < share; ++j) {
             // score buffer (j+1)&1 was last read for tile j-1, whose P has been waited for below
-            if (more) issue_scores(j + 1);
+            if (more && !issue_scores(j + 1)) goto out;
             // a new stretch's first product overwrites O: the softmax warps arrive for it after they have read the old one
-            dc_wait(p_full + 8 * (j & 1), (j >> 1) & 1, dead);
-            dc_wait(v_full + 8 * vs, vph, dead);
+            if (!tc_wait(p_full + 8 * (j & 1), (j >> 1) & 1, dead) || !tc_wait(v_full + 8 * vs, vph, dead)) goto out;
             g_tc_fence_after();
             if (g_elect_one()) {
                 const uint64_t vd = vdesc0 + static_cast<uint64_t>(vs * (TC_KV_TILE >> 4));
@@ -664,10 +647,11 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             const int limit = r >= rows ? -1 : (a.is_causal ? min(ctx - 1, l + (ctx - a.L)) : ctx - 1);  // the last key this row may see
             const int32_t *table = a.block_table + static_cast<size_t>(w.b) * a.max_pages;
             float m_used = -CUDART_INF_F, l_sum = 0.f;
+            bool ok = true;
             for (int i = 0; i < w.n; ++i, ++j) {
                 const int pid = table[(w.t0 + i) / a.tiles_per_page];
                 const int visible = pid >= 0 && pid < a.num_pages ? min(limit - (w.t0 + i) * TC_BN + 1, TC_BN) : 0;  // keys [0, visible) of the tile
-                dc_wait(s_full + 8 * (j & 1), (j >> 1) & 1, dead);
+                if (!(ok = tc_wait(s_full + 8 * (j & 1), (j >> 1) & 1, dead))) break;
                 g_tc_fence_after();
                 uint32_t sv[2][32];
                 g_tmem_ld32_nowait(tmem + lane_base + (j & 1) * TC_BN, sv[0]);
@@ -684,7 +668,7 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 // lazy rescale: keep the stale maximum unless this tile exceeds it by more than 2^8
                 const bool grow = tile_max > m_used + TC_RESCALE_THRESHOLD || (m_used == -CUDART_INF_F && tile_max != -CUDART_INF_F);
                 if (__any_sync(0xffffffffu, grow) && i > 0) {
-                    dc_wait(pv_done + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, dead);  // O must be stable while it is rescaled
+                    if (!(ok = tc_wait(pv_done + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, dead))) break;  // O must be stable while it is rescaled
                     g_tc_fence_after();
                     const float m_new = grow ? tile_max : m_used;
                     const float alpha = (grow && m_used != -CUDART_INF_F) ? exp2f(m_used - m_new) : (grow ? 0.f : 1.f);
@@ -719,11 +703,11 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 __syncwarp();
                 if (lane == 0) g_mbar_arrive(p_full + 8 * (j & 1));
             }
-            dc_wait(pv_done + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, dead);
+            ok = ok && tc_wait(pv_done + 8 * ((j - 1) & 1), ((j - 1) >> 1) & 1, dead);
             g_tc_fence_after();
             const size_t out_row = static_cast<size_t>(w.b * a.Hq + w.kvh * a.G + g) * a.L + l;
             const bool whole = w.n == w.tiles;
-            const float inv = whole ? (l_sum == 0.f ? 0.f : 1.0f / l_sum) : 1.f, bad = *dead ? CUDART_NAN_F : 1.f;
+            const float inv = whole ? (l_sum == 0.f ? 0.f : 1.0f / l_sum) : 1.f, bad = tc_verdict(ok, dead);
             const size_t slot = out_row * a.max_pieces + (whole ? 0 : blockIdx.x - (w.base + w.kvh * w.tiles) / deal.per);
 #pragma unroll
             for (int cb = 0; cb < TC_D / 32; ++cb) {
@@ -749,11 +733,11 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             if (!whole && r < rows) a.ws_m[slot] = m_used == -CUDART_INF_F ? -1e30f : m_used, a.ws_l[slot] = l_sum * bad;
         } while (w.next(a));
     }
+out:  // also from a role whose wait gave up
     g_tc_fence_before();
     __syncthreads();
     if (warp == 0) {
-        if (*dead)
-            for (int i = 0; i < 2000; ++i) __nanosleep(1000);  // copies in flight land first
+        tc_settle(dead);
         g_tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TC_TMEM_COLS) : "memory");
     }
@@ -837,6 +821,8 @@ static int cached_map(CUtensorMap *out, const void *ptr, int rank, const cuuint6
     *out = map;
     return TL_OK;
 }
+
+long long decode_tc_gave_up() { return read_gave_up(); }
 
 bool paged_prefill_tc_supported(int L, int num_pages, int page_size, int num_kv_heads, int num_heads) {
     static const bool off = [] { const char *e = getenv("TL_PREFILL_TC"); return e != nullptr && e[0] == '0'; }();

@@ -166,7 +166,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         for (int t = 0; t < n_tiles; ++t) {
             const int key = tile_key(t), page = table[key / a.page_size];
             const int row = (page >= 0 && page < a.num_pages ? page : a.num_pages) * a.page_size + key % a.page_size;  // past the last page: zeros
-            tc_wait(k_empty + 8 * ks, kph, dead);
+            if (!tc_wait(k_empty + 8 * ks, kph, dead)) break;
             if (g_elect_one()) {
                 g_mbar_expect_tx(k_full + 8 * ks, KB * Z::kv_block);
 #pragma unroll
@@ -178,7 +178,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             }
             __syncwarp();
             if (++ks == 2) ks = 0, kph ^= 1u;
-            tc_wait(v_empty + 8 * vs, vph, dead);
+            if (!tc_wait(v_empty + 8 * vs, vph, dead)) break;
             if (g_elect_one()) {
                 g_mbar_expect_tx(v_full + 8 * vs, VB * Z::kv_block);
 #pragma unroll
@@ -193,7 +193,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         int ks = 0, vs = 0;
         uint32_t kph = 0, vph = 0;
         auto scores = [&](int t) {
-            tc_wait(k_full + 8 * ks, kph, dead);
+            if (!tc_wait(k_full + 8 * ks, kph, dead)) return false;
             g_tc_fence_after();
             if (g_elect_one()) {
                 const uint64_t kd = kd0 + (uint64_t)(ks * KB * (Z::kv_block >> 4));
@@ -206,13 +206,12 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             }
             __syncwarp();
             if (++ks == 2) ks = 0, kph ^= 1u;
+            return true;
         };
-        tc_wait(q_full, 0, dead);
-        scores(0);
-        for (int t = 0; t < n_tiles; ++t) {
-            if (t + 1 < n_tiles) scores(t + 1);  // its buffer held P_(t-1), read by a product already queued ahead of this one
-            tc_wait(p_full + 8 * (t & 1), (t >> 1) & 1, dead);
-            tc_wait(v_full + 8 * vs, vph, dead);
+        const bool begun = tc_wait(q_full, 0, dead) && scores(0);
+        for (int t = 0; begun && t < n_tiles; ++t) {
+            if (t + 1 < n_tiles && !scores(t + 1)) break;  // its buffer held P_(t-1), read by a product already queued ahead of this one
+            if (!tc_wait(p_full + 8 * (t & 1), (t >> 1) & 1, dead) || !tc_wait(v_full + 8 * vs, vph, dead)) break;
             g_tc_fence_after();
             if (g_elect_one()) {
                 const uint64_t vd = vd0 + (uint64_t)(vs * VB * (Z::kv_block >> 4));
@@ -242,9 +241,10 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         float sum = a.sink || a.weights == 1 ? 1.f : 0.f;                 // the sink's term (m is its score), or the sigmoid form's constant
         int vs = 0;
         uint32_t vph = 0;
+        bool ok = true;
         for (int t = 0; t < n_tiles; ++t) {
             const int key0 = tile_key(t);
-            tc_wait(s_full + 8 * (t & 1), (t >> 1) & 1, dead);
+            if (!(ok = tc_wait(s_full + 8 * (t & 1), (t >> 1) & 1, dead))) break;
             g_tc_fence_after();
             uint32_t s[2][32];
             g_tmem_ld32_nowait(tmem + lanes + (t & 1) * kXKeys, s[0]);
@@ -279,7 +279,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 top *= mult;
                 const bool grow = top > m + 8.0f || (m == -INFINITY && top != -INFINITY);
                 if (__any_sync(0xffffffffu, grow) && t > 0) {
-                    tc_wait(pv_done + 8 * ((t - 1) & 1), ((t - 1) >> 1) & 1, dead);  // O has to be still while it is rescaled
+                    if (!(ok = tc_wait(pv_done + 8 * ((t - 1) & 1), ((t - 1) >> 1) & 1, dead))) break;  // O has to be still while it is rescaled
                     g_tc_fence_after();
                     const float to = grow ? top : m;
                     const float alpha = !grow ? 1.f : m == -INFINITY ? 0.f : x_ex2(m - to);
@@ -315,8 +315,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 // one stage that is V_(t-1), which may still be on its way when S_t is complete (nothing orders its load before K_t's).
                 // Its product is the proof that it landed and was read.  With two stages it is V_(t-2), whose product S_t follows.
                 if constexpr (VST == 1)
-                    if (t > 0) tc_wait(pv_done + 8 * ((t - 1) & 1), ((t - 1) >> 1) & 1, dead);
-                tc_wait(v_full + 8 * vs, vph, dead);
+                    if (t > 0 && !(ok = tc_wait(pv_done + 8 * ((t - 1) & 1), ((t - 1) >> 1) & 1, dead))) break;
+                if (!(ok = tc_wait(v_full + 8 * vs, vph, dead))) break;
                 if (r < kXKeys && key0 + r > hi) {
 #pragma unroll
                     for (int i = 0; i < VB * 8; ++i)
@@ -329,9 +329,9 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             __syncwarp();
             if (lane == 0) g_mbar_arrive(p_full + 8 * (t & 1));
         }
-        tc_wait(pv_done + 8 * ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, dead);
+        ok = ok && tc_wait(pv_done + 8 * ((n_tiles - 1) & 1), ((n_tiles - 1) >> 1) & 1, dead);
         g_tc_fence_after();
-        float inv = sum > 0.f ? 1.0f / sum : 0.f;
+        float inv = (sum > 0.f ? 1.0f / sum : 0.f) * tc_verdict(ok, dead);
         if (live && a.gate && !a.gate_wide) inv *= sigmoid(__bfloat162float(a.gate[(size_t)(first + tq) * a.g_token + head0 + hh]));
         bf16 *out = a.out + (size_t)(first + tq) * a.o_token + (size_t)(head0 + hh) * a.o_head;
         const bf16 *wide = a.gate_wide ? a.gate + (size_t)(first + tq) * a.g_token + (size_t)(head0 + hh) * a.dv : nullptr;
@@ -440,7 +440,7 @@ latent_rows_kernel(const bf16 *__restrict__ slab, int num_pages, int page_size, 
     }
 }
 
-long long flash_tc_gave_up() { return tc_read_gave_up(); }
+long long flash_tc_gave_up() { return tl::read_gave_up(); }
 
 static bool map_ok(const void *p, long long s0, long long s1) { return tl::aligned16(p) && s0 % 8 == 0 && s1 % 8 == 0; }
 

@@ -87,7 +87,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
             const int mb = tile % a.m_blocks, cols = (c.z + 15) & ~15;
             const int r0 = c.x * a.n + mb * (gated ? 128 : 256), r1 = gated ? r0 : r0 + 128;
             for (int kb = 0; kb < a.k_blocks; ++kb) {
-                tc_wait(empty + 8 * s, ph, dead);
+                if (!tc_wait(empty + 8 * s, ph, dead)) goto out;
                 if (g_elect_one()) {
                     const uint32_t at = base + s * a.stage_bytes;
                     g_mbar_expect_tx(full + 8 * s, 2 * kTcBlockBytes + (gathers ? 0 : cols * 128));
@@ -104,7 +104,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
         for (int tile = blockIdx.x; !gathers && tile < tiles; tile += gridDim.x) {
             const int4 c = a.chunks[tile / a.m_blocks];
             for (int kb = 0; kb < a.k_blocks; ++kb) {
-                tc_wait(empty + 8 * s, ph, dead);
+                if (!tc_wait(empty + 8 * s, ph, dead)) goto out;
                 if (lane * 16 < c.z) g_tma_load_2d(base + s * a.stage_bytes + 2 * kTcBlockBytes + lane * 16 * 128, &map_x, kb * 64, c.y + lane * 16, full + 8 * s);
                 __syncwarp();
                 if (++s == a.stages) s = 0, ph ^= 1u;
@@ -127,7 +127,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
 #pragma unroll
             for (int j = 0; j < 16; ++j) src[j] = r0 + 16 * j < c.z ? moe_src_row(a.sorted_pair[c.y + r0 + 16 * j], 0, a.top, a.gather) : -1;
             for (int kb = 0; kb < a.k_blocks; ++kb) {
-                tc_wait(empty + 8 * s, ph, dead);
+                if (!tc_wait(empty + 8 * s, ph, dead)) goto out;
                 const uint32_t at = base + s * a.stage_bytes + to;
                 const int k = kb * 64 + piece * 8;
 #pragma unroll
@@ -156,15 +156,15 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
             const bool whole = cols > 128;  // both halves of tensor memory
             if (whole) buf = 0;
             const uint32_t d0 = tmem + buf * 256, d1 = d0 + (whole ? 256 : 128), idesc = tc_idesc(cols);
-            tc_wait(acc_empty + 8 * buf, acc_ph[buf], dead);
+            if (!tc_wait(acc_empty + 8 * buf, acc_ph[buf], dead)) goto out;
             acc_ph[buf] ^= 1u;
             if (whole) {
-                tc_wait(acc_empty + 8, acc_ph[1], dead);
+                if (!tc_wait(acc_empty + 8, acc_ph[1], dead)) goto out;
                 acc_ph[1] ^= 1u;
             }
             g_tc_fence_after();
             for (int kb = 0; kb < a.k_blocks; ++kb) {
-                tc_wait(full + 8 * s, ph, dead);
+                if (!tc_wait(full + 8 * s, ph, dead)) goto out;
                 g_tc_fence_after();
                 if (g_elect_one()) {
                     const uint32_t at = base + s * a.stage_bytes;
@@ -196,7 +196,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
             if (whole) buf = 0;
             const uint32_t d0 = tmem + lanes + buf * 256, d1 = d0 + (whole ? 256 : 128);
             const int f0 = mb * (gated ? 128 : 256) + quarter * 32 + lane, f1 = f0 + 128;
-            tc_wait(acc_full + 8 * buf, acc_ph[buf], dead);
+            const bool ok = tc_wait(acc_full + 8 * buf, acc_ph[buf], dead);
+            const float bad = tc_verdict(ok, dead);  // of a marked CTA this tile and all that follow are stored as NaN
             acc_ph[buf] ^= 1u;
             g_tc_fence_after();
             const int begin = half * (cols / 2), end = min(begin + cols / 2, c.z);
@@ -211,15 +212,15 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
                     for (int i = 0; i < 8; ++i) {
                         if (i >= here) break;
                         float *o = a.pair_out + (size_t)a.sorted_pair[row + i] * a.n;
-                        if (f0 < a.n) o[f0] = __uint_as_float(u[i]);
-                        if (f1 < a.n) o[f1] = __uint_as_float(v[i]);
+                        if (f0 < a.n) o[f0] = __uint_as_float(u[i]) * bad;
+                        if (f1 < a.n) o[f1] = __uint_as_float(v[i]) * bad;
                     }
                 } else if (gated) {
                     if (f0 < a.n) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
                             if (i < here)
-                                a.inter[(size_t)(row + i) * a.n + f0] = __float2bfloat16_rn(gated_pair(__uint_as_float(u[i]), __uint_as_float(v[i]), a.act, a.limit, a.slope));
+                                a.inter[(size_t)(row + i) * a.n + f0] = __float2bfloat16_rn(gated_pair(__uint_as_float(u[i]), __uint_as_float(v[i]), a.act, a.limit, a.slope) * bad);
                     }
                 } else {
                     auto act = [&](float z) { return a.act == 2 ? (z > 0.f ? z * z : 0.f) : act_apply(z, a.act); };
@@ -227,8 +228,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
                     for (int i = 0; i < 8; ++i) {
                         if (i >= here) break;
                         bf16 *o = a.inter + (size_t)(row + i) * a.n;
-                        if (f0 < a.n) o[f0] = __float2bfloat16_rn(act(__uint_as_float(u[i])));
-                        if (f1 < a.n) o[f1] = __float2bfloat16_rn(act(__uint_as_float(v[i])));
+                        if (f0 < a.n) o[f0] = __float2bfloat16_rn(act(__uint_as_float(u[i])) * bad);
+                        if (f1 < a.n) o[f1] = __float2bfloat16_rn(act(__uint_as_float(v[i])) * bad);
                     }
                 }
             }
@@ -241,6 +242,8 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
             buf = whole ? 0 : buf ^ 1;
         }
     }
+out:  // also from a role whose wait gave up
+    asm volatile("cp.async.wait_all;" ::: "memory");
     g_tc_fence_before();
     __syncthreads();
     if (warp == 3) {
@@ -393,6 +396,9 @@ int tlb_moe_sort(const int32_t *idx, int tokens, int top, int experts, int32_t *
     return TL_OK;
 }
 
-long long tlb_tc_gave_up(void) { return tc_read_gave_up() + flash_tc_gave_up(); }
+long long tlb_tc_gave_up(void) {
+    const long long experts = tl::read_gave_up(), attention = flash_tc_gave_up();
+    return experts < 0 || attention < 0 ? -1 : experts + attention;
+}
 
 }  // extern "C"

@@ -1,7 +1,7 @@
-// What the tcgen05 kernels of the blocks library share beside tc05.cuh: waits that give up, tensor maps, descriptors.
+// What the tcgen05 kernels of the blocks library share beside tc05.cuh and tc_wait.cuh: tensor maps, descriptors.
 #pragma once
 
-#include "../tc05.cuh"
+#include "../tc_wait.cuh"
 #include "blocks_common.cuh"
 
 namespace tlb {
@@ -19,40 +19,11 @@ using tl::g_tc_mma;
 using tl::g_tc_mma_ts;
 using tl::g_tma_load_2d;
 
-// Every wait is bounded: past the limit the CTA is marked as given up (its own flag in shared memory, which ends all further
-// waits at once), so that a lost arrival ends in wrong numbers and a counter that the host can read, never in a hung GPU.
-static __device__ unsigned int g_tc_gave_up;
-
-static inline long long tc_read_gave_up() {
-    unsigned int n = 0;
-    return cudaMemcpyFromSymbol(&n, g_tc_gave_up, sizeof(n)) == cudaSuccess ? (long long)n : -1;
-}
+using tl::tc_settle;
+using tl::tc_verdict;
+using tl::tc_wait;
 
 long long flash_tc_gave_up();  // of the attention kernels
-
-__device__ __forceinline__ void tc_wait(uint32_t bar, uint32_t parity, volatile int *dead) {
-    for (uint32_t spins = 0;; ++spins) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done || *dead) return;
-        if (spins > (1u << 22)) {
-            *dead = 1;
-            atomicAdd(&g_tc_gave_up, 1u);
-            return;
-        }
-    }
-}
-
-// The last thing before a CTA frees its tensor memory: all warps are past their loops.  One that gave up leaves its copies in
-// flight some time to land first.
-__device__ __forceinline__ void tc_settle(volatile int *dead) {
-    if (*dead)
-        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-}
 
 // kind::f16 instruction descriptor: bf16 x bf16 -> f32, 128 rows, n columns; A K-major, B K-major or (b_mn) MN-major.
 __host__ __device__ __forceinline__ constexpr uint32_t tc_idesc(int n, bool b_mn = false) {

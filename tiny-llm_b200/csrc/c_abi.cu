@@ -59,6 +59,7 @@ int tl_abi_version(void) { return 1; }
 const char *tl_last_error(void) { return g_error; }
 
 long long tl_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
+long long tl_tc_gave_up(void) { return decode_tc_gave_up(); }
 
 int tl_device_info(int *sms, int *major, int *minor) {
     int dev = 0;

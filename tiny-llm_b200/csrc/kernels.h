@@ -109,6 +109,7 @@ int launch_paged_decode(const void *q, const void *kp, const void *vp, const int
                         cudaStream_t st);
 
 // attention_prefill_tc.cu (tcgen05 + TMA flash prefill; page_size % 64 == 0, Hq/Hkv divides 128)
+long long decode_tc_gave_up();
 bool paged_prefill_tc_supported(int L, int num_pages, int page_size, int num_kv_heads, int num_heads);
 int launch_paged_prefill_tc(const void *q, const void *kp, const void *vp, const int32_t *bt, const int32_t *cl, void *out, int rows,
                             int L, int num_pages, int page_size, int max_pages, float scale, int is_causal, int num_kv_heads,

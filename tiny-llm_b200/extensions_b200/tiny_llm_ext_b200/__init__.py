@@ -20,6 +20,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sys
 from pathlib import Path
 
 import torch
@@ -45,6 +46,7 @@ __all__ = [
     "set_pdl",
     "set_gemm_pairs",
     "launch_count",
+    "waits_given_up",
     "device_info",
     "current_library_path",
     "quantized_matmul_residual_norm",
@@ -96,6 +98,7 @@ _SIGNATURES = {
     "tl_paged_cache_append_chunk": (_I, [_VP] * 5 + [_I] * 4 + [ctypes.c_longlong, ctypes.c_longlong, _I, _VP]),
     "tl_set_pdl": (_I, [_I]),
     "tl_set_gemm_pairs": (_I, [_I]),
+    "tl_tc_gave_up": (ctypes.c_longlong, []),
 }
 
 EXPORTED_SYMBOLS = tuple(_SIGNATURES)
@@ -822,6 +825,18 @@ def set_gemm_pairs(mode: int) -> None:
 
 def launch_count() -> int:
     return int(_lib.tl_launch_count())
+
+
+def waits_given_up() -> int:
+    """How many waits of tensor-core kernels have run into their limit on the current device, in the libraries this process has loaded:
+    0 in a sound process; the rows such a launch left unfinished are NaN.  Synchronises the device."""
+    counts = [_lib.tl_tc_gave_up()] if _lib is not None else []
+    blocks = sys.modules.get(f"{__name__}.blocks")
+    if blocks is not None and blocks._lib is not None:
+        counts.append(blocks._lib.tlb_tc_gave_up())
+    if any(n < 0 for n in counts):
+        raise RuntimeError("waits_given_up: the device's counters cannot be read")
+    return sum(counts)
 
 
 def device_info() -> tuple[int, int, int]:

@@ -47,6 +47,10 @@ def _step(model, y, offsets, kv_cache):
     return greedy_tokens(logits[:, -1, :])
 
 
+def _waits_given_up() -> int:
+    return tiny_llm_ext_b200.waits_given_up() if torch.cuda.is_initialized() else 0
+
+
 class _TokenLog:
     """Detokenizer stand-in for token-id workloads (no tokenizer): keeps ids."""
 
@@ -198,6 +202,7 @@ class ContinuousBatcher:
         self.kv_cache = [BatchingKvCache(max_active_requests=batch_size, max_seq_len=max_seq_len) for _ in range(model.num_hidden_layers)]
         self.pending: Request | None = None
         self.results: list[tuple[int, str]] = []
+        self._given_up = _waits_given_up()
         self.next_request_idx = 0
         self.tick = 0
         self.started = datetime.now()
@@ -256,6 +261,13 @@ class ContinuousBatcher:
             return False
         return self.generated.get(request.prompt_idx, 0) >= self.max_new_tokens[request.prompt_idx]
 
+    def _deliver(self, request: Request, text: str) -> None:
+        """Hand a finished request's text over, unless a kernel's wait has run into its limit since this batcher began: what it left
+        unfinished is NaN, and tokens chosen from that are no answer.  Once a request, when its tokens have been read anyway."""
+        if _waits_given_up() > self._given_up:
+            raise RuntimeError("a tensor-core kernel gave up waiting: the running requests' numbers are not to be trusted")
+        self.results.append((request.prompt_idx, text))
+
     # -- one scheduler iteration ----------------------------------------------
     def _retire_or_seat(self, request: Request) -> bool:
         """A request whose prompt is consumed either ends (done, length or budget) or takes the first idle slot."""
@@ -263,7 +275,7 @@ class ContinuousBatcher:
             text = request.text()
             for layer_cache in request.kv_cache:
                 layer_cache.release()
-            self.results.append((request.prompt_idx, text))
+            self._deliver(request, text)
             self.pending = None
             return True
         for i in range(self.batch_size):
@@ -293,7 +305,7 @@ class ContinuousBatcher:
             text = request.text()
             for table in self.kv_cache:
                 table.remove_request(i)
-            self.results.append((request.prompt_idx, text))
+            self._deliver(request, text)
             self.slots[i] = None
 
     def _step_mixed(self) -> None:
@@ -381,7 +393,7 @@ class ContinuousBatcher:
                     text = request.text()
                     for layer_cache in request.kv_cache:
                         layer_cache.release()
-                    self.results.append((request.prompt_idx, text))
+                    self._deliver(request, text)
                     self.pending = None
                     moved = True
                 else:
@@ -430,7 +442,7 @@ class ContinuousBatcher:
                     text = request.text()
                     for table in self.kv_cache:
                         table.remove_request(i)
-                    self.results.append((request.prompt_idx, text))
+                    self._deliver(request, text)
                     self.slots[i] = None
             self._progress()
 
