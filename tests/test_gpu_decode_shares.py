@@ -69,3 +69,50 @@ def test_bad_entries_and_lengths_that_change_under_a_captured_launch():
         n.copy_(torch.tensor(lens))
         graph.replay()
         check(held, q, k, v, table, n, 16, 4, 1, True)
+
+
+@pytest.mark.parametrize("lens,heads,kv,L,rows", [
+    ([2000] * 32, 32, 8, 1, (32, 64, 100)),  # every (request, head) on its own
+    ([5000] + [70] * 15, 32, 8, 1, (16, 32, 64)), ([200 + 331 * i % 2900 for i in range(20)], 16, 4, 1, (20, 48)), ([1100, 3, 900], 16, 2, 4, (3, 16)),
+    ([700] * 37, 8, 8, 1, (37, 64)),
+])
+def test_idle_slots_leave_the_bits_alone(lens, heads, kv, L, rows):
+    q, k, v, table, n = inputs(lens + [0] * (max(rows) - len(lens)), heads, kv, L)
+    call = lambda r: ext.paged_attention(q[: r * heads], k, v, table[:r], n[:r], scale=128**-0.5, is_causal=True, num_heads=heads, num_kv_heads=kv)[: len(lens) * heads]
+    first = call(rows[0])
+    check(first, q, k, v, table, n[: len(lens)], heads, kv, L, True)
+    assert all(torch.equal(first, call(r)) for r in rows[1:])
+
+
+def test_row_variants_of_an_engine_with_long_tables(monkeypatch):
+    """64 slots of up to 1024 keys on 128-slot pages, one request long: the graphs over 16 and over all rows give the same bits."""
+    from tiny_llm_b200 import Qwen3ModelWeek3
+    from tiny_llm_b200.engine import DecodeEngine
+    from tiny_llm_b200.kv_cache import BatchingKvCache
+    from tiny_llm_b200.synthetic import synthetic_qwen3, to_device
+
+    dev, B = torch.device("cuda:0"), 64
+    ns = to_device(synthetic_qwen3("tiny-d128", seed=5, realistic=True, max_position_embeddings=2048), dev)
+    prompts = {b: [3 + (11 * b + j) % 400 for j in range(800 if b == 2 else 4 + b)] for b in (0, 1, 2, 5, 9)}
+
+    def run(variants):
+        monkeypatch.setenv("TL_ROW_VARIANTS", variants)
+        model = Qwen3ModelWeek3(ns, page_size=PAGE)
+        engine = DecodeEngine(model, B, 1024, dev)
+        engine.reserve_pools()
+        tables = [BatchingKvCache(max_active_requests=B, max_seq_len=1024) for _ in range(model.num_hidden_layers)]
+        for b, prompt in prompts.items():
+            cache = model.create_kv_cache()
+            model(torch.tensor([prompt], dtype=torch.int32, device=dev), 0, cache, logits_to_keep=1)
+            for layer_cache, table in zip(cache, tables):
+                table.add_request(layer_cache, b)
+        outs = []
+        for step in range(2):
+            logits, _ = engine.step([7 + b + step if b in prompts else 0 for b in range(B)], [len(prompts[b]) + step if b in prompts else 0 for b in range(B)], tables)
+            outs.append(logits[list(prompts)].clone())
+        assert not engine._attention_fused
+        return outs, engine.variant_replays
+
+    narrow, replays = run("1")
+    assert replays[16] == 2
+    assert all(torch.equal(a, b) for a, b in zip(narrow, run("0")[0]))

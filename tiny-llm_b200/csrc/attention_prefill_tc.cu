@@ -399,7 +399,7 @@ struct DecodeTcArgs {
     int page_size, max_pages, num_pages, tiles_per_page;
     float scale_log2;
     int is_causal;
-    int ctas, max_pieces;  // of the attention launch; pieces of a (request, head) that the workspace has room for (>= 2)
+    int slots, max_pieces;  // CTAs the GPU holds at a time; pieces of a (request, head) that the workspace has room for (>= 2)
     float *ws_o, *ws_m, *ws_l;
 };
 constexpr int DC_MIN_TILES = 4;  // of a share: below it a CTA's fixed cost (set-up, queries, first tile: 3 to 4 us) outweighs what it saves
@@ -410,14 +410,15 @@ __device__ __forceinline__ int dc_tiles(const DecodeTcArgs &a, int r) { return (
 // The tiles of all heads of all requests, those before `request` and the tiles of a share; called by whole warps.  Where every
 // (request, head) can have a CTA and the longest is within a quarter of an equal share, per is 0 and each keeps to its own: the launch is
 // bound by HBM then, and cutting only adds partial results (32 requests of 2000 tokens, 8 heads: 49 us cut, 45 whole; of 7200: 151 and 143).
+// Nothing here depends on how many requests of length 0 the launch has, so a step over more idle slots cuts the same way, to the bit.
 struct DecodeDeal {
     int total, before, per;
 };
 __device__ __forceinline__ DecodeDeal dc_deal(const DecodeTcArgs &a, int request) {
-    int total = 0, before = 0, longest = 0;
+    int total = 0, before = 0, longest = 0, live = 0;
     for (int r = threadIdx.x & 31; r < a.requests; r += 32) {
         const int n = dc_tiles(a, r);
-        total += n, longest = max(longest, n);
+        total += n, longest = max(longest, n), live += n > 0;
         if (r < request) before += n;
     }
 #pragma unroll
@@ -425,12 +426,24 @@ __device__ __forceinline__ DecodeDeal dc_deal(const DecodeTcArgs &a, int request
         total += __shfl_xor_sync(0xffffffffu, total, o);
         before += __shfl_xor_sync(0xffffffffu, before, o);
         longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+        live += __shfl_xor_sync(0xffffffffu, live, o);
     }
     total *= a.Hkv, before *= a.Hkv;
     // n tiles touch at most ceil(n / per) + 1 shares
-    if (a.requests * a.Hkv <= a.ctas && static_cast<long long>(longest) * 4 * a.ctas <= 5LL * total) return {total, before, 0};
-    const int per = max(max((total + a.ctas - 1) / a.ctas, (longest + a.max_pieces - 2) / (a.max_pieces - 1)), DC_MIN_TILES);
+    if (static_cast<long long>(live) * a.Hkv <= a.slots && static_cast<long long>(longest) * 4 * a.slots <= 5LL * total) return {total, before, 0};
+    const int per = max(max((total + a.slots - 1) / a.slots, (longest + a.max_pieces - 2) / (a.max_pieces - 1)), DC_MIN_TILES);
     return {total, before, per};
+}
+
+// The rank-th request that has keys, -1 past the last; whole warps.
+__device__ __forceinline__ int dc_live(const DecodeTcArgs &a, int rank) {
+    for (int r0 = 0; r0 < a.requests; r0 += 32) {
+        const int r = r0 + (threadIdx.x & 31);
+        const unsigned live = __ballot_sync(0xffffffffu, r < a.requests && dc_tiles(a, r) > 0);
+        if (rank < __popc(live)) return r0 + static_cast<int>(__fns(live, 0, rank + 1));
+        rank -= __popc(live);
+    }
+    return -1;
 }
 
 // A share's walk over the (request, key/value head) pairs it touches.  Every role of the CTA walks it by itself.
@@ -501,12 +514,12 @@ paged_decode_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     const DecodeDeal deal = dc_deal(a, 0);
     DecodeWalk w;
     const bool own = deal.per == 0;
-    const int request = own ? blockIdx.x / a.Hkv : 0, alone = own && request < a.requests ? dc_tiles(a, request) : 0;
-    if (own ? alone == 0 : static_cast<long long>(blockIdx.x) * deal.per >= deal.total) {
+    const int request = own ? dc_live(a, blockIdx.x / a.Hkv) : 0;
+    if (own ? request < 0 : static_cast<long long>(blockIdx.x) * deal.per >= deal.total) {
         griddep_wait();  // also without work: what follows relies on this launch ending after the one before it
         return;
     }
-    if (own) w.own(request, blockIdx.x - request * a.Hkv, alone);
+    if (own) w.own(request, blockIdx.x % a.Hkv, dc_tiles(a, request));
     else w.start(a, blockIdx.x * deal.per, min((blockIdx.x + 1) * deal.per, deal.total));
     const int share = w.end - w.pos;
     const int rows = a.G * a.L;
@@ -893,7 +906,10 @@ int launch_paged_decode_tc(const void *q, const void *kp, const void *vp, const 
     a.L = L, a.Hq = num_heads, a.Hkv = num_kv_heads, a.G = num_heads / num_kv_heads, a.requests = rows / num_heads;
     a.page_size = page_size, a.max_pages = max_pages, a.num_pages = num_pages, a.tiles_per_page = page_size / TC_BN;
     a.scale_log2 = scale * TC_LOG2E, a.is_causal = is_causal;
-    a.ctas = static_cast<int>(std::max(1LL, std::min(2LL * sm_count(), (most + DC_MIN_TILES - 1) / DC_MIN_TILES)));
+    a.slots = 2 * sm_count();
+    // a CTA for every share there can be (of at least DC_MIN_TILES tiles) and for every (request, head) on its own
+    const long long pairs = static_cast<long long>(num_kv_heads) * a.requests;
+    const unsigned ctas = static_cast<unsigned>(std::min<long long>(a.slots, std::max((most + DC_MIN_TILES - 1) / DC_MIN_TILES, pairs)));
     a.max_pieces = static_cast<int>(pieces);
     a.ws_o = static_cast<float *>(ws), a.ws_m = a.ws_o + rows_total * pieces * TC_D, a.ws_l = a.ws_m + rows_total * pieces;
     CUtensorMap mq, mk, mv;
@@ -904,8 +920,8 @@ int launch_paged_decode_tc(const void *q, const void *kp, const void *vp, const 
                                    cudaFuncSetAttribute(paged_decode_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeTcShape<4>::smem) == cudaSuccess &&
                                    cudaFuncSetAttribute(paged_decode_tc_kernel<4>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) == cudaSuccess;
     if (!configured) return fail(TL_ECUDA, "paged_attention: cannot raise shared memory limit");
-    cudaError_t le = narrow ? launch_chained(paged_decode_tc_kernel<1>, dim3(a.ctas), dim3(DecodeTcShape<1>::threads), DecodeTcShape<1>::smem, st, mq, mk, mv, a)
-                            : launch_chained(paged_decode_tc_kernel<4>, dim3(a.ctas), dim3(DecodeTcShape<4>::threads), DecodeTcShape<4>::smem, st, mq, mk, mv, a);
+    cudaError_t le = narrow ? launch_chained(paged_decode_tc_kernel<1>, dim3(ctas), dim3(DecodeTcShape<1>::threads), DecodeTcShape<1>::smem, st, mq, mk, mv, a)
+                            : launch_chained(paged_decode_tc_kernel<4>, dim3(ctas), dim3(DecodeTcShape<4>::threads), DecodeTcShape<4>::smem, st, mq, mk, mv, a);
     if (le != cudaSuccess) return fail(TL_ECUDA, "paged_attention: launch failed: %s", cudaGetErrorString(le));
     TL_LAUNCH_CHECK("paged_decode_tc");
     le = launch_chained(decode_merge_tc_kernel, dim3(static_cast<unsigned>(rows_total)), dim3(TC_D), 0, st, a);

@@ -173,8 +173,10 @@ class DecodeEngine:
         # occupied slots are a prefix of the table.  A step graph over the first 16 / 32 rows is captured beside the
         # full one and step() replays the smallest that covers the highest occupied slot: every kernel of the wide
         # path costs by rows (swap-AB column count, attention CTAs, reduction planes).  All variants stay on the
-        # >= 9-row kernels and the split counts do not depend on the row count, so a row's result is bit-identical
-        # whichever variant computed it.  (Config 4 runs 64 slots with ~20 live: decode step p50 3.31 -> 3.02 ms.)
+        # >= 9-row kernels, whose split counts do not depend on the row count, and the tcgen05 attention (tables of 1024 keys or more on
+        # 64-slot pages) cuts the key ranges by the requests' lengths alone: there a row's result is bit-identical whichever variant
+        # computed it.  The one-launch attention and the short-table kernel choose their splits by the rows of the launch, so where they
+        # split at all the variants differ by the rounding of the combination.  (64 slots with ~20 live: decode step p50 3.31 -> 3.02 ms.)
         rows_env = os.environ.get("TL_ROW_VARIANTS", "1")
         self._variants = sorted({r for r in (16, 32, 64) if r < self.B} | {self.B}) if (self.fused and self.B > 16 and rows_env != "0") else [self.B]
         self._graphs: dict = {}
