@@ -38,6 +38,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "per_device.h"
 #include "tc_wait.cuh"
 
 namespace tl {
@@ -845,6 +846,24 @@ bool paged_prefill_tc_supported(int L, int num_pages, int page_size, int num_kv_
     return L > 0 && num_pages > 0 && page_size >= TC_BN && page_size % TC_BN == 0;
 }
 
+// A chained launch with `smem` bytes of dynamic shared memory, the limit raised once per device and kernel.
+template <auto KERNEL, typename Args>
+static int attention_launch(dim3 grid, int threads, size_t smem, cudaStream_t st, const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const Args &a) {
+    static PerDevice ready;
+    int device = -1;
+    cudaGetDevice(&device);
+    const bool raised = ready(device, [&] {
+        return cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess &&
+               cudaFuncSetAttribute(KERNEL, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) == cudaSuccess;
+    });
+    if (!raised) {
+        cudaGetLastError();
+        return fail(TL_ECUDA, "paged_attention: cannot raise shared memory limit");
+    }
+    const cudaError_t e = launch_chained(KERNEL, grid, dim3(threads), smem, st, mq, mk, mv, a);
+    return e == cudaSuccess ? TL_OK : fail(TL_ECUDA, "paged_attention: launch failed: %s", cudaGetErrorString(e));
+}
+
 // Tensor maps of the queries (boxes of RH positions x G heads) and of the pages (boxes of one tile).
 static int attention_maps(CUtensorMap *mq, CUtensorMap *mk, CUtensorMap *mv, const void *q, const void *kp, const void *vp, int rows, int L, int RH, int G, int num_pages,
                           int page_size, int num_kv_heads) {
@@ -871,23 +890,14 @@ int launch_paged_prefill_tc(const void *q, const void *kp, const void *vp, const
     a.is_causal = is_causal;
     CUtensorMap mq, mk, mv;
     if (int e = attention_maps(&mq, &mk, &mv, q, kp, vp, rows, L, a.RH, G, num_pages, page_size, num_kv_heads)) return e;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(paged_prefill_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES) != cudaSuccess ||
-            cudaFuncSetAttribute(paged_prefill_tc_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess ||
-            cudaFuncSetAttribute(paged_prefill_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM_BYTES) != cudaSuccess ||
-            cudaFuncSetAttribute(paged_prefill_tc_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-            return fail(TL_ECUDA, "paged_attention: cannot raise shared memory limit");
-        configured = true;
-    }
     const int q_blocks = (L + a.RH - 1) / a.RH;
     a.out_token_major = out_token_major ? 1 : 0;
     dim3 grid(q_blocks, num_kv_heads, B);
     if (grid.y > 65535 || grid.z > 65535) return fail(TL_EINVAL, "paged_attention: too many heads / requests for one launch");
     static const bool p_tmem = [] { const char *e = getenv("TL_FA_P_TMEM"); return e == nullptr || e[0] != '0'; }();  // 0: P through shared memory (control)
-    cudaError_t le = p_tmem ? launch_chained(paged_prefill_tc_kernel<true>, grid, dim3(TC_THREADS), TC_SMEM_BYTES, st, mq, mk, mv, a)
-                            : launch_chained(paged_prefill_tc_kernel<false>, grid, dim3(TC_THREADS), TC_SMEM_BYTES, st, mq, mk, mv, a);
-    if (le != cudaSuccess) return fail(TL_ECUDA, "paged_attention: launch failed: %s", cudaGetErrorString(le));
+    if (int e = p_tmem ? attention_launch<paged_prefill_tc_kernel<true>>(grid, TC_THREADS, TC_SMEM_BYTES, st, mq, mk, mv, a)
+                       : attention_launch<paged_prefill_tc_kernel<false>>(grid, TC_THREADS, TC_SMEM_BYTES, st, mq, mk, mv, a))
+        return e;
     TL_LAUNCH_CHECK("paged_prefill_tc");
     return TL_OK;
 }
@@ -915,16 +925,11 @@ int launch_paged_decode_tc(const void *q, const void *kp, const void *vp, const 
     CUtensorMap mq, mk, mv;
     if (int e = attention_maps(&mq, &mk, &mv, q, kp, vp, rows, L, L, a.G, num_pages, page_size, num_kv_heads)) return e;
     const bool narrow = a.G * L <= 32;
-    static const bool configured = cudaFuncSetAttribute(paged_decode_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeTcShape<1>::smem) == cudaSuccess &&
-                                   cudaFuncSetAttribute(paged_decode_tc_kernel<1>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) == cudaSuccess &&
-                                   cudaFuncSetAttribute(paged_decode_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecodeTcShape<4>::smem) == cudaSuccess &&
-                                   cudaFuncSetAttribute(paged_decode_tc_kernel<4>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) == cudaSuccess;
-    if (!configured) return fail(TL_ECUDA, "paged_attention: cannot raise shared memory limit");
-    cudaError_t le = narrow ? launch_chained(paged_decode_tc_kernel<1>, dim3(ctas), dim3(DecodeTcShape<1>::threads), DecodeTcShape<1>::smem, st, mq, mk, mv, a)
-                            : launch_chained(paged_decode_tc_kernel<4>, dim3(ctas), dim3(DecodeTcShape<4>::threads), DecodeTcShape<4>::smem, st, mq, mk, mv, a);
-    if (le != cudaSuccess) return fail(TL_ECUDA, "paged_attention: launch failed: %s", cudaGetErrorString(le));
+    if (int e = narrow ? attention_launch<paged_decode_tc_kernel<1>>(dim3(ctas), DecodeTcShape<1>::threads, DecodeTcShape<1>::smem, st, mq, mk, mv, a)
+                       : attention_launch<paged_decode_tc_kernel<4>>(dim3(ctas), DecodeTcShape<4>::threads, DecodeTcShape<4>::smem, st, mq, mk, mv, a))
+        return e;
     TL_LAUNCH_CHECK("paged_decode_tc");
-    le = launch_chained(decode_merge_tc_kernel, dim3(static_cast<unsigned>(rows_total)), dim3(TC_D), 0, st, a);
+    const cudaError_t le = launch_chained(decode_merge_tc_kernel, dim3(static_cast<unsigned>(rows_total)), dim3(TC_D), 0, st, a);
     if (le != cudaSuccess) return fail(TL_ECUDA, "paged_attention: launch failed: %s", cudaGetErrorString(le));
     TL_LAUNCH_CHECK("decode_merge_tc");
     return TL_OK;
