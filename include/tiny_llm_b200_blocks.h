@@ -278,9 +278,11 @@ int tlb_paged_attention_tc(const void *q, long long q_token, long long q_head, i
                            long long g_token, int gate_wide, void *out, long long o_token, long long o_head, const float *head_bias, int weights,
                            void *stream);
 /* The cached rows of every sequence's context (start + tokens of seq_info) one after the other, each sequence from a whole 64-row
- * page on: rows [total_pages * 64, width], zeros past a sequence's newest token, and table [num_seqs, table_pages] of their pages. */
+ * page on: rows [total_pages * 64, width], zeros past a sequence's newest token, and table [num_seqs, table_pages] of their pages.
+ * window > 0: only from the 64-row tile on in which the first new token's window begins; seen [num_seqs, 4] (or NULL) then gets
+ * seq_info with its positions counted from there. */
 int tlb_latent_rows(const void *slab, int num_pages, int page_size, int width, const int32_t *seq_info, int num_seqs, const int32_t *block_table,
-                    int max_pages, void *rows, int32_t *table, int table_pages, int total_pages, void *stream);
+                    int max_pages, void *rows, int window, int32_t *table, int table_pages, int total_pages, int32_t *seen, void *stream);
 /* Latent attention with keys and values up-projected per head: q [tokens, heads, dim + rot] against k [rows, heads * dim] (head h's
  * part at h * dim), the part all heads share k_rot [rows, rot], and v (head h at v + h * v_head, rows v_row apart), rows found through
  * `table` (64-row pages).  dim % 64 == 0, rot <= 64, rot % 8 == 0, dim + rot and dv up to 256.  128 tokens a run. */

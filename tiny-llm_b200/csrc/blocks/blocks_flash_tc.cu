@@ -413,16 +413,21 @@ static int flash_tc_launch(const FlashTcOperands &x, const FlashTcArgs &a, cudaS
     return TL_OK;
 }
 
-// A latent layer's cached rows of every sequence, one after the other from whole 64-row pages on, and the block table that finds
-// them there: what the up projections of keys and values read.  Rows past a sequence's newest token are zeros.
+// A latent layer's cached rows of every sequence that a query of the step may see (window > 0: from the tile of the first query's first
+// visible key on), one after the other from whole 64-row pages on, and the block table that finds them there: what the up projections of
+// keys and values read.  Rows past a sequence's newest token are zeros.  `seen` [num_seqs, 4], or NULL: seq_info with positions counted
+// from the first row kept; that is a whole tile, so the attention takes the same tiles as over all rows.
 constexpr int kRowParts = 4;
 __global__ void __launch_bounds__(256)
 latent_rows_kernel(const bf16 *__restrict__ slab, int num_pages, int page_size, int width, const int32_t *__restrict__ seq_info, int num_seqs,
-                   const int32_t *__restrict__ block_table, int max_pages, bf16 *__restrict__ rows, int32_t *__restrict__ table, int table_pages, int total_pages) {
+                   const int32_t *__restrict__ block_table, int max_pages, int window, bf16 *__restrict__ rows, int32_t *__restrict__ table, int table_pages, int total_pages,
+                   int32_t *__restrict__ seen) {
     constexpr int ROWS = kXKeys / kRowParts;  // of a page a CTA
     const int s = blockIdx.y, p = blockIdx.x / kRowParts, row0 = blockIdx.x % kRowParts * ROWS, lane = threadIdx.x & 31;
-    auto context = [&](int i) { return seq_info[4 * i + 1] + seq_info[4 * i + 2]; };
-    const int ctx = context(s);
+    auto skipped = [&](int i) { return window > 0 ? max(0, seq_info[4 * i + 2] - window + 1) / kXKeys * kXKeys : 0; };
+    auto context = [&](int i) { return seq_info[4 * i + 1] + seq_info[4 * i + 2] - skipped(i); };
+    const int skip = skipped(s), ctx = context(s);
+    if (seen && blockIdx.x == 0 && threadIdx.x < 4) seen[4 * s + threadIdx.x] = seq_info[4 * s + threadIdx.x] - (threadIdx.x == 2 ? skip : 0);
     if (p * kXKeys >= ctx) return;
     int before = 0;
     for (int i = lane; i < s; i += 32) before += (context(i) + kXKeys - 1) / kXKeys;
@@ -432,8 +437,8 @@ latent_rows_kernel(const bf16 *__restrict__ slab, int num_pages, int page_size, 
     if (threadIdx.x == 0 && row0 == 0) table[(size_t)s * table_pages + p] = before + p;
     const int pieces = width / 8;
     for (int i = threadIdx.x; i < ROWS * pieces; i += 256) {
-        const int j = row0 + i / pieces, piece = i % pieces, key = p * kXKeys + j;
-        const int page = key < ctx && key / page_size < max_pages ? block_table[(size_t)s * max_pages + key / page_size] : -1;
+        const int j = row0 + i / pieces, piece = i % pieces, key = skip + p * kXKeys + j;
+        const int page = key < skip + ctx && key / page_size < max_pages ? block_table[(size_t)s * max_pages + key / page_size] : -1;
         uint4 v = make_uint4(0, 0, 0, 0);
         if (page >= 0 && page < num_pages) v = *reinterpret_cast<const uint4 *>(slab + ((size_t)page * page_size + key % page_size) * width + piece * 8);
         *reinterpret_cast<uint4 *>(rows + ((size_t)(before + p) * kXKeys + j) * width + piece * 8) = v;
@@ -485,13 +490,13 @@ int tlb_paged_attention_tc(const void *q, long long q_token, long long q_head, i
 }
 
 int tlb_latent_rows(const void *slab, int num_pages, int page_size, int width, const int32_t *seq_info, int num_seqs, const int32_t *block_table, int max_pages, void *rows,
-                    int32_t *table, int table_pages, int total_pages, void *stream) {
+                    int window, int32_t *table, int table_pages, int total_pages, int32_t *seen, void *stream) {
     if (num_seqs <= 0 || total_pages <= 0) return TL_OK;
-    if (!slab || !seq_info || !block_table || !rows || !table || num_pages <= 0 || page_size <= 0 || max_pages <= 0 || table_pages <= 0 || width <= 0 || width % 8 ||
+    if (!slab || !seq_info || !block_table || !rows || !table || num_pages <= 0 || page_size <= 0 || max_pages <= 0 || table_pages <= 0 || width <= 0 || width % 8 || window < 0 ||
         !tl::aligned16(slab) || !tl::aligned16(rows) || num_seqs > 65535)
         return tl::fail(TL_EINVAL, "latent_rows: bad argument");
     latent_rows_kernel<<<dim3(table_pages * kRowParts, num_seqs), 256, 0, as_stream(stream)>>>((const bf16 *)slab, num_pages, page_size, width, seq_info, num_seqs,
-                                                                                   block_table, max_pages, (bf16 *)rows, table, table_pages, total_pages);
+                                                                                   block_table, max_pages, window, (bf16 *)rows, table, table_pages, total_pages, seen);
     TL_LAUNCH_CHECK("latent_rows");
     return TL_OK;
 }

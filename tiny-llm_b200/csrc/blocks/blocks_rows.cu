@@ -398,7 +398,7 @@ using namespace tlb;
 
 extern "C" {
 
-int tlb_abi_version(void) { return 8; }
+int tlb_abi_version(void) { return 9; }
 const char *tlb_last_error(void) { return tl::g_error; }
 long long tlb_launch_count(void) { return tl::g_launches.load(std::memory_order_relaxed); }
 

@@ -61,7 +61,7 @@ _SIGNATURES = {
     "tlb_flash_tc_supported": (_I, [_I, _I, _I, _I, _I]),
     "tlb_paged_attention_tc": (_I, [_VP, _LL, _LL, _I, _VP, _I, _I, _I, _I, _I, _I, _VP, _I, _VP, _I, _I, _I, _I, _I, _F, _F, _I, _VP, _LL, _I, _VP, _LL, _LL, _VP, _I,
                                     _VP]),
-    "tlb_latent_rows": (_I, [_VP, _I, _I, _I, _VP, _I, _VP, _I, _VP, _VP, _I, _I, _VP]),
+    "tlb_latent_rows": (_I, [_VP, _I, _I, _I, _VP, _I, _VP, _I, _VP, _I, _VP, _I, _I, _VP, _VP]),
     "tlb_latent_attention_heads": (_I, [_VP, _LL, _LL, _I, _VP, _LL, _VP, _LL, _LL, _VP, _LL, _I, _I, _I, _I, _LL, _VP, _I, _VP, _I, _I, _I, _F, _VP, _LL, _LL, _VP, _VP]),
     "tlb_kv_prepare": (_I, [_VP, _LL, _LL, _I, _VP, _VP, _LL, _LL, _VP, _LL, _LL, _I, _I, _I, _VP, _F, _VP, _VP, _VP, _I, _I, _I, _VP, _I, _I, _VP]),
     "tlb_qk_whole_prepare": (_I, [_VP, _LL, _I, _VP, _VP, _LL, _VP, _LL, _I, _I, _I, _VP, _F, _I, _I, _D, _VP, _VP, _VP, _I, _I, _I, _VP, _VP, _VP, _I, _I, _VP]),
@@ -92,7 +92,7 @@ _SIGNATURES = {
 }
 EXPORTED_SYMBOLS = tuple(_SIGNATURES)
 
-ABI_VERSION = 8
+ABI_VERSION = 9
 ATTENTION_TILE_TOKENS = 4
 ACT_SILU, ACT_GELU_TANH, ACT_RELU_SQUARED, ACT_CLAMPED_SWISH, ACT_TANH = 0, 1, 2, 3, 4
 WEIGHTS_SOFTMAX, WEIGHTS_SIGMOID = 0, 1
@@ -770,19 +770,28 @@ def paged_attention_tc(q, slab, block_table, seq_info, runs: int, *, kv_heads: i
     return out
 
 
-def latent_rows(slab, block_table, seq_info, contexts: list):
+def latent_first_row(start: int, window: int) -> int:
+    """The first position of a sequence that ``latent_rows`` keeps: the 64-row tile of what the token at ``start`` sees first."""
+    return max(0, start - window + 1) // 64 * 64 if window else 0
+
+
+def latent_rows(slab, block_table, seq_info, contexts: list, window: int = 0, seen=None):
     """-> (rows ``[N, width]``: the cached rows of every sequence's ``contexts[s]`` positions, each sequence from a whole 64-row page
-    on, and the int32 table ``[S, pages]`` of where they are).  ``seq_info`` must say the same contexts (start + tokens)."""
-    _gpu("latent_rows", slab, block_table, seq_info)
-    _contig("latent_rows", slab, block_table, seq_info)
+    on, and the int32 table ``[S, pages]`` of where they are).  ``seq_info`` must say the same contexts (start + tokens).  With a
+    ``window`` the rows that no new token sees are left out: ``contexts[s]`` counts from ``latent_first_row(start, window)``, and so
+    do the positions in ``seen`` (given: int32 ``[S, 4]``, written), which stands for ``seq_info`` from there on."""
+    _gpu("latent_rows", slab, block_table, seq_info, seen)
+    _contig("latent_rows", slab, block_table, seq_info, seen)
+    if seen is not None and (seen.dtype != torch.int32 or seen.shape != seq_info.shape):
+        raise RuntimeError("latent_rows: seen must be int32 of seq_info's shape")
     P, page_size, width = slab.shape
     pages = [-(-n // 64) for n in contexts]
     if len(pages) != seq_info.shape[0] or block_table.shape[0] != len(pages) or slab.dtype != torch.bfloat16:
         raise RuntimeError("latent_rows: a bfloat16 cache, one context per sequence")
     rows = torch.empty((64 * sum(pages), width), dtype=slab.dtype, device=slab.device)
     table = torch.empty((len(pages), max(pages)), dtype=torch.int32, device=slab.device)
-    _check(library().tlb_latent_rows(_ptr(slab), P, page_size, width, _ptr(seq_info), len(pages), _ptr(block_table), block_table.shape[1], _ptr(rows), _ptr(table),
-                                     table.shape[1], sum(pages), _stream(slab)))
+    _check(library().tlb_latent_rows(_ptr(slab), P, page_size, width, _ptr(seq_info), len(pages), _ptr(block_table), block_table.shape[1], _ptr(rows), int(window or 0),
+                                     _ptr(table), table.shape[1], sum(pages), _ptr(seen), _stream(slab)))
     return rows, table
 
 

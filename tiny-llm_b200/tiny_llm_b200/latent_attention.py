@@ -77,34 +77,37 @@ class LatentAttention:
         """Whether this step's attention runs on keys and values up-projected per head instead of on the latents themselves.
 
         Per query, key and head the absorbed form multiplies ``2 rank + rot`` entries, this one ``dim + rot + vdim`` (1088 and 320 at
-        the larger benchmark size), and it runs on tcgen05; its price is the up projection of every cached row and three more
+        the larger benchmark size), and it runs on tcgen05; its price is the up projection of every cached row that is seen and three more
         launches.  Measured (us): absorbed about 30 + its operations at 110 TFLOP/s; this one about 25 + the up projection at 600
         TFLOP/s + 1.75 for every 64-key tile of the longest sequence and wave of CTAs.  2048 tokens, 16 heads: 723 and 158; 128 tokens
         after 4000: 250 and 172; 64 after 4000: 147 and 168.  Below 38 us the calls are bound by the host and launches count."""
         counts = getattr(plan, "counts", None)
         if not self.tc or counts is None or plan.max_tokens == 1:
             return False
+        from extensions_b200.tiny_llm_ext_b200 import blocks
+
         w = self.window or (1 << 60)
         pairs = sum(n * min(s, w) + n * min(n, w) // 2 for n, s in zip(counts, plan.starts))
-        rows = sum(counts) + sum(plan.starts)
+        rows = sum(n + s - blocks.latent_first_row(s, self.window) for n, s in zip(counts, plan.starts))
         tiles = min(plan.max_context, w + 128) / 64 * max(1.0, sum(-(-n // 128) for n in counts) * self.heads / 296)
         absorbed = 30 + pairs * self.heads * (2 * self.rank + self.rot_dim) * 2 / 110e6
         per_head = 25 + 1.75 * tiles + rows * self.rank * self.heads * (self.dim + self.vdim) * 2 / 600e6
         if absorbed <= max(per_head, 38) or rows * self.heads * (self.dim + self.vdim) > PER_HEAD_ENTRIES:
             return False
-        from extensions_b200.tiny_llm_ext_b200 import blocks
-
         return blocks.tma_rows(q3)
 
     def _attend_heads(self, q3: torch.Tensor, plan, slab: torch.Tensor) -> torch.Tensor:
-        """``[T, heads, vdim]``: the sequences' cached rows side by side, keys and values of every head from them, per-head attention."""
+        """``[T, heads, vdim]``: the sequences' cached rows (those that a new token sees) side by side, keys and values of every head from
+        them, per-head attention."""
         from extensions_b200.tiny_llm_ext_b200 import blocks
 
-        rows, table = blocks.latent_rows(slab, plan.block_table, plan.seq_info, [n + s for n, s in zip(plan.counts, plan.starts)])
+        contexts = [n + s - blocks.latent_first_row(s, self.window) for n, s in zip(plan.counts, plan.starts)]
+        seen = torch.empty_like(plan.seq_info) if self.window else None
+        rows, table = blocks.latent_rows(slab, plan.block_table, plan.seq_info, contexts, self.window, seen)
         c = rows[:, : self.rank]
         k = linear(c, self.w_uk.view(self.heads * self.dim, self.rank))
         v = torch.bmm(c.expand(self.heads, -1, -1), self.w_uv_t)  # [heads, rows, vdim]
-        return blocks.latent_attention_heads(q3, k, v, rows[:, self.rank :], table, plan.seq_info, sum(-(-n // 128) for n in plan.counts), dim=self.dim,
+        return blocks.latent_attention_heads(q3, k, v, rows[:, self.rank :], table, plan.seq_info if seen is None else seen, sum(-(-n // 128) for n in plan.counts), dim=self.dim,
                                              window=self.window, scale=self.scale, sink=self.sink)
 
     def __call__(self, h: torch.Tensor, plan, slab: torch.Tensor) -> torch.Tensor:
