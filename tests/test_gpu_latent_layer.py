@@ -1,9 +1,10 @@
 """The latent layer's own route to keys and values up-projected per head: through a page slab, with a window (rows that no query sees are
-left out), sinks and a query latent, against the absorbed form."""
+left out), sinks and a query latent, against the absorbed form; and back to that form when the buffers cannot be had."""
 
 import pytest
 import torch
 
+from tiny_llm_b200 import latent_attention
 from tiny_llm_b200.latent_attention import LatentAttention
 from tiny_llm_b200.latent_kv_cache import LatentPagedCache, LatentPagedPool
 from tiny_llm_b200.ragged import RaggedEntry, RaggedPlan
@@ -61,3 +62,21 @@ def test_layer_takes_the_rows_that_are_seen(sizes, counts, starts, rows, monkeyp
     # either form rounds about five tensors on its way to bf16 (2^-9 each, root mean square below that)
     assert float((got - want).norm() / want.norm()) < 2.0**-6
     assert blocks.library().tlb_tc_gave_up() == 0
+
+
+@pytest.mark.parametrize("where", ["linear", "bmm"])
+def test_without_memory_for_the_buffers_the_layer_runs_the_absorbed_form(where, monkeypatch):
+    layer, h, plan, slab = step([1200, 198], [0, 1025])
+    layer.tc = False
+    want = layer(h, plan, slab)
+    layer.tc = True
+    assert layer._per_head(plan, h.new_empty(h.shape[0], layer.heads, layer.dim + layer.rot_dim))
+    real, rows = {"linear": latent_attention.linear, "bmm": torch.bmm}[where], 64 * (19 + 20)
+
+    def short_of_memory(a, *rest, **kw):
+        if a.shape[-2] == rows:
+            raise torch.OutOfMemoryError("CUDA out of memory")
+        return real(a, *rest, **kw)
+
+    monkeypatch.setattr(latent_attention if where == "linear" else torch, where, short_of_memory)
+    assert torch.equal(layer(h, plan, slab), want)

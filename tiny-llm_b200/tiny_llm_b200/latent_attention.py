@@ -96,17 +96,20 @@ class LatentAttention:
             return False
         return blocks.tma_rows(q3)
 
-    def _attend_heads(self, q3: torch.Tensor, plan, slab: torch.Tensor) -> torch.Tensor:
+    def _attend_heads(self, q3: torch.Tensor, plan, slab: torch.Tensor) -> torch.Tensor | None:
         """``[T, heads, vdim]``: the sequences' cached rows (those that a new token sees) side by side, keys and values of every head from
-        them, per-head attention."""
+        them, per-head attention.  None where the memory for them cannot be had: the absorbed form needs none of it."""
         from extensions_b200.tiny_llm_ext_b200 import blocks
 
         contexts = [n + s - blocks.latent_first_row(s, self.window) for n, s in zip(plan.counts, plan.starts)]
         seen = torch.empty_like(plan.seq_info) if self.window else None
-        rows, table = blocks.latent_rows(slab, plan.block_table, plan.seq_info, contexts, self.window, seen)
-        c = rows[:, : self.rank]
-        k = linear(c, self.w_uk.view(self.heads * self.dim, self.rank))
-        v = torch.bmm(c.expand(self.heads, -1, -1), self.w_uv_t)  # [heads, rows, vdim]
+        try:
+            rows, table = blocks.latent_rows(slab, plan.block_table, plan.seq_info, contexts, self.window, seen)
+            c = rows[:, : self.rank]
+            k = linear(c, self.w_uk.view(self.heads * self.dim, self.rank))
+            v = torch.bmm(c.expand(self.heads, -1, -1), self.w_uv_t)  # [heads, rows, vdim]
+        except torch.OutOfMemoryError:
+            return None
         return blocks.latent_attention_heads(q3, k, v, rows[:, self.rank :], table, plan.seq_info if seen is None else seen, sum(-(-n // 128) for n in plan.counts), dim=self.dim,
                                              window=self.window, scale=self.scale, sink=self.sink)
 
@@ -142,7 +145,8 @@ class LatentAttention:
         kernel, tile_tokens = self.attention_kernel(slab)
         if kernel == "mma" and self._per_head(plan, q3):
             o = self._attend_heads(q3, plan, slab)
-            return linear_wide(o.view(T, H * self.vdim), self.w_o)
+            if o is not None:
+                return linear_wide(o.view(T, H * self.vdim), self.w_o)
         q_lat = torch.bmm(q3[:, :, :dn].transpose(0, 1), self.w_uk)          # [H, T, rank]
         o_lat = torch.empty_like(q_lat)
         blocks.latent_attention(q_lat.transpose(0, 1), q3[:, :, dn:], slab, plan.block_table, plan.tiles_for(tile_tokens), plan.tok_pos,
