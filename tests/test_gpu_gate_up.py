@@ -47,3 +47,20 @@ def test_layer_form_mixed_flags_and_refusals():
         quantized_gate_up(x, a, wrap(odd))
     with pytest.raises(RuntimeError, match="a must be the same dtype as scales"):
         quantized_gate_up(x.half(), a, b)
+
+
+def test_the_gate_is_kept_for_the_stream_that_reads_it():
+    """On a stream of its own the intermediate outlives the call: what the caller allocates meanwhile must not lie in its place."""
+    N, K, M = 1024, 2048, 6
+    weights = [weight(K, N, torch.bfloat16, seed) for seed in (1, 2)]
+    x = torch.randn(M, N, device="cuda").bfloat16()
+    want = ext.quantized_gate_up(x, *weights)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(20_000_000)  # about 10 ms: the products are queued, not run, when the call returns
+    got = ext.quantized_gate_up(x, *weights, stream=side)
+    taken = [torch.full((M, K), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    torch.cuda.current_stream().synchronize()
+    side.synchronize()
+    assert torch.equal(got, want) and all(bool(t.isnan().all()) for t in taken)

@@ -284,6 +284,8 @@ def quantized_gate_up(a, gate, up, gate_flags=(True, False), up_flags=(True, Fal
             None if ws is None else ws.data_ptr(), ws_bytes, _stream_ptr(stream, a),
         )
     )
+    if stream is not None:  # freed on return, while that stream may still have to read it
+        gate_out.record_stream(stream)
     return out
 
 
