@@ -15,6 +15,13 @@ using tl::warp_sum;
 
 typedef __nv_bfloat16 bf16;
 
+// Streaming multiprocessors of the current device.
+static inline int sm_count() {
+    int device = 0, n = 0;
+    cudaGetDevice(&device);
+    return cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && n > 0 ? n : 148;
+}
+
 // Sum over a CTA of `blockDim.x` threads (a multiple of 32, at most 1024); every thread gets the result.
 __device__ __forceinline__ float block_sum(float v, float *scratch /* [33] */) {
     v = warp_sum(v);

@@ -515,7 +515,7 @@ int tlb_decay_scan(const void *q, long long q_token, long long q_head, const voi
     const auto ctas = [&](int nc) { return (long long)heads * ceil_div(dv, kLaThreads / kLaLanes * nc) * num_seqs * max_segments; };
     int nc = 1;
     for (int more = kr <= 16 ? 4 : kr <= 32 ? 2 : 1; more > 1 && max_tokens_per_seq > 4 && nc == 1; more /= 2)
-        if (ctas(more) >= 3 * 148) nc = more;
+        if (ctas(more) >= 3LL * sm_count()) nc = more;
 #define TLB_DS_N(KRV, PASS, GZ, BON, SCA, NCV)                                                                                                           \
     decay_scan_kernel<T, KRV, (KRV > 32 ? 8 : 16), BON, SCA, NCV><<<dim3(num_seqs, heads * ceil_div(dv, kLaThreads / kLaLanes * NCV), GZ), kLaThreads, 0, st>>>(  \
         (const T *)q, q_token, q_head, (const T *)k, k_token, k_head, (const T *)v, v_token, v_head, z, z_token, (const T *)z_bias, z ? 1.0f / tau : 0.f, head_decay, \

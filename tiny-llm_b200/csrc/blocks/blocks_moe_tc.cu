@@ -277,11 +277,8 @@ int moe_tc_product(const MoeProduct &p, cudaStream_t st) {
         cudaGetLastError();
         return tl::fail(TL_ECUDA, "moe_tc: no shared memory");
     }
-    int device = 0, sms = 0;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const long long most = moe_max_chunks(p.tokens, p.top, p.experts) * a.m_blocks;  // tiles there can be
-    moe_tc_kernel<<<(unsigned)std::min<long long>(sms, most), kTcThreads, a.stages * a.stage_bytes + kTcBars, st>>>(m0, m1, mx, a);
+    moe_tc_kernel<<<(unsigned)std::min<long long>(sm_count(), most), kTcThreads, a.stages * a.stage_bytes + kTcBars, st>>>(m0, m1, mx, a);
     return TL_OK;
 }
 

@@ -89,7 +89,7 @@ class LatentAttention:
         w = self.window or (1 << 60)
         pairs = sum(n * min(s, w) + n * min(n, w) // 2 for n, s in zip(counts, plan.starts))
         rows = sum(n + s - blocks.latent_first_row(s, self.window) for n, s in zip(counts, plan.starts))
-        tiles = min(plan.max_context, w + 128) / 64 * max(1.0, sum(-(-n // 128) for n in counts) * self.heads / 296)
+        tiles = min(plan.max_context, w + 128) / 64 * max(1.0, sum(-(-n // 128) for n in counts) * self.heads / (2 * blocks.sm_count(q3.device)))
         absorbed = 30 + pairs * self.heads * (2 * self.rank + self.rot_dim) * 2 / 110e6
         per_head = 25 + 1.75 * tiles + rows * self.rank * self.heads * (self.dim + self.vdim) * 2 / 600e6
         if absorbed <= max(per_head, 38) or rows * self.heads * (self.dim + self.vdim) > PER_HEAD_ENTRIES:
