@@ -1,9 +1,9 @@
-"""Headline benchmark: Qwen3-4B W4A16 decode / prefill tokens/s on B200 (BASELINE.json).
+"""Headline benchmark: Qwen3-4B W4A16 decode / prefill tokens/s on B200.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
                     [--workload decode|prefill|serve|serve8k] [--no-extra] [--no-cpu-baseline]
 
-Workloads (BASELINE.json `configs`):
+Workloads:
 
   decode   (default; config 2, the one the metric is quoted on) Qwen3-4B-shaped random W4A16 weights,
            ONE request per GPU, 128-token prompt (chunk-prefilled through the paged path), greedy decode
@@ -32,22 +32,22 @@ Numbers on the JSON line (decode):
             decode graph issues them (2.137 GB of packed weights, > L2), replayed from a CUDA graph,
             CUDA-event timed; achieved = algorithmic bytes / time, traffic = ncu DRAM bytes of the same
             launches (read from the committed capture named in `traffic_source`, null if there is none)
-  --workload voluzen  (not a BASELINE config) the Voluzen design - latent attention + mixture of experts, bf16 weights - at
+  --workload voluzen  (beside the headline) the Voluzen design - latent attention + mixture of experts, bf16 weights - at
             two sizes beside Qwen3 W4A16 of equal width / depth / heads / active feed-forward width: prefill and decode tok/s,
             and the design's kernels alone against the measured peaks; its own JSON line
-  --workload senurax  (not a BASELINE config) the Senurax design - retention, gated delta rule and rotated attention mixers,
+  --workload senurax  (beside the headline) the Senurax design - retention, gated delta rule and rotated attention mixers,
                       looped layers, experts with identity experts - at a few real-layer sizes beside Bapovik of equal size, and its
                       kernels against their rooflines.
-  --workload norusun  (not a BASELINE config) the Norusun design - residual streams, time-mix linear attention, latent attention with
+  --workload norusun  (beside the headline) the Norusun design - residual streams, time-mix linear attention, latent attention with
                       learned sinks, chunked sigmoid attention beside a state-space mixer - at two real-layer sizes beside Senurax of
                       equal size, and its kernels against their rooflines.
-  --workload zalazen  (not a BASELINE config) the Zalazen design - windowed attention with kept first positions, sinks and gates beside a
+  --workload zalazen  (beside the headline) the Zalazen design - windowed attention with kept first positions, sinks and gates beside a
                       gated feed-forward, pair embedding - at two real-layer sizes beside Bapovik's attention layers of equal size, and its
                       kernels against their rooflines.
-  --workload nomudra  (not a BASELINE config) the Nomudra design - matrix memory and chunked attention in turn, tanh norms around every
+  --workload nomudra  (beside the headline) the Nomudra design - matrix memory and chunked attention in turn, tanh norms around every
                       sublayer, grouped experts with a gated shared expert - at two real-layer sizes beside Senurax of equal size, and its
                       kernels against their rooflines.
-  --workload bapovik  (not a BASELINE config) the Bapovik design - windowed / chunked attention beside a recurrent mixer, experts,
+  --workload bapovik  (beside the headline) the Bapovik design - windowed / chunked attention beside a recurrent mixer, experts,
             bf16 weights - at two sizes beside Voluzen of equal size, and the design's kernels alone against the measured peaks
   cpu_baseline  the reference's CPU path (oracle.model: dense bf16 weights, readable operators) on the
             host cores, bounded sample
@@ -353,7 +353,7 @@ def matvec_roofline(model, engine, ext, device) -> dict:
         stream.synchronize()
         times = [cuda_time_ms(graph.replay, stream) for _ in range(10)]
     ms = statistics.median(times)
-    # algorithmic bytes: every packed weight, scale and bias once (SURVEY 8d: 0.53125 B/weight) + activations in/out
+    # algorithmic bytes: every packed weight, scale and bias once (0.53125 B/weight) + activations in/out
     margs = model.mlx_model.args
     io = 2 * len(model.layers_inner) * (H + (engine.Hq + 2 * engine.Hkv) * engine.D + engine.Hq * engine.D + 2 * H + H + inter + inter + 2 * H)
     algorithmic = weight_stream_bytes(margs) + io + 2 * (H + margs.vocab_size)
@@ -380,7 +380,7 @@ def _prefill_request(model, device, prompt, chunk=2048):
 
 
 def context_sweep(model, device, margs) -> list:
-    """Config-2 context sweep (SURVEY 8d): B = 1, 64 device-resident decode steps after a real prefill of S tokens."""
+    """Config-2 context sweep: B = 1, 64 device-resident decode steps after a real prefill of S tokens."""
     from tiny_llm_b200.batch import greedy_tokens
     from tiny_llm_b200.synthetic import weight_stream_bytes
 
@@ -753,7 +753,7 @@ def run_cpu_baseline(sample_steps: int, warmup_steps: int = 1, mode: str = "deco
     8-token prompt and a few decode steps; the per-token time is scaled to the full depth by weight
     bytes (a decode step on the CPU is one pass over every dense weight).  Threads are pinned to
     min(32, cores): the bf16 GEMV of torch scales poorly past that and oversubscribed runs made the
-    round-1 number swing by 80x."""
+    number swing by 80x."""
     from oracle.model import ReferenceCpuModel, greedy_decode
 
     synthetic = _load_standalone("_bench_synthetic", ROOT / "tiny-llm_b200" / "tiny_llm_b200" / "synthetic.py")

@@ -3,7 +3,7 @@
   [TL_S5_HALF=0] [TL_S5_GRID=...] python tools/decode_ab.py [--batch 1] [--context 128] [--steps 128] [--tag name]
 
 Launch-geometry switches of the streaming kernel are read once per process, so every variant is
-its own process; the script appends one JSON line to gpurun_out/decode_ab.jsonl.
+its own process; the script prints one JSON line.
 """
 from __future__ import annotations
 
@@ -73,10 +73,6 @@ def main():
                tok_s=round(B * 1e3 / best, 1), kernels_per_step=engine.kernels_per_step,
                env={k: v for k, v in os.environ.items() if k.startswith("TL_")})
     print(json.dumps(rec), flush=True)
-    out = ROOT / "gpurun_out"
-    out.mkdir(exist_ok=True)
-    with open(out / "decode_ab.jsonl", "a") as f:
-        f.write(json.dumps(rec) + "\n")
 
 
 if __name__ == "__main__":

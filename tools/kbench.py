@@ -3,7 +3,7 @@ replays (so host launch overhead is out of the picture), rotating over enough
 distinct buffers that every launch misses L2 (126 MB), reported against the
 measured HBM peak of MEASURED_PEAKS.json.
 
-  python tools/kbench.py [--out gpurun_out/kbench.json] [--quick]
+  python tools/kbench.py [--out kbench.json] [--quick]
 """
 
 from __future__ import annotations
@@ -108,7 +108,7 @@ def small_ops():
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("--out", default=str(ROOT / "gpurun_out" / "kbench.json"))
+    ap.add_argument("--out", default="kbench.json")
     ap.add_argument("--quick", action="store_true")
     ap.add_argument("--lib", default=None, help="alternative libtiny_llm_b200*.so (experiment builds)")
     ap.add_argument("--only", default=None, help="comma-separated matvec shape names; skips attention and small ops")

@@ -1,7 +1,7 @@
 """Workloads for an ncu launch list (per-kernel gpu__time_duration of ONE step, captured graph included):
 
   ncu --metrics gpu__time_duration.sum --clock-control none --profile-from-start off --csv \
-      --log-file gpurun_out/launches.csv python tools/launch_list.py --mode decode --batch 64 --context 1024
+      --log-file launches.csv python tools/launch_list.py --mode decode --batch 64 --context 1024
   ... --mode chunk --chunk 128 --context 512      # one chunked-prefill step of the serving loop
 
 The profiler range covers exactly one decode step / one prefill chunk after warm-up.  Times under ncu are serialised

@@ -2,7 +2,7 @@
 Qwen3-4B layer shapes, paged causal prefill attention at L = S = 4096, and the whole-model chunked
 prefill of a 4096-token prompt through the public API.
 
-  python tools/prefill_bench.py [--out gpurun_out/prefill_bench.json]
+  python tools/prefill_bench.py [--out prefill_bench.json]
 """
 from __future__ import annotations
 
@@ -45,7 +45,7 @@ def timed(fn, reps=5):
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("--out", default=str(ROOT / "gpurun_out" / "prefill_bench.json"))
+    ap.add_argument("--out", default="prefill_bench.json")
     ap.add_argument("--tokens", type=int, default=4096)
     ap.add_argument("--skip-model", action="store_true")
     ap.add_argument("--profile", action="store_true", help="torch.profiler kernel table of one whole-model prefill")

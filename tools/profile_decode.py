@@ -2,7 +2,7 @@
 range so that ncu can be pointed at exactly the decode kernels:
 
   ncu --nvtx --nvtx-include "decode/" --metrics gpu__time_duration.sum --clock-control none \
-      --csv --log-file gpurun_out/launches.csv python tools/profile_decode.py --layers 36 --steps 2
+      --csv --log-file launches.csv python tools/profile_decode.py --layers 36 --steps 2
 """
 
 from __future__ import annotations
