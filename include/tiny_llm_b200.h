@@ -4,8 +4,8 @@
  *
  * This is the drop-in boundary: one launcher per native primitive of the
  * reference's extension (declared in
- * /root/reference/src/extensions_ref/src/tiny_llm_ext.h:10-141 and exported to
- * Python by /root/reference/src/extensions_ref/bindings.cpp:14-46).  Where the
+ * src/extensions_ref/src/tiny_llm_ext.h:10-141 and exported to
+ * Python by src/extensions_ref/bindings.cpp:14-46).  Where the
  * reference builds a lazy `mx::array` whose `eval_gpu` encodes a Metal
  * dispatch, a launcher here enqueues sm_100a kernels on the caller's CUDA
  * stream.  Conventions:
@@ -71,7 +71,7 @@ long long tl_tc_gave_up(void);
  *   !use_simdgroup                           : scalar control kernel.
  * (Shapes a tensor-core kernel cannot take - odd alignments - fall back to the streaming kernel, which
  * handles up to TL_MATVEC_MAX_ROWS rows per pass.)
- * The split of the reduction is a scheduling decision of this backend (SURVEY 8a' item 12): it depends only on
+ * The split of the reduction is a scheduling decision of this backend: it depends only on
  * (N, K), never on use_split_k, so a split request and a plain request run the very same kernel with
  * bit-identical results (tests_refsol/test_week_2_day_7.py:80-109).
  * workspace: tl_quantized_matmul_workspace() bytes (0 = none; fp32 partial planes of a split reduction,
@@ -228,7 +228,7 @@ int tl_paged_cache_append_chunk(void *key_pages, void *value_pages, const void *
  * q/k RMSNorm + RoPE, append of the newest K/V row and paged GQA attention in ONE launch (plus a
  * merge launch when the context is split over several CTAs).  Replaces, with the same rounding
  * points, the call sequence rms_norm, rms_norm, rope, rope, paged_cache_update, paged_attention
- * of /root/reference/src/tiny_llm_ref/qwen3_week3.py:62-105.  qkv [B, (Hq + 2 Hkv) * 128] is the
+ * of src/tiny_llm_ref/qwen3_week3.py:62-105.  qkv [B, (Hq + 2 Hkv) * 128] is the
  * row-concatenated projection output; context_lens are post-append; rope_inv_freq holds the 64
  * float64 frequencies base^(-i/64); out [B, Hq * 128]; max_context bounds every context_lens[b]
  * (it fixes the split count, so a captured launch stays valid as the contexts grow);

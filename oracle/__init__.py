@@ -7,7 +7,7 @@ Only ``tests/``, ``__graft_entry__.smoke()`` and the ``cpu_baseline`` /
 (``tiny-llm_b200/``) never imports ``oracle`` and has no CPU fallback: its
 operators raise when the CUDA extension is missing or when handed CPU tensors.
 
-What it restates (all paths relative to ``/root/reference``):
+What it restates (all paths are the reference's):
 
 * ``oracle.ops``      - the arithmetic of every native primitive in
   ``src/extensions_ref/src/*.metal`` with the same rounding points (fp32
@@ -24,7 +24,7 @@ What it restates (all paths relative to ``/root/reference``):
   ``_ext`` module (``src/extensions_ref/bindings.cpp:14-46``) so that tests can
   drive the product's host logic (page pools, scheduler, models) without a GPU.
 
-Pinning status (see DESIGN.md "Oracle"):
+Pinning status:
 
 * integer / structural behaviour (page ids, page_lens, block tables, context
   lengths, growth counters, scheduler call traces, validation errors) is pinned

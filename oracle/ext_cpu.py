@@ -1,7 +1,7 @@
 """CPU stand-in for the native extension module, for tests only.
 
 TEST INFRASTRUCTURE (see ``oracle/__init__.py``).  Exposes the function surface
-of ``_ext`` (``/root/reference/src/extensions_ref/bindings.cpp:14-46``) over
+of ``_ext`` (``src/extensions_ref/bindings.cpp:14-46``) over
 ``oracle.ops`` so that ``tests/`` can exercise the product's *host* logic
 (page pools, block tables, scheduler, model wiring) on CPU tensors by
 monkeypatching ``tiny_llm_ext_b200``'s entry points.  The product never does

@@ -37,7 +37,7 @@ def test_every_declared_symbol_is_exported_and_bound():
 
 
 def test_reference_entry_points_keep_names_and_defaults():
-    # /root/reference/src/extensions_ref/bindings.cpp:14-46
+    # src/extensions_ref/bindings.cpp:14-46
     import inspect
 
     expected = {

@@ -1,7 +1,7 @@
 // Decode-side attention kernels (HBM-bound K/V streaming, fp32 online softmax).
 //
 //  * decode_attention_kernel       - dense K/V, reference week2_decode_attention
-//    (/root/reference/src/extensions_ref/src/week2_kernels.metal:119-235).
+//    (src/extensions_ref/src/week2_kernels.metal:119-235).
 //  * paged_rowwise_kernel          - generic paged attention, one CTA per query
 //    row; any dtype/head-dim/page-size (reference paged_attention_decode and the
 //    f32 scalar path, paged_attention.metal:108-248, :508-674).

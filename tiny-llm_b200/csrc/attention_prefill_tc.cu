@@ -1,7 +1,7 @@
 // Paged causal FlashAttention prefill on the 5th-generation tensor cores (tcgen05 + TMEM + TMA),
 // bf16, head_dim 128, L > 8; and the same arithmetic for a few new tokens (L <= 8) further down.
 //
-// Replaces paged_attention_mma_bf16_d128 (/root/reference/src/extensions_ref/src/
+// Replaces paged_attention_mma_bf16_d128 (src/extensions_ref/src/
 // paged_attention.metal:250-506): same arithmetic - fp32 scores in base 2 (:414 scale_log2),
 // bottom-right causal limit key <= row + (context - L) (:411), fp32 running max / sum, the
 // probabilities rounded to bf16 before P V (:439-444), output = O / sum (0 when nothing is visible).

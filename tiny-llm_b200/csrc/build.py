@@ -1,7 +1,7 @@
 """Build libtiny_llm_b200.so (sm_100a only) in-tree with nvcc.
 
 The reference drives CMake through mlx.extension.CMakeBuild
-(/root/reference/src/extensions_ref/build.py:11-24, CMakeLists.txt:32-84) to
+(src/extensions_ref/build.py:11-24, CMakeLists.txt:32-84) to
 produce a metallib plus a nanobind module; here one nvcc invocation per
 translation unit produces objects that are linked into a C-ABI shared library
 loaded with ctypes.  nvcc cross-compiles without a GPU.

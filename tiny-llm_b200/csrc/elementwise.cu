@@ -3,7 +3,7 @@
 // 128-bit coalesced accesses when alignment allows, fp32 math, one rounding.
 //
 // Arithmetic follows the reference Metal kernels (paths relative to
-// /root/reference/src/extensions_ref/src): week2_kernels.metal:6-117,
+// src/extensions_ref/src): week2_kernels.metal:6-117,
 // quantized_matmul.metal:58-89, paged_attention.metal:82-106.
 #include <float.h>
 #include <limits.h>

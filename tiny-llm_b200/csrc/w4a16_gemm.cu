@@ -4,7 +4,7 @@
 //
 // (reference naming: a [M, N_red], b [K_out, N_red/8]; in this file m = token,
 // n = output feature, k = reduction index).  Replaces
-// quantized_matmul_simdgroup_w4a16_g128 (/root/reference/src/extensions_ref/src/
+// quantized_matmul_simdgroup_w4a16_g128 (src/extensions_ref/src/
 // quantized_matmul.metal:96-249): like that kernel the weight is rounded to the
 // activation dtype when it is dequantised into shared memory (:183-194) and the
 // accumulation is fp32.

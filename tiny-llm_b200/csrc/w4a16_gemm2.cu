@@ -17,7 +17,7 @@
 // accumulators of 256 features), warps 4-11 dequantisers then epilogue (lane = token row).
 // Barriers live at the same offsets in both CTAs: full (own TMA + own dequantisers; in the leader also the peer's
 // "my tiles of this stage are complete"), empty and tmem_full (arrived in BOTH CTAs by the leader's multicast commit).
-// Replaces quantized_matmul_simdgroup_w4a16_g128 (/root/reference/src/extensions_ref/src/quantized_matmul.metal:96-249)
+// Replaces quantized_matmul_simdgroup_w4a16_g128 (src/extensions_ref/src/quantized_matmul.metal:96-249)
 // for M > 256; same rounding points as w4a16_gemm.cu (weights rounded to the activation dtype, fp32 accumulation).
 #include <cuda.h>
 #include <stdlib.h>
@@ -352,7 +352,7 @@ static int gemm2_t(const void *scales, const void *biases, const void *a, const 
     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
     if (encode == nullptr) return fail(TL_ECUDA, "quantized_matmul: cuTensorMapEncodeTiled is unavailable");
     if (!aligned16(a) || !aligned16(b)) return fail(TL_EINVAL, "quantized_matmul: a and b must be 16-byte aligned");
-    // tensor maps cached per (pointer, shape): encoding costs ~2 us of host time per launch (VERDICT r1 item 7)
+    // tensor maps cached per (pointer, shape): encoding costs ~2 us of host time per launch
     struct Key {
         const void *p;
         int M, N;

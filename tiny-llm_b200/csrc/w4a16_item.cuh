@@ -1,7 +1,7 @@
 // Building blocks of the W4A16 weight-streaming kernel (w4a16_matvec.cu): activation staging,
 // the register-pipelined weight unit and the tensor-core consumer.
 //
-// Why this shape (measured on B200, profiles/r01_kbench_*): the first three streaming kernels
+// Why this shape (measured on B200): the first three streaming kernels
 // all stalled at ~2 TB/s no matter how the bytes were fetched: the profiler's executed-instruction
 // count per byte of weights made the cp.async-ring version instruction-issue bound, not memory
 // bound.  The form below does less work per weight:
@@ -196,7 +196,7 @@ enum { W4_PRO_NONE = 0, W4_PRO_RMSNORM = 1, W4_PRO_SWIGLU = 2 };
 // half of the register cache carries more chunks).
 // sum(x^2) is deterministic: every half-warp (= one 128-column group of one row) parks its partial
 // in sq[row * G + group]; after one barrier each thread adds the G partials of its row in index
-// order.  (Round 1 used shared-memory atomicAdd: run-to-run summation order.)
+// order.  (A shared-memory atomicAdd would sum in another order from run to run.)
 // sq: Mp * N/128 floats of scratch (may alias memory that is only used after staging).
 // Ends with __syncthreads().
 template <typename T, int MP, int NT>

@@ -3,10 +3,10 @@
 //   out[m, k] = sum_n a[m, n] * (code[k, n] * scale[k, n/128] + bias[k, n/128])
 //
 // a [M, N] (bf16|f16), b [K, N/8] packed u32 (code i of a word = (w >> 4i) & 15,
-// /root/reference/src/tiny_llm_ref/quantize.py:113-115), scales/biases [K, N/128].
+// src/tiny_llm_ref/quantize.py:113-115), scales/biases [K, N/128].
 //
 // w4a16_stream5_kernel is the decode kernel (reference: quantized_matvec_x4_fast,
-// /root/reference/src/extensions_ref/src/quantized_matmul.metal:441-538): every packed
+// src/extensions_ref/src/quantized_matmul.metal:441-538): every packed
 // weight byte is read exactly once with 128-bit loads that bypass L1; activations (tiny,
 // shared by every CTA) are staged once per CTA in shared memory.  The per-weight ALU work
 // would exceed the HBM time on CUDA cores (~3 ops/weight), so the 16 x 128 code tile of
@@ -36,7 +36,7 @@ int launch_w4a16_stream(const void *scales, const void *biases, const void *a, c
 // v5: register-pipelined streaming, contiguous rows per CTA (see w4a16_item.cuh for the
 // inner loop).
 //
-// History, all measured on B200 (profiles/r01_kbench_*, tools/s4_timeline.py):
+// History, all measured on B200:
 //   v1 (register prefetch, 2 KB in flight per warp), v2 (producer warp + 256-byte cp.async.bulk
 //   ring) and v3 (per-warp cp.async rings) stalled near 2 TB/s: issue bound.  v4 (register pipeline) reached 3.9 TB/s on
 //   the tied head but dealt 16-row tiles to fixed-size warp teams: 1216 tiles over 1184 teams
@@ -61,7 +61,7 @@ int launch_w4a16_stream(const void *scales, const void *biases, const void *a, c
 //   epilogue RESIDUAL: out = T(float(res) + float(T(acc)))   (qwen3_week3.py:204-206)
 //   epilogue SWIGLU_PAIRS: rows 16c+r / 16c+8+r hold gate / up feature 8c+r;
 //                     out[m, 8c+r] = T(silu(T(acc_gate)) * T(acc_up))  (week2_kernels.metal:115-116)
-// Round-2 experiments that did NOT pay and were removed again (numbers: DESIGN.md section 4, profiles/r02_decode_ab.jsonl):
+// Experiments that did NOT pay and were removed again (profiles/r02_decode_ab.json):
 //   * 8-warp CTAs, two per SM, one from each of two consecutive launches (so that launch n+1 prefetches while launch n
 //     consumes): the consume phase is issue-bound, half the warps per launch doubled it (gate|up 5.4 -> 11.9 us) and the
 //     token went 1.44 -> 1.75 ms;
@@ -73,7 +73,7 @@ int launch_w4a16_stream(const void *scales, const void *biases, const void *a, c
 //   * a sixth generation that moved the weight stream from registers to per-warp TMA rings in shared memory (512-thread
 //     CTAs at 64 registers, two per SM so that two consecutive launches overlap on every SM): parity-green, but the
 //     consume phase pays a shared-memory read per weight word and 296 CTAs hand over more slowly than 140 -
-//     1.43 -> 1.99 ms (profiles/r02_stream6_timeline.txt);
+//     1.43 -> 1.99 ms;
 //   * asking the CTA's whole weight slice into L2 (cp.async.bulk.prefetch.L2) before griddepcontrol.wait, so that the
 //     consume phase would stream from L2: gate|up consume 4.64 -> 4.48 us, but the prefetch traffic competes with the
 //     activation round trip of the staging step (2.75 -> 3.2 us): 1.426 -> 1.461 ms.
@@ -303,7 +303,7 @@ static size_t stream5_smem_bytes(int N, int K, int MP, int grid) {
 // ---- launch geometry
 // One CTA per SM minus TL_S5_RESERVE (default 8): the few CTAs of the kernel behind it (the 8-CTA attention launch, the
 // first CTAs of the next projection) then start early under programmatic dependent launch and issue their independent
-// loads while this one is still running (round 1: 1.499 -> 1.399 ms/token; 16 reserved: no further gain).
+// loads while this one is still running (1.499 -> 1.399 ms/token; 16 reserved: no further gain).
 static int stream5_grid(int K) {
     static const int reserve = [] { const char *e = getenv("TL_S5_RESERVE"); const int v = e ? atoi(e) : 8; return v < 0 ? 0 : v; }();
     const int all = (K + 15) / 16;
@@ -319,7 +319,7 @@ static int stream5_launch(StreamArgs args, cudaStream_t st) {
     const size_t limit = S5_SMEM_MAX;
     if (smem > limit)
         return fail(TL_EINVAL, "quantized_matmul: activations do not fit in shared memory (N=%d, K=%d, rows=%d)", args.N, args.K, MP);
-    static bool configured = false;  // per process: one device per process (DESIGN.md section 5)
+    static bool configured = false;  // per process: one device per process
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(w4a16_stream5_kernel<T, MP, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(limit));

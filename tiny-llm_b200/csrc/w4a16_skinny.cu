@@ -3,7 +3,7 @@
 //
 //   out[m, n] = sum_k a[m, k] * T(code[n, k] * scale[n, k/128] + bias[n, k/128])       (m = token, n = feature)
 //
-// Why (round-1 VERDICT, missing #5 / row N4): with M <= 128 the 128 x 128-tile GEMM has K_out/128
+// Why: with M <= 128 the 128 x 128-tile GEMM has K_out/128
 // CTAs (20 for the o / down projections of Qwen3-4B) and the streaming kernel re-reads the weights
 // once per 32 rows; a 64-slot decode step took 16 ms where the weights are worth 0.33 ms of HBM time.
 // Reference's answer on its hardware: quantized_matmul_splitk (quantized_matmul.metal:251-293, policy
@@ -22,7 +22,7 @@
 //     beyond M zero-filled); the MMA warp issues tcgen05.mma M128 N{16..128} K16 from an elected lane.
 // Two CTAs fit per SM (96-113 KB of shared memory, 256 TMEM columns each) at every column count.
 //
-// How it got here (lm_head at 64 rows, 2560 -> 151936, 218 MB: profiles/r02_skinny_history.md): 256 threads on the SAME
+// How it got here (lm_head at 64 rows, 2560 -> 151936, 218 MB): 256 threads on the SAME
 // 64-wide block with the tile in shared memory 156 us -> two alternating groups, thread = row 143 us -> tile in tensor
 // memory (6 stages instead of 2) 136 us -> MMA warp on elect.sync 112 us -> 128-wide blocks (one barrier round trip per
 // quantisation group) 94 us (36.5 % of the HBM rate; 16 rows: 79 us, 41 %).  The per-block cycle trace (tools/skinny_blocks.py) showed each time which actor the
@@ -543,7 +543,7 @@ int w4a16_skinny_splits(int M, int N, int K) {
     int best = 1;
     long long best_cost = -1;
     // (a sweep of the cap (4, 8, 16) and of the fixed cost (4, 10, 20) moved single shapes by +-10 % stand-alone and the
-    // 64-slot step by nothing or for the worse: tools/gpu_call27.sh)
+    // 64-slot step by nothing or for the worse)
     for (int s = 1; s <= 16 && s <= num_gb / 2 + (num_gb < 2); ++s) {
         const int gbps = (num_gb + s - 1) / s;
         const int real = (num_gb + gbps - 1) / gbps;  // splits that actually get blocks

@@ -2,7 +2,7 @@
 
 Same function names, positional order, keyword names and defaults as the
 nanobind module ``tiny_llm_ext_ref._ext``
-(``/root/reference/src/extensions_ref/bindings.cpp:14-46``), but the arrays are
+(``src/extensions_ref/bindings.cpp:14-46``), but the arrays are
 contiguous CUDA ``torch.Tensor`` s instead of ``mx.array`` s and ``stream`` is
 an optional ``torch.cuda.Stream``.  Every function is a thin ctypes call into
 ``libtiny_llm_b200.so`` (C ABI: ``include/tiny_llm_b200.h``); torch only owns

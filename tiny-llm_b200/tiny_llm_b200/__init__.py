@@ -1,6 +1,6 @@
 """tiny_llm_b200 - tiny-llm's Qwen3 inference operators, models and scheduler
 re-hosted on torch tensors over the sm_100a extension.  The public names are
-those of ``tiny_llm_ref`` (``/root/reference/src/tiny_llm_ref/__init__.py``)."""
+those of ``tiny_llm_ref`` (``src/tiny_llm_ref/__init__.py``)."""
 
 # The module and a public function share a name.  The module is loaded first, so that no later import of it rebinds the name.
 from . import paged_attention as _paged_attention_module  # noqa: F401

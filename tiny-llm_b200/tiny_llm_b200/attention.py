@@ -1,4 +1,4 @@
-"""Attention operators (``/root/reference/src/tiny_llm_ref/attention.py``).
+"""Attention operators (``src/tiny_llm_ref/attention.py``).
 
 ``paged_attention`` keeps the reference's model-facing contract - query
 ``[B, H_q, L, D]``, page storage ``[P, H_kv, page_size, D]``, int32

@@ -1,5 +1,5 @@
 """Single-request greedy generation with a KV cache
-(``/root/reference/src/tiny_llm_ref/generate.py:49-81``)."""
+(``src/tiny_llm_ref/generate.py:49-81``)."""
 
 from __future__ import annotations
 

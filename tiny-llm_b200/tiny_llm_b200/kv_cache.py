@@ -1,5 +1,5 @@
 """KV-cache interfaces and the dense caches
-(``/root/reference/src/tiny_llm_ref/kv_cache.py``).
+(``src/tiny_llm_ref/kv_cache.py``).
 
 ``BatchingKvCache`` is the decode-slot table of the continuous-batching
 scheduler: a fixed number of slots, each holding one request's cache (or

@@ -1,11 +1,11 @@
-"""Model dispatch (``/root/reference/src/tiny_llm/models.py:8-18``)."""
+"""Model dispatch (``src/tiny_llm/models.py:8-18``)."""
 
 from __future__ import annotations
 
 from .qwen3_week2 import Qwen3ModelWeek2
 from .qwen3_week3 import Qwen3ModelWeek3
 
-# /root/reference/model_names.py:1-8
+# model_names.py:1-8
 MODEL_SHORTCUTS = {
     "qwen3-0.6b": "Qwen/Qwen3-0.6B-MLX-4bit",
     "qwen3-1.7b": "Qwen/Qwen3-1.7B-MLX-4bit",

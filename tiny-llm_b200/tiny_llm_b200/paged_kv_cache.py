@@ -1,4 +1,4 @@
-"""Paged KV storage (``/root/reference/src/tiny_llm_ref/paged_kv_cache.py``).
+"""Paged KV storage (``src/tiny_llm_ref/paged_kv_cache.py``).
 
 One ``TinyKvPagedPool`` per transformer layer owns the physical page slab
 ``[capacity, H_kv, page_size, D]`` for keys and for values; every request holds

@@ -1,8 +1,7 @@
 """Data-parallel serving: one process per GPU, requests sharded statically,
 weights broadcast once.
 
-The reference is single-process (no distributed code at
-all).  Requests never interact - each owns its page lists, pools are per model
+The reference is single-process (no distributed code at all).  Requests never interact - each owns its page lists, pools are per model
 instance - so the path shards as independent units: request ``i`` goes to rank
 ``i mod world`` and every rank runs the unchanged scheduler on its own replica.
 The only collective is the start-up ``broadcast`` of the packed weights from

@@ -1,5 +1,5 @@
 """W4A16 operator layer: same callables as
-``/root/reference/src/tiny_llm_ref/quantize.py`` over torch tensors and the
+``src/tiny_llm_ref/quantize.py`` over torch tensors and the
 B200 extension.
 
 Packed weights are ``[K, N/8]`` 32-bit words (``torch.uint32`` or ``int32``
@@ -83,7 +83,7 @@ def quantized_matmul(
     use_split_k: bool = False,
 ) -> torch.Tensor:
     """quantize.py:124-148.  NOTE: the Python default ``use_simdgroup=False``
-    differs from the extension's ``True`` on purpose (SURVEY 8a' #8)."""
+    differs from the extension's ``True`` on purpose: that is the reference's default."""
     rows, lead = _flatten_rows(a)
     out = tiny_llm_ext_b200.quantized_matmul(
         scales.contiguous(),

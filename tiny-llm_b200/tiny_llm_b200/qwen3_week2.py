@@ -1,5 +1,5 @@
 """Week-2 Qwen3 model with its cumulative optimisation checkpoints
-(``/root/reference/src/tiny_llm_ref/qwen3_week2.py``).
+(``src/tiny_llm_ref/qwen3_week2.py``).
 
 ``checkpoint`` selects how far along the course the model is: ``"kv-cache"``
 runs dense bf16 weights through the readable operators, each later name turns

@@ -1,5 +1,5 @@
 """Week-3 Qwen3 model: W4A16 projections, fused norm/RoPE/SwiGLU kernels and
-paged-KV attention (``/root/reference/src/tiny_llm_ref/qwen3_week3.py``).
+paged-KV attention (``src/tiny_llm_ref/qwen3_week3.py``).
 
 Constructor, ``create_kv_cache`` and ``__call__(inputs, offset, cache,
 logits_to_keep)`` keep the reference's contract; the only contact with weights
@@ -194,7 +194,7 @@ class Qwen3ModelWeek3:
         for index, layer in enumerate(mlx_model.model.layers[: self.num_hidden_layers]):
             if is_qwen3_moe_sparse_layer(args, index):
                 raise NotImplementedError(
-                    "Qwen3-MoE layers are outside the B200 hot-path scope (SURVEY.md section 2, row 12)"
+                    "Qwen3-MoE layers are outside the B200 hot-path scope"
                 )
             attn = layer.self_attn
             mlp = Qwen3MLP(
@@ -303,8 +303,8 @@ class Qwen3ModelWeek3:
     def _graph_limit(self, cache) -> int:
         """Longest request the decode engine of this call must hold: the scheduler's own
         ``max_seq_len`` when it states one (rounded up to whole pages), capped by
-        ``decode_graph_max_seq_len``.  Round 1 always reserved for 8192 tokens per slot: 76 GB of
-        pages for 64 slots of Qwen3-4B regardless of the batcher's limit."""
+        ``decode_graph_max_seq_len``.  (8192 tokens per slot whatever the batcher's limit would be 76 GB of
+        pages for 64 slots of Qwen3-4B.)"""
         from .kv_cache import BatchingKvCache
 
         limit = self.decode_graph_max_seq_len
