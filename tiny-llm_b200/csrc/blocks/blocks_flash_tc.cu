@@ -10,13 +10,9 @@
 //              the rest from a matrix shared by all heads): a latent layer's up-projected keys and its rotated part.
 //   warp 5     tcgen05.mma, one elected lane: S = Q K^T into one of two score buffers, O += P V; the next tile's scores are
 //              issued ahead of this tile's values
-//   warps 0-3  softmax, thread = row: scores from tensor memory, maximum, 2^x, P back over its own score buffer as two bf16 terms,
-//              the second what the first's rounding left over (the value product reads its left operand from tensor memory).  O is
-//              rescaled in tensor memory only when a row's maximum has grown by more than 2^8 since the last time.
-//              Two terms, because a row's largest weights are exact against its own maximum (they are 1) but not against one that may be
-//              stale: in one term the layer's error against 64 bits was up to 2.8 % above that of the register kernel, which takes
-//              the maximum anew for every tile; in two it is 0 to 4 % below.  It costs 1 to 4 % of a layer's time (2048 tokens, 16 heads
-//              over 4 of 128: 82.0 -> 85.6 us; 192 + 128 causal 125.1 -> 128.5), and a maximum anew for every tile as much (86.7, 127.8).
+//   warps 0-3  softmax, thread = row: scores from tensor memory, maximum, 2^x, P as bf16 back over its own score buffer (the
+//              value product reads its left operand from tensor memory).  O is rescaled in tensor memory only when a row's
+//              maximum has grown by more than 2^8 since the last time; sums are of the rounded P, so the result is exact.
 // 256 columns of tensor memory and at most 113 KB of shared memory (head sizes up to 192 + 128) let two CTAs share an SM: one's
 // exponentials run beside the other's products, both of which take about 512 cycles a tile at 128 + 128 (64 x 128 exponentials
 // at 16 a cycle).  With 192 key columns that leaves room for one value stage.
@@ -220,8 +216,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             if (g_elect_one()) {
                 const uint64_t vd = vd0 + (uint64_t)(vs * VB * (Z::kv_block >> 4));
 #pragma unroll
-                for (int k = 0; k < 2 * kXKeys / 16; ++k)  // both terms against the same values
-                    g_tc_mma_ts(tmem + O, tmem + (t & 1) * kXKeys + 8 * k, vd + (k & 3) * (2048 >> 4), idesc_o, t > 0 || k > 0);
+                for (int k = 0; k < kXKeys / 16; ++k) g_tc_mma_ts(tmem + O, tmem + (t & 1) * kXKeys + 8 * k, vd + k * (2048 >> 4), idesc_o, t > 0 || k > 0);
                 g_tc_commit(v_empty + 8 * vs);
                 g_tc_commit(pv_done + 8 * (t & 1));
             }
@@ -270,16 +265,12 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                     if (key > see_hi || (key < see_lo && key >= first_kept)) s[c >> 5][c & 31] = 0xff800000u;
                 }
             }
-            uint32_t pk[32], rest[32];
-            auto weights = [&](int i, float x, float y) {  // keys 2 i and 2 i + 1
-                pk[i] = tl::pack2<bf16>(x, y);
-                rest[i] = tl::pack2<bf16>(x - __uint_as_float(pk[i] << 16), y - __uint_as_float(pk[i] & 0xffff0000u));
-            };
+            uint32_t pk[32];
             if (a.weights == 1) {  // every visible key by itself: no maximum, no sum, nothing to rescale
 #pragma unroll
                 for (int c = 0; c < kXKeys; c += 2) {
                     const float x = __uint_as_float(s[c >> 5][c & 31]), y = __uint_as_float(s[c >> 5][(c & 31) + 1]);
-                    weights(c / 2, x == -INFINITY ? 0.f : 1.0f / (1.0f + x_ex2(-(x + bias))), y == -INFINITY ? 0.f : 1.0f / (1.0f + x_ex2(-(y + bias))));
+                    pk[c / 2] = tl::pack2<bf16>(x == -INFINITY ? 0.f : 1.0f / (1.0f + x_ex2(-(x + bias))), y == -INFINITY ? 0.f : 1.0f / (1.0f + x_ex2(-(y + bias))));
                 }
             } else {
                 float top = -INFINITY;
@@ -311,14 +302,13 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 float s0 = 0.f, s1 = 0.f;
 #pragma unroll
                 for (int c = 0; c < kXKeys; c += 2) {
-                    const float x = x_ex2(fmaf(__uint_as_float(s[c >> 5][c & 31]), mult, -at)), y = x_ex2(fmaf(__uint_as_float(s[c >> 5][(c & 31) + 1]), mult, -at));
-                    weights(c / 2, x, y);
-                    s0 += x, s1 += y;
+                    const uint32_t u = tl::pack2<bf16>(x_ex2(fmaf(__uint_as_float(s[c >> 5][c & 31]), mult, -at)), x_ex2(fmaf(__uint_as_float(s[c >> 5][(c & 31) + 1]), mult, -at)));
+                    pk[c / 2] = u;
+                    s0 += __uint_as_float(u << 16), s1 += __uint_as_float(u & 0xffff0000u);  // numerator and denominator see the same rounded weights
                 }
                 sum += s0 + s1;
             }
-            g_tmem_st32(tmem + lanes + (t & 1) * kXKeys, pk);  // column c = keys 2 c and 2 c + 1, column 32 + c what their rounding left over
-            g_tmem_st32(tmem + lanes + (t & 1) * kXKeys + 32, rest);
+            g_tmem_st32(tmem + lanes + (t & 1) * kXKeys, pk);  // column c = keys 2 c and 2 c + 1
             g_tmem_st_wait();
             if (key0 + kXKeys - 1 > hi) {  // values past the newest key: cleared before the product may read them
                 // These warps wait on v_full here only, and a parity says nothing unless the phase before it is known to be over: with
