@@ -164,3 +164,30 @@ def test_latent_heads(heads, dim, rot, dv, rank, counts, starts, window, sink):
         assert float((got[first : first + n].double() - want).norm() / want.norm()) < 2.0**-6, s
         first += n
     assert blocks.library().tlb_tc_gave_up() == 0
+
+
+@pytest.mark.parametrize("dk,dv,mask,size", [(128, 128, 0, 0), (192, 128, 2, 512), (64, 64, 1, 700)])
+def test_weights_are_as_exact_as_against_their_own_maximum(dk, dv, mask, size):
+    """Peaked scores (standard deviation 2), where the maximum grows over many tiles: no further from float64 than weights that are rounded
+    against the maximum of the keys up to their own tile."""
+    from extensions_b200.tiny_llm_ext_b200 import blocks
+
+    gen = torch.Generator().manual_seed(dk)
+    n, H, G, page = 1000, 8, 2, 64
+    q = (2 * torch.randn(n, H, dk, generator=gen)).to(torch.bfloat16).to(DEV)
+    rows = torch.randn(n, G * (dk + dv), generator=gen).to(torch.bfloat16).to(DEV)
+    slab = torch.zeros(-(-n // page), page, G * (dk + dv), dtype=torch.bfloat16, device=DEV)
+    slab.view(-1, G * (dk + dv))[:n] = rows
+    table = torch.arange(slab.shape[0], dtype=torch.int32, device=DEV)[None]
+    info = torch.tensor([[0, n, 0, -1]], dtype=torch.int32, device=DEV)
+    run = blocks.flash_tc_run(torch.bfloat16, H, G, dk, dv, page)
+    got = blocks.paged_attention_tc(q, slab, table, info, -(-n // run), kv_heads=G, dv=dv, mask=mask, mask_size=size, scale=dk**-0.5).double()
+    r = rows.double()
+    k, v, see = r[:, : G * dk].view(-1, G, dk), r[:, G * dk :].view(-1, G, dv), visible(torch.arange(n, device=DEV), n, mask, size, 0)
+    want = reference(q.double(), k, v, torch.arange(n, device=DEV), scale=dk**-0.5, see=see)
+    s = torch.einsum("nhd,mhd->hnm", q.double(), k.repeat_interleave(H // G, 1)) * dk**-0.5 * 1.4426950408889634
+    s = s.masked_fill(~see, -math.inf)
+    top = torch.nn.functional.pad(s, (0, -n % 64), value=-math.inf).view(H, n, -1, 64).amax(3).cummax(2).values.repeat_interleave(64, 2)[:, :, :n]
+    p = torch.exp2((s - top).masked_fill(~see, -math.inf)).bfloat16().double() * torch.exp2(top - top[:, :, -1:]).masked_fill(~see, 0.0)
+    model = (torch.einsum("hnm,mhd->nhd", p, v.repeat_interleave(H // G, 1)) / p.sum(2).t()[:, :, None]).bfloat16().double()
+    assert float((got - want).norm()) < 1.02 * float((model - want).norm())  # 2 % for the 32-bit scores and sums

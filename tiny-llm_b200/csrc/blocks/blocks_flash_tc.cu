@@ -11,8 +11,11 @@
 //   warp 5     tcgen05.mma, one elected lane: S = Q K^T into one of two score buffers, O += P V; the next tile's scores are
 //              issued ahead of this tile's values
 //   warps 0-3  softmax, thread = row: scores from tensor memory, maximum, 2^x, P as bf16 back over its own score buffer (the
-//              value product reads its left operand from tensor memory).  O is rescaled in tensor memory only when a row's
-//              maximum has grown by more than 2^8 since the last time; sums are of the rounded P, so the result is exact.
+//              value product reads its left operand from tensor memory).  The maximum is taken anew for every tile, and O is
+//              rescaled in tensor memory in a tile where one of the warp's rows has a new one; sums are of the rounded P.  (A
+//              maximum kept until it had grown by 2^8 saves 1 to 4 % of a layer's time, but a row's largest weights are
+//              exact against its own maximum only, where they are 1: the layer's error against 64 bits was up to 2.8 % above
+//              that of the register kernel, now it is the same.)
 // 256 columns of tensor memory and at most 113 KB of shared memory (head sizes up to 192 + 128) let two CTAs share an SM: one's
 // exponentials run beside the other's products, both of which take about 512 cycles a tile at 128 + 128 (64 x 128 exponentials
 // at 16 a cycle).  With 192 key columns that leaves room for one value stage.
@@ -277,7 +280,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 #pragma unroll
                 for (int c = 0; c < kXKeys; ++c) top = fmaxf(top, __uint_as_float(s[c >> 5][c & 31]));
                 top *= mult;
-                const bool grow = top > m + 8.0f || (m == -INFINITY && top != -INFINITY);
+                const bool grow = top > m;
                 if (__any_sync(0xffffffffu, grow) && t > 0) {
                     if (!(ok = tc_wait(pv_done + 8 * ((t - 1) & 1), ((t - 1) >> 1) & 1, dead))) break;  // O has to be still while it is rescaled
                     g_tc_fence_after();
