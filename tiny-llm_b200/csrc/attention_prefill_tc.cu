@@ -21,14 +21,16 @@
 //                      operand straight from the page layout), accumulators S and O in TMEM;
 //   warps 0-3          softmax: thread = MMA row = TMEM lane.  tcgen05.ld the 64 scores of its row,
 //                      scale, mask, running max (no shuffles: a thread owns the row), exp2, row sum,
-//                      bf16 probabilities -> shared memory in the swizzled K-major layout (A operand
-//                      of P V).  O is rescaled IN TMEM (tcgen05.ld / st) only when a row's maximum
+//                      bf16 probabilities -> back over the scores in tensor memory (A operand of P V;
+//                      TL_FA_P_TMEM=0: through shared memory, a control).  O is rescaled IN TMEM (tcgen05.ld / st) only when a row's maximum
 //                      grows by more than 2^8 since the last rescale: P and the row sum always use
 //                      the same (possibly stale) maximum, so the result is exact.
 //                      Epilogue: O / sum -> bf16 -> global.
 //
 // 256 TMEM columns and 112 KB of shared memory per CTA: two CTAs per SM, so one CTA's softmax
 // overlaps the other's MMAs without an intra-CTA ping-pong.
+//
+// paged_decode_tc_kernel and decode_merge_tc_kernel (a few new tokens) have a comment of their own.
 #include <stdlib.h>
 #include <math_constants.h>
 
@@ -50,7 +52,6 @@ constexpr int TC_BM = 128;        // MMA rows per CTA (G heads x RH query positi
 constexpr int TC_BN = 64;         // keys per tile
 constexpr int TC_STAGES = 2;
 constexpr int TC_THREADS = 6 * 32;
-constexpr int TC_SOFTMAX_THREADS = 128;
 constexpr int TC_Q_BYTES = TC_BM * TC_D * 2;        // 32 KiB: two 64-column halves of [128 rows x 128 B]
 constexpr int TC_KV_TILE = TC_BN * TC_D * 2;        // 16 KiB: two 64-column halves of [64 rows x 128 B]
 constexpr int TC_P_BYTES = TC_BM * TC_BN * 2;       // 16 KiB: [128 rows x 128 B]
@@ -99,8 +100,9 @@ struct TcArgs {
 // PT: the probabilities of a tile stay in TENSOR memory - P_j (bf16 pairs, 32 columns) overwrites the first half of the
 // score buffer S_j it was computed from, and P V reads its A operand from there (the TS form of tcgen05.mma).  The
 // shared-memory form kept ONE P tile, so the exponentials of tile j could not start before P V of tile j-1 had finished
-// reading it; now the exponentials overlap it (the wait sits just before the barrier arrival, and in the rare rescale
-// of O), and the eight 16-byte stores + proxy fence per row become one tcgen05.st.  Buffer reuse needs no barrier: S_{j+2} is issued behind P V_j in the same MMA queue.
+// reading it; now the exponentials overlap it and nothing waits for it but the rare rescale of O, and the eight 16-byte stores +
+// proxy fence per row become one tcgen05.st.  Buffer reuse needs no barrier: S_{j+2} is issued behind P V_j in the same MMA queue.
+// S_j complete implies P V_{j-2} complete (the tensor core takes them in order), and nothing about P V_{j-1} or any load.
 template <bool PT>
 __global__ void __launch_bounds__(TC_THREADS, 2)
 paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -793,7 +795,7 @@ __global__ void __launch_bounds__(TC_D) decode_merge_tc_kernel(const DecodeTcArg
 
 // ---------------------------------------------------------------- host side --
 // Tensor maps are cached per (base pointer, shape): a prefill of 36 layers x N chunks re-uses a
-// handful of distinct operands, and cuTensorMapEncodeTiled costs microseconds per call.
+// handful of distinct operands.  (An encoding takes 0.05 us; a look-up costs no more.)
 struct MapKey {
     const void *ptr;
     unsigned long long d0, d1, d2, d3;

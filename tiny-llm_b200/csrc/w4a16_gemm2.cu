@@ -352,7 +352,7 @@ static int gemm2_t(const void *scales, const void *biases, const void *a, const 
     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
     if (encode == nullptr) return fail(TL_ECUDA, "quantized_matmul: cuTensorMapEncodeTiled is unavailable");
     if (!aligned16(a) || !aligned16(b)) return fail(TL_EINVAL, "quantized_matmul: a and b must be 16-byte aligned");
-    // tensor maps cached per (pointer, shape): encoding costs ~2 us of host time per launch
+    // tensor maps cached per (pointer, shape)
     struct Key {
         const void *p;
         int M, N;
