@@ -391,7 +391,8 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
 // partial result per share for decode_merge_tc_kernel.  What is dealt out are the requests' real lengths, read on the device, so a
 // captured launch follows them.  (Before, every (request, head) had its own CTAs, as many for all as suited a full block table: requests
 // of very different lengths waited for the longest, which alone on its SM takes 1.3 us a tile, and more than one wave of CTAs
-// waited for a last, emptier one.  One new token, 32 heads over 8: 32 requests of 200 to 7200 tokens 124 -> 72 us, 64 of 100 to 4100
+// waited for a last, emptier one.  A few short requests are cut into single tiles: one of 900 tokens 7.0 us, in shares of at least two,
+// three and four tiles 8.2, 8.6 and 10.5.  One new token, 32 heads over 8: 32 requests of 200 to 7200 tokens 124 -> 72 us, 64 of 100 to 4100
 // 123 -> 96, 8 of 300 to 7300 39 -> 28, one of 8000 beside 31 of 200 134 -> 18.)
 // The query rows sit side by side (row = head of the group x L + token), so that only the softmax warps that have rows
 // run; up to 32 rows there is one, and room for two query stages and a third key and value stage.
@@ -405,7 +406,6 @@ struct DecodeTcArgs {
     int slots, max_pieces;  // CTAs the GPU holds at a time; pieces of a (request, head) that the workspace has room for (>= 2)
     float *ws_o, *ws_m, *ws_l;
 };
-constexpr int DC_MIN_TILES = 4;  // of a share: below it a CTA's fixed cost (set-up, queries, first tile: 3 to 4 us) outweighs what it saves
 
 __device__ __forceinline__ int dc_context(const DecodeTcArgs &a, int r) { return min(max(a.context_lens[r], 0), a.max_pages * a.page_size); }
 __device__ __forceinline__ int dc_tiles(const DecodeTcArgs &a, int r) { return (dc_context(a, r) + TC_BN - 1) / TC_BN; }
@@ -434,8 +434,7 @@ __device__ __forceinline__ DecodeDeal dc_deal(const DecodeTcArgs &a, int request
     total *= a.Hkv, before *= a.Hkv;
     // n tiles touch at most ceil(n / per) + 1 shares
     if (static_cast<long long>(live) * a.Hkv <= a.slots && static_cast<long long>(longest) * 4 * a.slots <= 5LL * total) return {total, before, 0};
-    const int per = max(max((total + a.slots - 1) / a.slots, (longest + a.max_pieces - 2) / (a.max_pieces - 1)), DC_MIN_TILES);
-    return {total, before, per};
+    return {total, before, max((total + a.slots - 1) / a.slots, (longest + a.max_pieces - 2) / (a.max_pieces - 1))};
 }
 
 // The rank-th request that has keys, -1 past the last; whole warps.
@@ -921,9 +920,7 @@ int launch_paged_decode_tc(const void *q, const void *kp, const void *vp, const 
     a.page_size = page_size, a.max_pages = max_pages, a.num_pages = num_pages, a.tiles_per_page = page_size / TC_BN;
     a.scale_log2 = scale * TC_LOG2E, a.is_causal = is_causal;
     a.slots = 2 * sm_count();
-    // a CTA for every share there can be (of at least DC_MIN_TILES tiles) and for every (request, head) on its own
-    const long long pairs = static_cast<long long>(num_kv_heads) * a.requests;
-    const unsigned ctas = static_cast<unsigned>(std::min<long long>(a.slots, std::max((most + DC_MIN_TILES - 1) / DC_MIN_TILES, pairs)));
+    const unsigned ctas = static_cast<unsigned>(std::max(1LL, std::min<long long>(a.slots, most)));  // shares of one tile at least
     a.max_pieces = static_cast<int>(pieces);
     a.ws_o = static_cast<float *>(ws), a.ws_m = a.ws_o + rows_total * pieces * TC_D, a.ws_l = a.ws_m + rows_total * pieces;
     CUtensorMap mq, mk, mv;
