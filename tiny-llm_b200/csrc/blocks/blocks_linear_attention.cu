@@ -60,8 +60,11 @@ __device__ __forceinline__ bool la_segment(int p0, int n, int c, int &lo, int &h
 // state reads 8 bytes of its token's staged numbers instead of 16.
 // NC: state columns per thread.  A row's staged numbers are read from shared memory once for all of them: with one column the scan
 // was bound by those reads (16 bytes for three multiply-adds, and every 32 columns staged the decays anew).
+// One column a thread is the form of decoding steps, a wave of CTAs that load their state, take a token and store it, and of short
+// portions: as many CTAs to an SM as fitted before it had staging in batches (16 rows a lane: 160 registers without a bound, three
+// CTAs; 16 tokens of 8 heads of 64 x 128 then took two waves: 5.5 us became 7.4, with the bound 5.1).
 template <typename T, int KR /* rows per lane: dk <= 4 * KR */, int kLaTokens /* tokens staged at a time */, bool BONUS, bool SCALAR, int NC>
-__global__ void __launch_bounds__(kLaThreads, NC > 1 ? (KR == 32 ? 3 : 4) : SCALAR && KR == 32 ? 8 : 1)
+__global__ void __launch_bounds__(kLaThreads, NC > 1 ? (KR == 32 ? 3 : 4) : SCALAR && KR == 32 ? 8 : KR == 8 ? 5 : KR == 16 ? 4 : 1)
 decay_scan_kernel(const T *__restrict__ q, long long q_token, long long q_head, const T *__restrict__ k, long long k_token, long long k_head,
                   const T *__restrict__ v, long long v_token, long long v_head, const float *__restrict__ z, long long z_token,
                   const T *__restrict__ z_bias, float inv_tau, const float *__restrict__ head_decay, const float *__restrict__ rope_cos,
