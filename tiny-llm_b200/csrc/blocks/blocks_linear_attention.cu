@@ -41,10 +41,10 @@ __device__ __forceinline__ bool la_segment(int p0, int n, int c, int &lo, int &h
     return true;
 }
 
-// One kernel, two uses (pass):
+// One kernel, two uses (SEG):
 //   0  the whole portion of a sequence in one CTA per (head, column block): state from the slot (or zero at position 0),
 //      outputs, state back to the slot.  Single tokens and short portions.
-//   1  segment c alone, from a ZERO state (c = 0: as in pass 0): its outputs, and to the workspace its end state, the product of
+//   1  segment c alone, from a ZERO state (c = 0: as in the first use): its outputs, and to the workspace its end state, the product of
 //      its decays and (c > 0) its scaled queries times the decays from its first token on, decayed [T, heads, dk]; of a
 //      sequence's last segment also the steps themselves, last_steps [sequences, 64, heads, dk] = (decay, key).  A sequence that
 //      is one segment is done with that.
@@ -62,21 +62,24 @@ __device__ __forceinline__ bool la_segment(int p0, int n, int c, int &lo, int &h
 // was bound by those reads (16 bytes for three multiply-adds, and every 32 columns staged the decays anew).
 // One column a thread is the form of decoding steps, a wave of CTAs that load their state, take a token and store it, and of short
 // portions: as many CTAs to an SM as fitted before it had staging in batches (16 rows a lane: 160 registers without a bound, three
-// CTAs; 16 tokens of 8 heads of 64 x 128 then took two waves: 5.5 us became 7.4, with the bound 5.1).
-template <typename T, int KR /* rows per lane: dk <= 4 * KR */, int kLaTokens /* tokens staged at a time */, bool BONUS, bool SCALAR, int NC>
-__global__ void __launch_bounds__(kLaThreads, NC > 1 ? (KR == 32 ? 3 : 4) : SCALAR && KR == 32 ? 8 : KR == 8 ? 5 : KR == 16 ? 4 : 1)
+// CTAs; 16 tokens of 8 heads of 64 x 128 then took two waves: 5.5 us became 7.4, with the bound 5.1).  With one decay per head and 32
+// rows a lane eight CTAs an SM leave 64 registers, which staging in batches spilled: up to three times the time of the plain walk.
+// So there the entries are staged one at a time, and it is seven (six for segments).  8 heads of 128 x 256, one decay per head: 64 tokens of
+// one sequence 48 us as a plain walk, 152 spilled, 39 now; 16 sequences of a token 9.6, 11.6, 8.4.
+template <typename T, int KR /* rows per lane: dk <= 4 * KR */, int kLaTokens /* tokens staged at a time */, bool BONUS, bool SCALAR, int NC, bool SEG>
+__global__ void __launch_bounds__(kLaThreads, NC > 1 ? (KR == 32 ? 3 : 4) : SCALAR && KR == 32 ? (SEG ? 6 : 7) : KR == 8 ? 5 : KR == 16 ? 4 : 1)
 decay_scan_kernel(const T *__restrict__ q, long long q_token, long long q_head, const T *__restrict__ k, long long k_token, long long k_head,
                   const T *__restrict__ v, long long v_token, long long v_head, const float *__restrict__ z, long long z_token,
                   const T *__restrict__ z_bias, float inv_tau, const float *__restrict__ head_decay, const float *__restrict__ rope_cos,
                   const float *__restrict__ rope_sin, int rope_dims, int rope_interleaved, float q_scale, int heads, int dk, int dv,
                   const int32_t *__restrict__ seq_info,
-                  float *__restrict__ state, long long slot_stride, int num_slots, float *__restrict__ out, int pass, int max_segments,
+                  float *__restrict__ state, long long slot_stride, int num_slots, float *__restrict__ out, int max_segments,
                   float *__restrict__ seg_state, float *__restrict__ seg_decay, float *__restrict__ decayed, float2 *__restrict__ last_steps, int decay_kind, const T *__restrict__ a_log,
                   const T *__restrict__ bonus, int qk_heads, const T *__restrict__ skip, int v_cols) {
     __shared__ float4 sx[SCALAR ? 1 : kLaTokens * 4 * KR];   // per token and key channel: (decay, k, scaled q, k times the bonus), one 16-byte read per row
     __shared__ float2 skq[SCALAR ? kLaTokens * 4 * KR : 1];  // SCALAR: (k, scaled q)
     constexpr int COLS = kLaThreads / kLaLanes * NC;  // per CTA
-    constexpr int BATCH = 4;
+    constexpr int BATCH = NC == 1 && SCALAR && KR == 32 ? 1 : 4, VALUES = BATCH == 1 ? 1 : 8;
     __shared__ __align__(16) float sv[kLaTokens * COLS];
     __shared__ float sprod[4 * KR];
     __shared__ float2 s_step[kLaTokens];  // SCALAR: the token's (decay, key factor), worked out or read once per token
@@ -85,25 +88,25 @@ decay_scan_kernel(const T *__restrict__ q, long long q_token, long long q_head, 
     const int s = blockIdx.x, head = blockIdx.y / colblocks, col0 = (blockIdx.y % colblocks) * COLS, c = blockIdx.z;
     const int seq_first = seq_info[s * 4 + 0], seq_count = seq_info[s * 4 + 1], start = seq_info[s * 4 + 2], slot = seq_info[s * 4 + 3];
     int lo = start, hi = start + seq_count, nseg = 1;
-    if (pass != 0 && !la_segment(start, seq_count, c, lo, hi, nseg)) return;
+    if (SEG && !la_segment(start, seq_count, c, lo, hi, nseg)) return;
     const int first = seq_first + (lo - start), count = hi - lo;
     const int cidx = threadIdx.x / kLaLanes, r = threadIdx.x % kLaLanes;
     const int col = col0 + cidx * NC;  // .. col + NC - 1
     const int cols = min(NC, dv - col);  // <= 0: none
     const bool slot_ok = slot >= 0 && slot < num_slots;
     float *mine = state + (size_t)(slot_ok ? slot : 0) * slot_stride + (size_t)head * dk * dv;
-    float *seg = seg_state ? seg_state + (((size_t)s * max_segments + c) * heads + head) * dk * dv : nullptr;
-    const bool from_slot = pass == 0 || c == 0;  // else from zero
-    const bool to_slot = pass == 0 || nseg == 1;
-    const bool keeps_decays = !to_slot && col0 == 0;  // one column block per head
+    float *seg = SEG ? seg_state + (((size_t)s * max_segments + c) * heads + head) * dk * dv : nullptr;
+    const bool from_slot = !SEG || c == 0;  // else from zero
+    const bool to_slot = !SEG || nseg == 1;
+    const bool keeps_decays = SEG && !to_slot && col0 == 0;  // one column block per head
 
+    const bool has_state = from_slot && lo > 0 && slot_ok;
     float S[KR][NC];
 #pragma unroll
     for (int i = 0; i < KR; ++i) {
         const int row = r + kLaLanes * i;
-        const float *src = from_slot && lo > 0 && slot_ok ? mine : nullptr;
 #pragma unroll
-        for (int u = 0; u < NC; ++u) S[i][u] = src && row < dk && u < cols ? src[(size_t)row * dv + col + u] : 0.f;
+        for (int u = 0; u < NC; ++u) S[i][u] = has_state && row < dk && u < cols ? mine[(size_t)row * dv + col + u] : 0.f;
     }
     if (keeps_decays)
         for (int d = threadIdx.x; d < dk; d += blockDim.x) sprod[d] = 1.f;
@@ -167,15 +170,15 @@ decay_scan_kernel(const T *__restrict__ q, long long q_token, long long q_head, 
                 else sx[j * 4 * KR + d] = make_float4(alpha, kd, qd * q_scale, BONUS ? kd * s_chan[d].y : 0.f);
             }
         }
-        for (int e0 = threadIdx.x; e0 < n * COLS; e0 += 2 * BATCH * kLaThreads) {
-            T vs[2 * BATCH];
+        for (int e0 = threadIdx.x; e0 < n * COLS; e0 += VALUES * kLaThreads) {
+            T vs[VALUES];
 #pragma unroll
-            for (int u = 0; u < 2 * BATCH; ++u) {
+            for (int u = 0; u < VALUES; ++u) {
                 const int e = e0 + u * kLaThreads, j = e / COLS, d = e - j * COLS;
                 if (e < n * COLS && col0 + d < v_cols) vs[u] = v[(size_t)(first + t0 + j) * v_token + (size_t)head * v_head + col0 + d];
             }
 #pragma unroll
-            for (int u = 0; u < 2 * BATCH; ++u) {
+            for (int u = 0; u < VALUES; ++u) {
                 const int e = e0 + u * kLaThreads, d = e % COLS;
                 if (e < n * COLS) sv[e] = col0 + d < v_cols ? to_f(vs[u]) : col0 + d < dv ? 1.f : 0.f;
             }
@@ -227,7 +230,7 @@ decay_scan_kernel(const T *__restrict__ q, long long q_token, long long q_head, 
                     }
                 }
             };
-            if ((NC > 1 || KR <= 16) && dk == 4 * KR) rows(std::true_type{});
+            if ((NC > 1 || KR <= 16 || SCALAR) && dk == 4 * KR) rows(std::true_type{});
             else rows(std::false_type{});
             // the four lanes' sums: ((0 + 1) + (2 + 3)), each lane ending with its share of the columns
             float *to = out + ((size_t)(first + t0 + j) * heads + head) * dv + col;
@@ -520,9 +523,9 @@ int tlb_decay_scan(const void *q, long long q_token, long long q_head, const voi
     for (int more = kr <= 16 ? 4 : kr <= 32 ? 2 : 1; more > 1 && max_tokens_per_seq > 4 && nc == 1; more /= 2)
         if (ctas(more) >= 3LL * sm_count()) nc = more;
 #define TLB_DS_N(KRV, PASS, GZ, BON, SCA, NCV)                                                                                                           \
-    decay_scan_kernel<T, KRV, (KRV > 32 ? 8 : 16), BON, SCA, NCV><<<dim3(num_seqs, heads * ceil_div(dv, kLaThreads / kLaLanes * NCV), GZ), kLaThreads, 0, st>>>(  \
+    decay_scan_kernel<T, KRV, (KRV > 32 ? 8 : 16), BON, SCA, NCV, PASS != 0><<<dim3(num_seqs, heads * ceil_div(dv, kLaThreads / kLaLanes * NCV), GZ), kLaThreads, 0, st>>>(  \
         (const T *)q, q_token, q_head, (const T *)k, k_token, k_head, (const T *)v, v_token, v_head, z, z_token, (const T *)z_bias, z ? 1.0f / tau : 0.f, head_decay, \
-        rope_cos, rope_sin, rope_dims, rope_interleaved, q_scale, heads, dk, dv, seq_info, state, slot_stride, num_slots, out, PASS, max_segments, seg_state, seg_decay, \
+        rope_cos, rope_sin, rope_dims, rope_interleaved, q_scale, heads, dk, dv, seq_info, state, slot_stride, num_slots, out, max_segments, seg_state, seg_decay, \
         decayed, last_steps, decay_kind, (const T *)a_log, (const T *)bonus, qk_heads, (const T *)skip, v_cols)
 #define TLB_DS_B(KRV, PASS, GZ, BON, SCA)                                                                     \
     do {                                                                                                      \
