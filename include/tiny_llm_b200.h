@@ -240,6 +240,41 @@ int tl_decode_attention_fused(const void *qkv, const void *q_norm_weight, const 
                               float *workspace, int batch, int num_heads, int num_kv_heads, int head_dim, float eps,
                               float scale, int num_pages, int page_size, int max_pages, int max_context, int dtype,
                               void *stream);
+/* A whole decoding step of up to 8 requests as one launch (bf16, head_dim 128, 4-bit groups of 128): embedding, every block
+ * (src/tiny_llm_ref/qwen3_week3.py:55-121,139-146,196-207 at L == 1), final norm, head, greedy argmax.  The plan is a HOST struct,
+ * read during the call; every pointer in it is a device pointer.  Matrices other than the embedding table are tl_decode_step_pack()'s
+ * results: q|k|v (rows concatenated), o and down packed with halves = 1, gate (top) and up (bottom) together, the head with neither.  workspace: tl_decode_step_workspace() bytes, zeroed once, used by one step at a time and kept between steps;
+ * 0 bytes: these sizes are not taken. */
+typedef struct tl_packed_matrix {
+    const void *weight, *scales, *biases;
+} tl_packed_matrix;
+typedef struct tl_decode_step_layer {
+    const void *qkv, *o, *gate_up, *down;
+    const void *input_norm, *post_norm, *q_norm, *k_norm;
+    void *key_pages, *value_pages;
+    const int32_t *block_table; /* [batch, max_pages], -1 padded */
+    int num_pages;
+    float input_eps, post_eps, q_eps, k_eps, scale;
+} tl_decode_step_layer;
+typedef struct tl_decode_step_plan {
+    int batch, layers, num_heads, num_kv_heads, hidden, intermediate, vocab, page_size, max_pages;
+    float norm_eps;
+    const int32_t *tokens, *offsets, *context_lens; /* [batch]; context_lens count the new token, 0: idle */
+    const double *rope_inv_freq;                    /* [64] base^(-i/64) */
+    tl_packed_matrix embedding;
+    const void *head, *norm;
+    void *logits;         /* [batch, vocab] */
+    int32_t *next_tokens; /* [batch] */
+    void *workspace;
+    size_t workspace_bytes;
+    const tl_decode_step_layer *layer; /* [layers] */
+} tl_decode_step_plan;
+size_t tl_decode_step_workspace(int batch, int layers, int num_heads, int num_kv_heads, int hidden, int intermediate, int vocab);
+int tl_decode_step(const tl_decode_step_plan *plan, void *stream);
+/* Weights [rows, cols / 8] in the order in which tl_decode_step reads them: rows * cols / 4096 units of 2176 bytes (twice as many with a
+ * bottom matrix of the same shape), scales and biases included.  halves: rows in eights (cols a multiple of 512), else in sixteens, or in eights of
+ * top and bottom (cols a multiple of 256).  out is 16-byte aligned; concatenated rows are packed one after the other. */
+int tl_decode_step_pack(const tl_packed_matrix *top, const tl_packed_matrix *bottom, void *out, int rows, int cols, int halves, void *stream);
 /* Programmatic dependent launch for the streaming kernels (on by default; 0 turns it off,
  * TL_PDL=0 in the environment does the same). */
 int tl_set_pdl(int enabled);

@@ -1,0 +1,76 @@
+"""The decoding step in one launch against the operator sequence over the same buffers (``DecodeEngine._forward_unfused``)."""
+
+import pytest
+import torch
+
+from extensions_b200 import tiny_llm_ext_b200 as ext
+from tiny_llm_b200 import Qwen3ModelWeek3
+from tiny_llm_b200.engine import DecodeEngine
+from tiny_llm_b200.synthetic import synthetic_qwen3
+
+# the smallest sizes it takes (gate|up rows in every CTA), and one with a 19th of a piece's units odd, two heads a group and an untied head
+SMALL = dict(hidden_size=512, num_hidden_layers=3, num_attention_heads=8, num_key_value_heads=2, head_dim=128, intermediate_size=1536, vocab_size=528)
+WIDE = dict(hidden_size=1536, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=2, head_dim=128, intermediate_size=2560, vocab_size=1040)
+
+
+def test_sizes_it_does_not_take():
+    """0 bytes of workspace: the engine stays with the chain of launches."""
+    def takes(batch=1, layers=36, heads=32, kv=8, hidden=2560, inter=9728, vocab=151936):
+        return ext.DecodeStep.workspace_bytes(batch, layers, heads, kv, hidden, inter, vocab) > 0
+
+    assert takes() and takes(batch=4) and takes(heads=16, hidden=1024, inter=3072, layers=28)
+    assert not takes(batch=5) and not takes(layers=97) and not takes(heads=40) and not takes(hidden=2560 + 256) and not takes(inter=9728 + 256)
+    assert not takes(vocab=151930) and not takes(hidden=256, inter=512, heads=4, kv=2, vocab=512)
+    assert not takes(hidden=8192, batch=4)  # the rows of a norm in one batch
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", [SMALL, WIDE], ids=["small", "wide"])
+@pytest.mark.parametrize("page,contexts", [(16, [1]), (64, [64]), (64, [65]), (16, [129]), (128, [1500]), (128, [6000]), (16, [33, 0]), (8, [200, 7]), (64, [640, 1, 128]), (128, [1025, 63, 2200, 16])])
+def test_one_launch_equals_the_operator_sequence(cuda_device, dims, page, contexts):
+    dev, B = cuda_device, len(contexts)
+    model = Qwen3ModelWeek3(synthetic_qwen3(dims, seed=B, device=dev, realistic=True), page_size=page)
+    engine = DecodeEngine(model, B, max(contexts) + 3, dev)
+    assert engine._one_launch
+    need = [-(-c // page) for c in contexts]
+    engine.reserve_pools(sum(need) + 2)
+    g = torch.Generator(device=dev).manual_seed(7)
+    for pool in model.page_pools:
+        for pages in (pool._key_pages, pool._value_pages):
+            pages.copy_(torch.randn(pages.shape, generator=g, device=dev))
+    engine._ensure_graph()
+    order = torch.randperm(sum(need) + 2, generator=g, device=dev)[: sum(need)].to(torch.int32)
+    engine.tables.fill_(-1)
+    at = 0
+    for b, n in enumerate(need):
+        engine.tables[:, b, :n] = order[at : at + n]
+        at += n
+    if need[0] > 2:
+        engine.tables[:, 0, 1] = -1  # a page that is not there: its keys are not seen
+    engine.tokens.copy_(torch.randint(0, dims["vocab_size"], (B,), generator=g, device=dev))
+    engine.context_lens.copy_(torch.tensor(contexts, device=dev))
+    engine.offsets.copy_((engine.context_lens - 1).clamp(min=0))
+    before = [(p._key_pages.clone(), p._value_pages.clone()) for p in model.page_pools]
+
+    def run(step):
+        for pool, (k, v) in zip(model.page_pools, before):
+            pool._key_pages.copy_(k), pool._value_pages.copy_(v)
+        step()
+        return engine.logits.clone(), engine.next_tokens.clone(), [(p._key_pages.clone(), p._value_pages.clone()) for p in model.page_pools]
+
+    got, tokens, pages = run(engine._step.launch)
+    again, _, _ = run(engine._step.launch)
+    assert torch.equal(got, again), "the same bits every time"
+    assert torch.equal(tokens.long(), got.float().argmax(-1)), "the first of the largest"
+    want, _, want_pages = run(engine._forward_unfused)
+    # both round to bf16 a dozen times a block; an operator's own error is 2^-9 and they add up in quadrature
+    blocks = dims["num_hidden_layers"]
+    apart = ((got.double() - want.double()).norm(dim=-1) / want.double().norm(dim=-1)).max()
+    assert apart < 2**-8 * (12 * blocks) ** 0.5, float(apart)
+    for layer, ((k, v), (wk, wv), (k0, v0)) in enumerate(zip(pages, want_pages, before)):
+        for a, w, old in ((k, wk, k0), (v, wv, v0)):
+            touched = (w != old).any(-1)
+            assert torch.equal(a[~touched], old[~touched]), "only the newest token's rows are written"
+            if touched.any():
+                assert (a[touched].double() - w[touched].double()).norm() < 2**-8 * (12 * (layer + 1)) ** 0.5 * w[touched].double().norm()
+    assert ext.waits_given_up() == 0

@@ -36,6 +36,7 @@ SOURCES = [
     "attention_prefill.cu",
     "attention_prefill_tc.cu",
     "decode_attention_fused.cu",
+    "decode_step.cu",
 ]
 
 # The second library: building blocks for models with unquantised weights (include/tiny_llm_b200_blocks.h).  It links

@@ -59,7 +59,10 @@ int tl_abi_version(void) { return 1; }
 const char *tl_last_error(void) { return g_error; }
 
 long long tl_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
-long long tl_tc_gave_up(void) { return decode_tc_gave_up(); }
+long long tl_tc_gave_up(void) {
+    const long long attention = decode_tc_gave_up(), step = decode_step_gave_up();
+    return attention < 0 || step < 0 ? -1 : attention + step;
+}
 
 int tl_device_info(int *sms, int *major, int *minor) {
     int dev = 0;
@@ -421,6 +424,25 @@ int tl_decode_attention_fused(const void *qkv, const void *q_norm_weight, const 
     return launch_decode_attention_fused(qkv, q_norm_weight, k_norm_weight, offsets, block_table, context_lens, rope_inv_freq,
                                          key_pages, value_pages, out, workspace, batch, num_heads, num_kv_heads, head_dim, eps,
                                          scale, num_pages, page_size, max_pages, max_context, dtype, as_stream(stream));
+}
+
+size_t tl_decode_step_workspace(int batch, int layers, int num_heads, int num_kv_heads, int hidden, int intermediate, int vocab) {
+    return decode_step_workspace(batch, layers, num_heads, num_kv_heads, hidden, intermediate, vocab);
+}
+
+int tl_decode_step(const tl_decode_step_plan *plan, void *stream) {
+    if (!plan || !plan->tokens || !plan->offsets || !plan->context_lens || !plan->rope_inv_freq || !plan->norm || !plan->logits || !plan->next_tokens ||
+        !plan->workspace || !plan->layer)
+        return fail(TL_EINVAL, "decode_step: null pointer");
+    if (plan->page_size < 1 || plan->max_pages < 1) return fail(TL_EINVAL, "decode_step: bad sizes");
+    return launch_decode_step(*plan, as_stream(stream));
+}
+
+int tl_decode_step_pack(const tl_packed_matrix *top, const tl_packed_matrix *bottom, void *out, int rows, int cols, int halves, void *stream) {
+    for (const tl_packed_matrix *m : {top, bottom ? bottom : top})
+        if (!m || !m->weight || !m->scales || !m->biases) return fail(TL_EINVAL, "decode_step_pack: null pointer");
+    if (!out) return fail(TL_EINVAL, "decode_step_pack: null pointer");
+    return launch_decode_step_pack(*top, bottom, out, rows, cols, halves, as_stream(stream));
 }
 
 #if TL_TRACE

@@ -52,6 +52,8 @@ __all__ = [
     "quantized_matmul_residual_norm",
     "paged_attention_token_major",
     "qkv_project_rope_append",
+    "DecodeStep",
+    "decode_step_pack",
 ]
 
 _HERE = Path(__file__).resolve().parent
@@ -95,6 +97,9 @@ _SIGNATURES = {
     "tl_chunk_qk_norm_rope_append": (_I, [_VP] * 9 + [_I] * 4 + [_F, _F] + [_I] * 4 + [_VP]),
     "tl_decode_attention_fused_workspace": (_SZ, [_I, _I, _I]),
     "tl_decode_attention_fused": (_I, [_VP] * 11 + [_I] * 4 + [_F, _F] + [_I] * 5 + [_VP]),
+    "tl_decode_step_workspace": (_SZ, [_I] * 7),
+    "tl_decode_step": (_I, [_VP, _VP]),
+    "tl_decode_step_pack": (_I, [_VP, _VP, _VP, _I, _I, _I, _VP]),
     "tl_paged_cache_append_chunk": (_I, [_VP] * 5 + [_I] * 4 + [ctypes.c_longlong, ctypes.c_longlong, _I, _VP]),
     "tl_set_pdl": (_I, [_I]),
     "tl_set_gemm_pairs": (_I, [_I]),
@@ -813,6 +818,106 @@ def decode_attention_fused(qkv, q_norm_weight, k_norm_weight, offsets, block_tab
         )
     )
     return out
+
+
+class _PackedMatrix(ctypes.Structure):
+    _fields_ = [(n, _VP) for n in ("weight", "scales", "biases")]
+
+
+class _DecodeStepLayer(ctypes.Structure):
+    _fields_ = ([(n, _VP) for n in ("qkv", "o", "gate_up", "down", "input_norm", "post_norm", "q_norm", "k_norm", "key_pages", "value_pages", "block_table")]
+                + [("num_pages", _I)] + [(n, _F) for n in ("input_eps", "post_eps", "q_eps", "k_eps", "scale")])
+
+
+class _DecodeStepPlan(ctypes.Structure):
+    _fields_ = ([(n, _I) for n in ("batch", "layers", "num_heads", "num_kv_heads", "hidden", "intermediate", "vocab", "page_size", "max_pages")]
+                + [("norm_eps", _F)] + [(n, _VP) for n in ("tokens", "offsets", "context_lens", "rope_inv_freq")]
+                + [("embedding", _PackedMatrix)] + [(n, _VP) for n in ("head", "norm", "logits", "next_tokens", "workspace")]
+                + [("workspace_bytes", _SZ), ("layer", _VP)])
+
+
+def _tensor_ptr(t, shape, dtype) -> int:
+    if tuple(t.shape) != tuple(shape) or (t.dtype not in _PACKED if dtype is torch.int32 else t.dtype != dtype):
+        raise RuntimeError(f"decode_step: expected {dtype} {tuple(shape)}, got {t.dtype} {tuple(t.shape)}")
+    _gpu("decode_step", t)
+    _contig("decode_step", operand=t)
+    return t.data_ptr()
+
+
+def _packed_matrix(w, rows, cols):
+    return _PackedMatrix(_tensor_ptr(w.weight, (rows, cols // 8), torch.int32), *(_tensor_ptr(t, (rows, cols // 128), torch.bfloat16) for t in (w.scales, w.biases)))
+
+
+def decode_step_bytes(parts, bottom=None) -> int:
+    """What ``decode_step_pack`` makes of these packed layers: 2176 bytes for 4096 weights."""
+    weights = sum(w.weight.shape[0] * w.weight.shape[1] * 8 for w in parts)
+    return weights * (2 if bottom is not None else 1) // 4096 * 2176
+
+
+def decode_step_pack(parts, *, halves=False, bottom=None, out=None, stream=None) -> torch.Tensor:
+    """Packed layers (``weight`` / ``scales`` / ``biases``, rows concatenated) in the order in which ``DecodeStep`` reads them; ``bottom``: the up
+    projection beside a gate.  uint8, scales and biases included."""
+    cols, nbytes = parts[0].weight.shape[1] * 8, decode_step_bytes(parts, bottom)
+    if out is None:
+        out = torch.empty(nbytes, dtype=torch.uint8, device=parts[0].weight.device)
+    _tensor_ptr(out, (nbytes,), torch.uint8)
+    at = 0
+    for w in parts:
+        rows = w.weight.shape[0]
+        low = ctypes.byref(_packed_matrix(bottom, rows, cols)) if bottom is not None else None
+        _check(_lib.tl_decode_step_pack(ctypes.byref(_packed_matrix(w, rows, cols)), low, out.data_ptr() + at, rows, cols, int(halves), _stream_ptr(stream, out)))
+        at += decode_step_bytes([w], bottom)
+    return out
+
+
+class DecodeStep:
+    """A whole greedy decoding step of a few requests as one launch (``csrc/decode_step.cu``).  ``embedding`` is a packed layer, ``head`` and the
+    layers' ``qkv`` / ``o`` / ``gate_up`` / ``down`` come from ``decode_step_pack``; norms are ``(weight, eps)``; a layer is a dict of these with
+    ``input_norm``, ``post_norm``, ``q_norm``, ``k_norm``, ``key_pages``, ``value_pages``, ``block_table`` and ``scale``.  The object keeps the
+    tensors it points to; steps of one object follow one another in stream order."""
+
+    @staticmethod
+    def workspace_bytes(batch: int, layers: int, num_heads: int, num_kv_heads: int, hidden: int, intermediate: int, vocab: int) -> int:
+        """0: the one-launch step does not take these sizes."""
+        return int(_lib.tl_decode_step_workspace(batch, layers, num_heads, num_kv_heads, hidden, intermediate, vocab))
+
+    def __init__(self, *, tokens, offsets, context_lens, rope_inv_freq, embedding, head, norm, layers, logits, next_tokens, num_heads, num_kv_heads, intermediate):
+        B, V = logits.shape
+        hidden = embedding.weight.shape[1] * 8
+        P, Hkv, page_size, D = layers[0]["key_pages"].shape
+        max_pages = layers[0]["block_table"].shape[1]
+        nbytes = self.workspace_bytes(B, len(layers), num_heads, num_kv_heads, hidden, intermediate, V)
+        if nbytes == 0 or D != 128 or Hkv != num_kv_heads:
+            raise RuntimeError("decode_step: sizes the one-launch step does not take")
+        workspace = torch.zeros(nbytes, dtype=torch.uint8, device=logits.device)
+        q, qkv = num_heads * 128, (num_heads + 2 * num_kv_heads) * 128
+        bf, i32, u8 = torch.bfloat16, torch.int32, torch.uint8
+
+        def units(rows, cols):
+            return (rows * cols // 4096 * 2176,)
+
+        self._layers = (_DecodeStepLayer * len(layers))()
+        for to, one in zip(self._layers, layers):
+            for name, rows, cols in (("qkv", qkv, hidden), ("o", hidden, q), ("gate_up", 2 * intermediate, hidden), ("down", hidden, intermediate)):
+                setattr(to, name, _tensor_ptr(one[name], units(rows, cols), u8))
+            for name, n, eps in (("input_norm", hidden, "input_eps"), ("post_norm", hidden, "post_eps"), ("q_norm", 128, "q_eps"), ("k_norm", 128, "k_eps")):
+                setattr(to, name, _tensor_ptr(one[name][0], (n,), bf))
+                setattr(to, eps, one[name][1])
+            pages = one["key_pages"].shape[0]
+            for name in ("key_pages", "value_pages"):
+                setattr(to, name, _tensor_ptr(one[name], (pages, Hkv, page_size, D), bf))
+            to.num_pages, to.scale = pages, float(one["scale"])
+            to.block_table = _tensor_ptr(one["block_table"], (B, max_pages), i32)
+        self._plan = _DecodeStepPlan(
+            B, len(layers), num_heads, num_kv_heads, hidden, intermediate, V, page_size, max_pages, norm[1], _tensor_ptr(tokens, (B,), i32),
+            _tensor_ptr(offsets, (B,), i32), _tensor_ptr(context_lens, (B,), i32), _tensor_ptr(rope_inv_freq, (64,), torch.float64),
+            _packed_matrix(embedding, V, hidden), _tensor_ptr(head, units(V, hidden), u8), _tensor_ptr(norm[0], (hidden,), bf),
+            _tensor_ptr(logits, (B, V), bf), _tensor_ptr(next_tokens, (B,), i32), _tensor_ptr(workspace, (nbytes,), u8), nbytes, ctypes.addressof(self._layers))
+        self._keep = (tokens, offsets, context_lens, rope_inv_freq, embedding, head, norm, layers, logits, next_tokens, workspace)
+        self._ref = logits
+
+    def launch(self, stream=None) -> None:
+        _check(_lib.tl_decode_step(ctypes.byref(self._plan), _stream_ptr(stream, self._ref)))
 
 
 def set_pdl(enabled: bool) -> None:

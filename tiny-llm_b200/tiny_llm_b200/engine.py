@@ -26,7 +26,7 @@ front and the engine re-captures if a slab pointer changes.
 from __future__ import annotations
 
 import os
-
+from functools import cached_property
 from types import SimpleNamespace
 
 import numpy as np
@@ -64,6 +64,22 @@ def _interleave_gate_up(gate, up):
         group_size=gate.group_size,
         bits=gate.bits,
     )
+
+
+def _step_weights(model) -> dict:
+    """The packed matrices in the order in which the one-launch step reads them, made once for all of a model's engines (one allocation)."""
+    if model._step_weights is None:
+        head = model.w_lm_head if model.w_lm_head is not None else model.embedding.weight
+        wanted = [("head", dict(parts=[head]))]
+        for b in model.layers_inner:
+            at, mlp = b.self_attn, b.mlp
+            wanted += [("qkv", dict(parts=[at.wq, at.wk, at.wv], halves=True)), ("o", dict(parts=[at.wo], halves=True)),
+                       ("gate_up", dict(parts=[mlp.w_gate], bottom=mlp.w_up)), ("down", dict(parts=[mlp.w_down], halves=True))]
+        sizes = [ext.decode_step_bytes(w["parts"], w.get("bottom")) for _, w in wanted]
+        whole = torch.empty(sum(sizes), dtype=torch.uint8, device=head.scales.device).split(sizes)
+        made = [(name, ext.decode_step_pack(**w, out=out)) for (name, w), out in zip(wanted, whole)]
+        model._step_weights = {"head": made[0][1], "layers": [dict(made[i : i + 4]) for i in range(1, len(made), 4)]}
+    return model._step_weights
 
 
 class _LockstepGroup:
@@ -144,16 +160,6 @@ class DecodeEngine:
         self.kernels_per_step = 0
         rope = attn.rope
         self.fused = bool(fused) and not rope.traditional and rope.dims == self.D and self.D % 2 == 0
-        self._packed = None
-        if self.fused:
-            # q|k|v and gate|up share their input, so they stream as one launch each.
-            self._packed = [
-                SimpleNamespace(
-                    qkv=_concat_weights([b.self_attn.wq, b.self_attn.wk, b.self_attn.wv]),
-                    gate_up=_interleave_gate_up(b.mlp.w_gate, b.mlp.w_up),
-                )
-                for b in model.layers_inner
-            ]
         # one-launch attention (q/k norm + rope + append + paged GQA) when the head layout allows it
         attn0 = model.layers_inner[0].self_attn
         # The one-launch attention is a latency design (few CTAs, K/V rows staged per lane): it wins while the
@@ -169,6 +175,19 @@ class DecodeEngine:
         if self._attention_fused:
             self._rope_inv_freq = ext.rope_inv_freq_table(self.D, attn0.rope.base, self.device)
             self._attn_ws = torch.empty(ext.decode_attention_fused_workspace(self.B, self.Hq, self.Hkv), dtype=torch.float32, device=self.device)
+        # Up to four requests: the whole step is one launch (csrc/decode_step.cu) wherever the sizes fit it.  TL_DECODE_STEP=0: the chain of launches.
+        emb = model.embedding.weight
+        head = model.w_lm_head if model.w_lm_head is not None else emb
+        packed = [emb, head] + [w for b in model.layers_inner for w in (b.self_attn.wq, b.self_attn.wk, b.self_attn.wv, b.self_attn.wo, b.mlp.w_gate, b.mlp.w_up, b.mlp.w_down)]
+        hidden = emb.weight.shape[1] * 8
+        intermediate = model.layers_inner[0].mlp.w_gate.weight.shape[0]
+        self._one_launch = (self.fused and self.D == 128 and os.environ.get("TL_DECODE_STEP", "1") != "0"
+                            and all(w.group_size == 128 and w.bits == 4 and w.scales.dtype == torch.bfloat16
+                                    and all(t.is_contiguous() for t in (w.weight, w.scales, w.biases)) for w in packed)
+                            and head.weight.shape == emb.weight.shape
+                            and ext.DecodeStep.workspace_bytes(self.B, self.n_layers, self.Hq, self.Hkv, hidden, intermediate, self.V) > 0)
+        self._step = None
+        self._intermediate = intermediate
         # Row variants: the scheduler fills slots from index 0 (batch.py:220-226), so while few requests are live the
         # occupied slots are a prefix of the table.  A step graph over the first 16 / 32 rows is captured beside the
         # full one and step() replays the smallest that covers the highest occupied slot: every kernel of the wide
@@ -181,6 +200,17 @@ class DecodeEngine:
         self._variants = sorted({r for r in (16, 32, 64) if r < self.B} | {self.B}) if (self.fused and self.B > 16 and rows_env != "0") else [self.B]
         self._graphs: dict = {}
         self.variant_replays = {r: 0 for r in self._variants}
+
+    @cached_property
+    def _packed(self):
+        """q|k|v and gate|up share their input, so they stream as one launch each in the chain of launches (made when it is first run)."""
+        return [
+            SimpleNamespace(
+                qkv=_concat_weights([b.self_attn.wq, b.self_attn.wk, b.self_attn.wv]),
+                gate_up=_interleave_gate_up(b.mlp.w_gate, b.mlp.w_up),
+            )
+            for b in self.model.layers_inner
+        ]
 
     # ------------------------------------------------------------------ pools --
     def reserve_pools(self, pages_per_layer: int | None = None) -> None:
@@ -239,6 +269,9 @@ class DecodeEngine:
         ``rows``: only the first ``rows`` slots (a row variant, see __init__)."""
         m = self.model
         R = self.B if rows is None else rows
+        if self._step is not None:
+            self._step.launch()
+            return
         emb = m.embedding.weight
         x = ext.quantized_embedding(self.tokens[:R], emb.scales, emb.biases, emb.weight, emb.group_size, emb.bits)
         logits = self._forward_fused_layers(x, R)
@@ -305,9 +338,32 @@ class DecodeEngine:
         return ext.quantized_matmul_fused(head.scales, head.biases, head.weight, x, m.norm._weight_as(x.dtype, x.device),
                                           prologue=ext.PRO_RMSNORM, eps=m.norm.eps)
 
+    def _one_launch_step(self):
+        m, dev = self.model, self.device
+        if self.logits is None:
+            self.logits = torch.zeros((self.B, self.V), dtype=torch.bfloat16, device=dev)
+
+        def norm(n):
+            return n._weight_as(torch.bfloat16, dev), n.eps
+
+        layers = []
+        packed = _step_weights(m)
+        for i, (block, pk, pool) in enumerate(zip(m.layers_inner, packed["layers"], m.page_pools)):
+            at = block.self_attn
+            layers.append(dict(pk, input_norm=norm(block.input_layernorm),
+                               post_norm=norm(block.post_attention_layernorm), q_norm=norm(at.q_norm), k_norm=norm(at.k_norm), key_pages=pool._key_pages,
+                               value_pages=pool._value_pages, block_table=self.tables[i], scale=at.scale))
+        emb = m.embedding.weight
+        return ext.DecodeStep(tokens=self.tokens, offsets=self.offsets, context_lens=self.context_lens,
+                              rope_inv_freq=ext.rope_inv_freq_table(self.D, m.layers_inner[0].self_attn.rope.base, dev), embedding=emb,
+                              head=packed["head"], norm=norm(m.norm), layers=layers, logits=self.logits,
+                              next_tokens=self.next_tokens, num_heads=self.Hq, num_kv_heads=self.Hkv, intermediate=self._intermediate)
+
     def _capture(self) -> None:
         self.captures += 1
         self._slab_ptrs = self._slabs()
+        if self._one_launch:
+            self._step = self._one_launch_step()
         forward = self._forward_fused if self.fused else self._forward_unfused
         with torch.cuda.stream(self._stream):
             self._stream.wait_stream(torch.cuda.current_stream(self.device))

@@ -234,6 +234,7 @@ class Qwen3ModelWeek3:
         self.use_decode_graph: bool | None = None
         self.decode_graph_max_seq_len = 8192
         self._decode_engines: dict = {}
+        self._step_weights: dict | None = None
         self._applies_memo = None
         # B200 runtime: chunked-prefill steps (B == 1, 1 < L <= prefill_graph_len) of CUDA-resident paged requests
         # replay a captured chunk graph too (engine.PrefillEngine).  0 disables; None = automatic (128, the scheduler's
