@@ -89,6 +89,12 @@ int tl_quantized_matmul(const void *scales, const void *biases, const void *a, c
 int tl_quantized_gate_up(const void *gate_scales, const void *gate_biases, const void *gate_b, const void *up_scales, const void *up_biases,
                          const void *up_b, const void *a, void *gate_out, void *out, int M, int N, int K, int dtype, int gate_flags,
                          int up_flags, void *workspace, size_t workspace_bytes, void *stream);
+/* out alone, the same bits: both products come from one launch up to 128 rows.  scratch: M * K elements, undefined afterwards;
+ * workspace: tl_quantized_gated_workspace bytes (with less, as much as tl_quantized_gate_up wants, two launches). */
+size_t tl_quantized_gated_workspace(int M, int N, int K, int dtype, int gate_flags, int up_flags);
+int tl_quantized_gated(const void *gate_scales, const void *gate_biases, const void *gate_b, const void *up_scales, const void *up_biases,
+                       const void *up_b, const void *a, void *scratch, void *out, int M, int N, int K, int dtype, int gate_flags,
+                       int up_flags, void *workspace, size_t workspace_bytes, void *stream);
 
 /* Replaces quantized_embedding (tiny_llm_ext.h:40-41, quantized_matmul.cpp:82-101,
  * :242-273).  indices int32/uint32 [tokens] (bit pattern), weight [vocab, dim/8] u32,

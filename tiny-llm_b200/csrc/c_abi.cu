@@ -96,6 +96,13 @@ size_t tl_quantized_matmul_workspace(int M, int N, int K, int dtype, int use_sim
     return w4a16_gemm_workspace(M, N, K, dtype, use_split_k);
 }
 
+size_t tl_quantized_gated_workspace(int M, int N, int K, int dtype, int gate_flags, int up_flags) {
+    const size_t gate = tl_quantized_matmul_workspace(M, N, K, dtype, gate_flags & 1, gate_flags >> 1 & 1);
+    const size_t up = tl_quantized_matmul_workspace(M, N, K, dtype, up_flags & 1, up_flags >> 1 & 1);
+    const size_t one = gate > up ? gate : up;
+    return (gate_flags & up_flags & 1) && use_skinny_kernel(M, N, K, dtype, 1) ? 2 * one : one;
+}
+
 // gate (or NULL): out = silu(gate) * product, the product rounded to the storage type first
 static int quantized_product(const void *scales, const void *biases, const void *a, const void *b, void *out, const void *gate, int M, int N,
                              int K, int dtype, int use_simdgroup, int use_split_k, void *workspace, size_t workspace_bytes, cudaStream_t st) {
@@ -135,6 +142,22 @@ int tl_quantized_gate_up(const void *gate_scales, const void *gate_biases, const
     if (rc != TL_OK) return rc;
     return quantized_product(up_scales, up_biases, a, up_b, out, gate_out, M, N, K, dtype, up_flags & 1, up_flags >> 1 & 1, workspace, workspace_bytes,
                              as_stream(stream));
+}
+
+int tl_quantized_gated(const void *gate_scales, const void *gate_biases, const void *gate_b, const void *up_scales, const void *up_biases,
+                       const void *up_b, const void *a, void *scratch, void *out, int M, int N, int K, int dtype, int gate_flags,
+                       int up_flags, void *workspace, size_t workspace_bytes, void *stream) {
+    if (M > 0 && K > 0 && (!scratch || !out)) return fail(TL_EINVAL, "quantized_gate_up: null pointer");
+    // both products from one launch where they take the same kernel, which forms the same sums there
+    if (M > 0 && K > 0 && N > 0 && N % 128 == 0 && (gate_flags & up_flags & 1) && gate_scales && gate_biases && gate_b && up_scales && up_biases && up_b && a) {
+        int rc = TL_OK;
+        if (use_skinny_kernel(M, N, K, dtype, 1)
+                ? launch_w4a16_skinny_gate_up(gate_scales, gate_biases, gate_b, up_scales, up_biases, up_b, a, out, M, N, K, dtype, workspace, workspace_bytes, as_stream(stream), &rc)
+                : use_stream_kernel(M, N, K, dtype, 1) && launch_w4a16_gate_up(gate_scales, gate_biases, gate_b, up_scales, up_biases, up_b, a, out, M, N, K, dtype, as_stream(stream), &rc))
+            return rc;
+    }
+    return tl_quantized_gate_up(gate_scales, gate_biases, gate_b, up_scales, up_biases, up_b, a, scratch, out, M, N, K, dtype, gate_flags, up_flags, workspace,
+                                workspace_bytes, stream);
 }
 
 int tl_quantized_embedding(const void *indices, const void *scales, const void *biases, const void *weight, void *out,

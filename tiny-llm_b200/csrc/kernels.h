@@ -48,6 +48,9 @@ int launch_w4a16_stream(const void *scales, const void *biases, const void *a, c
 int launch_w4a16_fused(const void *scales, const void *biases, const void *b, void *out, const void *p0, const void *p1,
                        const void *residual, int M, int N, int K, int lda, int prologue, int epilogue, float eps, int dtype,
                        cudaStream_t st);
+// out = silu(a . gate^T) * (a . up^T) in one launch, the same bits as two; false: not these operands (more than 8 rows, alignment)
+bool launch_w4a16_gate_up(const void *gate_scales, const void *gate_biases, const void *gate_b, const void *up_scales, const void *up_biases, const void *up_b,
+                          const void *a, void *out, int M, int N, int K, int dtype, cudaStream_t st, int *rc);
 void set_use_pdl(bool on);
 bool use_pdl();
 int launch_w4a16_vanilla(const void *scales, const void *biases, const void *a, const void *b, void *out, int M,
@@ -75,6 +78,10 @@ bool qkv_planes_rope_supported(int Hq, int Hkv, int D, int dtype);
 int launch_qkv_planes_rope_append(const float *part, int splits, const void *q_norm_w, const void *k_norm_w, const int32_t *offsets,
                                   const int32_t *block_table, const int32_t *context_lens, void *q_out, void *key_pages, void *value_pages, int batch,
                                   int Hq, int Hkv, float base, float eps, int num_pages, int page_size, int max_pages, cudaStream_t st, bool chunk);
+
+// The same for 9 to 128 rows; ws holds the planes of both products (twice w4a16_skinny_workspace); false: one split, or a smaller workspace
+bool launch_w4a16_skinny_gate_up(const void *gate_scales, const void *gate_biases, const void *gate_b, const void *up_scales, const void *up_biases,
+                                 const void *up_b, const void *a, void *out, int M, int N, int K, int dtype, void *ws, size_t ws_bytes, cudaStream_t st, int *rc);
 
 // w4a16_gemm.cu (tcgen05 prefill GEMM)
 bool w4a16_gemm_supported(int M, int N, int K, int dtype);

@@ -79,6 +79,8 @@ struct SkArgs {
     int M, N, K;       // tokens, reduction, features
     int splits, gb_per_split;  // reduction split in units of 128-wide group blocks
     int epilogue;
+    const void *scales2, *biases2;  // DUAL: the up projection
+    int tiles;                      // DUAL: feature tiles of one projection
 };
 
 template <typename T>
@@ -102,9 +104,10 @@ __host__ __device__ constexpr uint32_t sk_instr_desc() {
            (static_cast<uint32_t>(SK_FEAT >> 4) << 24);
 }
 
-template <typename T, int NT, bool WIDE1>
+// DUAL: a gate and an up projection of one shape in one grid, the gate's tiles first, each cut as by itself (the planes, and so the sums, are the same).
+template <typename T, int NT, bool WIDE1, bool DUAL>
 __global__ void __launch_bounds__(SK_THREADS, SkSmem<NT, WIDE1>::CTAS_PER_SM)
-w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w, const SkArgs args) {
+w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_gate, const __grid_constant__ CUtensorMap tmap_up, const SkArgs args) {
     using Smem = SkSmem<NT, WIDE1>;
     constexpr int ASTAGES = Smem::ASTAGES;
     constexpr int PSTAGES = Smem::PSTAGES;
@@ -122,7 +125,10 @@ w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #define SK_TRC(role, i, k) do { } while (0)
 #endif
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tile = blockIdx.x / args.splits, split = blockIdx.x - tile * args.splits;
+    const int any_tile = blockIdx.x / args.splits, split = blockIdx.x - any_tile * args.splits;
+    const bool second = DUAL && any_tile >= args.tiles;
+    const int tile = second ? any_tile - args.tiles : any_tile;
+    const CUtensorMap &tmap_w = second ? tmap_up : tmap_gate;
     const int G = args.N / SK_GB;  // group blocks of the whole reduction = quantisation groups per row
     const int gb0 = min(split * args.gb_per_split, G), gb1 = min(gb0 + args.gb_per_split, G);
     const int n_gb = gb1 - gb0;
@@ -241,8 +247,8 @@ w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const uint32_t magic = SkNum<T>::MAGIC;
         const V2 offset2 = *reinterpret_cast<const V2 *>(&magic);
         const size_t srow = static_cast<size_t>(min(tile * SK_FEAT + row, args.K - 1)) * G;
-        const unsigned short *sc = reinterpret_cast<const unsigned short *>(args.scales) + srow + gb0;
-        const unsigned short *bi = reinterpret_cast<const unsigned short *>(args.biases) + srow + gb0;
+        const unsigned short *sc = reinterpret_cast<const unsigned short *>(second ? args.scales2 : args.scales) + srow + gb0;
+        const unsigned short *bi = reinterpret_cast<const unsigned short *>(second ? args.biases2 : args.biases) + srow + gb0;
         const uint32_t swz = static_cast<uint32_t>(row & 7);
         const unsigned char *p_row = ssm + Smem::P_OFF + row * 128;
         const uint32_t lane_base = tmem_d + (static_cast<uint32_t>((warp & 3) * 32) << 16) + Smem::D_COLS;
@@ -328,8 +334,8 @@ w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const int col0 = ((warp - 4) >> 2) * HALF_COLS;
         const bool reader = NT >= 64 || warp < 8;
         constexpr int CH = HALF_COLS < 32 ? HALF_COLS : 32;  // columns per tcgen05.ld (x16 or x32)
-        float *part = args.partials;
         const size_t plane = static_cast<size_t>(args.M) * args.K;
+        float *part = args.partials + (second ? args.splits * plane : 0);
         // ---- splits > 1: park the fp32 partial tile; w4a16_skinny_reduce_kernel adds the planes in split order
         if (args.splits > 1) {
             if (reader) {
@@ -416,8 +422,9 @@ void trace_bind_skinny(unsigned long long *buf, unsigned int *n, unsigned int ca
 // Adds the fp32 partial planes of a split reduction in split order (deterministic: same bits on every run and for
 // every CTA schedule) and applies the epilogue; one thread per output.  All `splits` loads of a thread are independent
 // and in flight together (the first version let the last CTA of a tile do this with dependent round trips: 40 us).
-// GATED: out = silu(res) * result, res the gate projection's output.
-template <typename T, bool GATED>
+// GATED: out = silu(res) * result, res the gate projection's output.  DUAL: out = silu(gate) * up, the planes of both, gate first.
+enum { SK_PLAIN = 0, SK_GATED = 1, SK_DUAL = 2 };
+template <typename T, int MODE>
 __global__ void __launch_bounds__(256) w4a16_skinny_reduce_kernel(const float *part, const T *res, T *out, int M, int K, int splits, int epilogue) {
     const size_t plane = static_cast<size_t>(M) * K;
     griddep_launch();
@@ -449,8 +456,12 @@ __global__ void __launch_bounds__(256) w4a16_skinny_reduce_kernel(const float *p
     const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= plane) return;
     T vb = from_f<T>(plane_sum(idx));
+    if (MODE == SK_DUAL) {
+        const float gate = to_f(vb);
+        vb = from_f<T>((gate / (1.0f + expf(-gate))) * to_f(from_f<T>(plane_sum(splits * plane + idx))));
+    }
     if (epilogue == SK_EPI_RESIDUAL) vb = from_f<T>(to_f(ld_cg(res + idx)) + to_f(vb));
-    if (GATED) {
+    if (MODE == SK_GATED) {
         const float gate = to_f(ld_cg(res + idx));
         vb = from_f<T>((gate / (1.0f + expf(-gate))) * to_f(vb));
     }
@@ -604,17 +615,17 @@ static int sk_cached_map(CUtensorMap *out, const void *ptr, int kind, cuuint64_t
     return TL_OK;
 }
 
-template <typename T, int NT, bool WIDE1 = false>
-static int skinny_launch(const CUtensorMap &ma, const CUtensorMap &mw, const SkArgs &args, int grid, cudaStream_t st) {
+template <typename T, int NT, bool WIDE1 = false, bool DUAL = false>
+static int skinny_launch(const CUtensorMap &ma, const CUtensorMap &mw, const CUtensorMap &mw2, const SkArgs &args, int grid, cudaStream_t st) {
     constexpr size_t smem = SkSmem<NT, WIDE1>::BYTES;
     static bool configured = false;
     if (!configured) {
-        if (cudaFuncSetAttribute(w4a16_skinny_kernel<T, NT, WIDE1>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
-            cudaFuncSetAttribute(w4a16_skinny_kernel<T, NT, WIDE1>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
+        if (cudaFuncSetAttribute(w4a16_skinny_kernel<T, NT, WIDE1, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
+            cudaFuncSetAttribute(w4a16_skinny_kernel<T, NT, WIDE1, DUAL>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
             return fail(TL_ECUDA, "quantized_matmul: cannot raise shared memory limit");
         configured = true;
     }
-    cudaError_t e = launch_chained(w4a16_skinny_kernel<T, NT, WIDE1>, dim3(grid), dim3(SK_THREADS), smem, st, ma, mw, args);
+    cudaError_t e = launch_chained(w4a16_skinny_kernel<T, NT, WIDE1, DUAL>, dim3(grid), dim3(SK_THREADS), smem, st, ma, mw, mw2, args);
     if (e != cudaSuccess) return fail(TL_ECUDA, "w4a16_skinny: launch failed: %s", cudaGetErrorString(e));
     TL_LAUNCH_CHECK("w4a16_skinny");
     return TL_OK;
@@ -643,10 +654,10 @@ static int skinny_t(const void *scales, const void *biases, const void *a, const
     const int grid = tiles * args.splits;
     int rc;
     switch (NT) {
-        case 16: rc = skinny_launch<T, 16>(ma, mw, args, grid, st); break;
-        case 32: rc = skinny_launch<T, 32>(ma, mw, args, grid, st); break;
-        case 64: rc = skinny_launch<T, 64>(ma, mw, args, grid, st); break;
-        default: rc = skinny_wide1() ? skinny_launch<T, 128, true>(ma, mw, args, grid, st) : skinny_launch<T, 128>(ma, mw, args, grid, st); break;
+        case 16: rc = skinny_launch<T, 16>(ma, mw, mw, args, grid, st); break;
+        case 32: rc = skinny_launch<T, 32>(ma, mw, mw, args, grid, st); break;
+        case 64: rc = skinny_launch<T, 64>(ma, mw, mw, args, grid, st); break;
+        default: rc = skinny_wide1() ? skinny_launch<T, 128, true>(ma, mw, mw, args, grid, st) : skinny_launch<T, 128>(ma, mw, mw, args, grid, st); break;
     }
     if (planes_out != nullptr) {  // the caller adds the planes itself (fused consumer); 1 = `out` holds the finished result
         *planes_out = args.splits;
@@ -665,12 +676,58 @@ static int skinny_t(const void *scales, const void *biases, const void *a, const
         return TL_OK;
     }
     const size_t outputs = static_cast<size_t>(M) * (epilogue == SK_EPI_SWIGLU_PAIRS ? K / 2 : K);
-    cudaError_t e = launch_chained(epilogue == SK_EPI_GATED ? w4a16_skinny_reduce_kernel<T, true> : w4a16_skinny_reduce_kernel<T, false>, dim3(static_cast<unsigned>((outputs + 255) / 256)), dim3(256), 0, st,
+    cudaError_t e = launch_chained(epilogue == SK_EPI_GATED ? w4a16_skinny_reduce_kernel<T, SK_GATED> : w4a16_skinny_reduce_kernel<T, SK_PLAIN>, dim3(static_cast<unsigned>((outputs + 255) / 256)), dim3(256), 0, st,
                                    static_cast<const float *>(args.partials), static_cast<const T *>(residual), static_cast<T *>(out), M, K,
                                    args.splits, epilogue);
     if (e != cudaSuccess) return fail(TL_ECUDA, "w4a16_skinny_reduce: launch failed: %s", cudaGetErrorString(e));
     TL_LAUNCH_CHECK("w4a16_skinny_reduce");
     return TL_OK;
+}
+
+// One launch for both products and one that adds the planes: 52 rows of 2560 -> 2 x 9728, four launches before.
+template <typename T>
+static bool skinny_gate_up(SkArgs args, const void *a, const void *gate_b, const void *up_b, void *ws, size_t ws_bytes, cudaStream_t st, int *rc) {
+    const int M = args.M, N = args.N, K = args.K;
+    args.splits = w4a16_skinny_splits(M, N, K);
+    if (args.splits == 1 || ws == nullptr || ws_bytes < 2 * w4a16_skinny_workspace(M, N, K) || !aligned16(a) || !aligned16(gate_b) || !aligned16(up_b)) return false;
+    const int NT = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
+    args.tiles = (K + SK_FEAT - 1) / SK_FEAT;
+    args.gb_per_split = (N / SK_GB + args.splits - 1) / args.splits;
+    args.partials = static_cast<float *>(ws);
+    args.epilogue = SK_EPI_NONE;
+    CUtensorMap ma, mg, mu;
+    const CUtensorMapDataType dt = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    *rc = sk_cached_map(&ma, a, 0, N, M, SK_KB, NT, dt, 2);
+    for (int i = 0; i < 2 && *rc == TL_OK; ++i)
+        *rc = sk_cached_map(i ? &mu : &mg, i ? up_b : gate_b, 1, static_cast<cuuint64_t>(N) / 2, K, SK_PG * SK_GB / 2, SK_FEAT, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1);
+    if (*rc != TL_OK) return true;
+    const int grid = 2 * args.tiles * args.splits;
+    switch (NT) {
+        case 16: *rc = skinny_launch<T, 16, false, true>(ma, mg, mu, args, grid, st); break;
+        case 32: *rc = skinny_launch<T, 32, false, true>(ma, mg, mu, args, grid, st); break;
+        case 64: *rc = skinny_launch<T, 64, false, true>(ma, mg, mu, args, grid, st); break;
+        default: *rc = skinny_launch<T, 128, false, true>(ma, mg, mu, args, grid, st); break;
+    }
+    if (*rc != TL_OK) return true;
+    const size_t outputs = static_cast<size_t>(M) * K;
+    const cudaError_t e = launch_chained(w4a16_skinny_reduce_kernel<T, SK_DUAL>, dim3(static_cast<unsigned>((outputs + 255) / 256)), dim3(256), 0, st,
+                                         static_cast<const float *>(args.partials), static_cast<const T *>(nullptr), static_cast<T *>(args.out), M, K, args.splits, SK_EPI_NONE);
+    if (e != cudaSuccess) {
+        *rc = fail(TL_ECUDA, "w4a16_skinny_reduce: launch failed: %s", cudaGetErrorString(e));
+        return true;
+    }
+    count_launch();
+    *rc = check_launch("w4a16_skinny_reduce");
+    return true;
+}
+
+bool launch_w4a16_skinny_gate_up(const void *gate_scales, const void *gate_biases, const void *gate_b, const void *up_scales, const void *up_biases,
+                                 const void *up_b, const void *a, void *out, int M, int N, int K, int dtype, void *ws, size_t ws_bytes, cudaStream_t st, int *rc) {
+    SkArgs args{};
+    args.scales = gate_scales, args.biases = gate_biases, args.scales2 = up_scales, args.biases2 = up_biases, args.out = out;
+    args.M = M, args.N = N, args.K = K;
+    return dtype == TL_F16 ? skinny_gate_up<__half>(args, a, gate_b, up_b, ws, ws_bytes, st, rc)
+                           : dtype == TL_BF16 && skinny_gate_up<__nv_bfloat16>(args, a, gate_b, up_b, ws, ws_bytes, st, rc);
 }
 
 int launch_w4a16_skinny(const void *scales, const void *biases, const void *a, const void *b, void *out, const void *residual, int M, int N,

@@ -75,6 +75,8 @@ _SIGNATURES = {
     "tl_quantized_matmul_workspace": (_SZ, [_I] * 6),
     "tl_quantized_matmul": (_I, [_VP] * 5 + [_I] * 6 + [_VP, _SZ, _VP]),
     "tl_quantized_gate_up": (_I, [_VP] * 9 + [_I] * 6 + [_VP, _SZ, _VP]),
+    "tl_quantized_gated_workspace": (_SZ, [_I] * 6),
+    "tl_quantized_gated": (_I, [_VP] * 9 + [_I] * 6 + [_VP, _SZ, _VP]),
     "tl_quantized_embedding": (_I, [_VP] * 5 + [_I] * 4 + [_VP]),
     "tl_rms_norm": (_I, [_VP] * 3 + [_I, _I, _F, _I, _VP]),
     "tl_rope": (_I, [_VP] * 3 + [_I] * 5 + [_F, _I, _I, _VP]),
@@ -270,8 +272,8 @@ def _check_quantized_matmul(scales, biases, group_size, bits, a, b, transpose_b)
 
 
 def quantized_gate_up(a, gate, up, gate_flags=(True, False), up_flags=(True, False), stream=None):
-    """``silu(a @ gate.T) * (a @ up.T)`` of two quantised weights ``(scales, biases, packed)`` of one shape: the gate's product, then the
-    up projection with the activation in its epilogue.  The flags are (use_simdgroup, use_split_k) of either product.  The same bits as two
+    """``silu(a @ gate.T) * (a @ up.T)`` of two quantised weights ``(scales, biases, packed)`` of one shape: both from one launch up to 128
+    rows, else the gate's product, then the up projection with the activation.  The flags are (use_simdgroup, use_split_k) of either product.  The same bits as two
     ``quantized_matmul`` calls and ``swiglu``."""
     for scales, biases, packed in (gate, up):
         if not _quantized_matmul_fits(scales, biases, 128, 4, a, packed):
@@ -280,12 +282,13 @@ def quantized_gate_up(a, gate, up, gate_flags=(True, False), up_flags=(True, Fal
     if up[2].shape[0] != K:
         raise RuntimeError("swiglu: gate and up must have the same shape and dtype")
     gate_out, out = a.new_empty((M, K)), a.new_empty((M, K))
-    ws_bytes = max(_lib.tl_quantized_matmul_workspace(M, N, K, code, int(s), int(k)) for s, k in {gate_flags, up_flags})
+    flags = int(gate_flags[0]) + 2 * int(gate_flags[1]), int(up_flags[0]) + 2 * int(up_flags[1])
+    ws_bytes = _lib.tl_quantized_gated_workspace(M, N, K, code, *flags)
     ws = _zero_workspace(ws_bytes, a.device) if ws_bytes else None
     _check(
-        _lib.tl_quantized_gate_up(
+        _lib.tl_quantized_gated(
             gate[0].data_ptr(), gate[1].data_ptr(), gate[2].data_ptr(), up[0].data_ptr(), up[1].data_ptr(), up[2].data_ptr(), a.data_ptr(),
-            gate_out.data_ptr(), out.data_ptr(), M, N, K, code, int(gate_flags[0]) + 2 * int(gate_flags[1]), int(up_flags[0]) + 2 * int(up_flags[1]),
+            gate_out.data_ptr(), out.data_ptr(), M, N, K, code, *flags,
             None if ws is None else ws.data_ptr(), ws_bytes, _stream_ptr(stream, a),
         )
     )

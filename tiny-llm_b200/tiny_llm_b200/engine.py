@@ -364,6 +364,8 @@ class DecodeEngine:
         self._slab_ptrs = self._slabs()
         if self._one_launch:
             self._step = self._one_launch_step()
+        elif self.fused:
+            self._packed  # made on the caller's stream, not on the one that captures
         forward = self._forward_fused if self.fused else self._forward_unfused
         with torch.cuda.stream(self._stream):
             self._stream.wait_stream(torch.cuda.current_stream(self.device))
