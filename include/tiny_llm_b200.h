@@ -95,6 +95,14 @@ size_t tl_quantized_gated_workspace(int M, int N, int K, int dtype, int gate_fla
 int tl_quantized_gated(const void *gate_scales, const void *gate_biases, const void *gate_b, const void *up_scales, const void *up_biases,
                        const void *up_b, const void *a, void *scratch, void *out, int M, int N, int K, int dtype, int gate_flags,
                        int up_flags, void *workspace, size_t workspace_bytes, void *stream);
+/* A whole gated MLP, out [M, out_features] = (silu(a . gate^T) * (a . up^T)) . down^T: tl_quantized_gated and tl_quantized_matmul in one call.
+ * flags: 2 bits (1 = use_simdgroup, 2 = use_split_k) each for gate, up and down, gate lowest.  scratch: 2 * M * K elements; the matrices' structs are HOST. */
+typedef struct tl_packed_matrix {
+    const void *weight, *scales, *biases;
+} tl_packed_matrix;
+size_t tl_quantized_mlp_workspace(int M, int N, int K, int out_features, int dtype, int flags);
+int tl_quantized_mlp(const tl_packed_matrix *gate, const tl_packed_matrix *up, const tl_packed_matrix *down, const void *a, void *scratch, void *out, int M, int N,
+                     int K, int out_features, int dtype, int flags, void *workspace, size_t workspace_bytes, void *stream);
 
 /* Replaces quantized_embedding (tiny_llm_ext.h:40-41, quantized_matmul.cpp:82-101,
  * :242-273).  indices int32/uint32 [tokens] (bit pattern), weight [vocab, dim/8] u32,
@@ -251,9 +259,6 @@ int tl_decode_attention_fused(const void *qkv, const void *q_norm_weight, const 
  * read during the call; every pointer in it is a device pointer.  Matrices other than the embedding table are tl_decode_step_pack()'s
  * results: q|k|v (rows concatenated), o and down packed with halves = 1, gate (top) and up (bottom) together, the head with neither.  workspace: tl_decode_step_workspace() bytes, zeroed once, used by one step at a time and kept between steps;
  * 0 bytes: these sizes are not taken. */
-typedef struct tl_packed_matrix {
-    const void *weight, *scales, *biases;
-} tl_packed_matrix;
 typedef struct tl_decode_step_layer {
     const void *qkv, *o, *gate_up, *down;
     const void *input_norm, *post_norm, *q_norm, *k_norm;

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from extensions_b200 import tiny_llm_ext_b200 as ext
-from tiny_llm_b200.quantize import QuantizedWeights, quantized_gate_up, quantized_linear
+from tiny_llm_b200.quantize import QuantizedWeights, quantized_gate_up, quantized_linear, quantized_mlp
 
 pytestmark = pytest.mark.gpu
 
@@ -64,3 +64,21 @@ def test_the_gate_is_kept_for_the_stream_that_reads_it():
     torch.cuda.current_stream().synchronize()
     side.synchronize()
     assert torch.equal(got, want) and all(bool(t.isnan().all()) for t in taken)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M", [1, 8, 9, 52, 128, 129, 700])
+def test_the_whole_mlp_in_one_call_equals_its_products(M, dtype):
+    wrap = lambda w, **flags: QuantizedWeights(scales=w[0], biases=w[1], group_size=128, bits=4, weight=w[2], **flags)
+    gate, up, down = (wrap(weight(k, n, dtype, s), use_simdgroup_matmul=True, use_split_k_matmul=True) for k, n, s in ((1408, 768, 1), (1408, 768, 2), (520, 1408, 3)))
+    x = torch.randn(2, M, 768, device="cuda").to(dtype) * 4
+    for form in (x[:1], x, x.transpose(0, 1), x[:, :, :768][0], x[:, ::2]):  # one, three and two dimensions, rows that do not follow one another
+        want = quantized_linear(quantized_gate_up(form, gate, up), down)
+        got = quantized_mlp(form, gate, up, down)
+        assert got.shape == want.shape and torch.equal(got, want)
+    with pytest.raises(RuntimeError, match="0 elements"):
+        quantized_mlp(x[:, :0], gate, up, down)
+    with pytest.raises(RuntimeError, match="a must be the same dtype as scales"):
+        quantized_mlp(x.float(), gate, up, down)
+    with pytest.raises(RuntimeError, match="one column per input group"):
+        quantized_mlp(x[..., :640].contiguous(), gate, up, down)

@@ -160,6 +160,25 @@ int tl_quantized_gated(const void *gate_scales, const void *gate_biases, const v
                                 workspace_bytes, stream);
 }
 
+size_t tl_quantized_mlp_workspace(int M, int N, int K, int out_features, int dtype, int flags) {
+    const size_t gated = tl_quantized_gated_workspace(M, N, K, dtype, flags & 3, flags >> 2 & 3);
+    const size_t down = tl_quantized_matmul_workspace(M, K, out_features, dtype, flags >> 4 & 1, flags >> 5 & 1);
+    return gated > down ? gated : down;
+}
+
+int tl_quantized_mlp(const tl_packed_matrix *gate, const tl_packed_matrix *up, const tl_packed_matrix *down, const void *a, void *scratch, void *out, int M, int N,
+                     int K, int out_features, int dtype, int flags, void *workspace, size_t workspace_bytes, void *stream) {
+    if (!gate || !up || !down || (M > 0 && K > 0 && !scratch)) return fail(TL_EINVAL, "quantized_mlp: null pointer");
+    if (dtype != TL_F16 && dtype != TL_BF16) return fail(TL_EDTYPE, "quantized_matmul: scales must be float16 or bfloat16");
+    if (M < 0 || N <= 0 || K <= 0 || K % 128 != 0) return fail(TL_EINVAL, "quantized_matmul: N must be divisible by group_size");
+    void *const gate_out = static_cast<unsigned char *>(scratch) + static_cast<size_t>(M) * K * 2;  // behind the activations
+    const int rc = tl_quantized_gated(gate->scales, gate->biases, gate->weight, up->scales, up->biases, up->weight, a, gate_out, scratch, M, N, K, dtype, flags & 3,
+                                      flags >> 2 & 3, workspace, workspace_bytes, stream);
+    if (rc != TL_OK) return rc;
+    return tl_quantized_matmul(down->scales, down->biases, scratch, down->weight, out, M, K, out_features, dtype, flags >> 4 & 1, flags >> 5 & 1, workspace,
+                               workspace_bytes, stream);
+}
+
 int tl_quantized_embedding(const void *indices, const void *scales, const void *biases, const void *weight, void *out,
                            int tokens, int vocab, int dim, int dtype, void *stream) {
     if (tokens < 0 || vocab <= 0 || dim <= 0 || dim % 128 != 0)

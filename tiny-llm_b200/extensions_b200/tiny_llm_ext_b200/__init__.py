@@ -67,6 +67,10 @@ _F = ctypes.c_float
 _LL = ctypes.c_longlong
 _SZ = ctypes.c_size_t
 
+class _PackedMatrix(ctypes.Structure):
+    _fields_ = [(n, _VP) for n in ("weight", "scales", "biases")]
+
+
 _SIGNATURES = {
     "tl_abi_version": (_I, []),
     "tl_last_error": (ctypes.c_char_p, []),
@@ -77,6 +81,8 @@ _SIGNATURES = {
     "tl_quantized_gate_up": (_I, [_VP] * 9 + [_I] * 6 + [_VP, _SZ, _VP]),
     "tl_quantized_gated_workspace": (_SZ, [_I] * 6),
     "tl_quantized_gated": (_I, [_VP] * 9 + [_I] * 6 + [_VP, _SZ, _VP]),
+    "tl_quantized_mlp_workspace": (_SZ, [_I] * 6),
+    "tl_quantized_mlp": (_I, [_VP] * 6 + [_I] * 6 + [_VP, _SZ, _VP]),
     "tl_quantized_embedding": (_I, [_VP] * 5 + [_I] * 4 + [_VP]),
     "tl_rms_norm": (_I, [_VP] * 3 + [_I, _I, _F, _I, _VP]),
     "tl_rope": (_I, [_VP] * 3 + [_I] * 5 + [_F, _I, _I, _VP]),
@@ -294,6 +300,38 @@ def quantized_gate_up(a, gate, up, gate_flags=(True, False), up_flags=(True, Fal
     )
     if stream is not None:  # freed on return, while that stream may still have to read it
         gate_out.record_stream(stream)
+    return out
+
+
+def quantized_mlp(a, gate, up, down, flags, stream=None):
+    """``(silu(a @ gate.T) * (a @ up.T)) @ down.T`` of three packed layers in one call, the bits of ``quantized_gate_up`` and ``quantized_matmul``; flags:
+    ``tl_quantized_mlp``'s.  None: operands that go through those two, for their checks and forms."""
+    dtype = a.dtype
+    code = _DTYPE_CODE.get(dtype)
+    (M, N), K = a.shape, gate.weight.shape[0]
+    made = []
+    for w, rows, cols in ((gate, K, N), (up, K, N), (down, down.weight.shape[0], K)):
+        s, b, p = w.scales, w.biases, w.weight
+        groups = (rows, cols // 128)
+        if not (s.dtype is dtype and b.dtype is dtype and p.dtype in _PACKED and w.bits == 4 and w.group_size == 128 and cols % 128 == 0
+                and p.shape == (rows, cols // 8) and s.shape == groups and b.shape == groups and s.is_cuda and b.is_cuda and p.is_cuda
+                and s.is_contiguous() and b.is_contiguous() and p.is_contiguous()):
+            return None
+        made.append(_PackedMatrix(p.data_ptr(), s.data_ptr(), b.data_ptr()))
+    if code not in (1, 2) or not a.is_cuda or not a.is_contiguous() or M == 0 or K == 0:
+        return None
+    out, scratch = a.new_empty((M, rows)), a.new_empty(2 * M * K)
+    ws_bytes = _lib.tl_quantized_mlp_workspace(M, N, K, rows, code, flags)
+    ws = _zero_workspace(ws_bytes, a.device) if ws_bytes else None
+    ref = ctypes.byref
+    _check(
+        _lib.tl_quantized_mlp(
+            ref(made[0]), ref(made[1]), ref(made[2]), a.data_ptr(), scratch.data_ptr(), out.data_ptr(), M, N, K, rows, code, flags,
+            None if ws is None else ws.data_ptr(), ws_bytes, _stream_ptr(stream, a),
+        )
+    )
+    if stream is not None:  # freed on return, while that stream may still have to read it
+        scratch.record_stream(stream)
     return out
 
 
@@ -821,10 +859,6 @@ def decode_attention_fused(qkv, q_norm_weight, k_norm_weight, offsets, block_tab
         )
     )
     return out
-
-
-class _PackedMatrix(ctypes.Structure):
-    _fields_ = [(n, _VP) for n in ("weight", "scales", "biases")]
 
 
 class _DecodeStepLayer(ctypes.Structure):

@@ -161,6 +161,20 @@ def quantized_gate_up(x: torch.Tensor, gate: QuantizedWeights, up: QuantizedWeig
     return tiny_llm_ext_b200.quantized_gate_up(rows, *parts, _kernel_flags(gate, rows.shape[0]), _kernel_flags(up, rows.shape[0])).reshape(*lead, -1)
 
 
+def quantized_mlp(x: torch.Tensor, gate: QuantizedWeights, up: QuantizedWeights, down: QuantizedWeights) -> torch.Tensor:
+    """``quantized_linear(quantized_gate_up(x, gate, up), down)``, in one call where the operands allow it."""
+    if x.is_cuda and x.dim() > 1 and gate.weight.shape == up.weight.shape:
+        rows = x.reshape(-1, x.shape[-1])
+        flags = 0
+        for i, w in enumerate((gate, up, down)):
+            simdgroup, split_k = _kernel_flags(w, rows.shape[0])
+            flags |= (bool(simdgroup) + 2 * bool(split_k)) << 2 * i
+        y = tiny_llm_ext_b200.quantized_mlp(rows, gate, up, down, flags)
+        if y is not None:
+            return y.view(*x.shape[:-1], -1)
+    return quantized_linear(quantized_gate_up(x, gate, up), down)
+
+
 def dequantize_weights(
     weight: torch.Tensor,
     scales: torch.Tensor,

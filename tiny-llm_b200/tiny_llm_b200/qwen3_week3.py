@@ -19,7 +19,7 @@ from .attention import paged_attention
 from .embedding import QuantizedEmbedding
 from .kv_cache import TinyKvCache
 from .paged_kv_cache import TinyKvPagedCache, TinyKvPagedPool
-from .quantize import QuantizedWeights, quantized_gate_up, quantized_linear
+from .quantize import QuantizedWeights, quantized_linear, quantized_mlp
 from .week2_kernels import (
     FastRMSNorm,
     FastRoPE,
@@ -106,7 +106,7 @@ class Qwen3MLP:
         self.w_gate, self.w_up, self.w_down = w_gate, w_up, w_down
 
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
-        return quantized_linear(quantized_gate_up(x, self.w_gate, self.w_up), self.w_down)
+        return quantized_mlp(x, self.w_gate, self.w_up, self.w_down)
 
 
 class Qwen3TransformerBlock:
