@@ -37,6 +37,63 @@ def test_decay_scan_against_float64(H, dk, dv, counts, dtype):
     assert torch.equal(state[0], start[0])
 
 
+@pytest.mark.parametrize("kind", [0, 2])
+@pytest.mark.parametrize("H,dk,dv", [(2, 32, 32), (1, 64, 160), (3, 64, 96), (2, 32, 128)])
+@pytest.mark.parametrize("counts,start", [([65], 0), ([64, 80], 63), ([200, 1, 17], 0), ([129, 128], 64)])
+def test_long_portions_on_the_tensor_cores_against_float64(H, dk, dv, counts, start, kind):
+    """Rows inside a fused projection, columns that end inside a warp's or a CTA's, strong and weak decays, a bias, a sequence without a slot."""
+    from extensions_b200.tiny_llm_ext_b200 import blocks
+
+    T, g = sum(counts), torch.Generator(device="cuda").manual_seed(11 + dk + dv)
+    fused = torch.randn(T, H * (2 * dk + dv) + 8, generator=g, device="cuda").bfloat16()
+    q, k, v = (x.unflatten(1, (H, -1)) for x in fused[:, 8:].split([H * dk, H * dk, H * dv], dim=1))
+    z = torch.randn(T, H * dk, generator=g, device="cuda") * 3 - (2 if kind == 2 else 0)  # some channels forget everything within a token
+    bias = torch.randn(H * dk, generator=g, device="cuda").bfloat16()
+    state = torch.randn(len(counts) + 1, H, dk, dv, generator=g, device="cuda")
+    before, first, info = state.clone(), 0, []
+    for s, n in enumerate(counts):
+        info.append((first, n, start, s + 1 if s != 1 else -1))
+        first += n
+    info_t = torch.tensor(info, dtype=torch.int32, device="cuda")
+    out = blocks.decay_scan(q, k, v, z, bias, q_scale=dk**-0.5, seq_info=info_t, state=state, max_tokens=max(counts), tau=2.0, decay_kind=kind)
+    zz = (z + bias.float()).double().view(T, H, dk)
+    decay = torch.exp(-torch.exp(zz)) if kind == 2 else torch.exp(torch.nn.functional.logsigmoid(zz) / 2.0)
+    for first, n, p, slot in info:
+        S = before[slot].double() if p and slot > 0 else torch.zeros(H, dk, dv, dtype=torch.float64, device="cuda")
+        size = S.abs()
+        for t in range(first, first + n):
+            pair = k[t].double()[:, :, None] * v[t].double()[:, None, :]
+            S, size = decay[t][:, :, None] * S + pair, decay[t][:, :, None] * size + pair.abs()
+            want, terms = (torch.einsum("hk,hkv->hv", x, y) * dk**-0.5 for x, y in ((q[t].double(), S), (q[t].double().abs(), size)))
+            # a term passes at most n decays, each off by a few units in 2^-24 and, as an exponential, by that times its exponent (at most 16 where it still counts)
+            assert bool(((out[t].double() - want).abs() <= 2.0**-24 * (24 * n + dk) * terms).all())
+        if slot > 0:
+            assert bool(((state[slot].double() - S).abs() <= 2.0**-24 * 24 * n * size).all())
+    assert torch.equal(state[0], before[0]) and (len(counts) < 2 or torch.equal(state[2], before[2]))
+
+
+@pytest.mark.parametrize("act", [0, 1, 2])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("T,H,dv", [(1, 1, 4), (5, 3, 128), (3, 2, 132), (4, 2, 256), (2, 2, 512), (2, 2, 516), (3, 2, 66)])
+def test_head_norm_and_gate_against_float64(T, H, dv, dtype, act):
+    """Widths of one, two and four pieces a lane, ragged ones, and those that are not taken whole."""
+    from extensions_b200.tiny_llm_ext_b200 import blocks
+
+    g = torch.Generator(device="cuda").manual_seed(T + dv)
+    o = torch.randn(T, H, dv, generator=g, device="cuda")
+    gate = torch.randn(T, H * dv + 4, generator=g, device="cuda").to(dtype)[:, 4:]
+    for w in (None, torch.randn(dv, generator=g, device="cuda").to(dtype), torch.randn(H * dv, generator=g, device="cuda").to(dtype)):
+        for first in (False, True):
+            got = blocks.head_norm_gate(o, w, 1e-5, gate, act=act, gate_first=first)
+            x, y = o.double(), gate.double().view(T, H, dv)
+            y = y * torch.sigmoid(y) if act == 1 else torch.sigmoid(y) if act == 2 else y
+            n = x * y if first else x
+            want = n * torch.rsqrt(n.square().mean(-1, keepdim=True) + 1e-5) * (1 if first else y)
+            want = want.reshape(T, -1) * (1 if w is None else w.double() if w.numel() == H * dv else w.double().repeat(H))
+            unit = 2.0**-8 if dtype == torch.bfloat16 else 2.0**-20
+            assert bool(((got.double() - want).abs() <= unit * want.abs() + 1e-30).all())
+
+
 @pytest.mark.parametrize("T,D,E,top", [(1, 64, 8, 2), (5, 1000, 16, 2), (37, 2048, 64, 6), (150, 520, 24, 3)])
 def test_router_and_expert_sum_against_float64(T, D, E, top):
     from extensions_b200.tiny_llm_ext_b200 import blocks

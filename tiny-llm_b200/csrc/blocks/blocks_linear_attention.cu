@@ -19,7 +19,8 @@
 // indices alone; the cuts depend on positions only, so how a prompt was cut into steps changes the result by the
 // rounding of the combination at most.
 // 2048 tokens in two sequences, 16 heads of 64 x 128: 208 + 9 + 208 us (the recurrence twice, a column a thread) -> 99 + 19 + 24.
-// The scan is bound by instructions and the staging's round trips: 25 M of its 50 M are multiply-adds.
+// The scan is bound by instructions and the staging's round trips: 25 M of its 50 M are multiply-adds.  Long portions with a decay per key channel take
+// the tensor cores instead (decay_chunk_kernel below).
 #include <type_traits>
 
 #include "blocks_common.cuh"
@@ -430,6 +431,346 @@ decay_output_kernel(const int32_t *__restrict__ seq_info, int heads, int dk, int
     }
 }
 
+// ---- portions of more than a segment with a decay per key channel, on the tensor cores ------------------------------------------------
+// Sixteen tokens at a time, A_t the product of the decays up to token t of the sixteen and R_s that of the decays behind token s:
+//     o_t = sum_d q_t[d] A_t[d] S[d, :]  +  sum_{s <= t} P[t, s] v_s        P[t, s] = sum_d q_t[d] k_s[d] decay(s+1 .. t)[d]
+//     S  <- diag(A_16) S + sum_s (k_s R_s) v_s^T
+// All factors are products of decays, at most 1, whatever the decays are.  P is formed in fp32 as it stands (each token's key times the decays
+// one after another); the three products run on mma.sync with fp32 sums.  Its operands are 16-bit: v is bf16 as it is; q A, k R, P and S, which are fp32, enter
+// as three bf16 terms each (24 bits; of nine products of two such operands the three below 2^-24 are left out).  The tensor cores cut their sums off where a
+// multiply-add rounds, so no long sum is left to them: products of 16 start from zero and are added in fp32.
+// S^T [columns, channels] stays in accumulator fragments, which are the A operand's layout too: a warp owns 32 columns.
+//
+// Three launches: every segment's end state from zero (its first one's from the sequence's own state) and its decay (MODE 0); the segments' start states, in
+// order; the outputs from the start states, and the last segment's end state to the slot (MODE 1).
+// 2048 tokens in two sequences of 16 heads of 64 x 128: the walk in segments 99 + 19 + 24 us, this 18 + 8 + 48 (8 + 8 heads 1.6 x, 65 tokens 1.1 x, 8000
+// tokens 2 x as fast); the error against 64 bits is 0.85 to 1.0 of the walk's (with long sums left to the tensor cores it was twice that, at 42 us).
+// What bounds it: instructions, of which the terms of S are a quarter, and three barriers every sixteen tokens with 14 warps an SM.
+constexpr int kCkTokens = 16, kCkCols = 128;
+
+__device__ __forceinline__ void ck_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ck_ldm(uint32_t (&r)[4], const bf16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p)))
+                 : "memory");
+}
+__device__ __forceinline__ void ck_ldm_t(uint32_t (&r)[4], const bf16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p)))
+                 : "memory");
+}
+// x, y as three pairs of bf16: x = x0 + x1 + x2 up to 2^-24 of it
+__device__ __forceinline__ void ck_split(float x, float y, uint32_t (&term)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        term[i] = tl::pack2<bf16>(x, y);
+        if (i < 2) {
+            const float2 f = tl::unpack2<bf16>(term[i]);
+            x -= f.x, y -= f.y;
+        }
+    }
+}
+
+template <int DK, int MODE>
+__global__ void __launch_bounds__(128, 4)
+decay_chunk_kernel(const bf16 *__restrict__ q, long long q_token, long long q_head, const bf16 *__restrict__ k, long long k_token, long long k_head,
+                   const bf16 *__restrict__ v, long long v_token, long long v_head, const float *__restrict__ z, long long z_token,
+                   const bf16 *__restrict__ z_bias, float inv_tau, float q_scale, int heads, int dv, const int32_t *__restrict__ seq_info,
+                   float *__restrict__ state, long long slot_stride, int num_slots, float *__restrict__ out, int max_segments,
+                   float *__restrict__ seg_state, float *__restrict__ seg_decay, int decay_kind) {
+    constexpr int ROW = DK + 8, VROW = kCkCols + 8, PROW = kCkTokens + 8, PER = DK / 8;  // padded rows (banks); channels a thread stages
+    constexpr int RAW_Q = 0, RAW_K = kCkTokens * DK * 2, RAW_Z = 2 * RAW_K, RAW = RAW_Z + kCkTokens * DK * 4;
+    constexpr int NT = DK / 8, KT = DK / 16;
+    __shared__ __align__(16) float s_alpha[kCkTokens][DK], s_q[MODE ? kCkTokens : 1][DK], s_k[kCkTokens][DK];
+    __shared__ __align__(16) bf16 t_q[MODE ? 3 : 1][kCkTokens][ROW], t_k[3][kCkTokens][ROW], t_p[MODE ? 3 : 1][kCkTokens][PROW], s_v[2][kCkTokens][VROW];
+    __shared__ __align__(16) unsigned char raw[RAW];  // the next tokens' q, k and decay logits as they lie in memory
+    __shared__ __align__(8) float s_all[DK];
+    const int colblocks = (dv + kCkCols - 1) / kCkCols;
+    const int s = blockIdx.x, head = blockIdx.y / colblocks, col0 = (blockIdx.y % colblocks) * kCkCols, c = blockIdx.z;
+    const int seq_first = seq_info[s * 4 + 0], seq_count = seq_info[s * 4 + 1], start = seq_info[s * 4 + 2], slot = seq_info[s * 4 + 3];
+    int lo, hi, nseg;
+    if (!la_segment(start, seq_count, c, lo, hi, nseg) || (MODE == 0 && c == nseg - 1)) return;
+    const int first = seq_first + (lo - start), count = hi - lo;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int wcol = col0 + warp * 32;
+    const bool live = wcol < dv;  // dv is a multiple of 32
+    const bool slot_ok = slot >= 0 && slot < num_slots;
+    float *const mine = state + (size_t)(slot_ok ? slot : 0) * slot_stride + (size_t)head * DK * dv;
+    float *const seg = seg_state + (((size_t)s * max_segments + c) * heads + head) * DK * dv;
+
+    float S[2][NT][4];
+    {
+        const bool from_slot = c == 0 && lo > 0 && slot_ok, from_seg = MODE == 1 && c > 0;
+        const float *const src = from_slot ? mine : seg;
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    S[m][n][i] = live && (from_slot || from_seg) ? src[(size_t)(n * 8 + 2 * t + (i & 1)) * dv + wcol + m * 16 + g + (i & 2) * 4] : 0.f;
+    }
+
+    // a thread stages channels d0 .. of token j and 16 columns of v
+    const int j = threadIdx.x >> 3, d0 = (threadIdx.x & 7) * PER, v0 = (threadIdx.x & 7) * 16;
+    float bias[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) bias[i] = z_bias ? to_f(z_bias[(size_t)head * DK + d0 + i]) : 0.f;
+    struct __align__(2 * PER) Row {
+        bf16 x[PER];
+    };
+    const auto copy = [](void *to, const void *from, int bytes) {
+        const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(to));
+        if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(from) : "memory");
+        else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(from) : "memory");
+    };
+    auto fetch = [&](int t0, int b) {  // a thread copies what it reads itself later, and v
+        if (t0 + j < count) {
+            const size_t tok = (size_t)(first + t0 + j);
+            if (MODE) copy(raw + RAW_Q + (j * DK + d0) * 2, q + tok * q_token + (size_t)head * q_head + d0, 2 * PER);
+            copy(raw + RAW_K + (j * DK + d0) * 2, k + tok * k_token + (size_t)head * k_head + d0, 2 * PER);
+#pragma unroll
+            for (int i = 0; i < PER; i += 4) copy(raw + RAW_Z + (j * DK + d0 + i) * 4, z + tok * z_token + (size_t)head * DK + d0 + i, 16);
+#pragma unroll
+            for (int i = 0; i < 16; i += 8)
+                if (col0 + v0 + i < dv) copy(&s_v[b][j][v0 + i], v + tok * v_token + (size_t)head * v_head + col0 + v0 + i, 16);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int i = 0; i < 16; i += 8)  // columns that are not there
+            if (col0 + v0 + i >= dv) *reinterpret_cast<uint4 *>(&s_v[b][j][v0 + i]) = make_uint4(0u, 0u, 0u, 0u);
+    float total = 1.f;  // threads below DK: the segment's decay of their channel
+    fetch(0, 0);
+    for (int t0 = 0, b = 0; t0 < count; t0 += kCkTokens, b ^= 1) {
+        const int n_tok = min(kCkTokens, count - t0);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        {  // past the last token: decay 1, key, query and value 0
+            const bool in = j < n_tok;
+            const float *const rz = reinterpret_cast<const float *>(raw + RAW_Z) + j * DK + d0;
+            const Row rk = *reinterpret_cast<const Row *>(raw + RAW_K + (j * DK + d0) * 2);
+            float a[PER], x[PER];
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                const float zz = rz[i] + bias[i];
+                a[i] = !in ? 1.f : decay_kind == 2 ? expf(-expf(zz)) : expf(log_sigmoid(zz) * inv_tau);
+                x[i] = in ? to_f(rk.x[i]) : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < PER; i += 4) {
+                *reinterpret_cast<float4 *>(&s_alpha[j][d0 + i]) = make_float4(a[i], a[i + 1], a[i + 2], a[i + 3]);
+                *reinterpret_cast<float4 *>(&s_k[j][d0 + i]) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+            }
+            if (MODE) {
+                const Row rq = *reinterpret_cast<const Row *>(raw + RAW_Q + (j * DK + d0) * 2);
+#pragma unroll
+                for (int i = 0; i < PER; ++i) x[i] = in ? to_f(rq.x[i]) * q_scale : 0.f;
+#pragma unroll
+                for (int i = 0; i < PER; i += 4) *reinterpret_cast<float4 *>(&s_q[j][d0 + i]) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+            }
+            if (!in)
+#pragma unroll
+                for (int i = 0; i < 16; i += 8) *reinterpret_cast<uint4 *>(&s_v[b][j][v0 + i]) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        __syncthreads();
+        if (t0 + kCkTokens < count) fetch(t0 + kCkTokens, b ^ 1);
+        // ---- q A and k R as terms: a thread a pair of channels and eight of the tokens, forward or backward (MODE 0: backward alone)
+        if (lane < DK / 2 && (MODE || warp < 2)) {
+            const int d = 2 * lane, back = MODE ? warp >> 1 : 1, late = warp & 1;  // late: behind the eight tokens of the other
+            float2 a = make_float2(1.f, 1.f);
+            if (late)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float2 x = *reinterpret_cast<const float2 *>(&s_alpha[back ? 15 - i : i][d]);
+                    a.x *= x.x, a.y *= x.y;
+                }
+            const float(*const from)[DK] = back ? s_k : s_q;
+            bf16(*const to)[kCkTokens][ROW] = back ? t_k : t_q;
+#pragma unroll
+            for (int i0 = 0; i0 < 8; ++i0) {
+                const int i = back ? 15 - late * 8 - i0 : late * 8 + i0;
+                const float2 x = *reinterpret_cast<const float2 *>(&s_alpha[i][d]), y = *reinterpret_cast<const float2 *>(&from[i][d]);
+                if (!back) a.x *= x.x, a.y *= x.y;
+                uint32_t term[3];
+                ck_split(y.x * a.x, y.y * a.y, term);
+#pragma unroll
+                for (int u = 0; u < 3; ++u) *reinterpret_cast<uint32_t *>(&to[u][i][d]) = term[u];
+                if (back) a.x *= x.x, a.y *= x.y;
+            }
+            if (back && late) *reinterpret_cast<float2 *>(&s_all[d]) = a;
+        }
+        // ---- P: sixteen lanes a token s, a warp two early and two late ones, so that all warps have as many steps
+        if (MODE) {
+            constexpr int CH = DK / 16;
+            const int dc = (lane & 15) * CH;
+#pragma unroll 1
+            for (int part = 0; part < 2; ++part) {
+                const int s0 = part ? 14 - 2 * warp : 2 * warp, ps = s0 + (lane >> 4), from = s0 & ~3;
+                float r[CH];
+#pragma unroll
+                for (int i = 0; i < CH; ++i) r[i] = s_k[ps][dc + i];
+#pragma unroll 1
+                for (int t4 = from; t4 < kCkTokens; t4 += 4) {  // four tokens t, whose sums over the sixteen lanes end in four of these
+                    float y[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        y[i] = 0.f;
+#pragma unroll
+                        for (int n = 0; n < CH; n += 2) {
+                            const float2 x = *reinterpret_cast<const float2 *>(&s_alpha[t4 + i][dc + n]), w = *reinterpret_cast<const float2 *>(&s_q[t4 + i][dc + n]);
+                            if (t4 + i > ps) r[n] *= x.x, r[n + 1] *= x.y;
+                            y[i] = fmaf(w.x, r[n], y[i]), y[i] = fmaf(w.y, r[n + 1], y[i]);
+                        }
+                    }
+                    const bool b3 = lane & 8, b2 = lane & 4;
+                    const float u0 = (b3 ? y[2] : y[0]) + __shfl_xor_sync(0xffffffffu, b3 ? y[0] : y[2], 8);
+                    const float u1 = (b3 ? y[3] : y[1]) + __shfl_xor_sync(0xffffffffu, b3 ? y[1] : y[3], 8);
+                    float sum = (b2 ? u1 : u0) + __shfl_xor_sync(0xffffffffu, b2 ? u0 : u1, 4);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+                    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                    const int tt = t4 + (b3 ? 2 : 0) + (b2 ? 1 : 0);
+                    if ((lane & 3) == 0) {
+                        uint32_t term[3];
+                        ck_split(tt >= ps ? sum : 0.f, 0.f, term);
+#pragma unroll
+                        for (int u = 0; u < 3; ++u) *reinterpret_cast<unsigned short *>(&t_p[u][tt][ps]) = static_cast<unsigned short>(term[u]);
+                    }
+                }
+                for (int e = lane; e < 2 * 3 * from; e += 32) t_p[e / 2 / from][e / 2 % from][s0 + (e & 1)] = from_f<bf16>(0.f);  // tokens before s
+            }
+        }
+        __syncthreads();
+        uint32_t va[2][4];  // v^T: 16 columns x 16 tokens
+#pragma unroll
+        for (int m = 0; m < 2; ++m) ck_ldm_t(va[m], &s_v[b][(lane & 7) + (lane >> 4) * 8][warp * 32 + m * 16 + (lane >> 3 & 1) * 8]);
+        if (MODE) {
+            const int row = (lane & 7) + (lane >> 4) * 8, half = (lane >> 3 & 1) * 8;  // B operands: tokens 0-7 | 8-15 x the two halves of 16
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                float o[2][4] = {}, low[2][4] = {};  // low: the products of all terms but the first two
+                const auto add = [](float (&to)[4], const float (&x)[4]) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) to[i] += x[i];
+                };
+#pragma unroll
+                for (int kk = 0; kk < KT; ++kk) {
+                    uint32_t w[3][4], a[3][4], term[3];
+#pragma unroll
+                    for (int u = 0; u < 3; ++u) ck_ldm(w[u], &t_q[u][row][kk * 16 + half]);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        ck_split(S[m][2 * kk + (i >> 1)][(i & 1) * 2], S[m][2 * kk + (i >> 1)][(i & 1) * 2 + 1], term);
+#pragma unroll
+                        for (int u = 0; u < 3; ++u) a[u][i] = term[u];
+                    }
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) {
+#pragma unroll
+                        for (int sum = 2; sum >= 1; --sum)
+#pragma unroll
+                            for (int u = 0; u <= sum; ++u) ck_mma(low[n], a[u], w[sum - u][2 * n], w[sum - u][2 * n + 1]);
+                        float high[4] = {};
+                        ck_mma(high, a[0], w[0][2 * n], w[0][2 * n + 1]);
+                        add(o[n], high);
+                    }
+                }
+#pragma unroll
+                for (int u = 2; u >= 0; --u) {
+                    uint32_t w[4];
+                    ck_ldm(w, &t_p[u][row][half]);
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) {
+                        float high[4] = {};
+                        ck_mma(u ? low[n] : high, va[m], w[2 * n], w[2 * n + 1]);
+                        if (!u) add(o[n], high), add(o[n], low[n]);
+                    }
+                }
+                if (live) {
+                    float *const to = out + ((size_t)(first + t0) * heads + head) * dv + wcol + m * 16 + g;
+#pragma unroll
+                    for (int n = 0; n < 2; ++n)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            const int tt = n * 8 + 2 * t + (i & 1);
+                            if (tt < n_tok) to[(size_t)tt * heads * dv + (i & 2) * 4] = o[n][i];
+                        }
+                }
+            }
+        }
+        // ---- S^T <- S^T diag(A_16) + v^T (k R)
+#pragma unroll
+        for (int n = 0; n < NT; n += 2) {
+            float more[2][2][4] = {};
+#pragma unroll
+            for (int u = 2; u >= 0; --u) {
+                uint32_t w[4];
+                ck_ldm_t(w, &t_k[u][(lane & 7) + (lane >> 3 & 1) * 8][n * 8 + (lane >> 4) * 8]);
+#pragma unroll
+                for (int m = 0; m < 2; ++m) ck_mma(more[m][0], va[m], w[0], w[1]), ck_mma(more[m][1], va[m], w[2], w[3]);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float2 x = *reinterpret_cast<const float2 *>(&s_all[(n + h) * 8 + 2 * t]);
+#pragma unroll
+                for (int m = 0; m < 2; ++m)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) S[m][n + h][i] = fmaf(i & 1 ? x.y : x.x, S[m][n + h][i], more[m][h][i]);
+            }
+        }
+        if (MODE == 0 && threadIdx.x < DK) total *= s_all[threadIdx.x];
+    }
+    float *const dst = MODE == 0 ? seg : c == nseg - 1 && slot_ok ? mine : nullptr;
+    if (dst != nullptr && live) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) dst[(size_t)(n * 8 + 2 * t + (i & 1)) * dv + wcol + m * 16 + g + (i & 2) * 4] = S[m][n][i];
+    }
+    if (MODE == 0 && col0 == 0 && threadIdx.x < DK) seg_decay[(((size_t)s * max_segments + c) * heads + head) * DK + threadIdx.x] = total;
+}
+
+// The segments' start states where their end states were, in order: start[c + 1] = decay[c] start[c] + end[c] (segment 0 began from the sequence's
+// own state, so its end is whole).  A thread four neighbouring columns of a row; eight segments' numbers are on their way at once.
+__global__ void __launch_bounds__(256)
+decay_starts_kernel(const int32_t *__restrict__ seq_info, int heads, int dk, int dv, int max_segments, float *__restrict__ seg_state, const float *__restrict__ seg_decay) {
+    const int s = blockIdx.x, head = blockIdx.y, e = (blockIdx.z * blockDim.x + threadIdx.x) * 4;
+    int lo, hi, nseg;
+    la_segment(seq_info[s * 4 + 2], seq_info[s * 4 + 1], 0, lo, hi, nseg);
+    if (nseg <= 1 || e >= dk * dv) return;
+    constexpr int kAhead = 8;
+    float *seg = seg_state + ((size_t)s * max_segments * heads + head) * dk * dv + e;
+    const float *dec = seg_decay + ((size_t)s * max_segments * heads + head) * dk + e / dv;
+    const size_t seg_step = (size_t)heads * dk * dv, dec_step = (size_t)heads * dk;
+    float4 S = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int c0 = 0; c0 < nseg; c0 += kAhead, seg += kAhead * seg_step, dec += kAhead * dec_step) {
+        float4 end[kAhead];
+        float decay[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (c0 + u + 1 < nseg) end[u] = *reinterpret_cast<const float4 *>(seg + u * seg_step), decay[u] = dec[u * dec_step];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+            if (c0 + u < nseg) {
+                *reinterpret_cast<float4 *>(seg + u * seg_step) = S;
+                if (c0 + u + 1 < nseg) {
+                    const float d = decay[u];
+                    S = make_float4(fmaf(d, S.x, end[u].x), fmaf(d, S.y, end[u].y), fmaf(d, S.z, end[u].z), fmaf(d, S.w, end[u].w));
+                }
+            }
+    }
+}
+
 // out[t, h, :] = o[t, h, :] / rms(o[t, h, :]) * w * act(gate[t, h, :]); one warp per (token, head).  act 0 = none, 1 = silu,
 // 2 = sigmoid; w == NULL: no weight; wide_weight: w is [heads * dv] (every head its own part) instead of [dv] shared by the
 // heads; gate_first: the gate multiplies o BEFORE the norm, out = n / rms(n) * w with n = o * act(gate).  floor: a row of o has one
@@ -463,6 +804,68 @@ head_norm_gate_kernel(const float *__restrict__ o, const T *__restrict__ w, floa
         float y = src[d] * share * inv * (wr ? to_f(wr[d]) : 1.f);
         if (gate) y *= gated(d);
         out[(size_t)row * dv + d] = from_f<T>(y);
+    }
+}
+
+// The same for rows of whole fours (16 bytes of o, 8 of a bf16 gate an access) and at most PIECES times 128 columns: a row's numbers are requested
+// together and kept, where the kernel above makes three round trips of 4-byte accesses (2048 tokens of 16 heads of 128 columns: 18 -> 12.6 us, now bound by
+// the exponentials and divisions).
+template <typename T, int PIECES>
+__global__ void __launch_bounds__(256)
+head_norm_gate_wide_kernel(const float *__restrict__ o, const T *__restrict__ w, float eps, const T *__restrict__ gate, long long g_token, int act,
+                           T *__restrict__ out, long long rows, int heads, int dv, int wide_weight, int gate_first, int o_row,
+                           const float *__restrict__ floor, float den_eps) {
+    const unsigned row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // below 2^31 (a division of 64 bits is a hundred instructions)
+    if (row >= rows) return;
+    const int lane = threadIdx.x & 31;
+    const unsigned t = row / (unsigned)heads;
+    const int head = (int)(row - t * heads);
+    const float *src = o + (size_t)row * o_row;
+    const T *wr = w ? w + (wide_weight ? (size_t)head * dv : 0) : nullptr;
+    const T *gr = gate ? gate + (size_t)t * g_token + (size_t)head * dv : nullptr;
+    struct __align__(4 * sizeof(T)) Four {
+        T v[4];
+    };
+    float4 x[PIECES];
+    Four g[PIECES], k[PIECES];
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+        const int d = (i * 32 + lane) * 4;
+        x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (d >= dv) continue;
+        x[i] = *reinterpret_cast<const float4 *>(src + d);
+        if (gr) g[i] = *reinterpret_cast<const Four *>(gr + d);
+        if (wr) k[i] = *reinterpret_cast<const Four *>(wr + d);
+    }
+    const float share = floor ? 1.0f / (fmaxf(fabsf(src[dv]), floor[row]) + den_eps) : 1.f;
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+        float *const v = &x[i].x;
+        const bool in = (i * 32 + lane) * 4 < dv;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float a = 1.f;
+            if (gr && in) {
+                const float gv = to_f(g[i].v[j]);
+                a = act == 1 ? gv / (1.0f + expf(-gv)) : act == 2 ? 1.0f / (1.0f + expf(-gv)) : gv;
+            }
+            v[j] *= share;
+            const float y = gate_first ? v[j] * a : v[j];
+            if (in) ss += y * y;
+            v[j] *= a;  // what is left is the norm and its weight
+        }
+    }
+    const float inv = 1.0f / sqrtf(warp_sum(ss) / (float)dv + eps);
+#pragma unroll
+    for (int i = 0; i < PIECES; ++i) {
+        const int d = (i * 32 + lane) * 4;
+        if (d >= dv) continue;
+        const float *const v = &x[i].x;
+        Four y;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) y.v[j] = from_f<T>(v[j] * inv * (wr ? to_f(k[i].v[j]) : 1.f));
+        *reinterpret_cast<Four *>(out + (size_t)row * dv + d) = y;
     }
 }
 
@@ -540,6 +943,25 @@ int tlb_decay_scan(const void *q, long long q_token, long long q_head, const voi
         TL_LAUNCH_CHECK("decay_scan");
         return TL_OK;
     }
+    // the tensor cores' form: a decay per key channel from logits, bf16, whole 16-byte rows; the rest (rotation, bonus, skip, a normaliser, grouped
+    // heads, other sizes) walks
+    const auto rows16 = [](const void *p, long long token, long long head) { return (uintptr_t)p % 16 == 0 && token % 8 == 0 && head % 8 == 0; };
+    if (dtype == TL_BF16 && !scalar && !bonus && !skip && rope_dims == 0 && qk_heads == heads && v_cols == dv && (dk == 32 || dk == 64) && dv % 32 == 0 &&
+        rows16(q, q_token, q_head) && rows16(k, k_token, k_head) && rows16(v, v_token, v_head) && tl::aligned16(z) && z_token % 4 == 0 && tl::aligned16(workspace)) {
+        const dim3 grid(num_seqs, heads * ceil_div(dv, kCkCols), max_segments);
+#define TLB_CHUNK(DKV, MODE)                                                                                                                                    \
+    decay_chunk_kernel<DKV, MODE><<<grid, 128, 0, st>>>((const bf16 *)q, q_token, q_head, (const bf16 *)k, k_token, k_head, (const bf16 *)v, v_token, v_head, z, \
+                                                        z_token, (const bf16 *)z_bias, 1.0f / tau, q_scale, heads, dv, seq_info, state, slot_stride, num_slots,  \
+                                                        out, max_segments, seg_state, seg_decay, decay_kind)
+        if (dk == 64) TLB_CHUNK(64, 0); else TLB_CHUNK(32, 0);
+        TL_LAUNCH_CHECK("decay_scan (end states)");
+        decay_starts_kernel<<<dim3(num_seqs, heads, ceil_div(dk * dv, 1024)), 256, 0, st>>>(seq_info, heads, dk, dv, max_segments, seg_state, seg_decay);
+        TL_LAUNCH_CHECK("decay_scan (start states)");
+        if (dk == 64) TLB_CHUNK(64, 1); else TLB_CHUNK(32, 1);
+        TL_LAUNCH_CHECK("decay_scan (outputs)");
+#undef TLB_CHUNK
+        return TL_OK;
+    }
     TLB_DS(1, max_segments);
     TL_LAUNCH_CHECK("decay_scan (segments)");
     const bool vec = dk % 4 == 0 && dv % 4 == 0 && tl::aligned16(workspace) && tl::aligned16(out);
@@ -567,6 +989,18 @@ int tlb_head_norm_gate(const float *o, const void *w, float eps, const void *gat
     if (o_row <= 0) o_row = dv;
     if (o_row < dv + (floor ? 1 : 0) || (floor && gate_first)) return tl::fail(TL_EINVAL, "head_norm_gate: bad row or normaliser");
     long long rows = (long long)tokens * heads;
+    const size_t four = dtype == TL_BF16 ? 8 : 16;
+    const auto fits = [&](const void *p) { return p == nullptr || (uintptr_t)p % four == 0; };
+    if (rows < (1ll << 31) && dv % 4 == 0 && dv <= 512 && o_row % 4 == 0 && g_token % 4 == 0 && tl::aligned16(o) && fits(w) && fits(gate) && fits(out)) {
+        const unsigned ctas = (unsigned)((rows + 7) / 8);
+#define TLB_WIDE(P)                                                                                                                                          \
+    head_norm_gate_wide_kernel<T, P><<<ctas, 256, 0, as_stream(stream)>>>(o, (const T *)w, eps, (const T *)gate, g_token, act, (T *)out, rows, heads, dv, \
+                                                                          wide_weight, gate_first, o_row, floor, den_eps)
+        TLB_DISPATCH(dtype, "head_norm_gate", if (dv <= 128) TLB_WIDE(1); else if (dv <= 256) TLB_WIDE(2); else TLB_WIDE(4));
+#undef TLB_WIDE
+        TL_LAUNCH_CHECK("head_norm_gate");
+        return TL_OK;
+    }
     TLB_DISPATCH(dtype, "head_norm_gate",
                  head_norm_gate_kernel<T><<<(unsigned)((rows + 3) / 4), 128, 0, as_stream(stream)>>>(o, (const T *)w, eps, (const T *)gate, g_token, act,
                                                                                                     (T *)out, rows, heads, dv, wide_weight, gate_first, o_row, floor, den_eps));
