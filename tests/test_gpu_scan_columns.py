@@ -72,6 +72,25 @@ def test_long_portions_on_the_tensor_cores_against_float64(H, dk, dv, counts, st
     assert torch.equal(state[0], before[0]) and (len(counts) < 2 or torch.equal(state[2], before[2]))
 
 
+def test_a_value_that_is_no_number_stays_behind_its_token():
+    from extensions_b200.tiny_llm_ext_b200 import blocks
+
+    T, H, dk, dv, bad = 130, 2, 64, 128, 72
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, k, v = (torch.randn(T, H, d, generator=g, device="cuda").bfloat16() for d in (dk, dk, dv))
+    z = torch.randn(T, H * dk, generator=g, device="cuda")
+    info = torch.tensor([(0, T, 0, 0)], dtype=torch.int32, device="cuda")
+    state = torch.zeros(1, H, dk, dv, device="cuda")
+    run = lambda: blocks.decay_scan(q, k, v, z, None, q_scale=1.0, seq_info=info, state=state, max_tokens=T)  # noqa: E731
+    want = run()
+    v[bad, 0, 5], v[bad, 1, 40] = float("inf"), float("nan")
+    got = run()
+    clean = torch.ones_like(got, dtype=torch.bool)
+    clean[bad:, 0, 5] = clean[bad:, 1, 40] = False
+    assert not got[~clean].isfinite().any() and bool(got[clean].isfinite().all())
+    assert torch.allclose(got[clean], want[clean], rtol=2.0**-18, atol=2.0**-18 * float(want.abs().max()))
+
+
 @pytest.mark.parametrize("act", [0, 1, 2])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("T,H,dv", [(1, 1, 4), (5, 3, 128), (3, 2, 132), (4, 2, 256), (2, 2, 512), (2, 2, 516), (3, 2, 66)])

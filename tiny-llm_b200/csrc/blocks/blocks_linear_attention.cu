@@ -683,16 +683,34 @@ decay_chunk_kernel(const bf16 *__restrict__ q, long long q_token, long long q_he
                         add(o[n], high);
                     }
                 }
+                float high[2][4] = {}, test = 0.f;
+                uint32_t w[4];
+                ck_ldm(w, &t_p[0][row][half]);
 #pragma unroll
-                for (int u = 2; u >= 0; --u) {
-                    uint32_t w[4];
-                    ck_ldm(w, &t_p[u][row][half]);
+                for (int n = 0; n < 2; ++n) {
+                    ck_mma(high[n], va[m], w[2 * n], w[2 * n + 1]);
+                    test += (high[n][0] + high[n][1]) + (high[n][2] + high[n][3]);
+                }
+                if (__any_sync(0xffffffffu, test - test != 0.f)) {  // a value is no number: zero times it must not reach the tokens before it
+#pragma unroll 1
+                    for (int n = 0; n < 8; ++n) {
+                        const int tt = (n >> 2) * 8 + 2 * t + (n & 1);
+                        float sum = 0.f;
+                        for (int ps = 0; ps <= tt; ++ps)
+                            sum = fmaf(to_f(t_p[0][tt][ps]) + (to_f(t_p[1][tt][ps]) + to_f(t_p[2][tt][ps])), to_f(s_v[b][ps][warp * 32 + m * 16 + g + (n & 2) * 4]), sum);
 #pragma unroll
-                    for (int n = 0; n < 2; ++n) {
-                        float high[4] = {};
-                        ck_mma(u ? low[n] : high, va[m], w[2 * n], w[2 * n + 1]);
-                        if (!u) add(o[n], high), add(o[n], low[n]);
+                        for (int i = 0; i < 8; ++i)
+                            if (i == n) o[i >> 2][i & 3] += low[i >> 2][i & 3] + sum;
                     }
+                } else {
+#pragma unroll
+                    for (int u = 2; u >= 1; --u) {
+                        ck_ldm(w, &t_p[u][row][half]);
+#pragma unroll
+                        for (int n = 0; n < 2; ++n) ck_mma(low[n], va[m], w[2 * n], w[2 * n + 1]);
+                    }
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) add(o[n], high[n]), add(o[n], low[n]);
                 }
                 if (live) {
                     float *const to = out + ((size_t)(first + t0) * heads + head) * dv + wcol + m * 16 + g;
