@@ -4,8 +4,7 @@
 // src/tiny_llm_ref/qwen3_week3.py:62-105 with the kernel arithmetic of
 // src/extensions_ref/src/paged_attention.metal:108-248, every rounding point kept.
 //
-// (A whole-step persistent kernel lost to the CUDA-graph + programmatic-dependent-launch path by 1.8x: 0.63 ms of grid
-// barriers and 0.47 ms of staging per token.)
+// (Up to four requests take decode_step.cu, the whole step in one launch; this is the chain's launch for the others.)
 #include <algorithm>
 #include <stdlib.h>
 #include <math_constants.h>
