@@ -74,3 +74,36 @@ def test_one_launch_equals_the_operator_sequence(cuda_device, dims, page, contex
             if touched.any():
                 assert (a[touched].double() - w[touched].double()).norm() < 2**-8 * (12 * (layer + 1)) ** 0.5 * w[touched].double().norm()
     assert ext.waits_given_up() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layers", [1, 2])
+def test_the_first_launch_on_a_fresh_workspace(cuda_device, layers):
+    """Zeroed memory must not pass for packets: a new object's first step is the step that it repeats later, and no packet carries memory's tag."""
+    dims, dev, contexts = dict(SMALL, num_hidden_layers=layers), cuda_device, [150, 200]
+    model = Qwen3ModelWeek3(synthetic_qwen3(dims, seed=3, device=dev, realistic=True), page_size=64)
+    engine = DecodeEngine(model, 2, 256, dev)
+    engine.reserve_pools(8)
+    g = torch.Generator(device=dev).manual_seed(5)
+    slabs = [t for p in model.page_pools for t in (p._key_pages, p._value_pages)]
+    for pages in slabs:
+        pages.copy_(torch.randn(pages.shape, generator=g, device=dev))
+    before = [t.clone() for t in slabs]
+    engine.tables[:, :, :4] = torch.randperm(8, generator=g, device=dev).view(2, 4).to(torch.int32)
+    engine.tokens.copy_(torch.tensor([7, 300], device=dev))
+    engine.context_lens.copy_(torch.tensor(contexts, device=dev))
+    engine.offsets.copy_(engine.context_lens - 1)
+
+    def run(step):
+        for pages, old in zip(slabs, before):
+            pages.copy_(old)
+        step.launch()
+        return engine.logits.clone(), engine.next_tokens.clone(), [t.clone() for t in slabs]
+
+    steps = [engine._one_launch_step() for _ in range(6)]
+    first = [run(step) for step in steps]
+    packets = steps[-1]._keep[-1][256:].view(torch.int32).view(-1, 2)
+    assert not bool(((packets[:, 0] != 0) & (packets[:, 1] == 0)).any()), "a packet with the tag of memory that was never written"
+    logits, tokens, pages = run(steps[0])
+    for got in first:
+        assert torch.equal(got[0], logits) and torch.equal(got[1], tokens) and all(torch.equal(a, b) for a, b in zip(got[2], pages))

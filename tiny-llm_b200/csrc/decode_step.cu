@@ -28,7 +28,8 @@
 //
 // Packets are reused every second block.  A CTA writes block l + 2's packets of a product only after it has received
 // block l + 1's sums, to which every CTA contributed behind its own reads of block l: all CTAs own rows of gate|up (the launch refuses sizes where one would not).
-// Tags never repeat between two writes of a place: step number x (blocks + 1) + block + 1.
+// Tags never repeat between two writes of a place: step number x (blocks + 1) + block + 2, the embedding's one less.  None is 0, which the
+// zeroed memory of a fresh workspace carries.
 //
 // A wait is bounded: one that runs out marks its CTA, which then waits for nothing more, its logits are NaN and the kernel's count of
 // given-up waits goes up.
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
 
     const int qkv_w = (a.Hq + 2 * a.Hkv) * DS_HEAD, q_w = a.Hq * DS_HEAD;
     const unsigned int epoch = *static_cast<volatile unsigned int *>(a.seq);
-    const uint32_t tag0 = epoch * static_cast<uint32_t>(a.layers + 1) + 1u;
+    const uint32_t tag0 = epoch * static_cast<uint32_t>(a.layers + 1) + 2u;
 
     // ---- this CTA's part of every attention: a request, a K/V head and a range of its keys
     const int item = cta / a.nsplit, split = cta - item * a.nsplit;
