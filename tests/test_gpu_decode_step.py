@@ -11,6 +11,8 @@ from tiny_llm_b200.synthetic import synthetic_qwen3
 # the smallest sizes it takes (gate|up rows in every CTA), and one with a 19th of a piece's units odd, two heads a group and an untied head
 SMALL = dict(hidden_size=512, num_hidden_layers=3, num_attention_heads=8, num_key_value_heads=2, head_dim=128, intermediate_size=1536, vocab_size=528)
 WIDE = dict(hidden_size=1536, num_hidden_layers=2, num_attention_heads=4, num_key_value_heads=2, head_dim=128, intermediate_size=2560, vocab_size=1040)
+# two heads a group and o wider than the model: o's staged activations lie over the keys and values of an attention that is not split
+OVER = dict(hidden_size=1024, num_hidden_layers=3, num_attention_heads=16, num_key_value_heads=8, head_dim=128, intermediate_size=3072, vocab_size=1040)
 
 
 def test_sizes_it_does_not_take():
@@ -107,3 +109,12 @@ def test_the_first_launch_on_a_fresh_workspace(cuda_device, layers):
     logits, tokens, pages = run(steps[0])
     for got in first:
         assert torch.equal(got[0], logits) and torch.equal(got[1], tokens) and all(torch.equal(a, b) for a, b in zip(got[2], pages))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("page,contexts", [(16, [60]), (16, [60, 0]), (64, [64, 3]), (16, [40, 1, 64, 0]), (8, [7, 64, 200, 33])])
+def test_short_contexts_where_o_is_wider_than_the_model(cuda_device, page, contexts):
+    """Requests of one split beside idle and longer ones: their values are read before o's activations are staged over them.  (What the order prevents shows
+    by timing alone.)"""
+    for _ in range(4):
+        test_one_launch_equals_the_operator_sequence(cuda_device, OVER, page, contexts)

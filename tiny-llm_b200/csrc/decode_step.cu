@@ -763,6 +763,9 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
             }
             unsigned char *const y = x + a.o_y + (static_cast<size_t>(ab) * (q_w / 2) + kvh * Gq * 64) * 8;  // the group's heads
             if (splits == 1) {
+                // o's activations go where the values lie: a warp that is done (or has no head) must not stage heads of other CTAs over rows that
+                // another warp still reads.  (With more splits the merge's barrier stands between.)
+                __syncthreads();
                 if (oh < Gq) {
                     const float v = l_run == 0.f ? 0.f : o_run * (1.0f / l_run);
                     const float next = __shfl_down_sync(0xffffffffu, v, 1);
