@@ -72,6 +72,12 @@ def test_long_portions_on_the_tensor_cores_against_float64(H, dk, dv, counts, st
     assert torch.equal(state[0], before[0]) and (len(counts) < 2 or torch.equal(state[2], before[2]))
 
 
+@pytest.mark.parametrize("counts,start", [([65] * 40, 64), ([128, 65, 2, 300], 191), ([1000], 100)])
+def test_portions_that_go_on_from_a_slot_and_write_it(counts, start):
+    """The first segment starts from the state that the last one (of a single token, too) replaces in the end."""
+    test_long_portions_on_the_tensor_cores_against_float64(2, 64, 96, counts, start, 0)
+
+
 def test_a_value_that_is_no_number_stays_behind_its_token():
     from extensions_b200.tiny_llm_ext_b200 import blocks
 

@@ -442,7 +442,8 @@ decay_output_kernel(const int32_t *__restrict__ seq_info, int heads, int dk, int
 // S^T [columns, channels] stays in accumulator fragments, which are the A operand's layout too: a warp owns 32 columns.
 //
 // Three launches: every segment's end state from zero (its first one's from the sequence's own state) and its decay (MODE 0); the segments' start states, in
-// order; the outputs from the start states, and the last segment's end state to the slot (MODE 1).
+// order, the first one's too; the outputs from the start states, and the last segment's end state to the slot (MODE 1).  The CTAs of a launch have no order, so
+// the launch that writes the slot of a sequence in several segments does not read it.
 // 2048 tokens in two sequences of 16 heads of 64 x 128: the walk in segments 99 + 19 + 24 us, this 18 + 8 + 48 (8 + 8 heads 1.6 x, 65 tokens 1.1 x, 8000
 // tokens 2 x as fast); the error against 64 bits is 0.85 to 1.0 of the walk's (with long sums left to the tensor cores it was twice that, at 42 us).
 // What bounds it: instructions, of which the terms of S are a quarter, and three barriers every sixteen tokens with 14 warps an SM.
@@ -506,7 +507,8 @@ decay_chunk_kernel(const bf16 *__restrict__ q, long long q_token, long long q_he
 
     float S[2][NT][4];
     {
-        const bool from_slot = c == 0 && lo > 0 && slot_ok, from_seg = MODE == 1 && c > 0;
+        // the slot of a sequence that is cut is read in the launches before this one only: here the CTA of its last segment writes it
+        const bool from_seg = MODE == 1 && nseg > 1, from_slot = !from_seg && c == 0 && lo > 0 && slot_ok;
         const float *const src = from_slot ? mine : seg;
 #pragma unroll
         for (int m = 0; m < 2; ++m)
@@ -758,15 +760,22 @@ decay_chunk_kernel(const bf16 *__restrict__ q, long long q_token, long long q_he
     if (MODE == 0 && col0 == 0 && threadIdx.x < DK) seg_decay[(((size_t)s * max_segments + c) * heads + head) * DK + threadIdx.x] = total;
 }
 
-// The segments' start states where their end states were, in order: start[c + 1] = decay[c] start[c] + end[c] (segment 0 began from the sequence's
-// own state, so its end is whole).  A thread four neighbouring columns of a row; eight segments' numbers are on their way at once.
+// The segments' start states where their end states were, in order: start[0] the sequence's own state (its slot's, or zero), start[1] = end[0] (that
+// segment began from it), start[c + 1] = decay[c] start[c] + end[c].  A thread four neighbouring columns of a row; eight segments' numbers are on their way at once.
 __global__ void __launch_bounds__(256)
-decay_starts_kernel(const int32_t *__restrict__ seq_info, int heads, int dk, int dv, int max_segments, float *__restrict__ seg_state, const float *__restrict__ seg_decay) {
+decay_starts_kernel(const int32_t *__restrict__ seq_info, int heads, int dk, int dv, int max_segments, float *__restrict__ seg_state, const float *__restrict__ seg_decay,
+                    const float *__restrict__ state, long long slot_stride, int num_slots) {
     const int s = blockIdx.x, head = blockIdx.y, e = (blockIdx.z * blockDim.x + threadIdx.x) * 4;
     int lo, hi, nseg;
-    la_segment(seq_info[s * 4 + 2], seq_info[s * 4 + 1], 0, lo, hi, nseg);
+    const int start = seq_info[s * 4 + 2], slot = seq_info[s * 4 + 3];
+    la_segment(start, seq_info[s * 4 + 1], 0, lo, hi, nseg);
     if (nseg <= 1 || e >= dk * dv) return;
     constexpr int kAhead = 8;
+    float4 own = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (start > 0 && slot >= 0 && slot < num_slots) {
+        const float *const mine = state + (size_t)slot * slot_stride + (size_t)head * dk * dv + e;
+        own = make_float4(mine[0], mine[1], mine[2], mine[3]);
+    }
     float *seg = seg_state + ((size_t)s * max_segments * heads + head) * dk * dv + e;
     const float *dec = seg_decay + ((size_t)s * max_segments * heads + head) * dk + e / dv;
     const size_t seg_step = (size_t)heads * dk * dv, dec_step = (size_t)heads * dk;
@@ -780,7 +789,7 @@ decay_starts_kernel(const int32_t *__restrict__ seq_info, int heads, int dk, int
 #pragma unroll
         for (int u = 0; u < kAhead; ++u)
             if (c0 + u < nseg) {
-                *reinterpret_cast<float4 *>(seg + u * seg_step) = S;
+                *reinterpret_cast<float4 *>(seg + u * seg_step) = c0 + u == 0 ? own : S;
                 if (c0 + u + 1 < nseg) {
                     const float d = decay[u];
                     S = make_float4(fmaf(d, S.x, end[u].x), fmaf(d, S.y, end[u].y), fmaf(d, S.z, end[u].z), fmaf(d, S.w, end[u].w));
@@ -973,7 +982,8 @@ int tlb_decay_scan(const void *q, long long q_token, long long q_head, const voi
                                                         out, max_segments, seg_state, seg_decay, decay_kind)
         if (dk == 64) TLB_CHUNK(64, 0); else TLB_CHUNK(32, 0);
         TL_LAUNCH_CHECK("decay_scan (end states)");
-        decay_starts_kernel<<<dim3(num_seqs, heads, ceil_div(dk * dv, 1024)), 256, 0, st>>>(seq_info, heads, dk, dv, max_segments, seg_state, seg_decay);
+        decay_starts_kernel<<<dim3(num_seqs, heads, ceil_div(dk * dv, 1024)), 256, 0, st>>>(seq_info, heads, dk, dv, max_segments, seg_state, seg_decay,
+                                                                                                 state, slot_stride, num_slots);
         TL_LAUNCH_CHECK("decay_scan (start states)");
         if (dk == 64) TLB_CHUNK(64, 1); else TLB_CHUNK(32, 1);
         TL_LAUNCH_CHECK("decay_scan (outputs)");
