@@ -258,7 +258,8 @@ int tl_decode_attention_fused(const void *qkv, const void *q_norm_weight, const 
  * (src/tiny_llm_ref/qwen3_week3.py:55-121,139-146,196-207 at L == 1), final norm, head, greedy argmax.  The plan is a HOST struct,
  * read during the call; every pointer in it is a device pointer.  Matrices other than the embedding table are tl_decode_step_pack()'s
  * results: q|k|v (rows concatenated), o and down packed with halves = 1, gate (top) and up (bottom) together, the head with neither.  workspace: tl_decode_step_workspace() bytes, zeroed once, used by one step at a time and kept between steps;
- * 0 bytes: these sizes are not taken. */
+ * 0 bytes: these sizes are not taken.  The CTAs of a step wait on one another, each wait for so many polls at most (the workspace's second 32-bit word, in 64s; 0:
+ * about half a second).  A step in which a wait gave up ends with NaN logits and next_tokens of -1 and raises tl_tc_gave_up(). */
 typedef struct tl_decode_step_layer {
     const void *qkv, *o, *gate_up, *down;
     const void *input_norm, *post_norm, *q_norm, *k_norm;

@@ -104,7 +104,7 @@ def test_the_first_launch_on_a_fresh_workspace(cuda_device, layers):
 
     steps = [engine._one_launch_step() for _ in range(6)]
     first = [run(step) for step in steps]
-    packets = steps[-1]._keep[-1][256:].view(torch.int32).view(-1, 2)
+    packets = steps[-1].workspace[256:].view(torch.int32).view(-1, 2)
     assert not bool(((packets[:, 0] != 0) & (packets[:, 1] == 0)).any()), "a packet with the tag of memory that was never written"
     logits, tokens, pages = run(steps[0])
     for got in first:

@@ -80,3 +80,52 @@ def test_batcher_hands_over_no_answer_after_a_wait_gave_up(cpu_ext, monkeypatch)
     with pytest.raises(RuntimeError, match="gave up waiting"):
         late.run()
     assert late.results == []
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("contexts", [[131072], [40, 131072, 0]])
+def test_a_decoding_step_whose_waits_run_out_shows_it(cuda_device, contexts):
+    """A limit of 64 polls, some 50 us, where others attend 7000 keys a CTA (about 360 us): no logit, token, key or value that looks right; the next step is
+    as before."""
+    from extensions_b200 import tiny_llm_ext_b200 as ext
+    from tiny_llm_b200 import Qwen3ModelWeek3
+    from tiny_llm_b200.engine import DecodeEngine
+    from tiny_llm_b200.synthetic import synthetic_qwen3
+
+    dims = dict(hidden_size=512, num_hidden_layers=3, num_attention_heads=8, num_key_value_heads=2, head_dim=128, intermediate_size=1536, vocab_size=528)
+    dev, B = cuda_device, len(contexts)
+    model = Qwen3ModelWeek3(synthetic_qwen3(dims, seed=1, device=dev, realistic=True), page_size=128)
+    pages = [-(-c // 128) for c in contexts]
+    engine = DecodeEngine(model, B, max(contexts), dev)
+    engine.reserve_pools(sum(pages))
+    slabs = [t for p in model.page_pools for t in (p._key_pages, p._value_pages)]
+    for slab in slabs:
+        slab.normal_()
+    before = [t.clone() for t in slabs]
+    engine.tables.fill_(-1)
+    for b, n in enumerate(pages):
+        engine.tables[:, b, :n] = torch.arange(sum(pages[:b]), sum(pages[: b + 1]), device=dev, dtype=torch.int32)
+    engine.tokens.fill_(9)
+    engine.context_lens.copy_(torch.tensor(contexts, device=dev))
+    engine.offsets.copy_((engine.context_lens - 1).clamp(min=0))
+    step = engine._one_launch_step()
+    limit = step.workspace[4:8].view(torch.int32)
+
+    def run(polls):
+        for slab, old in zip(slabs, before):
+            slab.copy_(old)
+        limit.fill_(polls)
+        step.launch()
+        return engine.logits.clone(), engine.next_tokens.tolist(), [t.clone() for t in slabs]
+
+    logits, tokens, right = run(0)
+    count = ext.waits_given_up()
+    assert bool(logits.isfinite().all()) and min(tokens) >= 0
+    late, none, _ = run(1)
+    assert bool(late.isnan().all()) and none == [-1] * B and ext.waits_given_up() > count
+    for k, old, good in zip(slabs, before, right):  # a row of the newest token is the right one or no number
+        changed = (k != old).any(-1)
+        assert bool((~k[changed].isfinite() | (k[changed] == good[changed])).all())
+    count = ext.waits_given_up()
+    again, same, kept = run(0)
+    assert torch.equal(again, logits) and same == tokens and all(torch.equal(a, b) for a, b in zip(kept, right)) and ext.waits_given_up() == count

@@ -31,8 +31,9 @@
 // Tags never repeat between two writes of a place: step number x (blocks + 1) + block + 2, the embedding's one less.  None is 0, which the
 // zeroed memory of a fresh workspace carries.
 //
-// A wait is bounded: one that runs out marks its CTA, which then waits for nothing more, its logits are NaN and the kernel's count of
-// given-up waits goes up.
+// A wait is bounded: one that runs out marks its CTA, whose further waits end soon.  Who gives up takes NaN for what did not come: packets, a unit's scales,
+// an attention's scores.  So every sum that needed it is NaN, the next norm makes everybody's rows NaN, and nothing checks the mark on the way (a read of it before the
+// stores took 3 % of the step).  The CTA's logits are NaN, the step's tokens -1, and the kernel's count of given-up waits goes up.
 #include <limits.h>
 #include <math_constants.h>
 
@@ -59,7 +60,8 @@ constexpr int DS_MAX_PIECES = 64;           // of a CTA and a product of a block
 constexpr int DS_MAX_SPLITS = 32;           // one lane per split in the merge
 constexpr float DS_LOG2E = 1.44269504089f;
 constexpr float DS_NEG = -1e30f;
-constexpr uint32_t DS_POLLS = 1u << 20;     // about half a second
+constexpr int DS_POLLS = 1 << 20;           // about half a second
+constexpr uint32_t DS_NAN2 = 0x7fff7fffu;   // two bf16
 
 struct DsMat {
     const uint32_t *w;
@@ -86,7 +88,7 @@ struct DsArgs {
     const bf16 *norm;
     bf16 *logits;
     int32_t *next_tokens;
-    unsigned int *seq;
+    unsigned int *seq;                  // step number, limit of a wait's polls (0: DS_POLLS)
     unsigned char *best;                // [grid][M] 16 bytes
     unsigned char *xchg[2];             // packets of even and odd blocks
     unsigned int o_y, o_xo, o_act, o_xd, o_part;  // byte offsets in xchg[.] (q|k|v first)
@@ -109,10 +111,10 @@ __device__ __forceinline__ void ds_st(void *p, uint32_t data, uint32_t tag) {
 }
 __device__ __forceinline__ uint32_t ds_tag(unsigned long long v) { return static_cast<uint32_t>(v >> 32); }
 
-// A failed poll: false when the wait is over for good (the CTA is marked).
+// A failed poll: false when the wait is over for good.  dead: whether the CTA is marked, and the limit.
 __device__ __forceinline__ bool ds_again(uint32_t &spins, volatile int *dead) {
     if ((++spins & 63u) != 0) return true;
-    if (spins > DS_POLLS) *dead = 1;
+    if (spins > static_cast<uint32_t>(dead[1])) *dead = 1;
     return *dead == 0;
 }
 __device__ __forceinline__ unsigned long long ds_poll(const void *p, uint32_t tag, volatile int *dead) {
@@ -120,13 +122,16 @@ __device__ __forceinline__ unsigned long long ds_poll(const void *p, uint32_t ta
     for (uint32_t spins = 0; ds_tag(v) != tag && ds_again(spins, dead);) v = ds_ld(p);
     return v;
 }
-// Whole warps: until the phase is over or the CTA is marked.
-__device__ __forceinline__ void ds_wait(uint32_t bar, uint32_t parity, volatile int *dead) {
+// Whole warps: until the phase is over (true) or the wait is.
+__device__ __forceinline__ bool ds_wait(uint32_t bar, uint32_t parity, volatile int *dead) {
     uint32_t done, spins = 0;
+    bool over;
     do {
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    } while (!__all_sync(0xffffffffu, done) && ds_again(spins, dead));
+        over = __all_sync(0xffffffffu, done);
+    } while (!over && ((spins & 63u) != 63u ? (++spins, true) : __all_sync(0xffffffffu, ds_again(spins, dead))));
     __syncwarp();
+    return over;
 }
 __device__ __forceinline__ float ds_exp2(float x) {
     float y;
@@ -313,7 +318,15 @@ __device__ __forceinline__ void ds_stage(const DsArgs &a, const unsigned char *s
                     put(m, idx - m * words, make_uint4(static_cast<uint32_t>(v[j][0].x), static_cast<uint32_t>(v[j][0].y), static_cast<uint32_t>(v[j][1].x), static_cast<uint32_t>(v[j][1].y)));
                     pending &= ~(1u << j);
                 }
-            if (pending != 0 && !ds_again(spins, dead)) break;
+            if (pending != 0 && !ds_again(spins, dead)) {
+#pragma unroll 1
+                for (int j = 0; j < FLIGHT; ++j)
+                    if (pending >> j & 1u) {
+                        const int idx = base + j * DS_THREADS, m = row_of(idx);
+                        put(m, idx - m * words, make_uint4(DS_NAN2, DS_NAN2, DS_NAN2, DS_NAN2));
+                    }
+                break;
+            }
         }
     }
     __syncwarp();
@@ -365,7 +378,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
     __shared__ int deals[5][4];                        // per kind of product: reduction, this CTA's first piece, its pieces, units of a piece
     __shared__ uchar2 span[4][DS_MAX_PIECES];          // the first and the last warp that have units of a piece
     __shared__ int4 shares[5][DS_WARPS];               // per kind and warp: first unit, one past the last, the first's piece and place in it
-    __shared__ int dead_s;
+    __shared__ int dead_s[2];
     __shared__ __align__(8) unsigned long long kv_bar[2], full[DS_WARPS][BATCHES];
     __shared__ __align__(16) bf16 q_s[8 * Q_ROW], k_cur[DS_HEAD], v_cur[DS_HEAD];  // query heads (rows past the group stay zero); the newest key and value
     __shared__ float2 cs_s[DS_HEAD / 2];
@@ -373,7 +386,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
     __shared__ float red_l[16];
     __shared__ float best_v[MP][DS_WARPS];
     __shared__ int best_i[MP][DS_WARPS];
-    volatile int *dead = &dead_s;
+    volatile int *dead = dead_s;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int cta = blockIdx.x, ctas = gridDim.x;
@@ -434,7 +447,8 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
         if (w == 0) deals[kind][0] = N, deals[kind][1] = c0, deals[kind][2] = pieces, deals[kind][3] = P;
     }
     if (threadIdx.x == 0) {
-        dead_s = 0;
+        const unsigned int limit = static_cast<volatile unsigned int *>(a.seq)[1];
+        dead_s[0] = 0, dead_s[1] = limit == 0 ? DS_POLLS : static_cast<int>(min(limit, 1u << 30));
         g_mbar_init(g_smem_u32(&kv_bar[0]), DS_THREADS);
         g_mbar_init(g_smem_u32(&kv_bar[1]), DS_THREADS);
 #pragma unroll 1
@@ -564,7 +578,11 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
             float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
             for (int i = share.x; i < share.y; i += BATCH) {
-                ds_wait(full0 + u_slot * 8, u_parity, dead);
+                if (!ds_wait(full0 + u_slot * 8, u_parity, dead)) {  // the copy may still be in flight: the warp requests nothing more
+                    l_left = 0, l_s = products;
+                    for (int k = 0; k < BATCH; ++k) *reinterpret_cast<uint32_t *>(smem + ((warp * BATCHES + u_slot) * BATCH + k) * DS_UNIT + 2048 + lane * 4) = DS_NAN2;
+                    __syncwarp();
+                }
                 const unsigned char *unit = smem + (warp * BATCHES + u_slot) * (BATCH * DS_UNIT);
                 const int n = min(BATCH, share.y - i);
 #pragma unroll 1
@@ -647,7 +665,13 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
                 const unsigned char *p = x + (static_cast<size_t>(ab) * (qkv_w / 2) + head * 64 + lane) * 8;
                 unsigned long long lo = ds_ld(p), hi = ds_ld(p + 256);
 #pragma unroll 1
-                for (uint32_t spins = 0; (ds_tag(lo) != tag || ds_tag(hi) != tag) && ds_again(spins, dead);) lo = ds_ld(p), hi = ds_ld(p + 256);
+                for (uint32_t spins = 0; ds_tag(lo) != tag || ds_tag(hi) != tag;) {
+                    if (!ds_again(spins, dead)) {
+                        lo = hi = DS_NAN2;
+                        break;
+                    }
+                    lo = ds_ld(p), hi = ds_ld(p + 256);
+                }
                 __syncwarp();
                 uint32_t o_lo = static_cast<uint32_t>(lo), o_hi = static_cast<uint32_t>(hi);
                 if (!is_v) {
@@ -666,7 +690,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
             }
             // values: thread = (head oh, 8 columns d8, token sub of a tile); afterwards it keeps column sub of the eight
             const int oh = threadIdx.x >> 7, sub = threadIdx.x & 7, d8 = (threadIdx.x >> 3) & 15;
-            const float scale2 = l.scale * DS_LOG2E;
+            float scale2 = l.scale * DS_LOG2E;
             float m_run = DS_NEG, l_run = 0.f, o_run = 0.f;
             if (!has_keys) __syncthreads();  // (each round begins with one) the sums of q|k|v have been read
 #pragma unroll 1
@@ -676,7 +700,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
                 const int *const pages = pg_s + b * (round + 4);
                 if (rb != k_begin) __syncthreads();  // the last round's page ids, rows and scores are dead
                 if (rb + round < k_end) request_keys(l, rb + round, b ^ 1);
-                ds_wait(g_smem_u32(&kv_bar[b]), kv_phase >> b & 1, dead);
+                if (!ds_wait(g_smem_u32(&kv_bar[b]), kv_phase >> b & 1, dead)) scale2 = m_run = CUDART_NAN_F;
                 kv_phase ^= 1 << b;
                 __syncthreads();  // q_s / k_cur / v_cur and all copies of the round
                 const int cur_slot = cur_tok - rb;
@@ -789,7 +813,13 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
                     unsigned long long o = ds_ld(po);
                     ulonglong2 ml = ds_ld2(pm);
 #pragma unroll 1
-                    for (uint32_t spins = 0; (ds_tag(o) != tag || ds_tag(ml.x) != tag || ds_tag(ml.y) != tag) && ds_again(spins, dead);) o = ds_ld(po), ml = ds_ld2(pm);
+                    for (uint32_t spins = 0; ds_tag(o) != tag || ds_tag(ml.x) != tag || ds_tag(ml.y) != tag;) {
+                        if (!ds_again(spins, dead)) {
+                            o = ml.x = ml.y = 0x7fffffffu;
+                            break;
+                        }
+                        o = ds_ld(po), ml = ds_ld2(pm);
+                    }
                     __syncwarp();
                     const float mj = lane < splits ? __uint_as_float(static_cast<uint32_t>(ml.x)) : DS_NEG;
                     const float top = warp_max(mj);
@@ -843,8 +873,6 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
         }
     }
     __syncthreads();
-    if (threadIdx.x == 0 && *dead) atomicAdd(&g_gave_up, 1u);
-    tc_settle(dead);
     const uint32_t tag = tag0 + a.layers;
     if (warp < M && lane == 0) {
         float bv = best_v[warp][0];
@@ -853,17 +881,19 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
             if (best_v[warp][w] > bv || (best_v[warp][w] == bv && best_i[warp][w] < bi)) bv = best_v[warp][w], bi = best_i[warp][w];
         unsigned char *const p = a.best + (static_cast<size_t>(cta) * M + warp) * 16;
         ds_st(p, __float_as_uint(bv), tag);
-        ds_st(p + 8, static_cast<uint32_t>(bi), tag);
+        ds_st(p + 8, *dead ? ~0u : static_cast<uint32_t>(bi), tag);
     }
     if (cta == 0) {  // the step's tokens
         if (warp < M) {
             float bv = -INFINITY;
             int bi = INT_MAX;
+            bool lost_one = false;
             for (int c = lane; c < ctas; c += 32) {
                 const unsigned char *p = a.best + (static_cast<size_t>(c) * M + warp) * 16;
                 const unsigned long long v = ds_poll(p, tag, dead), i = ds_poll(p + 8, tag, dead);
                 const float ov = __uint_as_float(static_cast<uint32_t>(v));
                 const int oi = static_cast<int>(static_cast<uint32_t>(i));
+                lost_one |= oi < 0 || ds_tag(v) != tag || ds_tag(i) != tag;
                 if (ov > bv || (ov == bv && oi < bi)) bv = ov, bi = oi;
             }
             __syncwarp();
@@ -873,11 +903,15 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
                 const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
                 if (ov > bv || (ov == bv && oi < bi)) bv = ov, bi = oi;
             }
-            if (lane == 0) a.next_tokens[warp] = bi == INT_MAX ? 0 : bi;
+            lost_one = __any_sync(0xffffffffu, lost_one);
+            if (lane == 0) a.next_tokens[warp] = lost_one ? -1 : bi == INT_MAX ? 0 : bi;
         }
         // every CTA has read the step number by now: its packets of this step were waited for
         if (threadIdx.x == 0) *static_cast<volatile unsigned int *>(a.seq) = epoch + 1u;
+        __syncthreads();
     }
+    if (threadIdx.x == 0 && *dead) atomicAdd(&g_gave_up, 1u);
+    tc_settle(dead);
 }
 
 // ---- weights as units: 16 rows of the MMA x 256 columns, in the order in which the lanes hold them, their scales and biases behind them.

@@ -926,7 +926,7 @@ class DecodeStep:
         nbytes = self.workspace_bytes(B, len(layers), num_heads, num_kv_heads, hidden, intermediate, V)
         if nbytes == 0 or D != 128 or Hkv != num_kv_heads:
             raise RuntimeError("decode_step: sizes the one-launch step does not take")
-        workspace = torch.zeros(nbytes, dtype=torch.uint8, device=logits.device)
+        self.workspace = workspace = torch.zeros(nbytes, dtype=torch.uint8, device=logits.device)
         q, qkv = num_heads * 128, (num_heads + 2 * num_kv_heads) * 128
         bf, i32, u8 = torch.bfloat16, torch.int32, torch.uint8
 
