@@ -118,3 +118,46 @@ def test_short_contexts_where_o_is_wider_than_the_model(cuda_device, page, conte
     by timing alone.)"""
     for _ in range(4):
         test_one_launch_equals_the_operator_sequence(cuda_device, OVER, page, contexts)
+
+
+@pytest.mark.gpu
+def test_a_request_that_grows_long_goes_on_with_the_chain(cuda_device, monkeypatch):
+    """Past so many keys a share the chain of launches is faster; the engine changes over between two steps, driven by the host or on the device."""
+    ckpt, dev, prompt = synthetic_qwen3(SMALL, seed=2, device=cuda_device, realistic=True), cuda_device, list(range(3, 60))
+    shares = torch.cuda.get_device_properties(dev).multi_processor_count // 2
+
+    def generate(on_device, limit):
+        model = Qwen3ModelWeek3(ckpt, page_size=16)
+        engine = DecodeEngine(model, 1, 256, dev)
+        engine.reserve_pools()
+        if limit is None:
+            assert not engine._one_launch
+        else:
+            assert engine._one_launch_keys == 700 * min(shares, 32)
+            engine._one_launch_keys = limit
+        cache = model.create_kv_cache()
+        token = int(model(torch.tensor([prompt], dtype=torch.int32, device=dev), 0, cache, logits_to_keep=1)[0, -1].argmax())
+        logits = []
+        if on_device:
+            tokens = engine.decode_on_device([token], [len(prompt)], cache, 24).reshape(-1).tolist()
+        else:
+            tokens = []
+            for i in range(24):
+                out, nxt = engine.step([token], [len(prompt) + i], cache)
+                logits.append(out.clone())
+                token = int(nxt[0])
+                tokens.append(token)
+        if limit is not None:
+            assert (engine._long is not None) == (len(prompt) + 24 > limit) and engine.captures == 1
+        for c in cache:
+            c.release()
+        return tokens, logits
+
+    whole, long, over = (generate(False, limit) for limit in (10**6, 10, 70))
+    monkeypatch.setenv("TL_DECODE_STEP", "0")
+    chain = generate(False, None)
+    monkeypatch.delenv("TL_DECODE_STEP")
+    assert all(torch.equal(a, b) for a, b in zip(long[1], chain[1])) and long[0] == chain[0]
+    at = 70 - len(prompt)  # steps of up to 70 tokens
+    assert all(torch.equal(a, b) for a, b in zip(over[1][:at], whole[1][:at]))
+    assert generate(True, 70)[0] == over[0]

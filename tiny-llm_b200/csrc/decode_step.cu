@@ -15,8 +15,9 @@
 //   * an attention's older keys and values are requested before the activations of its q|k|v are waited for;
 //   * the residual of a CTA's own rows never leaves its shared memory (o and down deal their rows to the same CTAs).
 //
-// Measured (eight Qwen3-4B blocks and the head, context 1011, a graph of the step alone): 483 us as 53 launches, 277 us here; 0.6B at 500: 315 -> 181; by
-// requests and context 1.2-1.75 x for one (30 to 8000 tokens), 1.0-1.4 x for two to four.  What it went through (the same case): weights in registers
+// Measured (eight Qwen3-4B blocks and the head, context 1011, a graph of the step alone): 483 us as 53 launches, 277 us here; 0.6B at 500: 315 -> 181.
+// A key of the longest share of an attention costs 49 ns a block, 4 to 15 in the chain, so long contexts belong to the chain (the engine's rule, with the figures): 4B, four
+// requests of 1000 tokens 485 us here and 660 there, of 8000 1170 and 871; one of 8000 440 and 612, of 32000 944 and 764.  What it went through (the same case): weights in registers
 // across the phases 398; units in the lanes' order by bulk copies 348; digits on the integer tensor cores (ds_digits) 319; two units a copy
 // and a barrier 303; sums by a thread an output instead of a half-warp, the norms' weights asked into L2 a block ahead 277.
 // A block takes 28 us where its bytes take 8: six exchanges of 1.2 to 2 us, 8 us of consuming, 5 us of staging, 4 us in the attention.

@@ -188,6 +188,14 @@ class DecodeEngine:
                             and ext.DecodeStep.workspace_bytes(self.B, self.n_layers, self.Hq, self.Hkv, hidden, intermediate, self.V) > 0)
         self._step = None
         self._intermediate = intermediate
+        # ... and as long as the longest request is short enough.  The one launch cuts every request's keys into as many shares and takes 49 ns a layer for
+        # a key of the longest share, where the chain takes 4 to 15; what it saves is launches.  It is ahead by this many keys a share at
+        # least (8 layers, equal lengths and one long request among short ones):  before the chain's fused attention 4B 700 to 970, 0.6B 740 to 1000; before its
+        # tensor-core attention 4B 710 to 1100, 0.6B 375 to 750.  (4B, 4 requests of 1000 / 8000 tokens: 485 / 1170 us against 660 / 871; 1 request of
+        # 8000 / 32000: 440 / 944 against 612 / 764.)
+        shares = min(max(torch.cuda.get_device_properties(self.device).multi_processor_count // (self.B * self.Hkv), 1), 32) if self._one_launch else 0
+        self._one_launch_keys = shares * (700 if self._attention_fused or hidden >= 2048 else 375)
+        self._long: tuple | None = None  # the chain's graphs beside it (step, self-advancing step), made when a request first grows longer
         # Row variants: the scheduler fills slots from index 0 (batch.py:220-226), so while few requests are live the
         # occupied slots are a prefix of the table.  A step graph over the first 16 / 32 rows is captured beside the
         # full one and step() replays the smallest that covers the highest occupied slot: every kernel of the wide
@@ -269,9 +277,6 @@ class DecodeEngine:
         ``rows``: only the first ``rows`` slots (a row variant, see __init__)."""
         m = self.model
         R = self.B if rows is None else rows
-        if self._step is not None:
-            self._step.launch()
-            return
         emb = m.embedding.weight
         x = ext.quantized_embedding(self.tokens[:R], emb.scales, emb.biases, emb.weight, emb.group_size, emb.bits)
         logits = self._forward_fused_layers(x, R)
@@ -359,37 +364,41 @@ class DecodeEngine:
                               head=packed["head"], norm=norm(m.norm), layers=layers, logits=self.logits,
                               next_tokens=self.next_tokens, num_heads=self.Hq, num_kv_heads=self.Hkv, intermediate=self._intermediate)
 
+    def _record(self, forward) -> tuple:
+        """(graph of a step, graph of a self-advancing step, kernels of libtiny_llm_b200.so recorded into the latter); on the engine's stream."""
+        # The warm-up passes really run: with the previous step's metadata still on the device they
+        # would append a stale token's K/V through a stale block table - possibly into a page that
+        # has been released and handed to another request since (slabs move when a second engine
+        # reserves more pages).  All slots idle: appends are skipped and attention returns zeros;
+        # step() / decode_on_device() upload the real block before they replay.
+        self.meta_dev[2 * self.B : 3 * self.B].zero_()
+        self.meta_dev[3 * self.B :].fill_(-1)
+        self._tables_dirty = True
+        for _ in range(2):  # warm-up: lazy kernel attribute setup must not happen under capture
+            forward()
+        self._stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with capture(graph, stream=self._stream):
+            forward()
+        loop = torch.cuda.CUDAGraph()
+        launched = ext.launch_count()
+        with capture(loop, stream=self._stream, pool=graph.pool()):
+            forward()
+            ext.decode_advance(self.tokens, self.next_tokens, self.offsets, self.context_lens, self.out_log, self.step_counter)
+        return graph, loop, ext.launch_count() - launched
+
     def _capture(self) -> None:
         self.captures += 1
         self._slab_ptrs = self._slabs()
+        self._long = None
         if self._one_launch:
             self._step = self._one_launch_step()
         elif self.fused:
             self._packed  # made on the caller's stream, not on the one that captures
-        forward = self._forward_fused if self.fused else self._forward_unfused
+        forward = self._step.launch if self._one_launch else self._forward_fused if self.fused else self._forward_unfused
         with torch.cuda.stream(self._stream):
             self._stream.wait_stream(torch.cuda.current_stream(self.device))
-            # The warm-up passes really run: with the previous step's metadata still on the device they
-            # would append a stale token's K/V through a stale block table - possibly into a page that
-            # has been released and handed to another request since (slabs move when a second engine
-            # reserves more pages).  All slots idle: appends are skipped and attention returns zeros;
-            # step() / decode_on_device() upload the real block before they replay.
-            self.meta_dev[2 * self.B : 3 * self.B].zero_()
-            self.meta_dev[3 * self.B :].fill_(-1)
-            self._tables_dirty = True
-            for _ in range(2):  # warm-up: lazy kernel attribute setup must not happen under capture
-                forward()
-            self._stream.synchronize()
-            self._graph = torch.cuda.CUDAGraph()
-            with capture(self._graph, stream=self._stream):
-                forward()
-            self._graph_loop = torch.cuda.CUDAGraph()
-            launched = ext.launch_count()
-            with capture(self._graph_loop, stream=self._stream, pool=self._graph.pool()):
-                forward()
-                ext.decode_advance(self.tokens, self.next_tokens, self.offsets, self.context_lens, self.out_log, self.step_counter)
-            # kernels of libtiny_llm_b200.so recorded into one self-advancing step
-            self.kernels_per_step = ext.launch_count() - launched
+            self._graph, self._graph_loop, self.kernels_per_step = self._record(forward)
             self._graphs = {self.B: self._graph}
             for rows in self._variants:
                 if rows == self.B:
@@ -403,9 +412,19 @@ class DecodeEngine:
                 self._graphs[rows] = g
         torch.cuda.current_stream(self.device).wait_stream(self._stream)
 
-    def _ensure_graph(self) -> None:
+    def _ensure_graph(self, longest: int = 0) -> None:
+        """The graphs for steps whose longest request has up to ``longest`` tokens."""
         if self._graph is None or self._slab_ptrs != self._slabs():
             self._capture()
+        if self._chain_for(longest) and self._long is None:
+            self._packed
+            with torch.cuda.stream(self._stream):
+                self._stream.wait_stream(torch.cuda.current_stream(self.device))
+                self._long = self._record(self._forward_fused)
+            torch.cuda.current_stream(self.device).wait_stream(self._stream)
+
+    def _chain_for(self, longest: int) -> bool:
+        return self._one_launch and longest > self._one_launch_keys
 
     # ------------------------------------------------------- host bookkeeping --
     def _slot_caches(self, caches, layer: int):
@@ -566,7 +585,8 @@ class DecodeEngine:
         B = self.B
         self._host_write_begin()
         ctx = self._advance_host(caches, 1)
-        self._ensure_graph()
+        longest = max(ctx)
+        self._ensure_graph(longest)
         if isinstance(tokens, torch.Tensor):
             tok_host = None
         else:
@@ -587,7 +607,7 @@ class DecodeEngine:
                     hi = b + 1
             rows = next(r for r in self._variants if r >= hi)
             self.variant_replays[rows] += 1
-        self._graphs[rows].replay()
+        (self._long[0] if self._chain_for(longest) else self._graphs[rows]).replay()
         self.graph_replays += 1
         return self.logits.view(B, 1, self.V), self.next_tokens
 
@@ -600,7 +620,8 @@ class DecodeEngine:
         B = self.B
         self._host_write_begin()
         ctx = self._advance_host(caches, steps)
-        self._ensure_graph()
+        longest = max(ctx)
+        self._ensure_graph(longest + steps - 1)
         self.meta_np[0:B] = tokens
         self.meta_np[B : 2 * B] = offsets
         self.meta_np[2 * B : 3 * B] = ctx
@@ -610,7 +631,7 @@ class DecodeEngine:
             self._upload()
             self.step_counter.zero_()
             for i in range(steps):
-                self._graph_loop.replay()
+                (self._long[1] if self._chain_for(longest + i) else self._graph_loop).replay()
         cur.wait_stream(self._stream)
         self.graph_replays += steps
         return self.out_log[: steps * B].view(steps, B)
