@@ -161,3 +161,35 @@ def test_a_request_that_grows_long_goes_on_with_the_chain(cuda_device, monkeypat
     at = 70 - len(prompt)  # steps of up to 70 tokens
     assert all(torch.equal(a, b) for a, b in zip(over[1][:at], whole[1][:at]))
     assert generate(True, 70)[0] == over[0]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["huge pages", "unaligned norms", "two rotations"])
+def test_what_the_chain_takes_is_still_taken(cuda_device, monkeypatch, form):
+    """Forms that the one launch does not take as they are: a product of the page sizes past 32 bits, norm weights inside another buffer, blocks that differ."""
+    ckpt, dev = synthetic_qwen3(SMALL, seed=4, device=cuda_device, realistic=True), cuda_device
+
+    def logits():
+        model = Qwen3ModelWeek3(ckpt, page_size=65536 if form == "huge pages" else 16)
+        if form == "unaligned norms":
+            for b in model.layers_inner:
+                for n in (b.self_attn.q_norm, b.self_attn.k_norm):
+                    n.weight = torch.cat([n.weight[:1], n.weight.to(torch.bfloat16)])[1:]
+        if form == "two rotations":
+            model.layers_inner[1].self_attn.rope.base = 5000
+        engine = DecodeEngine(model, 1, 100, dev)
+        engine.reserve_pools(8 if engine.page_size == 16 else 1)
+        cache = model.create_kv_cache()
+        model.use_decode_graph = False
+        model(torch.tensor([[5, 6, 7, 8, 9]], dtype=torch.int32, device=dev), 0, cache, logits_to_keep=1)
+        return engine._one_launch, [engine.step([11], [5 + i], cache)[0].clone() for i in range(3)]
+
+    if form == "two rotations":
+        monkeypatch.setenv("TL_ATTENTION_FUSED", "0")  # rotates block by block
+    one, got = logits()
+    assert one == (form == "unaligned norms")
+    monkeypatch.setenv("TL_DECODE_STEP", "0")
+    chain, want = logits()
+    assert not chain
+    for a, b in zip(got, want):
+        assert (a.double() - b.double()).norm() < 2**-8 * (12 * 3) ** 0.5 * b.double().norm()

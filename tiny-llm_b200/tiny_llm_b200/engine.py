@@ -178,13 +178,17 @@ class DecodeEngine:
         # Up to four requests: the whole step is one launch (csrc/decode_step.cu) wherever the sizes fit it.  TL_DECODE_STEP=0: the chain of launches.
         emb = model.embedding.weight
         head = model.w_lm_head if model.w_lm_head is not None else emb
-        packed = [emb, head] + [w for b in model.layers_inner for w in (b.self_attn.wq, b.self_attn.wk, b.self_attn.wv, b.self_attn.wo, b.mlp.w_gate, b.mlp.w_up, b.mlp.w_down)]
+        by_layer = [(b.self_attn.wq, b.self_attn.wk, b.self_attn.wv, b.self_attn.wo, b.mlp.w_gate, b.mlp.w_up, b.mlp.w_down) for b in model.layers_inner]
+        packed = [emb, head] + [w for ws in by_layer for w in ws]
         hidden = emb.weight.shape[1] * 8
         intermediate = model.layers_inner[0].mlp.w_gate.weight.shape[0]
         self._one_launch = (self.fused and self.D == 128 and os.environ.get("TL_DECODE_STEP", "1") != "0"
                             and all(w.group_size == 128 and w.bits == 4 and w.scales.dtype == torch.bfloat16
                                     and all(t.is_contiguous() for t in (w.weight, w.scales, w.biases)) for w in packed)
                             and head.weight.shape == emb.weight.shape
+                            # all blocks alike: one plan of shares and one table of angles for the step
+                            and len({tuple(w.weight.shape for w in ws) for ws in by_layer}) == 1 and len({b.self_attn.rope.base for b in model.layers_inner}) == 1
+                            and self.max_pages * self.page_size**2 < 2**32  # its division by the page size
                             and ext.DecodeStep.workspace_bytes(self.B, self.n_layers, self.Hq, self.Hkv, hidden, intermediate, self.V) > 0)
         self._step = None
         self._intermediate = intermediate
@@ -351,12 +355,16 @@ class DecodeEngine:
         def norm(n):
             return n._weight_as(torch.bfloat16, dev), n.eps
 
+        def head_norm(n):  # read in pairs; the chain reads single entries, so a view into a larger buffer may begin anywhere
+            w, eps = norm(n)
+            return (w if w.data_ptr() % 4 == 0 else w.clone()), eps
+
         layers = []
         packed = _step_weights(m)
         for i, (block, pk, pool) in enumerate(zip(m.layers_inner, packed["layers"], m.page_pools)):
             at = block.self_attn
             layers.append(dict(pk, input_norm=norm(block.input_layernorm),
-                               post_norm=norm(block.post_attention_layernorm), q_norm=norm(at.q_norm), k_norm=norm(at.k_norm), key_pages=pool._key_pages,
+                               post_norm=norm(block.post_attention_layernorm), q_norm=head_norm(at.q_norm), k_norm=head_norm(at.k_norm), key_pages=pool._key_pages,
                                value_pages=pool._value_pages, block_table=self.tables[i], scale=at.scale))
         emb = m.embedding.weight
         return ext.DecodeStep(tokens=self.tokens, offsets=self.offsets, context_lens=self.context_lens,
