@@ -193,3 +193,36 @@ def test_what_the_chain_takes_is_still_taken(cuda_device, monkeypatch, form):
     assert not chain
     for a, b in zip(got, want):
         assert (a.double() - b.double()).norm() < 2**-8 * (12 * 3) ** 0.5 * b.double().norm()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("on_device", [False, True])
+@pytest.mark.parametrize("what", ["o", "down", "head", "nothing"])
+def test_weights_written_in_place_are_seen(cuda_device, what, on_device):
+    """o, down and the head as in the chain, which reads them where they lie: by the engine's next step, and by an engine that is made afterwards."""
+    dev = cuda_device
+
+    def second_step(afterwards, write):
+        model = Qwen3ModelWeek3(synthetic_qwen3(SMALL, seed=6, device=dev, realistic=True), page_size=16)
+        engine = DecodeEngine(model, 1, 100, dev)
+        engine.reserve_pools()
+        cache = model.create_kv_cache()
+        model.use_decode_graph = False
+        model(torch.tensor([[5, 6, 7]], dtype=torch.int32, device=dev), 0, cache, logits_to_keep=1)
+        _, token = engine.step([8], [3], cache)
+        block = model.layers_inner[1]
+        w = {"o": block.self_attn.wo, "down": block.mlp.w_down, "head": model.w_lm_head if model.w_lm_head is not None else model.embedding.weight}.get(what)
+        if w is not None and write:
+            w.scales.mul_(0.5)
+        if afterwards:
+            token = token.clone()
+            engine = DecodeEngine(model, 1, 100, dev)
+        if on_device:
+            engine.decode_on_device([9], [4], cache, 1)
+            return engine.logits.clone(), engine.captures
+        return engine.step(token, [4], cache)[0].clone(), engine.captures  # (the static buffer of the step before)
+
+    got, captures = second_step(False, True)
+    want, _ = second_step(True, True)
+    old, _ = second_step(False, False)
+    assert torch.equal(got, want) and torch.equal(got, old) == (what == "nothing") and captures == (1 if what == "nothing" else 2)

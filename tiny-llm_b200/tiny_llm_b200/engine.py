@@ -27,6 +27,7 @@ from __future__ import annotations
 
 import os
 from functools import cached_property
+from operator import attrgetter
 from types import SimpleNamespace
 
 import numpy as np
@@ -37,6 +38,9 @@ from extensions_b200 import tiny_llm_ext_b200 as ext
 from .graphs import capture
 from .kv_cache import BatchingKvCache
 from .paged_kv_cache import TinyKvPagedCache
+
+
+_VERSION = attrgetter("_version")  # of a tensor: the number of writes in place
 
 
 def _concat_weights(parts):
@@ -67,14 +71,20 @@ def _interleave_gate_up(gate, up):
 
 
 def _step_weights(model) -> dict:
-    """The packed matrices in the order in which the one-launch step reads them, made once for all of a model's engines (one allocation)."""
+    """The packed matrices in the order in which the one-launch step reads them: a second copy of them all, shared by a model's engines (one allocation).
+    An engine that records its graphs after weights were changed in place finds other bytes and makes a new copy."""
+    head = model.w_lm_head if model.w_lm_head is not None else model.embedding.weight
+    wanted = [("head", dict(parts=[head]))]
+    for b in model.layers_inner:
+        at, mlp = b.self_attn, b.mlp
+        wanted += [("qkv", dict(parts=[at.wq, at.wk, at.wv], halves=True)), ("o", dict(parts=[at.wo], halves=True)),
+                   ("gate_up", dict(parts=[mlp.w_gate], bottom=mlp.w_up)), ("down", dict(parts=[mlp.w_down], halves=True))]
+    kept = model._step_weights
+    if kept is not None:
+        old = [kept["head"]] + [one[name] for one in kept["layers"] for name in ("qkv", "o", "gate_up", "down")]
+        if not all(torch.equal(ext.decode_step_pack(**w), was) for (_, w), was in zip(wanted, old)):
+            model._step_weights = None  # engines that have it keep it
     if model._step_weights is None:
-        head = model.w_lm_head if model.w_lm_head is not None else model.embedding.weight
-        wanted = [("head", dict(parts=[head]))]
-        for b in model.layers_inner:
-            at, mlp = b.self_attn, b.mlp
-            wanted += [("qkv", dict(parts=[at.wq, at.wk, at.wv], halves=True)), ("o", dict(parts=[at.wo], halves=True)),
-                       ("gate_up", dict(parts=[mlp.w_gate], bottom=mlp.w_up)), ("down", dict(parts=[mlp.w_down], halves=True))]
         sizes = [ext.decode_step_bytes(w["parts"], w.get("bottom")) for _, w in wanted]
         whole = torch.empty(sum(sizes), dtype=torch.uint8, device=head.scales.device).split(sizes)
         made = [(name, ext.decode_step_pack(**w, out=out)) for (name, w), out in zip(wanted, whole)]
@@ -192,6 +202,10 @@ class DecodeEngine:
                             and ext.DecodeStep.workspace_bytes(self.B, self.n_layers, self.Hq, self.Hkv, hidden, intermediate, self.V) > 0)
         self._step = None
         self._intermediate = intermediate
+        # The chain reads o, down and the head where they lie; the one launch reads copies, which are made anew when these are written to (see step()).
+        live = [head] + [w for ws in by_layer for w in (ws[3], ws[6])] if self._one_launch else []
+        self._live = [t for w in live for t in (w.weight, w.scales, w.biases) if not t.is_inference()]  # (those have no version)
+        self._live_version = 0
         # ... and as long as the longest request is short enough.  The one launch cuts every request's keys into as many shares and takes 49 ns a layer for
         # a key of the longest share, where the chain takes 4 to 15; what it saves is launches.  It is ahead by this many keys a share at
         # least (8 layers, equal lengths and one long request among short ones):  before the chain's fused attention 4B 700 to 970, 0.6B 740 to 1000; before its
@@ -395,11 +409,20 @@ class DecodeEngine:
             ext.decode_advance(self.tokens, self.next_tokens, self.offsets, self.context_lens, self.out_log, self.step_counter)
         return graph, loop, ext.launch_count() - launched
 
+    def _weights_written(self) -> bool:
+        """Whether the copied weights were changed in place since the graphs were recorded; then they are to be recorded again."""
+        if self._graph is not None and sum(map(_VERSION, self._live)) != self._live_version:
+            self._graph = None
+            self.__dict__.pop("_packed", None)
+            return True
+        return False
+
     def _capture(self) -> None:
         self.captures += 1
         self._slab_ptrs = self._slabs()
         self._long = None
         if self._one_launch:
+            self._live_version = sum(map(_VERSION, self._live))
             self._step = self._one_launch_step()
         elif self.fused:
             self._packed  # made on the caller's stream, not on the one that captures
@@ -616,6 +639,12 @@ class DecodeEngine:
             rows = next(r for r in self._variants if r >= hi)
             self.variant_replays[rows] += 1
         (self._long[0] if self._chain_for(longest) else self._graphs[rows]).replay()
+        if self._live and self._weights_written():  # asked while the step runs; the same token again, into the same slots
+            same = self.tokens.clone()
+            self._ensure_graph(longest)
+            self._upload()
+            self.tokens.copy_(same)
+            (self._long[0] if self._chain_for(longest) else self._graphs[rows]).replay()
         self.graph_replays += 1
         return self.logits.view(B, 1, self.V), self.next_tokens
 
@@ -629,6 +658,7 @@ class DecodeEngine:
         self._host_write_begin()
         ctx = self._advance_host(caches, steps)
         longest = max(ctx)
+        self._weights_written()
         self._ensure_graph(longest + steps - 1)
         self.meta_np[0:B] = tokens
         self.meta_np[B : 2 * B] = offsets
