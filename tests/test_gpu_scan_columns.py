@@ -97,6 +97,45 @@ def test_a_value_that_is_no_number_stays_behind_its_token():
     assert torch.allclose(got[clean], want[clean], rtol=2.0**-18, atol=2.0**-18 * float(want.abs().max()))
 
 
+@pytest.mark.parametrize("dk", [32, 64])
+@pytest.mark.parametrize("what", ["key", "value", "query", "decay", "state", "nothing"])
+def test_infinities_stay_what_they_are_token_by_token(dk, what):
+    """Against the walk, which 32-bit operands take: infinities and NaN in the same places, the rest the same up to the order of the sums."""
+    from extensions_b200.tiny_llm_ext_b200 import blocks
+
+    T, H, dv, start = 150, 2, 96, 30  # segments of 34, 64 and 52 tokens
+    g = torch.Generator(device="cuda").manual_seed(5 + dk)
+    q, k, v = (torch.randn(T, H, d, generator=g, device="cuda").bfloat16() for d in (dk, dk, dv))
+    z = torch.randn(T, H * dk, generator=g, device="cuda") + 3
+    state = torch.randn(2, H, dk, dv, generator=g, device="cuda")
+    for t, sign in ((0, 1), (20, -1), (33, 1), (60, 1), (T - 1, -1)):
+        if what == "key":
+            k[t, t % 2, t % dk] = sign * float("inf")
+        if what == "value":
+            v[t, t % 2, t % dv] = sign * float("inf")
+        if what == "query":
+            q[t, t % 2, t % dk] = sign * float("inf")
+        if what == "decay":
+            z[t, t % dk] = float("nan") if sign > 0 else float("inf")
+    if what == "state":
+        state[1, 0, 3, 5], state[1, 1, dk - 1, dv - 1], state[1, 1, 0, 40] = float("inf"), -float("inf"), float("nan")
+    info = torch.tensor([(0, T, start, 1)], dtype=torch.int32, device="cuda")
+
+    def run(*qkv):
+        s = state.clone()
+        return blocks.decay_scan(*qkv, z, None, q_scale=1.0, seq_info=info, state=s, max_tokens=T), s[1]
+
+    for got, want in zip(run(q, k, v), run(q.float(), k.float(), v.float())):
+        if what == "query":  # the walk adds two parts of a segment's outputs, which may be two infinities
+            assert torch.equal(got.isfinite(), want.isfinite())
+        else:
+            assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf()) and torch.equal(got[got.isinf()], want[want.isinf()])
+        fine = want.isfinite()
+        assert bool(fine.any()) and bool(fine.all()) == (what == "nothing" or (what == "query" and want.dim() == 3 and want.shape[0] == H))
+        # sums of up to 2 T dk terms of the size of the largest results, in another order
+        assert float((got[fine].double() - want[fine].double()).abs().max()) <= 2.0**-24 * 32 * float(want[fine].abs().max())
+
+
 @pytest.mark.parametrize("act", [0, 1, 2])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("T,H,dv", [(1, 1, 4), (5, 3, 128), (3, 2, 132), (4, 2, 256), (2, 2, 512), (2, 2, 516), (3, 2, 66)])

@@ -492,6 +492,7 @@ decay_chunk_kernel(const bf16 *__restrict__ q, long long q_token, long long q_he
     __shared__ __align__(16) bf16 t_q[MODE ? 3 : 1][kCkTokens][ROW], t_k[3][kCkTokens][ROW], t_p[MODE ? 3 : 1][kCkTokens][PROW], s_v[2][kCkTokens][VROW];
     __shared__ __align__(16) unsigned char raw[RAW];  // the next tokens' q, k and decay logits as they lie in memory
     __shared__ __align__(8) float s_all[DK];
+    __shared__ int s_odd;  // MODE 0: a key or value up to here was no number
     const int colblocks = (dv + kCkCols - 1) / kCkCols;
     const int s = blockIdx.x, head = blockIdx.y / colblocks, col0 = (blockIdx.y % colblocks) * kCkCols, c = blockIdx.z;
     const int seq_first = seq_info[s * 4 + 0], seq_count = seq_info[s * 4 + 1], start = seq_info[s * 4 + 2], slot = seq_info[s * 4 + 3];
@@ -550,6 +551,7 @@ decay_chunk_kernel(const bf16 *__restrict__ q, long long q_token, long long q_he
 #pragma unroll
         for (int i = 0; i < 16; i += 8)  // columns that are not there
             if (col0 + v0 + i >= dv) *reinterpret_cast<uint4 *>(&s_v[b][j][v0 + i]) = make_uint4(0u, 0u, 0u, 0u);
+    if (!MODE && threadIdx.x == 0) s_odd = 0;
     float total = 1.f;  // threads below DK: the segment's decay of their channel
     fetch(0, 0);
     for (int t0 = 0, b = 0; t0 < count; t0 += kCkTokens, b ^= 1) {
@@ -610,6 +612,22 @@ decay_chunk_kernel(const bf16 *__restrict__ q, long long q_token, long long q_he
             }
             if (back && late) *reinterpret_cast<float2 *>(&s_all[d]) = a;
         }
+        if (!MODE && warp >= 2) {  // the idle warps: is every key and value a number?
+            float test = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int e = ((warp - 2) * 32 + lane) * 4 + i;  // 16 bytes
+                const uint4 x = *reinterpret_cast<const uint4 *>(&s_v[b][e >> 4][(e & 15) * 8]);
+                const float2 x0 = tl::unpack2<bf16>(x.x), x1 = tl::unpack2<bf16>(x.y), x2 = tl::unpack2<bf16>(x.z), x3 = tl::unpack2<bf16>(x.w);
+                test = fmaf((x0.x + x0.y) + (x1.x + x1.y) + ((x2.x + x2.y) + (x3.x + x3.y)), 0.f, test);
+            }
+#pragma unroll
+            for (int e = (warp - 2) * 32 + lane; e < kCkTokens * DK / 2; e += 64) {
+                const float2 x = *reinterpret_cast<const float2 *>(&s_k[0][0] + 2 * e);
+                test = fmaf(x.x + x.y, 0.f, test);
+            }
+            if (test != 0.f) s_odd = 1;
+        }
         // ---- P: sixteen lanes a token s, a warp two early and two late ones, so that all warps have as many steps
         if (MODE) {
             constexpr int CH = DK / 16;
@@ -651,6 +669,12 @@ decay_chunk_kernel(const bf16 *__restrict__ q, long long q_token, long long q_he
             }
         }
         __syncthreads();
+        const auto step = [&](float (&x)[4], int tt, int n, float v0, float v8) {  // one token's step of channels n * 8 + 2t, + 1 and two columns
+            const float2 decay = *reinterpret_cast<const float2 *>(&s_alpha[tt][n * 8 + 2 * t]), key = *reinterpret_cast<const float2 *>(&s_k[tt][n * 8 + 2 * t]);
+            x[0] = fmaf(decay.x, x[0], key.x * v0), x[1] = fmaf(decay.y, x[1], key.y * v0);
+            x[2] = fmaf(decay.x, x[2], key.x * v8), x[3] = fmaf(decay.y, x[3], key.y * v8);
+        };
+        bool walked[2] = {false, false};
         uint32_t va[2][4];  // v^T: 16 columns x 16 tokens
 #pragma unroll
         for (int m = 0; m < 2; ++m) ck_ldm_t(va[m], &s_v[b][(lane & 7) + (lane >> 4) * 8][warp * 32 + m * 16 + (lane >> 3 & 1) * 8]);
@@ -686,36 +710,36 @@ decay_chunk_kernel(const bf16 *__restrict__ q, long long q_token, long long q_he
                     }
                 }
                 float high[2][4] = {}, test = 0.f;
-                uint32_t w[4];
-                ck_ldm(w, &t_p[0][row][half]);
+#pragma unroll
+                for (int u = 0; u < 3; ++u) {
+                    uint32_t w[4];
+                    ck_ldm(w, &t_p[u == 0 ? 0 : 3 - u][row][half]);
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) ck_mma(u == 0 ? high[n] : low[n], va[m], w[2 * n], w[2 * n + 1]);
+                }
 #pragma unroll
                 for (int n = 0; n < 2; ++n) {
-                    ck_mma(high[n], va[m], w[2 * n], w[2 * n + 1]);
-                    test += (high[n][0] + high[n][1]) + (high[n][2] + high[n][3]);
+                    add(o[n], high[n]), add(o[n], low[n]);
+                    test += (o[n][0] + o[n][1]) + (o[n][2] + o[n][3]);
                 }
-                if (__any_sync(0xffffffffu, test - test != 0.f)) {  // a value is no number: zero times it must not reach the tokens before it
+                float *const to = out + ((size_t)(first + t0) * heads + head) * dv + wcol + m * 16 + g;
+                walked[m] = __any_sync(0xffffffffu, test - test != 0.f);
+                if (walked[m]) {  // something is no number (an infinity's terms are infinity, NaN, NaN, and zero times it is NaN): token by token
 #pragma unroll 1
-                    for (int n = 0; n < 8; ++n) {
-                        const int tt = (n >> 2) * 8 + 2 * t + (n & 1);
-                        float sum = 0.f;
-                        for (int ps = 0; ps <= tt; ++ps)
-                            sum = fmaf(to_f(t_p[0][tt][ps]) + (to_f(t_p[1][tt][ps]) + to_f(t_p[2][tt][ps])), to_f(s_v[b][ps][warp * 32 + m * 16 + g + (n & 2) * 4]), sum);
+                    for (int tt = 0; tt < n_tok; ++tt) {
+                        const float v0 = to_f(s_v[b][tt][warp * 32 + m * 16 + g]), v8 = to_f(s_v[b][tt][warp * 32 + m * 16 + g + 8]);
+                        float y0 = 0.f, y8 = 0.f;
 #pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            if (i == n) o[i >> 2][i & 3] += low[i >> 2][i & 3] + sum;
+                        for (int n = 0; n < NT; ++n) {
+                            step(S[m][n], tt, n, v0, v8);
+                            const float2 x = *reinterpret_cast<const float2 *>(&s_q[tt][n * 8 + 2 * t]);
+                            y0 = fmaf(x.x, S[m][n][0], fmaf(x.y, S[m][n][1], y0)), y8 = fmaf(x.x, S[m][n][2], fmaf(x.y, S[m][n][3], y8));
+                        }
+#pragma unroll
+                        for (int i = 1; i < 4; i <<= 1) y0 += __shfl_xor_sync(0xffffffffu, y0, i), y8 += __shfl_xor_sync(0xffffffffu, y8, i);
+                        if (live && t == 0) to[(size_t)tt * heads * dv] = y0, to[(size_t)tt * heads * dv + 8] = y8;
                     }
-                } else {
-#pragma unroll
-                    for (int u = 2; u >= 1; --u) {
-                        ck_ldm(w, &t_p[u][row][half]);
-#pragma unroll
-                        for (int n = 0; n < 2; ++n) ck_mma(low[n], va[m], w[2 * n], w[2 * n + 1]);
-                    }
-#pragma unroll
-                    for (int n = 0; n < 2; ++n) add(o[n], high[n]), add(o[n], low[n]);
-                }
-                if (live) {
-                    float *const to = out + ((size_t)(first + t0) * heads + head) * dv + wcol + m * 16 + g;
+                } else if (live) {
 #pragma unroll
                     for (int n = 0; n < 2; ++n)
 #pragma unroll
@@ -727,23 +751,35 @@ decay_chunk_kernel(const bf16 *__restrict__ q, long long q_token, long long q_he
             }
         }
         // ---- S^T <- S^T diag(A_16) + v^T (k R)
+        if (MODE ? walked[0] || walked[1] : s_odd != 0) {
 #pragma unroll
-        for (int n = 0; n < NT; n += 2) {
-            float more[2][2][4] = {};
+            for (int m = 0; m < 2; ++m)
+                if (!walked[m])
+#pragma unroll 1
+                    for (int tt = 0; tt < n_tok; ++tt) {
+                        const float v0 = to_f(s_v[b][tt][warp * 32 + m * 16 + g]), v8 = to_f(s_v[b][tt][warp * 32 + m * 16 + g + 8]);
 #pragma unroll
-            for (int u = 2; u >= 0; --u) {
-                uint32_t w[4];
-                ck_ldm_t(w, &t_k[u][(lane & 7) + (lane >> 3 & 1) * 8][n * 8 + (lane >> 4) * 8]);
+                        for (int n = 0; n < NT; ++n) step(S[m][n], tt, n, v0, v8);
+                    }
+        } else {
 #pragma unroll
-                for (int m = 0; m < 2; ++m) ck_mma(more[m][0], va[m], w[0], w[1]), ck_mma(more[m][1], va[m], w[2], w[3]);
-            }
+            for (int n = 0; n < NT; n += 2) {
+                float more[2][2][4] = {};
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const float2 x = *reinterpret_cast<const float2 *>(&s_all[(n + h) * 8 + 2 * t]);
+                for (int u = 2; u >= 0; --u) {
+                    uint32_t w[4];
+                    ck_ldm_t(w, &t_k[u][(lane & 7) + (lane >> 3 & 1) * 8][n * 8 + (lane >> 4) * 8]);
 #pragma unroll
-                for (int m = 0; m < 2; ++m)
+                    for (int m = 0; m < 2; ++m) ck_mma(more[m][0], va[m], w[0], w[1]), ck_mma(more[m][1], va[m], w[2], w[3]);
+                }
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) S[m][n + h][i] = fmaf(i & 1 ? x.y : x.x, S[m][n + h][i], more[m][h][i]);
+                for (int h = 0; h < 2; ++h) {
+                    const float2 x = *reinterpret_cast<const float2 *>(&s_all[(n + h) * 8 + 2 * t]);
+#pragma unroll
+                    for (int m = 0; m < 2; ++m)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) S[m][n + h][i] = fmaf(i & 1 ? x.y : x.x, S[m][n + h][i], more[m][h][i]);
+                }
             }
         }
         if (MODE == 0 && threadIdx.x < DK) total *= s_all[threadIdx.x];
