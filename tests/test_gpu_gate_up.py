@@ -1,6 +1,11 @@
 """The gated MLP's first half in one call - the up projection applies the activation in its epilogue - against two products and swiglu:
 the same bits from every kernel that a number of rows takes, whole and ragged feature tiles, unaligned rows, both types."""
 
+import os
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -82,3 +87,23 @@ def test_the_whole_mlp_in_one_call_equals_its_products(M, dtype):
         quantized_mlp(x.float(), gate, up, down)
     with pytest.raises(RuntimeError, match="one column per input group"):
         quantized_mlp(x[..., :640].contiguous(), gate, up, down)
+
+
+def test_the_wide_geometry_is_not_mixed_with_the_other():
+    """TL_SKINNY_WIDE1=1 (A/B runs) at 65 to 128 rows: its splits go with its own launches, a product and a sum of planes each."""
+    program = """
+import sys, torch
+sys.path[:0] = ["tests", "tiny-llm_b200"]
+from test_gpu_gate_up import weight
+from extensions_b200 import tiny_llm_ext_b200 as ext
+gate, up = weight(2560, 2560, torch.bfloat16, 1), weight(2560, 2560, torch.bfloat16, 2)
+x = torch.randn(100, 2560, device="cuda").bfloat16()
+before = ext.launch_count()
+got = ext.quantized_gate_up(x, gate, up)
+launches = ext.launch_count() - before
+one, two = (ext.quantized_matmul(w[0], w[1], 128, 4, x, w[2], True) for w in (gate, up))
+assert torch.equal(got, ext.swiglu(one, two))
+print(launches)
+"""
+    run = lambda **env: int(subprocess.run([sys.executable, "-c", program], cwd=Path(__file__).parent.parent, env={**os.environ, **env}, check=True, capture_output=True, text=True).stdout)  # noqa: E731
+    assert run(TL_SKINNY_WIDE1="0") == 2 and run(TL_SKINNY_WIDE1="1") == 4

@@ -689,6 +689,7 @@ static bool skinny_gate_up(SkArgs args, const void *a, const void *gate_b, const
     args.splits = w4a16_skinny_splits(M, N, K);
     if (args.splits == 1 || ws == nullptr || ws_bytes < 2 * w4a16_skinny_workspace(M, N, K) || !aligned16(a) || !aligned16(gate_b) || !aligned16(up_b)) return false;
     const int NT = M <= 16 ? 16 : (M <= 32 ? 32 : (M <= 64 ? 64 : 128));
+    if (NT == 128 && skinny_wide1()) return false;  // the splits are those of the other geometry: two launches
     args.tiles = (K + SK_FEAT - 1) / SK_FEAT;
     args.gb_per_split = (N / SK_GB + args.splits - 1) / args.splits;
     args.partials = static_cast<float *>(ws);
