@@ -35,3 +35,9 @@ def test_the_paged_attention_kernels_use_it():
     source = (CSRC / "attention_prefill_tc.cu").read_text()
     assert source.count("cudaFuncSetAttribute") == 2 and source.count("static PerDevice") == 1  # in the one helper that all launches go through
     assert "static bool configured" not in source and "static const bool configured" not in source
+
+
+def test_the_kernels_of_packed_products_of_few_rows_use_it():
+    for name in ("w4a16_matvec.cu", "w4a16_skinny.cu", "decode_step.cu"):
+        source = (CSRC / name).read_text()
+        assert "cudaFuncSetAttribute" in source and "static PerDevice" in source and "static bool configured" not in source

@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "per_device.h"
 #include "w4a16_item.cuh"
 #include "trace.cuh"
 
@@ -344,13 +345,11 @@ static int stream5_launch(StreamArgs args, cudaStream_t st) {
     const size_t limit = S5_SMEM_MAX;
     if (smem > limit)
         return fail(TL_EINVAL, "quantized_matmul: activations do not fit in shared memory (N=%d, K=%d, rows=%d)", args.N, args.K, MP);
-    static bool configured = false;  // per process: one device per process
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(w4a16_stream5_kernel<T, MP, U, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(limit));
-        if (e != cudaSuccess) return fail(TL_ECUDA, "quantized_matmul: cannot raise shared memory limit: %s", cudaGetErrorString(e));
-        configured = true;
-    }
+    static PerDevice configured;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return fail(TL_ECUDA, "quantized_matmul: no device");
+    if (!configured(device, [&] { return cudaFuncSetAttribute(w4a16_stream5_kernel<T, MP, U, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(limit)) == cudaSuccess; }))
+        return fail(TL_ECUDA, "quantized_matmul: cannot raise shared memory limit: %s", cudaGetErrorString(cudaGetLastError()));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid_x, ceil_div(args.M, args.rows_per_pass));
     cfg.blockDim = dim3(S5_WARPS * 32);

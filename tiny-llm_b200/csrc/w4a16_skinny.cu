@@ -34,6 +34,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "per_device.h"
 #include "tc05.cuh"
 #include "trace.cuh"
 
@@ -616,13 +617,14 @@ static int sk_cached_map(CUtensorMap *out, const void *ptr, int kind, cuuint64_t
 template <typename T, int NT, bool WIDE1 = false, bool DUAL = false>
 static int skinny_launch(const CUtensorMap &ma, const CUtensorMap &mw, const CUtensorMap &mw2, const SkArgs &args, int grid, cudaStream_t st) {
     constexpr size_t smem = SkSmem<NT, WIDE1>::BYTES;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(w4a16_skinny_kernel<T, NT, WIDE1, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) != cudaSuccess ||
-            cudaFuncSetAttribute(w4a16_skinny_kernel<T, NT, WIDE1, DUAL>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-            return fail(TL_ECUDA, "quantized_matmul: cannot raise shared memory limit");
-        configured = true;
-    }
+    static PerDevice configured;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return fail(TL_ECUDA, "quantized_matmul: no device");
+    if (!configured(device, [] {
+            return cudaFuncSetAttribute(w4a16_skinny_kernel<T, NT, WIDE1, DUAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess &&
+                   cudaFuncSetAttribute(w4a16_skinny_kernel<T, NT, WIDE1, DUAL>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) == cudaSuccess;
+        }))
+        return fail(TL_ECUDA, "quantized_matmul: cannot raise shared memory limit");
     cudaError_t e = launch_chained(w4a16_skinny_kernel<T, NT, WIDE1, DUAL>, dim3(grid), dim3(SK_THREADS), smem, st, ma, mw, mw2, args);
     if (e != cudaSuccess) return fail(TL_ECUDA, "w4a16_skinny: launch failed: %s", cudaGetErrorString(e));
     TL_LAUNCH_CHECK("w4a16_skinny");
