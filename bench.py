@@ -28,10 +28,10 @@ Numbers on the JSON line (decode):
             token feedback on the device (CUDA events, max over ranks)
   e2e       same metric through the public model call, per step: pinned-host token -> device copy,
             model(...), device -> host read of the sampled token
-  roofline  the W4A16 weight-streaming kernel: the 145 projection launches of one token exactly as the
-            decode graph issues them (2.137 GB of packed weights, > L2), replayed from a CUDA graph,
-            CUDA-event timed; achieved = algorithmic bytes / time, traffic = ncu DRAM bytes of the same
-            launches (read from the committed capture named in `traffic_source`, null if there is none)
+  roofline  the kernel that a decode step is: decode_step_kernel, one launch a token (2.137 GB of packed weights, > L2, and the
+            request's K/V), replayed from a CUDA graph, CUDA-event timed; where the step is a chain of launches
+            (TL_DECODE_STEP=0), its 145 projection launches as the graph issues them.  achieved = algorithmic bytes / time,
+            traffic = ncu DRAM bytes of the same launches (read from the committed capture named in `traffic_source`, null if there is none)
   --workload voluzen  (beside the headline) the Voluzen design - latent attention + mixture of experts, bf16 weights - at
             two sizes beside Qwen3 W4A16 of equal width / depth / heads / active feed-forward width: prefill and decode tok/s,
             and the design's kernels alone against the measured peaks; its own JSON line
@@ -95,7 +95,7 @@ def measured_peaks() -> dict:
 
 
 def committed_traffic(kernel: str):
-    """(bytes per launch, file) from the committed ncu capture of this round, or (None, None)."""
+    """(bytes per launch, file) from the committed ncu capture, or (None, None)."""
     path = ROOT / "profiles" / "traffic.json"
     if not path.exists():
         return None, None
@@ -268,7 +268,10 @@ def run_decode(args) -> None:
     e2e_value = world * e2e_steps / e2e_s
     meta_bytes = engine.upload_bytes_per_step()
 
-    roofline = matvec_roofline(model, engine, ext, device) if rank == 0 else None
+    roofline = None
+    if rank == 0:
+        one_launch = engine._one_launch and not engine._chain_for(offset)
+        roofline = step_roofline(model, engine, offset) if one_launch else matvec_roofline(model, engine, ext, device)
     for c in cache:
         c.release()
 
@@ -313,8 +316,33 @@ def run_decode(args) -> None:
         print(json.dumps(line), flush=True)
 
 
+def step_roofline(model, engine, context: int) -> dict:
+    """The one launch that a decode step of the request just decoded is: its graph once more on the metadata of the last step (the same token
+    into the same slot)."""
+    from tiny_llm_b200.synthetic import weight_stream_bytes
+
+    stream = torch.cuda.current_stream()
+    for _ in range(3):
+        engine._graph.replay()
+    stream.synchronize()
+    ms = statistics.median(cuda_time_ms(engine._graph.replay, stream) for _ in range(20))
+    margs = model.mlx_model.args
+    # every packed weight, scale and bias once (0.53125 B/weight), the request's keys and values (36 layers x 8 heads x 128 x 2 x bf16), the logits
+    algorithmic = weight_stream_bytes(margs) + 4 * len(model.layers_inner) * engine.Hkv * engine.D * context + 2 * margs.vocab_size
+    peak = measured_peaks()
+    achieved = algorithmic / (ms / 1e3) / 1e9
+    traffic, traffic_source = committed_traffic("decode_step_kernel")
+    return {
+        "kernel": "decode_step_kernel<1 request> (embedding, all blocks, norm, head and argmax in one cooperative launch)",
+        "bound": "hbm", "achieved": round(achieved, 1), "peak": peak["hbm_gbs"], "peak_source": peak["source"], "unit": "GB/s",
+        "frac": round(achieved / peak["hbm_gbs"], 4), "traffic": traffic, "traffic_source": traffic_source, "launches": 1,
+        "avg_launch_us": round(ms * 1e3, 3), "algorithmic_bytes_per_launch": algorithmic,
+        "timing": "cuda events on the launching stream around a graph replay of one step, median of 20",
+    }
+
+
 def matvec_roofline(model, engine, ext, device) -> dict:
-    """The projection launches of one decode token exactly as the engine issues them (per layer:
+    """The projection launches of one decode token exactly as the engine issues them in the chain of launches (per layer:
     rms_norm+q|k|v, o+residual, rms_norm+gate|up+swiglu, down+residual; then rms_norm+head), M = 1,
     from one captured graph: 2.137 GB of distinct packed weights per replay, so every launch
     streams from HBM (L2 = 126 MB)."""

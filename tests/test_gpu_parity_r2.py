@@ -1,4 +1,4 @@
-"""Round-2 parity additions ("close the parity gaps that are closable"): every test
+"""Parity at serving sizes: every test
 compares the CUDA path with the CPU ORACLE (never GPU kernel against GPU kernel) at the sizes the
 serving configurations run: long contexts with split/merge, 64-slot batches with idle slots, the
 two-tile GEMM at the real down-projection shape, a full-depth Qwen3-4B step and the committed
@@ -336,7 +336,7 @@ def test_row_variant_graphs_give_the_bits_of_the_full_step(dev, monkeypatch):
 
 
 def test_engine_recapture_after_slab_growth_does_not_touch_released_pages(dev):
-    """a second, larger engine moves the page slabs; the first engine then re-captures its graph.
+    """A second, larger engine moves the page slabs; the first engine then re-captures its graph.
     The warm-up passes of that capture must not append through stale metadata into pages that were released
     and handed to another request in the meantime."""
     ns = to_device(synthetic_qwen3("tiny-d128", seed=0, realistic=True, max_position_embeddings=512), dev)

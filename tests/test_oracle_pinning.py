@@ -273,7 +273,7 @@ def test_paged_cache_update_writes_one_slice_in_place():
 
 
 # ---------------------------------------------------------------------------------------------
-# fp64 referee (VERDICT r1, weak #1): the float operators of the oracle are fp32 restatements of
+# fp64 referee: the float operators of the oracle are fp32 restatements of
 # the Metal kernels; MLX cannot run here, so their only other witness was a second restatement.
 # Each operator is evaluated once more in float64 straight from its mathematical definition (no
 # shared code with oracle/ops.py beyond the nibble unpacking spec of quantize.py:113-115) - an
