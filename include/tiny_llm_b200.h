@@ -254,7 +254,8 @@ int tl_decode_attention_fused(const void *qkv, const void *q_norm_weight, const 
                               float *workspace, int batch, int num_heads, int num_kv_heads, int head_dim, float eps,
                               float scale, int num_pages, int page_size, int max_pages, int max_context, int dtype,
                               void *stream);
-/* A whole decoding step of up to 8 requests as one launch (bf16, head_dim 128, 4-bit groups of 128): embedding, every block
+/* A whole decoding step of up to four requests as one launch (bf16, head_dim 128, 4-bit groups of 128; batch * hidden up to 12288; which sizes are taken
+ * tl_decode_step_workspace says): embedding, every block
  * (src/tiny_llm_ref/qwen3_week3.py:55-121,139-146,196-207 at L == 1), final norm, head, greedy argmax.  The plan is a HOST struct,
  * read during the call; every pointer in it is a device pointer.  Matrices other than the embedding table are tl_decode_step_pack()'s
  * results: q|k|v (rows concatenated), o and down packed with halves = 1, gate (top) and up (bottom) together, the head with neither.  workspace: tl_decode_step_workspace() bytes, zeroed once, used by one step at a time and kept between steps;

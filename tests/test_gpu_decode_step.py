@@ -226,3 +226,33 @@ def test_weights_written_in_place_are_seen(cuda_device, what, on_device):
     want, _ = second_step(True, True)
     old, _ = second_step(False, False)
     assert torch.equal(got, want) and torch.equal(got, old) == (what == "nothing") and captures == (1 if what == "nothing" else 2)
+
+
+@pytest.mark.gpu
+def test_two_engines_on_two_streams_at_once(cuda_device):
+    """Steps that fill the GPU by themselves follow one another, whatever stream they come from; other kernels run between them."""
+    dev = cuda_device
+    model = Qwen3ModelWeek3(synthetic_qwen3(OVER, seed=8, device=dev, realistic=True), page_size=64)
+    engines = [DecodeEngine(model, b, 256, dev) for b in (1, 3)]
+    engines[0].reserve_pools(16)
+    want = []
+    for i, engine in enumerate(engines):
+        engine._ensure_graph()
+        engine.tables[:, :, :4] = torch.arange(4 * i, 4 * i + 4 * engine.B, device=dev, dtype=torch.int32).view(engine.B, 4)
+        engine.tokens.fill_(3 + i)
+        engine.context_lens.fill_(200)
+        engine.offsets.fill_(199)
+        engine._graph.replay()
+        want.append(engine.logits.clone())
+    count = ext.waits_given_up()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.Stream()]
+    a = torch.randn(4096, 4096, device=dev).bfloat16()
+    torch.cuda.synchronize()
+    for _ in range(100):
+        for engine, stream in zip(engines, streams):
+            with torch.cuda.stream(stream):
+                engine._graph.replay()
+        with torch.cuda.stream(streams[2]):
+            a @ a
+    torch.cuda.synchronize()
+    assert all(torch.equal(e.logits, w) for e, w in zip(engines, want)) and ext.waits_given_up() == count

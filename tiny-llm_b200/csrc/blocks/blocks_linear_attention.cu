@@ -446,7 +446,8 @@ decay_output_kernel(const int32_t *__restrict__ seq_info, int heads, int dk, int
 // the launch that writes the slot of a sequence in several segments does not read it.
 // 2048 tokens in two sequences of 16 heads of 64 x 128: the walk in segments 99 + 19 + 24 us, this 18 + 8 + 48 (8 + 8 heads 1.6 x, 65 tokens 1.1 x, 8000
 // tokens 2 x as fast); the error against 64 bits is 0.85 to 1.0 of the walk's (with long sums left to the tensor cores it was twice that, at 42 us).
-// What bounds it: instructions, of which the terms of S are a quarter, and three barriers every sixteen tokens with 14 warps an SM.
+// What bounds it: instructions and their latencies, with 14 warps an SM: issue slots 49 % busy (MODE 1: 2900 instructions a warp and sixteen tokens, an eighth of them for the
+// terms of S), 1.8 of the 7.0 cycles between two instructions of a warp for the one before, 2.0 for loads, 0.4 at the three barriers.
 constexpr int kCkTokens = 16, kCkCols = 128;
 
 __device__ __forceinline__ void ck_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {

@@ -105,7 +105,7 @@ int launch_decode_attention_fused(const void *qkv, const void *q_norm_weight, co
                                   int num_kv_heads, int head_dim, float eps, float scale, int num_pages, int page_size,
                                   int max_pages, int max_context, int dtype, cudaStream_t st);
 
-// decode_step.cu (a whole decoding step of up to 8 requests in one launch)
+// decode_step.cu (a whole decoding step of up to four requests in one launch)
 long long decode_step_gave_up();
 size_t decode_step_workspace(int batch, int layers, int num_heads, int num_kv_heads, int hidden, int intermediate, int vocab);
 int launch_decode_step(const tl_decode_step_plan &plan, cudaStream_t st);
