@@ -303,6 +303,7 @@ __device__ __forceinline__ void ds_stage(const DsArgs &a, const unsigned char *s
         for (int k = 8; k > 0; k >>= 1) v += __shfl_xor_sync(0xffffffffu, v, k);
         return v;
     };
+    bool lost = false;  // chunks of this thread did not come: all of its chunks are NaN below
 #pragma unroll 1
     for (int base = threadIdx.x; base < total; base += DS_THREADS * FLIGHT) {
         const unsigned char *p = src + static_cast<size_t>(base) * 32;
@@ -324,12 +325,7 @@ __device__ __forceinline__ void ds_stage(const DsArgs &a, const unsigned char *s
                     pending &= ~(1u << j);
                 }
             if (pending != 0 && !ds_again(spins, dead)) {
-#pragma unroll 1
-                for (int j = 0; j < FLIGHT; ++j)
-                    if (pending >> j & 1u) {
-                        const int idx = base + j * DS_THREADS, m = row_of(idx);
-                        put(m, idx - m * words, make_uint4(DS_NAN2, DS_NAN2, DS_NAN2, DS_NAN2));
-                    }
+                lost = true;
                 break;
             }
         }
@@ -363,6 +359,7 @@ __device__ __forceinline__ void ds_stage(const DsArgs &a, const unsigned char *s
             raw = make_uint4(pack2<bf16>(x0.x * inv * w0.x, x0.y * inv * w0.y), pack2<bf16>(x1.x * inv * w1.x, x1.y * inv * w1.y),
                              pack2<bf16>(x2.x * inv * w2.x, x2.y * inv * w2.y), pack2<bf16>(x3.x * inv * w3.x, x3.y * inv * w3.y));
         }
+        if (lost) raw = make_uint4(DS_NAN2, DS_NAN2, DS_NAN2, DS_NAN2);
         const float2 f0 = unpack2<bf16>(raw.x), f1 = unpack2<bf16>(raw.y), f2 = unpack2<bf16>(raw.z), f3 = unpack2<bf16>(raw.w);
         const float part = half_warp_sum(((f0.x + f0.y) + (f1.x + f1.y)) + ((f2.x + f2.y) + (f3.x + f3.y)));
         if (MP == 1) {
