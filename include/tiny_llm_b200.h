@@ -288,6 +288,10 @@ int tl_decode_step(const tl_decode_step_plan *plan, void *stream);
  * bottom matrix of the same shape), scales and biases included.  halves: rows in eights (cols a multiple of 512), else in sixteens, or in eights of
  * top and bottom (cols a multiple of 256).  out is 16-byte aligned; concatenated rows are packed one after the other. */
 int tl_decode_step_pack(const tl_packed_matrix *top, const tl_packed_matrix *bottom, void *out, int rows, int cols, int halves, void *stream);
+/* The host copies of a paged call's metadata, before it is dispatched: 1 when every context length is 0 or at least query_length and covered by its row
+ * of the block table, every live entry names a page of physical_pages that no other names, and every other entry is -1; else 0.  Host memory; no GPU. */
+int tl_paged_metadata_clean(const int32_t *context_lens, const int32_t *block_table, int batch, int max_pages, long long page_size,
+                            long long physical_pages, long long query_length);
 /* Programmatic dependent launch for the streaming kernels (on by default; 0 turns it off,
  * TL_PDL=0 in the environment does the same). */
 int tl_set_pdl(int enabled);

@@ -350,3 +350,39 @@ def test_append_slots_equals_repeated_token_slots_and_is_all_or_nothing():
     with pytest.raises(RuntimeError, match="slab exhausted"):
         a.append_slots(100)
     assert (a.page_ids, a.page_lens, a.offset, a.pool.num_pages) == before
+
+
+@pytest.mark.parametrize("seed", range(40))
+def test_native_metadata_check_agrees_with_the_scan(seed):
+    """The one native pass against the row-by-row scan: clean tables, and tables with one entry or length changed; a strided or 64-bit
+    copy takes the other way and ends the same."""
+    from extensions_b200 import tiny_llm_ext_b200 as ext
+    from tiny_llm_b200 import attention
+
+    rng = np.random.RandomState(seed)
+    B, page, L = rng.randint(1, 9), int(rng.choice([1, 16, 128])), int(rng.choice([1, 9]))
+    ctx = np.where(rng.rand(B) < 0.2, 0, L + rng.randint(0, 4 * page, B)).astype(np.int32)
+    live = -(-ctx // page)
+    width, physical = int(live.max()) + rng.randint(0, 3) + 1, int(live.sum()) + rng.randint(1, 130)
+    table = np.full((B, width), -1, dtype=np.int32)
+    ids = rng.permutation(physical).astype(np.int32)
+    for b, at in enumerate(np.cumsum(live) - live):
+        table[b, : live[b]] = ids[at : at + live[b]]
+    if seed % 4:
+        b, i = rng.randint(B), rng.randint(width)
+        if seed % 8 < 5:
+            table[b, i] = rng.choice([-2, -1, 0, int(ids[0]), physical - 1, physical, 2**31 - 1])
+        else:
+            ctx[b] = rng.choice([-1, -page, 1, L - 1, width * page, width * page + 1, 2**31 - 1])
+
+    def verdict(check):
+        try:
+            check()
+        except ValueError as error:
+            return str(error)
+        return None
+
+    want = verdict(lambda: attention._raise_first_metadata_error(ctx.tolist(), table.tolist(), page, width, physical, L))
+    assert ext.paged_metadata_clean(ctx, table, page, physical, L) == (want is None)
+    for c, t in ((ctx, table), (ctx.astype(np.int64), table), (ctx, np.repeat(table, 2, axis=1)[:, ::2])):
+        assert verdict(lambda: attention.validate_paged_metadata(c, t, page, physical, L)) == want

@@ -6,6 +6,7 @@
 #include <stdio.h>
 
 #include <atomic>
+#include <vector>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -497,6 +498,35 @@ extern "C" int tl_debug_trace(unsigned long long *device_events, unsigned int *d
     return TL_OK;
 }
 #endif
+
+int tl_paged_metadata_clean(const int32_t *context_lens, const int32_t *block_table, int batch, int max_pages, long long page_size,
+                            long long physical_pages, long long query_length) {
+    // One pass with a bit per physical page; the same in numpy, an expression a check, took about 30 us of a decoding call's host time.
+    if (!context_lens || !block_table || batch < 0 || max_pages < 0 || page_size <= 0 || physical_pages <= 0) return 0;
+    std::vector<uint64_t> seen;
+    try {
+        seen.resize(static_cast<size_t>((physical_pages + 63) / 64));
+    } catch (...) {  // no exception leaves a C entry: the caller's own scan decides
+        return 0;
+    }
+    for (int b = 0; b < batch; ++b) {
+        const long long context = context_lens[b];
+        if (context < 0 || (context > 0 && context < query_length)) return 0;
+        const long long live = (context + page_size - 1) / page_size;
+        if (live > max_pages) return 0;
+        const int32_t *row = block_table + static_cast<size_t>(b) * max_pages;
+        for (int i = 0; i < live; ++i) {
+            const long long id = row[i];
+            if (id < 0 || id >= physical_pages) return 0;
+            const uint64_t bit = uint64_t{1} << (id & 63);
+            if (seen[id >> 6] & bit) return 0;
+            seen[id >> 6] |= bit;
+        }
+        for (int i = static_cast<int>(live); i < max_pages; ++i)
+            if (row[i] != -1) return 0;
+    }
+    return 1;
+}
 
 int tl_set_gemm_pairs(int mode) {
     set_gemm_pairs(mode);

@@ -109,6 +109,7 @@ _SIGNATURES = {
     "tl_decode_step": (_I, [_VP, _VP]),
     "tl_decode_step_pack": (_I, [_VP, _VP, _VP, _I, _I, _I, _VP]),
     "tl_paged_cache_append_chunk": (_I, [_VP] * 5 + [_I] * 4 + [ctypes.c_longlong, ctypes.c_longlong, _I, _VP]),
+    "tl_paged_metadata_clean": (_I, [_VP, _VP, _I, _I, _LL, _LL, _LL]),
     "tl_set_pdl": (_I, [_I]),
     "tl_set_gemm_pairs": (_I, [_I]),
     "tl_tc_gave_up": (ctypes.c_longlong, []),
@@ -667,6 +668,12 @@ def quantized_matmul_fused(scales, biases, b, p0, p1=None, residual=None, prolog
         )
     )
     return out
+
+
+def paged_metadata_clean(context_lens, block_table, page_size: int, physical_pages: int, query_length: int) -> bool:
+    """Whether host copies (contiguous int32 numpy arrays ``[B]`` and ``[B, max_pages]``) of a paged call's metadata pass all of its checks."""
+    return bool(_lib.tl_paged_metadata_clean(context_lens.ctypes.data, block_table.ctypes.data, block_table.shape[0], block_table.shape[1], page_size,
+                                             physical_pages, query_length))
 
 
 def paged_attention_token_major(query, key_pages, value_pages, block_table, context_lens, scale, is_causal, num_kv_heads, num_heads, stream=None):
