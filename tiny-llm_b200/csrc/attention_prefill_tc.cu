@@ -110,8 +110,8 @@ paged_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     extern __shared__ __align__(1024) unsigned char tsm[];
     griddep_launch();  // programmatic dependent launch (common.cuh): the successor may set itself up under this grid
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qb = static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x);  // long (late) query blocks first
-    const int kvh = blockIdx.y, b = blockIdx.z;
+    const int qb = static_cast<int>((gridDim.x - 1 - blockIdx.x) / a.Hkv);  // long (late) query blocks of all heads first
+    const int kvh = blockIdx.x % a.Hkv, b = blockIdx.z;
     const int q0 = qb * a.RH;
     const int ctx = min(a.context_lens[b], a.max_pages * a.page_size);
     // keys any row of this CTA may see: [0, key_end)
@@ -895,8 +895,10 @@ int launch_paged_prefill_tc(const void *q, const void *kp, const void *vp, const
     if (int e = attention_maps(&mq, &mk, &mv, q, kp, vp, rows, L, a.RH, G, num_pages, page_size, num_kv_heads)) return e;
     const int q_blocks = (L + a.RH - 1) / a.RH;
     a.out_token_major = out_token_major ? 1 : 0;
-    dim3 grid(q_blocks, num_kv_heads, B);
-    if (grid.y > 65535 || grid.z > 65535) return fail(TL_EINVAL, "paged_attention: too many heads / requests for one launch");
+    // Key/value heads vary fastest, so that a request's longest blocks start first in all heads and its shortest come last: with a head's blocks together
+    // the last head's longest ones started last (32 heads over 8, 2048 tokens of 3500: 104 -> 84 us; of 2048: 60 -> 41; 4096 of 4096: 157 -> 131).
+    dim3 grid(static_cast<unsigned>(q_blocks) * num_kv_heads, 1, B);
+    if (num_kv_heads > 65535 || grid.z > 65535 || static_cast<long long>(q_blocks) * num_kv_heads > 0x7fffffffLL) return fail(TL_EINVAL, "paged_attention: too many heads / requests for one launch");
     static const bool p_tmem = [] { const char *e = getenv("TL_FA_P_TMEM"); return e == nullptr || e[0] != '0'; }();  // 0: P through shared memory (control)
     if (int e = p_tmem ? attention_launch<paged_prefill_tc_kernel<true>>(grid, TC_THREADS, TC_SMEM_BYTES, st, mq, mk, mv, a)
                        : attention_launch<paged_prefill_tc_kernel<false>>(grid, TC_THREADS, TC_SMEM_BYTES, st, mq, mk, mv, a))
