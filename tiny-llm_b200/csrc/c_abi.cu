@@ -61,8 +61,8 @@ const char *tl_last_error(void) { return g_error; }
 
 long long tl_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 long long tl_tc_gave_up(void) {
-    const long long attention = decode_tc_gave_up(), step = decode_step_gave_up();
-    return attention < 0 || step < 0 ? -1 : attention + step;
+    const long long attention = decode_tc_gave_up(), step = decode_step_gave_up(), pairs = gemm2_gave_up();
+    return attention < 0 || step < 0 || pairs < 0 ? -1 : attention + step + pairs;
 }
 
 int tl_device_info(int *sms, int *major, int *minor) {
@@ -153,8 +153,10 @@ int tl_quantized_gated(const void *gate_scales, const void *gate_biases, const v
     if (M > 0 && K > 0 && N > 0 && N % 128 == 0 && (gate_flags & up_flags & 1) && gate_scales && gate_biases && gate_b && up_scales && up_biases && up_b && a) {
         int rc = TL_OK;
         if (use_skinny_kernel(M, N, K, dtype, 1)
-                ? launch_w4a16_skinny_gate_up(gate_scales, gate_biases, gate_b, up_scales, up_biases, up_b, a, out, M, N, K, dtype, workspace, workspace_bytes, as_stream(stream), &rc)
-                : use_stream_kernel(M, N, K, dtype, 1) && launch_w4a16_gate_up(gate_scales, gate_biases, gate_b, up_scales, up_biases, up_b, a, out, M, N, K, dtype, as_stream(stream), &rc))
+            ? launch_w4a16_skinny_gate_up(gate_scales, gate_biases, gate_b, up_scales, up_biases, up_b, a, out, M, N, K, dtype, workspace, workspace_bytes, as_stream(stream), &rc)
+            : use_stream_kernel(M, N, K, dtype, 1)
+                ? launch_w4a16_gate_up(gate_scales, gate_biases, gate_b, up_scales, up_biases, up_b, a, out, M, N, K, dtype, as_stream(stream), &rc)
+                : launch_w4a16_gemm2_gated({gate_b, gate_scales, gate_biases}, {up_b, up_scales, up_biases}, a, out, M, N, K, dtype, as_stream(stream), &rc))
             return rc;
     }
     return tl_quantized_gate_up(gate_scales, gate_biases, gate_b, up_scales, up_biases, up_b, a, scratch, out, M, N, K, dtype, gate_flags, up_flags, workspace,

@@ -382,6 +382,29 @@ static long long gemm_plan(int mt, int n_tiles, int m_tiles, GemmPlan &plan) {
     return static_cast<long long>(groups / sms) * gemm_block_cost(mt) + gemm_block_cost(plan.piece);
 }
 
+// The number of token tiles a CTA takes, with its plan and cost.
+static int gemm_choice(int M, int N, int K, GemmPlan &best_plan, long long &best_cost) {
+    static const int mt_max = [] { const char *e = getenv("TL_GEMM_MT"); return e ? atoi(e) : 4; }();  // caps the token tiles per CTA (A/B runs)
+    const int n_tiles = ceil_div(K, GN), m_tiles = ceil_div(M, GM);
+    GemmPlan plan;
+    int best = 0;
+    for (int mt = 1; mt <= 4 && mt <= max(mt_max, 1); ++mt) {
+        // Four token tiles leave room for a 2-stage ring only: good for the short reductions, not for the long ones (M = 4096:
+        // N = 2560 gains 13-20 % over two tiles, N = 9728 loses 7 %).
+        if ((mt == 4 && N > 3072) || mt > m_tiles) continue;
+        const long long cost = gemm_plan(mt, n_tiles, m_tiles, plan);
+        if (best == 0 || cost <= best_cost) best = mt, best_cost = cost, best_plan = plan;
+    }
+    return best;
+}
+
+long long w4a16_gemm_cost(int M, int N, int K) {
+    GemmPlan plan{};
+    long long cost = 0;
+    gemm_choice(M, N, K, plan, cost);
+    return cost;
+}
+
 template <typename T, int MT>
 static int gemm_launch(const CUtensorMap &map, const void *scales, const void *biases, const void *b, void *out, int M, int N, int K,
                        int vec_store, const GemmPlan &plan, cudaStream_t st) {
@@ -416,18 +439,9 @@ static int gemm_t(const void *scales, const void *biases, const void *a, const v
                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(TL_ECUDA, "quantized_matmul: cuTensorMapEncodeTiled failed (%d)", static_cast<int>(r));
     const int vec_store = (K % 8 == 0 && aligned16(out)) ? 1 : 0;
-    static const int mt_max = [] { const char *e = getenv("TL_GEMM_MT"); return e ? atoi(e) : 4; }();  // caps the token tiles per CTA (A/B runs)
-    const int n_tiles = ceil_div(K, GN), m_tiles = ceil_div(M, GM);
-    GemmPlan plan, best_plan{};
-    int best = 0;
+    GemmPlan best_plan{};
     long long best_cost = 0;
-    for (int mt = 1; mt <= 4 && mt <= max(mt_max, 1); ++mt) {
-        // Four token tiles leave room for a 2-stage ring only: good for the short reductions, not for the long ones (M = 4096:
-        // N = 2560 gains 13-20 % over two tiles, N = 9728 loses 7 %).
-        if ((mt == 4 && N > 3072) || mt > m_tiles) continue;
-        const long long cost = gemm_plan(mt, n_tiles, m_tiles, plan);
-        if (best == 0 || cost <= best_cost) best = mt, best_cost = cost, best_plan = plan;
-    }
+    const int best = gemm_choice(M, N, K, best_plan, best_cost);
     switch (best) {
         case 1: return gemm_launch<T, 1>(map, scales, biases, b, out, M, N, K, vec_store, best_plan, st);
         case 2: return gemm_launch<T, 2>(map, scales, biases, b, out, M, N, K, vec_store, best_plan, st);

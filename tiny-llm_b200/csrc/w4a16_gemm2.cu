@@ -2,49 +2,54 @@
 //
 //   out[m, n] = sum_k a[m, k] * T(code[n, k] * scale[n, k/128] + bias[n, k/128])       (m = token, n = feature)
 //
-// Why: the one-CTA kernel is bound by L2 -> SM bandwidth, not by the tensor core.  Its per-block cycle trace
-// (tools/gemm_blocks.py, profiles/r02_gemm_blocks.md) shows the activation tiles arriving just in time and the MMA warp
-// paced at ~1500 cycles per 64-wide block with four token tiles (1024 cycles of tensor work): 68 KB per block and SM is
-// 45 B/cycle, the chip's ~42 B/cycle/SM L2 ceiling (B300_MICROARCH.md: LTS cap ~6300 B/cycle).  Every CTA needs
-// tokens x 64 x 2 bytes of activations per 128 features it computes; the only way to need less is to compute more
-// features per activation byte - and the dequantisers cannot feed a second weight tile per CTA.  A CTA pair can: with
-// cta_group::2 one MMA spans 256 token rows (128 per CTA) x 256 features, each CTA dequantises HALF of the weight tile
-// (its 128 features) into its own shared memory and the tensor cores of both SMs read both halves.  Per CTA and block:
-// 32 KB of activations (two 256-token MMA tiles) + one dequantised tile for 1024 cycles of tensor work: 35 B/cycle.
+// Why pairs: with cta_group::2 one MMA spans 256 token rows (128 per CTA) x 256 weight rows, each CTA dequantises HALF of the weight tile into its own
+// shared memory and the tensor cores of both SMs read both halves.  Per CTA and 64-wide block that is 32 KB of activations (two 256-token MMA
+// tiles) and one dequantised tile for 1024 cycles of tensor work.  The one-CTA kernel needs 68 KB from L2 for the same (about 42 bytes a cycle and
+// SM is what the chip gives), and 208 KB through its shared memory (operands read, tiles written), 1640 cycles at 128 bytes a cycle;
+// here it is 112 KB.
 //
-// Roles per CTA (384 threads): warp 0 TMA producer (its 128 token rows of each MMA tile), warp 1 MMA issuer in the
+// Persistent: one pair of CTAs per two SMs takes tiles in turn, so that the next tile's activations and weights arrive, and are unpacked, while the last
+// one's results are read out by warps of their own and leave by TMA.  (With a CTA pair a tile, its dequantisers reading the results out in 16-byte
+// stores of 32 rows each, a tile cost 24 us beside its blocks.)
+//
+// Roles per CTA (640 threads): warp 0 TMA producer (its 128 token rows of each MMA tile), warp 1 MMA issuer in the
 // leader CTA (rank 0) / readiness forwarder in the peer, warp 2 TMEM allocation (cta_group::2, all 512 columns: two
-// accumulators of 256 features), warps 4-11 dequantisers then epilogue (lane = token row).
+// accumulators of 256 features), warps 4-11 dequantisers, warps 12-19 epilogue (lane = token row).
 // Barriers live at the same offsets in both CTAs: full (own TMA + own dequantisers; in the leader also the peer's
-// "my tiles of this stage are complete"), empty and tmem_full (arrived in BOTH CTAs by the leader's multicast commit).
+// "my tiles of this stage are complete"), empty and acc_full (arrived in BOTH CTAs by the leader's multicast commit), acc_empty (the leader's: both CTAs'
+// epilogue warps).  Every wait is bounded (tc_wait.cuh); a CTA whose wait gave up stores NaN.
 // Replaces quantized_matmul_simdgroup_w4a16_g128 (src/extensions_ref/src/quantized_matmul.metal:96-249)
-// for M > 256; same rounding points as w4a16_gemm.cu (weights rounded to the activation dtype, fp32 accumulation).
+// for larger M; same rounding points as w4a16_gemm.cu (weights rounded to the activation dtype, fp32 accumulation).
+//
+// Measured (bf16; before: a pair of CTAs a tile): 2048 rows of 2560 -> 19456 230 -> 139 us (1464 TF/s, 90 % of the measured burst), 4096 rows 442 -> 264
+// (1546 TF/s), 2560 -> 9728 131 -> 77; gate and up projection with their activation in one launch, 2048 rows of 2560 -> 9728: 245 (two
+// launches of the one-CTA kernel and one of the activation) -> 150 us.
 #include <cuda.h>
 #include <stdlib.h>
 #include <cudaTypedefs.h>
 
-#include <mutex>
-#include <unordered_map>
-
 #include "common.cuh"
 #include "kernels.h"
-#include "tc05.cuh"
+#include "per_device.h"
+#include "tc_wait.cuh"
 #include "trace.cuh"
 
 namespace tl {
 
 constexpr int P_TOK = 128;        // token rows per CTA and MMA tile (the pair's MMA spans 256)
-constexpr int P_FEAT = 128;       // features dequantised per CTA (the pair's MMA spans 256)
+constexpr int P_ROWS = 128;       // weight rows dequantised per CTA (the pair's MMA spans 256)
 constexpr int P_KB = 64;          // reduction elements per stage (one 128-byte swizzle atom)
 constexpr int P_MT = 2;           // 256-token MMA tiles per pair: 2 x 256 accumulator columns = all of TMEM
 constexpr int P_STAGES = 4;
 constexpr int P_TILE = P_TOK * P_KB * 2;          // 16 KiB, activation and weight tiles alike
 constexpr int P_A_STAGE = P_MT * P_TILE;
 constexpr int P_STAGE = P_A_STAGE + P_TILE;       // 48 KiB
-constexpr int P_BAR_OFF = P_STAGES * P_STAGE;     // 192 KiB
+constexpr int P_DEQ_WARPS = 8, P_EPI_WARPS = 8;
+constexpr int P_OUT_OFF = P_STAGES * P_STAGE;     // 192 KiB; then 32 token rows x 64 features of results per epilogue warp
+constexpr int P_OUT_BYTES = 32 * 128;
+constexpr int P_BAR_OFF = P_OUT_OFF + P_EPI_WARPS * P_OUT_BYTES;
 constexpr int P_SMEM = P_BAR_OFF + 256;
-constexpr int P_THREADS = 384;
-constexpr int P_DEQ_WARPS = 8;
+constexpr int P_THREADS = 32 * (4 + P_DEQ_WARPS + P_EPI_WARPS);
 constexpr int P_TMEM_COLS = 512;
 
 // ---- cluster / pair primitives ------------------------------------------------
@@ -56,24 +61,12 @@ __device__ __forceinline__ uint32_t p_cta_rank() {
 __device__ __forceinline__ void p_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// arrive on the barrier at the same shared-memory offset in CTA `rank` of the cluster
-__device__ __forceinline__ void p_mbar_arrive_remote(uint32_t local_bar, uint32_t rank) {
-    asm volatile(
-        "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tmbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}" ::"r"(local_bar),
-        "r"(rank)
-        : "memory");
-}
-// wait with cluster-scope acquire (the arrival came from the other CTA)
-__device__ __forceinline__ void p_mbar_wait_cluster(uint32_t bar, uint32_t parity) {
-    uint32_t done = 0, spins = 0;
-    while (!done) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (!done && ++spins > (1u << 24)) __trap();
-    }
+// An arrival on the barrier at this shared-memory offset in the leader.  What it reports (tiles in, or accumulators out of, the arriving CTA's own
+// memory) is read and written by that CTA's own SM and has been ordered there by a barrier or a proxy fence; a release at cluster
+// scope, which was here before, waits for all of the SM's memory traffic: 2000 cycles a stage under load (512 tokens of 2560 -> 18944:
+// 60 -> 45 us without it).
+__device__ __forceinline__ void p_mbar_arrive_leader(uint32_t bar) {
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, 0;\n\tmbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void p_tc_mma2(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -86,6 +79,43 @@ __device__ __forceinline__ void p_tc_commit2(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
                  "h"(static_cast<unsigned short>(3))
                  : "memory");
+}
+
+__device__ __forceinline__ void p_tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {  // without the wait
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
+          "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
+
+// silu(gate) * up as swiglu's kernel gives it, to the bit: the product of an exact quotient, rounded to T.  The quotient is taken from the
+// branch-free division first, so that sixteen of them overlap; where what it leaves open (2 ulp of the quotient, so at most 6 of the
+// product) could change the rounding to bf16, or the operands are out of that division's range, the exact one decides (0.03 % of them).
+template <typename T, int COUNT>
+__device__ __forceinline__ void p_gated(const float (&gate)[COUNT], const float (&up)[COUNT], float (&y)[COUNT]) {
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+        // how far above (the midpoint between two bf16) - 8 ulp, in the upper half of a word; how far a magnitude is above the smallest
+        auto above = [](float v) { return __float_as_uint(v) * 65536u + ((8u - 0x8000u) << 16); };
+        auto size = [](float v) { return (__float_as_uint(v) & 0x7fffffffu) - 1u; };  // of 0 (both ways give it) the largest
+        uint32_t nearest = 0xffffffffu, smallest = 0xffffffffu;
+        float lowest = 0.f;
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) {
+            y[i] = __fdividef(gate[i], 1.0f + expf(-gate[i])) * up[i];
+            nearest = min(nearest, above(y[i])), smallest = min(smallest, size(y[i])), lowest = fminf(lowest, gate[i]);
+        }
+        constexpr uint32_t kNear = 17u << 16, kSmall = 0x0da24260u;  // 1e-30
+        if (__any_sync(0xffffffffu, nearest < kNear || smallest < kSmall || lowest < -60.f)) {
+#pragma unroll
+            for (int i = 0; i < COUNT; ++i)
+                if (above(y[i]) < kNear || size(y[i]) < kSmall || gate[i] < -60.f) y[i] = (gate[i] / (1.0f + expf(-gate[i]))) * up[i];
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) y[i] = (gate[i] / (1.0f + expf(-gate[i]))) * up[i];
+    }
 }
 
 template <typename T>
@@ -107,45 +137,75 @@ struct PDeq<__half> {
     static constexpr uint32_t MAGIC = 0x64006400u;  // (1024, 1024)
 };
 
+// What a pair works on: n_tiles feature tiles x groups of two 256-token tiles, dealt to the pairs in turn.  The first `full` of them go out whole; the
+// rest, which would fill less than half of a last round, in single 256-token tiles.
+struct PairPlan {
+    int n_tiles, m_tiles, full, items;
+};
+struct PairItem {
+    int n_tile, m0, mt;  // feature tile, first 256-token tile, how many (0: nothing, a short group's second half)
+};
+__host__ __device__ __forceinline__ PairItem pair_item(const PairPlan &p, int i) {
+    int tile = i, m0 = 0, most = P_MT;
+    if (i >= p.full) tile = p.full + (i - p.full) / P_MT, m0 = (i - p.full) % P_MT, most = 1;
+    m0 += tile / p.n_tiles * P_MT;
+    const int left = p.m_tiles - m0;
+    return {tile % p.n_tiles, m0, left < most ? (left < 0 ? 0 : left) : most};
+}
+
 template <typename T>
-__global__ void __launch_bounds__(P_THREADS, 1) w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const T *__restrict__ scales,
-                                                                   const T *__restrict__ biases, const uint32_t *__restrict__ b, T *__restrict__ out,
-                                                                   int M, int N, int K, int vec_store) {
+struct PairWeights {
+    const T *scales, *biases;
+    const uint32_t *b;
+};
+
+// GATED: out = silu(a gate^T) * (a up^T), both rounded to T first.  The leader brings 128 rows of the gate, the peer the same 128 of the up projection, so
+// that both halves of a feature's pair lie in the same lane of tensor memory, 128 columns apart.
+template <typename T, bool GATED>
+__global__ void __launch_bounds__(P_THREADS, 1)
+w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_out, const PairWeights<T> w0, const PairWeights<T> w1,
+                   T *__restrict__ out, int M, int N, int K, int tma_store, const PairPlan plan) {
     extern __shared__ __align__(1024) unsigned char psm[];
 #if TL_TRACE
-    // per-block cycle stamps of the leader CTA (0,0) (tools/gemm_blocks.py): role 0 = MMA warp (k: stage complete in both
+    // per-block cycle stamps of the leader CTA's first tile (tools/gemm_blocks.py): role 0 = MMA warp (k: stage complete in both
     // CTAs, -, MMAs issued), role 1 = first dequantiser warp (k: loop top, math done, stage free, handed over)
     __shared__ unsigned long long trc[2][40][4];
 #define P_TRC(role, i, k)                                                                                                    \
     do {                                                                                                                     \
-        if (blockIdx.x == 0 && blockIdx.y == 0 && (threadIdx.x & 31) == 0 && (i) < 40) trc[role][i][k] = clock64();         \
+        if (blockIdx.x == 0 && it == 0 && (threadIdx.x & 31) == 0 && (i) < 40) trc[role][i][k] = clock64();                 \
     } while (0)
 #else
 #define P_TRC(role, i, k) do { } while (0)
 #endif
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = p_cta_rank();                    // 0 = leader (issues the MMAs)
-    const int n_pair = blockIdx.x >> 1, m_pair = blockIdx.y;
+    const int rank = static_cast<int>(p_cta_rank());       // 0 = leader (issues the MMAs)
+    const int unit = blockIdx.x >> 1, units = gridDim.x >> 1;
     const int num_kb = N / P_KB;
     const int G = N / 128;
+    constexpr int FEATURES = GATED ? P_ROWS : 2 * P_ROWS;  // of a tile
 
     const uint32_t smem0 = g_smem_u32(psm);
     const uint32_t bar = smem0 + P_BAR_OFF;
     // ONE "full" barrier per stage and CTA: own TMA (expect_tx arrival + bytes) + own eight dequantiser warps; in the
     // leader one more arrival, sent by the peer when ITS barrier of the stage has completed.  The MMA warp pays a single
     // try_wait per block: what it executes between two blocks' MMAs is time the tensor cores idle.
-    const uint32_t full = bar, empty = bar + 8 * P_STAGES;
-    const uint32_t tmem_full = bar + 16 * P_STAGES;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(psm + P_BAR_OFF + 16 * P_STAGES + 8);
+    const uint32_t full = bar, empty = full + 8 * P_STAGES, acc_full = empty + 8 * P_STAGES, acc_empty = acc_full + 8 * P_MT;
+    volatile int *dead = reinterpret_cast<volatile int *>(psm + P_BAR_OFF + 16 * P_STAGES + 16 * P_MT);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(const_cast<int *>(dead)) + 1;
 
-    if (warp == 0 && lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
     if (warp == 1 && lane == 0) {
         for (int i = 0; i < P_STAGES; ++i) {
             g_mbar_init(full + 8 * i, 1 + P_DEQ_WARPS + (rank == 0 ? 1 : 0));
             g_mbar_init(empty + 8 * i, 1);
         }
-        g_mbar_init(tmem_full, 1);
+        for (int i = 0; i < P_MT; ++i) {
+            g_mbar_init(acc_full + 8 * i, 1);
+            g_mbar_init(acc_empty + 8 * i, 2 * P_EPI_WARPS);  // both CTAs' (the leader's barrier is the one that is used)
+        }
+        *dead = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_out) : "memory");
     }
     if (warp == 2) {  // both CTAs of the pair issue the paired allocation (same shared-memory slot offset)
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(g_smem_u32(tmem_slot)), "n"(P_TMEM_COLS) : "memory");
@@ -160,159 +220,249 @@ __global__ void __launch_bounds__(P_THREADS, 1) w4a16_gemm2_kernel(const __grid_
         // ------------------------------------------------ TMA producer: this CTA's 128 token rows of each MMA tile
         int s = 0;
         uint32_t ph = 1;
-        for (int kb = 0; kb < num_kb; ++kb) {
-            g_mbar_wait(empty + 8 * s, ph);
-            if (g_elect_one()) {
-                g_mbar_expect_tx(full + 8 * s, P_A_STAGE);
+        for (int it = unit; it < plan.items; it += units) {
+            const PairItem item = pair_item(plan, it);
+            for (int kb = 0; item.mt > 0 && kb < num_kb; ++kb) {
+                if (!tc_wait(empty + 8 * s, ph, dead)) goto done;
+                if (g_elect_one()) {
+                    g_mbar_expect_tx(full + 8 * s, item.mt * P_TILE);
 #pragma unroll
-                for (int i = 0; i < P_MT; ++i)  // token rows beyond M are zero-filled by the TMA unit
-                    g_tma_load_2d(smem0 + s * P_STAGE + i * P_TILE, &tmap_a, kb * P_KB, (m_pair * P_MT + i) * 256 + static_cast<int>(rank) * P_TOK,
-                                  full + 8 * s);
+                    for (int i = 0; i < P_MT; ++i)  // token rows beyond M are zero-filled by the TMA unit
+                        if (i < item.mt)
+                            g_tma_load_2d(smem0 + s * P_STAGE + i * P_TILE, &tmap_a, kb * P_KB, (item.m0 + i) * 256 + rank * P_TOK, full + 8 * s);
+                }
+                __syncwarp();
+                if (++s == P_STAGES) s = 0, ph ^= 1u;
             }
-            __syncwarp();
-            if (++s == P_STAGES) s = 0, ph ^= 1u;
         }
-    } else if (warp == 1) {
+    } else if (warp == 1 && rank == 0) {
+        // ------------------------------------------------ MMA issuer (leader): 256 x 256 x 16 a time
+        constexpr uint32_t idesc = p_instr_desc<T>();
+        const uint64_t adesc0 = g_smem_desc_sw128(smem0, 0, 1024), bdesc0 = g_smem_desc_sw128(smem0 + P_A_STAGE, 0, 1024);
         int s = 0;
-        uint32_t ph = 0;
-        if (rank == 0) {
-            // ------------------------------------------------ MMA issuer (leader): 8 MMAs of 256 x 256 x 16 per stage
-            constexpr uint32_t idesc = p_instr_desc<T>();
-            const uint64_t adesc0 = g_smem_desc_sw128(smem0, 0, 1024), bdesc0 = g_smem_desc_sw128(smem0 + P_A_STAGE, 0, 1024);
-            for (int kb = 0; kb < num_kb; ++kb) {
-                p_mbar_wait_cluster(full + 8 * s, ph);  // cluster-scope acquire: one of the arrivals is the peer's
+        uint32_t ph = 0, e_ph[P_MT] = {1, 1};
+        auto products = [&](int stage, int i, int kb) {  // one lane: a block's four steps of one token tile
+            const uint64_t at = static_cast<uint64_t>(stage * (P_STAGE >> 4));
+#pragma unroll
+            for (int k = 0; k < P_KB / 16; ++k)  // +32 bytes along K per step: +2 in the (addr >> 4) field
+                p_tc_mma2(tmem_d + i * 256, adesc0 + at + i * (P_TILE >> 4) + 2 * k, bdesc0 + at + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        };
+        for (int it = unit; it < plan.items; it += units) {
+            const PairItem item = pair_item(plan, it);
+            if (item.mt == 0) continue;
+            // The first blocks, as many as there are stages, for the first token tile, then for the second: its accumulator is still being read
+            // out for the tile before, meanwhile.
+            const int head = min(P_STAGES, num_kb), s0 = s;
+            if (!tc_wait(acc_empty, e_ph[0], dead)) goto done;
+            e_ph[0] ^= 1u;
+            for (int kb = 0; kb < head; ++kb) {
+                if (!tc_wait(full + 8 * s, ph, dead)) goto done;
                 P_TRC(0, kb, 0);
                 P_TRC(0, kb, 1);
                 g_tc_fence_after();
                 if (g_elect_one()) {
-                    const uint64_t stage = static_cast<uint64_t>(s * (P_STAGE >> 4));
-#pragma unroll
-                    for (int i = 0; i < P_MT; ++i) {
-#pragma unroll
-                        for (int k = 0; k < P_KB / 16; ++k)  // +32 bytes along K per step: +2 in the (addr >> 4) field
-                            p_tc_mma2(tmem_d + i * 256, adesc0 + stage + i * (P_TILE >> 4) + 2 * k, bdesc0 + stage + 2 * k, idesc,
-                                      (kb > 0 || k > 0) ? 1u : 0u);
-                    }
-                    p_tc_commit2(empty + 8 * s);  // both CTAs may refill the stage once these MMAs have read it
+                    products(s, 0, kb);
+                    if (item.mt == 1) p_tc_commit2(empty + 8 * s);
                 }
                 __syncwarp();
                 P_TRC(0, kb, 2);
                 if (++s == P_STAGES) s = 0, ph ^= 1u;
             }
-            if (g_elect_one()) p_tc_commit2(tmem_full);
+            if (item.mt > 1) {
+                if (!tc_wait(acc_empty + 8, e_ph[1], dead)) goto done;
+                e_ph[1] ^= 1u;
+                g_tc_fence_after();
+                if (g_elect_one())
+                    for (int kb = 0; kb < head; ++kb) {
+                        const int at = (s0 + kb) % P_STAGES;
+                        products(at, 1, kb);
+                        p_tc_commit2(empty + 8 * at);  // both CTAs may refill the stage once these MMAs have read it
+                    }
+                __syncwarp();
+            }
+            for (int kb = head; kb < num_kb; ++kb) {
+                if (!tc_wait(full + 8 * s, ph, dead)) goto done;
+                P_TRC(0, kb, 0);
+                P_TRC(0, kb, 1);
+                g_tc_fence_after();
+                if (g_elect_one()) {
+                    products(s, 0, kb);
+                    if (kb == num_kb - 1) p_tc_commit2(acc_full);
+                    if (item.mt > 1) products(s, 1, kb);
+                    p_tc_commit2(empty + 8 * s);
+                }
+                __syncwarp();
+                P_TRC(0, kb, 2);
+                if (++s == P_STAGES) s = 0, ph ^= 1u;
+            }
+            if (g_elect_one()) {
+                if (head == num_kb) p_tc_commit2(acc_full);
+                if (item.mt > 1) p_tc_commit2(acc_full + 8);
+            }
             __syncwarp();
-        } else {
-            // ------------------------------------------------ peer: tell the leader when this CTA's tiles of a stage are complete
-            for (int kb = 0; kb < num_kb; ++kb) {
-                g_mbar_wait(full + 8 * s, ph);
-                if (lane == 0) p_mbar_arrive_remote(full + 8 * s, 0);
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------ peer: tell the leader when this CTA's tiles of a stage are complete
+        int s = 0;
+        uint32_t ph = 0;
+        for (int it = unit; it < plan.items; it += units)
+            for (int kb = 0; pair_item(plan, it).mt > 0 && kb < num_kb; ++kb) {
+                if (!tc_wait(full + 8 * s, ph, dead)) goto done;
+                if (lane == 0) p_mbar_arrive_leader(full + 8 * s);
                 __syncwarp();
                 if (++s == P_STAGES) s = 0, ph ^= 1u;
             }
-        }
-    } else if (warp >= 4) {
-        // ------------------------------------------------ dequantisers: this CTA's 128 features, thread = (row, 32-element half)
+    } else if (warp >= 4 && warp < 4 + P_DEQ_WARPS) {
+        // ------------------------------------------------ dequantisers: this CTA's 128 weight rows, thread = (row, 32-element half)
         const int dt = threadIdx.x - 128;
         const int row = dt >> 1, half = dt & 1;  // adjacent lanes = the two 16-byte halves of one weight row
-        const int n = min(n_pair * 256 + static_cast<int>(rank) * P_FEAT + row, K - 1);
-        const uint32_t *wrow = b + static_cast<size_t>(n) * (N / 8);
-        const T *srow = scales + static_cast<size_t>(n) * G;
-        const T *crow = biases + static_cast<size_t>(n) * G;
+        const PairWeights<T> &w = GATED && rank ? w1 : w0;
         using V2 = typename PDeq<T>::V2;
         const uint32_t magic = PDeq<T>::MAGIC;
         const V2 offset2 = *reinterpret_cast<const V2 *>(&magic);
-        uint4 packed = *reinterpret_cast<const uint4 *>(wrow + half * 4);
-        T sc_next = srow[0], bi_next = crow[0];
+        auto first_row = [&](int it) { return min(pair_item(plan, it).n_tile * FEATURES + (GATED ? 0 : rank * P_ROWS) + row, K - 1); };
+        auto next_item = [&](int it) {
+            do it += units;
+            while (it < plan.items && pair_item(plan, it).mt == 0);
+            return it;
+        };
         int s = 0;
         uint32_t ph = 1;
-        for (int kb = 0; kb < num_kb; ++kb) {
-            if (warp == 4) P_TRC(1, kb, 0);
-            const uint4 cur = packed;
-            const T sc = sc_next, bi = bi_next;
-            if (kb + 1 < num_kb) {  // next block's words and (every other block) the next group's scale pair: one round trip ahead
-                packed = *reinterpret_cast<const uint4 *>(wrow + (kb + 1) * 8 + half * 4);
-                sc_next = srow[(kb + 1) >> 1], bi_next = crow[(kb + 1) >> 1];
+        int it = next_item(unit - units), n = it < plan.items ? first_row(it) : 0, g = 0;  // the group that is fetched next
+        uint4 next[2];
+        T next_sc, next_bi;
+        auto fetch = [&]() {  // a quantisation group, two blocks, ahead of its use
+            const uint32_t *at = w.b + static_cast<size_t>(n) * (N / 8) + g * 16 + half * 4;
+            next[0] = *reinterpret_cast<const uint4 *>(at), next[1] = *reinterpret_cast<const uint4 *>(at + 8);
+            next_sc = w.scales[static_cast<size_t>(n) * G + g], next_bi = w.biases[static_cast<size_t>(n) * G + g];
+            if (++g == G) {
+                g = 0, it = next_item(it);
+                if (it < plan.items) n = first_row(it);
             }
-            V2 s2, b2;
-            s2.x = sc, s2.y = sc, b2.x = bi, b2.y = bi;
-            uint32_t outw[16];
-            const uint32_t wv[4] = {cur.x, cur.y, cur.z, cur.w};
+        };
+        if (it < plan.items) fetch();
+        for (int mine = next_item(unit - units); mine < plan.items; mine = next_item(mine))
+            for (int group = 0; group < G; ++group) {
+                const uint4 cur[2] = {next[0], next[1]};
+                V2 s2, b2;
+                s2.x = s2.y = next_sc, b2.x = b2.y = next_bi;
+                if (it < plan.items) fetch();
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                uint32_t p[4];
+                for (int u = 0; u < 2; ++u) {
+                    uint32_t outw[16];
+                    const uint32_t wv[4] = {cur[u].x, cur[u].y, cur[u].z, cur[u].w};
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    uint32_t bits;  // (128 + q_i, 128 + q_{i+4}) in one LOP3
-                    asm("lop3.b32 %0, %1, 0x000F000F, %2, 0xEA;" : "=r"(bits) : "r"(wv[j] >> (4 * i)), "r"(magic));
-                    V2 q = __hsub2(*reinterpret_cast<V2 *>(&bits), offset2);     // exact codes
-                    V2 v = __hfma2(q, s2, b2);                                    // q*scale+bias, one rounding
-                    p[i] = *reinterpret_cast<uint32_t *>(&v);
-                }
-                outw[4 * j + 0] = __byte_perm(p[0], p[1], 0x5410);  // (e0, e1)
-                outw[4 * j + 1] = __byte_perm(p[2], p[3], 0x5410);  // (e2, e3)
-                outw[4 * j + 2] = __byte_perm(p[0], p[1], 0x7632);  // (e4, e5)
-                outw[4 * j + 3] = __byte_perm(p[2], p[3], 0x7632);  // (e6, e7)
-            }
-            if (warp == 4) P_TRC(1, kb, 1);
-            g_mbar_wait(empty + 8 * s, ph);
-            if (warp == 4) P_TRC(1, kb, 2);
-            unsigned char *tile = psm + s * P_STAGE + P_A_STAGE + row * 128;
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t up4 = wv[j] >> 4;  // the pair of column q: code 2q beside code 2q + 1, by a permute of w and w >> 4
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int chunk = half * 4 + j;  // 16-byte chunk (8 elements) along K
-                *reinterpret_cast<uint4 *>(tile + ((chunk ^ (row & 7)) << 4)) = make_uint4(outw[4 * j], outw[4 * j + 1], outw[4 * j + 2], outw[4 * j + 3]);
-            }
-            g_fence_proxy_async();  // generic-proxy stores -> visible to the tensor cores' async proxy (of both SMs)
-            __syncwarp();
-            if (lane == 0) g_mbar_arrive(full + 8 * s);
-            if (warp == 4) P_TRC(1, kb, 3);
-            if (++s == P_STAGES) s = 0, ph ^= 1u;
-        }
-        // ---- epilogue: TMEM lane = token row of THIS CTA; warps 4-7 take features 0..127 of the pair, warps 8-11 features 128..255
-        g_mbar_wait(tmem_full, 0);
-        g_tc_fence_after();
-        const int q = warp & 3;
-        const int col_half = (warp - 4) >> 2;
-#pragma unroll 1
-        for (int i = 0; i < P_MT; ++i) {
-            const int m = (m_pair * P_MT + i) * 256 + static_cast<int>(rank) * P_TOK + q * 32 + lane;
-#pragma unroll
-            for (int cb = 0; cb < 4; ++cb) {
-                const int col0 = col_half * 128 + cb * 32;
-                uint32_t v[32];
-                g_tmem_ld32(tmem_d + (static_cast<uint32_t>(q * 32) << 16) + i * 256 + col0, v);
-                const int n0 = n_pair * 256 + col0;
-                if (m < M && n0 < K) {
-                    T *dst = out + static_cast<size_t>(m) * K + n0;
-                    const int valid = min(32, K - n0);
-                    if (vec_store && valid == 32) {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            uint4 o;
-                            o.x = pack2<T>(__uint_as_float(v[8 * j + 0]), __uint_as_float(v[8 * j + 1]));
-                            o.y = pack2<T>(__uint_as_float(v[8 * j + 2]), __uint_as_float(v[8 * j + 3]));
-                            o.z = pack2<T>(__uint_as_float(v[8 * j + 4]), __uint_as_float(v[8 * j + 5]));
-                            o.w = pack2<T>(__uint_as_float(v[8 * j + 6]), __uint_as_float(v[8 * j + 7]));
-                            *reinterpret_cast<uint4 *>(dst + 8 * j) = o;
+                        for (int q = 0; q < 4; ++q) {
+                            uint32_t bits;  // (128 + code_2q, 128 + code_2q+1) in one LOP3
+                            asm("lop3.b32 %0, %1, 0x000F000F, %2, 0xEA;" : "=r"(bits) : "r"(__byte_perm(wv[j], up4, 0x4400 + 0x1111 * q)), "r"(magic));
+                            const V2 code = __hsub2(*reinterpret_cast<V2 *>(&bits), offset2);  // exact codes
+                            const V2 v = __hfma2(code, s2, b2);                                // q*scale+bias, one rounding
+                            outw[4 * j + q] = *reinterpret_cast<const uint32_t *>(&v);
                         }
-                    } else {
-                        for (int j = 0; j < valid; ++j) dst[j] = from_f<T>(__uint_as_float(v[j]));
+                    }
+                    if (!tc_wait(empty + 8 * s, ph, dead)) goto done;
+                    unsigned char *tile = psm + s * P_STAGE + P_A_STAGE + row * 128;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int chunk = half * 4 + j;  // 16-byte chunk (8 elements) along K
+                        *reinterpret_cast<uint4 *>(tile + ((chunk ^ (row & 7)) << 4)) = make_uint4(outw[4 * j], outw[4 * j + 1], outw[4 * j + 2], outw[4 * j + 3]);
+                    }
+                    g_fence_proxy_async();  // generic-proxy stores -> visible to the tensor cores' async proxy (of both SMs)
+                    __syncwarp();
+                    if (lane == 0) g_mbar_arrive(full + 8 * s);
+                    if (++s == P_STAGES) s = 0, ph ^= 1u;
+                }
+            }
+    } else if (warp >= 4 + P_DEQ_WARPS) {
+        // ------------------------------------------------ epilogue: TMEM lane = token row of THIS CTA, a warp 32 rows of half of the columns
+        const int q = warp & 3, side = (warp - 4 - P_DEQ_WARPS) >> 2;
+        unsigned char *stage = psm + P_OUT_OFF + (warp - 4 - P_DEQ_WARPS) * P_OUT_BYTES;
+        uint32_t f_ph[P_MT] = {0, 0};
+        for (int it = unit; it < plan.items; it += units) {
+            const PairItem item = pair_item(plan, it);
+            for (int i = 0; i < item.mt; ++i) {
+                const bool ok = tc_wait(acc_full + 8 * i, f_ph[i], dead);
+                const float bad = tc_verdict(ok, dead);  // of a marked CTA this tile and all that follow are stored as NaN
+                f_ph[i] ^= 1u;
+                g_tc_fence_after();
+                const uint32_t d = tmem_d + (static_cast<uint32_t>(q * 32) << 16) + i * 256;
+                const int m0 = (item.m0 + i) * 256 + rank * P_TOK + q * 32;  // this warp's first token
+                constexpr int BOXES = GATED ? 1 : 2;                           // of 64 features
+#pragma unroll 1
+                for (int box = 0; box < BOXES; ++box) {
+                    const int col0 = (GATED ? side : side * 2 + box) * 64, n0 = item.n_tile * FEATURES + col0;
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // lane 0's store of the box before has left the staging rows
+                    __syncwarp();
+#pragma unroll
+                    for (int c = 0; c < 64; c += 16) {
+                        uint32_t v[16], u[16];
+                        p_tmem_ld16(d + col0 + c, v);
+                        if constexpr (GATED) p_tmem_ld16(d + 128 + col0 + c, u);
+                        g_tmem_ld_wait();
+                        float y[16];
+                        if constexpr (GATED) {  // both factors rounded as if they had been stored
+                            float gate[16], up[16];
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) gate[j] = to_f(from_f<T>(__uint_as_float(v[j]) * bad)), up[j] = to_f(from_f<T>(__uint_as_float(u[j])));
+                            p_gated<T>(gate, up, y);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) y[j] = __uint_as_float(v[j]) * bad;
+                        }
+                        uint32_t packed[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) packed[j] = pack2<T>(y[2 * j], y[2 * j + 1]);
+#pragma unroll
+                        for (int j = 0; j < 2; ++j)
+                            *reinterpret_cast<uint4 *>(stage + lane * 128 + (((c >> 3) + j) ^ (lane & 7)) * 16) =
+                                make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
+                    }
+                    if (box == BOXES - 1) {  // all of this accumulator's columns are read
+                        g_tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) {
+                            if (rank == 0) g_mbar_arrive(acc_empty + 8 * i);
+                            else p_mbar_arrive_leader(acc_empty + 8 * i);
+                        }
+                    }
+                    if (tma_store) {
+                        g_fence_proxy_async();
+                        __syncwarp();
+                        if (lane == 0 && m0 < M && n0 < K) {  // rows and features past the end are not written
+                            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(&tmap_out), "r"(n0), "r"(m0),
+                                         "r"(g_smem_u32(stage))
+                                         : "memory");
+                            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                        }
+                    } else {  // rows that TMA cannot address: one at a time, lanes along the features
+                        __syncwarp();
+                        for (int r = 0; r < 32 && m0 + r < M; ++r)
+                            for (int f = lane; f < 64 && n0 + f < K; f += 32)
+                                out[static_cast<size_t>(m0 + r) * K + n0 + f] = *reinterpret_cast<const T *>(stage + r * 128 + (((f >> 3) ^ (r & 7)) << 4) + (f & 7) * 2);
+                        __syncwarp();
                     }
                 }
             }
         }
+        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
+done:  // also from a role whose wait gave up
     g_tc_fence_before();
+    __syncthreads();
+    if (warp == 2) tc_settle(dead);
     p_cluster_sync();  // neither CTA frees tensor memory (or exits) while the other may still depend on it
     if (warp == 2) {
         g_tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "n"(P_TMEM_COLS) : "memory");
     }
 #if TL_TRACE
-    if (blockIdx.x == 0 && blockIdx.y == 0 && g_trace_buf != nullptr) {  // tag = 20000 + role * 1000 + block * 4 + k (as w4a16_gemm.cu)
+    if (blockIdx.x == 0 && g_trace_buf != nullptr) {  // tag = 20000 + role * 1000 + block * 4 + k (as w4a16_gemm.cu)
         for (int e = threadIdx.x; e < 2 * 40 * 4; e += P_THREADS) {
             const int role = e / 160, rest = e - role * 160;
-            if (rest / 4 < num_kb && !(role == 0 && (rest & 3) == 3)) {
+            if (rest / 4 < num_kb && role == 0 && (rest & 3) != 3) {
                 const unsigned at = atomicAdd(g_trace_n, 1u);
                 if (at < g_trace_cap) g_trace_buf[2 * at] = 20000 + role * 1000 + rest, g_trace_buf[2 * at + 1] = trc[role][rest / 4][rest & 3];
             }
@@ -335,62 +485,59 @@ static int pairs_default() {
 static int g_pairs_mode = pairs_default();
 void set_gemm_pairs(int mode) { g_pairs_mode = mode; }
 
-// Measured at M = 4096 (profiles/r02_gemm_bench.json): the pair kernel and the one-CTA kernel are within 2 % of each
-// other per CTA-second; what decides is the tail - a pair tile is 512 tokens x 256 features, so K = 2560 gives 160 CTAs
-// (1.08 waves of 148: 683 / 743 TF/s on o / down against 766 / 869), while q|k|v (384 CTAs) and gate|up (1216) fill
-// their last wave to > 85 % (896 / 965 TF/s against 891 / 950).
+static PairPlan pair_plan(int M, int K, int features, int units) {
+    PairPlan p;
+    p.n_tiles = ceil_div(K, features), p.m_tiles = ceil_div(M, 256);
+    const int tiles = p.n_tiles * ceil_div(p.m_tiles, P_MT), left = tiles % units;
+    p.full = left * P_MT <= units ? tiles - left : tiles;
+    p.items = p.full + (tiles - p.full) * P_MT;
+    return p;
+}
+
+// The pairs where their rounds of tiles cost less than the one-CTA kernel's waves, in that kernel's unit (w4a16_gemm.cu).  A round of whole tiles
+// is 1100 a block, of single ones 700; of reductions above 4096 a whole round takes 1750 (two rounds of 9728: 0.62 us a block each).  Measured over
+// 63 sizes of 300 to 4096 rows the choice is within 2 % of the better one; us, one-CTA kernel / pairs: 2560 -> 9728 300 rows 42 / 34, 2048 105 / 77,
+// 4096 211 / 140; 2560 -> 6144 300 rows 23.8 / 24.2, 700 29.8 / 33.9, 2048 70 / 51; 9728 -> 2560 700 rows 69 / 72, 3000 167 / 110, 4096 183 / 197.
 bool w4a16_gemm2_supported(int M, int N, int K, int dtype) {
     if (g_pairs_mode <= 0 || !(dtype == TL_BF16 || dtype == TL_F16) || M <= 256 || K <= 0 || N % 128 != 0) return false;
     if (g_pairs_mode >= 2) return true;
-    const long long ctas = 2LL * ceil_div(K, 256) * ceil_div(M, P_MT * 256);
-    const long long waves = (ctas + sm_count() - 1) / sm_count();
-    return M >= 1024 && ctas * 100 >= waves * sm_count() * 85;
+    const int units = sm_count() / 2;
+    const PairPlan p = pair_plan(M, K, 2 * P_ROWS, units);
+    const long long whole = ceil_div(p.full, units), single = ceil_div(p.items - p.full, units);
+    return whole * (N > 4096 ? 1750 : 1100) + single * 700 < w4a16_gemm_cost(M, N, K);
 }
 
 template <typename T>
-static int gemm2_t(const void *scales, const void *biases, const void *a, const void *b, void *out, int M, int N, int K, cudaStream_t st) {
+static int pair_map(CUtensorMap *map, const void *p, uint64_t cols, uint64_t rows, uint32_t box_rows) {
     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
     if (encode == nullptr) return fail(TL_ECUDA, "quantized_matmul: cuTensorMapEncodeTiled is unavailable");
-    if (!aligned16(a) || !aligned16(b)) return fail(TL_EINVAL, "quantized_matmul: a and b must be 16-byte aligned");
-    // tensor maps cached per (pointer, shape)
-    struct Key {
-        const void *p;
-        int M, N;
-        bool operator==(const Key &o) const { return p == o.p && M == o.M && N == o.N; }
-    };
-    struct Hash {
-        size_t operator()(const Key &k) const { return reinterpret_cast<size_t>(k.p) * 1000003u ^ (static_cast<size_t>(k.M) << 20) ^ static_cast<size_t>(k.N); }
-    };
-    static std::mutex mu;
-    static std::unordered_map<Key, CUtensorMap, Hash> cache;
-    CUtensorMap map;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        auto it = cache.find(Key{a, M, N});
-        if (it != cache.end()) {
-            map = it->second;
-        } else {
-            const cuuint64_t dims[2] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(M)};
-            const cuuint64_t strides[1] = {static_cast<cuuint64_t>(N) * 2};
-            const cuuint32_t box[2] = {P_KB, P_TOK};
-            const cuuint32_t estr[2] = {1, 1};
-            const CUtensorMapDataType dt = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-            CUresult r = encode(&map, dt, 2, const_cast<void *>(a), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-            if (r != CUDA_SUCCESS) return fail(TL_ECUDA, "quantized_matmul: cuTensorMapEncodeTiled failed (%d)", static_cast<int>(r));
-            if (cache.size() > 4096) cache.clear();
-            cache.emplace(Key{a, M, N}, map);
-        }
+    const cuuint64_t dims[2] = {cols, rows}, strides[1] = {cols * 2};
+    const cuuint32_t box[2] = {P_KB, box_rows}, estr[2] = {1, 1};
+    const CUtensorMapDataType dt = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    const CUresult r = encode(map, dt, 2, const_cast<void *>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? TL_OK : fail(TL_ECUDA, "quantized_matmul: cuTensorMapEncodeTiled failed (%d)", static_cast<int>(r));
+}
+
+template <typename T, bool GATED>
+static int gemm2_t(const PairWeights<T> &w0, const PairWeights<T> &w1, const void *a, void *out, int M, int N, int K, cudaStream_t st) {
+    if (!aligned16(a) || !aligned16(w0.b) || !aligned16(w1.b)) return fail(TL_EINVAL, "quantized_matmul: a and b must be 16-byte aligned");
+    const int tma_store = K % 8 == 0 && aligned16(out) ? 1 : 0;
+    CUtensorMap map_a, map_out;
+    if (int e = pair_map<T>(&map_a, a, N, M, P_TOK)) return e;
+    if (!tma_store) map_out = map_a;  // not used
+    else if (int e = pair_map<T>(&map_out, out, K, M, 32)) return e;
+    static PerDevice configured;
+    int device = 0;
+    cudaGetDevice(&device);
+    if (!configured(device, [] { return cudaFuncSetAttribute(w4a16_gemm2_kernel<T, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM) == cudaSuccess; })) {
+        cudaGetLastError();
+        return fail(TL_ECUDA, "quantized_matmul: cannot raise shared memory limit");
     }
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(w4a16_gemm2_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM);
-        if (e != cudaSuccess) return fail(TL_ECUDA, "quantized_matmul: cannot raise shared memory limit: %s", cudaGetErrorString(e));
-        configured = true;
-    }
-    const int vec_store = (K % 8 == 0 && aligned16(out)) ? 1 : 0;
+    const int units = sm_count() / 2;
+    const PairPlan plan = pair_plan(M, K, GATED ? P_ROWS : 2 * P_ROWS, units);
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(2 * ceil_div(K, 256), ceil_div(M, P_MT * 256));
+    cfg.gridDim = dim3(2 * (plan.items < units ? plan.items : units));
     cfg.blockDim = dim3(P_THREADS);
     cfg.dynamicSmemBytes = P_SMEM;
     cfg.stream = st;
@@ -401,19 +548,41 @@ static int gemm2_t(const void *scales, const void *biases, const void *a, const 
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, w4a16_gemm2_kernel<T>, map, static_cast<const T *>(scales), static_cast<const T *>(biases),
-                                       static_cast<const uint32_t *>(b), static_cast<T *>(out), M, N, K, vec_store);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, w4a16_gemm2_kernel<T, GATED>, map_a, map_out, w0, w1, static_cast<T *>(out), M, N, K, tma_store, plan);
     if (e != cudaSuccess) return fail(TL_ECUDA, "w4a16_gemm2: launch failed: %s", cudaGetErrorString(e));
     TL_LAUNCH_CHECK("w4a16_gemm2");
     return TL_OK;
 }
 
+template <typename T>
+static PairWeights<T> pair_weights(const void *scales, const void *biases, const void *b) {
+    return {static_cast<const T *>(scales), static_cast<const T *>(biases), static_cast<const uint32_t *>(b)};
+}
+
 int launch_w4a16_gemm2(const void *scales, const void *biases, const void *a, const void *b, void *out, int M, int N, int K, int dtype,
                        cudaStream_t st) {
     if (M == 0 || K == 0) return TL_OK;
-    if (dtype == TL_BF16) return gemm2_t<__nv_bfloat16>(scales, biases, a, b, out, M, N, K, st);
-    if (dtype == TL_F16) return gemm2_t<__half>(scales, biases, a, b, out, M, N, K, st);
+    if (dtype == TL_BF16) {
+        const auto w = pair_weights<__nv_bfloat16>(scales, biases, b);
+        return gemm2_t<__nv_bfloat16, false>(w, w, a, out, M, N, K, st);
+    }
+    if (dtype == TL_F16) {
+        const auto w = pair_weights<__half>(scales, biases, b);
+        return gemm2_t<__half, false>(w, w, a, out, M, N, K, st);
+    }
     return fail(TL_EDTYPE, "quantized_matmul: scales must be float16 or bfloat16");
 }
+
+bool launch_w4a16_gemm2_gated(const tl_packed_matrix &gate, const tl_packed_matrix &up, const void *a, void *out, int M, int N, int K, int dtype, cudaStream_t st, int *rc) {
+    if (g_pairs_mode <= 0 || M <= 128 || !(dtype == TL_BF16 || dtype == TL_F16) || N % 128 != 0) return false;
+    if (dtype == TL_BF16)
+        *rc = gemm2_t<__nv_bfloat16, true>(pair_weights<__nv_bfloat16>(gate.scales, gate.biases, gate.weight), pair_weights<__nv_bfloat16>(up.scales, up.biases, up.weight), a, out, M, N,
+                                           K, st);
+    else
+        *rc = gemm2_t<__half, true>(pair_weights<__half>(gate.scales, gate.biases, gate.weight), pair_weights<__half>(up.scales, up.biases, up.weight), a, out, M, N, K, st);
+    return true;
+}
+
+long long gemm2_gave_up() { return read_gave_up(); }
 
 }  // namespace tl
