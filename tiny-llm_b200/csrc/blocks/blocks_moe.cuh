@@ -22,8 +22,9 @@ struct MoeLists {
     int32_t *tile_expert, *sorted_pair;
 };
 
-// The most rows of a chunk: one tensor-core tile's columns, fewer where no expert can get that many (a token names an expert once).
-static inline int moe_chunk_rows(int tokens) { return std::min(256, (tokens + 15) / 16 * 16); }
+// The most rows of a chunk: one tensor-core tile's columns, fewer where no expert can get that many (a token names an expert once).  192: four
+// stages of two weight blocks and the rows fit in shared memory (blocks_moe_tc.cu).
+static inline int moe_chunk_rows(int tokens) { return std::min(192, (tokens + 15) / 16 * 16); }
 // An expert's rows make one chunk, and one more for every moe_chunk_rows of them.
 static inline long long moe_max_chunks(int tokens, int top, int experts) {
     const long long pairs = (long long)tokens * top;

@@ -1,7 +1,7 @@
 // The experts' grouped products on the 5th-generation tensor cores (bf16, fp32 accumulation): tcgen05.mma fed by TMA.
 //
 // Swapped operands: the M side of a product is the expert's WEIGHTS (128 rows of them, one tensor-memory lane each), the N side
-// the tokens that chose it, in a chunk of up to 256 rounded up to 16 - so an expert with 5 tokens pays for 16 columns and one
+// the tokens that chose it, in a chunk of up to 192 rounded up to 16 - so an expert with 5 tokens pays for 16 columns and one
 // with 190 for 192, and the same kernel serves a decoding batch (weights streamed once, bound by HBM) and a prompt portion.
 // A tile takes two 128-row blocks of weights over one chunk: the gate rows and the up rows of the same 128 features (their
 // product is formed in the epilogue from two accumulators of the same lane), or 256 rows of the other products.  Two blocks per
@@ -19,8 +19,13 @@
 //               gate and up of 2048 tokens.)
 // Columns past a chunk's tokens hold zeros or stale rows: columns do not mix, and they are not stored.
 //
-// Measured (64 experts of 2048 x 1408, 6 choices a token; before: mma.sync tiles of 64 x 128): 2048 tokens gate and up 714 ->
-// 230 us, down 352 -> 105 us (675 TF/s); 16 tokens 102 -> 96 us and 85 -> 52 us, 6.0 and 5.6 TB/s of weights.
+// Measured (64 experts of 2048 x 1408, 6 choices a token): 2048 tokens gate and up 226 -> 181 us (780 TF/s; the weights alone are 113 us of HBM time),
+// down 104 us; 1024 tokens 154 -> 140 and 80 -> 74; 16 tokens 89 and 49 us, 6.5 and 5.9 TB/s of weights.  What that step changed: the epilogue without
+// branches, chunks of at most 192 rows (four stages in place of three: 203 us with 256, 208 with 128, where every weight block is
+// fetched for fewer columns), tiles dealt largest first (the slowest CTA had worked 380,000 cycles, the fastest 259,000).  Tried
+// and taken back: pairs of CTAs sharing a chunk's columns (cta_group::2; 199 and 100 us where this form then took 191 and 103, at 512 tokens 134
+// against 129), the next blocks' weights asked into L2 ahead of the copies (235 us with four blocks, 286 with sixteen: more requests
+// than HBM takes), a ring of its own for the rows (no faster).
 #include "blocks_moe.cuh"
 #include "blocks_tc.cuh"
 
@@ -46,7 +51,54 @@ struct MoeTcArgs {
     bf16 *inter;
     float *pair_out;
     int stages, stage_bytes;
+    int turning;  // 1: tiles of different sizes: dealt forth and back
 };
+
+// A warp's part of a finished tile: 32 weight rows, tokens begin .. end - 1 of the chunk that starts at row0 of the sorted list, eight
+// at a time.  Neither the activation (a template argument) nor the division has a branch, so that the eight chains overlap: with an exact division
+// and a switch an element a tile of 192 tokens took 18,000 cycles, in which the tensor cores stand still, as such a tile has all of
+// tensor memory.  (The next eight read out of tensor memory ahead: no faster, and registers spilled.)
+constexpr int kStorePairs = 8, kStoreAct = 9;  // MODE: these, or the activation of a gated pair
+template <int MODE>
+__device__ __forceinline__ void epilogue(const MoeTcArgs &a, uint32_t d0, uint32_t d1, int row0, int begin, int end, int f0, int f1, float bad) {
+    for (int col = begin; col < end; col += 8) {
+        const int here = end - col, row = row0 + col;
+        uint32_t u[8], v[8];
+        tc_ld8(d0 + col, u);
+        tc_ld8(d1 + col, v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if constexpr (MODE == kStorePairs) {
+            int pair[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) pair[i] = i < here ? a.sorted_pair[row + i] : 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                float *o = a.pair_out + (size_t)pair[i] * a.n;
+                if (i < here) {
+                    if (f0 < a.n) o[f0] = __uint_as_float(u[i]) * bad;
+                    if (f1 < a.n) o[f1] = __uint_as_float(v[i]) * bad;
+                }
+            }
+        } else {
+            bf16 *o = a.inter + (size_t)row * a.n + f0;
+            bf16 x[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float p = __uint_as_float(u[i]), q = __uint_as_float(v[i]);
+                if constexpr (MODE == kStoreAct) {
+                    auto act = [&](float z) { return a.act == 2 ? (z > 0.f ? z * z : 0.f) : act_apply(z, a.act); };
+                    x[i] = __float2bfloat16_rn(act(p) * bad);
+                    if (i < here && f1 < a.n) o[(size_t)i * a.n + 128] = __float2bfloat16_rn(act(q) * bad);
+                } else {
+                    x[i] = __float2bfloat16_rn(gated_pair_bf16<MODE>(p, q, a.limit, a.slope) * bad);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i, o += a.n)
+                if (i < here && f0 < a.n) *o = x[i];
+        }
+    }
+}
 
 __global__ void __launch_bounds__(kTcThreads, 1)
 moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant__ CUtensorMap map_w1, const __grid_constant__ CUtensorMap map_x, const MoeTcArgs a) {
@@ -78,11 +130,14 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
     const uint32_t tmem = *tmem_slot;
     const int tiles = a.counters[2] * a.m_blocks;
     const bool gated = a.epilogue == kEpiGated;
+    // Tiles come largest first (moe_sort_kernel), dealt forth and back, so that the CTAs' sums differ by little more than the smallest tile.  (Tiles of one
+    // size always forth: of 16 tokens, where weights from HBM are all there is, the way back cost 2 %.)
+    auto tile_of = [&](int turn) { return turn * (int)gridDim.x + (int)(a.turning & turn ? gridDim.x - 1 - blockIdx.x : blockIdx.x); };
 
     if (warp == 0) {  // ---- weights
         int s = 0;
         uint32_t ph = 1;
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        for (int turn = 0, tile; (tile = tile_of(turn)) < tiles; ++turn) {
             const int4 c = a.chunks[tile / a.m_blocks];
             const int mb = tile % a.m_blocks, cols = (c.z + 15) & ~15;
             const int r0 = c.x * a.n + mb * (gated ? 128 : 256), r1 = gated ? r0 : r0 + 128;
@@ -101,7 +156,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
     } else if (warp == 2) {  // ---- consecutive rows of the second operand
         int s = 0;
         uint32_t ph = 1;
-        for (int tile = blockIdx.x; !gathers && tile < tiles; tile += gridDim.x) {
+        for (int turn = 0, tile; !gathers && (tile = tile_of(turn)) < tiles; ++turn) {
             const int4 c = a.chunks[tile / a.m_blocks];
             for (int kb = 0; kb < a.k_blocks; ++kb) {
                 if (!tc_wait(empty + 8 * s, ph, dead)) goto out;
@@ -120,7 +175,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
             __syncwarp();
             if (lane == 0) g_mbar_arrive(full + 8 * stage);
         };
-        for (int tile = blockIdx.x; gathers && tile < tiles; tile += gridDim.x) {
+        for (int turn = 0, tile; gathers && (tile = tile_of(turn)) < tiles; ++turn) {
             const int4 c = a.chunks[tile / a.m_blocks];
             const int groups = (c.z + 15) >> 4;
             int src[16];
@@ -151,7 +206,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
     } else if (warp == 1) {  // ---- the products
         int s = 0, buf = 0;
         uint32_t ph = 0, acc_ph[2] = {1, 1};
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        for (int turn = 0, tile; (tile = tile_of(turn)) < tiles; ++turn) {
             const int cols = (a.chunks[tile / a.m_blocks].z + 15) & ~15;
             const bool whole = cols > 128;  // both halves of tensor memory
             if (whole) buf = 0;
@@ -189,7 +244,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
         const uint32_t lanes = static_cast<uint32_t>(quarter * 32) << 16;
         int buf = 0;
         uint32_t acc_ph[2] = {0, 0};
-        for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        for (int turn = 0, tile; (tile = tile_of(turn)) < tiles; ++turn) {
             const int4 c = a.chunks[tile / a.m_blocks];
             const int mb = tile % a.m_blocks, cols = (c.z + 15) & ~15;
             const bool whole = cols > 128;
@@ -201,37 +256,14 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
             acc_ph[buf] ^= 1u;
             g_tc_fence_after();
             const int begin = half * (cols / 2), end = min(begin + cols / 2, c.z);
-            for (int col = begin; col < end; col += 8) {
-                uint32_t u[8], v[8];
-                tc_ld8(d0 + col, u);
-                tc_ld8(d1 + col, v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                const int row = c.y + col, here = min(8, c.z - col);
-                if (a.epilogue == kEpiPairs) {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        if (i >= here) break;
-                        float *o = a.pair_out + (size_t)a.sorted_pair[row + i] * a.n;
-                        if (f0 < a.n) o[f0] = __uint_as_float(u[i]) * bad;
-                        if (f1 < a.n) o[f1] = __uint_as_float(v[i]) * bad;
-                    }
-                } else if (gated) {
-                    if (f0 < a.n) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            if (i < here)
-                                a.inter[(size_t)(row + i) * a.n + f0] = __float2bfloat16_rn(gated_pair(__uint_as_float(u[i]), __uint_as_float(v[i]), a.act, a.limit, a.slope) * bad);
-                    }
-                } else {
-                    auto act = [&](float z) { return a.act == 2 ? (z > 0.f ? z * z : 0.f) : act_apply(z, a.act); };
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        if (i >= here) break;
-                        bf16 *o = a.inter + (size_t)(row + i) * a.n;
-                        if (f0 < a.n) o[f0] = __float2bfloat16_rn(act(__uint_as_float(u[i])) * bad);
-                        if (f1 < a.n) o[f1] = __float2bfloat16_rn(act(__uint_as_float(v[i])) * bad);
-                    }
-                }
+            if (gated) {
+                if (a.act == 0) epilogue<0>(a, d0, d1, c.y, begin, end, f0, f1, bad);
+                else if (a.act == 3) epilogue<3>(a, d0, d1, c.y, begin, end, f0, f1, bad);
+                else epilogue<1>(a, d0, d1, c.y, begin, end, f0, f1, bad);
+            } else if (a.epilogue == kEpiPairs) {
+                epilogue<kStorePairs>(a, d0, d1, c.y, begin, end, f0, f1, bad);
+            } else {
+                epilogue<kStoreAct>(a, d0, d1, c.y, begin, end, f0, f1, bad);
             }
             g_tc_fence_before();
             __syncwarp();
@@ -271,6 +303,7 @@ int moe_tc_product(const MoeProduct &p, cudaStream_t st) {
     a.k_blocks = ceil_div(p.K, 64);
     a.stage_bytes = 2 * kTcBlockBytes + moe_chunk_rows(p.tokens) * 128;
     a.stages = std::min(kTcMaxStages, (227 * 1024 - kTcBars) / a.stage_bytes);
+    a.turning = moe_chunk_rows(p.tokens) > 16;
     a.m_blocks = ceil_div(p.N, a.epilogue == kEpiGated ? 128 : 256);
     // the largest that any call asks for; on every call, because the attribute belongs to the device that is current
     if (cudaFuncSetAttribute(moe_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
@@ -293,6 +326,8 @@ moe_sort_kernel(const int32_t *__restrict__ idx, int pairs, int experts, int mos
     extern __shared__ int sm[];
     int *count = sm, *start = sm + experts, *first_chunk = sm + 2 * experts;  // [experts] each
     __shared__ int carry[2], part[2][32];
+    __shared__ int size_at[16];  // chunks by their size in groups of 16 rows
+    const int sizes = most / 16;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int e = threadIdx.x; e < experts; e += kSortThreads) count[e] = 0;
     if (threadIdx.x < 2) carry[threadIdx.x] = 0;
@@ -331,19 +366,49 @@ moe_sort_kernel(const int32_t *__restrict__ idx, int pairs, int experts, int mos
         __syncthreads();
         int r_before = carry[0], c_before = carry[1];
         for (int w = 0; w < warp; ++w) r_before += part[0][w], c_before += part[1][w];
-        if (e < experts) start[e] = r_before + r - rows, first_chunk[e] = c_before + c - cut;
+        // first_chunk: by expert, or, until the chunks are ordered by size below, the size and the number of the expert's chunks
+        if (e < experts) start[e] = r_before + r - rows, first_chunk[e] = sizes == 1 ? c_before + c - cut : n > 0 ? chunk_rows(n) / 16 << 27 | cut : 0;
         __syncthreads();
         if (threadIdx.x == kSortThreads - 1) carry[0] = r_before + r, carry[1] = c_before + c;
         __syncthreads();
     }
     if (threadIdx.x == 0) out.counters[0] = carry[0] / 32, out.counters[1] = carry[0], out.counters[2] = carry[1];
+    if (sizes == 1) {
+        if (threadIdx.x == 0) size_at[0] = 0;
+    } else if (warp < sizes) {  // the largest chunks first (the products' CTAs take tiles in this order), those of one size by expert: a warp a size
+        int at = 0;
+        for (int e0 = 0; e0 < experts; e0 += 32) {
+            // an entry is written by the warp of its size alone; to the others it is of no size before and after
+            volatile int *entry = first_chunk + e0 + lane;
+            const int has = e0 + lane < experts ? *entry : 0;
+            const int cut = has >> 27 == warp + 1 ? has & ((1 << 27) - 1) : 0;
+            int c = cut;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int c1 = __shfl_up_sync(0xffffffffu, c, o);
+                if (lane >= o) c += c1;
+            }
+            if (cut) *entry = at + c - cut;
+            at += __shfl_sync(0xffffffffu, c, 31);
+        }
+        if (lane == 0) size_at[warp] = at;
+    }
+    __syncthreads();
+    if (sizes > 1) {
+        if (threadIdx.x == 0)
+            for (int i = sizes - 1, at = 0; i >= 0; --i) {
+                const int n = size_at[i];
+                size_at[i] = at, at += n;
+            }
+        __syncthreads();
+    }
     for (int e = warp; e < experts; e += kSortThreads / 32) {
         const int n = count[e], row0 = start[e], cut = chunk_count(n);
         for (int i = lane; i < (n + 31) / 32; i += 32) tile_expert[row0 / 32 + i] = e;
         if (n % 32 && lane >= n % 32) sorted_pair[row0 + n / 32 * 32 + lane] = -1;  // the last tile's rows without a pair
         for (int i = lane; i < cut; i += 32) {
             const int size = chunk_rows(n);
-            out.chunks[first_chunk[e] + i] = make_int4(e, row0 + i * size, min(size, n - i * size), 0);
+            out.chunks[size_at[size / 16 - 1] + first_chunk[e] + i] = make_int4(e, row0 + i * size, min(size, n - i * size), 0);
         }
     }
     __syncthreads();
