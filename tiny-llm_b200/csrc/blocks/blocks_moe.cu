@@ -45,26 +45,41 @@ struct __align__(W * sizeof(T)) MoePiece {
 };
 
 // A CTA routes TOK tokens, so that a row of weights is fetched once for all of them: their rows of h are staged in shared memory,
-// the warps share the experts, two or four rows of weights in flight each (a logit is one warp's dot product in a lane order fixed by the
+// the warps share the experts, ROWS rows of weights in flight each (a logit is one warp's dot product in a lane order fixed by the
 // width, whatever TOK and the launch are), then warp i picks token i's top-k.  W: entries per access (16 bytes where rows allow).
 // aux_w: one more row of weights that is no router output; aux[t] = sigmoid(aux_w . h_t) (the gate of a shared expert).
-template <typename T, int TOK, int W>
-__global__ void __launch_bounds__(TOK == 1 ? 512 : 256, TOK == 1 ? 1 : 4)
+// Eight tokens a CTA are bound by the fp32 multiply-adds (268 M for 2048 tokens and 64 rows of 2048: 7.5 us): 32 of them a weight entry unpacked, the
+// tokens' entries unpacked once, at staging, the two halves of a lane's eight entries in separate planes so that its reads meet no bank conflict (2048
+// tokens 36 -> 27 us, 1024 48 -> 19; it was four tokens a CTA, unpacked by every warp).
+template <typename T, int TOK, int ROWS, int W>
+__global__ void __launch_bounds__(TOK == 1 ? 512 : 256, TOK == 1 ? 1 : 2)
 moe_route_kernel(const T *__restrict__ h, const T *__restrict__ w, const T *__restrict__ b, int tokens, int dim, int experts, int top, int scoring,
                  const T *__restrict__ choice_bias, float weight_scale, int group_count, int group_keep, const T *__restrict__ aux_w,
                  float *__restrict__ aux, int32_t *__restrict__ idx, float *__restrict__ gate) {
     extern __shared__ __align__(16) unsigned char route_smem[];
-    T *x = reinterpret_cast<T *>(route_smem);  // [TOK][dim]
-    float *logits = reinterpret_cast<float *>(route_smem + (((size_t)TOK * dim * sizeof(T) + 15) & ~(size_t)15));
+    using X = std::conditional_t<TOK == 1, T, float>;
+    constexpr bool PLANES = sizeof(X) * W > 16;  // float entries, eight an access
+    X *x = reinterpret_cast<X *>(route_smem);  // [TOK][dim]
+    float *logits = reinterpret_cast<float *>(route_smem + (((size_t)TOK * dim * sizeof(X) + 15) & ~(size_t)15));
     const int per_token = 2 * experts + group_count;  // [TOK][..]: see below
     const int t0 = blockIdx.x * TOK, here = min(TOK, tokens - t0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     for (int d = threadIdx.x * W; d < here * dim; d += blockDim.x * W) {
-        if constexpr (W == 1) x[d] = h[(size_t)t0 * dim + d];
-        else *reinterpret_cast<uint4 *>(x + d) = *reinterpret_cast<const uint4 *>(h + (size_t)t0 * dim + d);
+        if constexpr (PLANES) {  // entries 8 i .. 8 i + 3 of a row in its first half, 8 i + 4 .. 8 i + 7 in its second
+            float v[W];
+            moe_load<W>(h + (size_t)t0 * dim + d, v);
+            float *to = x + d / dim * dim + d % dim / 2;
+            *reinterpret_cast<float4 *>(to) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4 *>(to + dim / 2) = make_float4(v[4], v[5], v[6], v[7]);
+        } else if constexpr (W == 1) {
+            x[d] = from_f<X>(to_f(h[(size_t)t0 * dim + d]));
+        } else {
+            *reinterpret_cast<uint4 *>(x + d) = *reinterpret_cast<const uint4 *>(h + (size_t)t0 * dim + d);
+        }
     }
+    if (TOK > 1)  // of tokens that are not there: read below, not used
+        for (int d = here * dim + threadIdx.x; d < TOK * dim; d += blockDim.x) x[d] = from_f<X>(0.f);
     __syncthreads();
-    constexpr int ROWS = TOK == 1 ? 4 : 2;
     const int outputs = experts + (aux_w ? 1 : 0);
     for (int e0 = warp; e0 < outputs; e0 += warps * ROWS) {
         float acc[ROWS][TOK];
@@ -72,19 +87,18 @@ moe_route_kernel(const T *__restrict__ h, const T *__restrict__ w, const T *__re
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
             const int e = e0 + r * warps;
-            row[r] = e < experts ? w + (size_t)e * dim : aux_w;  // past the last one: not read
+            // past the last one: the last, not used (a condition in the loops below would keep the rows' chains from overlapping)
+            row[r] = e < experts ? w + (size_t)e * dim : aux_w ? aux_w : w + (size_t)(experts - 1) * dim;
 #pragma unroll
             for (int i = 0; i < TOK; ++i) acc[r][i] = 0.f;
         }
-        // a few tokens: two steps of weights are on their way while one is used (16 tokens: 14 -> 11 us).  Many tokens: two rows a warp
-        // and four CTAs an SM hide the round trips better than more registers for weights do (2048 tokens, 64 x 2048 weights: four
-        // rows at one, two and four steps ahead 55, 42 and 74 us, two rows 37).
+        // steps of weights on their way while one is used (16 tokens: one 14 us, two 11; 1024 tokens, eight a CTA: one 18.5, two 20)
         constexpr int AHEAD = TOK == 1 ? 2 : 1;
         MoePiece<T, W> next[AHEAD][ROWS];
         auto fetch = [&](int d, MoePiece<T, W> (&to)[ROWS]) {
 #pragma unroll
             for (int r = 0; r < ROWS; ++r)
-                if (d < dim && e0 + r * warps < outputs) to[r] = *reinterpret_cast<const MoePiece<T, W> *>(row[r] + d);
+                if (d < dim) to[r] = *reinterpret_cast<const MoePiece<T, W> *>(row[r] + d);
         };
 #pragma unroll
         for (int u = 0; u < AHEAD; ++u) fetch((u * 32 + lane) * W, next[u]);
@@ -100,27 +114,34 @@ moe_route_kernel(const T *__restrict__ h, const T *__restrict__ w, const T *__re
 #pragma unroll
                 for (int i = 0; i < TOK; ++i) {
                     float xv[W];
-                    moe_load<W>(x + (size_t)i * dim + d, xv);
+                    if constexpr (PLANES) {
+                        const float *from = x + (size_t)i * dim + d / 2;
+                        const float4 lo = load4(from), hi = load4(from + dim / 2);
+                        xv[0] = lo.x, xv[1] = lo.y, xv[2] = lo.z, xv[3] = lo.w, xv[4] = hi.x, xv[5] = hi.y, xv[6] = hi.z, xv[7] = hi.w;
+                    } else {
+                        moe_load<W>(x + (size_t)i * dim + d, xv);
+                    }
 #pragma unroll
-                    for (int r = 0; r < ROWS; ++r)
-                        if (e0 + r * warps < outputs) {
+                    for (int j = 0; j < W; ++j)
 #pragma unroll
-                            for (int j = 0; j < W; ++j) acc[r][i] = fmaf(xv[j], wv[r][j], acc[r][i]);
-                        }
+                        for (int r = 0; r < ROWS; ++r) acc[r][i] = fmaf(xv[j], wv[r][j], acc[r][i]);
                 }
             }
         }
+        // the sums one after another, then a lane each to write them: with a bias fetched and a store made behind every sum a CTA of eight
+        // tokens waited out 64 round trips (25 us)
+        float mine = 0.f;
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            const int e = e0 + r * warps;
-            if (e >= outputs) continue;
+        for (int r = 0; r < ROWS; ++r)
 #pragma unroll
             for (int i = 0; i < TOK; ++i) {
                 const float s = warp_sum(acc[r][i]);
-                if (lane != 0 || i >= here) continue;
-                if (e < experts) logits[i * per_token + e] = s + (b ? to_f(b[e]) : 0.f);
-                else aux[t0 + i] = sigmoid(s);
+                if (lane == r * TOK + i) mine = s;
             }
+        const int e = e0 + lane / TOK * warps, i = lane % TOK;
+        if (lane < ROWS * TOK && e < outputs && i < here) {
+            if (e < experts) logits[i * per_token + e] = mine + (b ? to_f(b[e]) : 0.f);
+            else aux[t0 + i] = sigmoid(mine);
         }
     }
     __syncthreads();
@@ -342,19 +363,33 @@ int tlb_moe_route(const void *h, const void *w, const void *b, int tokens, int d
         (group_count > 0 && (experts % group_count || group_keep * (experts / group_count) < top)))
         return tl::fail(TL_EINVAL, "moe_route: bad groups or side output");
     const size_t es = dtype == TL_BF16 ? 2 : 4;
-    const auto bytes = [&](int tok) { return (((size_t)tok * dim * es + 15) & ~(size_t)15) + (size_t)tok * (2 * (size_t)experts + group_count) * sizeof(float); };
+    const auto bytes = [&](int tok) { return (((size_t)tok * dim * (tok == 1 ? es : sizeof(float)) + 15) & ~(size_t)15) + (size_t)tok * (2 * (size_t)experts + group_count) * sizeof(float); };
     if (bytes(1) > 48 * 1024) return tl::fail(TL_EINVAL, "moe_route: width %d + %d experts do not fit", dim, experts);
     const bool wide = dim * es % 16 == 0 && tl::aligned16(h) && tl::aligned16(w) && (!aux_w || tl::aligned16(aux_w));
-    // four tokens a CTA once that fills the GPU; few tokens: more warps each, so that no warp walks many rows of weights
-    const bool many = tokens >= 4 * 148 * 2 && bytes(4) <= 48 * 1024;
+    // eight tokens a CTA as long as a CTA's share of shared memory allows it; few tokens: a CTA each with more warps, so that no warp walks many rows of
+    // weights (64 x 2048: 256 tokens a CTA each 11 us, eight a CTA 18; 400 20 and 19; 1024 39 and 19; 2048 68 and 27)
+    const bool many = tokens >= 400 && bytes(8) <= 227 * 1024;
+    const bool few = experts + (aux_w ? 1 : 0) <= 16;  // two rows a warp are all there are
     const int threads = many || tokens > 148 ? 256 : 512;
-#define TLB_ROUTE(TOK, WV)                                                                                                                         \
-    moe_route_kernel<T, TOK, WV><<<ceil_div(tokens, TOK), threads, bytes(TOK), as_stream(stream)>>>(                                                \
-        (const T *)h, (const T *)w, (const T *)b, tokens, dim, experts, top, scoring, (const T *)choice_bias, weight_scale, group_count, group_keep, \
-        (const T *)aux_w, aux, idx, gate)
+    const auto ready = [&](auto kernel, int tok) -> int {
+        // on every call, because the attribute belongs to the device that is current
+        if (bytes(tok) > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
+            cudaGetLastError();
+            return tl::fail(TL_ECUDA, "moe_route: no shared memory");
+        }
+        return TL_OK;
+    };
+#define TLB_ROUTE(TOK, ROWS, WV)                                                                                                                         \
+    do {                                                                                                                                            \
+        if (int e = ready(moe_route_kernel<T, TOK, ROWS, WV>, TOK)) return e;                                                                             \
+        moe_route_kernel<T, TOK, ROWS, WV><<<ceil_div(tokens, TOK), threads, bytes(TOK), as_stream(stream)>>>(                                            \
+            (const T *)h, (const T *)w, (const T *)b, tokens, dim, experts, top, scoring, (const T *)choice_bias, weight_scale, group_count,         \
+            group_keep, (const T *)aux_w, aux, idx, gate);                                                                                           \
+    } while (0)
     TLB_DISPATCH(dtype, "moe_route",
-                 if (wide) { if (many) TLB_ROUTE(4, (16 / (int)sizeof(T))); else TLB_ROUTE(1, (16 / (int)sizeof(T))); }
-                 else { if (many) TLB_ROUTE(4, 1); else TLB_ROUTE(1, 1); });
+                 if (wide && many) { if (few) TLB_ROUTE(8, 2, (16 / (int)sizeof(T))); else TLB_ROUTE(8, 4, (16 / (int)sizeof(T))); }
+                 else if (wide) TLB_ROUTE(1, 4, (16 / (int)sizeof(T)));
+                 else { if (many) TLB_ROUTE(8, 4, 1); else TLB_ROUTE(1, 4, 1); });
 #undef TLB_ROUTE
     TL_LAUNCH_CHECK("moe_route");
     return TL_OK;
