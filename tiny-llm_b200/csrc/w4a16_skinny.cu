@@ -468,49 +468,50 @@ __global__ void __launch_bounds__(256) w4a16_skinny_reduce_kernel(const float *p
 }
 
 // The same reduction for the residual epilogue when the RMSNorm of the NEXT projection follows (o -> post-attention norm,
-// down -> next layer's input norm): one CTA per token row adds the planes, adds the residual, writes the residual
-// stream and - the row being complete in its registers - the normalised row too (week2_kernels.metal:41-47 arithmetic:
-// T(x * rsqrt(mean(x^2) + eps) * w) on the ROUNDED residual sum).  Saves the rms_norm launch and its read of the row.
-constexpr int SK_NORM_PER = 16;  // elements per thread: K <= 4096
+// down -> next layer's input norm): a cluster of SK_NORM_CTAS CTAs per token row adds the planes, adds the residual, writes the residual
+// stream and - the row being complete in the cluster's registers - the normalised row too (week2_kernels.metal:41-47 arithmetic:
+// T(x * rsqrt(mean(x^2) + eps) * w) on the ROUNDED residual sum).  Saves the rms_norm launch and its read of the row.  The CTAs take neighbouring
+// quarters of the row and hand each other their sums of squares through shared memory, which are added in rank order.  What bounds it is round trips:
+// with one CTA a row each thread waited for ceil(splits / 4) of them, now for ceil(splits / 8), and a decoding batch's rows fill the chip.
+constexpr int SK_NORM_CTAS = 4, SK_NORM_PER = 4;  // elements per thread: K <= 4096
 template <typename T>
-__global__ void __launch_bounds__(256) w4a16_skinny_reduce_norm_kernel(const float *part, const T *res, const T *__restrict__ norm_w, T *out, T *normed,
-                                                                       int M, int K, int splits, float eps) {
-    __shared__ float warp_part[8];
+__global__ void __launch_bounds__(256) __cluster_dims__(SK_NORM_CTAS, 1, 1)
+w4a16_skinny_reduce_norm_kernel(const float *part, const T *res, const T *__restrict__ norm_w, T *out, T *normed, int M, int K, int splits, float eps) {
+    __shared__ float warp_part[8], rank_part[SK_NORM_CTAS];
     griddep_launch();
+    const int rank = blockIdx.x % SK_NORM_CTAS, quarter = (K + SK_NORM_CTAS - 1) / SK_NORM_CTAS, first = rank * quarter, last = min(first + quarter, K);
+    const size_t plane = static_cast<size_t>(M) * K, row = static_cast<size_t>(blockIdx.x / SK_NORM_CTAS) * K;
     griddep_wait();
-    const size_t plane = static_cast<size_t>(M) * K, row = static_cast<size_t>(blockIdx.x) * K;
-    // all loads of a round (four planes x the thread's elements, then the residual) are issued before the first is used:
+    // all loads of a round (eight planes x the thread's elements, the residual beside the first) are issued before the first is used:
     // ld_cg is a volatile asm, so a load-then-add loop per element would pay one L2 round trip per batch (measured: 14 us
     // for this kernel against 3 + 2 us for the two it replaces)
     float xs[SK_NORM_PER];
-#pragma unroll
-    for (int j = 0; j < SK_NORM_PER; ++j) xs[j] = 0.f;
-    for (int sp0 = 0; sp0 < splits; sp0 += 4) {
-        float v[SK_NORM_PER][4];
-#pragma unroll
-        for (int j = 0; j < SK_NORM_PER; ++j) {
-            const int n = threadIdx.x + j * 256;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) v[j][q] = (n < K && sp0 + q < splits) ? ld_cg(part + (sp0 + q) * plane + row + n) : 0.f;
-        }
-#pragma unroll
-        for (int j = 0; j < SK_NORM_PER; ++j) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (sp0 + q < splits) xs[j] += v[j][q];  // split order
-        }
-    }
-    T rs[SK_NORM_PER];
+    T rs[SK_NORM_PER], weight[SK_NORM_PER];
 #pragma unroll
     for (int j = 0; j < SK_NORM_PER; ++j) {
-        const int n = threadIdx.x + j * 256;
-        rs[j] = n < K ? ld_cg(res + row + n) : from_f<T>(0.f);
+        const int n = first + threadIdx.x + j * 256;
+        xs[j] = 0.f, rs[j] = n < last ? ld_cg(res + row + n) : from_f<T>(0.f), weight[j] = n < last ? norm_w[n] : from_f<T>(0.f);
+    }
+    for (int sp0 = 0; sp0 < splits; sp0 += 8) {
+        float v[SK_NORM_PER][8];
+#pragma unroll
+        for (int j = 0; j < SK_NORM_PER; ++j) {
+            const int n = first + threadIdx.x + j * 256;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[j][q] = (n < last && sp0 + q < splits) ? ld_cg(part + (sp0 + q) * plane + row + n) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < SK_NORM_PER; ++j) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (sp0 + q < splits) xs[j] += v[j][q];  // split order
+        }
     }
     float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < SK_NORM_PER; ++j) {
-        const int n = threadIdx.x + j * 256;
-        if (n < K) {
+        const int n = first + threadIdx.x + j * 256;
+        if (n < last) {
             const T vb = from_f<T>(to_f(rs[j]) + to_f(from_f<T>(xs[j])));
             out[row + n] = vb;
             xs[j] = to_f(vb);
@@ -520,12 +521,22 @@ __global__ void __launch_bounds__(256) w4a16_skinny_reduce_norm_kernel(const flo
     ss = warp_sum(ss);
     if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = ss;
     __syncthreads();
-    ss = warp_sum((threadIdx.x & 31) < 8 ? warp_part[threadIdx.x & 31] : 0.f);
+    if (threadIdx.x < 32) {
+        ss = warp_sum(threadIdx.x < 8 ? warp_part[threadIdx.x] : 0.f);
+        if (threadIdx.x < SK_NORM_CTAS)  // into rank_part[rank] of CTA `threadIdx.x`
+            asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.f32 [ra], %2;\n\t}" ::"r"(g_smem_u32(rank_part + rank)), "r"(threadIdx.x),
+                         "f"(ss)
+                         : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < SK_NORM_CTAS; ++i) ss += rank_part[i];
     const float inv = rsqrtf(ss / static_cast<float>(K) + eps);
 #pragma unroll
     for (int j = 0; j < SK_NORM_PER; ++j) {
-        const int n = threadIdx.x + j * 256;
-        if (n < K) normed[row + n] = from_f<T>(xs[j] * inv * to_f(norm_w[n]));
+        const int n = first + threadIdx.x + j * 256;
+        if (n < last) normed[row + n] = from_f<T>(xs[j] * inv * to_f(weight[j]));
     }
 }
 
@@ -666,8 +677,8 @@ static int skinny_t(const void *scales, const void *biases, const void *a, const
     if (rc == TL_OK && args.splits == 1 && epilogue == SK_EPI_GATED)  // the kernel's own epilogue has no activation
         return launch_swiglu(residual, out, out, static_cast<long long>(M) * K, std::is_same<T, __nv_bfloat16>::value ? TL_BF16 : TL_F16, st);
     if (rc != TL_OK || args.splits == 1) return rc;
-    if (normed != nullptr && epilogue == SK_EPI_RESIDUAL && K <= 256 * SK_NORM_PER) {
-        cudaError_t e = launch_chained(w4a16_skinny_reduce_norm_kernel<T>, dim3(M), dim3(256), 0, st, static_cast<const float *>(args.partials),
+    if (normed != nullptr && epilogue == SK_EPI_RESIDUAL && K <= 256 * SK_NORM_PER * SK_NORM_CTAS) {
+        cudaError_t e = launch_chained(w4a16_skinny_reduce_norm_kernel<T>, dim3(M * SK_NORM_CTAS), dim3(256), 0, st, static_cast<const float *>(args.partials),
                                        static_cast<const T *>(residual), static_cast<const T *>(norm_w), static_cast<T *>(out), static_cast<T *>(normed),
                                        M, K, args.splits, norm_eps);
         if (e != cudaSuccess) return fail(TL_ECUDA, "w4a16_skinny_reduce_norm: launch failed: %s", cudaGetErrorString(e));
