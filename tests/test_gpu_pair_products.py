@@ -44,3 +44,45 @@ def test_gates_outside_the_fast_division(M):
     want = ext.swiglu(quantized_linear(x, gate), quantized_linear(x, up))
     got = ext.quantized_gate_up(x, part(gate), part(up), (True, True), (True, True))
     assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(), want.nan_to_num())
+
+
+def unpacked(w):
+    """The weights as the kernels see them: code x scale + bias in fp32, rounded to the storage type."""
+    words = w.weight
+    codes = ((words.unsqueeze(-1) >> torch.arange(0, 32, 4, device="cuda", dtype=torch.int32)) & 15).reshape(words.shape[0], -1, 128).float()
+    return (codes * w.scales.float()[..., None] + w.biases.float()[..., None]).to(w.scales.dtype).reshape(words.shape[0], -1)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(129, 9728, 2560), (256, 4096, 1000), (257, 3072, 1028), (300, 9728, 264), (512, 6144, 2048), (700, 9728, 1004), (1024, 6144, 512), (300, 9728, 1001)])
+def test_reductions_in_runs(M, N, K, dtype):
+    """Planes of ragged sizes against 64 bits, no further off than the product in one run, the same bits every time.  1001 columns: not cut."""
+    w = weight(K, N, dtype, M)
+    x = torch.randn(M, N, generator=torch.Generator(device="cuda").manual_seed(K), device="cuda").to(dtype)
+    want = x.double() @ unpacked(w).double().t()
+    code = {torch.float16: 1, torch.bfloat16: 2}[dtype]
+    assert (ext._lib.tl_quantized_matmul_workspace(M, N, K, code, 1, 1) > 0) == (K % 4 == 0)
+    got = quantized_linear(x, w)
+    assert torch.equal(quantized_linear(x, w), got)
+    try:
+        ext.set_gemm_pairs(0)
+        whole = quantized_linear(x, w)
+    finally:
+        ext.set_gemm_pairs(1)
+    error = lambda y: float((y.double() - want).norm() / want.norm())  # noqa: E731
+    # the output's rounding is 2^-9 (2^-12) an entry at most, 0.4 of that in the mean; what the sums leave is a hundredth of it
+    assert error(got) <= 1.01 * error(whole) and error(got) < (2.0**-9 if dtype == torch.bfloat16 else 2.0**-12)
+
+
+def test_runs_on_two_streams_do_not_share_planes():
+    w = weight(2560, 9728, torch.bfloat16, 1)
+    xs = [torch.randn(m, 9728, device="cuda").bfloat16() for m in (140, 300)]
+    want = [quantized_linear(x, w) for x in xs]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in xs], [[], []]
+    for _ in range(20):
+        for i, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                got[i].append(quantized_linear(xs[i], w))
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[i]) for i in range(2) for y in got[i])
