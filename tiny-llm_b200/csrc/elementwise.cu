@@ -716,10 +716,35 @@ __global__ void __launch_bounds__(QKN_WARPS * 32) decode_qk_norm_rope_append_d12
     int bt_stride, long long q_row_stride, long long q_head_stride) {
     constexpr int D = 128, half = 64;
     griddep_launch();
-    griddep_wait();  // qkv is the previous kernel's output: read through L2 (common.cuh: programmatic dependent launch)
     const int b = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int heads = Hq + 2 * Hkv;
+    // Positions, lengths and block tables are step inputs uploaded before the chain: the angles and the row's place in the cache are worked out
+    // under the projection (behind its planes' sums they were on the chain, 0.8 us of it a layer).
+    // the 64 (sin, cos) pairs of this row's position: computed ONCE per CTA by its first two warps (one pair index per
+    // thread: a double-precision exp2 and a large-argument sincosf each) and shared; every lane doing its own kept the
+    // FP64 / slow-path trig pipes busy 16x over
+    __shared__ float sn_s[half], cs_s[half];
+    if (threadIdx.x < half) {
+        const int i = threadIdx.x;
+        const double inv_freq = exp2(-static_cast<double>(i) / static_cast<double>(half) * log2(static_cast<double>(base)));
+        const float angle = static_cast<float>(static_cast<double>(offsets[b]) * inv_freq);
+        sincosf(angle, &sn_s[i], &cs_s[i]);
+    }
+    // page slot of this row's token (k / v heads)
+    const int ctx = cl[b];
+    T *k_dst = nullptr, *v_dst = nullptr;
+    if (ctx > 0) {
+        const int tok = ctx - 1, lp = tok / page_size;
+        if (lp < max_pages) {
+            const int pid = bt[static_cast<size_t>(b) * bt_stride + lp];
+            if (pid >= 0 && pid < num_pages) {
+                const size_t slot = (static_cast<size_t>(pid) * Hkv * page_size + (tok - lp * page_size)) * D;
+                k_dst = kp + slot, v_dst = vp + slot;
+            }
+        }
+    }
+    griddep_wait();  // qkv is the previous kernel's output: read through L2 (common.cuh: programmatic dependent launch)
     float re[QKN_MAXH][2], im[QKN_MAXH][2];
     if constexpr (PLANES) {
         const float *prow = part + static_cast<size_t>(b) * heads * D;
@@ -762,33 +787,10 @@ __global__ void __launch_bounds__(QKN_WARPS * 32) decode_qk_norm_rope_append_d12
             }
         }
     }
-    // the 64 (sin, cos) pairs of this row's position: computed ONCE per CTA by its first two warps (one pair index per
-    // thread: a double-precision exp2 and a large-argument sincosf each) and shared; every lane doing its own kept the
-    // FP64 / slow-path trig pipes busy 16x over
-    __shared__ float sn_s[half], cs_s[half];
-    if (threadIdx.x < half) {
-        const int i = threadIdx.x;
-        const double inv_freq = exp2(-static_cast<double>(i) / static_cast<double>(half) * log2(static_cast<double>(base)));
-        const float angle = static_cast<float>(static_cast<double>(offsets[b]) * inv_freq);
-        sincosf(angle, &sn_s[i], &cs_s[i]);
-    }
     __syncthreads();
     float sn[2], cs[2];
 #pragma unroll
     for (int j = 0; j < 2; ++j) sn[j] = sn_s[lane + 32 * j], cs[j] = cs_s[lane + 32 * j];
-    // page slot of this row's token (k / v heads)
-    const int ctx = cl[b];
-    T *k_dst = nullptr, *v_dst = nullptr;
-    if (ctx > 0) {
-        const int tok = ctx - 1, lp = tok / page_size;
-        if (lp < max_pages) {
-            const int pid = bt[static_cast<size_t>(b) * bt_stride + lp];
-            if (pid >= 0 && pid < num_pages) {
-                const size_t slot = (static_cast<size_t>(pid) * Hkv * page_size + (tok - lp * page_size)) * D;
-                k_dst = kp + slot, v_dst = vp + slot;
-            }
-        }
-    }
 #pragma unroll
     for (int hh = 0; hh < QKN_MAXH; ++hh) {
         const int head = warp + QKN_WARPS * hh;
