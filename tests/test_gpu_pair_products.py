@@ -86,3 +86,22 @@ def test_runs_on_two_streams_do_not_share_planes():
                 got[i].append(quantized_linear(xs[i], w))
     torch.cuda.synchronize()
     assert all(torch.equal(y, want[i]) for i in range(2) for y in got[i])
+
+
+def test_without_memory_for_planes_the_reduction_stays_whole(monkeypatch):
+    w = weight(2560, 9728, torch.bfloat16, 1)
+    x = torch.randn(300, 9728, device="cuda").bfloat16()
+    try:
+        ext.set_gemm_pairs(0)
+        want = quantized_linear(x, w)
+    finally:
+        ext.set_gemm_pairs(1)
+
+    def empty(*args, **kwargs):
+        raise torch.OutOfMemoryError
+
+    monkeypatch.setattr(ext.torch, "empty", empty)
+    got = quantized_linear(x, w)
+    monkeypatch.undo()
+    # whole reductions have the same bits on either kernel
+    assert torch.equal(got, want)

@@ -182,10 +182,14 @@ def _workspace(nbytes: int, device) -> torch.Tensor | None:
 
 def _planes(nbytes: int, rows: int, device, stream) -> torch.Tensor | None:
     """The fp32 planes of a product whose reduction is split: above 128 rows the call's own memory, so that products on several streams
-    do not share it; up to 128 rows, where a step's captured launches need one address, the device's persistent buffer."""
+    do not share it; up to 128 rows, where a step's captured launches need one address, the device's persistent buffer.  None: there is
+    no memory for them, and the reduction stays whole."""
     if nbytes == 0 or rows <= 128:
         return _zero_workspace(nbytes, device)
-    ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    try:
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return None
     if stream is not None:  # freed on return, while that stream may still have to read it
         ws.record_stream(stream)
     return ws
