@@ -51,26 +51,26 @@ constexpr int SK_GROUP_WARPS = 4;   // dequantiser warps per group block (two gr
 constexpr int SK_THREADS = 128 + SK_DEQ_THREADS;
 enum { SK_EPI_NONE = 0, SK_EPI_RESIDUAL = 1, SK_EPI_SWIGLU_PAIRS = 2, SK_EPI_GATED = 3 };
 
-// Shared memory: activation ring (BSTAGES group blocks of two [NT x 64] tiles) + packed-weight ring (PSTAGES boxes) +
-// barriers.  Tensor memory: D[feature, token] in the first D_COLS columns, then ASTAGES dequantised tiles of 64
+// Shared memory: activation ring (STAGES group blocks of two [NT x 64] tiles) + packed-weight ring (PSTAGES boxes) +
+// barriers.  Tensor memory: D[feature, token] in the first D_COLS columns, then STAGES dequantised tiles of 64
 // columns (128 reduction elements as bf16 pairs, lane = feature row).
-// WIDE1 (NT = 128 only): the one-CTA-per-SM geometry of 128 token columns (deeper rings, six tile stages in all 512
-// TMEM columns); the default packs two CTAs per SM there too (two activation stages, two tile stages): the dequantiser
+// WIDE1 (NT = 128 only): the one-CTA-per-SM geometry of 128 token columns (three stages, 320 columns, for which 512 are
+// allocated); the default packs two CTAs per SM there too (two stages): the dequantiser
 // throughput of an SM is what bounds this kernel, and one CTA has half the warps.
 template <int NT, bool WIDE1 = false>
 struct SkSmem {
     static constexpr int B_BYTES = NT * SK_KB * 2;                 // one [NT x 64] activation tile
-    static constexpr int BSTAGES = NT >= 128 ? (WIDE1 ? 3 : 2) : (NT >= 64 ? 3 : 4);  // group blocks in flight (L2 round trip ~1 us)
-    static constexpr int PSTAGES = NT >= 128 && WIDE1 ? 4 : 3;     // packed boxes in flight (two group blocks each)
-    static constexpr int B_OFF = 0;
-    static constexpr int P_OFF = B_OFF + BSTAGES * 2 * B_BYTES;
-    static constexpr int BAR_OFF = P_OFF + PSTAGES * SK_PACKED_BYTES;
-    static constexpr int BYTES = BAR_OFF + 512;
     static constexpr int D_COLS = NT < 32 ? 32 : NT;               // accumulator columns (fp32)
     static constexpr int TMEM_COLS = NT >= 128 && WIDE1 ? 512 : 256;  // two CTAs per SM share the 512 columns
+    // group blocks in flight, of activations in shared memory and of dequantised weights in tensor memory alike: 3 (NT <= 64 and WIDE1) or 2 (NT = 128)
+    static constexpr int STAGES = (TMEM_COLS - D_COLS) / 64 < 3 ? (TMEM_COLS - D_COLS) / 64 : 3;
+    static constexpr int PSTAGES = NT >= 128 && WIDE1 ? 4 : 3;     // packed boxes in flight (two group blocks each)
+    static constexpr int B_OFF = 0;
+    static constexpr int P_OFF = B_OFF + STAGES * 2 * B_BYTES;
+    static constexpr int BAR_OFF = P_OFF + PSTAGES * SK_PACKED_BYTES;
+    static constexpr int BYTES = BAR_OFF + 512;
     static constexpr int CTAS_PER_SM = NT >= 128 && WIDE1 ? 1 : 2;
-    static constexpr int ASTAGES = (TMEM_COLS - D_COLS) / 64;      // 3 (NT <= 64) or 6 (NT = 128)
-    static_assert(BYTES <= 227 * 1024 && ASTAGES >= 2, "budget");
+    static_assert(BYTES <= 227 * 1024 && STAGES >= 2, "budget");
 };
 
 struct SkArgs {
@@ -110,9 +110,8 @@ template <typename T, int NT, bool WIDE1, bool DUAL>
 __global__ void __launch_bounds__(SK_THREADS, SkSmem<NT, WIDE1>::CTAS_PER_SM)
 w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_gate, const __grid_constant__ CUtensorMap tmap_up, const SkArgs args) {
     using Smem = SkSmem<NT, WIDE1>;
-    constexpr int ASTAGES = Smem::ASTAGES;
+    constexpr int STAGES = Smem::STAGES;
     constexpr int PSTAGES = Smem::PSTAGES;
-    constexpr int BSTAGES = Smem::BSTAGES;
     extern __shared__ __align__(1024) unsigned char ssm[];
 #if TL_TRACE
     // per-block cycle stamps of CTA 0 (tools/skinny_blocks.py): role 0 = MMA warp (k: A tile ready, B tiles ready, MMAs
@@ -142,22 +141,22 @@ w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 
     const uint32_t b_base = g_smem_u32(ssm + Smem::B_OFF), p_base = g_smem_u32(ssm + Smem::P_OFF);
     const uint32_t bar = g_smem_u32(ssm + Smem::BAR_OFF);
-    const uint32_t full_a = bar, empty = bar + 8 * ASTAGES, p_full = bar + 16 * ASTAGES, p_empty = p_full + 8 * PSTAGES;
-    const uint32_t full_b = p_empty + 8 * PSTAGES, b_empty = full_b + 8 * BSTAGES, tmem_full = b_empty + 8 * BSTAGES;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(ssm + Smem::BAR_OFF + 16 * ASTAGES + 16 * PSTAGES + 16 * BSTAGES + 8);
+    // ONE "full" barrier (the dequantiser group's warps and the activations' TMA) and ONE "empty" barrier a stage: a wait or a commit costs the MMA warp
+    // 100 to 200 cycles beside the dequantisers of its scheduler, and a block takes 900 cycles by the cycle trace, 260 of them the MMAs'.  Against a
+    // barrier of each kind for weights and activations: feed-forward of 24 rows (2560 -> 9728) 28.9 -> 28.4 us, of 52 rows 32.3 -> 31.6, of 52 rows of
+    // 1024 -> 3072 26.6 -> 25.3; 16 steps of 24 requests 11.38 -> 11.24 ms.
+    const uint32_t full = bar, empty = bar + 8 * STAGES, p_full = bar + 16 * STAGES, p_empty = p_full + 8 * PSTAGES;
+    const uint32_t tmem_full = p_empty + 8 * PSTAGES;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(ssm + Smem::BAR_OFF + 16 * STAGES + 16 * PSTAGES + 8);
 
     if (warp == 0 && lane == 0) {
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
     }
     if (warp == 1 && lane == 0) {
-        for (int i = 0; i < ASTAGES; ++i) {
-            g_mbar_init(full_a + 8 * i, SK_GROUP_WARPS);  // one arrival per warp of the dequantiser group that owns the block
+        for (int i = 0; i < STAGES; ++i) {
+            g_mbar_init(full + 8 * i, SK_GROUP_WARPS + 1);  // one arrival per warp of the dequantiser group that owns the block, and the activations
             g_mbar_init(empty + 8 * i, 1);
-        }
-        for (int i = 0; i < BSTAGES; ++i) {
-            g_mbar_init(full_b + 8 * i, 1);
-            g_mbar_init(b_empty + 8 * i, 1);
         }
         for (int i = 0; i < PSTAGES; ++i) {
             g_mbar_init(p_full + 8 * i, 1);
@@ -196,14 +195,14 @@ w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         int bs = 0;
         uint32_t ph = 1;
         for (int i = 0; i < n_gb; ++i) {
-            g_mbar_wait(b_empty + 8 * bs, ph);
+            g_mbar_wait(empty + 8 * bs, ph);
             if (g_elect_one()) {
-                g_mbar_expect_tx(full_b + 8 * bs, 2 * Smem::B_BYTES);
-                g_tma_load_2d(b_base + (2 * bs) * Smem::B_BYTES, &tmap_a, (gb0 + i) * SK_GB, 0, full_b + 8 * bs);
-                g_tma_load_2d(b_base + (2 * bs + 1) * Smem::B_BYTES, &tmap_a, (gb0 + i) * SK_GB + SK_KB, 0, full_b + 8 * bs);
+                g_mbar_expect_tx(full + 8 * bs, 2 * Smem::B_BYTES);
+                g_tma_load_2d(b_base + (2 * bs) * Smem::B_BYTES, &tmap_a, (gb0 + i) * SK_GB, 0, full + 8 * bs);
+                g_tma_load_2d(b_base + (2 * bs + 1) * Smem::B_BYTES, &tmap_a, (gb0 + i) * SK_GB + SK_KB, 0, full + 8 * bs);
             }
             __syncwarp();
-            if (++bs == BSTAGES) bs = 0, ph ^= 1u;
+            if (++bs == STAGES) bs = 0, ph ^= 1u;
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer: D[feature, token] += W_block . A_block^T, 8 K-steps per group block
@@ -211,27 +210,24 @@ w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         // uniform registers, no division per block), one elected lane issues.
         constexpr uint32_t idesc = sk_instr_desc<T, NT>();
         const uint64_t bdesc0 = g_smem_desc_sw128(b_base, 0, 1024);
-        int s = 0, bs = 0;
-        uint32_t pha = 0, phb = 0;
+        int s = 0;
+        uint32_t ph = 0;
         for (int i = 0; i < n_gb; ++i) {
-            g_mbar_wait(full_a + 8 * s, pha);
+            g_mbar_wait(full + 8 * s, ph);
             SK_TRC(0, i, 0);
-            g_mbar_wait(full_b + 8 * bs, phb);
-            SK_TRC(0, i, 1);
+            SK_TRC(0, i, 1);  // (one barrier for both)
             g_tc_fence_after();
             if (g_elect_one()) {
                 const uint32_t a_tmem = tmem_d + Smem::D_COLS + s * 64;  // 16 reduction elements = 8 columns per K step
-                const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(bs * (2 * Smem::B_BYTES >> 4));
+                const uint64_t bdesc = bdesc0 + static_cast<uint64_t>(s * (2 * Smem::B_BYTES >> 4));
 #pragma unroll
                 for (int k = 0; k < SK_GB / 16; ++k)
                     g_tc_mma_ts(tmem_d, a_tmem + 8 * k, bdesc + (k >> 2) * (Smem::B_BYTES >> 4) + 2 * (k & 3), idesc, (i > 0 || k > 0) ? 1u : 0u);
                 g_tc_commit(empty + 8 * s);
-                g_tc_commit(b_empty + 8 * bs);
             }
             __syncwarp();
             SK_TRC(0, i, 2);
-            if (++s == ASTAGES) s = 0, pha ^= 1u;
-            if (++bs == BSTAGES) bs = 0, phb ^= 1u;
+            if (++s == STAGES) s = 0, ph ^= 1u;
         }
         if (g_elect_one()) g_tc_commit(tmem_full);
         __syncwarp();
@@ -255,9 +251,9 @@ w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const uint32_t lane_base = tmem_d + (static_cast<uint32_t>((warp & 3) * 32) << 16) + Smem::D_COLS;
         unsigned short s_next = 0, b_next = 0;
         if (grp < n_gb) s_next = __ldg(sc + grp), b_next = __ldg(bi + grp);
-        int ps = 0, s = grp % ASTAGES;
+        int ps = 0, s = grp % STAGES;
         uint32_t php = 0, phe = 1;  // consumer of the packed ring; producer side of the tile ring (first pass does not wait)
-        if (grp >= ASTAGES) phe ^= 1u;
+        if (grp >= STAGES) phe ^= 1u;
         for (int i = grp; i < n_gb; i += 2) {
             const unsigned short s16 = s_next, b16 = b_next;
             if (i + 2 < n_gb) s_next = __ldg(sc + i + 2), b_next = __ldg(bi + i + 2);
@@ -304,7 +300,7 @@ w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             // the first version); __syncwarp orders the lanes' stores before it
             __syncwarp();
             if (lane == 0) {
-                g_mbar_arrive(full_a + 8 * s);
+                g_mbar_arrive(full + 8 * s);
                 // Release the packed box only now: the tensor-memory stores above consumed the loaded words, so this
                 // warp's shared-memory reads of the box have COMPLETED (an arrive issued right behind the load let the TMA
                 // refill the box under a load still in flight - mbarrier ops are not ordered behind the load/store
@@ -314,7 +310,7 @@ w4a16_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             if ((warp & 3) == 0) SK_TRC(1 + grp, i, 3);
             if (++ps == PSTAGES) ps = 0, php ^= 1u;
             s += 2;
-            if (s >= ASTAGES) s -= ASTAGES, phe ^= 1u;
+            if (s >= STAGES) s -= STAGES, phe ^= 1u;
         }
         // ------------------------------------------------ epilogue: TMEM lane = feature; warps 4-7 take token columns [0, NT/2), 8-11 the rest
         TL_TRACE_STAMP_T(33, 128);  // last weight tile handed to the MMA thread

@@ -1,6 +1,6 @@
 """Per-block cycle timeline of CTA 0 of the swap-AB GEMM (debug build with -DTL_TRACE=1):
   TL_LIB=.../libtiny_llm_b200_trace.so python tools/skinny_blocks.py [M N K]
-Columns (SM cycles since the first stamp): MMA thread: A tile ready / B tile ready / MMAs issued; dequantiser group
+Columns (SM cycles since the first stamp): MMA thread: A and B tiles ready (one barrier, two equal columns) / MMAs issued; dequantiser group
 owning the block: box ready / math done / stage free / handed over."""
 import ctypes
 import sys
