@@ -88,6 +88,24 @@ def test_runs_on_two_streams_do_not_share_planes():
     assert all(torch.equal(y, want[i]) for i in range(2) for y in got[i])
 
 
+def test_planes_belong_to_the_stream_that_works_in_them():
+    """Memory that the current stream has freed and has yet to write is no place for another stream's planes."""
+    w = weight(2560, 9728, torch.bfloat16, 1)
+    x = torch.randn(300, 9728, device="cuda").bfloat16()
+    want, side = quantized_linear(x, w), torch.cuda.Stream()
+    part = (w.scales, w.biases, 128, 4, x, w.weight, True, True, True)
+    ext.quantized_matmul(*part, stream=side)
+    torch.cuda.synchronize()
+    late = [torch.empty(n * 300 * 2560, device="cuda") for n in range(2, 13)]  # as large as the planes of 2 to 12 runs
+    torch.cuda._sleep(2_000_000)
+    for t in late:
+        t.fill_(float("nan"))
+    del t, late
+    got = ext.quantized_matmul(*part, stream=side)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+
+
 def test_without_memory_for_planes_the_reduction_stays_whole(monkeypatch):
     w = weight(2560, 9728, torch.bfloat16, 1)
     x = torch.randn(300, 9728, device="cuda").bfloat16()

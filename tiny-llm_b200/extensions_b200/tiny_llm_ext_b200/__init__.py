@@ -186,13 +186,14 @@ def _planes(nbytes: int, rows: int, device, stream) -> torch.Tensor | None:
     no memory for them, and the reduction stays whole."""
     if nbytes == 0 or rows <= 128:
         return _zero_workspace(nbytes, device)
+    # memory of the stream that works in it: nothing that another stream still has to do touches it, and it can be given back on return
+    if stream is not None and not isinstance(stream, torch.cuda.Stream):
+        stream = torch.cuda.ExternalStream(stream.cuda_stream, device=device)
     try:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        with torch.cuda.stream(stream):
+            return torch.empty(nbytes, dtype=torch.uint8, device=device)
     except torch.OutOfMemoryError:
         return None
-    if stream is not None:  # freed on return, while that stream may still have to read it
-        ws.record_stream(stream)
-    return ws
 
 
 _ZERO_WS: dict = {}
