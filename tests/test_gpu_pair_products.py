@@ -46,6 +46,15 @@ def test_gates_outside_the_fast_division(M):
     assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(), want.nan_to_num())
 
 
+@pytest.mark.parametrize("M,N,K", [(129, 4096, 2560), (300, 9728, 264), (512, 9728, 1004), (300, 9728, 1001)])
+def test_gated_products_whose_reductions_run_in_pieces(M, N, K):
+    gate, up = weight(K, N, torch.bfloat16, 1), weight(K, N, torch.bfloat16, 2)
+    x = torch.randn(M, N, generator=torch.Generator(device="cuda").manual_seed(M), device="cuda").bfloat16()
+    part = lambda w: (w.scales, w.biases, w.weight)  # noqa: E731
+    want = ext.swiglu(quantized_linear(x, gate), quantized_linear(x, up))
+    assert torch.equal(ext.quantized_gate_up(x, part(gate), part(up), (True, True), (True, True)), want)
+
+
 def unpacked(w):
     """The weights as the kernels see them: code x scale + bias in fp32, rounded to the storage type."""
     words = w.weight

@@ -645,6 +645,7 @@ int launch_w4a16_gemm2(const void *scales, const void *biases, const void *a, co
 
 bool launch_w4a16_gemm2_gated(const tl_packed_matrix &gate, const tl_packed_matrix &up, const void *a, void *out, int M, int N, int K, int dtype, cudaStream_t st, int *rc) {
     if (g_pairs_mode <= 0 || M <= 128 || !(dtype == TL_BF16 || dtype == TL_F16) || N % 128 != 0) return false;
+    if (w4a16_gemm2_splits(M, N, K, dtype) > 1) return false;  // each product by itself is added in runs, in another order than here
     if (dtype == TL_BF16)
         *rc = gemm2_t<__nv_bfloat16, true>(pair_weights<__nv_bfloat16>(gate.scales, gate.biases, gate.weight), pair_weights<__nv_bfloat16>(up.scales, up.biases, up.weight), a, out, M, N,
                                            K, st);
