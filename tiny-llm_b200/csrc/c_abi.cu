@@ -122,8 +122,8 @@ static int quantized_product(const void *scales, const void *biases, const void 
         return launch_w4a16_skinny(scales, biases, a, b, out, gate, M, N, K, gate ? TL_EPI_GATED : TL_EPI_NONE, dtype, workspace, workspace_bytes, st);
     if (use_stream_kernel(M, N, K, dtype, use_simdgroup))
         return launch_w4a16_fused(scales, biases, b, out, a, nullptr, gate, M, N, K, N, TL_PRO_NONE, gate ? TL_EPI_GATED : TL_EPI_NONE, 0.f, dtype, st);
-    // above 128 rows the activation is a launch of its own: in the GEMM's epilogue, which nothing overlaps, it cost more (2048 rows of
-    // 2560 -> 9728: 105 -> 150 us for the product, where the launch takes 24)
+    // above 128 rows the activation of a product by itself is a launch of its own (the one-CTA kernel's epilogue, which nothing overlaps, has no room
+    // for it: 2048 rows of 2560 -> 9728 105 -> 150 us, the launch 24); gate and up together take tl_quantized_gated's one launch instead
     const int rc = launch_w4a16_gemm(scales, biases, a, b, out, M, N, K, dtype, use_split_k, workspace, workspace_bytes, st);
     return rc != TL_OK || gate == nullptr ? rc : launch_swiglu(gate, out, out, static_cast<long long>(M) * K, dtype, st);
 }

@@ -57,10 +57,10 @@ int launch_w4a16_vanilla(const void *scales, const void *biases, const void *a, 
                          int N, int K, int dtype, cudaStream_t st);
 
 
-// w4a16_gemm2.cu (CTA pairs, tcgen05 cta_group::2: M > 256)
+// w4a16_gemm2.cu (CTA pairs, tcgen05 cta_group::2: M > 256; gated products and reductions in runs from 129 rows)
 long long w4a16_gemm_cost(int M, int N, int K);  // of the one-CTA kernel: cycles of a reduction block, summed over its waves of CTAs
 bool w4a16_gemm2_supported(int M, int N, int K, int dtype);
-void set_gemm_pairs(int mode);  // 0 never, 1 where the pair grid fills the SMs (default), 2 every M > 256
+void set_gemm_pairs(int mode);  // 0 never, 1 where its rounds of the SMs cost less (default), 2 every M > 256 and no reduction in runs
 // silu(a gate^T) * (a up^T) in one launch; false: the other way is better or the only one
 bool launch_w4a16_gemm2_gated(const tl_packed_matrix &gate, const tl_packed_matrix &up, const void *a, void *out, int M, int N, int K, int dtype, cudaStream_t st, int *rc);
 long long gemm2_gave_up();

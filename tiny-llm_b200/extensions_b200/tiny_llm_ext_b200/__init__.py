@@ -295,8 +295,8 @@ def _check_quantized_matmul(scales, biases, group_size, bits, a, b, transpose_b)
 
 
 def quantized_gate_up(a, gate, up, gate_flags=(True, False), up_flags=(True, False), stream=None):
-    """``silu(a @ gate.T) * (a @ up.T)`` of two quantised weights ``(scales, biases, packed)`` of one shape: both from one launch up to 128
-    rows, else the gate's product, then the up projection with the activation.  The flags are (use_simdgroup, use_split_k) of either product.  The same bits as two
+    """``silu(a @ gate.T) * (a @ up.T)`` of two quantised weights ``(scales, biases, packed)`` of one shape: both from one launch
+    where both may use the tensor cores, else the gate's product, then the up projection with the activation.  The flags are (use_simdgroup, use_split_k) of either product.  The same bits as two
     ``quantized_matmul`` calls and ``swiglu``."""
     for scales, biases, packed in (gate, up):
         if not _quantized_matmul_fits(scales, biases, 128, 4, a, packed):
