@@ -109,3 +109,28 @@ def test_lists(tokens, top, experts):
         assert all(flat[pair[r]] == e for r in range(first, first + n))
         covered += range(first, first + n)
     assert sorted(covered) == sorted(seen.values())
+
+
+def test_calls_that_follow_one_another_closely():
+    """A call's launches start while the one before is ending: of many sizes in a row, with nothing waited for, and replayed from a graph, the same bits as one by one."""
+    from extensions_b200.tiny_llm_ext_b200 import blocks
+
+    gen = torch.Generator().manual_seed(5)
+    bf = lambda *s, std=1.0: (torch.randn(*s, generator=gen) * std).to(torch.bfloat16).to(DEV)  # noqa: E731
+    experts, dim, ff, top = 8, 256, 200, 3
+    wg, wu, wd = bf(experts, ff, dim, std=dim**-0.5), bf(experts, ff, dim, std=dim**-0.5), bf(experts, dim, ff, std=ff**-0.5)
+    parts = [(bf(n, dim), choices(n, top, experts, n % 2 == 0, gen).to(DEV), torch.rand(n, top, generator=gen).to(DEV)) for n in (1, 16, 40, 300, 17, 700, 2)]
+    run = lambda i: blocks.moe_experts(*parts[i], wg, wu, wd, blocks.ACT_SILU)  # noqa: E731
+    want = []
+    for i in range(len(parts)):
+        torch.cuda.synchronize()
+        want.append(run(i).clone())
+    torch.cuda.synchronize()
+    got = [[run(i) for i in range(len(parts))] for _ in range(10)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        replayed = [run(i) for i in range(len(parts))]
+    for _ in range(10):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[i]) for row in got + [replayed] for i, y in enumerate(row))

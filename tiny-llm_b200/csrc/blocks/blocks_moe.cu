@@ -298,6 +298,7 @@ __global__ void __launch_bounds__(256)
 moe_combine_kernel(const float *__restrict__ pair_out, const float *__restrict__ gate, const T *__restrict__ shared,
                    const float *__restrict__ shared_gate, const int32_t *__restrict__ idx, int experts, const T *__restrict__ h, float *__restrict__ y, int top, int dim) {
     const int t = blockIdx.x, d = (blockIdx.y * 256 + threadIdx.x) * W;
+    tl::griddep_wait();
     if (d >= dim) return;
     constexpr int AT_ONCE = 8;
     float s[W] = {};
@@ -310,8 +311,12 @@ moe_combine_kernel(const float *__restrict__ pair_out, const float *__restrict__
                 if (idx != nullptr && idx[pair] >= experts) {
 #pragma unroll
                     for (int j = 0; j < W; ++j) x[u][j] = to_f(h[(size_t)t * dim + d + j]);
+                } else if constexpr (W == 4) {  // ld_cg: not to be read ahead of the wait
+                    const uint4 v = tl::ld_cg(reinterpret_cast<const uint4 *>(pair_out + pair * dim + d));
+                    x[u][0] = __uint_as_float(v.x), x[u][1] = __uint_as_float(v.y), x[u][2] = __uint_as_float(v.z), x[u][3] = __uint_as_float(v.w);
                 } else {
-                    moe_load<W>(pair_out + pair * dim + d, x[u]);
+                    static_assert(W == 1, "columns of a thread");
+                    x[u][0] = tl::ld_cg(pair_out + pair * dim + d);
                 }
             }
 #pragma unroll
@@ -436,7 +441,7 @@ int tlb_moe_combine(const float *pair_out, const float *gate, const void *shared
     if (!pair_out || !y || top <= 0 || dim <= 0 || (idx && !h)) return tl::fail(TL_EINVAL, "moe_combine: bad argument");
     const bool wide = dim % 4 == 0 && tl::aligned16(pair_out) && tl::aligned16(y);
     const dim3 grid(tokens, ceil_div(dim, wide ? 1024 : 256));
-#define TLB_COMBINE(WV) moe_combine_kernel<T, WV><<<grid, 256, 0, as_stream(stream)>>>(pair_out, gate, (const T *)shared, shared_gate, idx, experts, (const T *)h, y, top, dim)
+#define TLB_COMBINE(WV) moe_launch(moe_combine_kernel<T, WV>, grid, 256, 0, as_stream(stream), pair_out, gate, (const T *)shared, shared_gate, idx, experts, (const T *)h, y, top, dim)
     TLB_DISPATCH(dtype, "moe_combine", if (wide) TLB_COMBINE(4); else TLB_COMBINE(1));
 #undef TLB_COMBINE
     TL_LAUNCH_CHECK("moe_combine");

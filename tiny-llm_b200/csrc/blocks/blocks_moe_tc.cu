@@ -52,6 +52,7 @@ struct MoeTcArgs {
     float *pair_out;
     int stages, stage_bytes;
     int turning;  // 1: tiles of different sizes: dealt forth and back
+    int second;   // 1: the launch before this one is a product too, and the lists are older than both
 };
 
 // A warp's part of a finished tile: 32 weight rows, tokens begin .. end - 1 of the chunk that starts at row0 of the sorted list, eight
@@ -128,6 +129,10 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
     __syncthreads();
     g_tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if (!a.second) {
+        tl::griddep_wait();
+        tl::griddep_launch();  // the lists are complete: see moe_launch
+    }
     const int tiles = a.counters[2] * a.m_blocks;
     const bool gated = a.epilogue == kEpiGated;
     // Tiles come largest first (moe_sort_kernel), dealt forth and back, so that the CTAs' sums differ by little more than the smallest tile.  (Tiles of one
@@ -156,6 +161,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
     } else if (warp == 2) {  // ---- consecutive rows of the second operand
         int s = 0;
         uint32_t ph = 1;
+        if (a.second) tl::griddep_wait();
         for (int turn = 0, tile; !gathers && (tile = tile_of(turn)) < tiles; ++turn) {
             const int4 c = a.chunks[tile / a.m_blocks];
             for (int kb = 0; kb < a.k_blocks; ++kb) {
@@ -170,6 +176,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_w0, const __grid_constant_
         const uint32_t to = 2 * kTcBlockBytes + r0 * 128 + ((piece ^ (r0 & 7)) << 4);
         int s = 0, before = -1;  // the stage whose copies this thread has issued and not yet reported
         uint32_t ph = 1;
+        if (a.second) tl::griddep_wait();
         auto report = [&](int stage) {  // landed: visible to the tensor core's proxy, then one arrival per warp
             tl::g_fence_proxy_async();
             __syncwarp();
@@ -304,6 +311,7 @@ int moe_tc_product(const MoeProduct &p, cudaStream_t st) {
     a.stage_bytes = 2 * kTcBlockBytes + moe_chunk_rows(p.tokens) * 128;
     a.stages = std::min(kTcMaxStages, (227 * 1024 - kTcBars) / a.stage_bytes);
     a.turning = moe_chunk_rows(p.tokens) > 16;
+    a.second = a.epilogue == kEpiPairs;
     a.m_blocks = ceil_div(p.N, a.epilogue == kEpiGated ? 128 : 256);
     // the largest that any call asks for; on every call, because the attribute belongs to the device that is current
     if (cudaFuncSetAttribute(moe_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
@@ -311,7 +319,7 @@ int moe_tc_product(const MoeProduct &p, cudaStream_t st) {
         return tl::fail(TL_ECUDA, "moe_tc: no shared memory");
     }
     const long long most = moe_max_chunks(p.tokens, p.top, p.experts) * a.m_blocks;  // tiles there can be
-    moe_tc_kernel<<<(unsigned)std::min<long long>(sm_count(), most), kTcThreads, a.stages * a.stage_bytes + kTcBars, st>>>(m0, m1, mx, a);
+    moe_launch(moe_tc_kernel, (unsigned)std::min<long long>(sm_count(), most), kTcThreads, a.stages * a.stage_bytes + kTcBars, st, m0, m1, mx, a);
     return TL_OK;
 }
 
@@ -331,6 +339,7 @@ moe_sort_kernel(const int32_t *__restrict__ idx, int pairs, int experts, int mos
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int e = threadIdx.x; e < experts; e += kSortThreads) count[e] = 0;
     if (threadIdx.x < 2) carry[threadIdx.x] = 0;
+    tl::griddep_wait();
     __syncthreads();
     // chunks of an expert's n rows: of equal length, in whole groups of 16 rows
     auto chunk_rows = [&](int n) {
@@ -342,14 +351,14 @@ moe_sort_kernel(const int32_t *__restrict__ idx, int pairs, int experts, int mos
 #pragma unroll
     for (int i = 0; i < kSortKeep; ++i) {
         const int p = threadIdx.x + i * kSortThreads;
-        const int e = p < pairs ? idx[p] : -1;
+        const int e = p < pairs ? tl::ld_cg(idx + p) : -1;
         expert[i] = e >= 0 && e < experts ? e : -1;
     }
 #pragma unroll
     for (int i = 0; i < kSortKeep; ++i) rank[i] = expert[i] >= 0 ? atomicAdd(&count[expert[i]], 1) : 0;
     __syncthreads();  // the kept ones take an expert's first places
     for (int p = threadIdx.x + kSortKeep * kSortThreads; p < pairs; p += kSortThreads) {
-        const int e = idx[p];
+        const int e = tl::ld_cg(idx + p);
         if (e >= 0 && e < experts) atomicAdd(&count[e], 1);
     }
     __syncthreads();
@@ -423,7 +432,7 @@ moe_sort_kernel(const int32_t *__restrict__ idx, int pairs, int experts, int mos
             if (expert[i] >= 0) atomicAdd(&count[expert[i]], 1);
         __syncthreads();
         for (int p = threadIdx.x + kSortKeep * kSortThreads; p < pairs; p += kSortThreads) {
-            const int e = idx[p];
+            const int e = tl::ld_cg(idx + p);
             if (e >= 0 && e < experts) sorted_pair[start[e] + atomicAdd(&count[e], 1)] = p;
         }
     }
@@ -453,7 +462,7 @@ int tlb_moe_sort(const int32_t *idx, int tokens, int top, int experts, int32_t *
         cudaGetLastError();
         return tl::fail(TL_ECUDA, "moe_sort: no shared memory");
     }
-    moe_sort_kernel<<<1, kSortThreads, smem, as_stream(stream)>>>(idx, tokens * top, experts, moe_chunk_rows(tokens), moe_lists(lists, tokens, top, experts));
+    moe_launch(moe_sort_kernel, 1, kSortThreads, smem, as_stream(stream), idx, tokens * top, experts, moe_chunk_rows(tokens), moe_lists(lists, tokens, top, experts));
     TL_LAUNCH_CHECK("moe_sort");
     return TL_OK;
 }
