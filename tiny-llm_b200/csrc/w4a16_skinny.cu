@@ -526,6 +526,9 @@ __global__ void __launch_bounds__(256) __cluster_dims__(SK_NORM_CTAS, 1, 1)
 w4a16_skinny_reduce_norm_kernel(const float *part, const T *res, const T *__restrict__ norm_w, T *out, T *normed, int M, int K, int splits, float eps) {
     __shared__ float warp_part[8], rank_part[SK_NORM_CTAS];
     griddep_launch();
+    // Another CTA's shared memory may be written once that CTA runs, which only a cluster barrier says: arrived at here, waited for ahead of the store below,
+    // so that it is over long before the sums are.
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     const int rank = blockIdx.x % SK_NORM_CTAS, quarter = (K + SK_NORM_CTAS - 1) / SK_NORM_CTAS, first = rank * quarter, last = min(first + quarter, K);
     const size_t plane = static_cast<size_t>(M) * K, row = static_cast<size_t>(blockIdx.x / SK_NORM_CTAS) * K;
     griddep_wait();
@@ -568,6 +571,7 @@ w4a16_skinny_reduce_norm_kernel(const float *part, const T *res, const T *__rest
     ss = warp_sum(ss);
     if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = ss;
     __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // all CTAs of the cluster run
     if (threadIdx.x < 32) {
         ss = warp_sum(threadIdx.x < 8 ? warp_part[threadIdx.x] : 0.f);
         if (threadIdx.x < SK_NORM_CTAS)  // into rank_part[rank] of CTA `threadIdx.x`
