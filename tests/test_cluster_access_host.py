@@ -7,7 +7,7 @@ from pathlib import Path
 import pytest
 
 CSRC = Path(__file__).resolve().parent.parent / "tiny-llm_b200" / "csrc"
-ACCESS = re.compile(r"\bmapa\.|\bst\.shared::cluster|\bld\.shared::cluster|map_shared_rank|\bp_mbar_arrive_leader\(|\bp_tc_commit2\(|\bp_tc_mma2\(")
+ACCESS = re.compile(r"mapa\.|st\.shared::cluster|ld\.shared::cluster|map_shared_rank|\bp_mbar_arrive_leader\(|\bp_tc_commit2\(|\bp_tc_mma2\(")
 BARRIER = re.compile(r"barrier\.cluster\.wait|\bp_cluster_sync\(\)|cluster\.sync\(\)")
 
 
