@@ -517,20 +517,22 @@ __global__ void __launch_bounds__(128) w4a16_skinny_reduce4_kernel(const float *
 // The same reduction for the residual epilogue when the RMSNorm of the NEXT projection follows (o -> post-attention norm,
 // down -> next layer's input norm): a cluster of SK_NORM_CTAS CTAs per token row adds the planes, adds the residual, writes the residual
 // stream and - the row being complete in the cluster's registers - the normalised row too (week2_kernels.metal:41-47 arithmetic:
-// T(x * rsqrt(mean(x^2) + eps) * w) on the ROUNDED residual sum).  Saves the rms_norm launch and its read of the row.  The CTAs take neighbouring
-// quarters of the row and hand each other their sums of squares through shared memory, which are added in rank order.  What bounds it is round trips:
+// T(x * rsqrt(mean(x^2) + eps) * w) on the ROUNDED residual sum).  Saves the rms_norm launch and its read of the row.  What bounds it is round trips:
 // with one CTA a row each thread waited for ceil(splits / 4) of them, now for ceil(splits / 8), and a decoding batch's rows fill the chip.
-constexpr int SK_NORM_CTAS = 4, SK_NORM_PER = 4;  // elements per thread: K <= 4096
+// The sum of squares is that of ONE CTA of 256 threads, to the bit: thread t of it adds columns t, t + 256, .. in turn, then come its warps and their sums.
+// CTA `rank` has the columns of threads 64 rank .. 64 rank + 63, four threads a chain for the loads, and its first two warps add the chains.
+constexpr int SK_NORM_CTAS = 4, SK_NORM_PER = 4, SK_NORM_COLS = 256 / SK_NORM_CTAS;  // elements per thread: K <= 4096
 template <typename T>
 __global__ void __launch_bounds__(256) __cluster_dims__(SK_NORM_CTAS, 1, 1)
 w4a16_skinny_reduce_norm_kernel(const float *part, const T *res, const T *__restrict__ norm_w, T *out, T *normed, int M, int K, int splits, float eps) {
-    __shared__ float warp_part[8], rank_part[SK_NORM_CTAS];
+    __shared__ float entries[SK_NORM_PER * SK_NORM_CTAS][SK_NORM_COLS], warp_part[8];
     griddep_launch();
     // Another CTA's shared memory may be written once that CTA runs, which only a cluster barrier says: arrived at here, waited for ahead of the store below,
     // so that it is over long before the sums are.
     asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
-    const int rank = blockIdx.x % SK_NORM_CTAS, quarter = (K + SK_NORM_CTAS - 1) / SK_NORM_CTAS, first = rank * quarter, last = min(first + quarter, K);
+    const int rank = blockIdx.x % SK_NORM_CTAS, chain = threadIdx.x % SK_NORM_COLS, turn = threadIdx.x / SK_NORM_COLS;
     const size_t plane = static_cast<size_t>(M) * K, row = static_cast<size_t>(blockIdx.x / SK_NORM_CTAS) * K;
+    auto column = [&](int j) { return rank * SK_NORM_COLS + chain + (turn + j * SK_NORM_CTAS) * 256; };
     griddep_wait();
     // all loads of a round (eight planes x the thread's elements, the residual beside the first) are issued before the first is used:
     // ld_cg is a volatile asm, so a load-then-add loop per element would pay one L2 round trip per batch (measured: 14 us
@@ -539,16 +541,16 @@ w4a16_skinny_reduce_norm_kernel(const float *part, const T *res, const T *__rest
     T rs[SK_NORM_PER], weight[SK_NORM_PER];
 #pragma unroll
     for (int j = 0; j < SK_NORM_PER; ++j) {
-        const int n = first + threadIdx.x + j * 256;
-        xs[j] = 0.f, rs[j] = n < last ? ld_cg(res + row + n) : from_f<T>(0.f), weight[j] = n < last ? norm_w[n] : from_f<T>(0.f);
+        const int n = column(j);
+        xs[j] = 0.f, rs[j] = n < K ? ld_cg(res + row + n) : from_f<T>(0.f), weight[j] = n < K ? norm_w[n] : from_f<T>(0.f);
     }
     for (int sp0 = 0; sp0 < splits; sp0 += 8) {
         float v[SK_NORM_PER][8];
 #pragma unroll
         for (int j = 0; j < SK_NORM_PER; ++j) {
-            const int n = first + threadIdx.x + j * 256;
+            const int n = column(j);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) v[j][q] = (n < last && sp0 + q < splits) ? ld_cg(part + (sp0 + q) * plane + row + n) : 0.f;
+            for (int q = 0; q < 8; ++q) v[j][q] = (n < K && sp0 + q < splits) ? ld_cg(part + (sp0 + q) * plane + row + n) : 0.f;
         }
 #pragma unroll
         for (int j = 0; j < SK_NORM_PER; ++j) {
@@ -557,37 +559,36 @@ w4a16_skinny_reduce_norm_kernel(const float *part, const T *res, const T *__rest
                 if (sp0 + q < splits) xs[j] += v[j][q];  // split order
         }
     }
-    float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < SK_NORM_PER; ++j) {
-        const int n = first + threadIdx.x + j * 256;
-        if (n < last) {
+        const int n = column(j);
+        if (n < K) {
             const T vb = from_f<T>(to_f(rs[j]) + to_f(from_f<T>(xs[j])));
             out[row + n] = vb;
             xs[j] = to_f(vb);
-            ss += xs[j] * xs[j];
+            entries[turn + j * SK_NORM_CTAS][chain] = xs[j];
         }
     }
-    ss = warp_sum(ss);
-    if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = ss;
     __syncthreads();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // all CTAs of the cluster run
-    if (threadIdx.x < 32) {
-        ss = warp_sum(threadIdx.x < 8 ? warp_part[threadIdx.x] : 0.f);
-        if (threadIdx.x < SK_NORM_CTAS)  // into rank_part[rank] of CTA `threadIdx.x`
-            asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.f32 [ra], %2;\n\t}" ::"r"(g_smem_u32(rank_part + rank)), "r"(threadIdx.x),
-                         "f"(ss)
+    if (threadIdx.x < SK_NORM_COLS) {
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < SK_NORM_PER * SK_NORM_CTAS; ++j)
+            if (rank * SK_NORM_COLS + chain + j * 256 < K) ss = fmaf(entries[j][chain], entries[j][chain], ss);
+        ss = warp_sum(ss);
+        const int at = rank * (SK_NORM_COLS / 32) + (threadIdx.x >> 5), peer = threadIdx.x & 31;
+        if (peer < SK_NORM_CTAS)  // into warp_part[at] of CTA `peer`
+            asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\tst.shared::cluster.f32 [ra], %2;\n\t}" ::"r"(g_smem_u32(warp_part + at)), "r"(peer), "f"(ss)
                          : "memory");
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    ss = 0.f;
-#pragma unroll
-    for (int i = 0; i < SK_NORM_CTAS; ++i) ss += rank_part[i];
+    const float ss = warp_sum((threadIdx.x & 31) < 8 ? warp_part[threadIdx.x & 31] : 0.f);
     const float inv = rsqrtf(ss / static_cast<float>(K) + eps);
 #pragma unroll
     for (int j = 0; j < SK_NORM_PER; ++j) {
-        const int n = first + threadIdx.x + j * 256;
-        if (n < last) normed[row + n] = from_f<T>(xs[j] * inv * to_f(weight[j]));
+        const int n = column(j);
+        if (n < K) normed[row + n] = from_f<T>(xs[j] * inv * to_f(weight[j]));
     }
 }
 
