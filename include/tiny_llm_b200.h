@@ -89,7 +89,7 @@ int tl_quantized_matmul(const void *scales, const void *biases, const void *a, c
 int tl_quantized_gate_up(const void *gate_scales, const void *gate_biases, const void *gate_b, const void *up_scales, const void *up_biases,
                          const void *up_b, const void *a, void *gate_out, void *out, int M, int N, int K, int dtype, int gate_flags,
                          int up_flags, void *workspace, size_t workspace_bytes, void *stream);
-/* out alone, the same bits: both products come from one launch where their sums are formed in one order.  scratch: M * K elements, undefined afterwards;
+/* out alone, the same bits: both products come from one launch where both may use the tensor cores.  scratch: M * K elements, undefined afterwards;
  * workspace: tl_quantized_gated_workspace bytes (with less, as much as tl_quantized_gate_up wants, two launches). */
 size_t tl_quantized_gated_workspace(int M, int N, int K, int dtype, int gate_flags, int up_flags);
 int tl_quantized_gated(const void *gate_scales, const void *gate_biases, const void *gate_b, const void *up_scales, const void *up_biases,
@@ -295,9 +295,8 @@ int tl_paged_metadata_clean(const int32_t *context_lens, const int32_t *block_ta
 /* Programmatic dependent launch for the streaming kernels (on by default; 0 turns it off,
  * TL_PDL=0 in the environment does the same). */
 int tl_set_pdl(int enabled);
-/* Prefill GEMM on CTA pairs (tcgen05 cta_group::2, w4a16_gemm2.cu): 0 never, 1 where they take less time (default), 2 for every
- * M > 256.  Same rounding points either way; the same bits too, except that mode 1 adds a long reduction of few tiles in
- * runs (fp32, in run order) where the workspace holds their planes.  TL_GEMM2 sets the initial mode. */
+/* Prefill GEMM on CTA pairs (tcgen05 cta_group::2, w4a16_gemm2.cu): 0 never, 1 where they take less time
+ * (default), 2 for every M > 256.  Same results either way (same rounding points); TL_GEMM2 sets the initial mode. */
 int tl_set_gemm_pairs(int mode);
 /* Device-side bookkeeping between two decode steps of a CUDA-graph loop (the
  * per-request `req.decode_done(token)` + `offset += 1` of batch.py:241-247 done

@@ -122,3 +122,17 @@ def test_gate_up_interleave_layout_and_span_record():
         raise AssertionError("rows not divisible by 8 must be rejected")
     assert ctypes.sizeof(ext.PageSpanList) == 4 * 64 * 4 + 4
     assert ext.EPI_SWIGLU_PAIRS == 2 and ext.PAGE_SPANS == 64
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 0, 64), (2048, 0, 2560), (129, -128, 64), (0, 128, 64), (-5, 128, 64), (300, 128, 0), (300, 128, -8), (1, 0, 64)])
+def test_workspaces_of_sizes_that_no_product_has(M, N, K):
+    """A size that the product itself refuses, or that has nothing in it, wants no workspace; the question is answered on any machine."""
+    for dtype in (1, 2):
+        assert ext._lib.tl_quantized_matmul_workspace(M, N, K, dtype, 1, 1) == 0
+        assert ext._lib.tl_quantized_gated_workspace(M, N, K, dtype, 1, 1) == 0
+
+
+@pytest.mark.parametrize("M", [129, 256, 300, 1024, 4096])
+def test_no_planes_above_128_rows(M):
+    for N, K in ((9728, 2560), (6144, 2048), (3072, 1024), (2560, 9728)):
+        assert ext._lib.tl_quantized_matmul_workspace(M, N, K, 2, 1, 1) == 0

@@ -57,17 +57,15 @@ int launch_w4a16_vanilla(const void *scales, const void *biases, const void *a, 
                          int N, int K, int dtype, cudaStream_t st);
 
 
-// w4a16_gemm2.cu (CTA pairs, tcgen05 cta_group::2: M > 256; gated products and reductions in runs from 129 rows)
+// w4a16_gemm2.cu (CTA pairs, tcgen05 cta_group::2: M > 256; gated products from 129 rows)
 long long w4a16_gemm_cost(int M, int N, int K);  // of the one-CTA kernel: cycles of a reduction block, summed over its waves of CTAs
 bool w4a16_gemm2_supported(int M, int N, int K, int dtype);
-void set_gemm_pairs(int mode);  // 0 never, 1 where its rounds of the SMs cost less (default), 2 every M > 256 and no reduction in runs
+void set_gemm_pairs(int mode);  // 0 never, 1 where its rounds of the SMs cost less (default), 2 every M > 256
 // silu(a gate^T) * (a up^T) in one launch; false: the other way is better or the only one
 bool launch_w4a16_gemm2_gated(const tl_packed_matrix &gate, const tl_packed_matrix &up, const void *a, void *out, int M, int N, int K, int dtype, cudaStream_t st, int *rc);
 long long gemm2_gave_up();
-int w4a16_gemm2_splits(int M, int N, int K, int dtype);  // runs that the reduction is cut into (1: not), each with a plane [M, K] of fp32 sums
 int launch_w4a16_gemm2(const void *scales, const void *biases, const void *a, const void *b, void *out, int M, int N, int K, int dtype,
-                       cudaStream_t st, int splits = 1, float *planes = nullptr);
-int launch_w4a16_plane_sum(const float *planes, void *out, int M, int K, int splits, int dtype, cudaStream_t st);
+                       cudaStream_t st);
 
 // w4a16_skinny.cu (swap-AB tcgen05 GEMM with split reduction, 9 <= M <= 128)
 bool w4a16_skinny_supported(int M, int N, int K, int dtype);

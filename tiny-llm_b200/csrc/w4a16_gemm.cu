@@ -351,14 +351,12 @@ bool w4a16_gemm_supported(int M, int N, int K, int dtype) {
     return (dtype == TL_BF16 || dtype == TL_F16) && M > 0 && K > 0 && N % 128 == 0;
 }
 
-// Whether the reduction is split is decided by the sizes alone (w4a16_gemm2.cu): a split-K request runs the very same kernels
-// (bit-identical results, tests_refsol/test_week_2_day_7.py:80-109).
+// The B200 schedule never splits the reduction: a 128x128 tile already runs N/64
+// MMA stages back to back, and small-M problems go to the streaming kernel.  A
+// split-K request therefore runs the very same kernel (bit-identical results,
+// tests_refsol/test_week_2_day_7.py:80-109).
 int w4a16_gemm_split(int, int, int, int) { return 1; }
-size_t w4a16_gemm_workspace(int M, int N, int K, int dtype, int) {
-    if (!w4a16_gemm_supported(M, N, K, dtype)) return 0;
-    const int splits = w4a16_gemm2_splits(M, N, K, dtype);
-    return splits > 1 ? static_cast<size_t>(splits) * M * K * sizeof(float) : 0;
-}
+size_t w4a16_gemm_workspace(int, int, int, int, int) { return 0; }
 
 // Cycles of a 64-wide reduction block with mt token tiles per CTA, measured where every SM has one CTA (148 x 128 features; 9728
 // long: 55, 92 and 112 us for one to three tiles; 2560 long: 38 and 45 us for three and four).
@@ -453,11 +451,8 @@ static int gemm_t(const void *scales, const void *biases, const void *a, const v
 }
 
 int launch_w4a16_gemm(const void *scales, const void *biases, const void *a, const void *b, void *out, int M, int N, int K,
-                      int dtype, int use_split_k, void *ws, size_t ws_bytes, cudaStream_t st) {
+                      int dtype, int /*use_split_k*/, void * /*ws*/, size_t /*ws_bytes*/, cudaStream_t st) {
     if (M == 0 || K == 0) return TL_OK;
-    const size_t planes = w4a16_gemm_workspace(M, N, K, dtype, use_split_k);
-    if (planes > 0 && ws != nullptr && ws_bytes >= planes && aligned16(ws))
-        return launch_w4a16_gemm2(scales, biases, a, b, out, M, N, K, dtype, st, w4a16_gemm2_splits(M, N, K, dtype), static_cast<float *>(ws));
     if (w4a16_gemm2_supported(M, N, K, dtype)) return launch_w4a16_gemm2(scales, biases, a, b, out, M, N, K, dtype, st);  // CTA pairs
     if (dtype == TL_BF16) return gemm_t<__nv_bfloat16>(scales, biases, a, b, out, M, N, K, st);
     if (dtype == TL_F16) return gemm_t<__half>(scales, biases, a, b, out, M, N, K, st);

@@ -28,8 +28,6 @@
 #include <stdlib.h>
 #include <cudaTypedefs.h>
 
-#include <algorithm>
-
 #include "common.cuh"
 #include "kernels.h"
 #include "per_device.h"
@@ -141,25 +139,18 @@ struct PDeq<__half> {
 
 // What a pair works on: n_tiles feature tiles x groups of two 256-token tiles, dealt to the pairs in turn.  The first `full` of them go out whole; the
 // rest, which would fill less than half of a last round, in single 256-token tiles.
-// splits > 1: every tile's reduction is cut into that many runs of quantisation groups, each a piece of work of its own that leaves fp32 sums in a plane of
-// the workspace; a launch behind it adds the planes in order.
 struct PairPlan {
-    int n_tiles, m_tiles, full, items, splits, groups /* of a run */;
+    int n_tiles, m_tiles, full, items;
 };
 struct PairItem {
     int n_tile, m0, mt;  // feature tile, first 256-token tile, how many (0: nothing, a short group's second half)
-    int split, g0, g1;   // quantisation groups g0 .. g1 - 1 of the reduction
 };
-__host__ __device__ __forceinline__ PairItem pair_item(const PairPlan &p, int i, int groups) {
-    int tile = i, m0 = 0, most = P_MT, split = 0;
-    if (p.splits > 1) {
-        tile = i / (p.n_tiles * p.splits) * p.n_tiles + i % p.n_tiles, split = i / p.n_tiles % p.splits;
-    } else if (i >= p.full) {
-        tile = p.full + (i - p.full) / P_MT, m0 = (i - p.full) % P_MT, most = 1;
-    }
+__host__ __device__ __forceinline__ PairItem pair_item(const PairPlan &p, int i) {
+    int tile = i, m0 = 0, most = P_MT;
+    if (i >= p.full) tile = p.full + (i - p.full) / P_MT, m0 = (i - p.full) % P_MT, most = 1;
     m0 += tile / p.n_tiles * P_MT;
-    const int left = p.m_tiles - m0, g0 = split * p.groups, g1 = g0 + p.groups;
-    return {tile % p.n_tiles, m0, left < most ? (left < 0 ? 0 : left) : most, split, g0, g1 < groups ? g1 : groups};
+    const int left = p.m_tiles - m0;
+    return {tile % p.n_tiles, m0, left < most ? (left < 0 ? 0 : left) : most};
 }
 
 template <typename T>
@@ -189,6 +180,7 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = static_cast<int>(p_cta_rank());       // 0 = leader (issues the MMAs)
     const int unit = blockIdx.x >> 1, units = gridDim.x >> 1;
+    const int num_kb = N / P_KB;
     const int G = N / 128;
     constexpr int FEATURES = GATED ? P_ROWS : 2 * P_ROWS;  // of a tile
 
@@ -229,8 +221,8 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         int s = 0;
         uint32_t ph = 1;
         for (int it = unit; it < plan.items; it += units) {
-            const PairItem item = pair_item(plan, it, G);
-            for (int kb = 2 * item.g0; item.mt > 0 && kb < 2 * item.g1; ++kb) {
+            const PairItem item = pair_item(plan, it);
+            for (int kb = 0; item.mt > 0 && kb < num_kb; ++kb) {
                 if (!tc_wait(empty + 8 * s, ph, dead)) goto done;
                 if (g_elect_one()) {
                     g_mbar_expect_tx(full + 8 * s, item.mt * P_TILE);
@@ -256,11 +248,11 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 p_tc_mma2(tmem_d + i * 256, adesc0 + at + i * (P_TILE >> 4) + 2 * k, bdesc0 + at + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
         };
         for (int it = unit; it < plan.items; it += units) {
-            const PairItem item = pair_item(plan, it, G);
+            const PairItem item = pair_item(plan, it);
             if (item.mt == 0) continue;
             // The first blocks, as many as there are stages, for the first token tile, then for the second: its accumulator is still being read
             // out for the tile before, meanwhile.
-            const int num_kb = 2 * (item.g1 - item.g0), head = min(P_STAGES, num_kb), s0 = s;
+            const int head = min(P_STAGES, num_kb), s0 = s;
             if (!tc_wait(acc_empty, e_ph[0], dead)) goto done;
             e_ph[0] ^= 1u;
             for (int kb = 0; kb < head; ++kb) {
@@ -313,15 +305,13 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         // ------------------------------------------------ peer: tell the leader when this CTA's tiles of a stage are complete
         int s = 0;
         uint32_t ph = 0;
-        for (int it = unit; it < plan.items; it += units) {
-            const PairItem item = pair_item(plan, it, G);
-            for (int kb = 2 * item.g0; item.mt > 0 && kb < 2 * item.g1; ++kb) {
+        for (int it = unit; it < plan.items; it += units)
+            for (int kb = 0; pair_item(plan, it).mt > 0 && kb < num_kb; ++kb) {
                 if (!tc_wait(full + 8 * s, ph, dead)) goto done;
                 if (lane == 0) p_mbar_arrive_leader(full + 8 * s);
                 __syncwarp();
                 if (++s == P_STAGES) s = 0, ph ^= 1u;
             }
-        }
     } else if (warp >= 4 && warp < 4 + P_DEQ_WARPS) {
         // ------------------------------------------------ dequantisers: this CTA's 128 weight rows, thread = (row, 32-element half)
         const int dt = threadIdx.x - 128;
@@ -330,32 +320,29 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         using V2 = typename PDeq<T>::V2;
         const uint32_t magic = PDeq<T>::MAGIC;
         const V2 offset2 = *reinterpret_cast<const V2 *>(&magic);
-        auto first_row = [&](const PairItem &item) { return min(item.n_tile * FEATURES + (GATED ? 0 : rank * P_ROWS) + row, K - 1); };
+        auto first_row = [&](int it) { return min(pair_item(plan, it).n_tile * FEATURES + (GATED ? 0 : rank * P_ROWS) + row, K - 1); };
         auto next_item = [&](int it) {
             do it += units;
-            while (it < plan.items && pair_item(plan, it, G).mt == 0);
+            while (it < plan.items && pair_item(plan, it).mt == 0);
             return it;
         };
         int s = 0;
         uint32_t ph = 1;
-        int it = next_item(unit - units), n = 0, g = 0, g_end = 0;  // the group that is fetched next
-        auto enter = [&]() {
-            if (it >= plan.items) return;
-            const PairItem item = pair_item(plan, it, G);
-            n = first_row(item), g = item.g0, g_end = item.g1;
-        };
-        enter();
+        int it = next_item(unit - units), n = it < plan.items ? first_row(it) : 0, g = 0;  // the group that is fetched next
         uint4 next[2];
         T next_sc, next_bi;
         auto fetch = [&]() {  // a quantisation group, two blocks, ahead of its use
             const uint32_t *at = w.b + static_cast<size_t>(n) * (N / 8) + g * 16 + half * 4;
             next[0] = *reinterpret_cast<const uint4 *>(at), next[1] = *reinterpret_cast<const uint4 *>(at + 8);
             next_sc = w.scales[static_cast<size_t>(n) * G + g], next_bi = w.biases[static_cast<size_t>(n) * G + g];
-            if (++g == g_end) it = next_item(it), enter();
+            if (++g == G) {
+                g = 0, it = next_item(it);
+                if (it < plan.items) n = first_row(it);
+            }
         };
         if (it < plan.items) fetch();
         for (int mine = next_item(unit - units); mine < plan.items; mine = next_item(mine))
-            for (int left = pair_item(plan, mine, G).g1 - pair_item(plan, mine, G).g0; left > 0; --left) {
+            for (int group = 0; group < G; ++group) {
                 const uint4 cur[2] = {next[0], next[1]};
                 V2 s2, b2;
                 s2.x = s2.y = next_sc, b2.x = b2.y = next_bi;
@@ -394,16 +381,8 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         const int q = warp & 3, side = (warp - 4 - P_DEQ_WARPS) >> 2;
         unsigned char *stage = psm + P_OUT_OFF + (warp - 4 - P_DEQ_WARPS) * P_OUT_BYTES;
         uint32_t f_ph[P_MT] = {0, 0};
-        auto release = [&](int i) {  // all of this accumulator's columns are read
-            g_tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                if (rank == 0) g_mbar_arrive(acc_empty + 8 * i);
-                else p_mbar_arrive_leader(acc_empty + 8 * i);
-            }
-        };
         for (int it = unit; it < plan.items; it += units) {
-            const PairItem item = pair_item(plan, it, G);
+            const PairItem item = pair_item(plan, it);
             for (int i = 0; i < item.mt; ++i) {
                 const bool ok = tc_wait(acc_full + 8 * i, f_ph[i], dead);
                 const float bad = tc_verdict(ok, dead);  // of a marked CTA this tile and all that follow are stored as NaN
@@ -412,31 +391,6 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 const uint32_t d = tmem_d + (static_cast<uint32_t>(q * 32) << 16) + i * 256;
                 const int m0 = (item.m0 + i) * 256 + rank * P_TOK + q * 32;  // this warp's first token
                 constexpr int BOXES = GATED ? 1 : 2;                           // of 64 features
-                if constexpr (!GATED)
-                    if (plan.splits > 1) {  // fp32 sums, 32 features a box
-#pragma unroll 1
-                        for (int box = 0; box < 4; ++box) {
-                            const int col0 = side * 128 + box * 32, n0 = item.n_tile * FEATURES + col0;
-                            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                            __syncwarp();
-                            uint32_t v[32];
-                            g_tmem_ld32(d + col0, v);
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                *reinterpret_cast<float4 *>(stage + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                                    make_float4(__uint_as_float(v[4 * j]) * bad, __uint_as_float(v[4 * j + 1]) * bad, __uint_as_float(v[4 * j + 2]) * bad, __uint_as_float(v[4 * j + 3]) * bad);
-                            if (box == 3) release(i);
-                            g_fence_proxy_async();
-                            __syncwarp();
-                            if (lane == 0 && m0 < M && n0 < K) {
-                                asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(&tmap_out), "r"(n0), "r"(m0), "r"(item.split),
-                                             "r"(g_smem_u32(stage))
-                                             : "memory");
-                                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                            }
-                        }
-                        continue;
-                    }
 #pragma unroll 1
                 for (int box = 0; box < BOXES; ++box) {
                     const int col0 = (GATED ? side : side * 2 + box) * 64, n0 = item.n_tile * FEATURES + col0;
@@ -466,7 +420,14 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                             *reinterpret_cast<uint4 *>(stage + lane * 128 + (((c >> 3) + j) ^ (lane & 7)) * 16) =
                                 make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
                     }
-                    if (box == BOXES - 1) release(i);
+                    if (box == BOXES - 1) {  // all of this accumulator's columns are read
+                        g_tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) {
+                            if (rank == 0) g_mbar_arrive(acc_empty + 8 * i);
+                            else p_mbar_arrive_leader(acc_empty + 8 * i);
+                        }
+                    }
                     if (tma_store) {
                         g_fence_proxy_async();
                         __syncwarp();
@@ -501,7 +462,7 @@ done:  // also from a role whose wait gave up
     if (blockIdx.x == 0 && g_trace_buf != nullptr) {  // tag = 20000 + role * 1000 + block * 4 + k (as w4a16_gemm.cu)
         for (int e = threadIdx.x; e < 2 * 40 * 4; e += P_THREADS) {
             const int role = e / 160, rest = e - role * 160;
-            if (rest / 4 < N / P_KB && role == 0 && (rest & 3) != 3) {
+            if (rest / 4 < num_kb && role == 0 && (rest & 3) != 3) {
                 const unsigned at = atomicAdd(g_trace_n, 1u);
                 if (at < g_trace_cap) g_trace_buf[2 * at] = 20000 + role * 1000 + rest, g_trace_buf[2 * at + 1] = trc[role][rest / 4][rest & 3];
             }
@@ -524,13 +485,12 @@ static int pairs_default() {
 static int g_pairs_mode = pairs_default();
 void set_gemm_pairs(int mode) { g_pairs_mode = mode; }
 
-static PairPlan pair_plan(int M, int N, int K, int features, int units, int splits) {
+static PairPlan pair_plan(int M, int K, int features, int units) {
     PairPlan p;
     p.n_tiles = ceil_div(K, features), p.m_tiles = ceil_div(M, 256);
     const int tiles = p.n_tiles * ceil_div(p.m_tiles, P_MT), left = tiles % units;
-    p.groups = ceil_div(N / 128, splits), p.splits = ceil_div(N / 128, p.groups);
-    p.full = p.splits > 1 || left * P_MT > units ? tiles : tiles - left;
-    p.items = p.splits > 1 ? tiles * p.splits : p.full + (tiles - p.full) * P_MT;
+    p.full = left * P_MT <= units ? tiles - left : tiles;
+    p.items = p.full + (tiles - p.full) * P_MT;
     return p;
 }
 
@@ -538,64 +498,34 @@ static PairPlan pair_plan(int M, int N, int K, int features, int units, int spli
 // is 1100 a block, of single ones 700; of reductions above 4096 a whole round takes 1750 (two rounds of 9728: 0.62 us a block each).  Measured over
 // 63 sizes of 300 to 4096 rows the choice is within 2 % of the better one; us, one-CTA kernel / pairs: 2560 -> 9728 300 rows 42 / 34, 2048 105 / 77,
 // 4096 211 / 140; 2560 -> 6144 300 rows 23.8 / 24.2, 700 29.8 / 33.9, 2048 70 / 51; 9728 -> 2560 700 rows 69 / 72, 3000 167 / 110, 4096 183 / 197.
-static long long pair_block_cost(int M, int N, int K) {
-    const int units = sm_count() / 2;
-    const PairPlan p = pair_plan(M, N, K, 2 * P_ROWS, units, 1);
-    const long long whole = ceil_div(p.full, units), single = ceil_div(p.items - p.full, units);
-    return whole * (N > 4096 ? 1750 : 1100) + single * 700;
-}
 bool w4a16_gemm2_supported(int M, int N, int K, int dtype) {
     if (g_pairs_mode <= 0 || !(dtype == TL_BF16 || dtype == TL_F16) || M <= 256 || K <= 0 || N % 128 != 0) return false;
-    return g_pairs_mode >= 2 || pair_block_cost(M, N, K) < w4a16_gemm_cost(M, N, K);
-}
-
-// Into how many runs the pairs cut the reduction of a product whose tiles would leave most of them without work; 1: as one.  Times in ns, fitted to 72 sizes of 129 to
-// 2048 rows: a launch and its ends 10 us; a block 0.43 a unit of the one-CTA kernel's cost (one token tile a CTA: 350), 580 a round of whole tiles
-// and 410 of single ones; the launch that adds the planes 4 us and their bytes at 5.4 TB/s.  us, as one / in runs: 9728 -> 2560 129 rows 66 / 26 (7),
-// 300 68 / 34 (7), 512 68 / 41 (6), 2048 96 / 100; 6144 -> 2048 129 44 / 20 (8), 512 45 / 32 (6); 4096 -> 2560 129 33 / 23 (4); 2560 -> 6144 129 24, not cut.
-int w4a16_gemm2_splits(int M, int N, int K, int dtype) {
-    static const int most = [] { const char *e = getenv("TL_GEMM2_SPLITS"); return e ? atoi(e) : 12; }();  // 1: never (A/B runs)
-    if (g_pairs_mode != 1 || !(dtype == TL_BF16 || dtype == TL_F16) || M <= 128 || K <= 0 || K % 4 != 0 || N % 128 != 0) return 1;
-    const int units = sm_count() / 2, blocks = N / P_KB;
-    long long block = std::max(w4a16_gemm_cost(M, N, K), 815LL) * 43 / 100;
-    if (M > 256) {
-        const PairPlan p = pair_plan(M, N, K, 2 * P_ROWS, units, 1);
-        block = std::min<long long>(block, ceil_div(p.full, units) * 580 + ceil_div(p.items - p.full, units) * 410);
-    }
-    long long best_time = (10000 + block * blocks) * 9 / 10;  // worth it from a tenth on
-    int best = 1;
-    for (int s = 2; s <= most && s <= N / 256; ++s) {
-        const PairPlan p = pair_plan(M, N, K, 2 * P_ROWS, units, s);
-        const long long time = 14000 + static_cast<long long>(ceil_div(p.items, units)) * (2 * p.groups * (p.m_tiles > 1 ? 580 : 410) + 3000) - 3000 +
-                               static_cast<long long>(p.splits) * M * K * 8 / 5400;
-        if (p.splits == s && time < best_time) best = s, best_time = time;
-    }
-    return best;
+    if (g_pairs_mode >= 2) return true;
+    const int units = sm_count() / 2;
+    const PairPlan p = pair_plan(M, K, 2 * P_ROWS, units);
+    const long long whole = ceil_div(p.full, units), single = ceil_div(p.items - p.full, units);
+    return whole * (N > 4096 ? 1750 : 1100) + single * 700 < w4a16_gemm_cost(M, N, K);
 }
 
 template <typename T>
-static int pair_map(CUtensorMap *map, const void *p, uint64_t cols, uint64_t rows, uint32_t box_rows, int planes = 0) {
+static int pair_map(CUtensorMap *map, const void *p, uint64_t cols, uint64_t rows, uint32_t box_rows) {
     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
     if (encode == nullptr) return fail(TL_ECUDA, "quantized_matmul: cuTensorMapEncodeTiled is unavailable");
-    // planes: of fp32, 32 columns a box; the third dimension keeps a box that ends past the last row out of the next plane
-    const cuuint64_t wide = planes ? 4 : 2, dims[3] = {cols, rows, static_cast<cuuint64_t>(planes)}, strides[2] = {cols * wide, cols * wide * rows};
-    const cuuint32_t box[3] = {planes ? 32u : static_cast<cuuint32_t>(P_KB), box_rows, 1}, estr[3] = {1, 1, 1};
-    const CUtensorMapDataType dt = planes ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
-                                          : std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-    const CUresult r = encode(map, dt, planes ? 3 : 2, const_cast<void *>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+    const cuuint64_t dims[2] = {cols, rows}, strides[1] = {cols * 2};
+    const cuuint32_t box[2] = {P_KB, box_rows}, estr[2] = {1, 1};
+    const CUtensorMapDataType dt = std::is_same<T, __nv_bfloat16>::value ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+    const CUresult r = encode(map, dt, 2, const_cast<void *>(p), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? TL_OK : fail(TL_ECUDA, "quantized_matmul: cuTensorMapEncodeTiled failed (%d)", static_cast<int>(r));
 }
 
 template <typename T, bool GATED>
-static int gemm2_t(const PairWeights<T> &w0, const PairWeights<T> &w1, const void *a, void *out, int M, int N, int K, cudaStream_t st, int splits = 1, float *planes = nullptr) {
+static int gemm2_t(const PairWeights<T> &w0, const PairWeights<T> &w1, const void *a, void *out, int M, int N, int K, cudaStream_t st) {
     if (!aligned16(a) || !aligned16(w0.b) || !aligned16(w1.b)) return fail(TL_EINVAL, "quantized_matmul: a and b must be 16-byte aligned");
     const int tma_store = K % 8 == 0 && aligned16(out) ? 1 : 0;
     CUtensorMap map_a, map_out;
     if (int e = pair_map<T>(&map_a, a, N, M, P_TOK)) return e;
-    if (splits > 1) {
-        if (int e = pair_map<T>(&map_out, planes, K, M, 32, splits)) return e;
-    } else if (!tma_store) map_out = map_a;  // not used
+    if (!tma_store) map_out = map_a;  // not used
     else if (int e = pair_map<T>(&map_out, out, K, M, 32)) return e;
     static PerDevice configured;
     int device = 0;
@@ -605,7 +535,7 @@ static int gemm2_t(const PairWeights<T> &w0, const PairWeights<T> &w1, const voi
         return fail(TL_ECUDA, "quantized_matmul: cannot raise shared memory limit");
     }
     const int units = sm_count() / 2;
-    const PairPlan plan = pair_plan(M, N, K, GATED ? P_ROWS : 2 * P_ROWS, units, splits);
+    const PairPlan plan = pair_plan(M, K, GATED ? P_ROWS : 2 * P_ROWS, units);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(2 * (plan.items < units ? plan.items : units));
     cfg.blockDim = dim3(P_THREADS);
@@ -621,7 +551,7 @@ static int gemm2_t(const PairWeights<T> &w0, const PairWeights<T> &w1, const voi
     cudaError_t e = cudaLaunchKernelEx(&cfg, w4a16_gemm2_kernel<T, GATED>, map_a, map_out, w0, w1, static_cast<T *>(out), M, N, K, tma_store, plan);
     if (e != cudaSuccess) return fail(TL_ECUDA, "w4a16_gemm2: launch failed: %s", cudaGetErrorString(e));
     TL_LAUNCH_CHECK("w4a16_gemm2");
-    return splits > 1 ? launch_w4a16_plane_sum(planes, out, M, K, splits, std::is_same<T, __nv_bfloat16>::value ? TL_BF16 : TL_F16, st) : TL_OK;
+    return TL_OK;
 }
 
 template <typename T>
@@ -630,22 +560,21 @@ static PairWeights<T> pair_weights(const void *scales, const void *biases, const
 }
 
 int launch_w4a16_gemm2(const void *scales, const void *biases, const void *a, const void *b, void *out, int M, int N, int K, int dtype,
-                       cudaStream_t st, int splits, float *planes) {
+                       cudaStream_t st) {
     if (M == 0 || K == 0) return TL_OK;
     if (dtype == TL_BF16) {
         const auto w = pair_weights<__nv_bfloat16>(scales, biases, b);
-        return gemm2_t<__nv_bfloat16, false>(w, w, a, out, M, N, K, st, splits, planes);
+        return gemm2_t<__nv_bfloat16, false>(w, w, a, out, M, N, K, st);
     }
     if (dtype == TL_F16) {
         const auto w = pair_weights<__half>(scales, biases, b);
-        return gemm2_t<__half, false>(w, w, a, out, M, N, K, st, splits, planes);
+        return gemm2_t<__half, false>(w, w, a, out, M, N, K, st);
     }
     return fail(TL_EDTYPE, "quantized_matmul: scales must be float16 or bfloat16");
 }
 
 bool launch_w4a16_gemm2_gated(const tl_packed_matrix &gate, const tl_packed_matrix &up, const void *a, void *out, int M, int N, int K, int dtype, cudaStream_t st, int *rc) {
     if (g_pairs_mode <= 0 || M <= 128 || !(dtype == TL_BF16 || dtype == TL_F16) || N % 128 != 0) return false;
-    if (w4a16_gemm2_splits(M, N, K, dtype) > 1) return false;  // each product by itself is added in runs, in another order than here
     if (dtype == TL_BF16)
         *rc = gemm2_t<__nv_bfloat16, true>(pair_weights<__nv_bfloat16>(gate.scales, gate.biases, gate.weight), pair_weights<__nv_bfloat16>(up.scales, up.biases, up.weight), a, out, M, N,
                                            K, st);

@@ -758,15 +758,6 @@ static int skinny_t(const void *scales, const void *biases, const void *a, const
     return TL_OK;
 }
 
-// planes [splits][M][K] added in order, rounded once
-int launch_w4a16_plane_sum(const float *planes, void *out, int M, int K, int splits, int dtype, cudaStream_t st) {
-    const cudaError_t e = dtype == TL_BF16 ? reduce_launch<__nv_bfloat16, SK_PLAIN>(planes, nullptr, static_cast<__nv_bfloat16 *>(out), M, K, splits, SK_EPI_NONE, st)
-                                           : reduce_launch<__half, SK_PLAIN>(planes, nullptr, static_cast<__half *>(out), M, K, splits, SK_EPI_NONE, st);
-    if (e != cudaSuccess) return fail(TL_ECUDA, "w4a16_plane_sum: launch failed: %s", cudaGetErrorString(e));
-    TL_LAUNCH_CHECK("w4a16_plane_sum");
-    return TL_OK;
-}
-
 // One launch for both products and one that adds the planes: 52 rows of 2560 -> 2 x 9728, four launches before.
 template <typename T>
 static bool skinny_gate_up(SkArgs args, const void *a, const void *gate_b, const void *up_b, void *ws, size_t ws_bytes, cudaStream_t st, int *rc) {

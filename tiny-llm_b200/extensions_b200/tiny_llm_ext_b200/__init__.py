@@ -180,22 +180,6 @@ def _workspace(nbytes: int, device) -> torch.Tensor | None:
     return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
-def _planes(nbytes: int, rows: int, device, stream) -> torch.Tensor | None:
-    """The fp32 planes of a product whose reduction is split: above 128 rows the call's own memory, so that products on several streams
-    do not share it; up to 128 rows, where a step's captured launches need one address, the device's persistent buffer.  None: there is
-    no memory for them, and the reduction stays whole."""
-    if nbytes == 0 or rows <= 128:
-        return _zero_workspace(nbytes, device)
-    # memory of the stream that works in it: nothing that another stream still has to do touches it, and it can be given back on return
-    if stream is not None and not isinstance(stream, torch.cuda.Stream):
-        stream = torch.cuda.ExternalStream(stream.cuda_stream, device=device)
-    try:
-        with torch.cuda.stream(stream):
-            return torch.empty(nbytes, dtype=torch.uint8, device=device)
-    except torch.OutOfMemoryError:
-        return None
-
-
 _ZERO_WS: dict = {}
 _ZERO_WS_KEEP: list = []  # outgrown buffers may still be referenced by captured CUDA graphs
 
@@ -235,7 +219,7 @@ def quantized_matmul(
     out = a.new_empty((M, K))
     code = _DTYPE_CODE[dtype]
     ws_bytes = _lib.tl_quantized_matmul_workspace(M, N, K, code, int(use_simdgroup), int(use_split_k))
-    ws = _planes(ws_bytes, M, a.device, stream) if ws_bytes else None
+    ws = _zero_workspace(ws_bytes, a.device) if ws_bytes else None
     _check(
         _lib.tl_quantized_matmul(
             scales.data_ptr(), biases.data_ptr(), a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, code,
@@ -307,7 +291,7 @@ def quantized_gate_up(a, gate, up, gate_flags=(True, False), up_flags=(True, Fal
     gate_out, out = a.new_empty((M, K)), a.new_empty((M, K))
     flags = int(gate_flags[0]) + 2 * int(gate_flags[1]), int(up_flags[0]) + 2 * int(up_flags[1])
     ws_bytes = _lib.tl_quantized_gated_workspace(M, N, K, code, *flags)
-    ws = _planes(ws_bytes, M, a.device, stream) if ws_bytes else None
+    ws = _zero_workspace(ws_bytes, a.device) if ws_bytes else None
     _check(
         _lib.tl_quantized_gated(
             gate[0].data_ptr(), gate[1].data_ptr(), gate[2].data_ptr(), up[0].data_ptr(), up[1].data_ptr(), up[2].data_ptr(), a.data_ptr(),
@@ -339,7 +323,7 @@ def quantized_mlp(a, gate, up, down, flags, stream=None):
         return None
     out, scratch = a.new_empty((M, rows)), a.new_empty(2 * M * K)
     ws_bytes = _lib.tl_quantized_mlp_workspace(M, N, K, rows, code, flags)
-    ws = _planes(ws_bytes, M, a.device, stream) if ws_bytes else None
+    ws = _zero_workspace(ws_bytes, a.device) if ws_bytes else None
     ref = ctypes.byref
     _check(
         _lib.tl_quantized_mlp(
@@ -986,7 +970,7 @@ def set_pdl(enabled: bool) -> None:
 
 
 def set_gemm_pairs(mode: int) -> None:
-    """Prefill GEMM on CTA pairs: 0 never, 1 where the pair grid fills the SMs (default), 2 every M > 256."""
+    """Prefill GEMM on CTA pairs: 0 never, 1 where they take less time (default), 2 every M > 256."""
     _check(_lib.tl_set_gemm_pairs(int(mode)))
 
 
