@@ -124,7 +124,7 @@ def test_gate_up_interleave_layout_and_span_record():
     assert ext.EPI_SWIGLU_PAIRS == 2 and ext.PAGE_SPANS == 64
 
 
-@pytest.mark.parametrize("M,N,K", [(300, 0, 64), (2048, 0, 2560), (129, -128, 64), (0, 128, 64), (-5, 128, 64), (300, 128, 0), (300, 128, -8), (1, 0, 64)])
+@pytest.mark.parametrize("M,N,K", [(300, 0, 64), (2048, 0, 2560), (129, -128, 64), (0, 128, 64), (-5, 128, 64), (300, 128, 0), (300, 128, -8), (16, 0, 64), (128, -128, 64), (1, 0, 64)])
 def test_workspaces_of_sizes_that_no_product_has(M, N, K):
     """A size that the product itself refuses, or that has nothing in it, wants no workspace; the question is answered on any machine."""
     for dtype in (1, 2):
