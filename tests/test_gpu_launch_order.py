@@ -1,0 +1,36 @@
+"""Launches that follow one another closely, each on what the one before it wrote."""
+
+import pytest
+import torch
+
+from extensions_b200 import tiny_llm_ext_b200 as ext
+
+pytestmark = pytest.mark.gpu
+BF16 = torch.bfloat16
+
+
+@pytest.mark.parametrize("rows", [1, 24, 128])
+def test_positions_written_by_the_launch_before(rows):
+    """The step's bookkeeping, then at once the rotation and append that read it, many times over: every row turned by its own position and
+    every key in its own place, as when each launch is waited for."""
+    Hq, Hkv, D, page, pages, steps = 16, 8, 128, 16, 4, 60
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    normal = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(BF16)  # noqa: E731
+    qkv, qw, kw = normal(steps, rows, (Hq + 2 * Hkv) * D), normal(D), normal(D)
+    table = torch.randperm(rows * pages, generator=g, device="cuda").to(torch.int32).view(rows, pages)
+    ints = lambda n: torch.zeros(n, dtype=torch.int32, device="cuda")  # noqa: E731
+
+    def run(waiting):
+        slabs = [torch.zeros(rows * pages, Hkv, page, D, dtype=BF16, device="cuda") for _ in range(2)]
+        tokens, following, offsets, lens, log, counter = ints(rows), ints(rows), ints(rows), ints(rows) + 1, ints(steps * rows).view(steps, rows), ints(1)
+        out = []
+        for i in range(steps):
+            ext.decode_advance(tokens, following, offsets, lens, log, counter)
+            if waiting:
+                torch.cuda.synchronize()
+            out.append(ext.decode_qk_norm_rope_append(qkv[i], qw, kw, offsets, table, lens, *slabs, Hq, Hkv, 1e6, 1e-6))
+            if waiting:
+                torch.cuda.synchronize()
+        return torch.stack(out), *slabs
+
+    assert all(torch.equal(a, b) for a, b in zip(run(False), run(True)))

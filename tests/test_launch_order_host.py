@@ -1,0 +1,36 @@
+"""Operands that the launch before may have written are read behind the wait for it (programmatic dependent launch: a kernel may become resident while
+its predecessor still runs)."""
+
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "tiny-llm_b200" / "csrc"
+WAIT = re.compile(r"griddep_wait\(\)")
+
+
+def body_of(path, kernel):
+    source = re.sub(r"//[^\n]*", "", (CSRC / path).read_text())
+    head = re.search(r"\b" + kernel + r"\s*\([^;{]*\)\s*\{", source)
+    depth, end = 1, head.end()
+    while depth:
+        depth += {"{": 1, "}": -1}.get(source[end], 0)
+        end += 1
+    return source[head.end() : end]
+
+
+@pytest.mark.parametrize(
+    "path,kernel,operands",
+    [
+        ("elementwise.cu", "decode_qk_norm_rope_append_d128_kernel", "qkv part offsets bt cl kp vp"),
+        ("elementwise.cu", "decode_qk_norm_rope_append_kernel", "qkv offsets bt cl"),
+        ("w4a16_skinny.cu", "w4a16_skinny_reduce_norm_kernel", "part res norm_w"),
+        ("w4a16_skinny.cu", "w4a16_skinny_reduce4_kernel", "part res"),
+    ],
+)
+def test_nothing_of_the_predecessor_is_read_ahead(path, kernel, operands):
+    body = body_of(path, kernel)
+    ahead = body[: WAIT.search(body).start()]
+    read = [name for name in operands.split() if re.search(r"\b" + name + r"\s*\[|\b(ld_cg|__ldg|ldg_stream)\(\s*" + name + r"\b|\*\s*" + name + r"\b", ahead)]
+    assert not read, f"{kernel} reads {read} before griddep_wait()"

@@ -719,32 +719,15 @@ __global__ void __launch_bounds__(QKN_WARPS * 32) decode_qk_norm_rope_append_d12
     const int b = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int heads = Hq + 2 * Hkv;
-    // Positions, lengths and block tables are step inputs uploaded before the chain: the angles and the row's place in the cache are worked out
-    // under the projection (behind its planes' sums they were on the chain, 0.8 us of it a layer).
     // the 64 (sin, cos) pairs of this row's position: computed ONCE per CTA by its first two warps (one pair index per
     // thread: a double-precision exp2 and a large-argument sincosf each) and shared; every lane doing its own kept the
-    // FP64 / slow-path trig pipes busy 16x over
+    // FP64 / slow-path trig pipes busy 16x over.  The frequency depends on nothing that is read, so it is ready before the wait; positions, lengths
+    // and block tables may be the launch before's output (tl_decode_advance writes two of them) and are read behind it, requested ahead of the sums
+    // of the planes, which they arrive under.
     __shared__ float sn_s[half], cs_s[half];
-    if (threadIdx.x < half) {
-        const int i = threadIdx.x;
-        const double inv_freq = exp2(-static_cast<double>(i) / static_cast<double>(half) * log2(static_cast<double>(base)));
-        const float angle = static_cast<float>(static_cast<double>(offsets[b]) * inv_freq);
-        sincosf(angle, &sn_s[i], &cs_s[i]);
-    }
-    // page slot of this row's token (k / v heads)
-    const int ctx = cl[b];
-    T *k_dst = nullptr, *v_dst = nullptr;
-    if (ctx > 0) {
-        const int tok = ctx - 1, lp = tok / page_size;
-        if (lp < max_pages) {
-            const int pid = bt[static_cast<size_t>(b) * bt_stride + lp];
-            if (pid >= 0 && pid < num_pages) {
-                const size_t slot = (static_cast<size_t>(pid) * Hkv * page_size + (tok - lp * page_size)) * D;
-                k_dst = kp + slot, v_dst = vp + slot;
-            }
-        }
-    }
+    const double inv_freq = threadIdx.x < half ? exp2(-static_cast<double>(threadIdx.x) / static_cast<double>(half) * log2(static_cast<double>(base))) : 0.0;
     griddep_wait();  // qkv is the previous kernel's output: read through L2 (common.cuh: programmatic dependent launch)
+    const int position = ld_cg(offsets + b), ctx = ld_cg(cl + b);
     float re[QKN_MAXH][2], im[QKN_MAXH][2];
     if constexpr (PLANES) {
         const float *prow = part + static_cast<size_t>(b) * heads * D;
@@ -787,6 +770,19 @@ __global__ void __launch_bounds__(QKN_WARPS * 32) decode_qk_norm_rope_append_d12
             }
         }
     }
+    // page slot of this row's token (k / v heads)
+    T *k_dst = nullptr, *v_dst = nullptr;
+    if (ctx > 0) {
+        const int tok = ctx - 1, lp = tok / page_size;
+        if (lp < max_pages) {
+            const int pid = ld_cg(bt + static_cast<size_t>(b) * bt_stride + lp);
+            if (pid >= 0 && pid < num_pages) {
+                const size_t slot = (static_cast<size_t>(pid) * Hkv * page_size + (tok - lp * page_size)) * D;
+                k_dst = kp + slot, v_dst = vp + slot;
+            }
+        }
+    }
+    if (threadIdx.x < half) sincosf(static_cast<float>(static_cast<double>(position) * inv_freq), &sn_s[threadIdx.x], &cs_s[threadIdx.x]);
     __syncthreads();
     float sn[2], cs[2];
 #pragma unroll
