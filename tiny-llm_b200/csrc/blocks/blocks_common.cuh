@@ -66,17 +66,20 @@ __device__ __forceinline__ float gated_pair(float g, float u, int act, float lim
     return act_apply(g, act) * u;
 }
 
-// num / (1 + e^-z) of a bf16 gate: the quotient without the branch of the exact division, so that a thread's chains overlap; within 2 ulp of fp32
-// where the denominator is below 2^126, where it is not the result is 0 in place of less than 1e-36.
-__device__ __forceinline__ float over_one_plus_exp(float num, float z) { return __fdividef(num, 1.0f + expf(-z)); }
-template <int ACT>
-__device__ __forceinline__ float gated_pair_bf16(float g, float u, float limit, float slope) {
-    if constexpr (ACT == 0) return over_one_plus_exp(g, g) * u;
-    if constexpr (ACT == 3) {
-        g = fminf(g, limit), u = fminf(fmaxf(u, -limit), limit);
-        return over_one_plus_exp(g, slope * g) * (u + 1.0f);
+// The same for several pairs of a thread, which overlap; rounded to T the bits of gated_pair.
+template <typename T, int ACT, int COUNT>
+__device__ __forceinline__ void gated_pairs(const float (&g)[COUNT], const float (&u)[COUNT], float limit, float slope, float (&y)[COUNT], int live = COUNT) {
+    if constexpr (ACT == 0) {
+        tl::quotient_times<T>(g, [](float n) { return 1.0f + expf(-n); }, u, y, live);
+    } else if constexpr (ACT == 3) {
+        float num[COUNT], factor[COUNT];
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) num[i] = fminf(g[i], limit), factor[i] = fminf(fmaxf(u[i], -limit), limit) + 1.0f;
+        tl::quotient_times<T>(num, [&](float n) { return 1.0f + expf(-slope * n); }, factor, y, live);
+    } else {
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) y[i] = gated_pair(g[i], u[i], ACT, limit, slope);
     }
-    return gated_pair(g, u, ACT, limit, slope);
 }
 
 // 4 consecutive elements of a row as floats (one 8- or 16-byte access)

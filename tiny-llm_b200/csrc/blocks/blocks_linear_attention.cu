@@ -872,8 +872,8 @@ head_norm_gate_kernel(const float *__restrict__ o, const T *__restrict__ w, floa
 }
 
 // The same for rows of whole fours (16 bytes of o, 8 of a bf16 gate an access) and at most PIECES times 128 columns: a row's numbers are requested
-// together and kept, where the kernel above makes three round trips of 4-byte accesses (2048 tokens of 16 heads of 128 columns: 18 -> 12.6 us; with
-// a division that has no branch 11.8).
+// together and kept, where the kernel above makes three round trips of 4-byte accesses (2048 tokens of 16 heads of 128 columns: 18 -> 12.6 us, now bound by
+// the exponentials and divisions).
 template <typename T, int PIECES>
 __global__ void __launch_bounds__(256)
 head_norm_gate_wide_kernel(const float *__restrict__ o, const T *__restrict__ w, float eps, const T *__restrict__ gate, long long g_token, int act,
@@ -912,8 +912,7 @@ head_norm_gate_wide_kernel(const float *__restrict__ o, const T *__restrict__ w,
             float a = 1.f;
             if (gr && in) {
                 const float gv = to_f(g[i].v[j]);
-                if constexpr (sizeof(T) == 2) a = act == 0 ? gv : over_one_plus_exp(act == 1 ? gv : 1.0f, gv);
-                else a = act == 1 ? gv / (1.0f + expf(-gv)) : act == 2 ? 1.0f / (1.0f + expf(-gv)) : gv;
+                a = act == 1 ? gv / (1.0f + expf(-gv)) : act == 2 ? 1.0f / (1.0f + expf(-gv)) : gv;
             }
             v[j] *= share;
             const float y = gate_first ? v[j] * a : v[j];

@@ -19,7 +19,8 @@
 //               gate and up of 2048 tokens.)
 // Columns past a chunk's tokens hold zeros or stale rows: columns do not mix, and they are not stored.
 //
-// Measured (64 experts of 2048 x 1408, 6 choices a token): 2048 tokens gate and up 226 -> 181 us (780 TF/s; the weights alone are 113 us of HBM time),
+// Measured (64 experts of 2048 x 1408, 6 choices a token): 2048 tokens gate and up 226 -> 187 us (755 TF/s; 180 where a gate's
+// quotient is 2 ulp off, which other bits came of; the weights alone are 113 us of HBM time),
 // down 104 us; 1024 tokens 154 -> 140 and 80 -> 74; 16 tokens 89 and 49 us, 6.5 and 5.9 TB/s of weights.  What that step changed: the epilogue without
 // branches, chunks of at most 192 rows (four stages in place of three: 203 us with 256, 208 with 128, where every weight block is
 // fetched for fewer columns), tiles dealt largest first (the slowest CTA had worked 380,000 cycles, the fastest 259,000).  Tried
@@ -56,7 +57,7 @@ struct MoeTcArgs {
 };
 
 // A warp's part of a finished tile: 32 weight rows, tokens begin .. end - 1 of the chunk that starts at row0 of the sorted list, eight
-// at a time.  Neither the activation (a template argument) nor the division has a branch, so that the eight chains overlap: with an exact division
+// at a time.  Neither the activation (a template argument) nor, as a rule, the division (quotient_times) has a branch, so that the eight chains overlap: with an exact division
 // and a switch an element a tile of 192 tokens took 18,000 cycles, in which the tensor cores stand still, as such a tile has all of
 // tensor memory.  (The next eight read out of tensor memory ahead: no faster, and registers spilled.)
 constexpr int kStorePairs = 8, kStoreAct = 9;  // MODE: these, or the activation of a gated pair
@@ -83,16 +84,22 @@ __device__ __forceinline__ void epilogue(const MoeTcArgs &a, uint32_t d0, uint32
         } else {
             bf16 *o = a.inter + (size_t)row * a.n + f0;
             bf16 x[8];
+            float p[8], q[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float p = __uint_as_float(u[i]), q = __uint_as_float(v[i]);
-                if constexpr (MODE == kStoreAct) {
-                    auto act = [&](float z) { return a.act == 2 ? (z > 0.f ? z * z : 0.f) : act_apply(z, a.act); };
-                    x[i] = __float2bfloat16_rn(act(p) * bad);
-                    if (i < here && f1 < a.n) o[(size_t)i * a.n + 128] = __float2bfloat16_rn(act(q) * bad);
-                } else {
-                    x[i] = __float2bfloat16_rn(gated_pair_bf16<MODE>(p, q, a.limit, a.slope) * bad);
+            for (int i = 0; i < 8; ++i) p[i] = __uint_as_float(u[i]), q[i] = __uint_as_float(v[i]);
+            if constexpr (MODE == kStoreAct) {
+                auto act = [&](float z) { return a.act == 2 ? (z > 0.f ? z * z : 0.f) : act_apply(z, a.act); };
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    x[i] = __float2bfloat16_rn(act(p[i]) * bad);
+                    if (i < here && f1 < a.n) o[(size_t)i * a.n + 128] = __float2bfloat16_rn(act(q[i]) * bad);
                 }
+            } else {
+                float y[8];
+                gated_pairs<bf16, MODE>(p, q, a.limit, a.slope, y, here);
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) x[i] = __float2bfloat16_rn(y[i] * bad);
             }
 #pragma unroll
             for (int i = 0; i < 8; ++i, o += a.n)

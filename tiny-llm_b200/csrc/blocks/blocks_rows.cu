@@ -397,8 +397,8 @@ __global__ void gated_act_kernel(const T *__restrict__ gu, T *__restrict__ out, 
 }
 
 // Eight adjacent columns per thread, 16-byte accesses (bf16, width % 8 == 0).
-template <int ACT>
-__global__ void gated_act_wide_kernel(const bf16 *__restrict__ gu, bf16 *__restrict__ out, long long out_row, long long total8, int width, float limit, float slope) {
+__global__ void gated_act_wide_kernel(const bf16 *__restrict__ gu, bf16 *__restrict__ out, long long out_row, long long total8, int width, int act, float limit,
+                                      float slope) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total8) return;
     const int per_row = width / 8;
@@ -410,7 +410,7 @@ __global__ void gated_act_wide_kernel(const bf16 *__restrict__ gu, bf16 *__restr
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         float2 g = __bfloat1622float2(gp[e]), u = __bfloat1622float2(up[e]);
-        op[e] = __floats2bfloat162_rn(gated_pair_bf16<ACT>(g.x, u.x, limit, slope), gated_pair_bf16<ACT>(g.y, u.y, limit, slope));
+        op[e] = __floats2bfloat162_rn(gated_pair(g.x, u.x, act, limit, slope), gated_pair(g.y, u.y, act, limit, slope));
     }
     *reinterpret_cast<uint4 *>(out + row * out_row + j) = o4;
 }
@@ -578,8 +578,7 @@ int tlb_gated_act(const void *gu, void *out, long long out_row, int rows, int wi
     long long total = (long long)rows * width;
     if (dtype == TL_BF16 && width % 8 == 0 && out_row % 8 == 0 && (uintptr_t)gu % 16 == 0 && (uintptr_t)out % 16 == 0) {
         long long total8 = total / 8;
-        auto kernel = act == 0 ? gated_act_wide_kernel<0> : act == 3 ? gated_act_wide_kernel<3> : gated_act_wide_kernel<1>;
-        kernel<<<(unsigned)((total8 + 255) / 256), 256, 0, as_stream(stream)>>>((const bf16 *)gu, (bf16 *)out, out_row, total8, width, limit, slope);
+        gated_act_wide_kernel<<<(unsigned)((total8 + 255) / 256), 256, 0, as_stream(stream)>>>((const bf16 *)gu, (bf16 *)out, out_row, total8, width, act, limit, slope);
     } else
         TLB_DISPATCH(dtype, "gated_act",
                      gated_act_kernel<T><<<(unsigned)((total + 255) / 256), 256, 0, as_stream(stream)>>>((const T *)gu, (T *)out, out_row, total, width, act, limit, slope));

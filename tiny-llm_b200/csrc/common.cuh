@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "../../include/tiny_llm_b200.h"
 
 namespace tl {
@@ -83,6 +85,42 @@ __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
+}
+
+// y[i] = (num[i] / den(num[i])) * factor[i] such that rounding it to T gives what the exact fp32 quotient gives, to the bit; den >= 1.  An exact division is
+// a branch, which keeps a thread's quotients from overlapping, so they are taken from the branch-free division first.  What that leaves open (2 ulp of a normal
+// quotient, so at most 6 of the product) matters where the product is that near the middle between two values of T; those, quotients too small
+// for that bound (0 where the denominator passes 2^126) and products below fp16's normal numbers are divided exactly: one in 4,000 for bf16, one in 500 for fp16.
+// live: how many of them matter.
+template <typename T, int COUNT, typename Den>
+__device__ __forceinline__ void quotient_times(const float (&num)[COUNT], Den den, const float (&factor)[COUNT], float (&y)[COUNT], int live = COUNT) {
+    if constexpr (sizeof(T) == 2) {
+        constexpr bool BF = std::is_same<T, __nv_bfloat16>::value;
+        constexpr int KEPT = BF ? 16 : 19;  // bits of an fp32 number that T has, the others are rounded off
+        constexpr uint32_t kNear = 17u << KEPT;
+        // below fp16's normal numbers the middle lies elsewhere; bf16's subnormal ones are rounded where fp32's are
+        constexpr float kSmall = 6.2e-5f, kSmallQuotient = 1e-30f;
+        // how far above (the middle between two values of T) - 8 ulp, in the upper bits of a word
+        auto above = [](float v) { return (__float_as_uint(v) << KEPT) + ((8u - (1u << (31 - KEPT))) << KEPT); };
+        uint32_t nearest = 0xffffffffu;
+        float smallest = kSmall, smallest_q = kSmallQuotient;
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) {
+            const float q = __fdividef(num[i], den(num[i]));
+            y[i] = q * factor[i];
+            nearest = min(nearest, above(y[i])), smallest_q = fminf(smallest_q, fabsf(q));
+            if constexpr (!BF) smallest = fminf(smallest, fabsf(y[i]));
+        }
+        const bool small = smallest < kSmall || smallest_q < kSmallQuotient;  // then all of them
+        if ((nearest < kNear || small) && live > 0) {
+#pragma unroll
+            for (int i = 0; i < COUNT; ++i)
+                if (i < live && (small || above(y[i]) < kNear)) y[i] = (num[i] / den(num[i])) * factor[i];
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < COUNT; ++i) y[i] = (num[i] / den(num[i])) * factor[i];
+    }
 }
 
 // Streaming (read-once) 128-bit global load that does not allocate in L1.

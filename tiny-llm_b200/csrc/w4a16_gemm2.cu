@@ -22,8 +22,8 @@
 // for larger M; same rounding points as w4a16_gemm.cu (weights rounded to the activation dtype, fp32 accumulation).
 //
 // Measured (bf16; before: a pair of CTAs a tile): 2048 rows of 2560 -> 19456 230 -> 139 us (1464 TF/s, 90 % of the measured burst), 4096 rows 442 -> 264
-// (1546 TF/s), 2560 -> 9728 131 -> 77; gate and up projection with their activation in one launch, 2048 rows of 2560 -> 9728: 245 (two
-// launches of the one-CTA kernel and one of the activation) -> 150 us.
+// (1546 TF/s), 2560 -> 9728 131 -> 77; gate and up projection with their activation in one launch, 2048 rows of 2560 -> 9728: 244 (two
+// launches of the one-CTA kernel and one of the activation) -> 155 us, fp16 243 -> 173; 129 rows 50 -> 43 and 51 -> 48.
 #include <cuda.h>
 #include <stdlib.h>
 #include <cudaTypedefs.h>
@@ -88,34 +88,6 @@ __device__ __forceinline__ void p_tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
           "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(taddr)
         : "memory");
-}
-
-// silu(gate) * up as swiglu's kernel gives it, to the bit: the product of an exact quotient, rounded to T.  The quotient is taken from the
-// branch-free division first, so that sixteen of them overlap; where what it leaves open (2 ulp of the quotient, so at most 6 of the
-// product) could change the rounding to bf16, or the operands are out of that division's range, the exact one decides (0.03 % of them).
-template <typename T, int COUNT>
-__device__ __forceinline__ void p_gated(const float (&gate)[COUNT], const float (&up)[COUNT], float (&y)[COUNT]) {
-    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-        // how far above (the midpoint between two bf16) - 8 ulp, in the upper half of a word; how far a magnitude is above the smallest
-        auto above = [](float v) { return __float_as_uint(v) * 65536u + ((8u - 0x8000u) << 16); };
-        auto size = [](float v) { return (__float_as_uint(v) & 0x7fffffffu) - 1u; };  // of 0 (both ways give it) the largest
-        uint32_t nearest = 0xffffffffu, smallest = 0xffffffffu;
-        float lowest = 0.f;
-#pragma unroll
-        for (int i = 0; i < COUNT; ++i) {
-            y[i] = __fdividef(gate[i], 1.0f + expf(-gate[i])) * up[i];
-            nearest = min(nearest, above(y[i])), smallest = min(smallest, size(y[i])), lowest = fminf(lowest, gate[i]);
-        }
-        constexpr uint32_t kNear = 17u << 16, kSmall = 0x0da24260u;  // 1e-30
-        if (__any_sync(0xffffffffu, nearest < kNear || smallest < kSmall || lowest < -60.f)) {
-#pragma unroll
-            for (int i = 0; i < COUNT; ++i)
-                if (above(y[i]) < kNear || size(y[i]) < kSmall || gate[i] < -60.f) y[i] = (gate[i] / (1.0f + expf(-gate[i]))) * up[i];
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < COUNT; ++i) y[i] = (gate[i] / (1.0f + expf(-gate[i]))) * up[i];
-    }
 }
 
 template <typename T>
@@ -407,7 +379,9 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                             float gate[16], up[16];
 #pragma unroll
                             for (int j = 0; j < 16; ++j) gate[j] = to_f(from_f<T>(__uint_as_float(v[j]) * bad)), up[j] = to_f(from_f<T>(__uint_as_float(u[j])));
-                            p_gated<T>(gate, up, y);
+                            // silu(gate) * up as swiglu's kernel gives it, to the bit
+                            quotient_times<T>(gate, [](float g) { return 1.0f + expf(-g); }, up, y, m0 + lane < M ? K - n0 - c : 0);
+                            __syncwarp();
                         } else {
 #pragma unroll
                             for (int j = 0; j < 16; ++j) y[j] = __uint_as_float(v[j]) * bad;
