@@ -34,3 +34,12 @@ def test_nothing_of_the_predecessor_is_read_ahead(path, kernel, operands):
     ahead = body[: WAIT.search(body).start()]
     read = [name for name in operands.split() if re.search(r"\b" + name + r"\s*\[|\b(ld_cg|__ldg|ldg_stream)\(\s*" + name + r"\b|\*\s*" + name + r"\b", ahead)]
     assert not read, f"{kernel} reads {read} before griddep_wait()"
+
+
+def test_the_experts_sum_reads_through_l2():
+    """Its operands are the launch before's, or the other stream's joined right ahead of it: loads that the compiler may move ahead of the wait (plain ones,
+    of pointers that it takes for read-only) are not used."""
+    body = body_of("blocks/blocks_moe.cu", "moe_combine_kernel")
+    behind = body[WAIT.search(body).end() :]
+    plain = [name for name in ("pair_out", "gate", "shared", "shared_gate", "idx", "h") if re.search(r"\b" + name + r"\s*\[|moe_load<\w+>\(\s*" + name + r"\b", behind)]
+    assert not plain and "griddep_wait" not in behind

@@ -295,23 +295,31 @@ __global__ void moe_scale_rows_kernel(const T *__restrict__ h, const float *__re
 // choices and 2048 columns: 37 -> 22 us, 16 tokens: 13 -> 3 us; before, a column and a choice at a time).
 template <typename T, int W>
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const float *__restrict__ pair_out, const float *__restrict__ gate, const T *__restrict__ shared,
-                   const float *__restrict__ shared_gate, const int32_t *__restrict__ idx, int experts, const T *__restrict__ h, float *__restrict__ y, int top, int dim) {
+moe_combine_kernel(const float *pair_out, const float *gate, const T *shared, const float *shared_gate, const int32_t *idx, int experts, const T *h, float *__restrict__ y,
+                   int top, int dim) {
     const int t = blockIdx.x, d = (blockIdx.y * 256 + threadIdx.x) * W;
-    tl::griddep_wait();
+    tl::griddep_wait();  // all operands may be the launch before's: read by ld_cg, which stays behind it
     if (d >= dim) return;
     constexpr int AT_ONCE = 8;
     float s[W] = {};
+    T beside[W];
+    float beside_gate = 1.f;
+    if (shared) {
+        if (shared_gate) beside_gate = tl::ld_cg(shared_gate + t);
+#pragma unroll
+        for (int j = 0; j < W; ++j) beside[j] = tl::ld_cg(shared + (size_t)t * dim + d + j);
+    }
     for (int k0 = 0; k0 < top; k0 += AT_ONCE) {
-        float x[AT_ONCE][W];
+        float x[AT_ONCE][W], g[AT_ONCE];
 #pragma unroll
         for (int u = 0; u < AT_ONCE; ++u)
             if (k0 + u < top) {
                 const size_t pair = (size_t)t * top + k0 + u;
-                if (idx != nullptr && idx[pair] >= experts) {
+                g[u] = gate ? tl::ld_cg(gate + pair) : 1.f;
+                if (idx != nullptr && tl::ld_cg(idx + pair) >= experts) {
 #pragma unroll
-                    for (int j = 0; j < W; ++j) x[u][j] = to_f(h[(size_t)t * dim + d + j]);
-                } else if constexpr (W == 4) {  // ld_cg: not to be read ahead of the wait
+                    for (int j = 0; j < W; ++j) x[u][j] = to_f(tl::ld_cg(h + (size_t)t * dim + d + j));
+                } else if constexpr (W == 4) {
                     const uint4 v = tl::ld_cg(reinterpret_cast<const uint4 *>(pair_out + pair * dim + d));
                     x[u][0] = __uint_as_float(v.x), x[u][1] = __uint_as_float(v.y), x[u][2] = __uint_as_float(v.z), x[u][3] = __uint_as_float(v.w);
                 } else {
@@ -322,15 +330,13 @@ moe_combine_kernel(const float *__restrict__ pair_out, const float *__restrict__
 #pragma unroll
         for (int u = 0; u < AT_ONCE; ++u)
             if (k0 + u < top) {
-                const float g = gate ? gate[(size_t)t * top + k0 + u] : 1.f;
 #pragma unroll
-                for (int j = 0; j < W; ++j) s[j] = fmaf(g, x[u][j], s[j]);
+                for (int j = 0; j < W; ++j) s[j] = fmaf(g[u], x[u][j], s[j]);
             }
     }
     if (shared) {
-        const float g = shared_gate ? shared_gate[t] : 1.f;
 #pragma unroll
-        for (int j = 0; j < W; ++j) s[j] = fmaf(g, to_f(shared[(size_t)t * dim + d + j]), s[j]);
+        for (int j = 0; j < W; ++j) s[j] = fmaf(beside_gate, to_f(beside[j]), s[j]);
     }
     if constexpr (W == 4) *reinterpret_cast<float4 *>(y + (size_t)t * dim + d) = make_float4(s[0], s[1], s[2], s[3]);
     else y[(size_t)t * dim + d] = s[0];
