@@ -324,6 +324,10 @@ int tlb_moe_scale_rows(const void *h, const float *gate, void *out, int tokens, 
 /* pair_out[pair, :] = Wd[e] inter[row, :] (fp32); Wd [experts, dim, ff]. */
 int tlb_moe_down(const void *inter, const void *wd, int32_t *lists, int tokens, int top, int experts, int dim, int ff, float *pair_out, int dtype,
                  void *stream);
+/* The same as the launch right behind tlb_moe_gate_up or tlb_moe_up of the same lists on the same stream: it may read the lists and weights while that one
+ * still runs.  Behind anything else use tlb_moe_down. */
+int tlb_moe_down_next(const void *inter, const void *wd, int32_t *lists, int tokens, int top, int experts, int dim, int ff, float *pair_out, int dtype,
+                      void *stream);
 /* y[t,:] = sum_k gate[t,k] * pair_out[t*top+k,:] (+ shared_gate[t] * shared[t,:] if shared != NULL, stored in `dtype`; shared_gate
  * NULL: 1), fp32, in choice order;
  * gate == NULL: every weight is 1.  idx != NULL: a choice with idx[t,k] >= experts is an identity expert (the router has

@@ -34,3 +34,30 @@ def test_positions_written_by_the_launch_before(rows):
         return torch.stack(out), *slabs
 
     assert all(torch.equal(a, b) for a, b in zip(run(False), run(True)))
+
+
+def test_lists_made_by_the_launch_before():
+    """Experts' second product straight behind the sort of its lists, many times over lists of other routings: as when each launch is waited for."""
+    from extensions_b200.tiny_llm_ext_b200 import blocks
+
+    lib, tokens, top, experts, dim, ff = blocks.library(), 300, 3, 16, 256, 136
+    g = torch.Generator(device="cuda").manual_seed(1)
+    normal = lambda *shape: torch.randn(*shape, generator=g, device="cuda").to(BF16)  # noqa: E731
+    choices = [torch.rand(tokens, experts, generator=g, device="cuda").argsort(dim=1)[:, :top].to(torch.int32).contiguous() for _ in range(40)]
+    # rows all alike: an expert's pairs come in no particular order
+    inter, wd = normal(1, ff).repeat(int(lib.tlb_moe_max_rows(tokens, top, experts)), 1), normal(experts, dim, ff)
+    lists = torch.zeros(int(lib.tlb_moe_lists_ints(tokens, top, experts)), dtype=torch.int32, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def run(waiting):
+        out = [torch.zeros(tokens * top, dim, device="cuda") for _ in choices]
+        for idx, y in zip(choices, out):
+            assert lib.tlb_moe_sort(idx.data_ptr(), tokens, top, experts, lists.data_ptr(), stream) == 0
+            if waiting:
+                torch.cuda.synchronize()
+            assert lib.tlb_moe_down(inter.data_ptr(), wd.data_ptr(), lists.data_ptr(), tokens, top, experts, dim, ff, y.data_ptr(), 2, stream) == 0
+            if waiting:
+                torch.cuda.synchronize()
+        return torch.stack(out)
+
+    assert torch.equal(run(False), run(True))

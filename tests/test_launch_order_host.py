@@ -43,3 +43,14 @@ def test_the_experts_sum_reads_through_l2():
     behind = body[WAIT.search(body).end() :]
     plain = [name for name in ("pair_out", "gate", "shared", "shared_gate", "idx", "h") if re.search(r"\b" + name + r"\s*\[|moe_load<\w+>\(\s*" + name + r"\b", behind)]
     assert not plain and "griddep_wait" not in behind
+
+
+def test_lists_are_read_ahead_only_where_the_caller_says_what_is_before():
+    """The experts' second product reads the lists before its wait behind a first product of theirs, and nowhere else."""
+    kernel = body_of("blocks/blocks_moe_tc.cu", "moe_tc_kernel")
+    first_read = re.search(r"a\.(counters|chunks|sorted_pair)\b", kernel).start()
+    assert re.search(r"if \(!a\.second\) \{\s*tl::griddep_wait\(\);", kernel[:first_read])
+    assert re.search(r"a\.second = p\.second;", body_of("blocks/blocks_moe_tc.cu", "moe_tc_product"))
+    assert "stream, false)" in body_of("blocks/blocks_moe.cu", "tlb_moe_down")
+    for entry in ("tlb_moe_gate_up", "tlb_moe_up"):
+        assert "true" not in body_of("blocks/blocks_moe.cu", entry)

@@ -434,11 +434,18 @@ int tlb_moe_scale_rows(const void *h, const float *gate, void *out, int tokens, 
     return TL_OK;
 }
 
-int tlb_moe_down(const void *inter, const void *wd, int32_t *lists, int tokens, int top, int experts, int dim, int ff, float *pair_out, int dtype, void *stream) {
+static int moe_down(const void *inter, const void *wd, int32_t *lists, int tokens, int top, int experts, int dim, int ff, float *pair_out, int dtype, void *stream,
+                    bool second) {
     if (tokens <= 0) return TL_OK;
     if (!inter || !wd || !lists || !pair_out || experts <= 0 || dim <= 0 || ff <= 0 || top <= 0) return tl::fail(TL_EINVAL, "moe_down: bad argument");
-    return moe_product("moe_down", {inter, wd, nullptr, moe_lists(lists, tokens, top, experts), tokens, top, experts, ff, dim, 0, kGatherSorted, 0.f, 1.f, nullptr, pair_out},
+    return moe_product("moe_down", {inter, wd, nullptr, moe_lists(lists, tokens, top, experts), tokens, top, experts, ff, dim, 0, kGatherSorted, 0.f, 1.f, nullptr, pair_out, second},
                        dtype, as_stream(stream));
+}
+int tlb_moe_down(const void *inter, const void *wd, int32_t *lists, int tokens, int top, int experts, int dim, int ff, float *pair_out, int dtype, void *stream) {
+    return moe_down(inter, wd, lists, tokens, top, experts, dim, ff, pair_out, dtype, stream, false);
+}
+int tlb_moe_down_next(const void *inter, const void *wd, int32_t *lists, int tokens, int top, int experts, int dim, int ff, float *pair_out, int dtype, void *stream) {
+    return moe_down(inter, wd, lists, tokens, top, experts, dim, ff, pair_out, dtype, stream, true);
 }
 
 int tlb_moe_combine(const float *pair_out, const float *gate, const void *shared, const float *shared_gate, const int32_t *idx, int experts, const void *h, float *y, int tokens,

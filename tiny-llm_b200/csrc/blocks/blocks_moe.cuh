@@ -10,9 +10,9 @@
 namespace tlb {
 
 // The experts' launches follow one another closely: sort, gate|up, down and sum may each become resident while the one before is ending, and wait
-// (griddep_wait, in every CTA, before anything of it is read or overwritten).  Only gate|up lets its successor in early, once the sort is complete: the down
-// product then reads the lists and fills its ring with weights on every SM whose gate|up CTA is done, and waits for the rows alone.  (The sort lets nothing
-// in, so that lists read ahead of a wait are whole whatever follows it.)  16 tokens, 6 of 64 experts of 1408 x 2048: 189 -> 178 us the call; 2048 tokens 472 -> 469.
+// (griddep_wait, in every CTA, before anything of it is read or overwritten).  Only gate|up lets its successor in early, behind its own wait for the sort: a
+// down product that says that it follows one (tlb_moe_down_next) reads the lists ahead of its wait and fills its ring with weights on every SM whose gate|up
+// CTA is done, and waits for the rows alone.  Any other waits before it reads the lists, which may be the launch before's.  16 tokens, 6 of 64 experts of 1408 x 2048: 189 -> 178 us the call; 2048 tokens 472 -> 469.
 template <typename... P, typename... A>
 static inline cudaError_t moe_launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A &&...a) {
     static const bool chained = [] { const char *e = getenv("TL_PDL"); return !e || atoi(e) != 0; }();
@@ -65,6 +65,7 @@ struct MoeProduct {
     float limit, slope;
     void *inter;
     float *pair_out;
+    bool second = false;  // the launch before is the first product of these lists, which let this one in only once they were whole
 };
 
 bool moe_tc_ok(int dtype, int K, const void *x, const void *w0, const void *w1);

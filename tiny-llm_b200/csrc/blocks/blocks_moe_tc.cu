@@ -53,7 +53,7 @@ struct MoeTcArgs {
     float *pair_out;
     int stages, stage_bytes;
     int turning;  // 1: tiles of different sizes: dealt forth and back
-    int second;   // 1: the launch before this one is a product too, and the lists are older than both
+    int second;   // 1: the launch before this one is the first product of the same lists, which are older than both
 };
 
 // A warp's part of a finished tile: 32 weight rows, tokens begin .. end - 1 of the chunk that starts at row0 of the sorted list, eight
@@ -318,7 +318,7 @@ int moe_tc_product(const MoeProduct &p, cudaStream_t st) {
     a.stage_bytes = 2 * kTcBlockBytes + moe_chunk_rows(p.tokens) * 128;
     a.stages = std::min(kTcMaxStages, (227 * 1024 - kTcBars) / a.stage_bytes);
     a.turning = moe_chunk_rows(p.tokens) > 16;
-    a.second = a.epilogue == kEpiPairs;
+    a.second = p.second;
     a.m_blocks = ceil_div(p.N, a.epilogue == kEpiGated ? 128 : 256);
     // the largest that any call asks for; on every call, because the attribute belongs to the device that is current
     if (cudaFuncSetAttribute(moe_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {

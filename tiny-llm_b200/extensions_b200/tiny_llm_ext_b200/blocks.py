@@ -86,6 +86,7 @@ _SIGNATURES = {
     "tlb_moe_sort": (_I, [_VP, _I, _I, _I, _VP, _VP]),
     "tlb_moe_gate_up": (_I, [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _F, _F, _VP, _I, _VP]),
     "tlb_moe_down": (_I, [_VP, _VP, _VP, _I, _I, _I, _I, _I, _VP, _I, _VP]),
+    "tlb_moe_down_next": (_I, [_VP, _VP, _VP, _I, _I, _I, _I, _I, _VP, _I, _VP]),
     "tlb_tc_gave_up": (_LL, []),
     "tlb_moe_combine": (_I, [_VP, _VP, _VP, _VP, _VP, _I, _VP, _VP, _I, _I, _I, _I, _VP]),
     "tlb_argmax_rows": (_I, [_VP, _VP, _I, _I, _VP]),
@@ -465,7 +466,7 @@ def moe_experts(h, idx, gate, w_gate, w_up, w_down, act: int, shared=None, scale
         _check(lib.tlb_moe_gate_up(_ptr(h), _ptr(w_gate), _ptr(w_up), _ptr(lists), T, top, E, D, ff, act, float(limit), float(slope), _ptr(inter), code, st))
     else:
         _check(lib.tlb_moe_up(_ptr(rows_in), _ptr(w_up), _ptr(lists), T, top, E, D, ff, act, per_pair, _ptr(inter), code, st))
-    _check(lib.tlb_moe_down(_ptr(inter), _ptr(w_down), _ptr(lists), T, top, E, D, ff, _ptr(pair_out), code, st))
+    _check(lib.tlb_moe_down_next(_ptr(inter), _ptr(w_down), _ptr(lists), T, top, E, D, ff, _ptr(pair_out), code, st))
     if before_sum is not None:
         before_sum()
     if into is not None:
