@@ -26,6 +26,8 @@ extern "C" {
 #endif
 
 int tlb_abi_version(void);
+/* Programmatic dependent launch for the experts' launches (on by default; 0 turns it off, TL_PDL=0 in the environment does the same). */
+int tlb_set_pdl(int enabled);
 const char *tlb_last_error(void);
 long long tlb_launch_count(void);
 

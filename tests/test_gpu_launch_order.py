@@ -61,3 +61,20 @@ def test_lists_made_by_the_launch_before():
         return torch.stack(out)
 
     assert torch.equal(run(False), run(True))
+
+
+def test_experts_with_the_switch_off():
+    """``set_pdl(False)`` reaches the experts' launches; the same bits either way."""
+    from extensions_b200.tiny_llm_ext_b200 import blocks
+
+    g = torch.Generator(device="cuda").manual_seed(2)
+    normal = lambda *shape: (torch.randn(*shape, generator=g, device="cuda") * shape[-1] ** -0.5).to(BF16)  # noqa: E731
+    h, wg, wu, wd = normal(90, 256) * 16, normal(8, 136, 256), normal(8, 136, 256), normal(8, 256, 136)
+    idx = torch.rand(90, 8, generator=g, device="cuda").argsort(dim=1)[:, :2].to(torch.int32).contiguous()
+    weight = torch.rand(90, 2, generator=g, device="cuda")
+    want = blocks.moe_experts(h, idx, weight, wg, wu, wd, blocks.ACT_SILU)
+    try:
+        ext.set_pdl(False)
+        assert torch.equal(blocks.moe_experts(h, idx, weight, wg, wu, wd, blocks.ACT_SILU), want)
+    finally:
+        ext.set_pdl(True)

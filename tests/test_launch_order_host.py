@@ -54,3 +54,33 @@ def test_lists_are_read_ahead_only_where_the_caller_says_what_is_before():
     assert "stream, false)" in body_of("blocks/blocks_moe.cu", "tlb_moe_down")
     for entry in ("tlb_moe_gate_up", "tlb_moe_up"):
         assert "true" not in body_of("blocks/blocks_moe.cu", entry)
+
+
+@pytest.mark.parametrize("loaded_before", [True, False])
+def test_one_switch_for_both_libraries(monkeypatch, loaded_before):
+    """``set_pdl`` reaches the blocks library whether it was loaded before the call or after it."""
+    from extensions_b200 import tiny_llm_ext_b200 as ext
+    from extensions_b200.tiny_llm_ext_b200 import blocks
+
+    asked, real = [], ext.ctypes.CDLL
+
+    class Library:
+        def __init__(self, path):
+            self.real = real(path)
+
+        def __getattr__(self, name):
+            return asked.append if name == "tlb_set_pdl" else getattr(self.real, name)
+
+    monkeypatch.setattr(blocks, "_lib", None)
+    monkeypatch.setattr(blocks, "_pdl", None)
+    monkeypatch.setattr(blocks.ctypes, "CDLL", Library)
+    monkeypatch.setattr(blocks, "_SIGNATURES", {k: v for k, v in blocks._SIGNATURES.items() if k != "tlb_set_pdl"})
+    try:
+        if loaded_before:
+            blocks.load_library()
+        ext.set_pdl(False)
+        if not loaded_before:
+            blocks.load_library()
+        assert asked == [0]
+    finally:
+        ext.set_pdl(True)

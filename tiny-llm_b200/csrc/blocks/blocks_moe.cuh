@@ -3,8 +3,6 @@
 
 #include <algorithm>
 
-#include <stdlib.h>
-
 #include "blocks_common.cuh"
 
 namespace tlb {
@@ -15,14 +13,7 @@ namespace tlb {
 // CTA is done, and waits for the rows alone.  Any other waits before it reads the lists, which may be the launch before's.  16 tokens, 6 of 64 experts of 1408 x 2048: 189 -> 178 us the call; 2048 tokens 472 -> 469.
 template <typename... P, typename... A>
 static inline cudaError_t moe_launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A &&...a) {
-    static const bool chained = [] { const char *e = getenv("TL_PDL"); return !e || atoi(e) != 0; }();
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem, cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr, cfg.numAttrs = chained ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(a)...);
+    return tl::launch_chained(kernel, grid, dim3(threads), smem, st, static_cast<P>(a)...);
 }
 
 // Which rows of its operand a tile's rows read: the sorted rows themselves (the second product), the token of the pair, or the pair.

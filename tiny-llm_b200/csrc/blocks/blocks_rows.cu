@@ -2,6 +2,7 @@
 // positions, latent cache append, gated activations, arg-max; and the library's error / launch bookkeeping.
 #include <stdarg.h>
 #include <stdio.h>
+#include <stdlib.h>
 
 #include <atomic>
 #include <initializer_list>
@@ -26,7 +27,12 @@ int check_launch(const char *what) {
     return fail(TL_ECUDA, "%s: kernel launch failed: %s", what, cudaGetErrorString(e));
 }
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
-bool use_pdl() { return false; }
+static bool pdl_default() {
+    const char *e = getenv("TL_PDL");
+    return !(e != nullptr && e[0] == '0');
+}
+static std::atomic<bool> g_use_pdl{pdl_default()};
+bool use_pdl() { return g_use_pdl.load(std::memory_order_relaxed); }
 }  // namespace tl
 
 namespace tlb {
@@ -452,7 +458,11 @@ using namespace tlb;
 
 extern "C" {
 
-int tlb_abi_version(void) { return 9; }
+int tlb_abi_version(void) { return 10; }
+int tlb_set_pdl(int enabled) {
+    tl::g_use_pdl.store(enabled != 0, std::memory_order_relaxed);
+    return TL_OK;
+}
 const char *tlb_last_error(void) { return tl::g_error; }
 long long tlb_launch_count(void) { return tl::g_launches.load(std::memory_order_relaxed); }
 

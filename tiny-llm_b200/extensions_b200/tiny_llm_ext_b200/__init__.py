@@ -965,8 +965,11 @@ class DecodeStep:
 
 
 def set_pdl(enabled: bool) -> None:
-    """Programmatic dependent launch for the weight-streaming kernels."""
+    """Programmatic dependent launch, in this library and in ``blocks``."""
+    from . import blocks
+
     _check(_lib.tl_set_pdl(int(bool(enabled))))
+    blocks.set_pdl(enabled)
 
 
 def set_gemm_pairs(mode: int) -> None:

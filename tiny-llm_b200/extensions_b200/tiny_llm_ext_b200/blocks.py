@@ -17,11 +17,13 @@ import torch
 _HERE = Path(__file__).resolve().parent
 _LIB_NAME = "libtiny_llm_b200_blocks.so"
 _lib = None
+_pdl = None  # what set_pdl asked for, if it was called
 
 _VP, _I, _F, _D, _LL = ctypes.c_void_p, ctypes.c_int, ctypes.c_float, ctypes.c_double, ctypes.c_longlong
 
 _SIGNATURES = {
     "tlb_abi_version": (_I, []),
+    "tlb_set_pdl": (_I, [_I]),
     "tlb_last_error": (ctypes.c_char_p, []),
     "tlb_launch_count": (_LL, []),
     "tlb_embed_rows": (_I, [_VP, _VP, _VP, _VP, _I, _I, _I, _I, _VP]),
@@ -93,7 +95,7 @@ _SIGNATURES = {
 }
 EXPORTED_SYMBOLS = tuple(_SIGNATURES)
 
-ABI_VERSION = 9
+ABI_VERSION = 10
 ATTENTION_TILE_TOKENS = 4
 ACT_SILU, ACT_GELU_TANH, ACT_RELU_SQUARED, ACT_CLAMPED_SWISH, ACT_TANH = 0, 1, 2, 3, 4
 WEIGHTS_SOFTMAX, WEIGHTS_SIGMOID = 0, 1
@@ -139,7 +141,17 @@ def load_library(path: str | os.PathLike | None = None) -> None:
         fn = getattr(lib, name)
         fn.restype = restype
         fn.argtypes = argtypes
+    if _pdl is not None:
+        lib.tlb_set_pdl(int(_pdl))
     _lib = lib
+
+
+def set_pdl(enabled: bool) -> None:
+    """Programmatic dependent launch for the experts' launches; also before the library is loaded."""
+    global _pdl
+    _pdl = bool(enabled)
+    if _lib is not None:
+        _lib.tlb_set_pdl(int(_pdl))
 
 
 def library():
