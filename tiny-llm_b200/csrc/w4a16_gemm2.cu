@@ -450,7 +450,7 @@ void trace_bind_gemm2(unsigned long long *buf, unsigned int *n, unsigned int cap
 #endif
 
 // ---------------------------------------------------------------- host side --
-// Mode: 0 = never, 1 = where the pair grid fills the SMs (default), 2 = every M > 256 (tests, A/B runs).  TL_GEMM2 sets
+// Mode: 0 = never, 1 = where they take less time (default), 2 = every M > 256 (tests, A/B runs).  TL_GEMM2 sets
 // the initial value, tl_set_gemm_pairs() changes it.
 static int pairs_default() {
     const char *e = getenv("TL_GEMM2");
@@ -468,17 +468,18 @@ static PairPlan pair_plan(int M, int K, int features, int units) {
     return p;
 }
 
-// The pairs where their rounds of tiles cost less than the one-CTA kernel's waves, in that kernel's unit (w4a16_gemm.cu).  A round of whole tiles
-// is 1100 a block, of single ones 700; of reductions above 4096 a whole round takes 1750 (two rounds of 9728: 0.62 us a block each).  Measured over
-// 63 sizes of 300 to 4096 rows the choice is within 2 % of the better one; us, one-CTA kernel / pairs: 2560 -> 9728 300 rows 42 / 34, 2048 105 / 77,
-// 4096 211 / 140; 2560 -> 6144 300 rows 23.8 / 24.2, 700 29.8 / 33.9, 2048 70 / 51; 9728 -> 2560 700 rows 69 / 72, 3000 167 / 110, 4096 183 / 197.
+// The pairs where their rounds of tiles cost less than the one-CTA kernel's waves, in that kernel's unit (w4a16_gemm.cu).  A round of whole tiles is 1100 a
+// block, of single ones 700; of reductions above 4096 a whole round takes 1500 (0.69 us a block of 9728, 0.73 of 12288), above 16384 a single one
+// 1100 (0.52 us).  Measured over 260 sizes (13 matrices, 260 to 8192 rows) the choice is 0.3 % from the better one in the mean and 7 % at most; us, one-CTA kernel /
+// pairs: 2560 -> 9728 300 rows 39 / 31, 2048 103 / 75, 4096 208 / 135; 9728 -> 2560 700 rows 66 / 68, 3000 167 / 105, 4096 181 / 186, 6144 296 / 215;
+// 18944 -> 3584 800 rows 142 / 151, 2048 340 / 195, 4096 537 / 397.
 bool w4a16_gemm2_supported(int M, int N, int K, int dtype) {
     if (g_pairs_mode <= 0 || !(dtype == TL_BF16 || dtype == TL_F16) || M <= 256 || K <= 0 || N % 128 != 0) return false;
     if (g_pairs_mode >= 2) return true;
     const int units = sm_count() / 2;
     const PairPlan p = pair_plan(M, K, 2 * P_ROWS, units);
     const long long whole = ceil_div(p.full, units), single = ceil_div(p.items - p.full, units);
-    return whole * (N > 4096 ? 1750 : 1100) + single * 700 < w4a16_gemm_cost(M, N, K);
+    return whole * (N > 4096 ? 1500 : 1100) + single * (N > 16384 ? 1100 : 700) < w4a16_gemm_cost(M, N, K);
 }
 
 template <typename T>
@@ -547,6 +548,8 @@ int launch_w4a16_gemm2(const void *scales, const void *biases, const void *a, co
     return fail(TL_EDTYPE, "quantized_matmul: scales must be float16 or bfloat16");
 }
 
+// No comparison here: one launch of pairs took less time than two products and their activation at all of 210 sizes (129 to 4096 rows, 7 matrices, both types);
+// the least, fp16 of 129 rows of 2560 -> 9728 51 -> 48 us and bf16 of 2048 rows of 9728 -> 2560 192 -> 173, the most, 129 rows of 3072 -> 1024 48 -> 26.
 bool launch_w4a16_gemm2_gated(const tl_packed_matrix &gate, const tl_packed_matrix &up, const void *a, void *out, int M, int N, int K, int dtype, cudaStream_t st, int *rc) {
     if (g_pairs_mode <= 0 || M <= 128 || !(dtype == TL_BF16 || dtype == TL_F16) || N % 128 != 0) return false;
     if (dtype == TL_BF16)
