@@ -141,13 +141,13 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 #if TL_TRACE
     // per-block cycle stamps of the leader CTA's first tile (tools/gemm_blocks.py): role 0 = MMA warp (k: stage complete in both
     // CTAs, -, MMAs issued), role 1 = first dequantiser warp (k: loop top, math done, stage free, handed over)
-    __shared__ unsigned long long trc[2][40][4];
-#define P_TRC(role, i, k)                                                                                                    \
+    __shared__ unsigned int trc[2][40][4];  // (of 64 bits it would not fit beside the stages)
+#define P_TRC(role, item, i, k)                                                                                              \
     do {                                                                                                                     \
-        if (blockIdx.x == 0 && it == 0 && (threadIdx.x & 31) == 0 && (i) < 40) trc[role][i][k] = clock64();                 \
+        if (blockIdx.x == 0 && (item) == 0 && (threadIdx.x & 31) == 0 && (i) < 40) trc[role][i][k] = static_cast<unsigned int>(clock64()); \
     } while (0)
 #else
-#define P_TRC(role, i, k) do { } while (0)
+#define P_TRC(role, item, i, k) do { } while (0)
 #endif
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = static_cast<int>(p_cta_rank());       // 0 = leader (issues the MMAs)
@@ -229,15 +229,15 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             e_ph[0] ^= 1u;
             for (int kb = 0; kb < head; ++kb) {
                 if (!tc_wait(full + 8 * s, ph, dead)) goto done;
-                P_TRC(0, kb, 0);
-                P_TRC(0, kb, 1);
+                P_TRC(0, it, kb, 0);
+                P_TRC(0, it, kb, 1);
                 g_tc_fence_after();
                 if (g_elect_one()) {
                     products(s, 0, kb);
                     if (item.mt == 1) p_tc_commit2(empty + 8 * s);
                 }
                 __syncwarp();
-                P_TRC(0, kb, 2);
+                P_TRC(0, it, kb, 2);
                 if (++s == P_STAGES) s = 0, ph ^= 1u;
             }
             if (item.mt > 1) {
@@ -254,8 +254,8 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             }
             for (int kb = head; kb < num_kb; ++kb) {
                 if (!tc_wait(full + 8 * s, ph, dead)) goto done;
-                P_TRC(0, kb, 0);
-                P_TRC(0, kb, 1);
+                P_TRC(0, it, kb, 0);
+                P_TRC(0, it, kb, 1);
                 g_tc_fence_after();
                 if (g_elect_one()) {
                     products(s, 0, kb);
@@ -264,7 +264,7 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                     p_tc_commit2(empty + 8 * s);
                 }
                 __syncwarp();
-                P_TRC(0, kb, 2);
+                P_TRC(0, it, kb, 2);
                 if (++s == P_STAGES) s = 0, ph ^= 1u;
             }
             if (g_elect_one()) {
@@ -321,6 +321,7 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 if (it < plan.items) fetch();
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
+                    if (warp == 4) P_TRC(1, mine, 2 * group + u, 0);
                     uint32_t outw[16];
                     const uint32_t wv[4] = {cur[u].x, cur[u].y, cur[u].z, cur[u].w};
 #pragma unroll
@@ -335,7 +336,9 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                             outw[4 * j + q] = *reinterpret_cast<const uint32_t *>(&v);
                         }
                     }
+                    if (warp == 4) P_TRC(1, mine, 2 * group + u, 1);
                     if (!tc_wait(empty + 8 * s, ph, dead)) goto done;
+                    if (warp == 4) P_TRC(1, mine, 2 * group + u, 2);
                     unsigned char *tile = psm + s * P_STAGE + P_A_STAGE + row * 128;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
@@ -345,6 +348,7 @@ w4a16_gemm2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                     g_fence_proxy_async();  // generic-proxy stores -> visible to the tensor cores' async proxy (of both SMs)
                     __syncwarp();
                     if (lane == 0) g_mbar_arrive(full + 8 * s);
+                    if (warp == 4) P_TRC(1, mine, 2 * group + u, 3);
                     if (++s == P_STAGES) s = 0, ph ^= 1u;
                 }
             }
@@ -436,7 +440,7 @@ done:  // also from a role whose wait gave up
     if (blockIdx.x == 0 && g_trace_buf != nullptr) {  // tag = 20000 + role * 1000 + block * 4 + k (as w4a16_gemm.cu)
         for (int e = threadIdx.x; e < 2 * 40 * 4; e += P_THREADS) {
             const int role = e / 160, rest = e - role * 160;
-            if (rest / 4 < num_kb && role == 0 && (rest & 3) != 3) {
+            if (rest / 4 < num_kb && (role == 1 || (rest & 3) != 3)) {
                 const unsigned at = atomicAdd(g_trace_n, 1u);
                 if (at < g_trace_cap) g_trace_buf[2 * at] = 20000 + role * 1000 + rest, g_trace_buf[2 * at + 1] = trc[role][rest / 4][rest & 3];
             }
