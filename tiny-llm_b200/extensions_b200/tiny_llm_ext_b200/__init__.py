@@ -671,7 +671,12 @@ def quantized_matmul_fused(scales, biases, b, p0, p1=None, residual=None, prolog
 
 
 def paged_metadata_clean(context_lens, block_table, page_size: int, physical_pages: int, query_length: int) -> bool:
-    """Whether host copies (contiguous int32 numpy arrays ``[B]`` and ``[B, max_pages]``) of a paged call's metadata pass all of its checks."""
+    """Whether host copies (contiguous int32 numpy arrays ``[B]`` and ``[B, max_pages]``) of a paged call's metadata pass all of its checks.
+    Arrays of other types, layouts or shapes do not: nothing of them is read."""
+    if block_table.ndim != 2 or context_lens.shape != block_table.shape[:1]:
+        return False
+    if any(str(x.dtype) != "int32" or not x.flags.c_contiguous for x in (context_lens, block_table)):
+        return False
     return bool(_lib.tl_paged_metadata_clean(context_lens.ctypes.data, block_table.ctypes.data, block_table.shape[0], block_table.shape[1], page_size,
                                              physical_pages, query_length))
 

@@ -88,9 +88,8 @@ def _raise_first_metadata_error(ctx_rows, table_rows, page_size, max_pages, num_
 def validate_paged_metadata(ctx: np.ndarray, table: np.ndarray, page_size: int, num_physical_pages: int, L: int) -> None:
     """Integer validation of the paged metadata: one native pass over int32 arrays, the reference's exact error
     on failure (other integer types: vectorised here)."""
-    if ctx.dtype == np.int32 and table.dtype == np.int32 and ctx.flags.c_contiguous and table.flags.c_contiguous:
-        if tiny_llm_ext_b200.paged_metadata_clean(ctx, table, page_size, num_physical_pages, L):
-            return
+    if tiny_llm_ext_b200.paged_metadata_clean(ctx, table, page_size, num_physical_pages, L):
+        return
     max_pages = table.shape[1]
     ctx64 = ctx.astype(np.int64)
     live_pages = (ctx64 + page_size - 1) // page_size
