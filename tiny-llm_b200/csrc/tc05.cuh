@@ -1,5 +1,5 @@
 // tcgen05 / TMEM / TMA / mbarrier primitives shared by the tensor-core kernels (w4a16_gemm.cu,
-// attention_prefill_tc.cu).  Raw PTX for sm_100a; see /opt/skills/guides/blackwell_cuda_programming.md.
+// attention_prefill_tc.cu).  Raw PTX for sm_100a.
 #pragma once
 
 #include <cuda.h>

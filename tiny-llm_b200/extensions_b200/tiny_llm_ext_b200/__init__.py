@@ -675,8 +675,9 @@ def paged_metadata_clean(context_lens, block_table, page_size: int, physical_pag
     Arrays of other types, layouts or shapes do not: nothing of them is read."""
     if block_table.ndim != 2 or context_lens.shape != block_table.shape[:1]:
         return False
-    if any(str(x.dtype) != "int32" or not x.flags.c_contiguous for x in (context_lens, block_table)):
-        return False
+    for x in (context_lens, block_table):
+        if x.dtype.kind != "i" or x.dtype.itemsize != 4 or not x.dtype.isnative or not x.flags.c_contiguous:
+            return False
     return bool(_lib.tl_paged_metadata_clean(context_lens.ctypes.data, block_table.ctypes.data, block_table.shape[0], block_table.shape[1], page_size,
                                              physical_pages, query_length))
 
