@@ -91,7 +91,7 @@ def measured_peaks() -> dict:
         return {"hbm_gbs": float(data["hbm_gbs"]), "bf16_tflops": float(data.get("bf16_tflops", 1682.0)),
                 "bf16_tflops_sustained": float(data.get("bf16_tflops_sustained", data.get("bf16_tflops", 1442.5))),
                 "source": "MEASURED_PEAKS.json"}
-    return {"hbm_gbs": 6650.0, "bf16_tflops": 1680.0, "bf16_tflops_sustained": 1440.0, "source": "fallback (B200_PROFILING.md)"}
+    return {"hbm_gbs": 6650.0, "bf16_tflops": 1680.0, "bf16_tflops_sustained": 1440.0, "source": "fallback (an earlier measurement)"}
 
 
 def committed_traffic(kernel: str):

@@ -133,7 +133,9 @@ int tl_paged_cache_update(void *pages, const void *values, int num_pages, int he
 /* q,out [B*Hq, L, D]; pages [P, Hkv, page, D]; block_table int32 [B, max_pages]
  * (-1 padded); context_lens int32 [B] (post-append).  D <= 128; the tensor-core
  * prefill branch (L > 8, bf16) requires D == 128.  Rows that see no key are
- * written as zeros.  Workspace holds split-KV partials for the decode branch. */
+ * written as zeros.  Workspace holds split-KV partials for the decode branch.  block_table and context_lens are inputs of a step: with
+ * programmatic dependent launch (tl_set_pdl) they are read ahead of the wait for the launch before, so they must not be what that launch writes.  This
+ * holds for the other attention calls too; the append calls read theirs behind the wait. */
 size_t tl_paged_attention_workspace(int rows, int L, int D, int num_kv_heads, int num_heads, int dtype);
 int tl_paged_attention(const void *q, const void *key_pages, const void *value_pages, const int32_t *block_table,
                        const int32_t *context_lens, void *out, int rows, int L, int D, int num_pages,

@@ -19,8 +19,8 @@
 //               gate and up of 2048 tokens.)
 // Columns past a chunk's tokens hold zeros or stale rows: columns do not mix, and they are not stored.
 //
-// Measured (64 experts of 2048 x 1408, 6 choices a token): 2048 tokens gate and up 226 -> 187 us (755 TF/s; 180 where a gate's
-// quotient is 2 ulp off, which other bits came of; the weights alone are 113 us of HBM time),
+// Measured (64 experts of 2048 x 1408, 6 choices a token): 2048 tokens gate and up 226 -> 187 us (755 TF/s; 180 with quotients
+// 2 ulp off throughout, which gives other bits; the weights alone are 113 us of HBM time),
 // down 104 us; 1024 tokens 154 -> 140 and 80 -> 74; 16 tokens 89 and 49 us, 6.5 and 5.9 TB/s of weights.  What that step changed: the epilogue without
 // branches, chunks of at most 192 rows (four stages in place of three: 203 us with 256, 208 with 128, where every weight block is
 // fetched for fewer columns), tiles dealt largest first (the slowest CTA had worked 380,000 cycles, the fastest 259,000).  Tried

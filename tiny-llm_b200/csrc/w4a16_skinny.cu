@@ -518,7 +518,8 @@ __global__ void __launch_bounds__(128) w4a16_skinny_reduce4_kernel(const float *
 // down -> next layer's input norm): a cluster of SK_NORM_CTAS CTAs per token row adds the planes, adds the residual, writes the residual
 // stream and - the row being complete in the cluster's registers - the normalised row too (week2_kernels.metal:41-47 arithmetic:
 // T(x * rsqrt(mean(x^2) + eps) * w) on the ROUNDED residual sum).  Saves the rms_norm launch and its read of the row.  What bounds it is round trips:
-// with one CTA a row each thread waited for ceil(splits / 4) of them, now for ceil(splits / 8), and a decoding batch's rows fill the chip.
+// with one CTA a row each thread waited for ceil(splits / 4) of them, now for ceil(splits / 8), and a decoding batch's rows fill the chip (16 steps of 24
+// requests, eight 4B layers 11.91 -> 11.71 ms).
 // The sum of squares is that of ONE CTA of 256 threads, to the bit: thread t of it adds columns t, t + 256, .. in turn, then come its warps and their sums.
 // CTA `rank` has the columns of threads 64 rank .. 64 rank + 63, four threads a chain for the loads, and its first two warps add the chains.
 constexpr int SK_NORM_CTAS = 4, SK_NORM_PER = 4, SK_NORM_COLS = 256 / SK_NORM_CTAS;  // elements per thread: K <= 4096

@@ -28,7 +28,7 @@ def peak_gbs() -> float:
     path = ROOT / "MEASURED_PEAKS.json"
     if path.exists():
         return float(json.loads(path.read_text())["hbm_gbs"])
-    return 6650.0  # fallback stated in B200_PROFILING.md
+    return 6650.0  # fallback: an earlier measurement
 
 
 def time_graph(fn_list, reps=5, inner=1):
